@@ -1,0 +1,545 @@
+// The recurrence of a matrix state per head with one decay per token and head, written out over chunks of tokens:
+//
+//   S <- decay_t S + take_t k_t v_t^T,  n <- decay_t n + take_t k_t,   y_t = S^T q_t,  nq_t = n . q_t
+//
+// (`outer_state_scan_kernel` of recurrent.cu walks the same recurrence token by token.) With i, j tokens of a chunk and
+// W_ij = take_j decay_(j+1) .. decay_i, the chunk's outputs are
+//   y_i = (decay_0 .. decay_i) S0^T q_i + sum_{j <= i} W_ij (q_i . k_j) v_j
+// and its state afterwards is  (decay_0 .. decay_last) S0 + sum_j W_(last)j k_j v_j^T.  Three launches: (1) `parts`: every
+// chunk's own sum; (2) `chain`: the states before every chunk; (3) `outputs`.
+// What bounds it: the scan is a chain of one update per token (0.12 microseconds each, whatever the width of the GPU); here
+// the chain is one step per 128 tokens and everything else is products. Measured on one prompt of 2,048 tokens, 7 heads of
+// 64 x 128: 253 -> 27 microseconds; on 4,206 tokens in three sequences, 32 heads of 128 x 128: 773 -> 197.
+// (One block walking a sequence's chunks with its tile of S in registers moves fewer bytes than parts and chain, and took
+// 46 and 105 microseconds where these take 16 and 71: a link of that chain is a chunk's products, 3 microseconds.)
+// 128 tokens per chunk: with 64 the records (32 heads x 64 KB a chunk) are twice the bytes, with 256 the products inside
+// a chunk outgrow the others.
+//
+// Precision. q, k and v are bfloat16 numbers, so q . k is a bfloat16 product with float32 sums as it stands. Everything that
+// is float32 in the recurrence stays so: a float32 operand (S, the weighted scores, the weighted values) is cut into three
+// bfloat16 numbers whose sum is that operand exactly (eight bits of the significand each), one product for each. The
+// weights are products of decays, never quotients or differences of logarithms: a chunk is cut into eighths of 16 tokens,
+// and W_ij is (decays from the start of i's eighth to i) x (decays of the whole eighths between) x (decays behind j to the
+// end of j's eighth), each factor at most as large as the decays make it, so nothing overflows or cancels.
+#include <type_traits>
+
+#include "mma.cuh"
+
+#define SC_CHUNK 128
+#define SC_SUB 16
+#define SC_VT 64              // columns of v of a block, both kernels
+
+// x = hi + mid + lo, each a bfloat16 number (the upper half of a float32): cut off, subtract (exactly), twice.
+struct Thirds {
+    uint32_t hi, mid, lo;     // two neighbouring numbers each, the first in the lower half
+};
+__device__ __forceinline__ Thirds thirds(float x0, float x1) {
+    Thirds r;
+    uint32_t a = __float_as_uint(x0), b = __float_as_uint(x1);
+    r.hi = __byte_perm(a, b, 0x7632);
+    float s0 = x0 - __uint_as_float(a & 0xffff0000u), s1 = x1 - __uint_as_float(b & 0xffff0000u);
+    a = __float_as_uint(s0), b = __float_as_uint(s1);
+    r.mid = __byte_perm(a, b, 0x7632);
+    s0 -= __uint_as_float(a & 0xffff0000u), s1 -= __uint_as_float(b & 0xffff0000u);
+    r.lo = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);
+    return r;
+}
+__device__ __forceinline__ float lower_bf16(uint32_t pair) { return __uint_as_float(pair << 16); }
+__device__ __forceinline__ float upper_bf16(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
+
+// Byte offset of 16-byte piece `piece` of row `row` in a tile of WIDTH bfloat16 columns, pieces permuted so that eight
+// neighbouring rows read at one piece lie in eight different bank groups.
+template <int WIDTH>
+__device__ __forceinline__ uint32_t tile_at(int row, int piece) {
+    return (uint32_t)(row * (2 * WIDTH) + ((piece ^ (row & 7)) << 4));
+}
+// `rows` rows of a [.][WIDTH] tile from global rows `stride` elements apart; rows from n_here on become zeros.
+template <int WIDTH>
+__device__ __forceinline__ void fetch_tile(unsigned char* dst, const bf16* src, int stride, int n_here, int first, int threads) {
+    constexpr int PIECES = WIDTH / 8;
+    for (int i = first; i < SC_CHUNK * PIECES; i += threads) {
+        const int row = i / PIECES, piece = i % PIECES;
+        const bool there = row < n_here;
+        cp_async_16(dst + tile_at<WIDTH>(row, piece), there ? src + (size_t)row * stride + piece * 8 : src, there);
+    }
+}
+// The first record of a sequence: sequence s owns records cu_q[s] / SC_CHUNK + s onwards, as many as its chunks at most.
+__device__ __forceinline__ long long first_record(const int* cu_q, int seq) { return cu_q[seq] / SC_CHUNK + seq; }
+
+struct ChunkArgs {
+    const bf16 *q, *k, *v;
+    int q_stride, k_stride, v_stride;
+    const float *decay, *take;      // [T][heads]
+    const int *cu_q, *slots;
+    float* state;
+    long long slot_stride, s_offset, n_offset;   // n_offset < 0: no vector n
+    int n_heads, n_groups, vdim;
+    float q_scale;
+    float *records, *n_records, *whole;   // [record][heads][vdim][D], [record][heads][D], [record][heads]
+    float *y, *nq;
+};
+
+// ------------------------------------------------------------------------------------------------------------------
+// (1) A chunk's own part of the state after it, sum_j W_(last)j k_j v_j^T, for 64 columns of v (16 per warp) and all rows of S.
+// The products are S^T += (weighted v)^T k: rows of v, columns of k, so that a warp weights and cuts its own 16 columns of v
+// and nobody else's (about 400 instructions, against 3 D / 8 x 8 products). The fifth warp, where it is launched, makes the
+// part of n beside them (blocks of the first 64 columns only).
+template <int D>
+__global__ void __launch_bounds__(160)
+chunk_parts_kernel(const ChunkArgs a) {
+    grid_chain_entry();
+    extern __shared__ __align__(128) unsigned char sc_smem[];
+    unsigned char* k_s = sc_smem;                              // [128][D]
+    unsigned char* v_s = sc_smem + SC_CHUNK * D * 2;           // [128][64]
+    __shared__ __align__(16) float weight_s[SC_CHUNK];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunk = blockIdx.x, seq = blockIdx.z;
+    const int v_tiles = a.vdim / SC_VT, head = blockIdx.y / v_tiles, v0 = (blockIdx.y % v_tiles) * SC_VT;
+    const int t0 = a.cu_q[seq] + chunk * SC_CHUNK, n_here = min(SC_CHUNK, a.cu_q[seq + 1] - t0);
+    if (n_here <= 0) return;
+    const int group = head / (a.n_heads / a.n_groups);
+    fetch_tile<SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, blockDim.x);
+    fetch_tile<D>(k_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, blockDim.x);
+    cp_async_commit();
+    const long long record = (first_record(a.cu_q, seq) + chunk) * a.n_heads + head;
+    if (warp == 0) {
+        // What a token adds counts at the chunk's end: its take and the decays behind it. Four neighbouring tokens per lane,
+        // the products over the lanes above by shuffles.
+        float dec[4], w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const bool there = 4 * lane + e < n_here;
+            const size_t at = (size_t)(t0 + 4 * lane + e) * a.n_heads + head;
+            dec[e] = there ? a.decay[at] : 1.f;
+            w[e] = there ? a.take[at] : 0.f;
+        }
+        float inclusive = (dec[0] * dec[1]) * (dec[2] * dec[3]);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float above = __shfl_down_sync(0xffffffffu, inclusive, o);
+            if (lane + o < 32) inclusive *= above;
+        }
+        float behind = __shfl_down_sync(0xffffffffu, inclusive, 1);
+        if (lane == 31) behind = 1.f;
+#pragma unroll
+        for (int e = 3; e >= 0; --e) {
+            w[e] *= behind;
+            behind *= dec[e];
+        }
+        *reinterpret_cast<float4*>(weight_s + 4 * lane) = make_float4(w[0], w[1], w[2], w[3]);
+        if (lane == 0 && v0 == 0) a.whole[record] = inclusive;
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (warp == 4) {
+        if (v0 != 0) return;
+#pragma unroll
+        for (int u = 0; u < D / 32; ++u) {
+            const int d = lane + 32 * u;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+            for (int j = 0; j < SC_CHUNK; ++j)
+                sum[j & 3] = fmaf(weight_s[j], __bfloat162float(*reinterpret_cast<const bf16*>(k_s + tile_at<D>(j, d >> 3) + (d & 7) * 2)), sum[j & 3]);
+            a.n_records[record * D + d] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        }
+        return;
+    }
+    const int g = lane >> 2, t2 = (lane & 3) * 2;
+    float acc[D / 8][4];
+#pragma unroll
+    for (int nt = 0; nt < D / 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[nt][e] = 0.f;
+#pragma unroll 2
+    for (int kk = 0; kk < SC_CHUNK / 16; ++kk) {
+        // (v^T): rows of v's 16 columns, columns of 16 tokens
+        uint32_t raw[4], hi[4], mid[4], lo[4];
+        ldmatrix_x4_trans(raw, v_s + tile_at<SC_VT>(kk * 16 + (lane & 7) + ((lane >> 4) << 3), warp * 2 + ((lane >> 3) & 1)));
+        const float2 w0 = *reinterpret_cast<const float2*>(weight_s + kk * 16 + t2);
+        const float2 w1 = *reinterpret_cast<const float2*>(weight_s + kk * 16 + 8 + t2);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float2 w = r < 2 ? w0 : w1;
+            const Thirds x = thirds(lower_bf16(raw[r]) * w.x, upper_bf16(raw[r]) * w.y);
+            hi[r] = x.hi, mid[r] = x.mid, lo[r] = x.lo;
+        }
+#pragma unroll
+        for (int n4 = 0; n4 < D / 16; n4 += 4) {   // eight accumulators in turn: no product waits for the one before it
+            uint32_t b[4][4];
+#pragma unroll
+            for (int np = 0; np < 4; ++np) ldmatrix_x4_trans(b[np], k_s + tile_at<D>(kk * 16 + (lane & 15), (n4 + np) * 2 + (lane >> 4)));
+            auto part = [&](const uint32_t (&x)[4]) {
+#pragma unroll
+                for (int np = 0; np < 4; ++np) {
+                    mma_bf16_16816(acc[2 * (n4 + np)], x, b[np][0], b[np][1]);
+                    mma_bf16_16816(acc[2 * (n4 + np) + 1], x, b[np][2], b[np][3]);
+                }
+            };
+            part(lo);
+            part(mid);
+            part(hi);
+        }
+    }
+    float* rec = a.records + record * D * a.vdim + (size_t)(v0 + warp * 16 + g) * D + t2;
+#pragma unroll
+    for (int nt = 0; nt < D / 8; ++nt) {
+        *reinterpret_cast<float2*>(rec + nt * 8) = make_float2(acc[nt][0], acc[nt][1]);
+        *reinterpret_cast<float2*>(rec + 8 * D + nt * 8) = make_float2(acc[nt][2], acc[nt][3]);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// (2) The states before every chunk, in the place of the chunks' own parts, and the one after the last in the sequence's state: a
+// thread takes four neighbouring rows of S in one column of v and walks the chunks with eight records' loads on their way (a
+// link of the chain is one multiply-add; the records come from L2). A warp's 32 threads are 8 columns x 16 rows: whole
+// sectors of the records and, transposed, of the state. The last block of a head takes n.
+template <int D>
+__global__ void __launch_bounds__(256)
+chunk_chain_kernel(const ChunkArgs a) {
+    grid_chain_entry();
+    constexpr int AHEAD = 8;
+    const int lane = threadIdx.x & 31, head = blockIdx.y, seq = blockIdx.z;
+    const int len = a.cu_q[seq + 1] - a.cu_q[seq], slot = a.slots[seq];
+    const int n_chunks = (len + SC_CHUNK - 1) / SC_CHUNK;
+    if (n_chunks <= 0) return;
+    const long long first = first_record(a.cu_q, seq) * a.n_heads + head;
+    float* kept = slot >= 0 ? a.state + slot * a.slot_stride : nullptr;
+    const float* whole = a.whole + first;
+    const int item = (int)blockIdx.x * 8 + (threadIdx.x >> 5);   // (8 columns of v, 16 rows of S)
+    const int items = a.vdim / 8 * (D / 16);
+    if (item >= items) {
+        if (item != items || a.n_offset < 0) return;   // one warp of the grid carries n
+        float* n_kept = kept ? kept + a.n_offset + (long long)head * D : nullptr;
+        for (int d = lane; d < D; d += 32) {
+            float n = n_kept ? n_kept[d] : 0.f;
+            for (int c = 0; c < n_chunks; ++c) {
+                float* at = a.n_records + (first + (long long)c * a.n_heads) * D + d;
+                const float part = *at;
+                *at = n;
+                n = fmaf(n, whole[(long long)c * a.n_heads], part);
+            }
+            if (n_kept) n_kept[d] = n;
+        }
+        return;
+    }
+    const int col = item / (D / 16) * 8 + (lane >> 2), row = item % (D / 16) * 16 + (lane & 3) * 4;
+    const long long pitch = (long long)a.n_heads * D * a.vdim;
+    float* at = a.records + first * D * a.vdim + (size_t)col * D + row;
+    float* s_kept = kept ? kept + a.s_offset + ((long long)head * D + row) * a.vdim + col : nullptr;
+    float s[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] = s_kept ? s_kept[(size_t)e * a.vdim] : 0.f;
+    float4 part[AHEAD];
+    float w[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+        if (u < n_chunks) {
+            part[u] = *reinterpret_cast<const float4*>(at + u * pitch);
+            w[u] = whole[(long long)u * a.n_heads];
+        }
+    for (int c0 = 0; c0 < n_chunks; c0 += AHEAD, at += AHEAD * pitch) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (c0 + u < n_chunks) {
+                const float4 mine = part[u];
+                const float all = w[u];
+                if (c0 + u + AHEAD < n_chunks) {
+                    part[u] = *reinterpret_cast<const float4*>(at + (u + AHEAD) * pitch);
+                    w[u] = whole[(long long)(c0 + u + AHEAD) * a.n_heads];
+                }
+                *reinterpret_cast<float4*>(at + u * pitch) = make_float4(s[0], s[1], s[2], s[3]);
+                s[0] = fmaf(s[0], all, mine.x), s[1] = fmaf(s[1], all, mine.y);
+                s[2] = fmaf(s[2], all, mine.z), s[3] = fmaf(s[3], all, mine.w);
+            }
+    }
+    if (s_kept) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s_kept[(size_t)e * a.vdim] = s[e];
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// (3) Outputs of one chunk, one head, 64 columns of v. Four warps; a warp takes the chunk's eighths w and 7 - w (16 tokens each),
+// so that all have the same part of the triangle, and one load of a key's, value's or state's fragment serves both. First
+// S0^T q on the record's three parts, scaled by the decays up to the row; then, 16 earlier tokens at a time, scores, weights,
+// and the products with v added on top. Queries move to registers before the keys arrive in the same place, so that two
+// blocks fit an SM.
+template <int D>
+__global__ void __launch_bounds__(128, 2)
+chunk_outputs_kernel(const ChunkArgs a) {
+    grid_chain_entry();
+    extern __shared__ __align__(128) unsigned char sc_smem[];
+    constexpr int QK_BYTES = SC_CHUNK * D * 2, V_BYTES = SC_CHUNK * SC_VT * 2, S_PART = SC_VT * D * 2, SUBS = SC_CHUNK / SC_SUB;
+    unsigned char* qk_s = sc_smem;                 // [128][D]: the queries, then the keys
+    unsigned char* v_s = qk_s + QK_BYTES;          // [128][64]
+    unsigned char* s_s = v_s + V_BYTES;            // [3][64][D]: the state before the chunk, transposed, in three parts
+    __shared__ __align__(16) float decay_s[SC_CHUNK], upto_s[SC_CHUNK], behind_s[SC_CHUNK], n_s[D];
+    __shared__ float inner_s[SUBS][SC_SUB][SC_SUB + 1];   // W of one eighth: row, column
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunk = blockIdx.x, seq = blockIdx.z;
+    const int v_tiles = a.vdim / SC_VT, head = blockIdx.y / v_tiles, v0 = (blockIdx.y % v_tiles) * SC_VT;
+    const int t0 = a.cu_q[seq] + chunk * SC_CHUNK, n_here = min(SC_CHUNK, a.cu_q[seq + 1] - t0);
+    if (n_here <= 0) return;
+    const int group = head / (a.n_heads / a.n_groups);
+    const bool with_n = a.n_offset >= 0 && v0 == 0;
+    const long long record = (first_record(a.cu_q, seq) + chunk) * a.n_heads + head;
+
+    fetch_tile<D>(qk_s, a.q + (size_t)t0 * a.q_stride + group * D, a.q_stride, n_here, threadIdx.x, 128);
+    cp_async_commit();
+    fetch_tile<SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, 128);
+    cp_async_commit();
+    const bool there = threadIdx.x < n_here;       // this thread's token of the chunk
+    const size_t gate_at = (size_t)(t0 + threadIdx.x) * a.n_heads + head;
+    const float my_take = there ? a.take[gate_at] : 0.f;
+    decay_s[threadIdx.x] = there ? a.decay[gate_at] : 1.f;
+    if (with_n && threadIdx.x < D) n_s[threadIdx.x] = a.n_records[record * D + threadIdx.x];
+    const float* rec = a.records + record * D * a.vdim + (size_t)v0 * D;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        constexpr int EACH = SC_VT * D / 4 / 128 / 2;
+        float4 held[EACH];
+#pragma unroll
+        for (int u = 0; u < EACH; ++u) held[u] = *reinterpret_cast<const float4*>(rec + 4 * (threadIdx.x + 128 * (half * EACH + u)));
+#pragma unroll
+        for (int u = 0; u < EACH; ++u) {
+            const int i = 4 * (threadIdx.x + 128 * (half * EACH + u)), row = i / D, col = i % D;
+            const Thirds x = thirds(held[u].x, held[u].y), z = thirds(held[u].z, held[u].w);
+            unsigned char* at = s_s + tile_at<D>(row, col >> 3) + (col & 7) * 2;
+            *reinterpret_cast<uint2*>(at) = make_uint2(x.hi, z.hi);
+            *reinterpret_cast<uint2*>(at + S_PART) = make_uint2(x.mid, z.mid);
+            *reinterpret_cast<uint2*>(at + 2 * S_PART) = make_uint2(x.lo, z.lo);
+        }
+    }
+    cp_async_wait<1>();
+    __syncthreads();
+
+    const int tile[2] = {7 - warp, warp};             // this warp's eighths, the later one first
+    const int g = lane >> 2, t2 = (lane & 3) * 2;
+    uint32_t q_frag[2][D / 16][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int kd = 0; kd < D / 16; ++kd)
+            ldmatrix_x4(q_frag[m][kd], qk_s + tile_at<D>(tile[m] * 16 + (lane & 15), kd * 2 + (lane >> 4)));
+    {   // the weights' factors: a thread takes a token
+        const int sub = threadIdx.x / SC_SUB, p = threadIdx.x % SC_SUB;
+        float dec[SC_SUB], upto = 1.f, w = my_take;
+#pragma unroll
+        for (int l = 0; l < SC_SUB; l += 4) *reinterpret_cast<float4*>(dec + l) = *reinterpret_cast<const float4*>(decay_s + sub * SC_SUB + l);
+#pragma unroll
+        for (int l = 0; l < SC_SUB; ++l) {
+            if (l <= p) upto *= dec[l];
+            else w *= dec[l];
+            if (l >= p) inner_s[sub][l][p] = w;
+        }
+        upto_s[threadIdx.x] = upto;
+        behind_s[threadIdx.x] = w;     // (row 15 of the eighth: every decay behind the token)
+    }
+    cp_async_wait<0>();
+    __syncthreads();                   // the queries are in registers, v has arrived
+    fetch_tile<D>(qk_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, 128);
+    cp_async_commit();
+    // A row of v that is not finite must not reach the tokens before it through a weight of zero: looked for here, kept apart below.
+    int odd = 0;
+#pragma unroll
+    for (int i = 0; i < V_BYTES / 16 / 128; ++i) {
+        const uint4 x = *reinterpret_cast<const uint4*>(v_s + 16 * (threadIdx.x + 128 * i));
+        const uint32_t parts[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) odd |= (parts[e] & 0x7f80u) == 0x7f80u || (parts[e] & 0x7f800000u) == 0x7f800000u;
+    }
+
+    // ---- what the state before the chunk says
+    float acc[2][SC_VT / 8][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int nt = 0; nt < SC_VT / 8; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[m][nt][e] = 0.f;
+    float n_sum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};   // n . q of rows g and g + 8 (this thread's part), then the scores' sums as well
+#pragma unroll
+    for (int kd = 0; kd < D / 16; ++kd) {
+#pragma unroll
+        for (int part = 2; part >= 0; --part)
+#pragma unroll
+            for (int vp = 0; vp < SC_VT / 16; ++vp) {
+                uint32_t b[4];
+                ldmatrix_x4(b, s_s + part * S_PART + tile_at<D>(vp * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)));
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    mma_bf16_16816(acc[m][2 * vp], q_frag[m][kd], b[0], b[1]);
+                    mma_bf16_16816(acc[m][2 * vp + 1], q_frag[m][kd], b[2], b[3]);
+                }
+            }
+        if (with_n) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float* n_at = n_s + kd * 16 + (r >> 1) * 8 + t2;
+                    n_sum[m][r & 1] = fmaf(lower_bf16(q_frag[m][kd][r]), n_at[0], n_sum[m][r & 1]);
+                    n_sum[m][r & 1] = fmaf(upper_bf16(q_frag[m][kd][r]), n_at[1], n_sum[m][r & 1]);
+                }
+        }
+    }
+    cp_async_wait<0>();
+    const bool not_finite = __syncthreads_or(odd) != 0;   // (and the keys have arrived)
+    float f[2][2];                     // the decays from the eighth in hand up to rows g and g + 8, and the scale of q
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        f[m][0] = upto_s[tile[m] * 16 + g] * a.q_scale, f[m][1] = upto_s[tile[m] * 16 + g + 8] * a.q_scale;
+        float before = 1.f;            // the decays of the whole eighths before this one
+        for (int c = 0; c < tile[m]; ++c) before *= upto_s[c * 16 + 15];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float all = f[m][r] * before;
+#pragma unroll
+            for (int nt = 0; nt < SC_VT / 8; ++nt) acc[m][nt][2 * r] *= all, acc[m][nt][2 * r + 1] *= all;
+            n_sum[m][r] *= all;
+        }
+    }
+
+    // ---- what the chunk's own tokens say, from each eighth's own tokens back to the chunk's first
+    auto eighth = [&](int c, auto both) {   // eighth c, seen by the warp's later eighth, or by both
+        constexpr int M = decltype(both)::value ? 2 : 1;
+        float s[M][2][4], s_odd[M][2][4];   // (two sums each, so that a product waits for the one before the last)
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[m][h][e] = s_odd[m][h][e] = 0.f;
+#pragma unroll
+        for (int kd = 0; kd < D / 16; ++kd) {
+            uint32_t b[4];
+            ldmatrix_x4(b, qk_s + tile_at<D>(c * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)));
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                auto& sum = kd & 1 ? s_odd[m] : s[m];
+                mma_bf16_16816(sum[0], q_frag[m][kd], b[0], b[1]);
+                mma_bf16_16816(sum[1], q_frag[m][kd], b[2], b[3]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[m][h][e] += s_odd[m][h][e];
+        uint32_t hi[M][4], mid[M][4], lo[M][4];
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            if (c == tile[m]) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int row = g + (e >> 1) * 8, col = h * 8 + t2 + (e & 1);
+                        s[m][h][e] = col <= row ? s[m][h][e] * a.q_scale * inner_s[c][row][col] : 0.f;
+                    }
+            } else {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float2 w = *reinterpret_cast<const float2*>(behind_s + c * 16 + h * 8 + t2);
+                    s[m][h][0] *= f[m][0] * w.x, s[m][h][1] *= f[m][0] * w.y;
+                    s[m][h][2] *= f[m][1] * w.x, s[m][h][3] *= f[m][1] * w.y;
+                }
+                const float all = upto_s[c * 16 + 15];
+                f[m][0] *= all, f[m][1] *= all;
+            }
+            n_sum[m][0] += (s[m][0][0] + s[m][0][1]) + (s[m][1][0] + s[m][1][1]);
+            n_sum[m][1] += (s[m][0][2] + s[m][0][3]) + (s[m][1][2] + s[m][1][3]);
+            if (c == tile[m] && not_finite) {   // token by token, so that what lies behind a row is left out and not multiplied by zero
+#pragma unroll 1
+                for (int j = 0; j < SC_SUB; ++j) {
+                    const int from = (lane & ~3) | ((j & 7) >> 1);
+                    const float w0 = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? s[m][0][1] : s[m][0][0]) : (j & 1 ? s[m][1][1] : s[m][1][0]), from);
+                    const float w1 = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? s[m][0][3] : s[m][0][2]) : (j & 1 ? s[m][1][3] : s[m][1][2]), from);
+#pragma unroll
+                    for (int nt = 0; nt < SC_VT / 8; ++nt) {
+                        const uint32_t x = *reinterpret_cast<const uint32_t*>(v_s + tile_at<SC_VT>(c * 16 + j, nt) + t2 * 2);
+                        if (j <= g) acc[m][nt][0] = fmaf(w0, lower_bf16(x), acc[m][nt][0]), acc[m][nt][1] = fmaf(w0, upper_bf16(x), acc[m][nt][1]);
+                        if (j <= g + 8) acc[m][nt][2] = fmaf(w1, lower_bf16(x), acc[m][nt][2]), acc[m][nt][3] = fmaf(w1, upper_bf16(x), acc[m][nt][3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const Thirds x = thirds(s[m][r >> 1][(r & 1) * 2], s[m][r >> 1][(r & 1) * 2 + 1]);
+                hi[m][r] = x.hi, mid[m][r] = x.mid, lo[m][r] = x.lo;
+            }
+        }
+        uint32_t b[SC_VT / 16][4];
+#pragma unroll
+        for (int vp = 0; vp < SC_VT / 16; ++vp) ldmatrix_x4_trans(b[vp], v_s + tile_at<SC_VT>(c * 16 + (lane & 15), vp * 2 + (lane >> 4)));
+        auto part = [&](const uint32_t (&x)[M][4]) {
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                if (c == tile[m] && not_finite) continue;
+#pragma unroll
+                for (int vp = 0; vp < SC_VT / 16; ++vp) {
+                    mma_bf16_16816(acc[m][2 * vp], x[m], b[vp][0], b[vp][1]);
+                    mma_bf16_16816(acc[m][2 * vp + 1], x[m], b[vp][2], b[vp][3]);
+                }
+            }
+        };
+        part(lo);
+        part(mid);
+        part(hi);
+    };
+    for (int c = tile[0]; c > tile[1]; --c) eighth(c, std::false_type{});
+    for (int c = tile[1]; c >= 0; --c) eighth(c, std::true_type{});
+
+    const int width = a.n_heads * a.vdim;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const int row = tile[m] * 16 + g;
+        float* y0 = a.y + (size_t)(t0 + row) * width + head * a.vdim + v0 + t2;
+#pragma unroll
+        for (int nt = 0; nt < SC_VT / 8; ++nt) {
+            if (row < n_here) *reinterpret_cast<float2*>(y0 + nt * 8) = make_float2(acc[m][nt][0], acc[m][nt][1]);
+            if (row + 8 < n_here) *reinterpret_cast<float2*>(y0 + 8 * (size_t)width + nt * 8) = make_float2(acc[m][nt][2], acc[m][nt][3]);
+        }
+        if (with_n) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                float sum = n_sum[m][r];
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                if ((lane & 3) == 0 && row + 8 * r < n_here) a.nq[(size_t)(t0 + row + 8 * r) * a.n_heads + head] = sum;
+            }
+        }
+    }
+}
+
+template <int D>
+static int launch_chunks(const ChunkArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
+    const dim3 grid((max_q_len + SC_CHUNK - 1) / SC_CHUNK, a.vdim / SC_VT * a.n_heads, n_seqs);
+    constexpr size_t parts_smem = (size_t)SC_CHUNK * D * 2 + SC_CHUNK * SC_VT * 2, outputs_smem = parts_smem + 3 * (size_t)SC_VT * D * 2;
+    cudaError_t e = cudaFuncSetAttribute(chunk_parts_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)parts_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_outputs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outputs_smem);
+    if (e == cudaSuccess) e = launch_pdl(chunk_parts_kernel<D>, grid, dim3(a.n_offset >= 0 ? 160 : 128), parts_smem, stream, a);
+    const int items = a.vdim / 8 * (D / 16) + (a.n_offset >= 0 ? 1 : 0);
+    if (e == cudaSuccess) e = launch_pdl(chunk_chain_kernel<D>, dim3((items + 7) / 8, a.n_heads, n_seqs), dim3(256), 0, stream, a);
+    if (e == cudaSuccess) e = launch_pdl(chunk_outputs_kernel<D>, grid, dim3(128), outputs_smem, stream, a);
+    return (int)e;
+}
+
+// Whether the kernels are instantiated for these sizes (a state of dim x vdim per head).
+QF_EXPORT int qf_state_chunks_take(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim > 0 && vdim % SC_VT == 0; }
+
+// q, k: bfloat16 [T][groups * dim], v: bfloat16 [T][heads * vdim], rows strided in whole eights and 16-byte aligned; decay, take:
+// float32 [T][heads]; y: float32 [T][heads * vdim]; nq: float32 [T][heads] or null (then n_offset < 0). scratch: float32
+// [(n_tokens / 128 + n_seqs)][heads][dim * vdim + dim + 1], 16-byte aligned. max_q_len: the most tokens any sequence brings.
+QF_EXPORT int qf_state_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay,
+                              const float* take, const int* cu_q, const int* slots, int n_seqs, int max_q_len, float* state,
+                              long long slot_stride, long long s_offset, long long n_offset, int n_heads, int n_groups, int dim,
+                              int vdim, float q_scale, float* scratch, long long n_records, float* y, float* nq, cudaStream_t stream) {
+    if (n_seqs <= 0 || max_q_len <= 0) return 0;
+    if (!qf_state_chunks_take(dim, vdim) || n_groups <= 0 || n_heads <= 0 || n_heads % n_groups || n_seqs > 65535 ||
+        (long long)n_heads * (vdim / SC_VT) > 65535 || (n_offset >= 0 && !nq) || ((uintptr_t)scratch & 15))
+        return (int)cudaErrorInvalidValue;
+    float* n_parts = scratch + n_records * n_heads * dim * vdim;
+    const ChunkArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, decay, take, cu_q, slots, state,
+                      slot_stride, s_offset, n_offset, n_heads, n_groups, vdim, q_scale, scratch, n_parts, n_parts + n_records * n_heads * dim, y, nq};
+    return dim == 64 ? launch_chunks<64>(a, n_seqs, max_q_len, stream) : launch_chunks<128>(a, n_seqs, max_q_len, stream);
+}

@@ -1739,6 +1739,35 @@ def decay_gates(dt_pre: torch.Tensor, dt_bias: torch.Tensor, rate_log: torch.Ten
 OUTER_STATE_MAX_DIM = 256
 
 
+def _outer_state_args(who: str, q, k, v, decay, take, state, s_offset, n_offset, n_heads, n_groups, dim, vdim, y, nq) -> int:
+    """Checks the operands of the scan and of its chunked form; returns the tokens of the step."""
+    for name, t in (("q", q), ("k", k), ("v", v)):
+        _rows(name, t, q.dtype)
+    _is_bf16(q.dtype)
+    n = q.shape[0]
+    if n_groups <= 0 or n_heads % n_groups or q.shape[1] != n_groups * dim or k.shape != q.shape or v.shape != (n, n_heads * vdim):
+        raise KernelError(f"{who}: q, k must be [T, groups * dim], v [T, heads * vdim]")
+    if dim > OUTER_STATE_MAX_DIM:
+        raise KernelError(f"{who}: a state of {dim} rows per head exceeds the kernel's {OUTER_STATE_MAX_DIM}")
+    for name, t in (("decay", decay), ("take", take)):
+        if t is None and name == "take":
+            continue
+        _dev(name, t, torch.float32)
+        if t.shape != ((n, n_heads) if take is not None else (n_heads,)):
+            raise KernelError(f"{who}: {name} must be float32 [T, heads] (decay alone: [heads])")
+    _dev("y", y, torch.float32)
+    if y.shape != (n, n_heads * vdim):
+        raise KernelError(f"{who}: y must be float32 [T, heads * vdim]")
+    pieces = [(s_offset, n_heads * dim * vdim)]
+    if nq is not None:
+        _dev("nq", nq, torch.float32)
+        if nq.shape != (n, n_heads):
+            raise KernelError(f"{who}: nq must be float32 [T, heads]")
+        pieces.append((n_offset, n_heads * dim))
+    _state(state, *pieces)
+    return n
+
+
 def outer_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, take: Optional[torch.Tensor],
                      cu_q: torch.Tensor, slots: torch.Tensor, state: torch.Tensor, s_offset: int, n_offset: int,
                      n_heads: int, n_groups: int, dim: int, vdim: int, q_scale: float, y: torch.Tensor,
@@ -1749,35 +1778,46 @@ def outer_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
     and, with `nq`, a vector n <- decay_t n + take_t k_t beside it (at n_offset, [heads, dim]) and nq_t = n . (q_scale q_t).
     q, k: [T, groups * dim] (head h reads group h // (heads / groups)), v: [T, heads * vdim], in the activation dtype, rows
     may be strided; decay, take: float32 [T, heads]; y: float32 [T, heads * vdim]; nq: float32 [T, heads] or None."""
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        _rows(name, t, q.dtype)
-    _is_bf16(q.dtype)
-    n = q.shape[0]
-    if n_groups <= 0 or n_heads % n_groups or q.shape[1] != n_groups * dim or k.shape != q.shape or v.shape != (n, n_heads * vdim):
-        raise KernelError("outer_state_scan: q, k must be [T, groups * dim], v [T, heads * vdim]")
-    if dim > OUTER_STATE_MAX_DIM:
-        raise KernelError(f"outer_state_scan: a state of {dim} rows per head exceeds the kernel's {OUTER_STATE_MAX_DIM}")
-    for name, t in (("decay", decay), ("take", take)):
-        if t is None and name == "take":
-            continue
-        _dev(name, t, torch.float32)
-        if t.shape != ((n, n_heads) if take is not None else (n_heads,)):
-            raise KernelError(f"outer_state_scan: {name} must be float32 [T, heads] (decay alone: [heads])")
-    _dev("y", y, torch.float32)
-    if y.shape != (n, n_heads * vdim):
-        raise KernelError("outer_state_scan: y must be float32 [T, heads * vdim]")
-    pieces = [(s_offset, n_heads * dim * vdim)]
-    if nq is not None:
-        _dev("nq", nq, torch.float32)
-        if nq.shape != (n, n_heads):
-            raise KernelError("outer_state_scan: nq must be float32 [T, heads]")
-        pieces.append((n_offset, n_heads * dim))
-    _state(state, *pieces)
+    _outer_state_args("outer_state_scan", q, k, v, decay, take, state, s_offset, n_offset, n_heads, n_groups, dim, vdim, y, nq)
     _check(library("recurrent").qf_outer_state_scan(
         _I(_is_bf16(q.dtype)), _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay),
         _ptr(take), _ptr(cu_q), _ptr(slots), _I(cu_q.numel() - 1), _ptr(state), _LL(state.stride(0)), _LL(s_offset),
         _LL(n_offset if nq is not None else -1), _I(n_heads), _I(n_groups), _I(dim), _I(vdim), _F(q_scale), _ptr(y), _ptr(nq),
         _stream()), "outer_state_scan")
+
+
+STATE_CHUNK = 128   # SC_CHUNK of csrc/state_chunks.cu
+# The longest sequence of a step from which the chunked form is the faster one. Measured, one sequence, scan / chunks in microseconds:
+# 16 heads of 64 x 128: 96 tokens 14 / 13, 160: 26 / 15, 256: 41 / 17, 2,048: 315 / 42; 32 heads of 128 x 128: 96 tokens 23 / 20,
+# 160: 37 / 24. Three launches and a buffer instead of one launch cost the host about 10 microseconds more, which a step that is
+# issued launch by launch feels up to some 200 tokens.
+STATE_CHUNKS_MIN_TOKENS = 192
+
+
+def state_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dim: int, vdim: int, max_q_len: int) -> bool:
+    """Whether a step's recurrence runs on `state_chunks`: bfloat16 rows that 16-byte accesses can address, sizes the kernels are
+    made for, and a sequence long enough (STATE_CHUNKS_MIN_TOKENS). Otherwise `outer_state_scan` takes it."""
+    return (q.is_cuda and q.dtype == torch.bfloat16 and max_q_len >= STATE_CHUNKS_MIN_TOKENS
+            and bool(library("state_chunks").qf_state_chunks_take(_I(dim), _I(vdim)))
+            and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)))
+
+
+def state_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, take: torch.Tensor, cu_q: torch.Tensor,
+                 slots: torch.Tensor, max_q_len: int, state: torch.Tensor, s_offset: int, n_offset: int, n_heads: int, n_groups: int,
+                 dim: int, vdim: int, q_scale: float, y: torch.Tensor, nq: Optional[torch.Tensor]) -> None:
+    """`outer_state_scan` with a decay and a take per token and head, in chunks of `STATE_CHUNK` tokens on the tensor cores: the same
+    operands and results, the products' float32 operands in three bfloat16 parts each (exactly). `max_q_len`: the most tokens
+    any sequence brings. bfloat16 only (`state_chunks_take`)."""
+    n = _outer_state_args("state_chunks", q, k, v, decay, take, state, s_offset, n_offset, n_heads, n_groups, dim, vdim, y, nq)
+    n_seqs = cu_q.numel() - 1
+    if take is None or q.dtype != torch.bfloat16 or any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (q, k, v)):
+        raise KernelError("state_chunks: a take, and bfloat16 rows at strides and addresses of whole 16 bytes (state_chunks_take)")
+    records = n // STATE_CHUNK + n_seqs
+    scratch = torch.empty(records * n_heads * (dim * vdim + dim + 1), dtype=torch.float32, device=q.device)
+    _check(library("state_chunks").qf_state_chunks(
+        _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay), _ptr(take), _ptr(cu_q), _ptr(slots),
+        _I(n_seqs), _I(max_q_len), _ptr(state), _LL(state.stride(0)), _LL(s_offset), _LL(n_offset if nq is not None else -1), _I(n_heads),
+        _I(n_groups), _I(dim), _I(vdim), _F(q_scale), _ptr(scratch), _LL(records), _ptr(y), _ptr(nq), _stream()), "state_chunks")
 
 
 GATES = {"sigmoid": 0, "silu": 1}

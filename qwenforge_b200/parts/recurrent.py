@@ -58,6 +58,16 @@ from .base import Mixer, TensorSpec, fork, join, runs_side_by_side
 from .registry import build_part, register_part
 
 
+def _scan(ctx, q, k, v, decay, take, state, s_offset, n_offset, heads, groups, dim, vdim, q_scale, y, nq):
+    """The recurrence with a decay and a take per token and head: in chunks on the tensor cores where the step and its sizes allow
+    (`ops.state_chunks`), token by token otherwise (short steps, float32, other sizes)."""
+    if not ctx.is_decode and ops.state_chunks_take(q, k, v, dim, vdim, ctx.max_q_len):
+        ops.state_chunks(q, k, v, decay, take, ctx.cu_q, ctx.slots, ctx.max_q_len, state, s_offset, n_offset, heads, groups, dim, vdim,
+                         q_scale, y, nq)
+    else:
+        ops.outer_state_scan(q, k, v, decay, take, ctx.cu_q, ctx.slots, state, s_offset, n_offset, heads, groups, dim, vdim, q_scale, y, nq)
+
+
 class MatrixMemory(Mixer):
     """params: hidden_size, num_heads, head_dim, value_dim, gate_cap, eps, floor.
     tensors: q_weight, k_weight [H*dim, W], v_weight, g_weight [H*vdim, W], o_weight [W, H*vdim], norm [H*vdim],
@@ -85,7 +95,7 @@ class MatrixMemory(Mixer):
                 TensorSpec(f("i_bias"), (h,), init="bias", keep="float32"), TensorSpec(f("f_bias"), (h,), init="bias", keep="float32")]
 
     def kernel_libraries(self, dtype):
-        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm"})
+        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "state_chunks"})
 
     def cache_need(self):
         return StateNeed((self.state_floats,), torch.float32)
@@ -110,8 +120,8 @@ class MatrixMemory(Mixer):
         decay, take, floor = (torch.empty((n, h), **f32) for _ in range(3))
         ops.stabilized_gates(pre, self.gate_bias, self.cap, ctx.cu_q, ctx.slots, site.storage, self.m_offset, h, decay, take, floor)
         y, nq = torch.empty((n, h * v), **f32), torch.empty((n, h), **f32)
-        ops.outer_state_scan(proj[:, :h * d], proj[:, h * d:2 * h * d], proj[:, 2 * h * d:2 * h * d + h * v], decay, take,
-                             ctx.cu_q, ctx.slots, site.storage, self.s_offset, self.n_offset, h, h, d, v, d ** -0.5, y, nq)
+        _scan(ctx, proj[:, :h * d], proj[:, h * d:2 * h * d], proj[:, 2 * h * d:2 * h * d + h * v], decay, take, site.storage,
+              self.s_offset, self.n_offset, h, h, d, v, d ** -0.5, y, nq)
         out = torch.empty((n, h * v), dtype=x.dtype, device=x.device)
         ops.gated_group_norm(y, proj[:, 2 * h * d + h * v:], self.norm, self.eps, out, h, h, "sigmoid", False,
                              nq=nq, floor=floor, floor_add=self.floor)
@@ -150,7 +160,7 @@ class StateSpace(Mixer):
                 TensorSpec(f("o_weight"), (self.hidden, self.inner))]
 
     def kernel_libraries(self, dtype):
-        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm"})
+        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "state_chunks"})
 
     def cache_need(self):
         return StateNeed((self.state_floats,), torch.float32)
@@ -182,7 +192,7 @@ class StateSpace(Mixer):
         ops.decay_gates(dt_pre, self.dt_bias, self.rate_log, decay, take)
         y = torch.empty((n, self.inner), **f32)
         xs, b, c = xbc[:, :self.inner], xbc[:, self.inner:self.inner + g * s], xbc[:, self.inner + g * s:]
-        ops.outer_state_scan(c, b, xs, decay, take, ctx.cu_q, ctx.slots, site.storage, self.s_offset, -1, h, g, s, v, 1.0, y, None)
+        _scan(ctx, c, b, xs, decay, take, site.storage, self.s_offset, -1, h, g, s, v, 1.0, y, None)
         out = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_norm(y, main[:, :self.inner], self.norm, self.eps, out, self.norm_parts, h, "silu", True,
                              skip=self.skip, skip_x=xs)
