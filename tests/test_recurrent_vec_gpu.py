@@ -1,0 +1,52 @@
+"""The norm behind the scans in 16-byte pieces and the gates' maximum as a scan over a block, at the edges of their pieces."""
+import pytest
+import torch
+
+from tests import kernel_refs as refs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("part", [8, 64, 72, 128, 136, 256, 264, 512, 520, 2048, 2056, 4096, 4104, 8192, 8200])
+@pytest.mark.parametrize("gate,first,extras", [("sigmoid", False, "denominator"), ("silu", True, "skip"), ("silu", False, "")])
+def test_gated_group_norm_pieces(part, gate, first, extras):
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(part)
+    n, parts = 5, 3
+    c, heads = parts * part, 3
+    y, wide = torch.randn(n, c, generator=g, device=DEV), torch.randn(n, 2 * c + 8, generator=g, device=DEV).bfloat16()
+    weight = (1 + 0.2 * torch.randn(c, generator=g, device=DEV)).bfloat16()
+    more = {}
+    if extras == "denominator":
+        more = dict(nq=torch.randn(n, heads, generator=g, device=DEV), floor=torch.rand(n, heads, generator=g, device=DEV), floor_add=1e-6)
+    elif extras == "skip":
+        more = dict(skip=torch.randn(heads, generator=g, device=DEV), skip_x=wide[:, c + 8:])
+    for gates in (wide[:, :c], wide[:, 1:c + 1]):   # 16-byte places, and places that the scalar kernel takes
+        out, want = (torch.empty(n, c, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        ops.gated_group_norm(y, gates, weight, 1e-5, out, parts, heads, gate, first, **more)
+        refs.gated_group_norm(y, gates, weight, 1e-5, want, parts, heads, gate, first, **more)
+        # both sides round one float32 number to bfloat16 and so are neighbours at most; neighbours (8 significant bits) are up to
+        # 2^-7 of the value apart
+        assert float(((out.double() - want.double()).abs() / (want.double().abs() + 1e-3)).max()) <= 2 ** -7
+
+
+@pytest.mark.parametrize("lengths", [(1,), (255, 256, 257), (2047, 2048, 2049), (5000, 31)])
+def test_stabilized_gates_over_blocks_of_tokens(lengths):
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(len(lengths))
+    heads, n = 3, sum(lengths)
+    cu, slots = [0], [2, -1, 0][:len(lengths)]
+    for length in lengths:
+        cu.append(cu[-1] + length)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pre, bias = 6 * torch.randn(n, 2 * heads, generator=g, device=DEV), torch.randn(2 * heads, generator=g, device=DEV)
+    start = torch.rand(4, 20, generator=g, device=DEV)
+    results = []
+    for fn in (ops.stabilized_gates, refs.stabilized_gates):
+        state, trio = start.clone(), [torch.empty(n, heads, device=DEV) for _ in range(3)]
+        fn(pre, bias, 15.0, ints(cu), ints(slots), state, 7, heads, *trio)
+        results.append((state, *trio))
+    # m is a sum of up to a few dozen log gates of size up to 15 before a larger one takes over: 2^-24 x 15 x a few dozen
+    for got, want in zip(*results):
+        assert float(((got.double() - want.double()).abs() / (1 + want.double().abs())).max()) < 3e-5
