@@ -69,7 +69,9 @@ __device__ __forceinline__ long long first_record(const int* cu_q, int seq) { re
 struct ChunkArgs {
     const bf16 *q, *k, *v;
     int q_stride, k_stride, v_stride;
-    const float *decay, *take;      // [T][heads]
+    const float *decay, *take;      // [T][heads]; or, with rate_log, decay holds the pre-activations (rows gate_stride apart) of
+    const float *dt_bias, *rate_log;  // dt = softplus(pre + dt_bias), decay = exp(-exp(rate_log) dt), take = dt
+    int gate_stride;
     const int *cu_q, *slots;
     float* state;
     long long slot_stride, s_offset, n_offset;   // n_offset < 0: no vector n
@@ -78,6 +80,15 @@ struct ChunkArgs {
     float *records, *n_records, *whole;   // [record][heads][vdim][D], [record][heads][D], [record][heads]
     float *y, *nq;
 };
+
+// A token's decay and take (the arithmetic of `decay_gates_kernel` in recurrent.cu where they come as pre-activations: a launch
+// less, 4 microseconds of the device's time and 7 of the host's).
+__device__ __forceinline__ float2 gates_of(const ChunkArgs& a, int token, int head) {
+    const float x = a.decay[(size_t)token * a.gate_stride + head];
+    if (!a.rate_log) return make_float2(x, a.take[(size_t)token * a.gate_stride + head]);
+    const float z = x + a.dt_bias[head], dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
+    return make_float2(expf(-expf(a.rate_log[head]) * dt), dt);
+}
 
 // ------------------------------------------------------------------------------------------------------------------
 // (1) A chunk's own part of the state after it, sum_j W_(last)j k_j v_j^T, for 64 columns of v (16 per warp) and all rows of S.
@@ -107,10 +118,8 @@ chunk_parts_kernel(const ChunkArgs a) {
         float dec[4], w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const bool there = 4 * lane + e < n_here;
-            const size_t at = (size_t)(t0 + 4 * lane + e) * a.n_heads + head;
-            dec[e] = there ? a.decay[at] : 1.f;
-            w[e] = there ? a.take[at] : 0.f;
+            const float2 gate = 4 * lane + e < n_here ? gates_of(a, t0 + 4 * lane + e, head) : make_float2(1.f, 0.f);
+            dec[e] = gate.x, w[e] = gate.y;
         }
         float inclusive = (dec[0] * dec[1]) * (dec[2] * dec[3]);
 #pragma unroll
@@ -286,10 +295,9 @@ chunk_outputs_kernel(const ChunkArgs a) {
     cp_async_commit();
     fetch_tile<SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, 128);
     cp_async_commit();
-    const bool there = threadIdx.x < n_here;       // this thread's token of the chunk
-    const size_t gate_at = (size_t)(t0 + threadIdx.x) * a.n_heads + head;
-    const float my_take = there ? a.take[gate_at] : 0.f;
-    decay_s[threadIdx.x] = there ? a.decay[gate_at] : 1.f;
+    const float2 gate = threadIdx.x < n_here ? gates_of(a, t0 + threadIdx.x, head) : make_float2(1.f, 0.f);   // this thread's token
+    const float my_take = gate.y;
+    decay_s[threadIdx.x] = gate.x;
     if (with_n && threadIdx.x < D) n_s[threadIdx.x] = a.n_records[record * D + threadIdx.x];
     const float* rec = a.records + record * D * a.vdim + (size_t)v0 * D;
 #pragma unroll
@@ -524,22 +532,21 @@ static int launch_chunks(const ChunkArgs& a, int n_seqs, int max_q_len, cudaStre
     return (int)e;
 }
 
-// Whether the kernels are instantiated for these sizes (a state of dim x vdim per head).
-QF_EXPORT int qf_state_chunks_take(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim > 0 && vdim % SC_VT == 0; }
-
 // q, k: bfloat16 [T][groups * dim], v: bfloat16 [T][heads * vdim], rows strided in whole eights and 16-byte aligned; decay, take:
-// float32 [T][heads]; y: float32 [T][heads * vdim]; nq: float32 [T][heads] or null (then n_offset < 0). scratch: float32
+// float32 [T][heads] (rate_log null), or decay the pre-activations of both, rows gate_stride apart; y: float32 [T][heads * vdim]; nq: float32 [T][heads] or null (then n_offset < 0). scratch: float32
 // [(n_tokens / 128 + n_seqs)][heads][dim * vdim + dim + 1], 16-byte aligned. max_q_len: the most tokens any sequence brings.
 QF_EXPORT int qf_state_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay,
-                              const float* take, const int* cu_q, const int* slots, int n_seqs, int max_q_len, float* state,
+                              const float* take, const float* dt_bias, const float* rate_log, int gate_stride, const int* cu_q,
+                              const int* slots, int n_seqs, int max_q_len, float* state,
                               long long slot_stride, long long s_offset, long long n_offset, int n_heads, int n_groups, int dim,
                               int vdim, float q_scale, float* scratch, long long n_records, float* y, float* nq, cudaStream_t stream) {
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
-    if (!qf_state_chunks_take(dim, vdim) || n_groups <= 0 || n_heads <= 0 || n_heads % n_groups || n_seqs > 65535 ||
+    if ((dim != 64 && dim != 128) || vdim <= 0 || vdim % SC_VT || (!take && !rate_log) || ((q_stride | k_stride | v_stride) & 7) ||
+        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) || n_groups <= 0 || n_heads <= 0 || n_heads % n_groups || n_seqs > 65535 ||
         (long long)n_heads * (vdim / SC_VT) > 65535 || (n_offset >= 0 && !nq) || ((uintptr_t)scratch & 15))
         return (int)cudaErrorInvalidValue;
     float* n_parts = scratch + n_records * n_heads * dim * vdim;
-    const ChunkArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, decay, take, cu_q, slots, state,
+    const ChunkArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, decay, take, dt_bias, rate_log, gate_stride, cu_q, slots, state,
                       slot_stride, s_offset, n_offset, n_heads, n_groups, vdim, q_scale, scratch, n_parts, n_parts + n_records * n_heads * dim, y, nq};
     return dim == 64 ? launch_chunks<64>(a, n_seqs, max_q_len, stream) : launch_chunks<128>(a, n_seqs, max_q_len, stream);
 }

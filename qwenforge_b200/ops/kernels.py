@@ -1750,7 +1750,7 @@ def _outer_state_args(who: str, q, k, v, decay, take, state, s_offset, n_offset,
     if dim > OUTER_STATE_MAX_DIM:
         raise KernelError(f"{who}: a state of {dim} rows per head exceeds the kernel's {OUTER_STATE_MAX_DIM}")
     for name, t in (("decay", decay), ("take", take)):
-        if t is None and name == "take":
+        if t is None and (name == "take" or decay is take):   # (both absent: the caller's gates come as pre-activations)
             continue
         _dev(name, t, torch.float32)
         if t.shape != ((n, n_heads) if take is not None else (n_heads,)):
@@ -1778,6 +1778,8 @@ def outer_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
     and, with `nq`, a vector n <- decay_t n + take_t k_t beside it (at n_offset, [heads, dim]) and nq_t = n . (q_scale q_t).
     q, k: [T, groups * dim] (head h reads group h // (heads / groups)), v: [T, heads * vdim], in the activation dtype, rows
     may be strided; decay, take: float32 [T, heads]; y: float32 [T, heads * vdim]; nq: float32 [T, heads] or None."""
+    if decay is None:
+        raise KernelError("outer_state_scan: a decay per token and head, or one per head")
     _outer_state_args("outer_state_scan", q, k, v, decay, take, state, s_offset, n_offset, n_heads, n_groups, dim, vdim, y, nq)
     _check(library("recurrent").qf_outer_state_scan(
         _I(_is_bf16(q.dtype)), _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay),
@@ -1797,27 +1799,43 @@ STATE_CHUNKS_MIN_TOKENS = 192
 def state_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dim: int, vdim: int, max_q_len: int) -> bool:
     """Whether a step's recurrence runs on `state_chunks`: bfloat16 rows that 16-byte accesses can address, sizes the kernels are
     made for, and a sequence long enough (STATE_CHUNKS_MIN_TOKENS). Otherwise `outer_state_scan` takes it."""
-    return (q.is_cuda and q.dtype == torch.bfloat16 and max_q_len >= STATE_CHUNKS_MIN_TOKENS
-            and bool(library("state_chunks").qf_state_chunks_take(_I(dim), _I(vdim)))
-            and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)))
+    return (max_q_len >= STATE_CHUNKS_MIN_TOKENS and dim in (64, 128) and vdim % 64 == 0 and q.dtype == torch.bfloat16 and q.is_cuda
+            and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0)
 
 
-def state_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, take: torch.Tensor, cu_q: torch.Tensor,
-                 slots: torch.Tensor, max_q_len: int, state: torch.Tensor, s_offset: int, n_offset: int, n_heads: int, n_groups: int,
-                 dim: int, vdim: int, q_scale: float, y: torch.Tensor, nq: Optional[torch.Tensor]) -> None:
+def state_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: Optional[torch.Tensor], take: Optional[torch.Tensor],
+                 cu_q: torch.Tensor, slots: torch.Tensor, max_q_len: int, state: torch.Tensor, s_offset: int, n_offset: int,
+                 n_heads: int, n_groups: int, dim: int, vdim: int, q_scale: float, y: torch.Tensor, nq: Optional[torch.Tensor],
+                 decay_gates=None) -> None:
     """`outer_state_scan` with a decay and a take per token and head, in chunks of `STATE_CHUNK` tokens on the tensor cores: the same
     operands and results, the products' float32 operands in three bfloat16 parts each (exactly). `max_q_len`: the most tokens
-    any sequence brings. bfloat16 only (`state_chunks_take`)."""
+    any sequence brings. `decay_gates` = (dt_pre, dt_bias, rate_log) in the place of decay and take: the gates that the function of
+    that name makes of them, formed on the way in. bfloat16 only (`state_chunks_take`)."""
     n = _outer_state_args("state_chunks", q, k, v, decay, take, state, s_offset, n_offset, n_heads, n_groups, dim, vdim, y, nq)
+    dt_bias = rate_log = None
+    gate_stride = n_heads
+    if decay_gates is not None:
+        if decay is not None or take is not None:
+            raise KernelError("state_chunks: decay_gates stands in the place of decay and take")
+        decay, dt_bias, rate_log = decay_gates
+        _rows("dt_pre", decay, torch.float32)
+        _dev("dt_bias", dt_bias, torch.float32)
+        _dev("rate_log", rate_log, torch.float32)
+        gate_stride = decay.stride(0)
+        if decay.shape != (n, n_heads) or dt_bias.numel() != n_heads or rate_log.numel() != n_heads:
+            raise KernelError("state_chunks: dt_pre must be [T, heads], dt_bias and rate_log [heads]")
+    elif take is None:
+        raise KernelError("state_chunks: a decay and a take per token and head, or what to make them of")
+    if q.dtype != torch.bfloat16:
+        raise KernelError("state_chunks: bfloat16 rows only (state_chunks_take)")
     n_seqs = cu_q.numel() - 1
-    if take is None or q.dtype != torch.bfloat16 or any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (q, k, v)):
-        raise KernelError("state_chunks: a take, and bfloat16 rows at strides and addresses of whole 16 bytes (state_chunks_take)")
     records = n // STATE_CHUNK + n_seqs
     scratch = torch.empty(records * n_heads * (dim * vdim + dim + 1), dtype=torch.float32, device=q.device)
     _check(library("state_chunks").qf_state_chunks(
-        _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay), _ptr(take), _ptr(cu_q), _ptr(slots),
-        _I(n_seqs), _I(max_q_len), _ptr(state), _LL(state.stride(0)), _LL(s_offset), _LL(n_offset if nq is not None else -1), _I(n_heads),
-        _I(n_groups), _I(dim), _I(vdim), _F(q_scale), _ptr(scratch), _LL(records), _ptr(y), _ptr(nq), _stream()), "state_chunks")
+        _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay), _ptr(take), _ptr(dt_bias),
+        _ptr(rate_log), _I(gate_stride), _ptr(cu_q), _ptr(slots), _I(n_seqs), _I(max_q_len), _ptr(state), _LL(state.stride(0)),
+        _LL(s_offset), _LL(n_offset if nq is not None else -1), _I(n_heads), _I(n_groups), _I(dim), _I(vdim), _F(q_scale),
+        _ptr(scratch), _LL(records), _ptr(y), _ptr(nq), _stream()), "state_chunks")
 
 
 GATES = {"sigmoid": 0, "silu": 1}

@@ -58,16 +58,6 @@ from .base import Mixer, TensorSpec, fork, join, runs_side_by_side
 from .registry import build_part, register_part
 
 
-def _scan(ctx, q, k, v, decay, take, state, s_offset, n_offset, heads, groups, dim, vdim, q_scale, y, nq):
-    """The recurrence with a decay and a take per token and head: in chunks on the tensor cores where the step and its sizes allow
-    (`ops.state_chunks`), token by token otherwise (short steps, float32, other sizes)."""
-    if not ctx.is_decode and ops.state_chunks_take(q, k, v, dim, vdim, ctx.max_q_len):
-        ops.state_chunks(q, k, v, decay, take, ctx.cu_q, ctx.slots, ctx.max_q_len, state, s_offset, n_offset, heads, groups, dim, vdim,
-                         q_scale, y, nq)
-    else:
-        ops.outer_state_scan(q, k, v, decay, take, ctx.cu_q, ctx.slots, state, s_offset, n_offset, heads, groups, dim, vdim, q_scale, y, nq)
-
-
 class MatrixMemory(Mixer):
     """params: hidden_size, num_heads, head_dim, value_dim, gate_cap, eps, floor.
     tensors: q_weight, k_weight [H*dim, W], v_weight, g_weight [H*vdim, W], o_weight [W, H*vdim], norm [H*vdim],
@@ -117,14 +107,17 @@ class MatrixMemory(Mixer):
         f32 = dict(dtype=torch.float32, device=x.device)
         proj = ops.linear_rows(x, self.proj_weight)                                   # [T, q | k | v | g]
         pre = ops.linear_rows(x, self.gate_weight, out_dtype=torch.float32)           # [T, i | f], float32 sums
-        decay, take, floor = (torch.empty((n, h), **f32) for _ in range(3))
+        q, k, values, gate = proj.split((h * d, h * d, h * v, h * v), dim=1)
+        decay, take, floor, nq = torch.empty((4, n, h), **f32).unbind(0)
         ops.stabilized_gates(pre, self.gate_bias, self.cap, ctx.cu_q, ctx.slots, site.storage, self.m_offset, h, decay, take, floor)
-        y, nq = torch.empty((n, h * v), **f32), torch.empty((n, h), **f32)
-        _scan(ctx, proj[:, :h * d], proj[:, h * d:2 * h * d], proj[:, 2 * h * d:2 * h * d + h * v], decay, take, site.storage,
-              self.s_offset, self.n_offset, h, h, d, v, d ** -0.5, y, nq)
+        y = torch.empty((n, h * v), **f32)
+        sizes = (site.storage, self.s_offset, self.n_offset, h, h, d, v, d ** -0.5, y, nq)
+        if ops.state_chunks_take(q, k, values, d, v, ctx.max_q_len):   # in chunks on the tensor cores
+            ops.state_chunks(q, k, values, decay, take, ctx.cu_q, ctx.slots, ctx.max_q_len, *sizes)
+        else:                                                          # token by token: short steps, float32, other sizes
+            ops.outer_state_scan(q, k, values, decay, take, ctx.cu_q, ctx.slots, *sizes)
         out = torch.empty((n, h * v), dtype=x.dtype, device=x.device)
-        ops.gated_group_norm(y, proj[:, 2 * h * d + h * v:], self.norm, self.eps, out, h, h, "sigmoid", False,
-                             nq=nq, floor=floor, floor_add=self.floor)
+        ops.gated_group_norm(y, gate, self.norm, self.eps, out, h, h, "sigmoid", False, nq=nq, floor=floor, floor_add=self.floor)
         return ops.linear_rows(out, self.o_weight)
 
 
@@ -185,17 +178,22 @@ class StateSpace(Mixer):
         f32 = dict(dtype=torch.float32, device=x.device)
         main = ops.linear_rows(x, self.main_weight)                                   # [T, z | x | B | C]
         dt_pre = ops.linear_rows(x, self.dt_weight, out_dtype=torch.float32)          # [T, H], float32 sums
+        z, convolved = main.split((self.inner, self.channels), dim=1)
         xbc = torch.empty((n, self.channels), dtype=x.dtype, device=x.device)
-        ops.causal_conv_silu(main[:, self.inner:], self.conv_weight, self.conv_bias, ctx.cu_q, ctx.tok_seq, ctx.slots,
-                             site.storage, self.conv_offset, xbc, single=ctx.is_decode and n == ctx.n_seqs)
-        decay, take = torch.empty((n, h), **f32), torch.empty((n, h), **f32)
-        ops.decay_gates(dt_pre, self.dt_bias, self.rate_log, decay, take)
+        ops.causal_conv_silu(convolved, self.conv_weight, self.conv_bias, ctx.cu_q, ctx.tok_seq, ctx.slots, site.storage,
+                             self.conv_offset, xbc, single=ctx.is_decode and n == ctx.n_seqs)
         y = torch.empty((n, self.inner), **f32)
-        xs, b, c = xbc[:, :self.inner], xbc[:, self.inner:self.inner + g * s], xbc[:, self.inner + g * s:]
-        _scan(ctx, c, b, xs, decay, take, site.storage, self.s_offset, -1, h, g, s, v, 1.0, y, None)
+        xs, b, c = xbc.split((self.inner, g * s, g * s), dim=1)
+        sizes = (site.storage, self.s_offset, -1, h, g, s, v, 1.0, y, None)
+        if ops.state_chunks_take(c, b, xs, s, v, ctx.max_q_len):   # in chunks on the tensor cores, the gates formed inside
+            ops.state_chunks(c, b, xs, None, None, ctx.cu_q, ctx.slots, ctx.max_q_len, *sizes,
+                             decay_gates=(dt_pre, self.dt_bias, self.rate_log))
+        else:                                                      # token by token: short steps, float32, other sizes
+            decay, take = torch.empty((2, n, h), **f32).unbind(0)
+            ops.decay_gates(dt_pre, self.dt_bias, self.rate_log, decay, take)
+            ops.outer_state_scan(c, b, xs, decay, take, ctx.cu_q, ctx.slots, *sizes)
         out = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
-        ops.gated_group_norm(y, main[:, :self.inner], self.norm, self.eps, out, self.norm_parts, h, "silu", True,
-                             skip=self.skip, skip_x=xs)
+        ops.gated_group_norm(y, z, self.norm, self.eps, out, self.norm_parts, h, "silu", True, skip=self.skip, skip_x=xs)
         return ops.linear_rows(out, self.o_weight)
 
 

@@ -60,6 +60,28 @@ def test_chunks_against_the_recurrence(heads, groups, dim, vdim, with_n, lengths
         assert torch.equal(state[:, n_off:], start[:, n_off:])
 
 
+@pytest.mark.parametrize("lengths", [(1,), (130, 7)])
+def test_gates_from_their_pre_activations(lengths):
+    """The gates formed inside are those of `decay_gates` to a unit or two of their last place, whatever the rows' stride."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(5)
+    n, heads, dim, vdim = sum(lengths), 3, 128, 64
+    cu = [0, lengths[0], n][:len(lengths) + 1]
+    q, k, v = (torch.randn(n, heads * w, generator=g, device=DEV).bfloat16() for w in (dim, dim, vdim))
+    pre = 4 * torch.randn(n, heads + 2, generator=g, device=DEV)[:, :heads]
+    dt_bias, rate_log = torch.randn(heads, generator=g, device=DEV), torch.randn(heads, generator=g, device=DEV)
+    decay, take = torch.empty(n, heads, device=DEV), torch.empty(n, heads, device=DEV)
+    ops.decay_gates(pre, dt_bias, rate_log, decay, take)
+    results = []
+    for gates in ((decay, take, None), (None, None, (pre, dt_bias, rate_log))):
+        state, y = torch.ones(2, heads * dim * vdim, device=DEV), torch.empty(n, heads * vdim, device=DEV)
+        ops.state_chunks(q, k, v, *gates[:2], ints(cu), ints([1, 0][:len(lengths)]), max(lengths), state, 0, -1, heads, heads, dim, vdim, 1.0, y,
+                         None, decay_gates=gates[2])
+        results.append((y, state))
+    for got, want in zip(results[1], results[0]):
+        assert rel(got, want) < LIMIT
+
+
 def test_a_value_that_is_not_finite_reaches_no_earlier_token():
     from qwenforge_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(1)
