@@ -4,56 +4,131 @@
 // the same however the rows were grouped into calls.
 #include "mma.cuh"
 
-#define BM 64
-#define BN 64
-#define BK 16
+// Two neighbouring float32 as one 64-bit register pair: one instruction multiplies and adds both, each rounded as fmaf rounds it.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 both(float x) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float2 halves(f32x2 x) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+    return r;
+}
 
-__global__ void __launch_bounds__(256)
+// A block makes a BM x BN tile with 32 * WM * WN threads; a warp makes (BM / WM) x (BN / WN) of it, its 4 x 8 lanes TM x TN each in
+// runs of four rows and columns, so that the lanes of a warp read a k's rows and columns of both operands as whole 16-byte
+// pieces without conflicts. BK columns of K at a time, the next ones on their way through registers (they are turned on the
+// way into shared memory). What bounds it is the multiply-add pipe (72 TFLOP/s) and the last tiles' round: 1,031 rows of the
+// 0.5B model's products (30.6 GFLOP) took 1,441 microseconds with 64 x 64 tiles read by single words, 845 so; 2,048 x 22,016 x 2,048
+// runs at 51 TFLOP/s (27 before).
+template <int BM, int BN, int BK, int WM, int WN>
+__global__ void __launch_bounds__(32 * WM * WN)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
-    __shared__ float a_s[BK][BM + 1];
-    __shared__ float w_s[BK][BN + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+                float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int vec) {
+    constexpr int THREADS = 32 * WM * WN, TM = BM / WM / 4, TN = BN / WN / 8, LA = BM + 4, LW = BN + 4, Q = BK / 4;
+    constexpr int A_EACH = BM * Q / THREADS, W_EACH = BN * Q / THREADS;
+    static_assert(TM % 4 == 0 && TN % 4 == 0 && A_EACH >= 1 && W_EACH >= 1, "whole runs of four");
+    __shared__ __align__(16) float a_s[2][BK][LA], w_s[2][BK][LW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[4][4];
+    const int row0 = (warp / WN) * (BM / WM) + (lane >> 3) * 4, col0 = (warp % WN) * (BN / WN) + (lane & 7) * 4;
+    f32x2 acc[TM][TN / 2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // 64 rows x 16 k of each operand; 256 threads, 4 elements each
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int idx = threadIdx.x + i * 256;
-            const int r = idx / BK, k = idx % BK;
-            const int gm = m0 + r, gn = n0 + r, gk = k0 + k;
-            a_s[k][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.f;
-            w_s[k][r] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.f;
+    // four neighbouring k of a row per piece; rows beyond M or N and columns beyond K are zeros
+    float4 a_next[A_EACH], w_next[W_EACH];
+    auto piece = [&](const float* X, int ld, int row, int rows, int k) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < rows) {
+            const float* p = X + (size_t)row * ld + k;
+            if (vec) {
+                if (k < K) v = *reinterpret_cast<const float4*>(p);
+            } else {
+                if (k < K) v.x = p[0];
+                if (k + 1 < K) v.y = p[1];
+                if (k + 2 < K) v.z = p[2];
+                if (k + 3 < K) v.w = p[3];
+            }
         }
-        __syncthreads();
+        return v;
+    };
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < A_EACH; ++u) {
+            const int i = threadIdx.x + u * THREADS;
+            a_next[u] = piece(A, lda, m0 + i / Q, M, k0 + (i % Q) * 4);
+        }
+#pragma unroll
+        for (int u = 0; u < W_EACH; ++u) {
+            const int i = threadIdx.x + u * THREADS;
+            w_next[u] = piece(W, ldw, n0 + i / Q, N, k0 + (i % Q) * 4);
+        }
+    };
+    auto stash = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < A_EACH; ++u) {
+            const int i = threadIdx.x + u * THREADS, r = i / Q, k = (i % Q) * 4;
+            a_s[buf][k][r] = a_next[u].x, a_s[buf][k + 1][r] = a_next[u].y;
+            a_s[buf][k + 2][r] = a_next[u].z, a_s[buf][k + 3][r] = a_next[u].w;
+        }
+#pragma unroll
+        for (int u = 0; u < W_EACH; ++u) {
+            const int i = threadIdx.x + u * THREADS, r = i / Q, k = (i % Q) * 4;
+            w_s[buf][k][r] = w_next[u].x, w_s[buf][k + 1][r] = w_next[u].y;
+            w_s[buf][k + 2][r] = w_next[u].z, w_s[buf][k + 3][r] = w_next[u].w;
+        }
+    };
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    for (int k0 = 0, buf = 0; k0 < K; k0 += BK, buf ^= 1) {
+        if (k0 + BK < K) fetch(k0 + BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
-            float a[4], w[4];
+            float a[TM];
+            f32x2 w[TN / 2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = a_s[k][ty + 16 * i];
+            for (int i = 0; i < TM; i += 4) {   // runs of four rows, 16 rows apart
+                const float4 v = *reinterpret_cast<const float4*>(&a_s[buf][k][row0 + 4 * i]);
+                a[i] = v.x, a[i + 1] = v.y, a[i + 2] = v.z, a[i + 3] = v.w;
+            }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = w_s[k][tx + 16 * j];
+            for (int j = 0; j < TN; j += 4) {   // runs of four columns, 32 columns apart
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&w_s[buf][k][col0 + 8 * j]);
+                w[j / 2] = v.x, w[j / 2 + 1] = v.y;
+            }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < TM; ++i) {
+                const f32x2 ai = both(a[i]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+                for (int j = 0; j < TN / 2; ++j) acc[i][j] = fma2(ai, w[j], acc[i][j]);
+            }
         }
-        __syncthreads();
+        if (k0 + BK < K) {
+            stash(buf ^ 1);      // (read in the turn before, which ended with a barrier)
+            __syncthreads();
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty + 16 * i;
+    for (int i = 0; i < TM; ++i) {
+        const int gm = m0 + row0 + (i / 4) * 16 + i % 4;
         if (gm >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tx + 16 * j;
-            if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j] + (bias ? bias[gn] : 0.f);
+        for (int j = 0; j < TN / 2; ++j) {
+            const float2 v = halves(acc[i][j]);
+            const int gn = n0 + col0 + (j / 2) * 32 + (j % 2) * 2;
+            if (gn < N) C[(size_t)gm * ldc + gn] = v.x + (bias ? bias[gn] : 0.f);
+            if (gn + 1 < N) C[(size_t)gm * ldc + gn + 1] = v.y + (bias ? bias[gn + 1] : 0.f);
         }
     }
 }
@@ -147,7 +222,22 @@ QF_EXPORT int qf_gemm_f32(const float* A, const float* W, const float* bias, flo
         else gemm_f32_few_rows_kernel<4, 64><<<(N + 31) / 32, FR_N * FR_M, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc);
         return (int)cudaGetLastError();
     }
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    gemm_f32_kernel<<<grid, 256, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc);
+    const int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    // The tile with which the busiest SM is done first. Measured at K = 896, microseconds for 1, 2 and many tiles per SM: 64 x 128
+    // 60, 97, then 41 a tile; 64 x 64 37, 60, 25; 32 x 64 29, 44, 18 (32 x 32 was never the fastest, 128 x 128 leaves too many
+    // SMs without a last tile): a first wait and a time per tile.
+    struct { int bm, bn; float wait, each; } const tiles[] = {{64, 128, 19.f, 41.f}, {64, 64, 12.f, 25.f}, {32, 64, 10.f, 18.f}};
+    const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
+    int best = 0;
+    float least = 0.f;
+    for (int i = 0; i < 3; ++i) {
+        const long long count = (long long)((M + tiles[i].bm - 1) / tiles[i].bm) * ((N + tiles[i].bn - 1) / tiles[i].bn);
+        const float time = tiles[i].wait + (float)((count + sms - 1) / sms) * tiles[i].each;
+        if (i == 0 || time < least) best = i, least = time;
+    }
+    const dim3 grid((N + tiles[best].bn - 1) / tiles[best].bn, (M + tiles[best].bm - 1) / tiles[best].bm);
+    if (best == 0) gemm_f32_kernel<64, 128, 16, 2, 2><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec);
+    else if (best == 1) gemm_f32_kernel<64, 64, 32, 2, 2><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec);
+    else gemm_f32_kernel<32, 64, 32, 2, 2><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec);
     return (int)cudaGetLastError();
 }

@@ -1,0 +1,81 @@
+"""The float32 path's tile kernels at the edges of their tiles: the product against its own single rows, the attention against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("m", [17, 63, 64, 65, 127, 129, 300])
+@pytest.mark.parametrize("n,k", [(64, 16), (65, 20), (130, 33), (6200, 48), (19100, 17)])
+def test_products_keep_the_order_of_a_single_chain(m, n, k):
+    """Every element is one chain of fused multiply-adds over k, whatever the tile: the bits of the kernel of few rows."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    x, w, b = torch.randn(m, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV), torch.randn(n, generator=g, device=DEV)
+    out, rows = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+    ops.gemm_f32(x, w, b, out)
+    for at in range(0, m, 16):
+        ops.gemm_f32(x[at:at + 16], w, b, rows[at:at + 16])
+    assert torch.equal(out, rows)
+    wide = torch.zeros(m, k + 3, device=DEV)      # rows that no 16-byte load can address
+    wide[:, 1:k + 1] = x
+    ops.gemm_f32(wide[:, 1:k + 1], w, b, out)
+    assert torch.equal(out, rows)
+
+
+@pytest.mark.parametrize("dim,heads,kv_heads,window", [(64, 14, 2, 0), (128, 4, 4, 0), (64, 4, 1, 70), (128, 2, 1, 1)])
+def test_attention_tiles(dim, heads, kv_heads, window):
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(dim + heads + window)
+    spans = [(0, 1), (0, 64), (0, 65), (63, 130), (200, 2), (0, 40)]     # (tokens before, tokens of the step)
+    slots = [5, 3, 0, 1, 4, -1]
+    pages_each, n_slots = 5, 6
+    order = torch.randperm(n_slots * pages_each, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(n_slots, pages_each).to(DEV)
+    storage = torch.randn(n_slots * pages_each, 2, kv_heads, 64, dim, generator=g, device=DEV)
+    cu, pos, total = [0], [], 0
+    for start, n in spans:
+        cu.append(cu[-1] + n)
+        pos += range(start, start + n)
+    for (start, n), slot in zip(spans, slots):   # what a sequence has not written yet is no number
+        if slot >= 0:
+            for p in range(start + n, pages_each * 64):
+                storage[order[slot, p // 64], :, :, p % 64] = float("nan")
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q, out, err = torch.randn(cu[-1], heads * dim, generator=g, device=DEV), torch.empty(cu[-1], heads * dim, device=DEV), ints([0])
+    site = ops.KvSiteArgs(storage, order, kv_heads, dim)
+    ops.attention_generic(q, out, ints(cu), ints(pos), ints(slots), site, heads, len(spans), max(n for _, n in spans), dim ** -0.5, window, err)
+    assert int(err) == 0
+    for (start, n), slot, first in zip(spans, slots, cu):
+        got = out[first:first + n].view(n, heads, dim).double()
+        if slot < 0:
+            assert not bool(got.any())
+            continue
+        kv = storage[order[slot].long()].double().permute(1, 2, 0, 3, 4).reshape(2, kv_heads, -1, dim)[:, :, :start + n].repeat_interleave(heads // kv_heads, 1)
+        scores = torch.einsum("nhd,hkd->hnk", q[first:first + n].view(n, heads, dim).double(), kv[0]) * dim ** -0.5
+        i, j = torch.arange(start, start + n, device=DEV)[:, None], torch.arange(start + n, device=DEV)[None]
+        scores = scores.masked_fill((j > i) | ((j <= i - window) if window else torch.zeros_like(j > i)), float("-inf"))
+        want = torch.einsum("hnk,hkd->nhd", torch.softmax(scores, -1), kv[1])
+        # scores of size up to about 5 carry a rounding of 128 x 2^-24 of that at worst, the weights and sums as much again
+        assert float((got - want).abs().max()) < 2e-5 * float(want.abs().max())
+    # a row does not see what else is in the step
+    alone = torch.empty(130, heads * dim, device=DEV)
+    ops.attention_generic(q[cu[3]:cu[4]].contiguous(), alone, ints([0, 130]), ints(pos[cu[3]:cu[4]]), ints([slots[3]]), site, heads, 1, 130, dim ** -0.5, window, err)
+    assert torch.equal(alone, out[cu[3]:cu[4]])
+
+
+def test_a_value_that_is_not_finite_reaches_no_earlier_row():
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(3)
+    dim, heads, n, bad = 64, 2, 100, 70
+    storage = torch.randn(2, 2, 1, 64, dim, generator=g, device=DEV)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    site = ops.KvSiteArgs(storage, ints([[0, 1]]), 1, dim)
+    q, err, outs = torch.randn(n, heads * dim, generator=g, device=DEV), ints([0]), []
+    for value in (1.0, float("inf"), float("nan")):
+        storage[1, 1, 0, bad - 64, 5] = value
+        out = torch.empty_like(q)
+        ops.attention_generic(q, out, ints([0, n]), ints(list(range(n))), ints([0]), site, heads, 1, n, dim ** -0.5, 0, err)
+        outs.append(out.view(n, heads, dim))
+    for out in outs[1:]:
+        assert torch.equal(out[:bad], outs[0][:bad]) and not bool(torch.isfinite(out[bad:, :, 5]).any())
