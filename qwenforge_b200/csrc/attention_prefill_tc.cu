@@ -2,109 +2,136 @@
 // cores (tcgen05), bf16, head sizes 64 and 128. Same contract as the mma.sync kernel of attention_prefill.cu: the
 // span's own keys are in the cache already, a query at position p sees keys max(0, p - window + 1) <= j <= p.
 //
-// A block serves 128 consecutive query tokens of one (sequence, query head). Thread t of its first four warps owns
-// query row t, which is lane t of the block's tensor memory; one thread of a fifth warp issues every copy and every
-// product. Per 64-position page of the head's kv head:
-//   S = Q K^T     D / 16 products of 128 x 64 x 16 into 64 columns of tensor memory; Q (once) and the page's keys
-//                 come by tiled copies of the tensor memory accelerator, 128-byte swizzle
-//   softmax       every row thread loads its row of S (64 float32) into registers and says so on a barrier of 128
-//                 arrivals: S of the NEXT page is then multiplied under this page's softmax. Maximum, base-2
-//                 exponentials and sum need no exchange between threads; the weights go to shared memory as bf16
-//                 in the swizzled K-major layout the tensor cores read, and the thread arrives at a second barrier
-//   PV            when all rows have arrived there: four products of 128 x D x 16, the page's values read as they
-//                 lie (MN-major), ADDED to the running output O in D further columns of tensor memory
-//   O             stays in tensor memory. The exponentials of a row are taken against a reference maximum that is
-//                 only moved when the true maximum has grown by more than 2^8 since (weights stay below 256, well
-//                 inside bf16 and float32); only then does the warp rescale its rows of O (load, multiply, store).
-//                 Numerator and denominator carry the same reference, so the quotient at the end is unchanged.
-// Keys and values of the page after next are fetched as soon as a page's products are done (two stages). There is
-// no block-wide barrier inside the loop: rows and issuer hand over through shared-memory barriers. Several blocks
-// share an SM; one's exponentials overlap another's products. Every wait on a barrier is bounded: a wait that runs
-// out sets QF_ERR_COPY_TIMEOUT and ends the thread's loop, and the block still frees its tensor memory and returns.
-// No copy uses cluster multicast.
-// One prompt of a few thousand tokens gives too few blocks to fill the SMs, and its last tiles walk dozens of pages one
-// after the other. With SPLIT two blocks (a cluster) share a tile: each takes every second page, and at the end the
-// second block passes its rows' reference maxima, sums and outputs to the first through distributed shared memory
-// (column by column, so that a warp's 32 rows make one 128-byte store; row by row the same transfer cost 17
-// microseconds), which merges them with its own and writes the result.
+// A tile is 128 consecutive query tokens of one (sequence, query head). A block serves two tiles of one kv head that see
+// the same keys: two query heads of the group on the same tokens, and where the heads run out the next 128 tokens. It
+// walks the keys in blocks of two pages (128 keys), keys and values fetched once for both tiles by tiled copies (two
+// stages each), and keeps four matrices in tensor memory: per tile the scores S [128 x 128] and the output O [128 x D].
+//   warps 0-3, 4-7   a tile's rows, a thread each (lane = row): load the row of S, maximum, base-2 exponentials, sum without
+//                    exchange between threads; the weights go back to tensor memory as bf16 over the scores, where the
+//                    tensor cores read them as the left operand
+//   warp 8           issues the products: O += P V of a tile as soon as its weights are written, then S = Q K^T of its next
+//                    block when that product is done (the scores overwrite the weights it reads)
+//   warp 9           issues the copies
+// While one tile's products run, the other tile's rows are at their exponentials: a block of keys costs 16,384 of them a
+// tile, 1,024 cycles of the SM's special-function units, and as many cycles of products at D = 128, so the two alternate.
+// O stays in tensor memory. The exponentials of a row are taken against a reference maximum that is only moved when the
+// true maximum has grown by more than 2^8 since (weights stay below 256, well inside bf16 and float32); only then does the
+// warp rescale its rows of O (load, multiply, store), with no product on them in flight. Numerator and denominator
+// carry the same reference, so the quotient at the end is unchanged.
+// What bounds it: the chain scores -> exponentials -> product of a tile, of which two tiles overlap. (With one tile of 128
+// rows and 64 keys a turn per block, two or three blocks per SM, weights through shared memory, a turn's hand-overs cost more
+// than its work: 22% of the special-function rate, 32% of the tensor cores'.) Measured so and now, microseconds: one prompt of
+// 8,192 tokens, 28 heads of 128: 856, 449 (1,072 TFLOP/s); 1,024 tokens behind 15,360, 16 heads of 128: 268, 144; one prompt of
+// 4,096 tokens, 14 heads of 64: 89, 64; of 2,048: 29, 30. Masked keys cost nothing behind the comparison (their score is
+// -infinity), three-way maxima and two-way multiply-adds and additions take 640 instructions a row and turn to 400, and a warp
+// arrives once for its rows: 642 -> 1,072 TFLOP/s together. (A quarter or half of the exponentials by a polynomial on the
+// multiply-add pipe, and the exponentials of 16 to 64 weights laid out one after another, made no difference.)
+// There is no block-wide barrier inside the loop: rows and issuers hand over through shared-memory barriers. Every wait on
+// a barrier is bounded: a wait that runs out sets QF_ERR_COPY_TIMEOUT and ends the thread's loop, and the block still frees
+// its tensor memory and returns. No copy uses cluster multicast.
+// Few tiles of many pages leave SMs without a block. With SPLIT > 1 that many blocks (a cluster) share their tiles: each takes
+// every SPLIT-th block of keys, and at the end each brings a slice of the output's columns together: the others pass their sums
+// of that slice, and their rows' reference maxima and sums, through distributed shared memory (column by column, so that a
+// warp's 32 rows make one 128-byte store).
 #include <cooperative_groups.h>
 
 #include "tcgen05.cuh"
 
-#define TA_BM 128
-#define TA_ROW_THREADS 128
-#define TA_THREADS 160  // four warps of row threads and the issuing warp
+// The largest of three: one instruction.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 
-template <int D, bool SPLIT>
-__global__ void __launch_bounds__(TA_THREADS, D > 64 ? 2 : 3)
+#define TA_BM 128              // rows of a tile
+#define TA_BK 128              // keys of a turn: two pages
+
+template <int D, int SPLIT, int PER>
+__global__ void __launch_bounds__(128 * PER + 64, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                   bf16* __restrict__ out, const int* __restrict__ cu_q, const int* __restrict__ tok_pos,
-                  const int* __restrict__ slots, KvSite<bf16> site, int n_heads, int n_seqs, int row_tiles, int wave,
-                  float scale_log2, int window, int* err, const float* __restrict__ sinks, int planes) {
+                  const int* __restrict__ slots, KvSite<bf16> site, int n_heads, int n_seqs, float scale_log2, int window,
+                  int* err, const float* __restrict__ sinks, int planes) {
     constexpr int CB = D / 64;                    // blocks of 64 columns in a row of Q, K or V
     constexpr int Q_BLOCK = TA_BM * 128;          // bytes of one [128][64] block of Q
-    constexpr int KV_BLOCK = QF_PAGE * 128;       // bytes of one [64][64] block of a page's keys or values
-    constexpr int KV_BYTES = CB * KV_BLOCK;
-    constexpr int TMEM_COLS = D == 64 ? 128 : 256;  // S in columns 0..63, PV in columns 64..64 + D - 1
-    constexpr int PV_COL = 64;
+    constexpr int KV_BLOCK = TA_BK * 128;         // bytes of one [128][64] block of two pages' keys or values
+    constexpr int PAGE_BYTES = QF_PAGE * 128;     // one page's part of it
+    constexpr int Q_BYTES = CB * Q_BLOCK, KV_BYTES = CB * KV_BLOCK;
+    constexpr uint32_t TMEM_COLS = 256 * PER, O_COL = 128 * PER;   // S (and P) of tile t in columns 128 t .., O behind them
+    constexpr int PRODUCTS = 4 * PER, COPIES = 4 * PER + 1;         // the issuing warps
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
-    unsigned char* q_s = smem;                          // [CB][128][64]
-    unsigned char* k_s = q_s + CB * Q_BLOCK;            // [2][CB][64][64]
-    unsigned char* v_s = k_s + 2 * KV_BYTES;            // [2][CB][64][64]
-    unsigned char* p_s = v_s + 2 * KV_BYTES;            // [128][64]
-    // SPLIT: [D + 2][128] of the cluster's second block (a warp writes 32 neighbouring rows at once). It lies over Q and the pages' stages, which are free when both
-    // blocks have left their loops (the first barrier of the cluster below).
+    unsigned char* q_s = smem;                          // [PER][CB][128][64]
+    unsigned char* k_s = q_s + PER * Q_BYTES;             // [2][CB][128][64]
+    unsigned char* v_s = k_s + 2 * KV_BYTES;            // [2][CB][128][64]
+    // SPLIT > 1: what the cluster's other blocks send, over Q and the stages, which are free when all have left their loops (the
+    // first barrier of the cluster below): [SPLIT][PER][DS][128] sums of this block's columns, [SPLIT][PER][2][128] references and sums
+    constexpr int DS = D / SPLIT;                       // columns of the output that a block of the cluster brings together
     float* merge_s = reinterpret_cast<float*>(smem);
-    constexpr int STRIDE = SPLIT ? 2 : 1;               // this block takes every STRIDE-th page of the tile
-    const int rank = SPLIT ? (int)(blockIdx.x & 1) : 0;
-    // Launched as a programmatic dependent: what a block works out and sets up before its first copy (its tile, the
-    // barriers, its tensor memory) runs under the tail of the kernel before, which wrote the queries and the new keys
-    // and values; they are read, and the output written, only after the wait.
-    grid_launch_dependents();
-    __shared__ __align__(8) uint64_t bar_q, bar_kv[2], bar_s, bar_sfree, bar_pv, bar_p;
+    float* merge_ml = merge_s + SPLIT * PER * DS * TA_BM;
+    const int rank = (int)(blockIdx.x % SPLIT);
+    __shared__ __align__(8) uint64_t bar_q, bar_k[2], bar_v[2], bar_k_free[2], bar_v_free[2], bar_s[2], bar_p[2], bar_pv[2];
     __shared__ uint32_t tmem_base_s;
 
-    // Which (tile, head, sequence) this block serves (with SPLIT: this pair of blocks). Tiles further down a prompt walk
-    // more pages and an SM holds two or three blocks, so the blocks are taken in waves of `wave` (one per SM): the first
-    // wave gets the longest tiles in falling order, the second the next longest in rising order, and so on, so that the
-    // blocks that share an SM have about the same work together.
-    const int unit = SPLIT ? (int)(blockIdx.x / 2) : (int)blockIdx.x, units = SPLIT ? (int)(gridDim.x / 2) : (int)gridDim.x;
-    const int w = unit / wave, in_wave = min(wave, units - w * wave), at = unit % wave;
-    const int item = w * wave + ((w & 1) ? in_wave - 1 - at : at);
-    const int per_tile = n_heads * n_seqs;
-    const int tile = row_tiles - 1 - item / per_tile, head = (item % per_tile) % n_heads, seq = (item % per_tile) / n_heads;
+    // Which pair of tiles this block serves (PER 1: which single tile): those further down a prompt walk more keys, so they come first.
+    const int unit = (int)(blockIdx.x / SPLIT), units = (int)(gridDim.x / SPLIT);
+    const int per_pair = site.kv_heads * n_seqs, group = n_heads / site.kv_heads;
+    const int pair = units / per_pair - 1 - unit / per_pair, kvh = (unit % per_pair) % site.kv_heads, seq = (unit % per_pair) / site.kv_heads;
+    // Launched as a programmatic dependent: what a block works out and sets up before its first copy (its tiles, the barriers, its
+    // tensor memory) runs under the tail of the kernel before, which wrote the queries and the new keys and values; they are
+    // read, and the output written, only after the wait. (No kernel that takes tensor memory itself leaves room for this one's
+    // shared memory beside it, so the kernel before is not kept from finishing by what this one holds.)
+    grid_launch_dependents();
     const int q_begin = cu_q[seq], q_len = cu_q[seq + 1] - q_begin;
-    const int row0 = tile * TA_BM;
-    if (row0 >= q_len) return;
-    const int n_rows = min(TA_BM, q_len - row0);
+    const int tiles_here = (q_len + TA_BM - 1) / TA_BM * group;   // of this sequence and kv head; tile n: head n % group, rows n / group
+    if (PER * pair >= tiles_here) return;
     const int slot = slots[seq];
-    const int t = threadIdx.x, warp = t >> 5;
+    const int warp = threadIdx.x >> 5, t = PER == 2 && warp < 8 ? warp >> 2 : 0, row = threadIdx.x & 127;   // row threads: tile t, row `row`
     const int q_width = n_heads * D;
-    const int kvh = head / (n_heads / site.kv_heads);
-    bf16* out_row = out + (size_t)(q_begin + row0 + t) * q_width + (size_t)head * D;
+    int row0[2], head[2], n_rows[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int tile = PER * pair + i;
+        row0[i] = tile / group * TA_BM, head[i] = kvh * group + tile % group;
+        n_rows[i] = i < PER && tile < tiles_here ? min(TA_BM, q_len - row0[i]) : 0;
+    }
+    const int my_row0 = t ? row0[1] : row0[0], my_head = t ? head[1] : head[0], my_rows = t ? n_rows[1] : n_rows[0];
+    bf16* out_row = out + (size_t)(q_begin + my_row0 + row) * q_width + (size_t)my_head * D;
     if (slot < 0) {  // padding entry: defined output, no cache access
         grid_dependency_wait();
-        if (t < n_rows)
+        if (warp < PRODUCTS && row < my_rows)
             for (int c = 0; c < D; c += 8) *reinterpret_cast<uint4*>(out_row + c) = make_uint4(0, 0, 0, 0);
         return;
     }
-    const int pos0 = tok_pos[q_begin + row0];  // position of the tile's first row; row t is at pos0 + t
-    const int last_pos = pos0 + n_rows - 1;
-    const int p_first = (window > 0 ? max(0, pos0 - window + 1) : 0) / QF_PAGE, p_end = last_pos / QF_PAGE + 1;
-    const int p_begin = p_first + rank;  // this block's pages: p_begin, p_begin + STRIDE, ...
-    const int n_tiles = p_end > p_begin ? (p_end - p_begin + STRIDE - 1) / STRIDE : 0;
-
-    if (t == 0) {
-        mbar_init(&bar_q, 1);
-        mbar_init(&bar_kv[0], 1);
-        mbar_init(&bar_kv[1], 1);
-        mbar_init(&bar_s, 1);
-        mbar_init(&bar_pv, 1);
-        mbar_init(&bar_p, TA_ROW_THREADS);
-        mbar_init(&bar_sfree, TA_ROW_THREADS);
+    // The first tile's rows are never behind the second's. Blocks of keys: two pages from page p_first on; this block takes
+    // every SPLIT-th of them, tile i the first turns[i] of those.
+    const int pos_first = tok_pos[q_begin + row0[0]];   // position of the first tile's first row; positions run on from there
+    const int p_first = (window > 0 ? max(0, pos_first - window + 1) : 0) / QF_PAGE;
+    int turns[2], p_end[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int last = pos_first + row0[i] - row0[0] + n_rows[i] - 1;
+        p_end[i] = n_rows[i] > 0 ? last / QF_PAGE + 1 : 0;
+        const int blocks = p_end[i] > p_first ? (p_end[i] - p_first + 1) / 2 : 0;
+        turns[i] = blocks > rank ? (blocks - rank + SPLIT - 1) / SPLIT : 0;
     }
-    if (warp == 4) {
+    const int all_turns = max(turns[0], turns[1]), p_last = max(p_end[0], p_end[1]) - 1;
+
+    if (threadIdx.x == 0) {
+        mbar_init(&bar_q, 1);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bar_k[i], 1);
+            mbar_init(&bar_v[i], 1);
+            mbar_init(&bar_k_free[i], 1);
+            mbar_init(&bar_v_free[i], 1);
+            mbar_init(&bar_s[i], 1);
+            mbar_init(&bar_p[i], TA_BM / 32);
+            mbar_init(&bar_pv[i], 1);
+        }
+    }
+    if (warp == PRODUCTS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_s)), "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
@@ -119,135 +146,140 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     // the lanes of a warp must leave their loop together if a wait runs out.
     auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
 
-    if (warp == 4) {
-        {
-            // ---- the issuing warp: copies and products. All lanes run the loop (uniform values); one lane issues.
-            const bool leader = elect_one();
-            const int* table_row = site.table + (long long)slot * site.table_stride;
-            auto fetch_page = [&](int j) {  // keys and values of the j-th page of the run into stage j & 1
-                const int stage = j & 1;
-                int page = table_row[p_begin + j * STRIDE];
-                if (page < 0) {  // a page the sequence does not hold: reported; some held memory is read instead
+    if (warp == COPIES) {
+        // ---- the copies. All lanes run the loop (uniform values); one lane issues.
+        const bool leader = elect_one();
+        const int* table_row = site.table + (long long)slot * site.table_stride;
+        if (all_turns > 0 && leader) {
+            mbar_expect_tx(&bar_q, (n_rows[1] > 0 ? 2 : 1) * Q_BYTES);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (n_rows[i] > 0)
+#pragma unroll
+                    for (int cb = 0; cb < CB; ++cb)
+                        tma_load_2d(q_s + i * Q_BYTES + cb * Q_BLOCK, &q_map, head[i] * D + cb * 64, q_begin + row0[i], &bar_q);
+        }
+        __syncwarp();
+        for (int j = 0; j < all_turns; ++j) {
+            const int stage = j & 1, first = p_first + 2 * (rank + j * SPLIT);
+            const uint32_t freed = ((j >> 1) + 1) & 1;   // the turn before last has been read
+            int page[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                page[h] = table_row[min(first + h, p_last)];   // (beyond the last page: masked keys, some finite numbers)
+                if (page[h] < 0) {  // a page the sequence does not hold: reported; some held memory is read instead
                     if (leader) atomicOr(err, QF_ERR_NO_PAGE);
-                    page = 0;
+                    page[h] = 0;
                 }
-                // row of the cache seen as one matrix [pages * planes * kv_heads * 64][D]; with one plane per page the values
-                // are the keys themselves (the same rows fetched into the values' stage)
-                const long long k_row = ((long long)page * planes * site.kv_heads + kvh) * QF_PAGE;
-                const long long v_row = planes == 2 ? k_row + (long long)site.kv_heads * QF_PAGE : k_row;
-                if (leader) {
-                    mbar_expect_tx(&bar_kv[stage], 2 * KV_BYTES);
+            }
+            if (j >= 2 && !wait_all(&bar_k_free[stage], freed)) {
+                timed_out = true;
+                break;
+            }
+            // row of the cache seen as one matrix [pages * planes * kv_heads * 64][D]; with one plane per page the values
+            // are the keys themselves (the same rows fetched into the values' stage)
+            if (leader) {
+                mbar_expect_tx(&bar_k[stage], KV_BYTES);
 #pragma unroll
-                    for (int cb = 0; cb < CB; ++cb) {
-                        tma_load_2d(k_s + stage * KV_BYTES + cb * KV_BLOCK, &kv_map, cb * 64, (int)k_row, &bar_kv[stage]);
-                        tma_load_2d(v_s + stage * KV_BYTES + cb * KV_BLOCK, &kv_map, cb * 64, (int)v_row, &bar_kv[stage]);
-                    }
-                }
-                __syncwarp();
-            };
-            // descriptors: an address field counts 16 bytes, so 16 columns of a K-major row (32 bytes) are 2 units
-            const uint64_t desc_q = smem_desc_sw128(q_s), desc_p = smem_desc_sw128(p_s);
-            const uint64_t desc_k = smem_desc_sw128(k_s), desc_v = smem_desc_mn_sw128(v_s, KV_BLOCK);
-            constexpr uint32_t idesc_s = umma_idesc_bf16(TA_BM, QF_PAGE, false), idesc_pv = umma_idesc_bf16(TA_BM, D, true);
-            auto issue_s = [&](int j) {  // S = Q K^T of page j; false if its keys did not arrive
-                if (!wait_all(&bar_kv[j & 1], (j >> 1) & 1)) return false;
-                tc_fence_after();
-                const uint64_t dk = desc_k + (uint64_t)((j & 1) * (KV_BYTES >> 4));
-                if (leader) {
+                for (int h = 0; h < 2; ++h)
 #pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)
-                        umma_bf16(tmem, desc_q + (uint64_t)((ks / 4) * (Q_BLOCK >> 4) + 2 * (ks % 4)),
-                                  dk + (uint64_t)((ks / 4) * (KV_BLOCK >> 4) + 2 * (ks % 4)), idesc_s, ks > 0 ? 1u : 0u);
-                    umma_commit(&bar_s);
-                }
-                __syncwarp();
-                return true;
-            };
-            if (leader && n_tiles > 0) {
-                mbar_expect_tx(&bar_q, CB * Q_BLOCK);
-#pragma unroll
-                for (int cb = 0; cb < CB; ++cb) tma_load_2d(q_s + cb * Q_BLOCK, &q_map, head * D + cb * 64, q_begin + row0, &bar_q);
+                    for (int cb = 0; cb < CB; ++cb)
+                        tma_load_2d(k_s + stage * KV_BYTES + cb * KV_BLOCK + h * PAGE_BYTES, &kv_map, cb * 64,
+                                    (int)(((long long)page[h] * planes * site.kv_heads + kvh) * QF_PAGE), &bar_k[stage]);
             }
             __syncwarp();
-            if (n_tiles > 0) fetch_page(0);
-            if (n_tiles > 1) fetch_page(1);
-            if (n_tiles > 0) timed_out = !wait_all(&bar_q, 0) || !issue_s(0);
-            for (int j = 0; j < n_tiles && !timed_out; ++j) {
-                // as soon as every row holds its S in registers, S of the next page is multiplied under their softmax
-                if (!wait_all(&bar_sfree, j & 1)) {
-                    timed_out = true;
-                    break;
-                }
-                tc_fence_after();
-                if (j + 1 < n_tiles && !issue_s(j + 1)) {
-                    timed_out = true;
-                    break;
-                }
-                if (!wait_all(&bar_p, j & 1)) {  // every row has written its weights
-                    timed_out = true;
-                    break;
-                }
-                tc_fence_after();
-                // PV of page j: weights [128][64 keys] K-major; values [64 keys][D] as they lie, 16 keys are two groups
-                // of 8 rows (2048 bytes)
-                const uint64_t dv = desc_v + (uint64_t)((j & 1) * (KV_BYTES >> 4));
-                if (leader) {
+            if (j >= 2 && !wait_all(&bar_v_free[stage], freed)) {
+                timed_out = true;
+                break;
+            }
+            if (leader) {
+                mbar_expect_tx(&bar_v[stage], KV_BYTES);
 #pragma unroll
-                    for (int kk = 0; kk < QF_PAGE / 16; ++kk)
-                        umma_bf16(tmem + PV_COL, desc_p + (uint64_t)(2 * kk), dv + (uint64_t)(kk * (2048 >> 4)), idesc_pv,
-                                  (j > 0 || kk > 0) ? 1u : 0u);
-                    umma_commit(&bar_pv);
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int cb = 0; cb < CB; ++cb)
+                        tma_load_2d(v_s + stage * KV_BYTES + cb * KV_BLOCK + h * PAGE_BYTES, &kv_map, cb * 64,
+                                    (int)((((long long)page[h] * planes + planes - 1) * site.kv_heads + kvh) * QF_PAGE), &bar_v[stage]);
+            }
+            __syncwarp();
+        }
+    } else if (warp == PRODUCTS) {
+        // ---- the products
+        const bool leader = elect_one();
+        // descriptors: an address field counts 16 bytes, so 16 columns of a K-major row (32 bytes) are 2 units
+        const uint64_t desc_q = smem_desc_sw128(q_s), desc_k = smem_desc_sw128(k_s), desc_v = smem_desc_mn_sw128(v_s, KV_BLOCK);
+        constexpr uint32_t idesc_s = umma_idesc_bf16(TA_BM, TA_BK, false), idesc_pv = umma_idesc_bf16(TA_BM, D, true);
+        // S of tile i, turn j; the last tile that reads a turn's keys hands their stage back
+        auto issue_s = [&](int i, int j) {
+            if (!wait_all(&bar_k[j & 1], (j >> 1) & 1)) return false;
+            tc_fence_after();
+            if (leader) {
+                const uint64_t dq = desc_q + (uint64_t)(i * (Q_BYTES >> 4)), dk = desc_k + (uint64_t)((j & 1) * (KV_BYTES >> 4));
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_bf16(tmem + 128 * i, dq + (uint64_t)((ks / 4) * (Q_BLOCK >> 4) + 2 * (ks % 4)),
+                              dk + (uint64_t)((ks / 4) * (KV_BLOCK >> 4) + 2 * (ks % 4)), idesc_s, ks > 0 ? 1u : 0u);
+                umma_commit(&bar_s[i]);
+                if (i == 1 || j >= turns[1]) umma_commit(&bar_k_free[j & 1]);
+            }
+            __syncwarp();
+            return true;
+        };
+        if (all_turns > 0) timed_out = !wait_all(&bar_q, 0);
+        for (int i = 0; i < 2 && !timed_out; ++i)
+            if (turns[i] > 0) timed_out = !issue_s(i, 0);
+        for (int j = 0; j < all_turns && !timed_out; ++j) {
+            for (int i = 0; i < 2 && !timed_out; ++i) {
+                if (j >= turns[i]) continue;
+                if (!wait_all(&bar_v[j & 1], (j >> 1) & 1) || !wait_all(&bar_p[i], j & 1)) {   // every row has written its weights
+                    timed_out = true;
+                    break;
+                }
+                tc_fence_after();
+                if (leader) {   // values [128 keys][D] as they lie (MN-major), 16 keys are two groups of 8 rows (2048 bytes)
+                    const uint64_t dv = desc_v + (uint64_t)((j & 1) * (KV_BYTES >> 4));
+#pragma unroll
+                    for (int kk = 0; kk < TA_BK / 16; ++kk)
+                        umma_bf16_tmem_a(tmem + O_COL + 128 * i, tmem + 128 * i + 8 * kk, dv + (uint64_t)(kk * (2048 >> 4)), idesc_pv,
+                                         (j > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit(&bar_pv[i]);
+                    if (i == 1 || j >= turns[1]) umma_commit(&bar_v_free[j & 1]);
                 }
                 __syncwarp();
-                if (j + 2 < n_tiles && !timed_out) {
-                    // keys and values of page j have been read when its PV is done: their stage takes the page after next
-                    if (!wait_all(&bar_pv, j & 1)) timed_out = true;
-                    else fetch_page(j + 2);
-                }
+                if (j + 1 < turns[i] && (!wait_all(&bar_pv[i], j & 1) || !issue_s(i, j + 1))) timed_out = true;
             }
         }
     } else {
         // ---- the row threads
-        const int row_pos = pos0 + t, row_lo = window > 0 ? max(0, row_pos - window + 1) : 0;
-        const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int j = 0; j < n_tiles; ++j) {
-            if (!wait_all(&bar_s, j & 1)) {
+        const int my_turns = t ? turns[1] : turns[0];
+        const int pos0 = pos_first + my_row0 - row0[0], row_pos = pos0 + row, row_lo = window > 0 ? max(0, row_pos - window + 1) : 0;
+        const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16), s_at = lanes + 128 * t, o_at = lanes + O_COL + 128 * t;
+        for (int j = 0; j < my_turns; ++j) {
+            if (!wait_all(&bar_s[t], j & 1)) {   // (the product of the turn before is done too: S was issued after it)
                 timed_out = true;
                 break;
             }
             tc_fence_after();
-            float s[QF_PAGE];
-            {
-                uint32_t raw[32];
-                tmem_load_32(lane_base, raw);
+            float s[TA_BK];
+            tmem_load_row_128(s_at, s);
+            const int key0 = (p_first + 2 * (rank + j * SPLIT)) * QF_PAGE;
+            // a block of keys that every row of the tile sees whole needs no mask
+            const bool full = key0 + TA_BK - 1 <= pos0 && key0 >= (window > 0 ? max(0, pos0 + TA_BM - 1 - window + 1) : 0);
+            if (!full) {   // a key that the row does not see gets the weight 2^-inf = 0
 #pragma unroll
-                for (int i = 0; i < 32; ++i) s[i] = __uint_as_float(raw[i]);
-                tmem_load_32(lane_base + 32, raw);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) s[32 + i] = __uint_as_float(raw[i]);
+                for (int i = 0; i < TA_BK; ++i) s[i] = (key0 + i <= row_pos && key0 + i >= row_lo) ? s[i] : -INFINITY;
             }
-            tc_fence_before();
-            mbar_arrive(&bar_sfree);  // S is in this thread's registers
-            const int key0 = (p_begin + j * STRIDE) * QF_PAGE;
-            // a page that every row of the block sees whole needs no mask
-            const bool full = key0 + QF_PAGE - 1 <= pos0 && key0 >= (window > 0 ? max(0, pos0 + TA_BM - 1 - window + 1) : 0);
             float mx[4];  // four chains instead of one: the comparisons do not wait for each other
-            if (full) {  // the scores stay unscaled; the scale is folded into the exponent below
 #pragma unroll
-                for (int i = 0; i < QF_PAGE; ++i) mx[i & 3] = i < 4 ? s[i] : fmaxf(mx[i & 3], s[i]);
+            for (int i = 0; i < 4; ++i) mx[i] = s[i];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) mx[i] *= scale_log2;
-            } else {
+            for (int i = 4; i < TA_BK - 4; i += 8)
 #pragma unroll
-                for (int i = 0; i < QF_PAGE; ++i) {
-                    const int kj = key0 + i;
-                    s[i] = (kj <= row_pos && kj >= row_lo) ? s[i] * scale_log2 : QF_NEG_BIG;
-                    mx[i & 3] = i < 4 ? s[i] : fmaxf(mx[i & 3], s[i]);
-                }
-            }
-            const float m_true = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
-            // The reference maximum moves before the exponentials; O, which carries the old one, is rescaled after them,
-            // when the products of the page before are surely done.
+                for (int c = 0; c < 4; ++c) mx[c] = max3(mx[c], s[i + c], s[i + 4 + c]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) mx[c] = fmaxf(mx[c], s[TA_BK - 4 + c]);
+            // (the scores stay unscaled; the scale is folded into the exponent)
+            const float m_true = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2);
             float f_o = 1.0f;
             bool moved = false;
             if (j == 0) {
@@ -258,58 +290,43 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 m_ref = m_true;
                 l_run *= f_o;
             }
-            float part[4] = {0.f, 0.f, 0.f, 0.f};
-            if (full) {
-#pragma unroll
-                for (int i = 0; i < QF_PAGE; ++i) {
-                    s[i] = fast_exp2(fmaf(s[i], scale_log2, -m_ref));
-                    part[i & 3] += s[i];
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < QF_PAGE; ++i) {
-                    // a masked score is QF_NEG_BIG: its weight is 0 even while the reference is QF_NEG_BIG too
-                    s[i] = s[i] > 0.5f * QF_NEG_BIG ? fast_exp2(s[i] - m_ref) : 0.f;
-                    part[i & 3] += s[i];
-                }
-            }
-            l_run += (part[0] + part[1]) + (part[2] + part[3]);
-            // the products of the page before read the weights' buffer and add to O: both must be done before this
-            // thread writes either
-            if (j > 0 && !wait_all(&bar_pv, (j - 1) & 1)) {
-                timed_out = true;
-                break;
-            }
             if (__any_sync(0xffffffffu, moved)) {  // the warp's 32 rows of O are loaded and stored together
-                tc_fence_after();
-                // (16 columns at a time: the row of weights is still in this thread's registers)
 #pragma unroll 1
                 for (int c0 = 0; c0 < D; c0 += 16) {
                     uint32_t raw[16];
-                    tmem_load_16(lane_base + PV_COL + c0, raw);
+                    tmem_load_16(o_at + c0, raw);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) raw[i] = __float_as_uint(__uint_as_float(raw[i]) * f_o);
-                    tmem_store_16(lane_base + PV_COL + c0, raw);
+                    tmem_store_16(o_at + c0, raw);
                 }
-                tmem_store_wait();
             }
-            // the row of weights, bf16, 16-byte chunk c at chunk position c ^ (row % 8) of the row's 128 bytes
+            // two neighbouring weights an instruction where the pipes allow it: s * scale - reference, and the sums
+            const float2 by = make_float2(scale_log2, scale_log2), less = make_float2(-m_ref, -m_ref);
+            float2 part[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint4 chunk = make_uint4(pack_bf16(s[8 * c], s[8 * c + 1]), pack_bf16(s[8 * c + 2], s[8 * c + 3]),
-                                               pack_bf16(s[8 * c + 4], s[8 * c + 5]), pack_bf16(s[8 * c + 6], s[8 * c + 7]));
-                *reinterpret_cast<uint4*>(p_s + t * 128 + ((c ^ (t & 7)) << 4)) = chunk;
+            for (int h = 0; h < 2; ++h) {   // half of the weights at a time: the first are stored while the others are formed
+                uint32_t packed[32];
+#pragma unroll
+                for (int i = 0; i < 64; i += 2) {
+                    float2 p = __ffma2_rn(make_float2(s[64 * h + i], s[64 * h + i + 1]), by, less);
+                    p.x = fast_exp2(p.x), p.y = fast_exp2(p.y);
+                    part[(i >> 1) & 1] = __fadd2_rn(part[(i >> 1) & 1], p);
+                    packed[i / 2] = pack_bf16(p.x, p.y);
+                }
+                tmem_store_32(s_at + 32 * h, packed);
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read what this thread wrote
+            l_run += (part[0].x + part[0].y) + (part[1].x + part[1].y);
+            tmem_store_wait();
             tc_fence_before();
-            mbar_arrive(&bar_p);
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) mbar_arrive(&bar_p[t]);
         }
-        if (!timed_out && n_tiles > 0 && !wait_all(&bar_pv, (n_tiles - 1) & 1)) timed_out = true;
+        if (!timed_out && my_turns > 0 && !wait_all(&bar_pv[t], (my_turns - 1) & 1)) timed_out = true;
         tc_fence_after();
-        if (!SPLIT && !timed_out) {  // the loads are collective: every lane of the warp takes part, rows beyond the span store nothing
+        if (SPLIT == 1 && !timed_out && my_turns > 0) {  // the loads are collective: every lane of the warp takes part, rows beyond the span store nothing
             float den = l_run, keep = 1.f;
             if (sinks) {  // a sink's term joins the sum of weights once, in base-2 units like the scores, on a common maximum
-                const float s2 = sinks[head] * 1.4426950408889634f, m_new = fmaxf(m_ref, s2);
+                const float s2 = sinks[my_head] * 1.4426950408889634f, m_new = fmaxf(m_ref, s2);
                 keep = exp2f(m_ref - m_new);
                 den = l_run * keep + exp2f(s2 - m_new);
             }
@@ -317,8 +334,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 #pragma unroll
             for (int c0 = 0; c0 < D; c0 += 32) {
                 uint32_t raw[32];
-                tmem_load_32(lane_base + PV_COL + c0, raw);
-                if (t < n_rows) {
+                tmem_load_32(o_at + c0, raw);
+                if (row < my_rows) {
 #pragma unroll
                     for (int c = 0; c < 32; c += 8) {
                         float v[8];
@@ -331,92 +348,105 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             }
         }
     }
-    if (SPLIT) {
-        cooperative_groups::this_cluster().sync();  // every thread of both blocks: both have left their loops, their stages are free
-        if (rank == 1 && warp < 4) {
-            // this block's part of every row goes to the first block: output sums, reference maximum, sum of weights
-            const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-            float* theirs = cooperative_groups::this_cluster().map_shared_rank(merge_s, 0) + t;
-            const bool have = n_tiles > 0 && !timed_out;
-#pragma unroll 1
-            for (int c0 = 0; c0 < D; c0 += 16) {
-                uint32_t raw[16];
-                if (have) tmem_load_16(lane_base + PV_COL + c0, raw);
+    if (SPLIT > 1) {
+        const int my_turns = t ? turns[1] : turns[0];
+        const bool have = my_turns > 0 && !timed_out;
+        const uint32_t o_at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + O_COL + 128 * t;
+        cooperative_groups::this_cluster().sync();  // every thread of all blocks: all have left their loops, their stages are free
+        if (warp < PRODUCTS && my_rows > 0) {
+            // every block brings a slice of the columns together: this block's sums of every other slice go to its block, its rows'
+            // reference maxima and sums of weights to all
 #pragma unroll
-                for (int i = 0; i < 16; ++i) theirs[(c0 + i) * TA_BM] = have ? __uint_as_float(raw[i]) : 0.f;
+            for (int to = 0; to < SPLIT; ++to) {
+                float* ml = cooperative_groups::this_cluster().map_shared_rank(merge_ml, to) + (rank * PER + t) * 2 * TA_BM + row;
+                ml[0] = have ? m_ref : QF_NEG_BIG;
+                ml[TA_BM] = have ? l_run : 0.f;
+                if (to == rank) continue;
+                float* sums = cooperative_groups::this_cluster().map_shared_rank(merge_s, to) + (size_t)(rank * PER + t) * DS * TA_BM + row;
+#pragma unroll 1
+                for (int c0 = 0; c0 < DS; c0 += 8) {
+                    uint32_t raw[8];
+                    if (have) tmem_load_8(o_at + to * DS + c0, raw);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) sums[(c0 + i) * TA_BM] = have ? __uint_as_float(raw[i]) : 0.f;
+                }
             }
-            theirs[D * TA_BM] = have ? m_ref : QF_NEG_BIG;
-            theirs[(D + 1) * TA_BM] = have ? l_run : 0.f;
         }
-        cooperative_groups::this_cluster().sync();  // the second block's parts have arrived
-        if (rank == 0 && warp < 4) {
-            // merge: both parts carry a reference maximum of their own; the common one is the larger
-            const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-            const float* theirs = merge_s + t;
-            const float m_other = theirs[D * TA_BM], l_other = theirs[(D + 1) * TA_BM];
-            const float m_all = fmaxf(m_ref, m_other);
-            const float f_mine = fast_exp2(m_ref - m_all), f_theirs = fast_exp2(m_other - m_all);
-            float l_all = l_run * f_mine + l_other * f_theirs, keep = 1.f;
-            if (sinks) {
-                const float s2 = sinks[head] * 1.4426950408889634f, m_new = fmaxf(m_all, s2);
+        cooperative_groups::this_cluster().sync();  // the other blocks' parts have arrived
+        if (warp < PRODUCTS && my_rows > 0) {
+            // every part carries a reference maximum of its own; the common one is the largest
+            float m_all = QF_NEG_BIG, l_all = 0.f, keep = 1.f, by[SPLIT];
+#pragma unroll
+            for (int r = 0; r < SPLIT; ++r) m_all = fmaxf(m_all, by[r] = merge_ml[(r * PER + t) * 2 * TA_BM + row]);
+#pragma unroll
+            for (int r = 0; r < SPLIT; ++r) {
+                by[r] = fast_exp2(by[r] - m_all);
+                l_all = fmaf(merge_ml[((r * PER + t) * 2 + 1) * TA_BM + row], by[r], l_all);
+            }
+            if (sinks) {  // a sink's term joins the sum of weights once, in base-2 units like the scores, on a common maximum
+                const float s2 = sinks[my_head] * 1.4426950408889634f, m_new = fmaxf(m_all, s2);
                 keep = exp2f(m_all - m_new);
                 l_all = l_all * keep + exp2f(s2 - m_new);
             }
             const float inv = l_all > 0.f ? keep / l_all : 0.f;
-            const bool have = n_tiles > 0 && !timed_out;
+#pragma unroll 1
+            for (int c0 = 0; c0 < DS; c0 += 8) {
+                uint32_t raw[8];
+                if (have) tmem_load_8(o_at + rank * DS + c0, raw);
+                float v[8];
 #pragma unroll
-            for (int c0 = 0; c0 < D; c0 += 32) {
-                uint32_t raw[32];
-                if (have) tmem_load_32(lane_base + PV_COL + c0, raw);
-                if (t < n_rows) {
+                for (int i = 0; i < 8; ++i) {
+                    v[i] = 0.f;
 #pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        float v[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            v[i] = ((have ? __uint_as_float(raw[c + i]) * f_mine : 0.f) + theirs[(c0 + c + i) * TA_BM] * f_theirs) * inv;
-                        *reinterpret_cast<uint4*>(out_row + c0 + c) =
-                            make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                    for (int r = 0; r < SPLIT; ++r) {
+                        const float part = r == rank ? (have ? __uint_as_float(raw[i]) : 0.f) : merge_s[((size_t)(r * PER + t) * DS + c0 + i) * TA_BM + row];
+                        v[i] = fmaf(part, by[r], v[i]);
                     }
+                    v[i] *= inv;
                 }
+                if (row < my_rows)
+                    *reinterpret_cast<uint4*>(out_row + rank * DS + c0) =
+                        make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
             }
         }
     }
     if (timed_out) atomicOr(err, QF_ERR_COPY_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    if (warp == 4)
+    if (warp == PRODUCTS)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32  %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-template <int D, bool SPLIT>
+template <int D, int SPLIT, int PER>
 static int launch_variant(const CUtensorMap& q_map, const CUtensorMap& kv_map, void* out, const int* cu_q, const int* tok_pos,
-                          const int* slots, KvSite<bf16> site, int n_heads, int n_seqs, int max_q_len, float scale, int window,
-                          int* err, const float* sinks, int planes, cudaStream_t stream) {
-    size_t smem = (size_t)(D / 64) * TA_BM * 128 + 4 * (size_t)(D / 64) * QF_PAGE * 128 + TA_BM * 128 + 1024;
-    auto kernel = prefill_tc_kernel<D, SPLIT>;
+                          const int* slots, KvSite<bf16> site, int n_heads, int n_seqs, long long tiles, float scale,
+                          int window, int* err, const float* sinks, int planes, cudaStream_t stream) {
+    // One block per SM, also where two would find room: a block with two tiles holds all of its SM's tensor memory, and the blocks
+    // of clusters that wait for one another must not wait for one another's tensor memory as well.
+    constexpr size_t stages = (size_t)(D / 64) * (PER * TA_BM + 4 * TA_BK) * 128 + 1024, alone = 120 * 1024;
+    constexpr size_t merge = (size_t)PER * (D + 2 * SPLIT) * TA_BM * sizeof(float) + 1024;
+    constexpr size_t smem = stages > merge ? (stages > alone ? stages : alone) : (merge > alone ? merge : alone);
+    auto kernel = prefill_tc_kernel<D, SPLIT, PER>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    const int row_tiles = (max_q_len + TA_BM - 1) / TA_BM;
-    const long long blocks = (long long)row_tiles * n_heads * n_seqs * (SPLIT ? 2 : 1);
+    const long long blocks = (tiles + PER - 1) / PER * site.kv_heads * n_seqs * SPLIT;
     if (blocks > 0x7fffffffll) return (int)cudaErrorInvalidValue;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)blocks);
-    config.blockDim = dim3(TA_THREADS);
+    config.blockDim = dim3(128 * PER + 64);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.x = SPLIT;
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = 1;
     config.attrs = attr;
-    config.numAttrs = SPLIT ? 2 : 1;
+    config.numAttrs = SPLIT > 1 ? 2 : 1;
     return (int)cudaLaunchKernelEx(&config, kernel, q_map, kv_map, (bf16*)out, cu_q, tok_pos, slots, site, n_heads, n_seqs,
-                                   row_tiles, SPLIT ? qf_sm_count() / 2 : qf_sm_count(), scale * 1.4426950408889634f, window, err,
-                                   sinks, planes);
+                                   scale * 1.4426950408889634f, window, err, sinks, planes);
 }
 
 template <int D>
@@ -434,18 +464,36 @@ static int launch(const void* q, void* out, const int* cu_q, const int* tok_pos,
     // The cache of this entry as one matrix of rows of D elements. The map is given more rows than any cache has
     // (its extent only bounds what a copy may address; copies address rows of held pages only).
     if (!qf_make_map_bf16(&kv_map, base, 1ll << 31, D, D, QF_PAGE)) return (int)cudaErrorNotSupported;
-    // Two blocks per tile when a tile's chain of pages is what takes the time. Measured on one prompt, head size 64, 14
-    // heads (three blocks fit an SM): 1,024 tokens 21 -> 17 microseconds, 2,048 tokens 38 -> 27, 3,072 tokens 54 -> 48,
-    // 4,096 tokens no gain; so chains of 16 pages and more, while the pairs need no more than two rounds on the SMs.
-    // Head size 128 (two blocks per SM, a merge twice as large): 8 tiles of 16 pages 24 -> 29 and pairs in two rounds 51 ->
-    // 64, so chains of 32 pages and room for every pair at once.
-    // (tiles that hold rows: the grid also has blocks for the rows that shorter sequences lack, which end at once)
-    const long long blocks = (long long)min((max_q_len + TA_BM - 1) / TA_BM * n_seqs, n_tokens / TA_BM + n_seqs) * n_heads;
+    const int q_tiles = (max_q_len + TA_BM - 1) / TA_BM;
+    const long long tiles = (long long)q_tiles * (n_heads / kv_heads);   // of the longest sequence and a kv head
+    // How many tiles a block takes and how many blocks share them: the choice that is done first by this estimate, in
+    // microseconds as measured (prompts and portions, 14 to 28 heads, inside a graph): a turn takes 1.75 with one tile and 2.05
+    // with two at D = 128, 1.5 and 1.85 at D = 64; a block's start and end take 3 to 6.5 with one tile and 5 to 13 with two, the more
+    // the more blocks a cluster has; clusters of four and of eight do not find room on every SM. Tiles x blocks 1 x 1, 2 x 1, 2 x 2
+    // and 2 x 8, chosen first: one prompt of 4,096 tokens, 14 heads of 64: 91, [62], 73, 211; of 1,024: 15.4, 19, [14], 45; 256 tokens
+    // behind 8,000: 99, 115, 63, [25]; 64 behind 8,000, 16 heads of 128: 112, 127, 71, [31]; four prompts of 183 to 275: [7.2], 9.1, 10, 53.
     const int span = window > 0 && window + TA_BM < max_kv_len ? window + TA_BM : max_kv_len;
-    const long long room = (long long)qf_sm_count() * (D <= 64 ? 3 : 2);
-    const bool split = D <= 64 ? span >= 16 * QF_PAGE && blocks <= room : span >= 32 * QF_PAGE && blocks * 2 <= room;
-    return split ? launch_variant<D, true>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, sinks, planes, stream)
-                 : launch_variant<D, false>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, sinks, planes, stream);
+    const float longest = (float)((span + TA_BK - 1) / TA_BK), mean = longest > q_tiles ? longest - 0.5f * q_tiles : 0.5f * longest + 0.5f;
+    // (tiles that hold rows: the grid also has blocks for the rows that shorter sequences lack, which end at once)
+    const long long live = min((long long)q_tiles * n_seqs, max((2ll * n_tokens + (long long)TA_BM * n_seqs + TA_BM - 1) / (2 * TA_BM), 1ll)) * n_heads;
+    const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
+    const float turn[2] = {D <= 64 ? 1.5f : 1.75f, D <= 64 ? 1.85f : 2.05f}, ends[2][4] = {{3.f, 5.f, 5.5f, 6.5f}, {5.f, 6.5f, 9.f, 13.f}};
+    const int room[4] = {sms, sms, sms - sms / 8, sms * 77 / 100 > 0 ? sms * 77 / 100 : 1};
+    int per = 2, split = 1;
+    float least = -1.f;
+    for (int p = 2; p >= 1; --p)
+        for (int n = 0; n < 4; ++n) {
+            const long long blocks = (live + p - 1) / p << n;
+            const float alone = ceilf(longest / (1 << n)) * turn[p - 1] + ends[p - 1][n];
+            const float all = (float)((blocks + room[n] - 1) / room[n]) * (mean / (1 << n) * turn[p - 1] + ends[p - 1][n]);
+            const float time = alone > all ? alone : all;
+            if (least < 0.f || time < least) least = time, per = p, split = 1 << n;
+        }
+#define QF_TC_LAUNCH(SPLIT, PER) \
+    launch_variant<D, SPLIT, PER>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, tiles, scale, window, err, sinks, planes, stream)
+    if (per == 1) return split == 1 ? QF_TC_LAUNCH(1, 1) : split == 2 ? QF_TC_LAUNCH(2, 1) : split == 4 ? QF_TC_LAUNCH(4, 1) : QF_TC_LAUNCH(8, 1);
+    return split == 1 ? QF_TC_LAUNCH(1, 2) : split == 2 ? QF_TC_LAUNCH(2, 2) : split == 4 ? QF_TC_LAUNCH(4, 2) : QF_TC_LAUNCH(8, 2);
+#undef QF_TC_LAUNCH
 }
 
 // The arguments of qf_attention_prefill (with `max_kv_len`, the bound that steers the sharing of a tile) and the number

@@ -54,12 +54,20 @@ from .base import Mixer, TensorSpec
 from .registry import build_part, register_part
 
 
-# Fewest new tokens of a step, by head size, from which the tcgen05 prefill attention runs instead of the mma.sync one.
-# Measured on one prompt (`python -m qwenforge_b200.measure attention`): head size 64, 14 heads: 17 against 21
-# microseconds at 1,024 tokens, 27 against 42 at 2,048, 72 against 116 at 4,096, 199 against 415 at 8,192 (at 512 tokens
-# 15 against 13); head size 128, 16 heads: 16 against 17 at 512 tokens, 24 against 36 at 1,024, 52 against 72 at 2,048,
-# 140 against 245 at 4,096. Below, its tiles of 128 rows are too few to fill the SMs.
-TC_PREFILL_MIN_TOKENS = {64: 1024, 128: 512}
+# Head sizes of the tcgen05 prefill attention, with the fewest new tokens of a step from which it runs, and the fewest keys: it walks
+# keys in blocks of 128, below which the mma.sync kernel is done first. Measured inside a graph, microseconds, mma.sync / tcgen05:
+# 14 heads of 64: 40 tokens 3.8 / 4.2, 100 tokens 4.8 / 4.9, 12 x 100 tokens 8.0 / 7.4, four prompts of 183 to 275 10.7 / 7.2, 1,024
+# tokens 23 / 14, 20 tokens behind 1,000 17 / 8, 256 behind 8,000 137 / 25; 28 heads of 128: 130 tokens 9.0 / 6.9, 2 x 100 behind 3,000
+# 72 / 26, five of 33 behind 3,295 73 / 64; 16 heads of 128: 64 behind 8,000 180 / 31.
+TC_PREFILL_MIN_TOKENS = {64: 2, 128: 2}
+TC_PREFILL_MIN_KEYS = 128
+
+
+def prefill_attention(head_dim: int, n_tokens: int, max_kv_len: int, window: int = 0):
+    """The attention kernel of a step of several tokens per sequence: the tcgen05 one where it has the head size and enough to do."""
+    least = TC_PREFILL_MIN_TOKENS.get(head_dim)
+    keys = min(max_kv_len, window) if window > 0 else max_kv_len
+    return ops.attention_prefill_tc if least is not None and n_tokens >= least and keys >= TC_PREFILL_MIN_KEYS else ops.attention_prefill
 
 
 class GqaAttention(Mixer):
@@ -287,11 +295,7 @@ class GqaAttention(Mixer):
             ops.attention_decode(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,
                                  self.scale, self.window, self.decode_splits(ctx), ctx.decode_scratch, ctx.err, plan)
         elif fast:
-            # the tcgen05 kernel works on blocks of 128 query rows, a long chain of pages per block: it pays for steps
-            # with many rows
-            least = TC_PREFILL_MIN_TOKENS.get(self.head_dim)
-            prefill = (ops.attention_prefill_tc if least is not None and n >= least and ctx.max_q_len >= 128
-                       else ops.attention_prefill)
+            prefill = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window)
             prefill(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,
                     ctx.max_q_len, self.scale, self.window, ctx.err, max_kv_len=ctx.max_kv_len)
         else:

@@ -18,7 +18,7 @@ import torch
 
 from .. import ops
 from ..config.spec import PartSpec
-from .attention import TC_PREFILL_MIN_TOKENS, GqaAttention
+from .attention import GqaAttention, prefill_attention
 from .base import TensorSpec
 from .registry import build_part, register_part
 
@@ -92,8 +92,7 @@ class DifferentialAttention(GqaAttention):
         attended = torch.empty_like(q)
         common = (q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs)
         if fast:
-            least = TC_PREFILL_MIN_TOKENS.get(self.head_dim)
-            run = ops.attention_prefill_tc if least is not None and n >= least and ctx.max_q_len >= 128 else ops.attention_prefill
+            run = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window)
             run(*common, ctx.max_q_len, self.scale, self.window, ctx.err, max_kv_len=ctx.max_kv_len)
         else:
             ops.attention_generic(*common, ctx.max_q_len, self.scale, self.window, ctx.err, scratch=ctx.decode_scratch,

@@ -29,7 +29,7 @@ import torch
 
 from .. import ops
 from ..cache import PAGE_TOKENS, KvNeed
-from .attention import TC_PREFILL_MIN_TOKENS
+from .attention import prefill_attention
 from .base import Mixer, TensorSpec
 from .registry import build_part, register_part
 
@@ -150,10 +150,7 @@ class LatentAttention(Mixer):
                                  self.window, n_splits, ctx.decode_scratch, ctx.err, self.decode_plan(ctx, n_splits),
                                  sinks=self.sinks, shared_values=True)
         elif fast:
-            # long steps on the tcgen05 kernel (blocks of 128 query rows), from the same sizes as any attention's
-            least = TC_PREFILL_MIN_TOKENS.get(r)
-            prefill = (ops.attention_prefill_tc if least is not None and n >= least and ctx.max_q_len >= 128
-                       else ops.attention_prefill)
+            prefill = prefill_attention(r, n, ctx.max_kv_len, self.window)
             prefill(q_in_latent, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, h, ctx.n_seqs, ctx.max_q_len,
                                   self.scale, self.window, ctx.err, max_kv_len=ctx.max_kv_len, sinks=self.sinks,
                                   shared_values=True)

@@ -1,0 +1,57 @@
+"""The tcgen05 prompt attention at sizes for which it takes one or two tiles a block and shares them among 1, 2, 4 or 8 blocks."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+CASES = [([200] * 6, 0, 14, 2, 64, 0), ([1024], 0, 14, 2, 64, 0), ([256], 8000, 14, 2, 64, 0), ([64], 3000, 14, 2, 64, 0),
+         ([200], 2000, 14, 2, 64, 0), ([183, 275, 1, 246], 0, 14, 2, 64, 0), ([300, 17], 3000, 16, 2, 128, 0), ([512], 0, 16, 2, 128, 0),
+         ([129, 5], 1215, 3, 1, 128, 0), ([300, 128], 700, 14, 2, 64, 150), ([2], 129, 6, 2, 128, 1000), ([130], 4000, 5, 5, 64, 3000)]
+
+
+@pytest.mark.parametrize("lens,before,heads,kv_heads,dim,window", CASES)
+@pytest.mark.parametrize("with_sinks", [False, True])
+def test_against_float64(lens, before, heads, kv_heads, dim, window, with_sinks):
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(sum(lens) + before)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    totals = [n + before for n in lens] + [70]          # a padding entry of 70 rows stands last
+    pages = [-(-t // 64) for t in totals[:-1]]
+    storage = torch.randn(sum(pages), 2, kv_heads, 64, dim, generator=g, device=DEV).bfloat16()
+    order, table, at = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(1)).tolist(), [], 0
+    for count in pages:
+        table.append(order[at:at + count] + [-1] * (max(pages) - count))
+        at += count
+    rows = [*lens, 70]
+    cu, pos = [0], []
+    for n in rows:
+        cu.append(cu[-1] + n)
+        pos += range(before, before + n)
+    q = (1.5 * torch.randn(cu[-1], heads * dim, generator=g, device=DEV)).bfloat16()
+    out, err = torch.full_like(q, 7.0), ints([0])
+    sinks = torch.randn(heads, generator=g, device=DEV) if with_sinks else None
+    site, table_t = ops.KvSiteArgs(storage, ints(table), kv_heads, dim), ints(table)
+    ops.attention_prefill_tc(q, out, ints(cu), ints(pos), ints([*range(len(lens)), -1]), site, heads, len(rows), max(rows), dim ** -0.5, window, err,
+                             max_kv_len=max(totals), sinks=sinks)
+    assert int(err) == 0 and not bool(out[cu[-2]:].any())
+    for s, n in enumerate(lens):
+        kv = storage[table_t[s, :pages[s]].long()].double().permute(1, 2, 0, 3, 4).reshape(2, kv_heads, -1, dim)[:, :, :totals[s]]
+        i, j = torch.arange(before, totals[s], device=DEV)[:, None], torch.arange(totals[s], device=DEV)[None]
+        hidden = (j > i) | (j <= i - window if window else torch.zeros_like(j > i))
+        for h in sorted({0, heads // 2, heads - 1}):
+            kvh = h // (heads // kv_heads)
+            scores = (q[cu[s]:cu[s + 1]].view(n, heads, dim)[:, h].double() @ kv[0, kvh].T * dim ** -0.5).masked_fill(hidden, float("-inf"))
+            if with_sinks:
+                scores = torch.cat((scores, sinks[h].double().expand(n, 1)), dim=1)
+            want = torch.softmax(scores, -1)[:, :totals[s]] @ kv[1, kvh]
+            got = out[cu[s]:cu[s + 1]].view(n, heads, dim)[:, h].double()
+            # weights and outputs are rounded to bfloat16 (2^-9 of each at most, independent: about 2^-9 of the norm)
+            assert float((got - want).norm() / want.norm()) < 2 ** -8
+
+
+def test_which_kernel_a_step_takes():
+    from qwenforge_b200 import ops
+    from qwenforge_b200.parts.attention import prefill_attention
+    assert prefill_attention(64, 2, 128) is ops.attention_prefill_tc and prefill_attention(128, 500, 4000, 200) is ops.attention_prefill_tc
+    assert prefill_attention(64, 100, 100) is ops.attention_prefill and prefill_attention(32, 500, 500) is ops.attention_prefill
+    assert prefill_attention(64, 500, 4000, 100) is ops.attention_prefill
