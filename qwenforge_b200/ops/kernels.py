@@ -876,22 +876,44 @@ def wide_gemm_takes(epilogue: int, weight: torch.Tensor, **tensors) -> bool:
     return answer
 
 
-def wide_gemm_takes_rows(epilogue: int, m: int, weight: torch.Tensor) -> bool:
+def wide_gemm_takes_rows(epilogue: int, m: int, weight: torch.Tensor, *, n_heads: int = 0, kv_heads: int = 0, head_dim: int = 0,
+                         rot_dim: int = 0) -> bool:
     """`wide_gemm_takes` for planning, before the step's tensors exist: `m` contiguous, aligned token rows against
-    `weight`, for the epilogues without further arguments (EPI_RESIDUAL, EPI_SWIGLU, EPI_PLAIN)."""
-    if not (weight.is_cuda and weight.dtype == torch.bfloat16) or epilogue == EPI_QKV:
+    `weight`; with EPI_QKV the heads, their size and how many components of each are rotated."""
+    if not (weight.is_cuda and weight.dtype == torch.bfloat16):
         return False
-    key = (weight.device.index, epilogue, tuple(weight.shape), weight.stride(0), m, weight.data_ptr() % 16)
+    key = (weight.device.index, epilogue, tuple(weight.shape), weight.stride(0), m, weight.data_ptr() % 16, n_heads, kv_heads, head_dim, rot_dim)
     answer = _wide_answers.get(key)
     if answer is None:
         a = _SkinnyArgs()
         a.w, a.n, a.k, a.ldw = weight.data_ptr(), weight.shape[0], weight.shape[1], weight.stride(0)
         a.x, a.ldx, a.m = 256, weight.shape[1], m          # only the alignment of the rows is looked at
         a.inter = a.n // 2 if epilogue == EPI_SWIGLU else 0
+        a.n_heads, a.kv_heads, a.head_dim, a.rot_dim = n_heads, kv_heads, head_dim, rot_dim
+        a.inv_freq = 256 if rot_dim > 0 else 0
         with torch.cuda.device(weight.device):
             answer = library("wide_gemm").qf_wide_gemm_takes(_I(epilogue), ctypes.byref(a)) != 0
         _wide_answers[key] = answer
     return answer
+
+
+def qkv_product_way(m: int, weight: torch.Tensor, n_heads: int, kv_heads: int, head_dim: int, rot_dim: int) -> str:
+    """How `m` token rows (64 at most) are normalised, multiplied by a QKV weight [N, K], rotated and stored fastest: "skinny" (the
+    mma.sync streamer with all of it inside), "wide" (a norm kernel, then the tcgen05 streamer with the rest) or "unfused" (norm,
+    library product, rotation). Measured as a whole decode step, microseconds, skinny / wide: Qwen2.5-0.5B (2 MB) 8 rows 673 / 703, 12 rows
+    960 / 850, 16 rows 963 / 863; 3B (10 MB) 1 row 1,908 / 1,876, 4 rows 2,040 / 1,973, 8 rows 2,238 / 2,144, 16 rows 2,365 / 2,173;
+    eight layers of 7B (33 MB) 1 row 982 / 1,000, 8 rows 1,004 / 1,020, 16 rows 1,062 / 1,037. So the tcgen05 streamer from 9 rows on, where
+    the other's token rows take a second pass over the tile, and below for weights whose tiles are too many for one wave of
+    the other's blocks and too few to fill its ring (8 to 20 MB). From 17 rows on the other way is "unfused" (against "wide": 0.5B
+    17 rows 918 / 871, 32 rows 932 / 888, 64 rows 991 / 990; twelve layers of 3B 890 / 841, 906 / 876, 979 / 968; 7B 1,073 / 1,050,
+    1,086 / 1,064, 1,205 / 1,209), which is no slower with 49 to 64 rows of a large weight."""
+    size = weight.numel() * weight.element_size()
+    heads = dict(n_heads=n_heads, kv_heads=kv_heads, head_dim=head_dim, rot_dim=rot_dim)
+    skinny = m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_QKV, True, **heads)
+    wide = m <= WIDE_MAX_ROWS and wide_gemm_takes_rows(EPI_QKV, m, weight, **heads)
+    if skinny and (not wide or (m <= 8 and not 8e6 <= size < 20e6)):
+        return "skinny"
+    return "wide" if wide and (m <= 48 or size < 20e6) else "unfused"
 
 
 def residual_product_way(m: int, weight: torch.Tensor) -> str:

@@ -409,11 +409,7 @@ class GqaAttention(Mixer):
     def _ways(self, ctx):
         rows = ctx.n_tokens
         rotary = self.position.fused_rotary() if self.position is not None else None
-        qkv = "unfused"
-        if rows <= ops.SKINNY_MAX_ROWS and ops.skinny_gemm_takes(rows, self.qkv_weight, ops.EPI_QKV, True, n_heads=self.n_heads,
-                                                                 kv_heads=self.n_kv, head_dim=self.head_dim,
-                                                                 rot_dim=rotary[1] if rotary else 0):
-            qkv = "skinny"
+        qkv = ops.qkv_product_way(rows, self.qkv_weight, self.n_heads, self.n_kv, self.head_dim, rotary[1] if rotary else 0)
         return qkv, ops.residual_product_way(rows, self.o_weight)
 
     def fused_takes(self, ctx) -> bool:
@@ -442,8 +438,13 @@ class GqaAttention(Mixer):
         else:
             x = torch.empty(hidden.shape, dtype=torch.bfloat16, device=hidden.device)
             ops.add_rms_norm(hidden, delta, rms[0], rms[1], x)   # the norm kernel adds the pending delta on its way
-            ops.rope_cache_write(ops.linear(x, self.qkv_weight), ctx.tok_seq, ctx.tok_pos, ctx.slots, inv_freq, rot_dim,
-                                 self.n_heads, q, args, writes_cache, ctx.err, bias=self.qkv_bias_t)
+            if qkv_way == "wide":
+                ops.wide_gemm(ops.EPI_QKV, self.qkv_weight, x=x, bias=self.qkv_bias_t,
+                              qkv=dict(n_heads=self.n_heads, site=args, inv_freq=inv_freq, rot_dim=rot_dim, tok_pos=ctx.tok_pos,
+                                       tok_seq=ctx.tok_seq, slots=ctx.slots, q_out=q, write_cache=writes_cache, err=ctx.err))
+            else:
+                ops.rope_cache_write(ops.linear(x, self.qkv_weight), ctx.tok_seq, ctx.tok_pos, ctx.slots, inv_freq, rot_dim,
+                                     self.n_heads, q, args, writes_cache, ctx.err, bias=self.qkv_bias_t)
         n_splits = self.decode_splits(ctx)
         if (o_way == "skinny" and n == ctx.n_seqs and ops.fold_project_pays(n, self.o_weight)
                 and ops.fold_project_takes(n, self.o_weight, hidden, self.n_heads, self.head_dim)):
