@@ -23,48 +23,11 @@
 // end of j's eighth), each factor at most as large as the decays make it, so nothing overflows or cancels.
 #include <type_traits>
 
-#include "mma.cuh"
+#include "chunks.cuh"
 
 #define SC_CHUNK 128
 #define SC_SUB 16
 #define SC_VT 64              // columns of v of a block, both kernels
-
-// x = hi + mid + lo, each a bfloat16 number (the upper half of a float32): cut off, subtract (exactly), twice.
-struct Thirds {
-    uint32_t hi, mid, lo;     // two neighbouring numbers each, the first in the lower half
-};
-__device__ __forceinline__ Thirds thirds(float x0, float x1) {
-    Thirds r;
-    uint32_t a = __float_as_uint(x0), b = __float_as_uint(x1);
-    r.hi = __byte_perm(a, b, 0x7632);
-    float s0 = x0 - __uint_as_float(a & 0xffff0000u), s1 = x1 - __uint_as_float(b & 0xffff0000u);
-    a = __float_as_uint(s0), b = __float_as_uint(s1);
-    r.mid = __byte_perm(a, b, 0x7632);
-    s0 -= __uint_as_float(a & 0xffff0000u), s1 -= __uint_as_float(b & 0xffff0000u);
-    r.lo = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);
-    return r;
-}
-__device__ __forceinline__ float lower_bf16(uint32_t pair) { return __uint_as_float(pair << 16); }
-__device__ __forceinline__ float upper_bf16(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
-
-// Byte offset of 16-byte piece `piece` of row `row` in a tile of WIDTH bfloat16 columns, pieces permuted so that eight
-// neighbouring rows read at one piece lie in eight different bank groups.
-template <int WIDTH>
-__device__ __forceinline__ uint32_t tile_at(int row, int piece) {
-    return (uint32_t)(row * (2 * WIDTH) + ((piece ^ (row & 7)) << 4));
-}
-// `rows` rows of a [.][WIDTH] tile from global rows `stride` elements apart; rows from n_here on become zeros.
-template <int WIDTH>
-__device__ __forceinline__ void fetch_tile(unsigned char* dst, const bf16* src, int stride, int n_here, int first, int threads) {
-    constexpr int PIECES = WIDTH / 8;
-    for (int i = first; i < SC_CHUNK * PIECES; i += threads) {
-        const int row = i / PIECES, piece = i % PIECES;
-        const bool there = row < n_here;
-        cp_async_16(dst + tile_at<WIDTH>(row, piece), there ? src + (size_t)row * stride + piece * 8 : src, there);
-    }
-}
-// The first record of a sequence: sequence s owns records cu_q[s] / SC_CHUNK + s onwards, as many as its chunks at most.
-__device__ __forceinline__ long long first_record(const int* cu_q, int seq) { return cu_q[seq] / SC_CHUNK + seq; }
 
 struct ChunkArgs {
     const bf16 *q, *k, *v;
@@ -108,10 +71,10 @@ chunk_parts_kernel(const ChunkArgs a) {
     const int t0 = a.cu_q[seq] + chunk * SC_CHUNK, n_here = min(SC_CHUNK, a.cu_q[seq + 1] - t0);
     if (n_here <= 0) return;
     const int group = head / (a.n_heads / a.n_groups);
-    fetch_tile<SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, blockDim.x);
-    fetch_tile<D>(k_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, blockDim.x);
+    fetch_tile<SC_CHUNK, SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, blockDim.x);
+    fetch_tile<SC_CHUNK, D>(k_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, blockDim.x);
     cp_async_commit();
-    const long long record = (first_record(a.cu_q, seq) + chunk) * a.n_heads + head;
+    const long long record = (first_record<SC_CHUNK>(a.cu_q, seq) + chunk) * a.n_heads + head;
     if (warp == 0) {
         // What a token adds counts at the chunk's end: its take and the decays behind it. Four neighbouring tokens per lane,
         // the products over the lanes above by shuffles.
@@ -210,7 +173,7 @@ chunk_chain_kernel(const ChunkArgs a) {
     const int len = a.cu_q[seq + 1] - a.cu_q[seq], slot = a.slots[seq];
     const int n_chunks = (len + SC_CHUNK - 1) / SC_CHUNK;
     if (n_chunks <= 0) return;
-    const long long first = first_record(a.cu_q, seq) * a.n_heads + head;
+    const long long first = first_record<SC_CHUNK>(a.cu_q, seq) * a.n_heads + head;
     float* kept = slot >= 0 ? a.state + slot * a.slot_stride : nullptr;
     const float* whole = a.whole + first;
     const int item = (int)blockIdx.x * 8 + (threadIdx.x >> 5);   // (8 columns of v, 16 rows of S)
@@ -289,11 +252,11 @@ chunk_outputs_kernel(const ChunkArgs a) {
     if (n_here <= 0) return;
     const int group = head / (a.n_heads / a.n_groups);
     const bool with_n = a.n_offset >= 0 && v0 == 0;
-    const long long record = (first_record(a.cu_q, seq) + chunk) * a.n_heads + head;
+    const long long record = (first_record<SC_CHUNK>(a.cu_q, seq) + chunk) * a.n_heads + head;
 
-    fetch_tile<D>(qk_s, a.q + (size_t)t0 * a.q_stride + group * D, a.q_stride, n_here, threadIdx.x, 128);
+    fetch_tile<SC_CHUNK, D>(qk_s, a.q + (size_t)t0 * a.q_stride + group * D, a.q_stride, n_here, threadIdx.x, 128);
     cp_async_commit();
-    fetch_tile<SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, 128);
+    fetch_tile<SC_CHUNK, SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, 128);
     cp_async_commit();
     const float2 gate = threadIdx.x < n_here ? gates_of(a, t0 + threadIdx.x, head) : make_float2(1.f, 0.f);   // this thread's token
     const float my_take = gate.y;
@@ -343,7 +306,7 @@ chunk_outputs_kernel(const ChunkArgs a) {
     }
     cp_async_wait<0>();
     __syncthreads();                   // the queries are in registers, v has arrived
-    fetch_tile<D>(qk_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, 128);
+    fetch_tile<SC_CHUNK, D>(qk_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, 128);
     cp_async_commit();
     // A row of v that is not finite must not reach the tokens before it through a weight of zero: looked for here, kept apart below.
     int odd = 0;

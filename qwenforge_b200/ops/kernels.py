@@ -2249,6 +2249,37 @@ def channel_decay(pre: torch.Tensor, bias: Optional[torch.Tensor], kind: str, ou
                                                  _I(DECAYS[kind]), _F(1.0 / tau), _ptr(out), _stream()), "channel_decay")
 
 
+def _outer_rows_args(who: str, q, k, v, decay, state, s_offset, n_heads, dim, vdim, y, bonus, decay_from) -> tuple:
+    """Checks the operands of the scan with a decay per row and of its chunked form; returns (kind, bias, 1 / tau) of the decays."""
+    for name, t in (("q", q), ("k", k), ("v", v)):
+        _rows(name, t, q.dtype)
+    _is_bf16(q.dtype)
+    n = q.shape[0]
+    if q.shape[1] != n_heads * dim or k.shape != q.shape or v.shape != (n, n_heads * vdim):
+        raise KernelError(f"{who}: q, k must be [T, heads * dim], v [T, heads * vdim]")
+    if dim > OUTER_STATE_MAX_DIM:
+        raise KernelError(f"{who}: a state of {dim} rows per head exceeds the kernel's {OUTER_STATE_MAX_DIM}")
+    _dev("decay", decay, torch.float32)
+    _dev("y", y, torch.float32)
+    if decay.shape != (n, n_heads * dim) or y.shape != (n, n_heads * vdim):
+        raise KernelError(f"{who}: decay must be float32 [T, heads * dim], y float32 [T, heads * vdim]")
+    if bonus is not None:
+        _dev("bonus", bonus, torch.float32)
+        if bonus.numel() != n_heads * dim:
+            raise KernelError(f"{who}: bonus must be float32 [heads, dim]")
+    kind, decay_bias, inv_tau = 0, None, 1.0
+    if decay_from is not None:
+        name, decay_bias, tau = decay_from
+        if name not in DECAYS or tau <= 0:
+            raise KernelError(f"{who}: decay_from names 'double_exp' or 'sigmoid_root' and a positive tau")
+        _dev("decay bias", decay_bias, torch.float32)
+        if decay_bias.numel() != n_heads * dim:
+            raise KernelError(f"{who}: the decays' bias must be float32 [heads * dim]")
+        kind, inv_tau = DECAYS[name] + 1, 1.0 / tau
+    _state(state, (s_offset, n_heads * dim * vdim))
+    return kind, decay_bias, inv_tau
+
+
 def outer_state_scan_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, cu_q: torch.Tensor,
                           slots: torch.Tensor, state: torch.Tensor, s_offset: int, n_heads: int, dim: int, vdim: int,
                           q_scale: float, y: torch.Tensor, bonus: Optional[torch.Tensor] = None, decay_from=None) -> None:
@@ -2259,36 +2290,45 @@ def outer_state_scan_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dec
     y float32 [T, heads * vdim]; S in `state` at s_offset as [heads, dim, vdim].
     `decay_from` = (kind, bias float32 [heads * dim], tau): `decay` holds the decays' pre-activations instead, and the kernel forms
     the decays on its way in, with the arithmetic of `channel_decay` (kind "double_exp" or "sigmoid_root")."""
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        _rows(name, t, q.dtype)
-    _is_bf16(q.dtype)
-    n = q.shape[0]
-    if q.shape[1] != n_heads * dim or k.shape != q.shape or v.shape != (n, n_heads * vdim):
-        raise KernelError("outer_state_scan_rows: q, k must be [T, heads * dim], v [T, heads * vdim]")
-    if dim > OUTER_STATE_MAX_DIM:
-        raise KernelError(f"outer_state_scan_rows: a state of {dim} rows per head exceeds the kernel's {OUTER_STATE_MAX_DIM}")
-    _dev("decay", decay, torch.float32)
-    _dev("y", y, torch.float32)
-    if decay.shape != (n, n_heads * dim) or y.shape != (n, n_heads * vdim):
-        raise KernelError("outer_state_scan_rows: decay must be float32 [T, heads * dim], y float32 [T, heads * vdim]")
-    if bonus is not None:
-        _dev("bonus", bonus, torch.float32)
-        if bonus.numel() != n_heads * dim:
-            raise KernelError("outer_state_scan_rows: bonus must be float32 [heads, dim]")
-    kind, decay_bias, inv_tau = 0, None, 1.0
-    if decay_from is not None:
-        name, decay_bias, tau = decay_from
-        if name not in DECAYS or tau <= 0:
-            raise KernelError("outer_state_scan_rows: decay_from names 'double_exp' or 'sigmoid_root' and a positive tau")
-        _dev("decay bias", decay_bias, torch.float32)
-        if decay_bias.numel() != n_heads * dim:
-            raise KernelError("outer_state_scan_rows: the decays' bias must be float32 [heads * dim]")
-        kind, inv_tau = DECAYS[name] + 1, 1.0 / tau
-    _state(state, (s_offset, n_heads * dim * vdim))
+    kind, decay_bias, inv_tau = _outer_rows_args("outer_state_scan_rows", q, k, v, decay, state, s_offset, n_heads, dim, vdim, y, bonus, decay_from)
     _check(library("recurrent").qf_outer_state_scan_rows(
         _I(_is_bf16(q.dtype)), _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay), _ptr(cu_q),
         _ptr(slots), _I(cu_q.numel() - 1), _ptr(state), _LL(state.stride(0)), _LL(s_offset), _I(n_heads), _I(n_heads), _I(dim),
         _I(vdim), _F(q_scale), _ptr(y), _ptr(bonus), _ptr(decay_bias), _I(kind), _F(inv_tau), _stream()), "outer_state_scan_rows")
+
+
+ROW_CHUNK = 64   # RC_CHUNK of csrc/row_chunks.cu
+# The longest sequence of a step from which the chunked form is the faster one however the step is issued. Inside a graph, one sequence,
+# scan / chunks in microseconds, 16 heads of 64 x 128: 128 tokens 23 / 33, 200: 35 / 34, 512: 83 / 36, 1,031: 164 / 52; 7 heads: 200
+# tokens 29 / 31, 512: 67 / 34. A step issued launch by launch waits for the host up to some 550 tokens, and two launches and a
+# buffer more cost it 5 of 103 microseconds.
+ROW_CHUNKS_MIN_TOKENS = 512
+
+
+def row_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, dim: int, vdim: int, max_q_len: int) -> bool:
+    """Whether a step's recurrence with a decay per row runs on `row_chunks`: bfloat16 rows that 16-byte accesses can address, 64 rows and
+    whole 64 columns (up to 512) of a head's state, and a sequence long enough. Otherwise `outer_state_scan_rows` takes it."""
+    return (max_q_len >= ROW_CHUNKS_MIN_TOKENS and dim == 64 and vdim % 64 == 0 and vdim <= 512 and q.dtype == torch.bfloat16 and q.is_cuda
+            and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0
+            and (q.data_ptr() | k.data_ptr() | v.data_ptr() | decay.data_ptr()) % 16 == 0)
+
+
+def row_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, cu_q: torch.Tensor, slots: torch.Tensor,
+               max_q_len: int, state: torch.Tensor, s_offset: int, n_heads: int, dim: int, vdim: int, q_scale: float, y: torch.Tensor,
+               bonus: Optional[torch.Tensor] = None, decay_from=None) -> None:
+    """`outer_state_scan_rows` in chunks of `ROW_CHUNK` tokens on the tensor cores: the same operands and results, the products'
+    float32 operands in three bfloat16 parts each. `max_q_len`: the most tokens any sequence brings. bfloat16 only
+    (`row_chunks_take`)."""
+    kind, decay_bias, inv_tau = _outer_rows_args("row_chunks", q, k, v, decay, state, s_offset, n_heads, dim, vdim, y, bonus, decay_from)
+    if q.dtype != torch.bfloat16:
+        raise KernelError("row_chunks: bfloat16 rows only (row_chunks_take)")
+    n, n_seqs = q.shape[0], cu_q.numel() - 1
+    records = n // ROW_CHUNK + n_seqs
+    scratch = torch.empty(records * n_heads * (dim * vdim + dim) + (n * n_heads * dim if kind else 0), dtype=torch.float32, device=q.device)
+    _check(library("row_chunks").qf_row_chunks(
+        _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay), _ptr(decay_bias), _I(kind), _F(inv_tau),
+        _ptr(bonus), _ptr(cu_q), _ptr(slots), _I(n_seqs), _I(max_q_len), _ptr(state), _LL(state.stride(0)), _LL(s_offset), _I(n_heads),
+        _I(dim), _I(vdim), _F(q_scale), _ptr(scratch), _LL(records), _ptr(y), _stream()), "row_chunks")
 
 
 def rows_prepare(x: torch.Tensor, runs, eps: float, mix=None) -> None:

@@ -215,6 +215,15 @@ def _low_rank(x, first, second, activation):
     return ops.linear_rows(low, second, out_dtype=torch.float32)
 
 
+def _scan_rows(ctx, q, k, v, pre, state, s_offset, heads, dim, vdim, q_scale, y, **decays):
+    """The recurrence with a decay per row of the state: in chunks on the tensor cores where the step and its sizes allow
+    (`ops.row_chunks`), token by token otherwise (short steps, float32, other sizes)."""
+    if ops.row_chunks_take(q, k, v, pre, dim, vdim, ctx.max_q_len):
+        ops.row_chunks(q, k, v, pre, ctx.cu_q, ctx.slots, ctx.max_q_len, state, s_offset, heads, dim, vdim, q_scale, y, **decays)
+    else:
+        ops.outer_state_scan_rows(q, k, v, pre, ctx.cu_q, ctx.slots, state, s_offset, heads, dim, vdim, q_scale, y, **decays)
+
+
 class TimeMix(Mixer):
     """params: hidden_size, num_heads, head_dim, eps, and optionally rank (of the decay's low-rank pair; read from the
     tensors where absent).
@@ -245,7 +254,7 @@ class TimeMix(Mixer):
                         TensorSpec(f("norm"), (c,), init="norm"), TensorSpec(f("o_weight"), (w, c))]
 
     def kernel_libraries(self, dtype):
-        return {"recurrent", "activation", "grouped_gemm"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm"})
+        return {"recurrent", "activation", "grouped_gemm"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "row_chunks"})
 
     def cache_need(self):
         return StateNeed((self.state_floats,), torch.float32)
@@ -285,10 +294,10 @@ class TimeMix(Mixer):
             ops.head_linear(mixes[:, :4 * w], self.proj_weight, proj)
             pre = _low_rank(mixes[:, 4 * w:], self.w1, self.w2, "tanh")
         y = torch.empty((n, c), **f32)   # (the scan forms the decays exp(-exp(pre + w0)) on its way in)
-        ops.outer_state_scan_rows(proj[:, :c], proj[:, c:2 * c], proj[:, 2 * c:3 * c], pre, ctx.cu_q, ctx.slots, site.storage,
-                                  self.s_offset, h, d, d, 1.0, y, bonus=self.bonus, decay_from=("double_exp", self.w0, 1.0))
+        q, k, values, gate = proj.split((c, c, c, c), dim=1)
+        _scan_rows(ctx, q, k, values, pre, site.storage, self.s_offset, h, d, d, 1.0, y, bonus=self.bonus, decay_from=("double_exp", self.w0, 1.0))
         out = torch.empty((n, c), dtype=x.dtype, device=x.device)
-        ops.gated_group_norm(y, proj[:, 3 * c:], self.norm, self.eps, out, h, h, "silu", False)
+        ops.gated_group_norm(y, gate, self.norm, self.eps, out, h, h, "silu", False)
         return ops.linear_rows(out, self.o_weight)
 
 
@@ -316,7 +325,7 @@ class GatedLinearAttention(Mixer):
                 TensorSpec(f("a2_bias"), (h * d,), init="logit", keep="float32")]
 
     def kernel_libraries(self, dtype):
-        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm"})
+        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "row_chunks"})
 
     def cache_need(self):
         return StateNeed((self.state_floats,), torch.float32)
@@ -348,10 +357,10 @@ class GatedLinearAttention(Mixer):
             proj = ops.linear_rows(x, self.proj_weight)                                  # [T, q | k | v | g]
             pre = _low_rank(x, self.a1, self.a2, None)                                   # float32 sums
         y = torch.empty((n, h * v), **f32)   # (the scan forms the decays sigmoid(pre + b)^(1 / tau) on its way in)
-        ops.outer_state_scan_rows(proj[:, :h * d], proj[:, h * d:2 * h * d], proj[:, 2 * h * d:2 * h * d + h * v], pre, ctx.cu_q,
-                                  ctx.slots, site.storage, 0, h, d, v, d ** -0.5, y, decay_from=("sigmoid_root", self.a2_bias, self.tau))
+        q, k, values, gate = proj.split((h * d, h * d, h * v, h * v), dim=1)
+        _scan_rows(ctx, q, k, values, pre, site.storage, 0, h, d, v, d ** -0.5, y, decay_from=("sigmoid_root", self.a2_bias, self.tau))
         out = torch.empty((n, h * v), dtype=x.dtype, device=x.device)
-        ops.gated_group_norm(y, proj[:, 2 * h * d + h * v:], self.norm, self.eps, out, h, h, "silu", False)
+        ops.gated_group_norm(y, gate, self.norm, self.eps, out, h, h, "silu", False)
         return ops.linear_rows(out, self.o_weight)
 
 
