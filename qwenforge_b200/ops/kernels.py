@@ -421,9 +421,9 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor,
                          slots: torch.Tensor, site: KvSiteArgs, n_heads: int, n_seqs: int, max_q_len: int, scale: float,
                          window: int, err: torch.Tensor, max_kv_len: Optional[int] = None,
                          sinks: Optional[torch.Tensor] = None, shared_values: bool = False) -> None:
-    """The same attention on the fifth-generation tensor cores (tcgen05, accumulators in tensor memory): blocks of
-    128 query rows; bfloat16, head sizes 64 and 128, cache pages without gaps. `max_kv_len` as in `attention_prefill`:
-    with few tiles of many pages, two blocks of a cluster share a tile."""
+    """The same attention on the fifth-generation tensor cores (tcgen05, accumulators in tensor memory): one or two tiles of
+    128 query rows a block; bfloat16, head sizes 64 and 128, cache pages without gaps. `max_kv_len` as in `attention_prefill`:
+    few tiles of many pages are shared by the two, four or eight blocks of a cluster."""
     _dev("q", q, torch.bfloat16)
     _dev("out", out, torch.bfloat16)
     _dev("cache", site.storage, torch.bfloat16)

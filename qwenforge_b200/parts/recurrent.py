@@ -1,8 +1,8 @@
 """Recurrent mixers: a state of fixed size per sequence instead of keys and values per position.
 
 Both kinds here keep, per head, a matrix S that every token decays and adds an outer product to, and read it with a
-query:  S <- decay_t S + take_t k_t v_t^T,  y_t = S^T q_t  (`ops.outer_state_scan`, float32 inside). They differ in where
-k, v, q and the two gates come from and in what follows the scan:
+query:  S <- decay_t S + take_t k_t v_t^T,  y_t = S^T q_t  (`ops.outer_state_scan`, and for long steps in chunks
+`ops.state_chunks`; float32 inside). They differ in where k, v, q and the two gates come from and in what follows the scan:
 
   matrix_memory (the mLSTM of xLSTM)
       q = Wq h / sqrt(dim), k = Wk h, v = Wv h in heads; exponential gates with a running maximum m (0 at a sequence's start):
@@ -14,7 +14,8 @@ k, v, q and the two gates come from and in what follows the scan:
       decay = exp(-exp(A_log) dt), take = dt, k = B, q = C (shared by the heads of a group), v = x;
       y <- y + D x;  out = Wo (rms_in_parts(y * silu(z)) * w)
 
-Two more kinds decay every ROW of S by a number of its own (a decay per head and key channel, `ops.outer_state_scan_rows`):
+Two more kinds decay every ROW of S by a number of its own (a decay per head and key channel, `ops.outer_state_scan_rows`,
+for long steps `ops.row_chunks`):
 
   time_mix (RWKV-style time mixing)
       with h' the token before (zeros at a sequence's start) each of r, k, v, g, w reads its own mix  h + (h' - h) mu_s;
