@@ -45,7 +45,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 }
 
 #define TA_BM 128              // rows of a tile
+// (also of attention_prefill_page.cuh)
 #define TA_BK 128              // keys of a turn: two pages
+
+#include "attention_prefill_page.cuh"
 
 template <int D, int SPLIT, int PER>
 __global__ void __launch_bounds__(128 * PER + 64, 1)
@@ -477,6 +480,9 @@ static int launch(const void* q, void* out, const int* cu_q, const int* tok_pos,
     // (tiles that hold rows: the grid also has blocks for the rows that shorter sequences lack, which end at once)
     const long long live = min((long long)q_tiles * n_seqs, max((2ll * n_tokens + (long long)TA_BM * n_seqs + TA_BM - 1) / (2 * TA_BM), 1ll)) * n_heads;
     const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
+    if (D == 64 && pages_pay(live, span, q_tiles, sms))
+        return launch_pages<true>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, sinks,
+                                  planes, stream);
     const float turn[2] = {D <= 64 ? 1.5f : 1.75f, D <= 64 ? 1.85f : 2.05f}, ends[2][4] = {{3.f, 5.f, 5.5f, 6.5f}, {5.f, 6.5f, 9.f, 13.f}};
     const int room[4] = {sms, sms, sms - sms / 8, sms * 77 / 100 > 0 ? sms * 77 / 100 : 1};
     int per = 2, split = 1;

@@ -6,7 +6,10 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 CASES = [([200] * 6, 0, 14, 2, 64, 0), ([1024], 0, 14, 2, 64, 0), ([256], 8000, 14, 2, 64, 0), ([64], 3000, 14, 2, 64, 0),
          ([200], 2000, 14, 2, 64, 0), ([183, 275, 1, 246], 0, 14, 2, 64, 0), ([300, 17], 3000, 16, 2, 128, 0), ([512], 0, 16, 2, 128, 0),
-         ([129, 5], 1215, 3, 1, 128, 0), ([300, 128], 700, 14, 2, 64, 150), ([2], 129, 6, 2, 128, 1000), ([130], 4000, 5, 5, 64, 3000)]
+         ([129, 5], 1215, 3, 1, 128, 0), ([300, 128], 700, 14, 2, 64, 150), ([2], 129, 6, 2, 128, 1000), ([130], 4000, 5, 5, 64, 3000),
+         # prompts that small blocks take (three on an SM, two a tile), and their neighbours that they do not
+         ([1153], 0, 16, 2, 64, 0), ([1500, 300, 1], 0, 14, 2, 64, 0), ([1409], 0, 14, 14, 64, 1100), ([3500], 0, 14, 2, 64, 0),
+         ([1000], 0, 14, 2, 64, 0), ([1153], 64, 16, 2, 64, 0)]
 
 
 @pytest.mark.parametrize("lens,before,heads,kv_heads,dim,window", CASES)
