@@ -61,8 +61,8 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const int rank = SPLIT ? (int)(blockIdx.x & 1) : 0;
     // Launched as a programmatic dependent: what a block works out and sets up before its first copy (its tile, the
     // barriers, its tensor memory) runs under the tail of the kernel before, which wrote the queries and the new keys
-    // and values; they are read, and the output written, only after the wait.
-    grid_launch_dependents();
+    // and values; they are read, and the output written, only after the wait. The kernel after it may start when every block
+    // has its tensor memory (or has ended).
     __shared__ __align__(8) uint64_t bar_q, bar_kv[2], bar_s, bar_sfree, bar_pv, bar_p;
     __shared__ uint32_t tmem_base_s;
 
@@ -112,6 +112,7 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_launch_dependents();
     grid_dependency_wait();
     const uint32_t tmem = tmem_base_s;
     bool timed_out = false;
@@ -395,7 +396,8 @@ static int launch_pages(const CUtensorMap& q_map, const CUtensorMap& kv_map, voi
                           const int* slots, KvSite<bf16> site, int n_heads, int n_seqs, int max_q_len, float scale, int window,
                           int* err, const float* sinks, int planes, cudaStream_t stream) {
     constexpr int D = 64;
-    size_t smem = (size_t)(D / 64) * TA_BM * 128 + 4 * (size_t)(D / 64) * QF_PAGE * 128 + TA_BM * 128 + 1024;
+    constexpr size_t smem = (size_t)(D / 64) * TA_BM * 128 + 4 * (size_t)(D / 64) * QF_PAGE * 128 + TA_BM * 128 + 1024;
+    static_assert(qf_tmem_fits(128, smem), "the rule of tcgen05.cuh");
     auto kernel = prefill_page_kernel<SPLIT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;

@@ -83,9 +83,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     const int pair = units / per_pair - 1 - unit / per_pair, kvh = (unit % per_pair) % site.kv_heads, seq = (unit % per_pair) / site.kv_heads;
     // Launched as a programmatic dependent: what a block works out and sets up before its first copy (its tiles, the barriers, its
     // tensor memory) runs under the tail of the kernel before, which wrote the queries and the new keys and values; they are
-    // read, and the output written, only after the wait. (No kernel that takes tensor memory itself leaves room for this one's
-    // shared memory beside it, so the kernel before is not kept from finishing by what this one holds.)
-    grid_launch_dependents();
+    // read, and the output written, only after the wait. The kernel after it may start when every block has its tensor memory (or has ended).
     const int q_begin = cu_q[seq], q_len = cu_q[seq + 1] - q_begin;
     const int tiles_here = (q_len + TA_BM - 1) / TA_BM * group;   // of this sequence and kv head; tile n: head n % group, rows n / group
     if (PER * pair >= tiles_here) return;
@@ -141,6 +139,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_launch_dependents();
     grid_dependency_wait();
     const uint32_t tmem = tmem_base_s;
     bool timed_out = false;
@@ -424,11 +423,12 @@ template <int D, int SPLIT, int PER>
 static int launch_variant(const CUtensorMap& q_map, const CUtensorMap& kv_map, void* out, const int* cu_q, const int* tok_pos,
                           const int* slots, KvSite<bf16> site, int n_heads, int n_seqs, long long tiles, float scale,
                           int window, int* err, const float* sinks, int planes, cudaStream_t stream) {
-    // One block per SM, also where two would find room: a block with two tiles holds all of its SM's tensor memory, and the blocks
-    // of clusters that wait for one another must not wait for one another's tensor memory as well.
-    constexpr size_t stages = (size_t)(D / 64) * (PER * TA_BM + 4 * TA_BK) * 128 + 1024, alone = 120 * 1024;
+    // One block per SM, also where two would find room, and no other kernel's that takes tensor memory: a block with two tiles holds
+    // all of its SM's, and the blocks of clusters that wait for one another must not wait for tensor memory as well.
+    constexpr size_t stages = (size_t)(D / 64) * (PER * TA_BM + 4 * TA_BK) * 128 + 1024, alone = QF_TMEM_SMEM_ALONE;
     constexpr size_t merge = (size_t)PER * (D + 2 * SPLIT) * TA_BM * sizeof(float) + 1024;
     constexpr size_t smem = stages > merge ? (stages > alone ? stages : alone) : (merge > alone ? merge : alone);
+    static_assert(qf_tmem_fits(256 * PER, smem) && smem <= 227 * 1024, "the rule of tcgen05.cuh");
     auto kernel = prefill_tc_kernel<D, SPLIT, PER>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;

@@ -99,6 +99,7 @@ template <int BN> struct TcGeometry {
     static constexpr int stages = BN == 128 ? 3 : 4;
     static constexpr int stage_bytes = (TC_BM + BN) * TC_BK * 2;
     static constexpr size_t smem = (size_t)stages * stage_bytes + 1024;
+    static_assert(qf_tmem_fits(BN, smem), "the rule of tcgen05.cuh");
 };
 
 // Instruction descriptor: float32 accumulator, bf16 A and B, both K-major, N = BN, M = 128.
@@ -487,7 +488,8 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 template <int EPI>
 static int launch_persistent(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int m, int n_out, int k, int inter,
                              int ldo, int m_tiles, int n_tiles, int* err, cudaStream_t stream) {
-    const size_t smem = (size_t)TP_STAGES * TP_STAGE_BYTES + 1024;
+    constexpr size_t smem = (size_t)TP_STAGES * TP_STAGE_BYTES + 1024;
+    static_assert(qf_tmem_fits(2 * TP_BN, smem), "the rule of tcgen05.cuh");
     cudaError_t e = cudaFuncSetAttribute(tc_gemm_persistent_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int total = m_tiles * n_tiles, sms = qf_sm_count();

@@ -4,6 +4,21 @@
 #pragma once
 #include "tma.cuh"
 
+// Tensor memory is handed out by an instruction that waits, without a limit, until the columns are free, and not by the launch. So no
+// block may ever have to wait for a block that waits for it in turn:
+// (1) A kernel lets the kernel after it start (grid_launch_dependents) only when it has its columns: the one after it allocates before
+//     it waits for this one, and would otherwise take the columns that this one still needs in order to end.
+// (2) Blocks that find room on one SM together find their columns there too, whatever kernels they belong to (several streams;
+//     blocks of clusters that wait for one another): a kernel of up to 128 columns asks for QF_TMEM_SMEM_SHARED bytes of shared memory or
+//     more, so that three fit an SM (384 of 512 columns), one of more columns for QF_TMEM_SMEM_ALONE, beside which none fits (an
+//     SM has 228 KB, a block costs 1 KB more than it asks for).
+#define QF_TMEM_SMEM_SHARED (65 * 1024)
+#define QF_TMEM_SMEM_ALONE (193 * 1024)
+__host__ __device__ constexpr bool qf_tmem_fits(int columns, size_t smem) {
+    return columns <= 128 ? smem >= QF_TMEM_SMEM_SHARED : smem >= QF_TMEM_SMEM_ALONE;
+}
+static_assert(4 * (QF_TMEM_SMEM_SHARED + 1024) > 228 * 1024 && QF_TMEM_SMEM_ALONE + QF_TMEM_SMEM_SHARED + 2048 > 228 * 1024, "see above");
+
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes, stored with the 128-byte swizzle:
 // start address / 16; leading byte offset 1 (unused for swizzled K-major); stride between 8-row groups 1024 bytes;
 // descriptor version 1 (sm_100); layout type 2 (SWIZZLE_128B).

@@ -441,6 +441,7 @@ static bool wide_plan(int epilogue, const SkinnyArgs& a, int sms, WideGeometry& 
     if (geo.group < 1 || geo.stages < 1) return false;
     geo.stamps = nullptr;
     smem = (size_t)geo.stages * geo.stage_bytes + extra + 1024;
+    if (smem < QF_TMEM_SMEM_SHARED) smem = QF_TMEM_SMEM_SHARED;   // (64 or 128 columns: the rule of tcgen05.cuh)
     return smem <= 224 * 1024;
 }
 
