@@ -5,9 +5,8 @@
 // A state row of a sequence is `state + slot * slot_stride`; every kernel is told at which float of the row its piece
 // starts. A sequence whose slot is -1 (a padding entry of the batch) runs from a zero state and stores nothing.
 // Everything is float32 inside; q, k, v, the gate of the output and the convolution's input and output carry the
-// activation dtype. A token's result depends on its own sequence only, and on the tokens before it in their order; the scans and
-// the convolution walk a sequence token by token in one fixed order of operations, so that how it was cut into steps changes
-// nothing (the exponential gates' running maximum: by rounding).
+// activation dtype. A token's result depends on its own sequence only, and on the tokens before it in their order, never
+// on how they were cut into steps: every kernel walks a sequence token by token in one fixed order of operations.
 #include <float.h>
 
 #include "common.cuh"
@@ -22,17 +21,15 @@ template <typename T> __device__ __forceinline__ float silu_for(float z) { retur
 template <> __device__ __forceinline__ float silu_for<bf16>(float z) { return __fdividef(z, 1.f + __expf(-z)); }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Exponential gates with a running maximum (the mLSTM's): one block per (sequence, head), GATE_TOKENS tokens at a time, up to
-// GATE_EACH neighbouring tokens to a thread. Every thread works out its tokens' two log gates (tanh, logsigmoid) and what they do
-// together to the maximum before them, m -> max(F + m, M); these pairs compose, so that a scan over the block hands every thread the
-// maximum before its first token. From there it runs m' = max(f + m, a) through its own tokens in order and forms their
-// exponentials. (With one warp running the maximum through all tokens, 32 links at a time, 2,048 tokens of 7 heads took 38
-// microseconds; 9 so.) How the sums of f are grouped depends on the cut of a sequence into steps, so m does by rounding; what a
-// token's gates say is always exp(f + m - m') and exp(a - m') of the very m and m' beside it, whose rounding cancels in the
-// mixer's quotient.
+// Exponential gates with a running maximum (the mLSTM's): one block per (sequence, head), GATE_TOKENS tokens at a time. Every
+// thread works out its tokens' two log gates (tanh, logsigmoid); then one thread runs the maximum m' = max(f + m, a) through the
+// tokens in order, eight at a time with the next eight's gates already on their way; then every thread forms its tokens'
+// three exponentials. Neighbouring tokens share the very same m, so what a token's gates say cancels in the mixer's quotient, and the
+// chain is the same operations in the same order for every cut of a sequence, in both precisions. What bounds it is that chain,
+// an addition and a maximum a token.
 #define GATE_THREADS 256
-#define GATE_EACH 8
-#define GATE_TOKENS (GATE_THREADS * GATE_EACH)
+#define GATE_TOKENS 2048
+#define GATE_LINKS 8
 
 __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
@@ -42,62 +39,74 @@ stabilized_gates_kernel(const float* __restrict__ pre, int pre_stride, const flo
                         long long slot_stride, long long m_offset, int n_heads, float* __restrict__ decay,
                         float* __restrict__ take, float* __restrict__ floor_out) {
     grid_chain_entry();
-    __shared__ float warp_f[GATE_THREADS / 32], warp_m[GATE_THREADS / 32], last_m;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int EACH = GATE_TOKENS / GATE_THREADS;
+    __shared__ __align__(16) float a_s[GATE_TOKENS], f_s[GATE_TOKENS], m_s[GATE_TOKENS];   // m_s: the maximum behind each token
     const int seq = blockIdx.x / n_heads, head = blockIdx.x % n_heads;
     const int begin = cu_q[seq], end = cu_q[seq + 1], slot = slots[seq];
     float* m_ptr = slot >= 0 ? state + slot * slot_stride + m_offset + head : nullptr;
     float m = m_ptr ? *m_ptr : 0.f;   // the maximum before the tokens in hand
     const float bi = bias[head], bf = bias[n_heads + head];
     for (int t0 = begin; t0 < end; t0 += GATE_TOKENS) {
-        const int n_here = min(GATE_TOKENS, end - t0), each = (n_here + GATE_THREADS - 1) / GATE_THREADS;
-        const int first = threadIdx.x * each, count = max(0, min(each, n_here - first));   // this thread's tokens
-        float a[GATE_EACH], f[GATE_EACH];
-        float all_f = 0.f, all_m = -INFINITY;                                               // together: m -> max(all_f + m, all_m)
+        const int n_here = min(GATE_TOKENS, end - t0), n_links = (n_here + GATE_LINKS - 1) / GATE_LINKS * GATE_LINKS;
+        float a[EACH], f[EACH];
 #pragma unroll
-        for (int i = 0; i < GATE_EACH; ++i) {
-            if (i < count) {
-                const float* row = pre + (size_t)(t0 + first + i) * pre_stride + head;
+        for (int i = 0; i < EACH; ++i) {
+            const int j = threadIdx.x + GATE_THREADS * i;
+            a[i] = f[i] = 0.f;   // (behind the last token: links that nobody reads)
+            if (j < n_here) {
+                const float* row = pre + (size_t)(t0 + j) * pre_stride + head;
                 a[i] = row[0], f[i] = row[n_heads];
             }
         }
 #pragma unroll
-        for (int i = 0; i < GATE_EACH; ++i) {
-            if (i < count) {
+        for (int i = 0; i < EACH; ++i) {
+            const int j = threadIdx.x + GATE_THREADS * i;
+            if (j < n_here) {
                 a[i] = cap * tanhf((a[i] + bi) / cap);
                 f[i] = log_sigmoid(cap * tanhf((f[i] + bf) / cap));
-                all_f += f[i];
-                all_m = fmaxf(f[i] + all_m, a[i]);
             }
+            if (j < n_links) a_s[j] = a[i], f_s[j] = f[i];
         }
-        // the tokens before this thread's, as one pair: within the warp by shuffles, then the warps before
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float before_f = __shfl_up_sync(0xffffffffu, all_f, o), before_m = __shfl_up_sync(0xffffffffu, all_m, o);
-            if (lane >= o) {
-                all_m = fmaxf(all_f + before_m, all_m);
-                all_f += before_f;
-            }
-        }
-        if (lane == 31) warp_f[warp] = all_f, warp_m[warp] = all_m;
-        const float lane_f = __shfl_up_sync(0xffffffffu, all_f, 1), lane_m = __shfl_up_sync(0xffffffffu, all_m, 1);
         __syncthreads();
-        for (int w = 0; w < warp; ++w) m = fmaxf(warp_f[w] + m, warp_m[w]);
-        if (lane > 0) m = fmaxf(lane_f + m, lane_m);
+        if (threadIdx.x == 0) {
+            const float4 *a4 = reinterpret_cast<const float4*>(a_s), *f4 = reinterpret_cast<const float4*>(f_s);
+            float4* m4 = reinterpret_cast<float4*>(m_s);
+            float4 next_a[GATE_LINKS / 4], next_f[GATE_LINKS / 4];
+            float run = m;
 #pragma unroll
-        for (int i = 0; i < GATE_EACH; ++i) {
-            if (i < count) {
-                const float m_new = fmaxf(f[i] + m, a[i]);
-                const size_t at = (size_t)(t0 + first + i) * n_heads + head;
-                decay[at] = expf(f[i] + m - m_new);
-                take[at] = expf(a[i] - m_new);
-                floor_out[at] = expf(-m_new);
-                m = m_new;
+            for (int u = 0; u < GATE_LINKS / 4; ++u) next_a[u] = a4[u], next_f[u] = f4[u];
+            for (int g = 0; g < n_links / 4; g += GATE_LINKS / 4) {
+                float4 at[GATE_LINKS / 4], ft[GATE_LINKS / 4];
+#pragma unroll
+                for (int u = 0; u < GATE_LINKS / 4; ++u) {
+                    at[u] = next_a[u], ft[u] = next_f[u];
+                    const int ahead = min(g + GATE_LINKS / 4, n_links / 4 - GATE_LINKS / 4) + u;
+                    next_a[u] = a4[ahead], next_f[u] = f4[ahead];
+                }
+#pragma unroll
+                for (int u = 0; u < GATE_LINKS / 4; ++u) {
+                    float4 out;
+                    run = out.x = fmaxf(ft[u].x + run, at[u].x);
+                    run = out.y = fmaxf(ft[u].y + run, at[u].y);
+                    run = out.z = fmaxf(ft[u].z + run, at[u].z);
+                    run = out.w = fmaxf(ft[u].w + run, at[u].w);
+                    m4[g + u] = out;
+                }
             }
         }
-        if (count > 0 && first + count == n_here) last_m = m;
         __syncthreads();
-        m = last_m;
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            const int j = threadIdx.x + GATE_THREADS * i;
+            if (j < n_here) {
+                const float before = j > 0 ? m_s[j - 1] : m, mine = m_s[j];
+                const size_t at = (size_t)(t0 + j) * n_heads + head;
+                decay[at] = expf(f[i] + before - mine);
+                take[at] = expf(a[i] - mine);
+                floor_out[at] = expf(-mine);
+            }
+        }
+        m = m_s[n_here - 1];   // (written again only behind the next barrier)
     }
     if (m_ptr && threadIdx.x == 0 && begin < end) *m_ptr = m;
 }

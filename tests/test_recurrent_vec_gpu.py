@@ -1,4 +1,4 @@
-"""The norm behind the scans in 16-byte pieces and the gates' maximum as a scan over a block, at the edges of their pieces."""
+"""The norm behind the scans in 16-byte pieces and the gates' maximum over blocks of tokens, at the edges of their pieces."""
 import pytest
 import torch
 
@@ -50,3 +50,24 @@ def test_stabilized_gates_over_blocks_of_tokens(lengths):
     # m is a sum of up to a few dozen log gates of size up to 15 before a larger one takes over: 2^-24 x 15 x a few dozen
     for got, want in zip(*results):
         assert float(((got.double() - want.double()).abs() / (1 + want.double().abs())).max()) < 3e-5
+
+
+@pytest.mark.parametrize("pieces", [[1] * 300, [255, 256, 257, 2048, 1], [7, 2049, 8, 9, 2040]])
+def test_stabilized_gates_do_not_depend_on_the_cut(pieces):
+    """The maximum is one chain of additions and maxima in the tokens' order: bit for bit the same numbers however a sequence is cut,
+    and every token is decayed with the very maximum that the token before it was scaled by."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(len(pieces))
+    heads, n = 3, sum(pieces)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pre, bias = 2 * torch.randn(n, 2 * heads, generator=g, device=DEV), torch.tensor([0.0] * heads + [3.0] * heads, device=DEV)
+    results = []
+    for cut in ([n], pieces):
+        state, trio, at = torch.zeros(1, heads, device=DEV), [torch.empty(n, heads, device=DEV) for _ in range(3)], 0
+        for length in cut:
+            here = slice(at, at + length)
+            ops.stabilized_gates(pre[here], bias, 15.0, ints([0, length]), ints([0]), state, 0, heads, *(t[here] for t in trio))
+            at += length
+        results.append((state, *trio))
+    for whole, cut in zip(*results):
+        assert torch.equal(whole, cut)
