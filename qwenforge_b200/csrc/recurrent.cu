@@ -11,15 +11,6 @@
 
 #include "common.cuh"
 
-// Sigmoid and silu of a float32 number. Where the result is rounded to bfloat16 next, by the hardware's exponential and
-// reciprocal (relative error below 1e-5 for |z| up to 88 and below 1e-6 where the result matters; a bfloat16 keeps 2^-9): the exact
-// division and exponential are some thirty instructions an element, which bound the convolution and the norm below
-// rather than memory.
-template <typename T> __device__ __forceinline__ float sigmoid_for(float z) { return 1.f / (1.f + expf(-z)); }
-template <> __device__ __forceinline__ float sigmoid_for<bf16>(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
-template <typename T> __device__ __forceinline__ float silu_for(float z) { return z / (1.f + expf(-z)); }
-template <> __device__ __forceinline__ float silu_for<bf16>(float z) { return __fdividef(z, 1.f + __expf(-z)); }
-
 // ------------------------------------------------------------------------------------------------------------------
 // Exponential gates with a running maximum (the mLSTM's): one block per (sequence, head), GATE_TOKENS tokens at a time. Every
 // thread works out its tokens' two log gates (tanh, logsigmoid); then one thread runs the maximum m' = max(f + m, a) through the
@@ -673,8 +664,12 @@ gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict_
             add[i] = skip[head];
             extra[i] = *reinterpret_cast<const uint4*>(skip_x + (size_t)t * skip_stride + c);
         }
-        if (nq) by[i] = 1.f / (fmaxf(fabsf(nq[(size_t)t * n_heads + head]), floor_in[(size_t)t * n_heads + head]) + floor_add);
+        if (nq) by[i] = fmaxf(fabsf(nq[(size_t)t * n_heads + head]), floor_in[(size_t)t * n_heads + head]) + floor_add;
     }
+    auto gate_of = [&](float raw) {
+        const float sig = 1.f / (1.f + expf(-raw));
+        return gate_kind == 0 ? sig : raw * sig;
+    };
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < P; ++i) {
@@ -683,13 +678,13 @@ gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict_
         const __nv_bfloat162* ep = reinterpret_cast<const __nv_bfloat162*>(&extra[i]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            if (nq) v[e] *= by[i];
+            if (nq) v[e] /= by[i];
             const float2 x2 = __bfloat1622float2(ep[e >> 1]);
             if (skip) v[e] = fmaf(add[i], e & 1 ? x2.y : x2.x, v[e]);
             if (gate_first) {
                 const float2 g2 = __bfloat1622float2(gp[e >> 1]);
                 const float raw = e & 1 ? g2.y : g2.x;
-                v[e] *= gate_kind == 0 ? sigmoid_for<bf16>(raw) : silu_for<bf16>(raw);
+                v[e] *= gate_of(raw);
             }
             sum = has[i] ? fmaf(v[e], v[e], sum) : sum;
         }
@@ -713,8 +708,8 @@ gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict_
             const float2 w2 = __bfloat1622float2(wp[e >> 1]), g2 = __bfloat1622float2(gp[e >> 1]);
             float a = v[e] * inv * w2.x, b = v[e + 1] * inv * w2.y;
             if (!gate_first) {
-                a *= gate_kind == 0 ? sigmoid_for<bf16>(g2.x) : silu_for<bf16>(g2.x);
-                b *= gate_kind == 0 ? sigmoid_for<bf16>(g2.y) : silu_for<bf16>(g2.y);
+                a *= gate_of(g2.x);
+                b *= gate_of(g2.y);
             }
             const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
             packed[e >> 1] = *reinterpret_cast<const uint32_t*>(&two);
@@ -821,7 +816,7 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ x, int x_stride, c
     if (single && before && taps > 1) before[(size_t)(taps - 2) * channels + c] = Num<T>::to_f(x[(size_t)t * x_stride + c]);
     T* dst = out + (size_t)t * channels + c;
     if (CACHED) dst = c < cache.tail ? out + (size_t)t * cache.tail + c : conv_cache_place(cache, slot, t, c);
-    if (!CACHED || dst) *dst = Num<T>::from_f(plain ? z : silu_for<T>(z));
+    if (!CACHED || dst) *dst = Num<T>::from_f(plain ? z : z / (1.f + expf(-z)));
 }
 
 // The same convolution for long steps: a thread takes 16 bytes of channels and a run of CONV_RUN(TAPS) consecutive tokens, asks for
@@ -906,7 +901,7 @@ causal_conv_run_kernel(const T* __restrict__ x, int x_stride, const float* __res
 #pragma unroll
             for (int r = 0; r < TAPS - 1; ++r) z = fmaf(w[v][r], hist[r][v], z);
             z = fmaf(w[v][TAPS - 1], u, z);
-            res[v] = Num<T>::from_f(plain ? z : silu_for<T>(z));
+            res[v] = Num<T>::from_f(plain ? z : z / (1.f + expf(-z)));
 #pragma unroll
             for (int r = 0; r + 1 < TAPS - 1; ++r) hist[r][v] = hist[r + 1][v];
             if (TAPS > 1) hist[H - 1][v] = u;

@@ -71,3 +71,24 @@ def test_stabilized_gates_do_not_depend_on_the_cut(pieces):
         results.append((state, *trio))
     for whole, cut in zip(*results):
         assert torch.equal(whole, cut)
+
+
+def test_gates_far_below_zero():
+    """sigmoid and silu as float32 forms them, down to where e^-z overflows (z = -88.7): nothing becomes zero before that."""
+    from qwenforge_b200 import ops
+    n, c, taps = 64, 64, 4
+    z = torch.linspace(-88.5, -60, n, device=DEV).bfloat16()[:, None].expand(n, c).contiguous()
+    want = z.double() * torch.sigmoid(z.double())
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    weight = torch.zeros(c, taps, device=DEV)
+    weight[:, -1] = 1.0                                        # only the newest input counts
+    for single in (False, True):   # one sequence of n tokens, n sequences of one token
+        cu, seqs = (list(range(n + 1)), list(range(n))) if single else ([0, n], [0] * n)
+        state, got = torch.zeros(n, (taps - 1) * c, device=DEV), torch.empty(n, c, dtype=torch.bfloat16, device=DEV)
+        ops.causal_conv_silu(z, weight, None, ints(cu), ints(seqs), ints(list(range(n))[:len(cu) - 1]), state, 0, got, single=single)
+        assert float(((got.double() - want) / want).abs().max()) <= 2 ** -8
+    ones, out = torch.ones(n, c, device=DEV), torch.empty(n, c, dtype=torch.bfloat16, device=DEV)
+    for gate, size in (("silu", want), ("sigmoid", torch.sigmoid(z.double()))):
+        ops.gated_group_norm(ones, z, torch.ones(c, dtype=torch.bfloat16, device=DEV), 0.0, out, 1, 1, gate, False)
+        # (a sigmoid below 2^-126 has fewer bits: 2^-149 is its unit, and a bfloat16 below 2^-126 has 2^-133)
+        assert float(((out.double() - size).abs() / (size.abs() * 2 ** -7 + 2.0 ** -133)).max()) <= 1
