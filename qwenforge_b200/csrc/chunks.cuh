@@ -2,23 +2,59 @@
 #pragma once
 #include "mma.cuh"
 
-// x = hi + mid + lo, each a bfloat16 number (the upper half of a float32): cut off, subtract (exactly), twice.
+// x = hi + mid + lo, each a bfloat16 number: round to the nearest, subtract (exactly), twice; the last remainder is one as it stands. (Cut
+// off instead of rounded, the remainders are up to twice as large and all of one sign, and what a product of two such sums
+// leaves out adds up.)
 struct Thirds {
     uint32_t hi, mid, lo;     // two neighbouring numbers each, the first in the lower half
 };
+__device__ __forceinline__ float lower_bf16(uint32_t pair) { return __uint_as_float(pair << 16); }
+__device__ __forceinline__ float upper_bf16(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
 __device__ __forceinline__ Thirds thirds(float x0, float x1) {
     Thirds r;
-    uint32_t a = __float_as_uint(x0), b = __float_as_uint(x1);
-    r.hi = __byte_perm(a, b, 0x7632);
-    float s0 = x0 - __uint_as_float(a & 0xffff0000u), s1 = x1 - __uint_as_float(b & 0xffff0000u);
-    a = __float_as_uint(s0), b = __float_as_uint(s1);
-    r.mid = __byte_perm(a, b, 0x7632);
-    s0 -= __uint_as_float(a & 0xffff0000u), s1 -= __uint_as_float(b & 0xffff0000u);
+    r.hi = pack_bf16(x0, x1);
+    float s0 = x0 - lower_bf16(r.hi), s1 = x1 - upper_bf16(r.hi);
+    r.mid = pack_bf16(s0, s1);
+    s0 -= lower_bf16(r.mid), s1 -= upper_bf16(r.mid);
     r.lo = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);
     return r;
 }
-__device__ __forceinline__ float lower_bf16(uint32_t pair) { return __uint_as_float(pair << 16); }
-__device__ __forceinline__ float upper_bf16(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
+
+// A product of many decays with what its roundings left out beside it (the remainder of a product of two float32 is one itself): the
+// scan rounds a state once a token, so a chunk's weights must not bring as many roundings of their own on top of its sums'.
+struct Running {
+    float value, rest;
+    __device__ __forceinline__ void times(float w) {
+        const float p = value * w, left = fmaf(value, w, -p);
+        rest = fmaf(rest, w, left), value = p;
+    }
+    __device__ __forceinline__ void times(const Running& w) {
+        const float p = value * w.value, left = fmaf(value, w.value, -p);
+        rest = fmaf(value, w.rest, fmaf(rest, w.value, left)), value = p;
+    }
+    __device__ __forceinline__ float of(float x) const { return fmaf(x, value, x * rest); }   // x times the product, rounded once
+};
+
+// D = A[16x16] B[16x8], the first product of a sum of its own. The tensor cores cut a sum off behind its 24th bit, towards zero, with every
+// product that is added to it. So the recurrences' sums over tokens and state rows are not left to them: the products of 16
+// tokens or rows (least parts first) make a sum of their own, and that is added to the running one by a float32 addition, which rounds.
+struct MmaFirst {
+    __device__ __forceinline__ void operator()(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) const {
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+    }
+};
+struct MmaNext {
+    __device__ __forceinline__ void operator()(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) const { mma_bf16_16816(d, a, b0, b1); }
+};
+template <int N> __device__ __forceinline__ void add_sums(float (*to)[4], const float (&sum)[N][4]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) to[i][e] += sum[i][e];
+}
 
 // Byte offset of 16-byte piece `piece` of row `row` in a tile of WIDTH bfloat16 columns, pieces permuted so that eight
 // neighbouring rows read at one piece lie in eight different bank groups.

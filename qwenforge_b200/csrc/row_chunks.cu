@@ -13,7 +13,7 @@
 // quarters W(j, i) is (decays of i's quarter up to i) x (decays of the whole quarters between) x (decays behind j in its quarter),
 // put on q, q and k; within a quarter the products run along with j. Each factor is a product of decays, at most 1: nothing overflows
 // or is divided. Every float32 operand of a product on the tensor cores is the exact sum of three bfloat16 numbers; of
-// the nine products of two of them the six largest are taken (what is left out is below 2^-24 of the product).
+// the nine products of two of them the six largest are taken (what is left out is below 2^-24 of the product, of either sign).
 // What bounds it: the scan is a chain of one update per token (0.18 microseconds each); here the chain is one step per 64 tokens, the
 // rest products and the quarters' own pairs. Measured, 16 heads of 64 x 128, 2,048 + 1,031 tokens: 342 -> 139
 // microseconds (parts 42, chain 13, outputs 74); 7 heads: 305 -> 66.
@@ -54,7 +54,7 @@ row_parts_kernel(const RowChunkArgs a) {
     float* w_s = reinterpret_cast<float*>(kw_s + 3 * RC_PLANE);           // [64][RC_LD]
     bf16* k_s = reinterpret_cast<bf16*>(w_s + RC_CHUNK * RC_LD);          // [64][RC_LH]
     unsigned char* v_s = reinterpret_cast<unsigned char*>(k_s + RC_CHUNK * RC_LH);   // [vdim / 64][64][64]
-    __shared__ float total_s[2][RC_D];
+    __shared__ Running total_s[2][RC_D];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, head = blockIdx.y, seq = blockIdx.z;
     const int t0 = a.cu_q[seq] + blockIdx.x * RC_CHUNK, n_here = min(RC_CHUNK, a.cu_q[seq + 1] - t0);
     if (n_here <= 0) return;
@@ -90,48 +90,59 @@ row_parts_kernel(const RowChunkArgs a) {
         }
     }
     {
-        float total = 1.f;
-        for (int i = 0; i < RC_CHUNK / 2; ++i) total *= w_s[(half * (RC_CHUNK / 2) + i) * RC_LD + d];
+        Running total{1.f, 0.f};
+        for (int i = 0; i < RC_CHUNK / 2; ++i) total.times(w_s[(half * (RC_CHUNK / 2) + i) * RC_LD + d]);
         total_s[half][d] = total;
     }
     cp_async_wait<0>();
     __syncthreads();
-    if (half == 0) a.whole[record * RC_D + d] = total_s[0][d] * total_s[1][d];
-    float behind = half == 0 ? total_s[1][d] : 1.f;
+    Running behind{1.f, 0.f};
+    if (half == 0) {
+        Running all = total_s[0][d];
+        behind = total_s[1][d];
+        all.times(behind);
+        a.whole[record * RC_D + d] = all.value + all.rest;
+    }
 #pragma unroll 4
     for (int i = RC_CHUNK / 2 - 1; i >= 0; --i) {
         const int row = half * (RC_CHUNK / 2) + i;
-        const Thirds x = thirds(__bfloat162float(k_s[row * RC_LH + d]) * behind, 0.f);
+        const Thirds x = thirds(behind.of(__bfloat162float(k_s[row * RC_LH + d])), 0.f);
         unsigned char* at = kw_s + tile_at<RC_D>(row, d >> 3) + (d & 7) * 2;
         *reinterpret_cast<unsigned short*>(at) = (unsigned short)x.hi;
         *reinterpret_cast<unsigned short*>(at + RC_PLANE) = (unsigned short)x.mid;
         *reinterpret_cast<unsigned short*>(at + 2 * RC_PLANE) = (unsigned short)x.lo;
-        behind *= w_s[row * RC_LD + d];
+        behind.times(w_s[row * RC_LD + d]);
     }
     __syncthreads();
     const int g = lane >> 2, t2 = (lane & 3) * 2;
     for (int v0 = warp * 16; v0 < a.vdim; v0 += 64) {
         const unsigned char* vt = v_s + (v0 / RC_VT) * RC_CHUNK * RC_VT * 2;
         const int piece = (v0 % RC_VT) / 8;
-        float acc[RC_D / 8][4];
+        float acc[RC_D / 8][4], low[RC_D / 8][4];   // (low: the products of the lesser parts)
 #pragma unroll
         for (int nt = 0; nt < RC_D / 8; ++nt)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[nt][e] = 0.f;
+            for (int e = 0; e < 4; ++e) acc[nt][e] = low[nt][e] = 0.f;
 #pragma unroll
         for (int kk = 0; kk < RC_CHUNK / 16; ++kk) {
             uint32_t x[4];
             ldmatrix_x4_trans(x, vt + tile_at<RC_VT>(kk * 16 + (lane & 7) + ((lane >> 4) << 3), piece + ((lane >> 3) & 1)));
-#pragma unroll
-            for (int part = 2; part >= 0; --part)
+            float sum[RC_D / 8][4];
+            auto part = [&](auto mma, float (&to)[RC_D / 8][4], int which) {
 #pragma unroll
                 for (int np = 0; np < RC_D / 16; ++np) {
                     uint32_t b[4];
-                    ldmatrix_x4_trans(b, kw_s + part * RC_PLANE + tile_at<RC_D>(kk * 16 + (lane & 15), np * 2 + (lane >> 4)));
-                    mma_bf16_16816(acc[2 * np], x, b[0], b[1]);
-                    mma_bf16_16816(acc[2 * np + 1], x, b[2], b[3]);
+                    ldmatrix_x4_trans(b, kw_s + which * RC_PLANE + tile_at<RC_D>(kk * 16 + (lane & 15), np * 2 + (lane >> 4)));
+                    mma(to[2 * np], x, b[0], b[1]);
+                    mma(to[2 * np + 1], x, b[2], b[3]);
                 }
+            };
+            part(MmaNext{}, low, 2);
+            part(MmaNext{}, low, 1);
+            part(MmaFirst{}, sum, 0);
+            add_sums(acc, sum);
         }
+        add_sums(acc, low);
         float* rec = a.records + record * RC_D * a.vdim + (size_t)(v0 + g) * RC_D + t2;
 #pragma unroll
         for (int nt = 0; nt < RC_D / 8; ++nt) {
@@ -323,9 +334,9 @@ row_outputs_kernel(const RowChunkArgs a) {
     __syncthreads();
 
     const int g = lane >> 2, t2 = (lane & 3) * 2;
-    // The tensor cores cut a sum off behind its 24th bit with every product that is added, so the products of the leading parts and
-    // the others are summed apart: the latter, 2^8 times smaller, lose nothing that counts (all in one sum: an error of 1.0e-6
-    // of the outputs on 1,031 tokens against 64 bits; 2.5e-7 so; token by token 1.6e-7).
+    // The products of the lesser parts, 2^8 times smaller, are summed apart; those of the leading parts 16 rows or tokens at a time
+    // (MmaFirst). Errors against 64 bits, outputs / states, 2,048 tokens of 7 heads of 64 x 128, decays sigmoid(z)^(1/16): 1.20e-7 /
+    // 6.0e-8, token by token 1.45e-7 / 1.14e-7 (the leading parts' sums left to the tensor cores: 2.5e-7 / 1.8e-7).
     float acc[RC_VT / 8][4], low[RC_VT / 8][4];
 #pragma unroll
     for (int nt = 0; nt < RC_VT / 8; ++nt)
@@ -346,8 +357,11 @@ row_outputs_kernel(const RowChunkArgs a) {
         for (int r = 0; r < 4; ++r) hi[r] = x[r].hi, mid[r] = x[r].mid, lo[r] = x[r].lo;
 #pragma unroll
         for (int p = 0; p < 3; ++p) ldmatrix_x4(b[p], base + p * plane + at);
-        mma_bf16_16816(s0, hi, b[0][0], b[0][1]);
-        mma_bf16_16816(s1, hi, b[0][2], b[0][3]);
+        float sum[2][4];
+        MmaFirst{}(sum[0], hi, b[0][0], b[0][1]);
+        MmaFirst{}(sum[1], hi, b[0][2], b[0][3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s0[e] += sum[0][e], s1[e] += sum[1][e];
         mma_bf16_16816(l0, lo, b[0][0], b[0][1]);
         mma_bf16_16816(l1, lo, b[0][2], b[0][3]);
         mma_bf16_16816(l0, mid, b[1][0], b[1][1]);
@@ -369,14 +383,20 @@ row_outputs_kernel(const RowChunkArgs a) {
         uint32_t b[RC_VT / 16][4];
 #pragma unroll
         for (int vp = 0; vp < RC_VT / 16; ++vp) ldmatrix_x4_trans(b[vp], v_s + tile_at<RC_VT>(c * 16 + (lane & 15), vp * 2 + (lane >> 4)));
+        float sum[RC_VT / 8][4];
 #pragma unroll
-        for (int p = 2; p >= 0; --p)
+        for (int vp = 0; vp < RC_VT / 16; ++vp) {
+            MmaFirst{}(sum[2 * vp], part[0], b[vp][0], b[vp][1]);
+            MmaFirst{}(sum[2 * vp + 1], part[0], b[vp][2], b[vp][3]);
+        }
+#pragma unroll
+        for (int p = 2; p >= 1; --p)
 #pragma unroll
             for (int vp = 0; vp < RC_VT / 16; ++vp) {
-                auto& sum = p == 0 ? acc : low;
-                mma_bf16_16816(sum[2 * vp], part[p], b[vp][0], b[vp][1]);
-                mma_bf16_16816(sum[2 * vp + 1], part[p], b[vp][2], b[vp][3]);
+                mma_bf16_16816(low[2 * vp], part[p], b[vp][0], b[vp][1]);
+                mma_bf16_16816(low[2 * vp + 1], part[p], b[vp][2], b[vp][3]);
             }
+        add_sums(acc, sum);
     };
     // ---- this quarter's own pairs
     {
