@@ -109,15 +109,19 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     // every SPLIT-th of them, tile i the first turns[i] of those.
     const int pos_first = tok_pos[q_begin + row0[0]];   // position of the first tile's first row; positions run on from there
     const int p_first = (window > 0 ? max(0, pos_first - window + 1) : 0) / QF_PAGE;
-    int turns[2], p_end[2];
+    int turns[2], p_lo[2], p_end[2];   // (p_lo, p_end: the pages that any row of the tile sees)
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const int last = pos_first + row0[i] - row0[0] + n_rows[i] - 1;
+        const int pos = pos_first + row0[i] - row0[0], last = pos + n_rows[i] - 1;
+        p_lo[i] = (window > 0 ? max(0, pos - window + 1) : 0) / QF_PAGE;
         p_end[i] = n_rows[i] > 0 ? last / QF_PAGE + 1 : 0;
         const int blocks = p_end[i] > p_first ? (p_end[i] - p_first + 1) / 2 : 0;
         turns[i] = blocks > rank ? (blocks - rank + SPLIT - 1) / SPLIT : 0;
     }
     const int all_turns = max(turns[0], turns[1]), p_last = max(p_end[0], p_end[1]) - 1;
+    // What lies in a page that none of a tile's rows sees is not multiplied by their weights of zero (0 times infinity is not 0): the
+    // second page behind the last, or behind the other tile's window. A second tile's first turn may have no page left.
+    const bool first_empty = rank == 0 && p_lo[1] >= p_first + 2;
 
     if (threadIdx.x == 0) {
         mbar_init(&bar_q, 1);
@@ -168,7 +172,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             int page[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                page[h] = table_row[min(first + h, p_last)];   // (beyond the last page: masked keys, some finite numbers)
+                page[h] = table_row[min(first + h, p_last)];   // (beyond the last page: masked keys, values that nothing reads)
                 if (page[h] < 0) {  // a page the sequence does not hold: reported; some held memory is read instead
                     if (leader) atomicOr(err, QF_ERR_NO_PAGE);
                     page[h] = 0;
@@ -240,10 +244,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 tc_fence_after();
                 if (leader) {   // values [128 keys][D] as they lie (MN-major), 16 keys are two groups of 8 rows (2048 bytes)
                     const uint64_t dv = desc_v + (uint64_t)((j & 1) * (KV_BYTES >> 4));
+                    const int first = p_first + 2 * (rank + j * SPLIT);
+                    const int k0 = first >= p_lo[i] ? 0 : first + 1 >= p_lo[i] ? 4 : 8, k1 = first + 1 < p_end[i] ? 8 : 4;
 #pragma unroll
                     for (int kk = 0; kk < TA_BK / 16; ++kk)
-                        umma_bf16_tmem_a(tmem + O_COL + 128 * i, tmem + 128 * i + 8 * kk, dv + (uint64_t)(kk * (2048 >> 4)), idesc_pv,
-                                         (j > 0 || kk > 0) ? 1u : 0u);
+                        if (kk >= k0 && kk < k1)
+                            umma_bf16_tmem_a(tmem + O_COL + 128 * i, tmem + 128 * i + 8 * kk, dv + (uint64_t)(kk * (2048 >> 4)), idesc_pv,
+                                             (j > 0 || kk > k0) ? 1u : 0u);
                     umma_commit(&bar_pv[i]);
                     if (i == 1 || j >= turns[1]) umma_commit(&bar_v_free[j & 1]);
                 }
@@ -286,6 +293,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             bool moved = false;
             if (j == 0) {
                 m_ref = m_true;  // nothing to rescale yet: the first products overwrite O
+                if (t && first_empty) {   // (no products in this turn: O begins as zeros)
+                    uint32_t zeros[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) zeros[i] = 0u;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < D; c0 += 16) tmem_store_16(o_at + c0, zeros);
+                }
             } else if (m_true - m_ref > 8.0f) {
                 moved = true;
                 f_o = fast_exp2(m_ref - m_true);

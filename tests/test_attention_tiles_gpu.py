@@ -52,6 +52,40 @@ def test_against_float64(lens, before, heads, kv_heads, dim, window, with_sinks)
             assert float((got - want).norm() / want.norm()) < 2 ** -8
 
 
+@pytest.mark.parametrize("n,before,heads,kv_heads,dim,window", [(300, 0, 5, 5, 64, 0), (300, 0, 3, 1, 128, 0), (700, 130, 6, 2, 64, 0), (64, 3000, 2, 2, 128, 0),
+                                                               (400, 700, 4, 4, 64, 150), (400, 690, 4, 4, 128, 200), (130, 4000, 5, 5, 64, 3000), (1153, 0, 16, 2, 64, 0)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_values_of_pages_that_a_tile_does_not_see(n, before, heads, kv_heads, dim, window, bad):
+    """A value that is not finite reaches no tile of 128 rows none of whose rows sees its page."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(n + before)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pages = -(-(n + before) // 64)
+    storage = torch.randn(pages, 2, kv_heads, 64, dim, generator=g, device=DEV).bfloat16()
+    q, err = torch.randn(n, heads * dim, generator=g, device=DEV).bfloat16(), ints([0])
+    site = ops.KvSiteArgs(storage, ints([list(range(pages))]), kv_heads, dim)
+
+    def run():
+        out = torch.empty_like(q)
+        ops.attention_prefill_tc(q, out, ints([0, n]), ints(list(range(before, before + n))), ints([0]), site, heads, 1, n, dim ** -0.5, window, err,
+                                 max_kv_len=n + before)
+        return out
+    want = run()
+    seen = []
+    for t0 in range(0, n, 128):
+        first, last = before + t0, before + min(t0 + 128, n) - 1
+        seen.append(((max(0, first - window + 1) if window else 0) // 64, last // 64))
+    for page in range(max(0, pages - 12), pages):
+        held = storage[page, 1].clone()
+        storage[page, 1] = bad
+        got = run()
+        storage[page, 1] = held
+        for i, (lo, hi) in enumerate(seen):
+            if not lo <= page <= hi:
+                assert torch.equal(got[128 * i:128 * i + 128], want[128 * i:128 * i + 128]), (page, i)
+    assert int(err) == 0
+
+
 def test_which_kernel_a_step_takes():
     from qwenforge_b200 import ops
     from qwenforge_b200.parts.attention import prefill_attention
