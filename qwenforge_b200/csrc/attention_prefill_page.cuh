@@ -63,7 +63,7 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     // barriers, its tensor memory) runs under the tail of the kernel before, which wrote the queries and the new keys
     // and values; they are read, and the output written, only after the wait. The kernel after it may start when every block
     // has its tensor memory (or has ended).
-    __shared__ __align__(8) uint64_t bar_q, bar_kv[2], bar_s, bar_sfree, bar_pv, bar_p;
+    __shared__ __align__(8) uint64_t bar_q, bar_kv[2], bar_s, bar_sfree, bar_pv, bar_p, bar_end;
     __shared__ uint32_t tmem_base_s;
 
     // Which (tile, head, sequence) this block serves (with SPLIT: this pair of blocks). Tiles further down a prompt walk
@@ -98,6 +98,7 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 
     if (t == 0) {
         mbar_init(&bar_q, 1);
+        mbar_init(&bar_end, 1);
         mbar_init(&bar_kv[0], 1);
         mbar_init(&bar_kv[1], 1);
         mbar_init(&bar_s, 1);
@@ -126,8 +127,10 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             // ---- the issuing warp: copies and products. All lanes run the loop (uniform values); one lane issues.
             const bool leader = elect_one();
             const int* table_row = site.table + (long long)slot * site.table_stride;
+            int fetched = 0;
             auto fetch_page = [&](int j) {  // keys and values of the j-th page of the run into stage j & 1
                 const int stage = j & 1;
+                ++fetched;
                 int page = table_row[p_begin + j * STRIDE];
                 if (page < 0) {  // a page the sequence does not hold: reported; some held memory is read instead
                     if (leader) atomicOr(err, QF_ERR_NO_PAGE);
@@ -207,6 +210,13 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     else fetch_page(j + 2);
                 }
             }
+            // The block ends, also after a wait that ran out, only when nothing is on its way to its shared memory and no product of its
+            // is at work (long so otherwise).
+            if (n_tiles > 0) timed_out |= !wait_all(&bar_q, 0);
+            for (int j = max(fetched - 2, 0); j < fetched; ++j) timed_out |= !wait_all(&bar_kv[j & 1], (j >> 1) & 1);
+            if (leader) umma_commit(&bar_end);
+            __syncwarp();
+            timed_out |= !wait_all(&bar_end, 0);
         }
     } else {
         // ---- the row threads

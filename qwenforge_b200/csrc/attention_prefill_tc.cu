@@ -74,7 +74,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     float* merge_s = reinterpret_cast<float*>(smem);
     float* merge_ml = merge_s + SPLIT * PER * DS * TA_BM;
     const int rank = (int)(blockIdx.x % SPLIT);
-    __shared__ __align__(8) uint64_t bar_q, bar_k[2], bar_v[2], bar_k_free[2], bar_v_free[2], bar_s[2], bar_p[2], bar_pv[2];
+    __shared__ __align__(8) uint64_t bar_q, bar_k[2], bar_v[2], bar_k_free[2], bar_v_free[2], bar_s[2], bar_p[2], bar_pv[2], bar_end;
     __shared__ uint32_t tmem_base_s;
 
     // Which pair of tiles this block serves (PER 1: which single tile): those further down a prompt walk more keys, so they come first.
@@ -125,6 +125,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 
     if (threadIdx.x == 0) {
         mbar_init(&bar_q, 1);
+        mbar_init(&bar_end, 1);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_k[i], 1);
@@ -166,6 +167,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                         tma_load_2d(q_s + i * Q_BYTES + cb * Q_BLOCK, &q_map, head[i] * D + cb * 64, q_begin + row0[i], &bar_q);
         }
         __syncwarp();
+        int keys = 0, values = 0;   // turns whose copies have been asked for
         for (int j = 0; j < all_turns; ++j) {
             const int stage = j & 1, first = p_first + 2 * (rank + j * SPLIT);
             const uint32_t freed = ((j >> 1) + 1) & 1;   // the turn before last has been read
@@ -184,6 +186,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             }
             // row of the cache seen as one matrix [pages * planes * kv_heads * 64][D]; with one plane per page the values
             // are the keys themselves (the same rows fetched into the values' stage)
+            ++keys;
             if (leader) {
                 mbar_expect_tx(&bar_k[stage], KV_BYTES);
 #pragma unroll
@@ -198,6 +201,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 timed_out = true;
                 break;
             }
+            ++values;
             if (leader) {
                 mbar_expect_tx(&bar_v[stage], KV_BYTES);
 #pragma unroll
@@ -209,6 +213,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             }
             __syncwarp();
         }
+        // The block ends, also after a wait that ran out, only when nothing is on its way to its shared memory (long arrived otherwise).
+        if (all_turns > 0) timed_out |= !wait_all(&bar_q, 0);
+        for (int j = max(keys - 2, 0); j < keys; ++j) timed_out |= !wait_all(&bar_k[j & 1], (j >> 1) & 1);
+        for (int j = max(values - 2, 0); j < values; ++j) timed_out |= !wait_all(&bar_v[j & 1], (j >> 1) & 1);
     } else if (warp == PRODUCTS) {
         // ---- the products
         const bool leader = elect_one();
@@ -258,6 +266,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 if (j + 1 < turns[i] && (!wait_all(&bar_pv[i], j & 1) || !issue_s(i, j + 1))) timed_out = true;
             }
         }
+        if (leader) umma_commit(&bar_end);   // nor while a product of its is at work
+        __syncwarp();
+        timed_out |= !wait_all(&bar_end, 0);
     } else {
         // ---- the row threads
         const int my_turns = t ? turns[1] : turns[0];
