@@ -274,6 +274,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         const int my_turns = t ? turns[1] : turns[0];
         const int pos0 = pos_first + my_row0 - row0[0], row_pos = pos0 + row, row_lo = window > 0 ? max(0, row_pos - window + 1) : 0;
         const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16), s_at = lanes + 128 * t, o_at = lanes + O_COL + 128 * t;
+        const float folded = scale_log2 > 0.f ? scale_log2 : 1.f;
         for (int j = 0; j < my_turns; ++j) {
             if (!wait_all(&bar_s[t], j & 1)) {   // (the product of the turn before is done too: S was issued after it)
                 timed_out = true;
@@ -282,6 +283,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             tc_fence_after();
             float s[TA_BK];
             tmem_load_row_128(s_at, s);
+            if (!(scale_log2 > 0.f)) {   // below, the scale is folded into the exponent, behind the maximum and the mask: above zero only
+#pragma unroll
+                for (int i = 0; i < TA_BK; ++i) s[i] *= scale_log2;
+            }
             const int key0 = (p_first + 2 * (rank + j * SPLIT)) * QF_PAGE;
             // a block of keys that every row of the tile sees whole needs no mask
             const bool full = key0 + TA_BK - 1 <= pos0 && key0 >= (window > 0 ? max(0, pos0 + TA_BM - 1 - window + 1) : 0);
@@ -299,7 +304,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 #pragma unroll
             for (int c = 0; c < 4; ++c) mx[c] = fmaxf(mx[c], s[TA_BK - 4 + c]);
             // (the scores stay unscaled; the scale is folded into the exponent)
-            const float m_true = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2);
+            const float m_true = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * folded);
             float f_o = 1.0f;
             bool moved = false;
             if (j == 0) {
@@ -328,7 +333,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 }
             }
             // two neighbouring weights an instruction where the pipes allow it: s * scale - reference, and the sums
-            const float2 by = make_float2(scale_log2, scale_log2), less = make_float2(-m_ref, -m_ref);
+            const float2 by = make_float2(folded, folded), less = make_float2(-m_ref, -m_ref);
             float2 part[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
             for (int h = 0; h < 2; ++h) {   // half of the weights at a time: the first are stored while the others are formed

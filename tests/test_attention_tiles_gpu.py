@@ -86,6 +86,25 @@ def test_values_of_pages_that_a_tile_does_not_see(n, before, heads, kv_heads, di
     assert int(err) == 0
 
 
+@pytest.mark.parametrize("n,heads,kv_heads,dim", [(300, 4, 2, 128), (130, 3, 3, 64), (1153, 16, 2, 64)])
+@pytest.mark.parametrize("scale", [0.0, -0.05, 0.05])
+def test_any_scale(n, heads, kv_heads, dim, scale):
+    """A scale of zero weighs all keys alike, one below zero prefers the unlike ones."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(n)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pages = -(-n // 64)
+    storage = torch.randn(pages, 2, kv_heads, 64, dim, generator=g, device=DEV).bfloat16()
+    q, err = torch.randn(n, heads * dim, generator=g, device=DEV).bfloat16(), ints([0])
+    out, site = torch.empty_like(q), ops.KvSiteArgs(storage, ints([list(range(pages))]), kv_heads, dim)
+    ops.attention_prefill_tc(q, out, ints([0, n]), ints(list(range(n))), ints([0]), site, heads, 1, n, scale, 0, err, max_kv_len=n)
+    kv = storage.double().permute(1, 2, 0, 3, 4).reshape(2, kv_heads, -1, dim)[:, :, :n].repeat_interleave(heads // kv_heads, 1)
+    scores = torch.einsum("ihd,hjd->hij", q.view(n, heads, dim).double(), kv[0]) * scale
+    want = torch.softmax(scores.masked_fill(torch.ones(n, n, dtype=torch.bool, device=DEV).triu(1), float("-inf")), -1) @ kv[1]
+    got = out.view(n, heads, dim).transpose(0, 1).double()
+    assert int(err) == 0 and float((got - want).norm() / want.norm()) < 2 ** -8   # (weights and outputs rounded to bfloat16)
+
+
 def test_which_kernel_a_step_takes():
     from qwenforge_b200 import ops
     from qwenforge_b200.parts.attention import prefill_attention
