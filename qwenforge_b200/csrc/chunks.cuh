@@ -72,5 +72,13 @@ __device__ __forceinline__ void fetch_tile(unsigned char* dst, const bf16* src, 
         cp_async_16(dst + tile_at<WIDTH>(row, piece), there ? src + (size_t)row * stride + piece * 8 : src, there);
     }
 }
-// The first record of a sequence: sequence s owns records cu_q[s] / CHUNK + s onwards, as many as its chunks at most.
-template <int CHUNK> __device__ __forceinline__ long long first_record(const int* cu_q, int seq) { return cu_q[seq] / CHUNK + seq; }
+// A call works through its chunks in portions of the same `each` chunks of every sequence, so that what it keeps per chunk has a bound:
+// portion [chunk0, chunk0 + each). each == 0: all chunks at once.
+struct Portion {
+    int chunk0, each;
+    float* carry;     // each > 0: a state per sequence [heads][D][vdim], [heads][D] between the portions of those that have no slot
+};
+// The record of a sequence's chunk, all at once: sequence s owns records cu_q[s] / CHUNK + s onwards, as many as its chunks at most.
+template <int CHUNK> __device__ __forceinline__ long long record_of(const Portion& p, const int* cu_q, int seq, int chunk) {
+    return p.each > 0 ? (long long)seq * p.each + chunk - p.chunk0 : (long long)cu_q[seq] / CHUNK + seq + chunk;
+}

@@ -40,6 +40,7 @@ struct RowChunkArgs {
     float q_scale;
     float *records, *whole, *made;   // [record][heads][vdim][64], [record][heads][64], [T][heads * 64] (kind 0: not written)
     float* y;
+    Portion portion;
 };
 
 __device__ __forceinline__ float row_log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
@@ -56,9 +57,9 @@ row_parts_kernel(const RowChunkArgs a) {
     unsigned char* v_s = reinterpret_cast<unsigned char*>(k_s + RC_CHUNK * RC_LH);   // [vdim / 64][64][64]
     __shared__ Running total_s[2][RC_D];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, head = blockIdx.y, seq = blockIdx.z;
-    const int t0 = a.cu_q[seq] + blockIdx.x * RC_CHUNK, n_here = min(RC_CHUNK, a.cu_q[seq + 1] - t0);
+    const int chunk = a.portion.chunk0 + (int)blockIdx.x, t0 = a.cu_q[seq] + chunk * RC_CHUNK, n_here = min(RC_CHUNK, a.cu_q[seq + 1] - t0);
     if (n_here <= 0) return;
-    const long long record = (first_record<RC_CHUNK>(a.cu_q, seq) + blockIdx.x) * a.n_heads + head;
+    const long long record = record_of<RC_CHUNK>(a.portion, a.cu_q, seq, chunk) * a.n_heads + head;
     for (int i = threadIdx.x; i < RC_CHUNK * (RC_D / 8); i += 128) {
         const int row = i / 8, c = (i % 8) * 8;
         const bf16* src = a.k + (size_t)t0 * a.k_stride + head * RC_D + c;
@@ -161,17 +162,21 @@ row_chain_kernel(const RowChunkArgs a) {
     grid_chain_entry();
     constexpr int AHEAD = 8;
     const int lane = threadIdx.x & 31, head = blockIdx.y, seq = blockIdx.z;
-    const int len = a.cu_q[seq + 1] - a.cu_q[seq], slot = a.slots[seq], n_chunks = (len + RC_CHUNK - 1) / RC_CHUNK;
+    const int len = a.cu_q[seq + 1] - a.cu_q[seq], slot = a.slots[seq], chunk0 = a.portion.chunk0, left = (len + RC_CHUNK - 1) / RC_CHUNK - chunk0;
+    const int n_chunks = a.portion.each > 0 ? min(left, a.portion.each) : left;
     const int item = (int)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (n_chunks <= 0 || item >= a.vdim / 8 * (RC_D / 16)) return;
-    const long long first = first_record<RC_CHUNK>(a.cu_q, seq) * a.n_heads + head, pitch = (long long)a.n_heads * RC_D * a.vdim;
+    const long long first = record_of<RC_CHUNK>(a.portion, a.cu_q, seq, chunk0) * a.n_heads + head, pitch = (long long)a.n_heads * RC_D * a.vdim;
     const int col = item / (RC_D / 16) * 8 + (lane >> 2), row = item % (RC_D / 16) * 16 + (lane & 3) * 4;
     const float* whole = a.whole + first * RC_D + row;
     float* at = a.records + first * RC_D * a.vdim + (size_t)col * RC_D + row;
-    float* kept = slot >= 0 ? a.state + slot * a.slot_stride + a.s_offset + ((long long)head * RC_D + row) * a.vdim + col : nullptr;
+    // the sequence's state, or what stands for it between portions (zeros before the first)
+    float* base = slot >= 0 ? a.state + slot * a.slot_stride + a.s_offset : a.portion.carry ? a.portion.carry + (long long)seq * a.n_heads * RC_D * a.vdim : nullptr;
+    float* kept = base ? base + ((long long)head * RC_D + row) * a.vdim + col : nullptr;
+    const bool fresh = !kept || (slot < 0 && chunk0 == 0);
     float s[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) s[e] = kept ? kept[(size_t)e * a.vdim] : 0.f;
+    for (int e = 0; e < 4; ++e) s[e] = fresh ? 0.f : kept[(size_t)e * a.vdim];
     float4 part[AHEAD], w[AHEAD];
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u)
@@ -217,9 +222,9 @@ row_outputs_kernel(const RowChunkArgs a) {
     __shared__ float pair_s[4][RC_SUB][RC_SUB + 1], all_s[4][RC_D];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seq = blockIdx.z;
     const int v_tiles = a.vdim / RC_VT, head = blockIdx.y / v_tiles, v0 = (blockIdx.y % v_tiles) * RC_VT;
-    const int t0 = a.cu_q[seq] + blockIdx.x * RC_CHUNK, n_here = min(RC_CHUNK, a.cu_q[seq + 1] - t0);
+    const int chunk = a.portion.chunk0 + (int)blockIdx.x, t0 = a.cu_q[seq] + chunk * RC_CHUNK, n_here = min(RC_CHUNK, a.cu_q[seq + 1] - t0);
     if (n_here <= 0) return;
-    const long long record = (first_record<RC_CHUNK>(a.cu_q, seq) + blockIdx.x) * a.n_heads + head;
+    const long long record = record_of<RC_CHUNK>(a.portion, a.cu_q, seq, chunk) * a.n_heads + head;
     const size_t width = (size_t)a.n_heads * RC_D;
     for (int i = threadIdx.x; i < RC_CHUNK * (RC_D / 8); i += 128) {
         const int row = i / 8, c = (i % 8) * 8;
@@ -474,28 +479,37 @@ row_outputs_kernel(const RowChunkArgs a) {
 
 // q, k: bfloat16 [T][heads * 64], v: bfloat16 [T][heads * vdim], rows strided in whole eights and 16-byte aligned; decay: float32
 // [T][heads * 64], 16-byte aligned; kind, decay_bias, inv_tau, bonus as in qf_outer_state_scan_rows; y: float32 [T][heads * vdim].
-// scratch: float32, 16-byte aligned: [n_records][heads][64 * vdim + 64], then (kind not 0) [T][heads * 64]; n_records = n_tokens / 64 + n_seqs.
+// scratch: float32, 16-byte aligned: [n_records][heads][64 * vdim + 64], then (each > 0) [n_seqs][heads][64 * vdim] for what passes from one
+// portion to the next, then (kind not 0) [T][heads * 64]. n_records = n_tokens / 64 + n_seqs with each == 0, else n_seqs * each, and
+// the call goes through `each` chunks of every sequence at a time.
 QF_EXPORT int qf_row_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay,
                             const float* decay_bias, int kind, float inv_tau, const float* bonus, const int* cu_q, const int* slots,
                             int n_seqs, int max_q_len, float* state, long long slot_stride, long long s_offset, int n_heads, int dim,
-                            int vdim, float q_scale, float* scratch, long long n_records, float* y, cudaStream_t stream) {
+                            int vdim, float q_scale, float* scratch, long long n_records, int each, float* y, cudaStream_t stream) {
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
     if (dim != RC_D || vdim <= 0 || vdim % RC_VT || vdim > 512 || n_heads <= 0 || n_seqs > 65535 || (long long)n_heads * (vdim / RC_VT) > 65535 ||
         kind < 0 || kind > 2 || (kind != 0 && !decay_bias) || ((q_stride | k_stride | v_stride) & 7) ||
         (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)decay | (uintptr_t)scratch) & 15))
         return (int)cudaErrorInvalidValue;
-    float* whole = scratch + n_records * n_heads * dim * vdim;
-    const RowChunkArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, decay, decay_bias, bonus, kind, inv_tau,
-                         cu_q, slots, state, slot_stride, s_offset, n_heads, vdim, q_scale, scratch, whole, whole + n_records * n_heads * dim, y};
+    if (each < 0 || (each > 0 && n_records < (long long)n_seqs * each)) return (int)cudaErrorInvalidValue;
+    float *whole = scratch + n_records * n_heads * dim * vdim, *carry = whole + n_records * n_heads * dim;
+    float* made = carry + (each > 0 ? (long long)n_seqs * n_heads * dim * vdim : 0);
+    RowChunkArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, decay, decay_bias, bonus, kind, inv_tau,
+                         cu_q, slots, state, slot_stride, s_offset, n_heads, vdim, q_scale, scratch, whole, made, y, Portion{0, each, each > 0 ? carry : nullptr}};
     const int chunks = (max_q_len + RC_CHUNK - 1) / RC_CHUNK;
     const size_t parts_smem = 3 * RC_PLANE + RC_CHUNK * RC_LD * 4 + RC_CHUNK * RC_LH * 2 + (size_t)RC_CHUNK * vdim * 2;
     const size_t outputs_smem = 3 * RC_PLANE + 2 * RC_CHUNK * RC_LD * 4 + 2 * RC_CHUNK * RC_LH * 2 + RC_CHUNK * RC_VT * 2;
     auto outputs = bonus ? row_outputs_kernel<true> : row_outputs_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(row_parts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)parts_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(outputs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outputs_smem);
-    if (e == cudaSuccess) e = launch_pdl(row_parts_kernel, dim3(chunks, n_heads, n_seqs), dim3(128), parts_smem, stream, a);
-    if (e == cudaSuccess)
-        e = launch_pdl(row_chain_kernel, dim3((vdim / 8 * (RC_D / 16) + 7) / 8, n_heads, n_seqs), dim3(256), 0, stream, a);
-    if (e == cudaSuccess) e = launch_pdl(outputs, dim3(chunks, vdim / RC_VT * n_heads, n_seqs), dim3(128), outputs_smem, stream, a);
+    const int at_once = each > 0 ? min(each, chunks) : chunks;
+    for (int chunk0 = 0; chunk0 < chunks && e == cudaSuccess; chunk0 += at_once) {
+        a.portion.chunk0 = chunk0;
+        const int here = min(at_once, chunks - chunk0);
+        e = launch_pdl(row_parts_kernel, dim3(here, n_heads, n_seqs), dim3(128), parts_smem, stream, a);
+        if (e == cudaSuccess)
+            e = launch_pdl(row_chain_kernel, dim3((vdim / 8 * (RC_D / 16) + 7) / 8, n_heads, n_seqs), dim3(256), 0, stream, a);
+        if (e == cudaSuccess) e = launch_pdl(outputs, dim3(here, vdim / RC_VT * n_heads, n_seqs), dim3(128), outputs_smem, stream, a);
+    }
     return (int)e;
 }

@@ -45,6 +45,7 @@ struct ChunkArgs {
     float q_scale;
     float *records, *n_records, *whole;   // [record][heads][vdim][D], [record][heads][D], [record][heads]
     float *y, *nq;
+    Portion portion;
 };
 
 // A token's decay and take (the arithmetic of `decay_gates_kernel` in recurrent.cu where they come as pre-activations: a launch
@@ -69,7 +70,7 @@ chunk_parts_kernel(const ChunkArgs a) {
     unsigned char* k_s = sc_smem;                              // [128][D]
     unsigned char* v_s = sc_smem + SC_CHUNK * D * 2;           // [128][64]
     __shared__ __align__(16) float weight_s[SC_CHUNK];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunk = blockIdx.x, seq = blockIdx.z;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunk = a.portion.chunk0 + (int)blockIdx.x, seq = blockIdx.z;
     const int v_tiles = a.vdim / SC_VT, head = blockIdx.y / v_tiles, v0 = (blockIdx.y % v_tiles) * SC_VT;
     const int t0 = a.cu_q[seq] + chunk * SC_CHUNK, n_here = min(SC_CHUNK, a.cu_q[seq + 1] - t0);
     if (n_here <= 0) return;
@@ -77,7 +78,7 @@ chunk_parts_kernel(const ChunkArgs a) {
     fetch_tile<SC_CHUNK, SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, blockDim.x);
     fetch_tile<SC_CHUNK, D>(k_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, blockDim.x);
     cp_async_commit();
-    const long long record = (first_record<SC_CHUNK>(a.cu_q, seq) + chunk) * a.n_heads + head;
+    const long long record = record_of<SC_CHUNK>(a.portion, a.cu_q, seq, chunk) * a.n_heads + head;
     if (warp == 0) {
         // What a token adds counts at the chunk's end: its take and the decays behind it. Four neighbouring tokens per lane,
         // the products over the lanes above by shuffles.
@@ -179,18 +180,23 @@ chunk_chain_kernel(const ChunkArgs a) {
     constexpr int AHEAD = 8;
     const int lane = threadIdx.x & 31, head = blockIdx.y, seq = blockIdx.z;
     const int len = a.cu_q[seq + 1] - a.cu_q[seq], slot = a.slots[seq];
-    const int n_chunks = (len + SC_CHUNK - 1) / SC_CHUNK;
+    const int chunk0 = a.portion.chunk0, left = (len + SC_CHUNK - 1) / SC_CHUNK - chunk0;
+    const int n_chunks = a.portion.each > 0 ? min(left, a.portion.each) : left;
     if (n_chunks <= 0) return;
-    const long long first = first_record<SC_CHUNK>(a.cu_q, seq) * a.n_heads + head;
-    float* kept = slot >= 0 ? a.state + slot * a.slot_stride : nullptr;
+    const long long first = record_of<SC_CHUNK>(a.portion, a.cu_q, seq, chunk0) * a.n_heads + head;
+    // the sequence's state, or what stands for it between portions (zeros before the first)
+    const bool held = slot >= 0;
+    float* kept = held ? a.state + slot * a.slot_stride : a.portion.carry ? a.portion.carry + (long long)seq * a.n_heads * D * (a.vdim + 1) : nullptr;
+    const long long s_offset = held ? a.s_offset : 0, n_offset = held ? a.n_offset : (long long)a.n_heads * D * a.vdim;
+    const bool fresh = !kept || (!held && chunk0 == 0);
     const float* whole = a.whole + first;
     const int item = (int)blockIdx.x * 8 + (threadIdx.x >> 5);   // (8 columns of v, 16 rows of S)
     const int items = a.vdim / 8 * (D / 16);
     if (item >= items) {
         if (item != items || a.n_offset < 0) return;   // one warp of the grid carries n
-        float* n_kept = kept ? kept + a.n_offset + (long long)head * D : nullptr;
+        float* n_kept = kept ? kept + n_offset + (long long)head * D : nullptr;
         for (int d = lane; d < D; d += 32) {
-            float n = n_kept ? n_kept[d] : 0.f;
+            float n = fresh ? 0.f : n_kept[d];
             for (int c = 0; c < n_chunks; ++c) {
                 float* at = a.n_records + (first + (long long)c * a.n_heads) * D + d;
                 const float part = *at;
@@ -204,10 +210,10 @@ chunk_chain_kernel(const ChunkArgs a) {
     const int col = item / (D / 16) * 8 + (lane >> 2), row = item % (D / 16) * 16 + (lane & 3) * 4;
     const long long pitch = (long long)a.n_heads * D * a.vdim;
     float* at = a.records + first * D * a.vdim + (size_t)col * D + row;
-    float* s_kept = kept ? kept + a.s_offset + ((long long)head * D + row) * a.vdim + col : nullptr;
+    float* s_kept = kept ? kept + s_offset + ((long long)head * D + row) * a.vdim + col : nullptr;
     float s[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) s[e] = s_kept ? s_kept[(size_t)e * a.vdim] : 0.f;
+    for (int e = 0; e < 4; ++e) s[e] = fresh ? 0.f : s_kept[(size_t)e * a.vdim];
     float4 part[AHEAD];
     float w[AHEAD];
 #pragma unroll
@@ -254,13 +260,13 @@ chunk_outputs_kernel(const ChunkArgs a) {
     unsigned char* s_s = v_s + V_BYTES;            // [3][64][D]: the state before the chunk, transposed, in three parts
     __shared__ __align__(16) float decay_s[SC_CHUNK], upto_s[SC_CHUNK], behind_s[SC_CHUNK], n_s[D];
     __shared__ float inner_s[SUBS][SC_SUB][SC_SUB + 1];   // W of one eighth: row, column
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunk = blockIdx.x, seq = blockIdx.z;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunk = a.portion.chunk0 + (int)blockIdx.x, seq = blockIdx.z;
     const int v_tiles = a.vdim / SC_VT, head = blockIdx.y / v_tiles, v0 = (blockIdx.y % v_tiles) * SC_VT;
     const int t0 = a.cu_q[seq] + chunk * SC_CHUNK, n_here = min(SC_CHUNK, a.cu_q[seq + 1] - t0);
     if (n_here <= 0) return;
     const int group = head / (a.n_heads / a.n_groups);
     const bool with_n = a.n_offset >= 0 && v0 == 0;
-    const long long record = (first_record<SC_CHUNK>(a.cu_q, seq) + chunk) * a.n_heads + head;
+    const long long record = record_of<SC_CHUNK>(a.portion, a.cu_q, seq, chunk) * a.n_heads + head;
 
     fetch_tile<SC_CHUNK, D>(qk_s, a.q + (size_t)t0 * a.q_stride + group * D, a.q_stride, n_here, threadIdx.x, 128);
     cp_async_commit();
@@ -497,33 +503,42 @@ chunk_outputs_kernel(const ChunkArgs a) {
 }
 
 template <int D>
-static int launch_chunks(const ChunkArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
-    const dim3 grid((max_q_len + SC_CHUNK - 1) / SC_CHUNK, a.vdim / SC_VT * a.n_heads, n_seqs);
+static int launch_chunks(ChunkArgs a, int n_seqs, int max_q_len, cudaStream_t stream) {
     constexpr size_t parts_smem = (size_t)SC_CHUNK * D * 2 + SC_CHUNK * SC_VT * 2, outputs_smem = parts_smem + 3 * (size_t)SC_VT * D * 2;
     cudaError_t e = cudaFuncSetAttribute(chunk_parts_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)parts_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_outputs_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outputs_smem);
-    if (e == cudaSuccess) e = launch_pdl(chunk_parts_kernel<D>, grid, dim3(a.n_offset >= 0 ? 160 : 128), parts_smem, stream, a);
-    const int items = a.vdim / 8 * (D / 16) + (a.n_offset >= 0 ? 1 : 0);
-    if (e == cudaSuccess) e = launch_pdl(chunk_chain_kernel<D>, dim3((items + 7) / 8, a.n_heads, n_seqs), dim3(256), 0, stream, a);
-    if (e == cudaSuccess) e = launch_pdl(chunk_outputs_kernel<D>, grid, dim3(128), outputs_smem, stream, a);
+    const int items = a.vdim / 8 * (D / 16) + (a.n_offset >= 0 ? 1 : 0), chunks = (max_q_len + SC_CHUNK - 1) / SC_CHUNK;
+    const int each = a.portion.each > 0 ? min(a.portion.each, chunks) : chunks;
+    for (int chunk0 = 0; chunk0 < chunks && e == cudaSuccess; chunk0 += each) {
+        a.portion.chunk0 = chunk0;
+        const dim3 grid(min(each, chunks - chunk0), a.vdim / SC_VT * a.n_heads, n_seqs);
+        e = launch_pdl(chunk_parts_kernel<D>, grid, dim3(a.n_offset >= 0 ? 160 : 128), parts_smem, stream, a);
+        if (e == cudaSuccess) e = launch_pdl(chunk_chain_kernel<D>, dim3((items + 7) / 8, a.n_heads, n_seqs), dim3(256), 0, stream, a);
+        if (e == cudaSuccess) e = launch_pdl(chunk_outputs_kernel<D>, grid, dim3(128), outputs_smem, stream, a);
+    }
     return (int)e;
 }
 
 // q, k: bfloat16 [T][groups * dim], v: bfloat16 [T][heads * vdim], rows strided in whole eights and 16-byte aligned; decay, take:
 // float32 [T][heads] (rate_log null), or decay the pre-activations of both, rows gate_stride apart; y: float32 [T][heads * vdim]; nq: float32 [T][heads] or null (then n_offset < 0). scratch: float32
-// [(n_tokens / 128 + n_seqs)][heads][dim * vdim + dim + 1], 16-byte aligned. max_q_len: the most tokens any sequence brings.
+// [n_records][heads][dim * vdim + dim + 1], 16-byte aligned; n_records = n_tokens / 128 + n_seqs with each == 0, else n_seqs * each, and
+// the call goes through `each` chunks of every sequence at a time, with [n_seqs][heads][dim * vdim + dim] floats behind the scratch
+// for what passes from one portion to the next. max_q_len: the most tokens any sequence brings.
 QF_EXPORT int qf_state_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* decay,
                               const float* take, const float* dt_bias, const float* rate_log, int gate_stride, const int* cu_q,
                               const int* slots, int n_seqs, int max_q_len, float* state,
                               long long slot_stride, long long s_offset, long long n_offset, int n_heads, int n_groups, int dim,
-                              int vdim, float q_scale, float* scratch, long long n_records, float* y, float* nq, cudaStream_t stream) {
+                              int vdim, float q_scale, float* scratch, long long n_records, int each, float* y, float* nq,
+                              cudaStream_t stream) {
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
     if ((dim != 64 && dim != 128) || vdim <= 0 || vdim % SC_VT || (!take && !rate_log) || ((q_stride | k_stride | v_stride) & 7) ||
         (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) || n_groups <= 0 || n_heads <= 0 || n_heads % n_groups || n_seqs > 65535 ||
         (long long)n_heads * (vdim / SC_VT) > 65535 || (n_offset >= 0 && !nq) || ((uintptr_t)scratch & 15))
         return (int)cudaErrorInvalidValue;
-    float* n_parts = scratch + n_records * n_heads * dim * vdim;
+    if (each < 0 || (each > 0 && n_records < (long long)n_seqs * each)) return (int)cudaErrorInvalidValue;
+    float *n_parts = scratch + n_records * n_heads * dim * vdim, *whole = n_parts + n_records * n_heads * dim;
     const ChunkArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, decay, take, dt_bias, rate_log, gate_stride, cu_q, slots, state,
-                      slot_stride, s_offset, n_offset, n_heads, n_groups, vdim, q_scale, scratch, n_parts, n_parts + n_records * n_heads * dim, y, nq};
+                      slot_stride, s_offset, n_offset, n_heads, n_groups, vdim, q_scale, scratch, n_parts, whole, y, nq,
+                      Portion{0, each, each > 0 ? whole + n_records * n_heads : nullptr}};
     return dim == 64 ? launch_chunks<64>(a, n_seqs, max_q_len, stream) : launch_chunks<128>(a, n_seqs, max_q_len, stream);
 }

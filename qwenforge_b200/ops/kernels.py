@@ -1810,6 +1810,21 @@ def outer_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
         _stream()), "outer_state_scan")
 
 
+# What the chunked recurrences keep per chunk between their three launches, in all, or four chunks of every sequence where that is
+# more. A step that would need more goes through the chunks of its sequences in portions of this size: without one, 32 heads of
+# 128 x 128 took 16 KB a token, 0.5 GB for a prompt of 32,768 tokens. (A portion's launches cost about as much as the chain between
+# two of its chunks: 32 heads of 128 x 128, 8 x 2,048 tokens in portions of eight chunks 823 microseconds, a sequence alone 102.)
+CHUNK_SCRATCH_BYTES = 128 << 20
+
+
+def _chunk_portions(n: int, n_seqs: int, chunk: int, floats: int) -> tuple:
+    """(records, chunks of every sequence at a time or 0 for all at once) of a chunked recurrence over `n` tokens, `floats` a record."""
+    records, most = n // chunk + n_seqs, max(CHUNK_SCRATCH_BYTES // (4 * floats), 4 * n_seqs)
+    if records <= most:
+        return records, 0
+    return n_seqs * (most // n_seqs), most // n_seqs
+
+
 STATE_CHUNK = 128   # SC_CHUNK of csrc/state_chunks.cu
 # The longest sequence of a step from which the chunked form is the faster one. Measured, one sequence, scan / chunks in microseconds:
 # 16 heads of 64 x 128: 96 tokens 14 / 13, 160: 26 / 15, 256: 41 / 17, 2,048: 315 / 42; 32 heads of 128 x 128: 96 tokens 23 / 20,
@@ -1851,13 +1866,14 @@ def state_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: Optio
     if q.dtype != torch.bfloat16:
         raise KernelError("state_chunks: bfloat16 rows only (state_chunks_take)")
     n_seqs = cu_q.numel() - 1
-    records = n // STATE_CHUNK + n_seqs
-    scratch = torch.empty(records * n_heads * (dim * vdim + dim + 1), dtype=torch.float32, device=q.device)
+    records, each = _chunk_portions(n, n_seqs, STATE_CHUNK, n_heads * (dim * vdim + dim + 1))
+    carry = n_seqs * n_heads * (dim * vdim + dim) if each else 0
+    scratch = torch.empty(records * n_heads * (dim * vdim + dim + 1) + carry, dtype=torch.float32, device=q.device)
     _check(library("state_chunks").qf_state_chunks(
         _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay), _ptr(take), _ptr(dt_bias),
         _ptr(rate_log), _I(gate_stride), _ptr(cu_q), _ptr(slots), _I(n_seqs), _I(max_q_len), _ptr(state), _LL(state.stride(0)),
         _LL(s_offset), _LL(n_offset if nq is not None else -1), _I(n_heads), _I(n_groups), _I(dim), _I(vdim), _F(q_scale),
-        _ptr(scratch), _LL(records), _ptr(y), _ptr(nq), _stream()), "state_chunks")
+        _ptr(scratch), _LL(records), _I(each), _ptr(y), _ptr(nq), _stream()), "state_chunks")
 
 
 GATES = {"sigmoid": 0, "silu": 1}
@@ -2323,12 +2339,14 @@ def row_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     if q.dtype != torch.bfloat16:
         raise KernelError("row_chunks: bfloat16 rows only (row_chunks_take)")
     n, n_seqs = q.shape[0], cu_q.numel() - 1
-    records = n // ROW_CHUNK + n_seqs
-    scratch = torch.empty(records * n_heads * (dim * vdim + dim) + (n * n_heads * dim if kind else 0), dtype=torch.float32, device=q.device)
+    records, each = _chunk_portions(n, n_seqs, ROW_CHUNK, n_heads * (dim * vdim + dim))
+    carry = n_seqs * n_heads * dim * vdim if each else 0
+    scratch = torch.empty(records * n_heads * (dim * vdim + dim) + carry + (n * n_heads * dim if kind else 0), dtype=torch.float32,
+                          device=q.device)
     _check(library("row_chunks").qf_row_chunks(
         _ptr(q), _I(q.stride(0)), _ptr(k), _I(k.stride(0)), _ptr(v), _I(v.stride(0)), _ptr(decay), _ptr(decay_bias), _I(kind), _F(inv_tau),
         _ptr(bonus), _ptr(cu_q), _ptr(slots), _I(n_seqs), _I(max_q_len), _ptr(state), _LL(state.stride(0)), _LL(s_offset), _I(n_heads),
-        _I(dim), _I(vdim), _F(q_scale), _ptr(scratch), _LL(records), _ptr(y), _stream()), "row_chunks")
+        _I(dim), _I(vdim), _F(q_scale), _ptr(scratch), _LL(records), _I(each), _ptr(y), _stream()), "row_chunks")
 
 
 def rows_prepare(x: torch.Tensor, runs, eps: float, mix=None) -> None:

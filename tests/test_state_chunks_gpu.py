@@ -109,6 +109,37 @@ def test_no_less_exact_than_token_by_token(rows, dim, vdim, slow):
         assert rel(chunks, want) <= 1.1 * rel(scan, want)
 
 
+@pytest.mark.parametrize("lengths,floor", [((700,), 0), ((300, 1, 2113), 0), ((300, 1, 1300), 13)])
+@pytest.mark.parametrize("rows", [False, True])
+def test_portions_leave_the_same_bits(lengths, floor, rows, monkeypatch):
+    """A step whose records would need more than their bound goes through its chunks in portions: the same operations, also for a
+    sequence without a slot, whose state passes from portion to portion in the scratch."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.ops import kernels
+    g = torch.Generator(device=DEV).manual_seed(len(lengths) + floor)
+    heads, dim, vdim, slots, cu = 2, 64, 128, [3, 0, -1][:len(lengths)], [0]
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    n = cu[-1]
+    size, sizes = heads * dim * vdim, [heads * dim, heads * dim, heads * vdim]
+    q, k, v = (torch.randn(n, w, generator=g, device=DEV).bfloat16() for w in sizes)
+    decay = torch.rand(n, heads * dim if rows else heads, generator=g, device=DEV)
+    take, start = torch.rand(n, heads, generator=g, device=DEV), torch.randn(4, size + heads * dim, generator=g, device=DEV)
+    record = 4 * heads * (dim * vdim + dim + 1)
+    results = []
+    for bound in (1 << 30, record * floor):
+        monkeypatch.setattr(kernels, "CHUNK_SCRATCH_BYTES", bound)
+        state, y, nq = start.clone(), torch.empty(n, heads * vdim, device=DEV), torch.empty(n, heads, device=DEV)
+        if rows:
+            ops.row_chunks(q, k, v, decay, ints(cu), ints(slots), max(lengths), state, 0, heads, dim, vdim, 0.3, y,
+                           decay_from=("sigmoid_root", torch.ones(heads * dim, device=DEV), 8.0))
+        else:
+            ops.state_chunks(q, k, v, decay, take, ints(cu), ints(slots), max(lengths), state, 0, size, heads, heads, dim, vdim, 0.3, y, nq)
+        results.append((state, y) if rows else (state, y, nq))
+    for whole, portions in zip(*results):
+        assert torch.equal(whole, portions)
+
+
 def test_a_value_that_is_not_finite_reaches_no_earlier_token():
     from qwenforge_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(1)
