@@ -1825,19 +1825,37 @@ def _chunk_portions(n: int, n_seqs: int, chunk: int, floats: int) -> tuple:
     return n_seqs * (most // n_seqs), most // n_seqs
 
 
+def _chunks_pay(n: int, n_seqs: int, longest: int, state: int, chunk: int, scan: tuple, chunks: tuple) -> bool:
+    """Whether the chunked form of a recurrence is done before the scan, by what both cost on the device: the scan walks its longest
+    sequence and moves every sequence's state in and out; the chunked form works on one record per started chunk of every
+    sequence, also of one that brings a single token. `state`: numbers of one sequence's state. In microseconds, `state` in units of
+    65,536 numbers: scan = (per token of the longest sequence: fixed, per unit; per token and unit; per sequence and unit),
+    chunks = (fixed, per record and unit)."""
+    unit, longest = state / 65536, min(longest, n)
+    walk = max((scan[0] + scan[1] * unit) * longest, scan[2] * unit * n) + scan[3] * unit * n_seqs
+    return chunks[0] + chunks[1] * unit * (n // chunk + n_seqs) < walk
+
+
 STATE_CHUNK = 128   # SC_CHUNK of csrc/state_chunks.cu
 # The longest sequence of a step from which the chunked form is the faster one. Measured, one sequence, scan / chunks in microseconds:
 # 16 heads of 64 x 128: 96 tokens 14 / 13, 160: 26 / 15, 256: 41 / 17, 2,048: 315 / 42; 32 heads of 128 x 128: 96 tokens 23 / 20,
 # 160: 37 / 24. Three launches and a buffer instead of one launch cost the host about 10 microseconds more, which a step that is
 # issued launch by launch feels up to some 200 tokens.
 STATE_CHUNKS_MIN_TOKENS = 192
+# Beside other sequences (`_chunks_pay`), inside a graph, scan / chunks: 7 heads of 64 x 128: 192 + 31 x 1 tokens 24 / 41, 512 + 31 x 1
+# 55 / 43, 64 x 512 738 / 214; 16 heads: 512 + 31 x 1 69 / 78; 32 heads of 128 x 128: 192 43.8 / 31.0, 192 + 63 x 1 250 / 505,
+# 192 + 7 x 64 122 / 71, 2,048 + 15 x 1 434 / 234; of 128 x 64: 1,024 + 31 x 1 216 / 153.
+STATE_CHUNKS_COSTS = ((0.09, 0.015, 0.022, 0.25), (14.0, 0.98))
 
 
-def state_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dim: int, vdim: int, max_q_len: int) -> bool:
+def state_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dim: int, vdim: int, max_q_len: int, n_seqs: int = 1) -> bool:
     """Whether a step's recurrence runs on `state_chunks`: bfloat16 rows that 16-byte accesses can address, sizes the kernels are
-    made for, and a sequence long enough (STATE_CHUNKS_MIN_TOKENS). Otherwise `outer_state_scan` takes it."""
+    made for, a sequence long enough (STATE_CHUNKS_MIN_TOKENS) and not too many short ones beside it. Otherwise
+    `outer_state_scan` takes it."""
     return (max_q_len >= STATE_CHUNKS_MIN_TOKENS and dim in (64, 128) and vdim % 64 == 0 and q.dtype == torch.bfloat16 and q.is_cuda
-            and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0)
+            and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0
+            and v.shape[1] // 64 <= 65535 and n_seqs <= 65535   # (a grid's second and third extent)
+            and _chunks_pay(q.shape[0], n_seqs, max_q_len, dim * v.shape[1], STATE_CHUNK, *STATE_CHUNKS_COSTS))
 
 
 def state_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: Optional[torch.Tensor], take: Optional[torch.Tensor],
@@ -2319,14 +2337,22 @@ ROW_CHUNK = 64   # RC_CHUNK of csrc/row_chunks.cu
 # tokens 29 / 31, 512: 67 / 34. A step issued launch by launch waits for the host up to some 550 tokens, and two launches and a
 # buffer more cost it 5 of 103 microseconds.
 ROW_CHUNKS_MIN_TOKENS = 512
+# Beside other sequences (`_chunks_pay`), inside a graph, scan / chunks: 7 heads of 64 x 128: 512 + 31 x 1 tokens 71 / 60, 512 + 63 x 1
+# 77 / 93, 64 x 512 1,235 / 598; 16 heads: 512 + 31 x 1 89 / 109, 1,024 + 31 x 1 173 / 138; 32 heads of 64 x 64: 1,024 + 63 x 1
+# 178 / 266, 4 x 1,024 406 / 230.
+ROW_CHUNKS_COSTS = ((0.13, 0.0, 0.04, 0.2), (20.0, 1.3))
 
 
-def row_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, dim: int, vdim: int, max_q_len: int) -> bool:
+def row_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, dim: int, vdim: int, max_q_len: int,
+                    n_seqs: int = 1) -> bool:
     """Whether a step's recurrence with a decay per row runs on `row_chunks`: bfloat16 rows that 16-byte accesses can address, 64 rows and
-    whole 64 columns (up to 512) of a head's state, and a sequence long enough. Otherwise `outer_state_scan_rows` takes it."""
+    whole 64 columns (up to 512) of a head's state, a sequence long enough and not too many short ones beside it. Otherwise
+    `outer_state_scan_rows` takes it."""
     return (max_q_len >= ROW_CHUNKS_MIN_TOKENS and dim == 64 and vdim % 64 == 0 and vdim <= 512 and q.dtype == torch.bfloat16 and q.is_cuda
             and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0
-            and (q.data_ptr() | k.data_ptr() | v.data_ptr() | decay.data_ptr()) % 16 == 0)
+            and (q.data_ptr() | k.data_ptr() | v.data_ptr() | decay.data_ptr()) % 16 == 0
+            and v.shape[1] // 64 <= 65535 and n_seqs <= 65535   # (a grid's second and third extent)
+            and _chunks_pay(q.shape[0], n_seqs, max_q_len, dim * v.shape[1], ROW_CHUNK, *ROW_CHUNKS_COSTS))
 
 
 def row_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, cu_q: torch.Tensor, slots: torch.Tensor,

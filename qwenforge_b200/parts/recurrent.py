@@ -113,7 +113,7 @@ class MatrixMemory(Mixer):
         ops.stabilized_gates(pre, self.gate_bias, self.cap, ctx.cu_q, ctx.slots, site.storage, self.m_offset, h, decay, take, floor)
         y = torch.empty((n, h * v), **f32)
         sizes = (site.storage, self.s_offset, self.n_offset, h, h, d, v, d ** -0.5, y, nq)
-        if ops.state_chunks_take(q, k, values, d, v, ctx.max_q_len):   # in chunks on the tensor cores
+        if ops.state_chunks_take(q, k, values, d, v, ctx.max_q_len, ctx.n_seqs):   # in chunks on the tensor cores
             ops.state_chunks(q, k, values, decay, take, ctx.cu_q, ctx.slots, ctx.max_q_len, *sizes)
         else:                                                          # token by token: short steps, float32, other sizes
             ops.outer_state_scan(q, k, values, decay, take, ctx.cu_q, ctx.slots, *sizes)
@@ -186,7 +186,7 @@ class StateSpace(Mixer):
         y = torch.empty((n, self.inner), **f32)
         xs, b, c = xbc.split((self.inner, g * s, g * s), dim=1)
         sizes = (site.storage, self.s_offset, -1, h, g, s, v, 1.0, y, None)
-        if ops.state_chunks_take(c, b, xs, s, v, ctx.max_q_len):   # in chunks on the tensor cores, the gates formed inside
+        if ops.state_chunks_take(c, b, xs, s, v, ctx.max_q_len, ctx.n_seqs):   # in chunks on the tensor cores, the gates formed inside
             ops.state_chunks(c, b, xs, None, None, ctx.cu_q, ctx.slots, ctx.max_q_len, *sizes,
                              decay_gates=(dt_pre, self.dt_bias, self.rate_log))
         else:                                                      # token by token: short steps, float32, other sizes
@@ -219,7 +219,7 @@ def _low_rank(x, first, second, activation):
 def _scan_rows(ctx, q, k, v, pre, state, s_offset, heads, dim, vdim, q_scale, y, **decays):
     """The recurrence with a decay per row of the state: in chunks on the tensor cores where the step and its sizes allow
     (`ops.row_chunks`), token by token otherwise (short steps, float32, other sizes)."""
-    if ops.row_chunks_take(q, k, v, pre, dim, vdim, ctx.max_q_len):
+    if ops.row_chunks_take(q, k, v, pre, dim, vdim, ctx.max_q_len, ctx.n_seqs):
         ops.row_chunks(q, k, v, pre, ctx.cu_q, ctx.slots, ctx.max_q_len, state, s_offset, heads, dim, vdim, q_scale, y, **decays)
     else:
         ops.outer_state_scan_rows(q, k, v, pre, ctx.cu_q, ctx.slots, state, s_offset, heads, dim, vdim, q_scale, y, **decays)
