@@ -507,19 +507,21 @@ static int launch(const void* q, void* out, const int* cu_q, const int* tok_pos,
     // behind 8,000: 99, 115, 63, [25]; 64 behind 8,000, 16 heads of 128: 112, 127, 71, [31]; four prompts of 183 to 275: [7.2], 9.1, 10, 53.
     const int span = window > 0 && window + TA_BM < max_kv_len ? window + TA_BM : max_kv_len;
     const float longest = (float)((span + TA_BK - 1) / TA_BK), mean = longest > q_tiles ? longest - 0.5f * q_tiles : 0.5f * longest + 0.5f;
-    // (tiles that hold rows: the grid also has blocks for the rows that shorter sequences lack, which end at once)
-    const long long live = min((long long)q_tiles * n_seqs, max((2ll * n_tokens + (long long)TA_BM * n_seqs + TA_BM - 1) / (2 * TA_BM), 1ll)) * n_heads;
+    // (tiles that hold rows: the grid also has blocks for the rows that shorter sequences lack, which end at once. Every sequence has one,
+    // and half of a last one is counted on average)
+    const long long live = min((long long)q_tiles * n_seqs, max((2ll * n_tokens + (long long)TA_BM * n_seqs + TA_BM - 1) / (2 * TA_BM), (long long)n_seqs)) * n_heads;
     const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
     if (D == 64 && pages_pay(live, span, q_tiles, sms))
         return launch_pages<true>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, sinks,
                                   planes, stream);
     const float turn[2] = {D <= 64 ? 1.5f : 1.75f, D <= 64 ? 1.85f : 2.05f}, ends[2][4] = {{3.f, 5.f, 5.5f, 6.5f}, {5.f, 6.5f, 9.f, 13.f}};
     const int room[4] = {sms, sms, sms - sms / 8, sms * 77 / 100 > 0 ? sms * 77 / 100 : 1};
+    const float units = (float)live / ((float)n_seqs * kv_heads);   // tiles of an average sequence and kv head: a block takes two of the same
     int per = 2, split = 1;
     float least = -1.f;
     for (int p = 2; p >= 1; --p)
         for (int n = 0; n < 4; ++n) {
-            const long long blocks = (live + p - 1) / p << n;
+            const long long blocks = (long long)n_seqs * kv_heads * (long long)ceilf(units / p - 0.01f) << n;
             const float alone = ceilf(longest / (1 << n)) * turn[p - 1] + ends[p - 1][n];
             const float all = (float)((blocks + room[n] - 1) / room[n]) * (mean / (1 << n) * turn[p - 1] + ends[p - 1][n]);
             const float time = alone > all ? alone : all;

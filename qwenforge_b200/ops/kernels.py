@@ -422,8 +422,8 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor,
                          window: int, err: torch.Tensor, max_kv_len: Optional[int] = None,
                          sinks: Optional[torch.Tensor] = None, shared_values: bool = False) -> None:
     """The same attention on the fifth-generation tensor cores (tcgen05, accumulators in tensor memory): one or two tiles of
-    128 query rows a block; bfloat16, head sizes 64 and 128, cache pages without gaps. `max_kv_len` as in `attention_prefill`:
-    few tiles of many pages are shared by the two, four or eight blocks of a cluster."""
+    128 query rows a block; bfloat16, head sizes 64 and 128, cache pages without gaps. `max_kv_len` as in `attention_prefill` (None:
+    as long as the page table has room for): few tiles of many pages are shared by the two, four or eight blocks of a cluster."""
     _dev("q", q, torch.bfloat16)
     _dev("out", out, torch.bfloat16)
     _dev("cache", site.storage, torch.bfloat16)
@@ -442,7 +442,7 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor,
     _check(library("attention_prefill_tc").qf_attention_prefill_tc_ex(
         _ptr(q), _ptr(out), _ptr(cu_q), _ptr(tok_pos), _ptr(slots), _ptr(site.storage), _ptr(site.table),
         _LL(site.page_elems), _I(site.table_stride), _I(site.kv_heads), _I(d), _I(n_heads), _I(n_seqs), _I(q.shape[0]),
-        _I(max_q_len), _I(1 << 30 if max_kv_len is None else int(max_kv_len)), _F(scale), _I(window), _ptr(err),
+        _I(max_q_len), _I(int(max_kv_len) if max_kv_len is not None else min(1 << 30, site.table.shape[-1] * site.storage.shape[-2])), _F(scale), _I(window), _ptr(err),
         _ptr(sinks), _I(int(bool(shared_values))), _stream()), "attention_prefill_tc")
 
 

@@ -63,11 +63,32 @@ TC_PREFILL_MIN_TOKENS = {64: 2, 128: 2}
 TC_PREFILL_MIN_KEYS = 128
 
 
-def prefill_attention(head_dim: int, n_tokens: int, max_kv_len: int, window: int = 0):
+# A tile of the tcgen05 kernel is 128 rows of one sequence and head, one of the mma.sync kernel 64: with many sequences of up to 64
+# tokens the former multiplies mostly padding. Where its tiles, two of a kv head to a block, are more than one round of blocks,
+# both are estimated, in microseconds as measured, and the earlier one is taken: mma.sync T (per key page x pages + per tile) with T
+# tiles; tcgen05 a round's turns of 128 keys and a block's ends. Measured inside a graph, mma.sync / tcgen05: 14 heads of 64, 2
+# tokens a sequence, 64 sequences behind 127 tokens 14 / 30, behind 1,000 53 / 70, behind 3,000 146 / 176; 32 behind 127 8 / 16,
+# behind 500 15 / 23, behind 3,000 99 / 89; 28 heads of 128: 32 sequences behind 127 27 / 34, behind 500 60 / 50. Below one round the
+# tcgen05 kernel loses only where up to 16 tokens see up to three pages (14 heads of 64, 16 sequences of 2 behind 127: 7 / 9).
+SHORT_SEQUENCES = {64: (0.0036, 0.006, 1.85, 5.0), 128: (0.0070, 0.007, 2.05, 6.5)}
+
+
+def prefill_attention(head_dim: int, n_tokens: int, max_kv_len: int, window: int = 0, *, max_q_len: int = 0, n_seqs: int = 1,
+                      n_heads: int = 1, kv_heads: int = 1):
     """The attention kernel of a step of several tokens per sequence: the tcgen05 one where it has the head size and enough to do."""
     least = TC_PREFILL_MIN_TOKENS.get(head_dim)
-    keys = min(max_kv_len, window) if window > 0 else max_kv_len
-    return ops.attention_prefill_tc if least is not None and n_tokens >= least and keys >= TC_PREFILL_MIN_KEYS else ops.attention_prefill
+    keys = min(max_kv_len, window + max_q_len) if window > 0 else max_kv_len
+    if least is None or n_tokens < least or (min(max_kv_len, window) if window > 0 else max_kv_len) < TC_PREFILL_MIN_KEYS:
+        return ops.attention_prefill
+    blocks = n_seqs * kv_heads * -(-n_heads // (2 * kv_heads))
+    if max_q_len <= 64 and blocks > 100:
+        pages, (a_page, a_tile, a_turn, ends) = -(-keys // 64), SHORT_SEQUENCES[head_dim]
+        rounds = blocks / ops.sm_count("cuda")
+        if rounds > 1 and n_seqs * n_heads * (a_page * pages + a_tile) < rounds * (a_turn * pages / 2 + ends):
+            return ops.attention_prefill
+        if rounds <= 1 and max_q_len <= 16 and pages <= 3:
+            return ops.attention_prefill
+    return ops.attention_prefill_tc
 
 
 class GqaAttention(Mixer):
@@ -295,7 +316,8 @@ class GqaAttention(Mixer):
             ops.attention_decode(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,
                                  self.scale, self.window, self.decode_splits(ctx), ctx.decode_scratch, ctx.err, plan)
         elif fast:
-            prefill = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window)
+            prefill = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window, max_q_len=ctx.max_q_len, n_seqs=ctx.n_seqs,
+                                        n_heads=self.n_heads, kv_heads=self.n_kv)
             prefill(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,
                     ctx.max_q_len, self.scale, self.window, ctx.err, max_kv_len=ctx.max_kv_len)
         else:

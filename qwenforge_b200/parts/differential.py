@@ -92,7 +92,8 @@ class DifferentialAttention(GqaAttention):
         attended = torch.empty_like(q)
         common = (q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs)
         if fast:
-            run = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window)
+            run = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window, max_q_len=ctx.max_q_len, n_seqs=ctx.n_seqs,
+                                    n_heads=self.n_heads, kv_heads=self.n_kv)
             run(*common, ctx.max_q_len, self.scale, self.window, ctx.err, max_kv_len=ctx.max_kv_len)
         else:
             ops.attention_generic(*common, ctx.max_q_len, self.scale, self.window, ctx.err, scratch=ctx.decode_scratch,

@@ -150,7 +150,7 @@ class LatentAttention(Mixer):
                                  self.window, n_splits, ctx.decode_scratch, ctx.err, self.decode_plan(ctx, n_splits),
                                  sinks=self.sinks, shared_values=True)
         elif fast:
-            prefill = prefill_attention(r, n, ctx.max_kv_len, self.window)
+            prefill = prefill_attention(r, n, ctx.max_kv_len, self.window, max_q_len=ctx.max_q_len, n_seqs=ctx.n_seqs, n_heads=h)
             prefill(q_in_latent, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, h, ctx.n_seqs, ctx.max_q_len,
                                   self.scale, self.window, ctx.err, max_kv_len=ctx.max_kv_len, sinks=self.sinks,
                                   shared_values=True)

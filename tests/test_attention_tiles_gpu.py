@@ -111,3 +111,14 @@ def test_which_kernel_a_step_takes():
     assert prefill_attention(64, 2, 128) is ops.attention_prefill_tc and prefill_attention(128, 500, 4000, 200) is ops.attention_prefill_tc
     assert prefill_attention(64, 100, 100) is ops.attention_prefill and prefill_attention(32, 500, 500) is ops.attention_prefill
     assert prefill_attention(64, 500, 4000, 100) is ops.attention_prefill
+
+
+def test_many_short_sequences_keep_the_smaller_tiles():
+    """Where both kernels were measured, the rule names the faster one."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.parts.attention import prefill_attention
+    pick = lambda dim, heads, kv, seqs, tokens, before: prefill_attention(dim, seqs * tokens, before + tokens, max_q_len=tokens, n_seqs=seqs,
+                                                                         n_heads=heads, kv_heads=kv) is ops.attention_prefill_tc
+    assert not pick(64, 14, 2, 64, 2, 127) and not pick(64, 14, 2, 64, 2, 1000) and not pick(64, 14, 14, 64, 16, 1000)
+    assert not pick(128, 28, 4, 64, 8, 127) and not pick(64, 14, 2, 16, 2, 127) and not pick(128, 4, 4, 64, 16, 127)
+    assert pick(128, 28, 4, 64, 8, 1000) and pick(64, 14, 2, 16, 2, 1000) and pick(64, 14, 2, 64, 100, 500) and pick(64, 14, 2, 4, 32, 500)
