@@ -902,16 +902,18 @@ def qkv_product_way(m: int, weight: torch.Tensor, n_heads: int, kv_heads: int, h
     mma.sync streamer with all of it inside), "wide" (a norm kernel, then the tcgen05 streamer with the rest) or "unfused" (norm,
     library product, rotation). Measured as a whole decode step, microseconds, skinny / wide: Qwen2.5-0.5B (2 MB) 8 rows 673 / 703, 12 rows
     960 / 850, 16 rows 963 / 863; 3B (10 MB) 1 row 1,908 / 1,876, 4 rows 2,040 / 1,973, 8 rows 2,238 / 2,144, 16 rows 2,365 / 2,173;
-    eight layers of 7B (33 MB) 1 row 982 / 1,000, 8 rows 1,004 / 1,020, 16 rows 1,062 / 1,037. So the tcgen05 streamer from 9 rows on, where
-    the other's token rows take a second pass over the tile, and below for weights whose tiles are too many for one wave of
-    the other's blocks and too few to fill its ring (8 to 20 MB). From 17 rows on the other way is "unfused" (against "wide": 0.5B
+    eight layers of 7B (33 MB) 1 row 982 / 1,000, 8 rows 1,004 / 1,020, 16 rows 1,062 / 1,037; twelve layers of other sizes, 1, 2, 4 and 8
+    rows: 12.6 MB (32 + 8 heads of 64) 591 / 599, 632 / 622, 666 / 657, 722 / 705; 13.0 MB 669 / 665, 690 / 680, 754 / 737, 766 / 745; 18.4 MB
+    728 / 749, 749 / 750, 754 / 757, 789 / 779; 22 MB 776 / 800, 792 / 801, 800 / 800, 817 / 817. So the tcgen05 streamer from 9 rows on,
+    where the other's token rows take a second pass over the tile, and below for weights whose tiles are too many for one wave of
+    the other's blocks and too few to fill its ring: 8 to 16 MB, to 12 MB for a single row. From 17 rows on the other way is "unfused" (against "wide": 0.5B
     17 rows 918 / 871, 32 rows 932 / 888, 64 rows 991 / 990; twelve layers of 3B 890 / 841, 906 / 876, 979 / 968; 7B 1,073 / 1,050,
     1,086 / 1,064, 1,205 / 1,209), which is no slower with 49 to 64 rows of a large weight."""
     size = weight.numel() * weight.element_size()
     heads = dict(n_heads=n_heads, kv_heads=kv_heads, head_dim=head_dim, rot_dim=rot_dim)
     skinny = m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_QKV, True, **heads)
     wide = m <= WIDE_MAX_ROWS and wide_gemm_takes_rows(EPI_QKV, m, weight, **heads)
-    if skinny and (not wide or (m <= 8 and not 8e6 <= size < 20e6)):
+    if skinny and (not wide or (m <= 8 and not 8e6 <= size < (12e6 if m == 1 else 16e6))):
         return "skinny"
     return "wide" if wide and (m <= 48 or size < 20e6) else "unfused"
 

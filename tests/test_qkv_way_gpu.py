@@ -68,3 +68,11 @@ def test_the_rule():
     assert [way(m, small, 14, 2, 64, 64) for m in (1, 8, 9, 16, 17, 64)] == ["skinny", "skinny", "wide", "wide", "wide", "wide"]
     assert [way(m, middle, 16, 2, 128, 128) for m in (1, 8, 9, 64)] == ["wide"] * 4
     assert way(65, small, 14, 2, 64, 64) == "unfused" and way(9, small[:, :895], 14, 2, 64, 64) == "unfused"
+
+
+def test_the_rule_beyond_its_band():
+    """The band in which the tcgen05 streamer is the faster one for few rows ends at 16 MB, for a single row at 12."""
+    from qwenforge_b200 import ops
+    between, large = (torch.zeros(n, k, dtype=torch.bfloat16, device=DEV) for n, k in ((3072, 2048), (3584, 2560)))
+    assert [ops.qkv_product_way(m, between, 32, 8, 64, 64) for m in (1, 2, 8, 9)] == ["skinny", "wide", "wide", "wide"]
+    assert [ops.qkv_product_way(m, large, 20, 4, 128, 128) for m in (1, 2, 8, 9)] == ["skinny", "skinny", "skinny", "wide"]
