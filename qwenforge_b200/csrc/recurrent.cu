@@ -12,15 +12,18 @@
 #include "common.cuh"
 
 // ------------------------------------------------------------------------------------------------------------------
-// Exponential gates with a running maximum (the mLSTM's): one block per (sequence, head), GATE_TOKENS tokens at a time. Every
-// thread works out its tokens' two log gates (tanh, logsigmoid); then one thread runs the maximum m' = max(f + m, a) through the
-// tokens in order, eight at a time with the next eight's gates already on their way; then every thread forms its tokens'
-// three exponentials. Neighbouring tokens share the very same m, so what a token's gates say cancels in the mixer's quotient, and the
-// chain is the same operations in the same order for every cut of a sequence, in both precisions. What bounds it is that chain,
-// an addition and a maximum a token.
-#define GATE_THREADS 256
-#define GATE_TOKENS 2048
-#define GATE_LINKS 8
+// Exponential gates with a running maximum (the mLSTM's): m' = max(f + m, a), one block per (sequence, head), GATE_TOKENS tokens at a
+// time, a run of four neighbouring tokens to a thread. Every thread works out its tokens' two log gates (tanh, logsigmoid). What
+// its run does to the maximum m before it is  max(f_4 + (f_3 + (f_2 + (f_1 + m))), b)  with b the chain of the run alone (from minus
+// infinity): a rounded addition keeps the order of its arguments, so that the maxima may be taken after the additions, with the very
+// bits of the chain token by token. So one thread takes m from run to run by four additions and a maximum, and every thread then
+// walks its own tokens from the m before them. Neighbouring tokens share the very same m, so what a token's gates say cancels in
+// the mixer's quotient, and the bits are the same for every cut of a sequence, in both precisions. What bounds it is that one
+// thread's chain: 2,048 tokens of 7 heads take 14.5 microseconds (37 with a warp that hands every link on by shuffles; 256 tokens 4.1
+// and 5.9, a single token 2.1 either way).
+#define GATE_THREADS 512
+#define GATE_EACH 4
+#define GATE_TOKENS (GATE_THREADS * GATE_EACH)
 
 __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
@@ -30,74 +33,67 @@ stabilized_gates_kernel(const float* __restrict__ pre, int pre_stride, const flo
                         long long slot_stride, long long m_offset, int n_heads, float* __restrict__ decay,
                         float* __restrict__ take, float* __restrict__ floor_out) {
     grid_chain_entry();
-    constexpr int EACH = GATE_TOKENS / GATE_THREADS;
-    __shared__ __align__(16) float a_s[GATE_TOKENS], f_s[GATE_TOKENS], m_s[GATE_TOKENS];   // m_s: the maximum behind each token
+    __shared__ __align__(16) float4 f_s[GATE_THREADS];
+    __shared__ __align__(8) float end_s[GATE_THREADS], before_s[GATE_THREADS + 2];   // a run's own chain at its end; the maximum before a run
     const int seq = blockIdx.x / n_heads, head = blockIdx.x % n_heads;
     const int begin = cu_q[seq], end = cu_q[seq + 1], slot = slots[seq];
     float* m_ptr = slot >= 0 ? state + slot * slot_stride + m_offset + head : nullptr;
     float m = m_ptr ? *m_ptr : 0.f;   // the maximum before the tokens in hand
     const float bi = bias[head], bf = bias[n_heads + head];
     for (int t0 = begin; t0 < end; t0 += GATE_TOKENS) {
-        const int n_here = min(GATE_TOKENS, end - t0), n_links = (n_here + GATE_LINKS - 1) / GATE_LINKS * GATE_LINKS;
-        float a[EACH], f[EACH];
+        const int n_here = min(GATE_TOKENS, end - t0), n_pairs = (n_here + 2 * GATE_EACH - 1) / (2 * GATE_EACH);   // two runs a turn of the chain
+        const int first = threadIdx.x * GATE_EACH, count = max(0, min(GATE_EACH, n_here - first));   // this thread's tokens
+        float a[GATE_EACH], f[GATE_EACH], b = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < EACH; ++i) {
-            const int j = threadIdx.x + GATE_THREADS * i;
-            a[i] = f[i] = 0.f;   // (behind the last token: links that nobody reads)
-            if (j < n_here) {
-                const float* row = pre + (size_t)(t0 + j) * pre_stride + head;
-                a[i] = row[0], f[i] = row[n_heads];
-            }
+        for (int i = 0; i < GATE_EACH; ++i) a[i] = f[i] = 0.f;   // (behind the last token: additions of zero)
+#pragma unroll
+        for (int i = 0; i < GATE_EACH; ++i) {
+            if (i >= count) break;
+            const float* row = pre + (size_t)(t0 + first + i) * pre_stride + head;
+            a[i] = row[0], f[i] = row[n_heads];
         }
 #pragma unroll
-        for (int i = 0; i < EACH; ++i) {
-            const int j = threadIdx.x + GATE_THREADS * i;
-            if (j < n_here) {
-                a[i] = cap * tanhf((a[i] + bi) / cap);
-                f[i] = log_sigmoid(cap * tanhf((f[i] + bf) / cap));
-            }
-            if (j < n_links) a_s[j] = a[i], f_s[j] = f[i];
+        for (int i = 0; i < GATE_EACH; ++i) {
+            if (i >= count) break;
+            a[i] = cap * tanhf((a[i] + bi) / cap);
+            f[i] = log_sigmoid(cap * tanhf((f[i] + bf) / cap));
+            b = i == 0 ? a[i] : fmaxf(f[i] + b, a[i]);
         }
+        if (threadIdx.x < 2 * n_pairs) f_s[threadIdx.x] = make_float4(f[0], f[1], f[2], f[3]), end_s[threadIdx.x] = b;
         __syncthreads();
         if (threadIdx.x == 0) {
-            const float4 *a4 = reinterpret_cast<const float4*>(a_s), *f4 = reinterpret_cast<const float4*>(f_s);
-            float4* m4 = reinterpret_cast<float4*>(m_s);
-            float4 next_a[GATE_LINKS / 4], next_f[GATE_LINKS / 4];
+            const float2* e2 = reinterpret_cast<const float2*>(end_s);
+            float4 x = f_s[0], y = f_s[1];
+            float2 e = e2[0];
             float run = m;
-#pragma unroll
-            for (int u = 0; u < GATE_LINKS / 4; ++u) next_a[u] = a4[u], next_f[u] = f4[u];
-            for (int g = 0; g < n_links / 4; g += GATE_LINKS / 4) {
-                float4 at[GATE_LINKS / 4], ft[GATE_LINKS / 4];
-#pragma unroll
-                for (int u = 0; u < GATE_LINKS / 4; ++u) {
-                    at[u] = next_a[u], ft[u] = next_f[u];
-                    const int ahead = min(g + GATE_LINKS / 4, n_links / 4 - GATE_LINKS / 4) + u;
-                    next_a[u] = a4[ahead], next_f[u] = f4[ahead];
-                }
-#pragma unroll
-                for (int u = 0; u < GATE_LINKS / 4; ++u) {
-                    float4 out;
-                    run = out.x = fmaxf(ft[u].x + run, at[u].x);
-                    run = out.y = fmaxf(ft[u].y + run, at[u].y);
-                    run = out.z = fmaxf(ft[u].z + run, at[u].z);
-                    run = out.w = fmaxf(ft[u].w + run, at[u].w);
-                    m4[g + u] = out;
-                }
+            for (int p = 0; p < n_pairs; ++p) {
+                const float4 u = x, v = y;
+                const float2 at = e;
+                const int next = min(p + 1, n_pairs - 1);
+                x = f_s[2 * next], y = f_s[2 * next + 1], e = e2[next];
+                float2 before;
+                before.x = run;
+                before.y = fmaxf(u.w + (u.z + (u.y + (u.x + run))), at.x);
+                run = fmaxf(v.w + (v.z + (v.y + (v.x + before.y))), at.y);
+                reinterpret_cast<float2*>(before_s)[p] = before;
             }
+            before_s[2 * n_pairs] = run;
         }
         __syncthreads();
+        if (count > 0) {
+            m = before_s[threadIdx.x];
 #pragma unroll
-        for (int i = 0; i < EACH; ++i) {
-            const int j = threadIdx.x + GATE_THREADS * i;
-            if (j < n_here) {
-                const float before = j > 0 ? m_s[j - 1] : m, mine = m_s[j];
-                const size_t at = (size_t)(t0 + j) * n_heads + head;
-                decay[at] = expf(f[i] + before - mine);
-                take[at] = expf(a[i] - mine);
-                floor_out[at] = expf(-mine);
+            for (int i = 0; i < GATE_EACH; ++i) {
+                if (i >= count) break;
+                const float m_new = fmaxf(f[i] + m, a[i]);
+                const size_t at = (size_t)(t0 + first + i) * n_heads + head;
+                decay[at] = expf(f[i] + m - m_new);
+                take[at] = expf(a[i] - m_new);
+                floor_out[at] = expf(-m_new);
+                m = m_new;
             }
         }
-        m = m_s[n_here - 1];   // (written again only behind the next barrier)
+        m = before_s[2 * n_pairs];   // (written again only behind the next barrier)
     }
     if (m_ptr && threadIdx.x == 0 && begin < end) *m_ptr = m;
 }
@@ -628,8 +624,9 @@ gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ gate,
 
 // The same in bfloat16 where every run of eight columns lies within a head and all rows are addressable by 16 bytes: G threads take a
 // part (a power of two of lanes up to a warp, or a block), each P pieces of eight columns, all of whose inputs are asked for at
-// once and read once. What bounds it is memory: 4,206 rows of 4,096 columns with a gate and a skip (172 MB) took 133
-// microseconds with scalar loads (whose parts beyond 2,048 columns were also read twice), 50 here.
+// once and read once. What bounds it is memory, and beside it the exponentials and divisions of the gates: 4,206 rows of 4,096 columns
+// with a gate and a skip (172 MB) took 116 microseconds with scalar loads (whose parts beyond 2,048 columns were also read twice),
+// 54 here.
 template <int G, int P>
 __global__ void __launch_bounds__(256)
 gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict__ gate, int gate_stride, const bf16* __restrict__ weight,
@@ -820,8 +817,8 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ x, int x_stride, c
 }
 
 // The same convolution for long steps: a thread takes 16 bytes of channels and a run of CONV_RUN(TAPS) consecutive tokens, asks for
-// all of the run's rows at once (4,206 tokens of 4,352 channels, 73 MB: 73 microseconds with a row and its sequence fetched token by
-// token, 53 so, 32 with the hardware's exponential as well), keeps
+// all of the run's rows at once (4,206 tokens of 4,352 channels, 73 MB: 69 microseconds with a row and its sequence fetched token by
+// token, 54 so; the exponentials and divisions of silu bound it), keeps
 // the last TAPS - 1 inputs in registers as it walks down the run, and fetches them afresh (from the state, or zeros) where a
 // sequence begins inside the run. Every output is the same chain of fused multiply-adds, oldest input first, as in the
 // kernel of one thread per (token, channel): the two agree bit for bit.
