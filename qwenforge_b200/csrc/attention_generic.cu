@@ -259,67 +259,72 @@ __global__ void attention_generic_fold_kernel(T* __restrict__ out, const int* __
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// The plain form (no option but a window) of float32 steps of several tokens, head sizes 64 and 128: a block serves 64
-// consecutive tokens of one query head and walks the keys a page at a time; its 16 x 16 threads hold 4 rows x 4 keys of
-// the scores, then 4 rows x D / 16 columns of the output, so that a load from shared memory feeds four multiply-adds (in
-// the kernel above: one). Every score is one chain over the components, every output one chain over the keys in rising
-// order, pages at multiples of 64, so a row's arithmetic depends on its own position and window only, as above (the two
-// kernels differ by rounding). What bounds it is the multiply-add pipe and the walk of the longest tile: one prompt of
-// 1,031 tokens, 14 heads of 64: 893 -> 122 microseconds.
-#define FT_ROWS 64
+// The plain form (no option but a window) of float32 steps of several tokens, head sizes 64 and 128: a block serves 16 * RT rows of
+// one kv head (a row is a token and a query head of the group, the heads of a token neighbours) and walks the keys a page at a
+// time; its 16 x 16 threads hold RT rows x 4 keys of the scores, then RT rows x D / 16 columns of the output, so that with RT = 4
+// a load from shared memory feeds four multiply-adds (in the kernel above: one). Every score is one chain over the components,
+// every output one chain over the keys in rising order, pages at multiples of 64, so a row's arithmetic depends on its own
+// position and window only, as above and whatever RT (the two kernels differ by rounding). What bounds it is the
+// multiply-add pipe and the walk of the longest tile: one prompt of 1,031 tokens, 14 heads of 64: 893 -> 122 microseconds.
 #define FT_THREADS 256
-template <int D>
+template <int D, int RT>
 __global__ void __launch_bounds__(FT_THREADS)
 attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, const int* __restrict__ cu_q,
                           const int* __restrict__ tok_pos, const int* __restrict__ slots, KvSite<float> site, int n_heads, float scale,
                           int window, int* err) {
-    constexpr int LD = D + 4, LP = QF_PAGE + 4, PIECES = D / 4, DT = D / 16;
+    constexpr int LD = D + 4, LP = QF_PAGE + 4, PIECES = D / 4, DT = D / 16, ROWS = 16 * RT;
     extern __shared__ __align__(16) float ft_smem[];
-    float* q_s = ft_smem;                   // [64][LD]
-    float* k_s = q_s + FT_ROWS * LD;        // [64][LD]
+    float* q_s = ft_smem;                   // [ROWS][LD]
+    float* k_s = q_s + ROWS * LD;           // [64][LD]
     float* v_s = k_s + QF_PAGE * LD;        // [64][LD]
-    float* p_s = v_s + QF_PAGE * LD;        // [64][LP]: the page's weights, a row per query
-    const int tile = (int)gridDim.y - 1 - (int)blockIdx.y, head = blockIdx.x, seq = blockIdx.z;   // the longest walks first
-    const int q_begin = cu_q[seq], q_len = cu_q[seq + 1] - q_begin, t0 = tile * FT_ROWS;
-    if (t0 >= q_len) return;
-    const int n_rows = min(FT_ROWS, q_len - t0), slot = slots[seq], width = n_heads * D;
-    const float* q_src = q + (size_t)(q_begin + t0) * width + head * D;
-    float* o_dst = out + (size_t)(q_begin + t0) * width + head * D;
+    float* p_s = v_s + QF_PAGE * LD;        // [ROWS][LP]: the page's weights, a row per query
+    const int tile = (int)gridDim.y - 1 - (int)blockIdx.y, kvh = blockIdx.x, seq = blockIdx.z;   // the longest walks first
+    const int group = n_heads / site.kv_heads, row0 = tile * ROWS;
+    const int q_begin = cu_q[seq], q_rows = (cu_q[seq + 1] - q_begin) * group;
+    if (row0 >= q_rows) return;
+    const int n_rows = min(ROWS, q_rows - row0), slot = slots[seq], width = n_heads * D;
+    auto place = [&](int r) {   // where row r of the tile begins, in q and in out
+        const int token = (row0 + r) / group, head = kvh * group + (row0 + r) % group;
+        return (size_t)(q_begin + token) * width + (size_t)head * D;
+    };
     if (slot < 0) {  // a padding entry of the batch: defined output, no cache access
         for (int i = threadIdx.x; i < n_rows * PIECES; i += FT_THREADS)
-            *reinterpret_cast<float4*>(o_dst + (size_t)(i / PIECES) * width + i % PIECES * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>(out + place(i / PIECES) + i % PIECES * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    const int kvh = head / (n_heads / site.kv_heads), first_pos = tok_pos[q_begin + t0], last_pos = first_pos + n_rows - 1;
+    const int first_token = row0 / group, first_pos = tok_pos[q_begin + first_token];
+    const int last_pos = first_pos + (row0 + n_rows - 1) / group - first_token;
     const int lo_min = window > 0 ? max(0, first_pos - window + 1) : 0, page_begin = lo_min / QF_PAGE, page_end = last_pos / QF_PAGE + 1;
     const int* table = site.table + (long long)slot * site.table_stride;
     // one page's keys or values; positions that no row of the tile sees, and pages that are not held, become zeros
+    // RT = 1: how many of a page's keys, from its first, any row sees, in whole 16s. (Beyond them scores are masked and weights are zeros.)
+    auto keys_of = [&](int page) { return RT == 1 ? min(QF_PAGE, (last_pos - page * QF_PAGE + 16) & ~15) : QF_PAGE; };
     auto fetch = [&](float* dst, int page, int which) {
         const int held = table[page];
         if (held < 0 && threadIdx.x == 0) atomicOr(err, QF_ERR_NO_PAGE);
         const float* src = site.base + (long long)max(held, 0) * site.page_elems + (long long)(which * site.kv_heads + kvh) * QF_PAGE * D;
         const int lo = max(lo_min - page * QF_PAGE, 0), hi = last_pos - page * QF_PAGE;
-        for (int i = threadIdx.x; i < QF_PAGE * PIECES; i += FT_THREADS) {
+        for (int i = threadIdx.x; i < keys_of(page) * PIECES; i += FT_THREADS) {
             const int j = i / PIECES, c = i % PIECES * 4;
             const bool there = held >= 0 && j >= lo && j <= hi;
             cp_async_16(dst + j * LD + c, src + j * D + c, there);
         }
         cp_async_commit();
     };
-    for (int i = threadIdx.x; i < FT_ROWS * PIECES; i += FT_THREADS) {
+    for (int i = threadIdx.x; i < ROWS * PIECES; i += FT_THREADS) {
         const int r = i / PIECES, c = i % PIECES * 4;
-        cp_async_16(q_s + r * LD + c, r < n_rows ? q_src + (size_t)r * width + c : q_src, r < n_rows);
+        cp_async_16(q_s + r * LD + c, r < n_rows ? q + place(r) + c : q, r < n_rows);
     }
     fetch(k_s, page_begin, 0);
     fetch(v_s, page_begin, 1);
 
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float m[4], l[4], o[4][DT];
-    int pos[4], lo[4];
+    float m[RT], l[RT], o[RT][DT];
+    int pos[RT], lo[RT];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < RT; ++r) {
         m[r] = -FLT_MAX, l[r] = 0.f;
-        pos[r] = first_pos + ty * 4 + r;
+        pos[r] = first_pos + (row0 + ty * RT + r) / group - first_token;
         lo[r] = window > 0 ? max(0, pos[r] - window + 1) : 0;
 #pragma unroll
         for (int c = 0; c < DT; ++c) o[r][c] = 0.f;
@@ -327,22 +332,25 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
     for (int page = page_begin; page < page_end; ++page) {
         cp_async_wait<1>();
         __syncthreads();     // the queries and the page's keys are there
-        float s[4][4];       // rows ty * 4 + r, keys tx + 16 * j
+        const int n_keys = keys_of(page);
+        float s[RT][4];      // rows ty * RT + r, keys tx + 16 * j
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < RT; ++r)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[r][j] = 0.f;
 #pragma unroll 4
         for (int d = 0; d < D; d += 4) {
-            float4 a[4], b[4];
+            float4 a[RT], b[4];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(q_s + (ty * 4 + r) * LD + d);
+            for (int r = 0; r < RT; ++r) a[r] = *reinterpret_cast<const float4*>(q_s + (ty * RT + r) * LD + d);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(k_s + (tx + 16 * j) * LD + d);
+            for (int j = 0; j < 4; ++j)
+                if (16 * j < n_keys) b[j] = *reinterpret_cast<const float4*>(k_s + (tx + 16 * j) * LD + d);
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
+            for (int r = 0; r < RT; ++r)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
+                    if (16 * j >= n_keys) continue;
                     s[r][j] = fmaf(a[r].x, b[j].x, s[r][j]);
                     s[r][j] = fmaf(a[r].y, b[j].y, s[r][j]);
                     s[r][j] = fmaf(a[r].z, b[j].z, s[r][j]);
@@ -351,7 +359,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
         }
         const int key0 = page * QF_PAGE + tx;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < RT; ++r) {
             float top = -FLT_MAX;
             bool seen[4];
 #pragma unroll
@@ -368,7 +376,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const float p = seen[j] ? expf(s[r][j] - m_new) : 0.f;
-                p_s[(ty * 4 + r) * LP + tx + 16 * j] = p;
+                p_s[(ty * RT + r) * LP + tx + 16 * j] = p;
                 sum += p;
             }
 #pragma unroll
@@ -387,17 +395,17 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
         int odd = 0;
         if (page * QF_PAGE + QF_PAGE - 1 > first_pos || (window > 0 && page * QF_PAGE < last_pos - window + 1)) {
             __syncthreads();
-            for (int i = threadIdx.x; i < QF_PAGE * PIECES; i += FT_THREADS) {
+            for (int i = threadIdx.x; i < n_keys * PIECES; i += FT_THREADS) {
                 const float4 x = *reinterpret_cast<const float4*>(v_s + i / PIECES * LD + i % PIECES * 4);
                 odd |= !(fabsf(x.x) <= FLT_MAX) || !(fabsf(x.y) <= FLT_MAX) || !(fabsf(x.z) <= FLT_MAX) || !(fabsf(x.w) <= FLT_MAX);
             }
         }
         if (__syncthreads_or(odd)) {
-            for (int j = 0; j < QF_PAGE; ++j) {
+            for (int j = 0; j < n_keys; ++j) {
                 const int key = page * QF_PAGE + j;
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float p = p_s[(ty * 4 + r) * LP + j];
+                for (int r = 0; r < RT; ++r) {
+                    const float p = p_s[(ty * RT + r) * LP + j];
                     if (key > pos[r] || key < lo[r]) continue;
 #pragma unroll
                     for (int c = 0; c < DT; ++c) o[r][c] = fmaf(p, v_s[j * LD + (c / 4) * 64 + tx * 4 + c % 4], o[r][c]);
@@ -405,17 +413,17 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
             }
         } else {
 #pragma unroll 4
-            for (int j = 0; j < QF_PAGE; j += 4) {
-                float4 p[4];
+            for (int j = 0; j < n_keys; j += 4) {
+                float4 p[RT];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) p[r] = *reinterpret_cast<const float4*>(p_s + (ty * 4 + r) * LP + j);
+                for (int r = 0; r < RT; ++r) p[r] = *reinterpret_cast<const float4*>(p_s + (ty * RT + r) * LP + j);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
 #pragma unroll
                     for (int c = 0; c < DT; c += 4) {   // runs of four columns, 64 columns apart
                         const float4 v = *reinterpret_cast<const float4*>(v_s + (j + e) * LD + c * 16 + tx * 4);
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) {
+                        for (int r = 0; r < RT; ++r) {
                             const float w = e == 0 ? p[r].x : e == 1 ? p[r].y : e == 2 ? p[r].z : p[r].w;
                             o[r][c] = fmaf(w, v.x, o[r][c]);
                             o[r][c + 1] = fmaf(w, v.y, o[r][c + 1]);
@@ -430,23 +438,24 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
         else cp_async_commit();
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        if (ty * 4 + r >= n_rows) continue;
+    for (int r = 0; r < RT; ++r) {
+        if (ty * RT + r >= n_rows) continue;
         const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
 #pragma unroll
         for (int c = 0; c < DT; c += 4)
-            *reinterpret_cast<float4*>(o_dst + (size_t)(ty * 4 + r) * width + c * 16 + tx * 4) =
+            *reinterpret_cast<float4*>(out + place(ty * RT + r) + c * 16 + tx * 4) =
                 make_float4(o[r][c] * inv, o[r][c + 1] * inv, o[r][c + 2] * inv, o[r][c + 3] * inv);
     }
 }
 
-template <int D>
+template <int D, int RT>
 static int launch_f32_tile(const float* q, float* out, const int* cu_q, const int* tok_pos, const int* slots, KvSite<float> site,
                            int n_heads, int n_seqs, int max_q_len, float scale, int window, int* err, cudaStream_t stream) {
-    constexpr size_t smem = (size_t)(3 * 64 * (D + 4) + FT_ROWS * (QF_PAGE + 4)) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t smem = (size_t)((16 * RT + 2 * QF_PAGE) * (D + 4) + 16 * RT * (QF_PAGE + 4)) * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<D, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    attention_f32_tile_kernel<D><<<dim3(n_heads, (max_q_len + FT_ROWS - 1) / FT_ROWS, n_seqs), FT_THREADS, smem, stream>>>(
+    const int rows = max_q_len * (n_heads / site.kv_heads);
+    attention_f32_tile_kernel<D, RT><<<dim3(site.kv_heads, (rows + 16 * RT - 1) / (16 * RT), n_seqs), FT_THREADS, smem, stream>>>(
         q, out, cu_q, tok_pos, slots, site, n_heads, scale, window, err);
     return (int)cudaGetLastError();
 }
@@ -527,11 +536,16 @@ QF_EXPORT int qf_attention_generic_biased(int is_bf16, const void* q, void* out,
     if (!bias_scale != !bias_rate) return (int)cudaErrorInvalidValue;
     // the plain float32 form of the sizes the tile kernel is made for, wherever more than one token stands in its tiles
     if (!is_bf16 && (head_dim == 64 || head_dim == 128) && max_q_len > 1 && !sinks && !shared_values && chunk <= 0 && !(softcap > 0.f) &&
-        pool <= 0 && !bias_scale && kv_heads > 0 && n_heads % kv_heads == 0 && max_q_len <= 65535 * FT_ROWS && n_seqs <= 65535 && page_elems % 4 == 0 &&
-        (((uintptr_t)q | (uintptr_t)out | (uintptr_t)base) & 15) == 0) {
+        pool <= 0 && !bias_scale && kv_heads > 0 && n_heads % kv_heads == 0 && (long long)max_q_len * (n_heads / kv_heads) <= 65535ll * 64 && n_seqs <= 65535 &&
+        page_elems % 4 == 0 && (((uintptr_t)q | (uintptr_t)out | (uintptr_t)base) & 15) == 0) {
         const KvSite<float> site{(float*)base, table, page_elems, table_stride, kv_heads, head_dim};
-        return head_dim == 64 ? launch_f32_tile<64>((const float*)q, (float*)out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, stream)
-                              : launch_f32_tile<128>((const float*)q, (float*)out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, stream);
+        // sequences of few rows in tiles of 16 (the same bits): 64 of two tokens from position 0, 14 kv heads of 64: 40 -> 13 microseconds
+        const bool few = (long long)max_q_len * (n_heads / kv_heads) <= 16;
+#define QF_F32_TILE(D, RT) \
+    launch_f32_tile<D, RT>((const float*)q, (float*)out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, stream)
+        if (head_dim == 64) return few ? QF_F32_TILE(64, 1) : QF_F32_TILE(64, 4);
+        return few ? QF_F32_TILE(128, 1) : QF_F32_TILE(128, 4);
+#undef QF_F32_TILE
     }
     QF_GENERIC_DISPATCH(launch, q, out, cu_q, tok_pos, slots, base, table, page_elems, table_stride, kv_heads, head_dim,
                         n_heads, n_seqs, max_q_len, scale, window, err, sinks, shared_values, chunk, softcap, blocks_base,

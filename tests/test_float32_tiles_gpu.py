@@ -79,3 +79,27 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_row():
         outs.append(out.view(n, heads, dim))
     for out in outs[1:]:
         assert torch.equal(out[:bad], outs[0][:bad]) and not bool(torch.isfinite(out[bad:, :, 5]).any())
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(14, 2, 64), (3, 3, 128), (8, 2, 128), (40, 2, 64)])
+def test_short_sequences_alone_and_beside_long_ones(heads, kv_heads, dim):
+    """Rows in tiles of 16 and of 64 (a step of few tokens, the same beside a longer sequence): the same bits."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(heads)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    storage = torch.randn(12, 2, kv_heads, 64, dim, generator=g, device=DEV)
+    site, err = ops.KvSiteArgs(storage, ints([[0, 1, 2, 3], [4, 5, 6, 7], [8, 9, 10, 11]]), kv_heads, dim), ints([0])
+    spans = [(130, 2), (50, 150), (0, 5)]
+    cu, pos = [0], []
+    for start, n in spans:
+        cu.append(cu[-1] + n)
+        pos += range(start, start + n)
+    q = torch.randn(cu[-1], heads * dim, generator=g, device=DEV)
+    out = torch.empty_like(q)
+    ops.attention_generic(q, out, ints(cu), ints(pos), ints([0, 1, 2]), site, heads, 3, 150, dim ** -0.5, 0, err)
+    for s, (start, n) in enumerate(spans):
+        rows = slice(cu[s], cu[s + 1])
+        alone = torch.empty(n, heads * dim, device=DEV)
+        ops.attention_generic(q[rows].contiguous(), alone, ints([0, n]), ints(pos[rows]), ints([s]), site, heads, 1, n, dim ** -0.5, 0, err)
+        assert torch.equal(alone, out[rows])
+    assert int(err) == 0
