@@ -1,7 +1,7 @@
 // The prompt attention of attention_prefill_tc.cu (included there) with small blocks, head size 64: one tile of 128 rows and one page
-// (64 keys) a turn, 64 KB of shared memory and 128 columns of tensor memory, so three blocks fit an SM. A turn costs more than in the
-// kernel of that file, but up to 444 blocks are at work at once: a prompt of one to two thousand tokens, whose tiles are too many
-// for one block per SM and too few for two rounds of them, is done in one round (`pages_pay` says which steps).
+// (64 keys) a turn, 65 KB of shared memory and 128 columns of tensor memory, so three blocks fit an SM. A turn costs more than in the
+// kernel of that file, but up to 444 blocks are at work at once, finer grains for many tiles and for last rounds (`pages_time` says
+// which steps).
 //
 // A block serves 128 consecutive query tokens of one (sequence, query head). Thread t of its first four warps owns
 // query row t, which is lane t of the block's tensor memory; one thread of a fifth warp issues every copy and every
@@ -433,11 +433,19 @@ static int launch_pages(const CUtensorMap& q_map, const CUtensorMap& kv_map, voi
                                    sinks, planes);
 }
 
-// Whether a step of `tiles` tiles of prompts from their first token on, the longest of `span` tokens, is done first by two small
-// blocks a tile (SPLIT). As a whole step inside a graph, 24 layers of 14 heads of 64, microseconds, this / the larger blocks: one
-// prompt of 800 tokens (98 tiles) 1,793 / 1,660, 1,024 (112) 1,738 / 1,764, 1,750 (196) 2,490 / 2,562, 2,048 (224) 2,545 / 2,648, 3,072
-// (336) 3,797 / 3,890, 3,584 (392) 4,366 / 4,495, 4,096 (448, more than three a SM) 5,252 / 4,960; 3 x 700 tokens 2,521 / 2,503,
-// 2 x 1,024 (224) 2,427 / 2,419. Behind a context the larger blocks win: 1,024 tokens behind 15,360, 174 / 117 a layer.
-static bool pages_pay(long long tiles, int span, int q_tiles, int sms) {
-    return tiles * 4 >= sms * 3 && tiles <= 3ll * sms && span >= 16 * QF_PAGE && span <= q_tiles * TA_BM;
+// How long small blocks take, in microseconds, and whether two of a cluster share a tile (`two`: chains of 16 pages and more, while the pairs
+// need no more than two rounds on the SMs). `live` tiles of an average sequence and head. A turn takes 0.95 with one block on an SM
+// and 1.45 with two or three, a block's ends 4; a last round that is not full takes its blocks' share of a round, or, the more
+// alike the chains are, a whole chain. Measured inside a graph, small blocks / the larger ones (of 1,188 shapes): 14 heads of 64, one prompt of 2,048 tokens 26.8 / 28.9, 4,096 78.7 / 61.1,
+// 8,192 199 / 227; eight of 300 12.5 / 16.7, 32 of 256 25.5 / 33.1, four of 2,048 63.9 / 66.7; 256 tokens behind 2,000 22.5 / 14.0,
+// eight of 300 behind 2,000 54.7 / 70.1, eight of 256 48.8 / 39.9; a window of 256 over 4,096 tokens 19.8 / 26.7.
+static float pages_time(float live, int n_heads, int n_seqs, int n_tokens, int span, int q_tiles, int sms, bool& two) {
+    const long long tiles = min((long long)q_tiles * n_seqs, (long long)n_tokens / TA_BM + n_seqs) * n_heads;
+    two = span >= 16 * QF_PAGE && tiles <= 3ll * sms;
+    const float share = two ? 2.f : 1.f, pages = (float)((span + QF_PAGE - 1) / QF_PAGE);
+    const float mean = (pages > 2 * q_tiles ? pages - q_tiles : 0.5f * pages + 0.5f) / share, longest = ceilf(pages / share);
+    const float room = 3.f * sms, blocks = live * n_heads * n_seqs * share, rounds = floorf(blocks / room), last = blocks / room - rounds;
+    const float turn = fminf(0.95f + 0.9f * last, 1.45f), alike = fmaxf(2.f * mean / longest - 1.f, 0.f);   // of the last round
+    const float end = last <= 0.f ? 0.f : rounds < 1.f ? longest * turn + 3.7f : (mean * turn + 3.7f) * fmaxf(last, 0.35f + 0.65f * alike);
+    return fmaxf(rounds * (mean * 1.45f + 4.f) + end, longest * 0.95f + 3.7f);
 }

@@ -22,7 +22,8 @@
 // rows and 64 keys a turn per block, two or three blocks per SM, weights through shared memory, a turn's hand-overs cost more
 // than its work: 22% of the special-function rate, 32% of the tensor cores'.) Measured so and now, microseconds: one prompt of
 // 8,192 tokens, 28 heads of 128: 856, 449 (1,072 TFLOP/s); 1,024 tokens behind 15,360, 16 heads of 128: 268, 144; one prompt of
-// 4,096 tokens, 14 heads of 64: 89, 64; of 2,048: 29, 30. Masked keys cost nothing behind the comparison (their score is
+// 4,096 tokens, 14 heads of 64: 89, 64. (At head size 64 many tiles are done first in the small blocks of
+// attention_prefill_page.cuh: `launch` chooses.) Masked keys cost nothing behind the comparison (their score is
 // -infinity), three-way maxima and two-way multiply-adds and additions take 640 instructions a row and turn to 400, and a warp
 // arrives once for its rows: 642 -> 1,072 TFLOP/s together. (A quarter or half of the exponentials by a polynomial on the
 // multiply-add pipe, and the exponentials of 16 to 64 weights laid out one after another, made no difference.)
@@ -507,26 +508,33 @@ static int launch(const void* q, void* out, const int* cu_q, const int* tok_pos,
     // behind 8,000: 99, 115, 63, [25]; 64 behind 8,000, 16 heads of 128: 112, 127, 71, [31]; four prompts of 183 to 275: [7.2], 9.1, 10, 53.
     const int span = window > 0 && window + TA_BM < max_kv_len ? window + TA_BM : max_kv_len;
     const float longest = (float)((span + TA_BK - 1) / TA_BK), mean = longest > q_tiles ? longest - 0.5f * q_tiles : 0.5f * longest + 0.5f;
-    // (tiles that hold rows: the grid also has blocks for the rows that shorter sequences lack, which end at once. Every sequence has one,
-    // and half of a last one is counted on average)
-    const long long live = min((long long)q_tiles * n_seqs, max((2ll * n_tokens + (long long)TA_BM * n_seqs + TA_BM - 1) / (2 * TA_BM), (long long)n_seqs)) * n_heads;
+    // Tiles that hold rows, of an average sequence and query head (the grid also has blocks for the rows that shorter sequences lack, which
+    // end at once): the longest sequence, and the others as long as what is left.
+    const float rest = n_seqs > 1 ? fmaxf((float)(n_tokens - max_q_len) / (float)(n_seqs - 1), 1.f) : 0.f;
+    const float live = (q_tiles + (n_seqs - 1) * fminf((float)q_tiles, ceilf(rest / TA_BM))) / (float)n_seqs;
     const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
-    if (D == 64 && pages_pay(live, span, q_tiles, sms))
-        return launch_pages<true>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, sinks,
-                                  planes, stream);
     const float turn[2] = {D <= 64 ? 1.5f : 1.75f, D <= 64 ? 1.85f : 2.05f}, ends[2][4] = {{3.f, 5.f, 5.5f, 6.5f}, {5.f, 6.5f, 9.f, 13.f}};
     const int room[4] = {sms, sms, sms - sms / 8, sms * 77 / 100 > 0 ? sms * 77 / 100 : 1};
-    const float units = (float)live / ((float)n_seqs * kv_heads);   // tiles of an average sequence and kv head: a block takes two of the same
+    // Blocks of one tile and of two: the tiles of a sequence and kv head go in pairs, of which an odd count leaves half a block.
+    const int group = n_heads / kv_heads;
+    const float pairs = n_seqs == 1 ? ceilf(live * group / 2) : fmaxf(live * group / 2 + (group & 1 ? 0.25f : 0.f), (float)((group + 1) / 2));
+    const float count[2] = {live * n_heads * n_seqs, pairs * kv_heads * n_seqs};
     int per = 2, split = 1;
     float least = -1.f;
     for (int p = 2; p >= 1; --p)
         for (int n = 0; n < 4; ++n) {
-            const long long blocks = (long long)n_seqs * kv_heads * (long long)ceilf(units / p - 0.01f) << n;
+            const long long blocks = (long long)ceilf(count[p - 1] - 0.01f) << n;
             const float alone = ceilf(longest / (1 << n)) * turn[p - 1] + ends[p - 1][n];
             const float all = (float)((blocks + room[n] - 1) / room[n]) * (mean / (1 << n) * turn[p - 1] + ends[p - 1][n]);
             const float time = alone > all ? alone : all;
             if (least < 0.f || time < least) least = time, per = p, split = 1 << n;
         }
+    if (D == 64) {   // (in favour of the small blocks by what the estimates are uncertain of, less where every chain is alike)
+        bool two;
+        if ((q_tiles > 1 ? 0.85f : 0.95f) * pages_time(live, n_heads, n_seqs, n_tokens, span, q_tiles, sms, two) <= least)
+            return two ? launch_pages<true>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, sinks, planes, stream)
+                       : launch_pages<false>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, sinks, planes, stream);
+    }
 #define QF_TC_LAUNCH(SPLIT, PER) \
     launch_variant<D, SPLIT, PER>(q_map, kv_map, out, cu_q, tok_pos, slots, site, n_heads, n_seqs, tiles, scale, window, err, sinks, planes, stream)
     if (per == 1) return split == 1 ? QF_TC_LAUNCH(1, 1) : split == 2 ? QF_TC_LAUNCH(2, 1) : split == 4 ? QF_TC_LAUNCH(4, 1) : QF_TC_LAUNCH(8, 1);

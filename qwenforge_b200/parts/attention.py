@@ -70,7 +70,7 @@ TC_PREFILL_MIN_KEYS = 128
 # tokens a sequence, 64 sequences behind 127 tokens 14 / 30, behind 1,000 53 / 70, behind 3,000 146 / 176; 32 behind 127 8 / 16,
 # behind 500 15 / 23, behind 3,000 99 / 89; 28 heads of 128: 32 sequences behind 127 27 / 34, behind 500 60 / 50. Below one round the
 # tcgen05 kernel loses only where up to 16 tokens see up to three pages (14 heads of 64, 16 sequences of 2 behind 127: 7 / 9).
-SHORT_SEQUENCES = {64: (0.0036, 0.006, 1.85, 5.0), 128: (0.0070, 0.007, 2.05, 6.5)}
+SHORT_SEQUENCES = {64: (0.0031, 0.005, 1.85, 5.0), 128: (0.0070, 0.007, 2.05, 6.5)}
 
 
 def prefill_attention(head_dim: int, n_tokens: int, max_kv_len: int, window: int = 0, *, max_q_len: int = 0, n_seqs: int = 1,
