@@ -525,7 +525,9 @@ static int launch(const void* q, void* out, const int* cu_q, const int* tok_pos,
         for (int n = 0; n < 4; ++n) {
             const long long blocks = (long long)ceilf(count[p - 1] - 0.01f) << n;
             const float alone = ceilf(longest / (1 << n)) * turn[p - 1] + ends[p - 1][n];
-            const float all = (float)((blocks + room[n] - 1) / room[n]) * (mean / (1 << n) * turn[p - 1] + ends[p - 1][n]);
+            // (of several sequences the count is an estimate itself: a twentieth more than a round is taken for one)
+            const long long rounds = n_seqs > 1 && blocks * 20 <= room[n] * 21ll ? 1 : (blocks + room[n] - 1) / room[n];
+            const float all = (float)rounds * (mean / (1 << n) * turn[p - 1] + ends[p - 1][n]);
             const float time = alone > all ? alone : all;
             if (least < 0.f || time < least) least = time, per = p, split = 1 << n;
         }
