@@ -42,17 +42,14 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                   const int* __restrict__ slots, KvSite<bf16> site, int n_heads, int n_seqs, int row_tiles, int wave,
                   float scale_log2, int window, int* err, const float* __restrict__ sinks, int planes) {
     constexpr int D = 64;
-    constexpr int CB = D / 64;                    // blocks of 64 columns in a row of Q, K or V
-    constexpr int Q_BLOCK = TA_BM * 128;          // bytes of one [128][64] block of Q
-    constexpr int KV_BLOCK = QF_PAGE * 128;       // bytes of one [64][64] block of a page's keys or values
-    constexpr int KV_BYTES = CB * KV_BLOCK;
-    constexpr int TMEM_COLS = D == 64 ? 128 : 256;  // S in columns 0..63, PV in columns 64..64 + D - 1
-    constexpr int PV_COL = 64;
+    constexpr int Q_BYTES = TA_BM * 128;          // the tile of Q, [128][64]
+    constexpr int KV_BYTES = QF_PAGE * 128;       // a page's keys or values, [64][64]
+    constexpr int TMEM_COLS = 128, PV_COL = 64;   // S in columns 0..63, O in columns 64..127
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
-    unsigned char* q_s = smem;                          // [CB][128][64]
-    unsigned char* k_s = q_s + CB * Q_BLOCK;            // [2][CB][64][64]
-    unsigned char* v_s = k_s + 2 * KV_BYTES;            // [2][CB][64][64]
+    unsigned char* q_s = smem;                          // [128][64]
+    unsigned char* k_s = q_s + Q_BYTES;                 // [2][64][64]
+    unsigned char* v_s = k_s + 2 * KV_BYTES;            // [2][64][64]
     unsigned char* p_s = v_s + 2 * KV_BYTES;            // [128][64]
     // SPLIT: [D + 2][128] of the cluster's second block (a warp writes 32 neighbouring rows at once). It lies over Q and the pages' stages, which are free when both
     // blocks have left their loops (the first barrier of the cluster below).
@@ -142,17 +139,14 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                 const long long v_row = planes == 2 ? k_row + (long long)site.kv_heads * QF_PAGE : k_row;
                 if (leader) {
                     mbar_expect_tx(&bar_kv[stage], 2 * KV_BYTES);
-#pragma unroll
-                    for (int cb = 0; cb < CB; ++cb) {
-                        tma_load_2d(k_s + stage * KV_BYTES + cb * KV_BLOCK, &kv_map, cb * 64, (int)k_row, &bar_kv[stage]);
-                        tma_load_2d(v_s + stage * KV_BYTES + cb * KV_BLOCK, &kv_map, cb * 64, (int)v_row, &bar_kv[stage]);
-                    }
+                    tma_load_2d(k_s + stage * KV_BYTES, &kv_map, 0, (int)k_row, &bar_kv[stage]);
+                    tma_load_2d(v_s + stage * KV_BYTES, &kv_map, 0, (int)v_row, &bar_kv[stage]);
                 }
                 __syncwarp();
             };
             // descriptors: an address field counts 16 bytes, so 16 columns of a K-major row (32 bytes) are 2 units
             const uint64_t desc_q = smem_desc_sw128(q_s), desc_p = smem_desc_sw128(p_s);
-            const uint64_t desc_k = smem_desc_sw128(k_s), desc_v = smem_desc_mn_sw128(v_s, KV_BLOCK);
+            const uint64_t desc_k = smem_desc_sw128(k_s), desc_v = smem_desc_mn_sw128(v_s, KV_BYTES);
             constexpr uint32_t idesc_s = umma_idesc_bf16(TA_BM, QF_PAGE, false), idesc_pv = umma_idesc_bf16(TA_BM, D, true);
             auto issue_s = [&](int j) {  // S = Q K^T of page j; false if its keys did not arrive
                 if (!wait_all(&bar_kv[j & 1], (j >> 1) & 1)) return false;
@@ -161,17 +155,15 @@ prefill_page_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                 if (leader) {
 #pragma unroll
                     for (int ks = 0; ks < D / 16; ++ks)
-                        umma_bf16(tmem, desc_q + (uint64_t)((ks / 4) * (Q_BLOCK >> 4) + 2 * (ks % 4)),
-                                  dk + (uint64_t)((ks / 4) * (KV_BLOCK >> 4) + 2 * (ks % 4)), idesc_s, ks > 0 ? 1u : 0u);
+                        umma_bf16(tmem, desc_q + (uint64_t)(2 * ks), dk + (uint64_t)(2 * ks), idesc_s, ks > 0 ? 1u : 0u);
                     umma_commit(&bar_s);
                 }
                 __syncwarp();
                 return true;
             };
             if (leader && n_tiles > 0) {
-                mbar_expect_tx(&bar_q, CB * Q_BLOCK);
-#pragma unroll
-                for (int cb = 0; cb < CB; ++cb) tma_load_2d(q_s + cb * Q_BLOCK, &q_map, head * D + cb * 64, q_begin + row0, &bar_q);
+                mbar_expect_tx(&bar_q, Q_BYTES);
+                tma_load_2d(q_s, &q_map, head * D, q_begin + row0, &bar_q);
             }
             __syncwarp();
             if (n_tiles > 0) fetch_page(0);
@@ -405,8 +397,7 @@ template <bool SPLIT>
 static int launch_pages(const CUtensorMap& q_map, const CUtensorMap& kv_map, void* out, const int* cu_q, const int* tok_pos,
                           const int* slots, KvSite<bf16> site, int n_heads, int n_seqs, int max_q_len, float scale, int window,
                           int* err, const float* sinks, int planes, cudaStream_t stream) {
-    constexpr int D = 64;
-    constexpr size_t smem = (size_t)(D / 64) * TA_BM * 128 + 4 * (size_t)(D / 64) * QF_PAGE * 128 + TA_BM * 128 + 1024;
+    constexpr size_t smem = TA_BM * 128 + 4 * QF_PAGE * 128 + TA_BM * 128 + 1024;   // Q, two stages of keys and values, the weights
     static_assert(qf_tmem_fits(128, smem), "the rule of tcgen05.cuh");
     auto kernel = prefill_page_kernel<SPLIT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

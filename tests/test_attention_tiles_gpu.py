@@ -52,6 +52,13 @@ def test_against_float64(lens, before, heads, kv_heads, dim, window, with_sinks)
             assert float((got - want).norm() / want.norm()) < 2 ** -8
 
 
+@pytest.mark.parametrize("lens,before,heads,kv_heads,window", [([300] * 8, 0, 14, 2, 0), ([257, 130, 1] * 8, 0, 14, 14, 0), ([4100], 0, 14, 2, 256),
+                                                              ([200] * 20, 70, 16, 4, 0), ([129, 300] * 9, 700, 12, 2, 0)])
+def test_small_blocks_alone_and_in_pairs(lens, before, heads, kv_heads, window):
+    """Steps of many tiles at head size 64, which small blocks take: a tile each below 16 pages or beyond two rounds of them, else in pairs."""
+    test_against_float64(lens, before, heads, kv_heads, 64, window, True)
+
+
 @pytest.mark.parametrize("n,before,heads,kv_heads,dim,window", [(300, 0, 5, 5, 64, 0), (300, 0, 3, 1, 128, 0), (700, 130, 6, 2, 64, 0), (64, 3000, 2, 2, 128, 0),
                                                                (400, 700, 4, 4, 64, 150), (400, 690, 4, 4, 128, 200), (130, 4000, 5, 5, 64, 3000), (1153, 0, 16, 2, 64, 0)])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
