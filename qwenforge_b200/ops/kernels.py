@@ -1839,10 +1839,10 @@ def _chunks_pay(n: int, n_seqs: int, longest: int, state: int, chunk: int, scan:
 
 
 STATE_CHUNK = 128   # SC_CHUNK of csrc/state_chunks.cu
-# The longest sequence of a step from which the chunked form is the faster one. Measured, one sequence, scan / chunks in microseconds:
-# 16 heads of 64 x 128: 96 tokens 14 / 13, 160: 26 / 15, 256: 41 / 17, 2,048: 315 / 42; 32 heads of 128 x 128: 96 tokens 23 / 20,
-# 160: 37 / 24. Three launches and a buffer instead of one launch cost the host about 10 microseconds more, which a step that is
-# issued launch by launch feels up to some 200 tokens.
+# The longest sequence of a step from which the chunked form is the faster one. Measured inside a graph, one sequence, scan / chunks in
+# microseconds: 7 heads of 64 x 128: 192 tokens 21 / 18, 256: 28 / 18, 2,048: 200 / 30; 16 heads 23 / 23, 29 / 23, 214 / 41; 32 heads of
+# 128 x 128: 43 / 32, 57 / 32, 427 / 104. Three launches and a buffer instead of one launch cost the host about 10 microseconds more,
+# which a step that is issued launch by launch feels up to some 200 tokens.
 STATE_CHUNKS_MIN_TOKENS = 192
 # Beside other sequences (`_chunks_pay`), inside a graph, scan / chunks: 7 heads of 64 x 128: 192 + 31 x 1 tokens 24 / 41, 512 + 31 x 1
 # 55 / 43, 64 x 512 738 / 214; 16 heads: 512 + 31 x 1 69 / 78; 32 heads of 128 x 128: 192 43.8 / 31.0, 192 + 63 x 1 250 / 505,
@@ -2335,9 +2335,9 @@ def outer_state_scan_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dec
 
 ROW_CHUNK = 64   # RC_CHUNK of csrc/row_chunks.cu
 # The longest sequence of a step from which the chunked form is the faster one however the step is issued. Inside a graph, one sequence,
-# scan / chunks in microseconds, 16 heads of 64 x 128: 128 tokens 23 / 33, 200: 35 / 34, 512: 83 / 36, 1,031: 164 / 52; 7 heads: 200
-# tokens 29 / 31, 512: 67 / 34. A step issued launch by launch waits for the host up to some 550 tokens, and two launches and a
-# buffer more cost it 5 of 103 microseconds.
+# scan / chunks in microseconds, 16 heads of 64 x 128: 512 tokens 78 / 37, 1,024: 143 / 53; 7 heads: 512 tokens 68 / 32, 1,024: 133 / 39
+# (the forms meet at about 200 tokens there). A step issued launch by launch waits for the host up to some 550 tokens, and two
+# launches and a buffer more cost it 5 of 103 microseconds.
 ROW_CHUNKS_MIN_TOKENS = 512
 # Beside other sequences (`_chunks_pay`), inside a graph, scan / chunks: 7 heads of 64 x 128: 512 + 31 x 1 tokens 71 / 60, 512 + 63 x 1
 # 77 / 93, 64 x 512 1,235 / 598; 16 heads: 512 + 31 x 1 89 / 109, 1,024 + 31 x 1 173 / 138; 32 heads of 64 x 64: 1,024 + 63 x 1
