@@ -262,8 +262,7 @@ def measure_attention(args) -> None:
         variants = [("mma.sync, a tile's pages by one group of warps", ops.attention_prefill, 64),
                     ("mma.sync, as the model runs it", ops.attention_prefill, n)]
         if d in ops.TC_ATTENTION_HEAD_DIMS:
-            variants += [("tcgen05, one block per tile", ops.attention_prefill_tc, 64),
-                         ("tcgen05, as the model runs it", ops.attention_prefill_tc, n)]
+            variants += [("tcgen05, as the model runs it", ops.attention_prefill_tc, n)]
         for name, fn, bound in variants:
             run = lambda: fn(q, out, cu, pos, slots, pages.args(), heads, 1, n, d ** -0.5, 0, err, max_kv_len=bound)
             for _ in range(3):
