@@ -9,7 +9,7 @@
 // through shared memory in tiles of 32 positions whose origin is always a multiple of 32, so the
 // order of every row's arithmetic depends only on that row's own position and window: results
 // are bitwise independent of what else is in the batch and of how the tokens were cut into steps.
-// (Steps of several tokens of the plain float32 form run on a tile kernel with the same property, below.)
+// (The plain float32 form at head sizes 64 and 128 runs on a tile kernel with the same property, below.)
 //
 // Query i at position p sees keys j with max(0, p - window + 1) <= j <= p (window 0: all j <= p); with `chunk` > 0 also
 // only the keys of its own block of `chunk` positions, j >= floor(p / chunk) * chunk (blocks counted from position 0 of
@@ -259,7 +259,7 @@ __global__ void attention_generic_fold_kernel(T* __restrict__ out, const int* __
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// The plain form (no option but a window) of float32 steps of several tokens, head sizes 64 and 128: a block serves 16 * RT rows of
+// The plain form (no option but a window) of float32 steps, head sizes 64 and 128: a block serves 16 * RT rows of
 // one kv head (a row is a token and a query head of the group, the heads of a token neighbours) and walks the keys a page at a
 // time; its 16 x 16 threads hold RT rows x 4 keys of the scores, then RT rows x D / 16 columns of the output, so that with RT = 4
 // a load from shared memory feeds four multiply-adds (in the kernel above: one). Every score is one chain over the components,
@@ -534,8 +534,9 @@ QF_EXPORT int qf_attention_generic_biased(int is_bf16, const void* q, void* out,
                                           const int* blocks_table, long long blocks_page_elems, int blocks_table_stride, int pool,
                                           const float* bias_scale, const float* bias_rate, cudaStream_t stream) {
     if (!bias_scale != !bias_rate) return (int)cudaErrorInvalidValue;
-    // the plain float32 form of the sizes the tile kernel is made for, wherever more than one token stands in its tiles
-    if (!is_bf16 && (head_dim == 64 || head_dim == 128) && max_q_len > 1 && !sinks && !shared_values && chunk <= 0 && !(softcap > 0.f) &&
+    // the plain float32 form of the sizes the tile kernel is made for (also of single tokens: a row's bits are the same beside a longer
+    // sequence; single tokens with many keys take the chunks of qf_attention_generic_decode_biased)
+    if (!is_bf16 && (head_dim == 64 || head_dim == 128) && max_q_len > 0 && !sinks && !shared_values && chunk <= 0 && !(softcap > 0.f) &&
         pool <= 0 && !bias_scale && kv_heads > 0 && n_heads % kv_heads == 0 && (long long)max_q_len * (n_heads / kv_heads) <= 65535ll * 64 && n_seqs <= 65535 &&
         page_elems % 4 == 0 && (((uintptr_t)q | (uintptr_t)out | (uintptr_t)base) & 15) == 0) {
         const KvSite<float> site{(float*)base, table, page_elems, table_stride, kv_heads, head_dim};

@@ -87,16 +87,16 @@ def test_short_sequences_alone_and_beside_long_ones(heads, kv_heads, dim):
     from qwenforge_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(heads)
     ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
-    storage = torch.randn(12, 2, kv_heads, 64, dim, generator=g, device=DEV)
-    site, err = ops.KvSiteArgs(storage, ints([[0, 1, 2, 3], [4, 5, 6, 7], [8, 9, 10, 11]]), kv_heads, dim), ints([0])
-    spans = [(130, 2), (50, 150), (0, 5)]
+    storage = torch.randn(20, 2, kv_heads, 64, dim, generator=g, device=DEV)
+    site, err = ops.KvSiteArgs(storage, ints([list(range(4 * i, 4 * i + 4)) for i in range(5)]), kv_heads, dim), ints([0])
+    spans = [(130, 2), (50, 150), (0, 5), (200, 1), (0, 1)]
     cu, pos = [0], []
     for start, n in spans:
         cu.append(cu[-1] + n)
         pos += range(start, start + n)
     q = torch.randn(cu[-1], heads * dim, generator=g, device=DEV)
     out = torch.empty_like(q)
-    ops.attention_generic(q, out, ints(cu), ints(pos), ints([0, 1, 2]), site, heads, 3, 150, dim ** -0.5, 0, err)
+    ops.attention_generic(q, out, ints(cu), ints(pos), ints([0, 1, 2, 3, 4]), site, heads, 5, 150, dim ** -0.5, 0, err)
     for s, (start, n) in enumerate(spans):
         rows = slice(cu[s], cu[s + 1])
         alone = torch.empty(n, heads * dim, device=DEV)
