@@ -294,24 +294,34 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// The persistent form, for products of many tiles: one block per SM walks tiles of 128 x 256 (tile index = block,
-// block + blocks, ...; neighbouring blocks work on the same 256 weight rows, which the L2 then serves). The ring of
-// stages runs on across tiles, and the accumulator is double: while the tensor cores fill one half of tensor memory
-// (256 columns) with a tile's sums, eight epilogue warps read the other half, so a tile's epilogue and the start of
-// the next tile's copies hide under products. Warp 0 issues copies, warp 1 products, warps 2 to 9 own the epilogue:
-// warp w reads accumulator lanes 32 (w % 4) .. + 31 (the lanes a warp may read are fixed by its number) and one half
-// of the tile's columns.
+// The persistent form, for products of many tiles: pairs of SMs walk tiles of 256 x BN (tile index = pair, pair + pairs, ...;
+// neighbouring pairs work on the same weight rows, which the L2 then serves). A pair is a cluster of two blocks, each of
+// which brings 128 rows of A and BN / 2 rows of W per stage; one thread of its first block issues the products of both
+// (tcgen05.mma, cta_group::2: 256 x BN x 16), which read the two blocks' shared memory, and each block's tensor memory gets
+// the sums of its own 128 rows. The ring of stages runs on across tiles, and the accumulator is double: while the tensor
+// cores fill one half of tensor memory with a tile's sums, eight epilogue warps read the other half, so a tile's epilogue and
+// the start of the next tile's copies hide under products. Warp 0 issues copies, warp 1 of the first block products, warps 2
+// to 9 own the epilogue: warp w reads accumulator lanes 32 (w % 4) .. + 31 (the lanes a warp may read are fixed by its number)
+// and one half of the tile's columns. The launch is a programmatic dependent one: barriers and tensor memory are set up under
+// the tail of the kernel before (a 905-token prompt of 24 layers: 1,548 -> 1,512 microseconds).
+// What bounds it: at large K the tensor cores (7358 x 22016 x 2048: 413 microseconds, 1,608 TFLOP/s; one block a tile of 128 x 256,
+// which reads 1.5 times the bytes from the L2 per product, took 476); at K = 896 the tiles' last round and 1.5 microseconds a
+// tile that the ring takes to fill and the sums to drain (2048 x 9728 x 896 with the gate: 31 microseconds, 36 before).
+// (The first tile's weights asked for before the wait for the kernel ahead: 1,528 instead of 1,512. Not kept.)
 #define TP_THREADS 320
 #define TP_EPI_WARPS 8
-#define TP_BN 256
-#define TP_STAGES 4
-#define TP_STAGE_BYTES ((TC_BM + TP_BN) * TC_BK * 2)
+template <int BN> struct PairGeometry {   // BN 256 or 192: six or seven stages
+    static constexpr int stage_bytes = (TC_BM + BN / 2) * TC_BK * 2;
+    static constexpr int stages = BN == 256 ? 6 : 7;
+    static constexpr size_t smem = (size_t)stages * stage_bytes + 1024;
+    static_assert(qf_tmem_fits(512, smem), "the rule of tcgen05.cuh");
+};
 
 __device__ __forceinline__ float fast_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 
-// Tile t of the persistent walk. The blocks of the grid work on neighbouring t at any time, so the order decides what
+// Tile t of the persistent walk. The pairs of the grid work on neighbouring t at any time, so the order decides what
 // the L2 holds: tiles go by groups of `group_n` column tiles (their weight rows together fit in a quarter of the L2),
-// and inside a group the column runs fastest, so that the blocks at work share a few row tiles of A and the group's
+// and inside a group the column runs fastest, so that the pairs at work share a few row tiles of A and the group's
 // weights, A streams through once per group, and the weights are read once. (With the row tile running fastest over
 // the whole matrix, A was read again for every column tile once it outgrew the L2: 838 instead of 330 milliseconds
 // for a 32,768-token step at Qwen2.5-7B sizes.)
@@ -322,104 +332,127 @@ __device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles, int gro
     tile_n = first + local % width;
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(TP_THREADS, 1)
-tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                          bf16* __restrict__ out, int M, int n_out, int K, int inter, int ldo, int m_tiles, int n_tiles, int group_n,
-                          int* err) {
+// Eight neighbouring results of a row (n_out is a multiple of eight: a piece is whole or beyond the matrix).
+__device__ __forceinline__ void store_8(bf16* dst, const uint32_t* packed) {
+    *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+}
+
+template <int EPI, int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
+tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                    bf16* __restrict__ out, int M, int n_out, int K, int inter, int ldo, int m_tiles, int n_tiles, int group_n,
+                    int* err) {
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
-    constexpr int HALF = TP_BN / 2;  // TC_SWIGLU: gate columns [0, HALF), up columns [HALF, BN)
-    __shared__ __align__(8) uint64_t full_bar[TP_STAGES], empty_bar[TP_STAGES], acc_full[2], acc_empty[2];
+    constexpr int STAGES = PairGeometry<BN>::stages, STAGE_BYTES = PairGeometry<BN>::stage_bytes;
+    constexpr int HALF = BN / 2;      // the columns whose weight rows a block brings; TC_SWIGLU: gate columns [0, HALF), up columns [HALF, BN)
+    __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
     const int n_k = (K + TC_BK - 1) / TC_BK, total = m_tiles * n_tiles;
 
+    // Both blocks' copies of a stage arrive at the first block's full_bar (one arrival, which announces both blocks' bytes); a
+    // stage's and a tile's end are told to both blocks' empty_bar and acc_full; all sixteen epilogue warps arrive at the
+    // first block's acc_empty.
     if (threadIdx.x == 0) {
-        for (int s = 0; s < TP_STAGES; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], TP_EPI_WARPS);
+            mbar_init(&acc_empty[b], 2 * TP_EPI_WARPS);
         }
     }
-    if (warp == 0) {  // both accumulators: all 512 columns of tensor memory
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_s)), "r"(2 * TP_BN));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    if (warp == 0) {  // both accumulators: all 512 columns of either block's tensor memory
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_s)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();                   // the other block's barriers and tensor memory are there too
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
     bool timed_out = false;
+    grid_launch_dependents();         // (this kernel has its tensor memory)
 
     if (warp == 0) {
         // ---- copies: all lanes run the loops, one issues
         const bool leader = elect_one();
-        int it = 0;
-        for (int t = blockIdx.x; t < total && !timed_out; t += gridDim.x) {
+        const uint32_t full0 = cluster_addr(full_bar, 0);
+        int s = 0, issued = 0;
+        uint32_t turn = 0;            // of the ring: its parity is that of the stage's copies in hand
+        grid_dependency_wait();
+        for (int t = pair; t < total && !timed_out; t += pairs) {
             int tile_m, tile_n;
             tile_of(t, m_tiles, n_tiles, group_n, tile_m, tile_n);
-            for (int kb = 0; kb < n_k; ++kb, ++it) {
-                const int s = it % TP_STAGES;
-                if (it >= TP_STAGES && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((it / TP_STAGES) - 1) & 1))) {
+            const int a_row = (2 * tile_m + (int)rank) * TC_BM;
+            // the first block brings the tile's first half of weight rows (TC_SWIGLU: the gate rows), the second the other (the up rows)
+            const int w_row = EPI == TC_SWIGLU ? (int)rank * inter + tile_n * HALF : tile_n * BN + (int)rank * HALF;
+            for (int kb = 0; kb < n_k; ++kb) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], (turn & 1) ^ 1))) {   // (true at once in the first turn)
                     timed_out = true;
                     break;
                 }
                 if (leader) {
-                    unsigned char* a_s = smem + (size_t)s * TP_STAGE_BYTES;
-                    unsigned char* b_s = a_s + TC_BM * TC_BK * 2;
-                    mbar_expect_tx(&full_bar[s], TP_STAGE_BYTES);
-                    tma_load_2d(a_s, &map_a, kb * TC_BK, tile_m * TC_BM, &full_bar[s]);
-                    // two boxes of 128 weight rows: the tile's halves, or HALF gate rows and the HALF matching up rows
-                    const int w_row0 = EPI == TC_SWIGLU ? tile_n * HALF : tile_n * TP_BN;
-                    const int w_row1 = EPI == TC_SWIGLU ? inter + tile_n * HALF : tile_n * TP_BN + HALF;
-                    tma_load_2d(b_s, &map_b, kb * TC_BK, w_row0, &full_bar[s]);
-                    tma_load_2d(b_s + (size_t)HALF * TC_BK * 2, &map_b, kb * TC_BK, w_row1, &full_bar[s]);
+                    unsigned char* a_s = smem + (size_t)s * STAGE_BYTES;
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
+                    tma_load_2d_pair(a_s, &map_a, kb * TC_BK, a_row, full0 + 8 * s);
+                    tma_load_2d_pair(a_s + TC_BM * TC_BK * 2, &map_b, kb * TC_BK, w_row, full0 + 8 * s);
                 }
                 __syncwarp();
+                if (issued < STAGES) ++issued;
+                if (++s == STAGES) s = 0, ++turn;
             }
         }
-    } else if (warp == 1) {
-        // ---- products
+        // what is on its way into either block has arrived before they end (as far as a bounded wait can say): the last stages'
+        // releases, or after a wait that ran out the copies
+        for (; issued > 0; --issued) {
+            if (--s < 0) s = STAGES - 1, --turn;
+            if (!timed_out) mbar_wait(&empty_bar[s], turn & 1);
+            else if (rank == 0) mbar_wait(&full_bar[s], turn & 1);
+        }
+    } else if (warp == 1 && rank == 0) {
+        // ---- products of both blocks
         const bool leader = elect_one();
-        int it = 0, i = 0;
-        for (int t = blockIdx.x; t < total && !timed_out; t += gridDim.x, ++i) {
+        int s = 0, i = 0;
+        uint32_t turn = 0;
+        for (int t = pair; t < total && !timed_out; t += pairs, ++i) {
             const int buf = i & 1;
-            if (i >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((i >> 1) - 1) & 1))) {  // the epilogue has read this half
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((i >> 1) & 1) ^ 1))) {  // both epilogues have read this half
                 timed_out = true;
                 break;
             }
             tc_fence_after();
-            const uint32_t acc = tmem + (uint32_t)(buf * TP_BN);
-            for (int kb = 0; kb < n_k; ++kb, ++it) {
-                const int s = it % TP_STAGES;
-                if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], (it / TP_STAGES) & 1))) {
+            const uint32_t acc = tmem + (uint32_t)(buf * 256);
+            for (int kb = 0; kb < n_k; ++kb) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], turn & 1))) {
                     timed_out = true;
                     break;
                 }
                 tc_fence_after();
                 if (leader) {
-                    const unsigned char* a_s = smem + (size_t)s * TP_STAGE_BYTES;
+                    const unsigned char* a_s = smem + (size_t)s * STAGE_BYTES;
                     const uint64_t da = smem_desc_sw128(a_s), db = smem_desc_sw128(a_s + TC_BM * TC_BK * 2);
 #pragma unroll
                     for (int k4 = 0; k4 < TC_BK / 16; ++k4)
-                        umma_bf16(acc, da + 2 * k4, db + 2 * k4, tc_idesc<TP_BN>(), (kb > 0 || k4 > 0) ? 1u : 0u);
-                    umma_commit(&empty_bar[s]);
+                        umma_bf16_pair(acc, da + 2 * k4, db + 2 * k4, umma_idesc_bf16(2 * TC_BM, BN, false), (kb > 0 || k4 > 0) ? 1u : 0u);
+                    umma_commit_pair(&empty_bar[s]);
                 }
                 __syncwarp();
+                if (++s == STAGES) s = 0, ++turn;
             }
             if (timed_out) break;
-            if (leader) umma_commit(&acc_full[buf]);  // arrives when the tile's products have finished
+            if (leader) umma_commit_pair(&acc_full[buf]);  // arrives when the tile's products have finished
             __syncwarp();
         }
-    } else {
+    } else if (warp >= 2) {
         // ---- epilogue
         const int quad = warp & 3, half = (warp - 2) >> 2;
         int i = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
+        for (int t = pair; t < total; t += pairs, ++i) {
             const int buf = i & 1;
             int tile_m, tile_n;
             tile_of(t, m_tiles, n_tiles, group_n, tile_m, tile_n);
@@ -428,77 +461,102 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 break;
             }
             tc_fence_after();
-            const int row = tile_m * TC_BM + quad * 32 + lane;
-            const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * TP_BN);
+            const int row = (2 * tile_m + (int)rank) * TC_BM + quad * 32 + lane;
+            const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 256);
             if (EPI == TC_SWIGLU) {
+                constexpr int W = HALF / 2 % 32 == 0 ? 32 : 16;   // columns a turn
 #pragma unroll
-                for (int c0 = half * (HALF / 2); c0 < (half + 1) * (HALF / 2); c0 += 32) {
-                    uint32_t g[32], u[32];
-                    tmem_load_32(lane_base + c0, g);
-                    tmem_load_32(lane_base + HALF + c0, u);
+                for (int c = 0; c < HALF / 2; c += W) {
+                    const int c0 = half * (HALF / 2) + c;
+                    uint32_t g[W], u[W];
+                    if constexpr (W == 32) {
+                        tmem_load_32(lane_base + c0, g);
+                        tmem_load_32(lane_base + HALF + c0, u);
+                    } else {
+                        tmem_load_16(lane_base + c0, g);
+                        tmem_load_16(lane_base + HALF + c0, u);
+                    }
                     const int col = tile_n * HALF + c0;
-                    if (row < M && col < n_out) {
-                        uint32_t packed[16];
+                    if (row < M) {
+                        uint32_t packed[W / 2];
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
+                        for (int j = 0; j < W / 2; ++j)
                             packed[j] = pack_bf16(fast_silu(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
                                                   fast_silu(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
                         bf16* dst = out + (size_t)row * ldo + col;
-                        if (col + 32 <= n_out) {
 #pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                *reinterpret_cast<uint4*>(dst + 8 * j) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-                        } else {
-                            for (int j = 0; j < n_out - col; ++j) dst[j] = reinterpret_cast<const bf16*>(packed)[j];
-                        }
+                        for (int j = 0; j < W / 8; ++j)
+                            if (col + 8 * j < n_out) store_8(dst + 8 * j, packed + 4 * j);
                     }
                 }
             } else {
 #pragma unroll
-                for (int c0 = half * HALF; c0 < (half + 1) * HALF; c0 += 32) {
+                for (int c = 0; c < HALF; c += 32) {
+                    const int c0 = half * HALF + c;
                     uint32_t v[32];
                     tmem_load_32(lane_base + c0, v);
-                    const int col = tile_n * TP_BN + c0;
-                    if (row < M && col < n_out) {
+                    const int col = tile_n * BN + c0;
+                    if (row < M) {
                         uint32_t packed[16];
 #pragma unroll
                         for (int j = 0; j < 16; ++j) packed[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
                         bf16* dst = out + (size_t)row * ldo + col;
-                        if (col + 32 <= n_out) {
 #pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                *reinterpret_cast<uint4*>(dst + 8 * j) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-                        } else {
-                            for (int j = 0; j < n_out - col; ++j) dst[j] = reinterpret_cast<const bf16*>(packed)[j];
-                        }
+                        for (int j = 0; j < 4; ++j)
+                            if (col + 8 * j < n_out) store_8(dst + 8 * j, packed + 4 * j);
                     }
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[buf]);  // this warp has read its part of the half
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));  // this warp has read its part of the half
         }
     }
     if (timed_out && lane == 0) atomicOr(err, QF_ERR_COPY_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32  %0, %1;" ::"r"(tmem), "r"(2 * TP_BN));
+    cluster_sync();                   // nothing of the other block's reaches into this one any more
+    tc_fence_after();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32  %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+template <int EPI, int BN>
+static int launch_pair(const CUtensorMap& map_a, const void* w, int w_rows, int ldw, void* out, int m, int n_out, int k, int inter,
+                       int ldo, int* err, cudaStream_t stream) {
+    constexpr size_t smem = PairGeometry<BN>::smem;
+    CUtensorMap map_b;                // boxes of a block's half of a tile's weight rows
+    if (!qf_make_map_bf16(&map_b, w, w_rows, k, ldw, BN / 2)) return (int)cudaErrorNotSupported;
+    cudaError_t e = cudaFuncSetAttribute(tc_gemm_pair_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    const int tile_cols = EPI == TC_SWIGLU ? BN / 2 : BN;
+    const int m_tiles = (m + 2 * TC_BM - 1) / (2 * TC_BM), n_tiles = (n_out + tile_cols - 1) / tile_cols;
+    const int total = m_tiles * n_tiles, pairs = qf_sm_count() / 2;
+    // column tiles whose weight rows together take about 32 MB, a quarter of the L2; 4 at least
+    long long group_n = (32ll << 20) / ((long long)BN * k * 2);
+    group_n = group_n < 4 ? 4 : group_n;
+    group_n = group_n > n_tiles ? n_tiles : group_n;
+    return (int)launch_pdl(tc_gemm_pair_kernel<EPI, BN>, dim3(2 * (total < pairs ? total : pairs)), dim3(TP_THREADS), smem, stream, map_a,
+                           map_b, (bf16*)out, m, n_out, k, inter, ldo, m_tiles, n_tiles, (int)group_n, err);
+}
+
+// Tiles of 256 columns, or of 192 where the wide ones' last round would leave many pairs idle: a round of the narrow ones takes
+// 0.8 of a wide one's time (measured 0.75 at K = 896, 0.81 at 2,048; 905 x 9728 x 896: 204 narrow tiles in three rounds of 74 pairs
+// 18.9 microseconds, 152 wide ones in three rounds 21.4; 1024 x 22016 x 2048: seven rounds 67.7, five 65.0). Tiles of 128
+// columns were never the fastest (23.5 and 86.4).
+static int pair_columns(int epilogue, int m, int n_out) {
+    const long long pairs = qf_sm_count() / 2 > 0 ? qf_sm_count() / 2 : 1, m_tiles = (m + 255) / 256;
+    auto rounds = [&](int columns) {
+        const int cols = epilogue == TC_SWIGLU ? columns / 2 : columns;
+        return (m_tiles * ((n_out + cols - 1) / cols) + pairs - 1) / pairs;
+    };
+    return 4 * rounds(192) < 5 * rounds(256) ? 192 : 256;
 }
 
 template <int EPI>
-static int launch_persistent(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int m, int n_out, int k, int inter,
-                             int ldo, int m_tiles, int n_tiles, int* err, cudaStream_t stream) {
-    constexpr size_t smem = (size_t)TP_STAGES * TP_STAGE_BYTES + 1024;
-    static_assert(qf_tmem_fits(2 * TP_BN, smem), "the rule of tcgen05.cuh");
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_persistent_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    const int total = m_tiles * n_tiles, sms = qf_sm_count();
-    // column tiles whose weight rows (256 rows of k) together take about 32 MB, a quarter of the L2; 4 at least
-    long long group_n = (32ll << 20) / ((long long)TP_BN * k * 2);
-    group_n = group_n < 4 ? 4 : group_n > n_tiles ? n_tiles : group_n;
-    tc_gemm_persistent_kernel<EPI><<<total < sms ? total : sms, TP_THREADS, smem, stream>>>(map_a, map_b, (bf16*)out, m, n_out, k, inter,
-                                                                                          ldo, m_tiles, n_tiles, (int)group_n, err);
-    return (int)cudaGetLastError();
+static int launch_persistent(const CUtensorMap& map_a, const void* w, int w_rows, int ldw, void* out, int m, int n_out, int k, int inter,
+                             int ldo, int* err, cudaStream_t stream) {
+    return pair_columns(EPI, m, n_out) == 192 ? launch_pair<EPI, 192>(map_a, w, w_rows, ldw, out, m, n_out, k, inter, ldo, err, stream)
+                                              : launch_pair<EPI, 256>(map_a, w, w_rows, ldw, out, m, n_out, k, inter, ldo, err, stream);
 }
 
 template <int EPI, int BN>
@@ -558,7 +616,9 @@ static int g_persistent = 1;
 // A measuring aid: 0 sends every product to the one-tile-per-block kernel.
 QF_EXPORT void qf_tc_gemm_set_persistent(int on) { g_persistent = on; }
 
-// Whether a product of these sizes has tiles for every SM and so runs in the persistent kernel (n as in qf_tc_gemm).
+// Whether a product of these sizes has tiles for every SM and so runs in the persistent kernel (n as in qf_tc_gemm), and the
+// columns of its tiles there.
+QF_EXPORT int qf_tc_gemm_pair_columns(int epilogue, int m, int n) { return pair_columns(epilogue, m, epilogue == TC_SWIGLU ? n / 2 : n); }
 QF_EXPORT int qf_tc_gemm_is_persistent(int epilogue, int m, int n) {
     if (!g_persistent || m <= 0 || n <= 0) return 0;
     const long long m_tiles = (m + TC_BM - 1) / TC_BM;
@@ -584,19 +644,13 @@ QF_EXPORT int qf_tc_gemm(int epilogue, const void* a, int lda, const void* w, in
         if (n % 2 || (n / 2) % 8) return (int)cudaErrorInvalidValue;
         const int inter = n / 2;
         const bool wide = (long long)m_tiles * ((inter + 127) / 128) >= qf_sm_count();
-        if (wide && g_persistent) {
-            if (!qf_make_map_bf16(&map_b, w, n, k, ldw, 128)) return (int)cudaErrorNotSupported;  // boxes of 128 weight rows
-            return launch_persistent<TC_SWIGLU>(map_a, map_b, out, m, inter, k, inter, ldo, m_tiles, (inter + 127) / 128, err, stream);
-        }
+        if (wide && g_persistent) return launch_persistent<TC_SWIGLU>(map_a, w, n, ldw, out, m, inter, k, inter, ldo, err, stream);
         return wide ? launch_tc<TC_SWIGLU, 256>(map_a, map_b, out, m, inter, k, inter, ldo, err, dim3((inter + 127) / 128, m_tiles), stream)
                     : launch_tc<TC_SWIGLU, 128>(map_a, map_b, out, m, inter, k, inter, ldo, err, dim3((inter + 63) / 64, m_tiles), stream);
     }
     if (epilogue != TC_PLAIN) return (int)cudaErrorInvalidValue;
     const bool wide = (long long)m_tiles * ((out_cols + 255) / 256) >= qf_sm_count();
-    if (wide && g_persistent) {
-        if (!qf_make_map_bf16(&map_b, w, n, k, ldw, 128)) return (int)cudaErrorNotSupported;
-        return launch_persistent<TC_PLAIN>(map_a, map_b, out, m, n, k, 0, ldo, m_tiles, (n + 255) / 256, err, stream);
-    }
+    if (wide && g_persistent) return launch_persistent<TC_PLAIN>(map_a, w, n, ldw, out, m, n, k, 0, ldo, err, stream);
     return wide ? launch_tc<TC_PLAIN, 256>(map_a, map_b, out, m, n, k, 0, ldo, err, dim3((n + 255) / 256, m_tiles), stream)
                 : launch_tc<TC_PLAIN, 128>(map_a, map_b, out, m, n, k, 0, ldo, err, dim3((n + 127) / 128, m_tiles), stream);
 }

@@ -14,8 +14,8 @@ import torch
 from . import kernels
 
 # Plain products of 128 or more token rows can run on this library's own tcgen05 kernel (`csrc/tc_gemm.cu`) instead of
-# the cuBLAS call. Off by default: measured on a B200 at 2048 x 9728 x 896 its persistent form reaches 800 TFLOP/s where
-# cuBLAS reaches 1,140 (at 2048 x 37888 x 3584: 1,215 against 1,620). The gate/up product with the gate in its epilogue
+# the cuBLAS call. Off by default: measured on a B200 at 7358 x 2560 x 2048 its persistent form reaches 1,424 TFLOP/s where
+# cuBLAS reaches 1,507 (at 11788 x 3584 x 18944: 1,542 against 1,462; at 2048 x 896 x 4864: 475 against 1,023). The gate/up product with the gate in its epilogue
 # does not wait for this switch: it is the faster way wherever the persistent kernel runs (`parts/swiglu.py`).
 _own_tensor_core_products = False
 OWN_PRODUCT_MIN_ROWS = 128
