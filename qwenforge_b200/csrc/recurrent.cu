@@ -9,7 +9,28 @@
 // on how they were cut into steps: every kernel walks a sequence token by token in one fixed order of operations.
 #include <float.h>
 
+#include <type_traits>
+
 #include "common.cuh"
+
+// 1 / d for d >= 1 (infinity and NaN as the division gives them) and z / d with it, by Newton's step and Markstein's correction of the
+// quotient ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): the remainders are exact in a fused
+// multiply-add, so both come out rounded to the nearest as the division rounds them, without the division's branches. Compared
+// with `/` on every d from 1 to 2^128 and on 2^32 pairs: the same bits, below 2^-126 (1 / d for d beyond 2^126) but for the last.
+struct Over {
+    float d, r;
+    __device__ __forceinline__ explicit Over(float d_) : d(d_) {
+        const float part = 0.0625f * d;   // whose reciprocal is never too small for the steps
+        float r0;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(part));
+        const float left = fmaf(-part, r0, 1.f);
+        r = 0.0625f * (fabsf(left) <= 1.f ? fmaf(r0, left, r0) : r0);
+    }
+    __device__ __forceinline__ float of(float z) const {
+        const float q = z * r, over = fmaf(d, q, -z);
+        return fabsf(over) <= FLT_MAX ? fmaf(-over, r, q) : q;   // (the sign of a zero stays)
+    }
+};
 
 // ------------------------------------------------------------------------------------------------------------------
 // Exponential gates with a running maximum (the mLSTM's): m' = max(f + m, a), one block per (sequence, head), GATE_TOKENS tokens at a
@@ -625,8 +646,8 @@ gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ gate,
 // The same in bfloat16 where every run of eight columns lies within a head and all rows are addressable by 16 bytes: G threads take a
 // part (a power of two of lanes up to a warp, or a block), each P pieces of eight columns, all of whose inputs are asked for at
 // once and read once. What bounds it is memory, and beside it the exponentials and divisions of the gates: 4,206 rows of 4,096 columns
-// with a gate and a skip (172 MB) took 116 microseconds with scalar loads (whose parts beyond 2,048 columns were also read twice),
-// 54 here.
+// with a gate and a skip (172 MB) took 116 microseconds with scalar loads (whose parts beyond 2,048 columns were also read twice), 54
+// with the options looked at for every number and the gates' reciprocals by `/`, 32 here (5.4 TB/s); 3,079 of 2,048 in parts of 128: 17 and 10.
 template <int G, int P>
 __global__ void __launch_bounds__(256)
 gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict__ gate, int gate_stride, const bf16* __restrict__ weight,
@@ -641,7 +662,7 @@ gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict_
     const int t = live ? (int)(item / n_parts) : 0, part = live ? (int)(item % n_parts) : 0;
     const int part_width = width / n_parts, head_width = width / n_heads, c0 = part * part_width;
     float4 z[P][2];
-    uint4 gates[P], weights[P], extra[P];
+    uint4 gates[P], extra[P];
     float by[P], add[P];
     bool has[P];
 #pragma unroll
@@ -649,13 +670,13 @@ gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict_
         const int at = (member + G * i) * 8, c = c0 + at;
         has[i] = live && at < part_width;
         z[i][0] = z[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-        gates[i] = weights[i] = extra[i] = make_uint4(0, 0, 0, 0);
+        gates[i] = extra[i] = make_uint4(0, 0, 0, 0);
         by[i] = 1.f, add[i] = 0.f;
         if (!has[i]) continue;
         const float4* src = reinterpret_cast<const float4*>(y + (size_t)t * width + c);
         z[i][0] = src[0], z[i][1] = src[1];
         gates[i] = *reinterpret_cast<const uint4*>(gate + (size_t)t * gate_stride + c);
-        weights[i] = *reinterpret_cast<const uint4*>(weight + c);
+        if (!skip && !nq) continue;
         const int head = c / head_width;
         if (skip) {
             add[i] = skip[head];
@@ -663,27 +684,38 @@ gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict_
         }
         if (nq) by[i] = fmaxf(fabsf(nq[(size_t)t * n_heads + head]), floor_in[(size_t)t * n_heads + head]) + floor_add;
     }
-    auto gate_of = [&](float raw) {
-        const float sig = 1.f / (1.f + expf(-raw));
-        return gate_kind == 0 ? sig : raw * sig;
+    auto eight = [](const uint4& raw, float (&x)[8]) {
+        const uint32_t pairs[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[2 * e] = __uint_as_float(pairs[e] << 16), x[2 * e + 1] = __uint_as_float(pairs[e] & 0xffff0000u);
+    };
+    auto times_gates = [&](float* v, const uint4& raw) {
+        float g[8];
+        eight(raw, g);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float sig = Over(1.f + expf(-g[e])).r;
+            v[e] *= gate_kind == 0 ? sig : g[e] * sig;
+        }
     };
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < P; ++i) {
         float* v = reinterpret_cast<float*>(z[i]);
-        const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&gates[i]);
-        const __nv_bfloat162* ep = reinterpret_cast<const __nv_bfloat162*>(&extra[i]);
+        if (nq) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            if (nq) v[e] /= by[i];
-            const float2 x2 = __bfloat1622float2(ep[e >> 1]);
-            if (skip) v[e] = fmaf(add[i], e & 1 ? x2.y : x2.x, v[e]);
-            if (gate_first) {
-                const float2 g2 = __bfloat1622float2(gp[e >> 1]);
-                const float raw = e & 1 ? g2.y : g2.x;
-                v[e] *= gate_of(raw);
-            }
-            sum = has[i] ? fmaf(v[e], v[e], sum) : sum;
+            for (int e = 0; e < 8; ++e) v[e] /= by[i];
+        }
+        if (skip) {
+            float x[8];
+            eight(extra[i], x);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = fmaf(add[i], x[e], v[e]);
+        }
+        if (gate_first) times_gates(v, gates[i]);
+        if (has[i]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum = fmaf(v[e], v[e], sum);
         }
     }
     if (G <= 32) {
@@ -696,19 +728,16 @@ gated_group_norm_vec_kernel(const float* __restrict__ y, const bf16* __restrict_
 #pragma unroll
     for (int i = 0; i < P; ++i) {
         if (!has[i]) continue;
-        const float* v = reinterpret_cast<const float*>(z[i]);
-        const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&gates[i]);
-        const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&weights[i]);
+        float* v = reinterpret_cast<float*>(z[i]);
+        float w[8];
+        eight(*reinterpret_cast<const uint4*>(weight + c0 + (member + G * i) * 8), w);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * w[e];
+        if (!gate_first) times_gates(v, gates[i]);
         uint32_t packed[4];
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {
-            const float2 w2 = __bfloat1622float2(wp[e >> 1]), g2 = __bfloat1622float2(gp[e >> 1]);
-            float a = v[e] * inv * w2.x, b = v[e + 1] * inv * w2.y;
-            if (!gate_first) {
-                a *= gate_of(g2.x);
-                b *= gate_of(g2.y);
-            }
-            const __nv_bfloat162 two = __floats2bfloat162_rn(a, b);
+            const __nv_bfloat162 two = __floats2bfloat162_rn(v[e], v[e + 1]);
             packed[e >> 1] = *reinterpret_cast<const uint32_t*>(&two);
         }
         *reinterpret_cast<uint4*>(out + (size_t)t * width + c0 + (member + G * i) * 8) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
@@ -813,17 +842,17 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ x, int x_stride, c
     if (single && before && taps > 1) before[(size_t)(taps - 2) * channels + c] = Num<T>::to_f(x[(size_t)t * x_stride + c]);
     T* dst = out + (size_t)t * channels + c;
     if (CACHED) dst = c < cache.tail ? out + (size_t)t * cache.tail + c : conv_cache_place(cache, slot, t, c);
-    if (!CACHED || dst) *dst = Num<T>::from_f(plain ? z : z / (1.f + expf(-z)));
+    if (!CACHED || dst) *dst = Num<T>::from_f(plain ? z : Over(1.f + expf(-z)).of(z));
 }
 
-// The same convolution for long steps: a thread takes 16 bytes of channels and a run of CONV_RUN(TAPS) consecutive tokens, asks for
-// all of the run's rows at once (4,206 tokens of 4,352 channels, 73 MB: 69 microseconds with a row and its sequence fetched token by
-// token, 54 so; the exponentials and divisions of silu bound it), keeps
-// the last TAPS - 1 inputs in registers as it walks down the run, and fetches them afresh (from the state, or zeros) where a
-// sequence begins inside the run. Every output is the same chain of fused multiply-adds, oldest input first, as in the
-// kernel of one thread per (token, channel): the two agree bit for bit.
-// tokens of a run: the more taps, the more a longer run saves (taps - 1 inputs are fetched again at the start of every run)
-#define CONV_RUN(TAPS) ((TAPS) >= 4 ? 8 : 4)
+// The same convolution for long steps: a thread takes four channels and a run of CONV_RUN consecutive tokens. Where the run and the
+// TAPS - 1 tokens before it lie in one sequence of the step (nearly always), it asks for all their rows at once and walks down
+// the run with the last TAPS - 1 inputs in registers; otherwise it takes its tokens one by one, each with the inputs that it finds (in
+// the step, in the state, or zeros). Every output is the same chain of fused multiply-adds, oldest input first, as in the
+// kernel of one thread per (token, channel): they agree bit for bit. 4,206 tokens of
+// 4,352 channels (73 MB) took 53 microseconds with eight channels a thread (153 registers, a sixth of the warps that an SM holds), every
+// token's sequence looked up and the gates by `/`; 25 so. The exponentials and divisions of silu bound it.
+#define CONV_RUN 8
 
 template <typename T, int TAPS, bool CACHED>
 __global__ void __launch_bounds__(128)
@@ -831,16 +860,16 @@ causal_conv_run_kernel(const T* __restrict__ x, int x_stride, const float* __res
                        const int* __restrict__ cu_q, const int* __restrict__ tok_seq, const int* __restrict__ slots,
                        const float* __restrict__ state, long long slot_stride, long long offset, int n_tokens, int channels,
                        T* __restrict__ out, int plain, ConvCache<T> cache) {
-    constexpr int V = 16 / (int)sizeof(T);
-    constexpr int H = TAPS > 1 ? TAPS - 1 : 1;
+    constexpr int V = 4, RUN = CONV_RUN, H = TAPS - 1;
+    typedef typename std::conditional<sizeof(T) == 2, uint2, uint4>::type Four;
     grid_chain_entry();
     const int groups = channels / V;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    constexpr int RUN = CONV_RUN(TAPS);
     const int n_runs = (n_tokens + RUN - 1) / RUN;
     if (i >= (long long)n_runs * groups) return;
-    const int t0 = (int)(i / groups) * RUN, c0 = (int)(i % groups) * V;
-    float w[V][TAPS], b[V], hist[H][V];
+    const int t0 = (int)(i / groups) * RUN, c0 = (int)(i % groups) * V, last = min(t0 + RUN, n_tokens) - 1;
+    const int seq = tok_seq[t0], seq_last = tok_seq[last], begin = cu_q[seq];
+    float w[V][TAPS], b[V];
     if (((uintptr_t)weight & 15) == 0) {   // (V channels' taps are V * TAPS neighbouring numbers from a multiple of 16 bytes on)
 #pragma unroll
         for (int i = 0; i < V * TAPS / 4; ++i) {
@@ -856,56 +885,68 @@ causal_conv_run_kernel(const T* __restrict__ x, int x_stride, const float* __res
     }
 #pragma unroll
     for (int v = 0; v < V; ++v) b[v] = bias ? bias[c0 + v] : 0.f;
-    // the run's rows and places, all asked for before the first is used
-    uint4 rows[RUN];
-    int seqs[RUN], at[RUN];
+    auto numbers = [](const Four& raw, float (&in)[V]) {
+        const T* p = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-    for (int k = 0; k < RUN; ++k) {
-        const int t = min(t0 + k, n_tokens - 1);
-        rows[k] = *reinterpret_cast<const uint4*>(x + (size_t)t * x_stride + c0);
-        seqs[k] = tok_seq[t];
-    }
-#pragma unroll
-    for (int k = 0; k < RUN; ++k) at[k] = t0 + k - cu_q[seqs[k]];
-#pragma unroll
-    for (int k = 0; k < RUN; ++k) {
-        const int t = t0 + k;
-        if (t >= n_tokens) break;
-        if (TAPS > 1 && (k == 0 || at[k] == 0)) {
-            const int slot = slots[seqs[k]];
-            const float* before = slot >= 0 ? state + slot * slot_stride + offset : nullptr;
-#pragma unroll
-            for (int r = 0; r < TAPS - 1; ++r) {   // hist[r]: the input TAPS - 1 - r tokens back
-                const int back = TAPS - 1 - r;
-                if (at[k] - back >= 0) {
-                    T in[V];
-                    *reinterpret_cast<uint4*>(in) = *reinterpret_cast<const uint4*>(x + (size_t)(t - back) * x_stride + c0);
-#pragma unroll
-                    for (int v = 0; v < V; ++v) hist[r][v] = Num<T>::to_f(in[v]);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < V; ++v)
-                        hist[r][v] = before ? before[(size_t)(TAPS - 1 + at[k] - back) * channels + c0 + v] : 0.f;
-                }
-            }
-        }
-        T in[V], res[V];
-        *reinterpret_cast<uint4*>(in) = rows[k];
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const float u = Num<T>::to_f(in[v]);
-            float z = b[v];
-#pragma unroll
-            for (int r = 0; r < TAPS - 1; ++r) z = fmaf(w[v][r], hist[r][v], z);
-            z = fmaf(w[v][TAPS - 1], u, z);
-            res[v] = Num<T>::from_f(plain ? z : z / (1.f + expf(-z)));
-#pragma unroll
-            for (int r = 0; r + 1 < TAPS - 1; ++r) hist[r][v] = hist[r + 1][v];
-            if (TAPS > 1) hist[H - 1][v] = u;
-        }
+        for (int v = 0; v < V; ++v) in[v] = Num<T>::to_f(p[v]);
+    };
+    auto row_of = [&](int t) { return *reinterpret_cast<const Four*>(x + (size_t)t * x_stride + c0); };
+    auto store = [&](int t, int slot, const float (&z)[V]) {
         T* dst = out + (size_t)t * channels + c0;
-        if (CACHED) dst = c0 < cache.tail ? out + (size_t)t * cache.tail + c0 : conv_cache_place(cache, slots[seqs[k]], t, c0);
-        if (!CACHED || dst) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(res);
+        if (CACHED) dst = c0 < cache.tail ? out + (size_t)t * cache.tail + c0 : conv_cache_place(cache, slot, t, c0);
+        Four res;
+        T* p = reinterpret_cast<T*>(&res);
+#pragma unroll
+        for (int v = 0; v < V; ++v) p[v] = Num<T>::from_f(plain ? z[v] : Over(1.f + expf(-z[v])).of(z[v]));
+        if (!CACHED || dst) *reinterpret_cast<Four*>(dst) = res;
+    };
+    if (seq == seq_last && t0 - begin >= H && last == t0 + RUN - 1) {
+        Four rows[RUN + H];
+#pragma unroll
+        for (int k = 0; k < RUN + H; ++k) rows[k] = row_of(t0 - H + k);
+        const int slot = CACHED ? slots[seq] : 0;
+        float hist[H][V];              // hist[r]: the input H - r tokens back
+#pragma unroll
+        for (int r = 0; r < H; ++r) numbers(rows[r], hist[r]);
+#pragma unroll
+        for (int k = 0; k < RUN; ++k) {
+            float in[V], z[V];
+            numbers(rows[H + k], in);
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                z[v] = b[v];
+#pragma unroll
+                for (int r = 0; r < H; ++r) z[v] = fmaf(w[v][r], hist[r][v], z[v]);
+                z[v] = fmaf(w[v][H], in[v], z[v]);
+#pragma unroll
+                for (int r = 0; r + 1 < H; ++r) hist[r][v] = hist[r + 1][v];
+                hist[H - 1][v] = in[v];
+            }
+            store(t0 + k, slot, z);
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int t = t0; t <= last; ++t) {
+        const int mine = tok_seq[t], at = t - cu_q[mine], slot = slots[mine];
+        const float* before = slot >= 0 ? state + slot * slot_stride + offset : nullptr;   // [H][channels]
+        float z[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) z[v] = b[v];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            const int back = H - j;
+            float u[V] = {0.f, 0.f, 0.f, 0.f};
+            if (at - back >= 0) {
+                numbers(row_of(t - back), u);
+            } else if (before) {
+#pragma unroll
+                for (int v = 0; v < V; ++v) u[v] = before[(size_t)(H + at - back) * channels + c0 + v];
+            }
+#pragma unroll
+            for (int v = 0; v < V; ++v) z[v] = fmaf(w[v][j], u[v], z[v]);
+        }
+        store(t, slot, z);
     }
 }
 
@@ -939,8 +980,7 @@ static int launch_conv(const void* x, int x_stride, const float* weight, const f
                       (!CACHED || (cache.tail % V == 0 && cache.site.head_dim % V == 0 && ((uintptr_t)cache.site.base & 15) == 0));
     cudaError_t e;
     if (runs) {
-        const int run = CONV_RUN(taps);
-        const long long items = (long long)((n_tokens + run - 1) / run) * (channels / V);
+        const long long items = (long long)((n_tokens + CONV_RUN - 1) / CONV_RUN) * (channels / 4);
         const dim3 grid((unsigned)((items + 127) / 128)), block(128);
 #define QF_CONV_RUN(TAPS) launch_pdl(causal_conv_run_kernel<T, TAPS, CACHED>, grid, block, 0, stream, (const T*)x, x_stride, weight, bias, \
                                      cu_q, tok_seq, slots, (const float*)state, slot_stride, offset, n_tokens, channels, (T*)out, plain, cache)

@@ -92,3 +92,26 @@ def test_gates_far_below_zero():
         ops.gated_group_norm(ones, z, torch.ones(c, dtype=torch.bfloat16, device=DEV), 0.0, out, 1, 1, gate, False)
         # (a sigmoid below 2^-126 has fewer bits: 2^-149 is its unit, and a bfloat16 below 2^-126 has 2^-133)
         assert float(((out.double() - size).abs() / (size.abs() * 2 ** -7 + 2.0 ** -133)).max()) <= 1
+
+
+def test_silu_behind_the_convolution():
+    """Taps of zero and one leave the input: silu of float32 numbers over their whole range. Two roundings of the exponential (2 ulp)
+    count at most |z| / (1 + e^z) <= 1 each, then one of the sum and one of the quotient."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x = torch.randn(64, 4096, generator=g, device=DEV) * torch.logspace(-6, 1.4, 64, device=DEV)[:, None]
+    x[:, 0] = 0.0                                              # (what is not finite stays in its own token: no tap in front of it)
+    odd = torch.tensor([0.0, -0.0, 100.0, -100.0, -88.0, float("inf"), float("nan")], device=DEV)
+    n, c = x.shape
+    cu, slots = torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.tensor([-1], dtype=torch.int32, device=DEV)
+    seq, taps = torch.zeros(n, dtype=torch.int32, device=DEV), torch.tensor([[0.0, 1.0]], device=DEV).repeat(c, 1)
+    last = x.clone()
+    last[-1, :odd.numel()] = odd
+    out, state = torch.empty_like(x), torch.zeros(1, c, device=DEV)
+    ops.causal_conv_silu(last, taps, None, cu, seq, slots, state, 0, out)
+    z = last.double()
+    want, got = z / (1 + torch.exp(-z)), out.double()
+    fine = torch.isfinite(want) & (z.abs() < 80)
+    assert bool(((got - want).abs()[fine] <= 4 * 2.0 ** -23 * want.abs()[fine]).all())
+    row = out[-1, :odd.numel()].tolist()
+    assert row[0] == row[1] == 0 and row[2] == 100 and abs(row[3]) < 1e-35 and abs(row[4]) < 1e-35 and row[5] == float("inf") and row[6] != row[6]
