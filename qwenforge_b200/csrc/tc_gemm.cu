@@ -304,18 +304,25 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // to 9 own the epilogue: warp w reads accumulator lanes 32 (w % 4) .. + 31 (the lanes a warp may read are fixed by its number)
 // and one half of the tile's columns. The launch is a programmatic dependent one: barriers and tensor memory are set up under
 // the tail of the kernel before (a 905-token prompt of 24 layers: 1,548 -> 1,512 microseconds).
-// What bounds it: at large K the tensor cores (7358 x 22016 x 2048: 413 microseconds, 1,608 TFLOP/s; one block a tile of 128 x 256,
-// which reads 1.5 times the bytes from the L2 per product, took 476); at K = 896 the tiles' last round and 1.5 microseconds a
-// tile that the ring takes to fill and the sums to drain (2048 x 9728 x 896 with the gate: 31 microseconds, 36 before).
+// What bounds it: at large K the tensor cores (7358 x 22016 x 2048: 407 microseconds, 1,631 TFLOP/s; one block a tile of 128 x 256,
+// which reads 1.5 times the bytes from the L2 per product, took 476); at K = 896 the tiles' last round and what the
+// ring takes to fill and the sums to drain (2048 x 9728 x 896 with the gate: 27 microseconds, 36 on single blocks).
 // (The first tile's weights asked for before the wait for the kernel ahead: 1,528 instead of 1,512. Not kept.)
 #define TP_THREADS 320
 #define TP_EPI_WARPS 8
-template <int BN> struct PairGeometry {   // BN 256 or 192: six or seven stages
-    static constexpr int stage_bytes = (TC_BM + BN / 2) * TC_BK * 2;
-    static constexpr int stages = BN == 256 ? 6 : 7;
-    static constexpr size_t smem = (size_t)stages * stage_bytes + 1024;
-    static_assert(qf_tmem_fits(512, smem), "the rule of tcgen05.cuh");
+#define TP_PATCH_BYTES (32 * 128)
+template <int BN> struct PairGeometry {   // BN 256 or 192
+    static constexpr int stage_bytes = (TC_BM + BN / 2) * TC_BK * 2, stages = 6;
+    static constexpr size_t smem = (size_t)stages * stage_bytes + TP_EPI_WARPS * TP_PATCH_BYTES + 1024;
+    static_assert(qf_tmem_fits(512, smem) && smem + 512 <= 227 * 1024, "the rule of tcgen05.cuh; what an SM gives a block");
 };
+
+// A warp's patch of results on its way out: 32 rows of 128 bytes, their 16-byte pieces permuted so that a row per lane is written and a
+// row per eight lanes read without conflicts. (A row per lane stored straight to memory touches 32 lines an instruction, 1
+// microsecond for 64 columns of a tile: 2048 x 9728 x 896 with the gate took 31 microseconds so, 27 by way of patches; 905 rows 18.9 and 16.8.)
+__device__ __forceinline__ uint4* patch_at(unsigned char* patch, int row, int piece) {
+    return reinterpret_cast<uint4*>(patch + row * 128 + ((piece ^ (row & 7)) << 4));
+}
 
 __device__ __forceinline__ float fast_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 
@@ -330,11 +337,6 @@ __device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles, int gro
     const int width = min(group_n, n_tiles - first), local = t - g * per_group;
     tile_m = local / width;
     tile_n = first + local % width;
-}
-
-// Eight neighbouring results of a row (n_out is a multiple of eight: a piece is whole or beyond the matrix).
-__device__ __forceinline__ void store_8(bf16* dst, const uint32_t* packed) {
-    *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
 }
 
 template <int EPI, int BN>
@@ -353,6 +355,10 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
     const int n_k = (K + TC_BK - 1) / TC_BK, total = m_tiles * n_tiles;
 
+    if (threadIdx.x == 32) {
+        tma_prefetch_map(&map_a);
+        tma_prefetch_map(&map_b);
+    }
     // Both blocks' copies of a stage arrive at the first block's full_bar (one arrival, which announces both blocks' bytes); a
     // stage's and a tile's end are told to both blocks' empty_bar and acc_full; all sixteen epilogue warps arrive at the
     // first block's acc_empty.
@@ -451,65 +457,69 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else if (warp >= 2) {
         // ---- epilogue
         const int quad = warp & 3, half = (warp - 2) >> 2;
+        unsigned char* patches = smem + (size_t)STAGES * STAGE_BYTES;
+        unsigned char* patch = patches + (warp - 2) * TP_PATCH_BYTES;   // this warp's own
         int i = 0;
         for (int t = pair; t < total; t += pairs, ++i) {
             const int buf = i & 1;
             int tile_m, tile_n;
             tile_of(t, m_tiles, n_tiles, group_n, tile_m, tile_n);
-            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (i >> 1) & 1))) {
+            const int row0 = (2 * tile_m + (int)rank) * TC_BM + quad * 32;
+            const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 256);
+            auto sums_there = [&]() {
+                const bool there = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (i >> 1) & 1));
+                tc_fence_after();
+                return there;
+            };
+            auto sums_read = [&]() {     // the warp has read its part of the half
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));
+            };
+            if (!sums_there()) {
                 timed_out = true;
                 break;
             }
-            tc_fence_after();
-            const int row = (2 * tile_m + (int)rank) * TC_BM + quad * 32 + lane;
-            const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 256);
-            if (EPI == TC_SWIGLU) {
-                constexpr int W = HALF / 2 % 32 == 0 ? 32 : 16;   // columns a turn
+            // this warp's columns of results, up to 64 at a time
+            constexpr int OWN = EPI == TC_SWIGLU ? HALF / 2 : HALF;
+            const int col0 = (EPI == TC_SWIGLU ? tile_n * HALF : tile_n * BN) + half * OWN;
 #pragma unroll
-                for (int c = 0; c < HALF / 2; c += W) {
-                    const int c0 = half * (HALF / 2) + c;
-                    uint32_t g[W], u[W];
-                    if constexpr (W == 32) {
-                        tmem_load_32(lane_base + c0, g);
-                        tmem_load_32(lane_base + HALF + c0, u);
-                    } else {
-                        tmem_load_16(lane_base + c0, g);
-                        tmem_load_16(lane_base + HALF + c0, u);
-                    }
-                    const int col = tile_n * HALF + c0;
-                    if (row < M) {
-                        uint32_t packed[W / 2];
+            for (int c = 0; c < OWN; c += 64) {
+                constexpr int W = OWN % 32 == 0 ? 32 : 16;   // columns a turn
+                const int n_cols = OWN - c < 64 ? OWN - c : 64;
+#pragma unroll
+                for (int e = 0; e < n_cols; e += W) {
+                    uint32_t packed[W / 2];
+                    if constexpr (EPI == TC_SWIGLU) {
+                        uint32_t g[W], u[W];
+                        tmem_load_two(lane_base + half * OWN + c + e, lane_base + HALF + half * OWN + c + e, g, u);
 #pragma unroll
                         for (int j = 0; j < W / 2; ++j)
                             packed[j] = pack_bf16(fast_silu(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
                                                   fast_silu(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
-                        bf16* dst = out + (size_t)row * ldo + col;
+                    } else {
+                        uint32_t v[W];
+                        if constexpr (W == 32) tmem_load_32(lane_base + half * OWN + c + e, v);
+                        else tmem_load_16(lane_base + half * OWN + c + e, v);
 #pragma unroll
-                        for (int j = 0; j < W / 8; ++j)
-                            if (col + 8 * j < n_out) store_8(dst + 8 * j, packed + 4 * j);
+                        for (int j = 0; j < W / 2; ++j) packed[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
                     }
+#pragma unroll
+                    for (int j = 0; j < W / 8; ++j)
+                        *patch_at(patch, lane, e / 8 + j) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
                 }
-            } else {
+                if (c + 64 >= OWN) sums_read();
+                else __syncwarp();
+                // n_out is a multiple of eight: a piece is whole or beyond the matrix
+                const int pieces = n_cols / 8;
 #pragma unroll
-                for (int c = 0; c < HALF; c += 32) {
-                    const int c0 = half * HALF + c;
-                    uint32_t v[32];
-                    tmem_load_32(lane_base + c0, v);
-                    const int col = tile_n * BN + c0;
-                    if (row < M) {
-                        uint32_t packed[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) packed[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-                        bf16* dst = out + (size_t)row * ldo + col;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (col + 8 * j < n_out) store_8(dst + 8 * j, packed + 4 * j);
-                    }
+                for (int u = 0; u < pieces; ++u) {
+                    const int r = (u * 32 + lane) / pieces, piece = (u * 32 + lane) % pieces, col = col0 + c + 8 * piece;
+                    if (row0 + r < M && col < n_out)
+                        *reinterpret_cast<uint4*>(out + (size_t)(row0 + r) * ldo + col) = *patch_at(patch, r, piece);
                 }
+                __syncwarp();
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));  // this warp has read its part of the half
         }
     }
     if (timed_out && lane == 0) atomicOr(err, QF_ERR_COPY_TIMEOUT);
@@ -535,14 +545,14 @@ static int launch_pair(const CUtensorMap& map_a, const void* w, int w_rows, int 
     long long group_n = (32ll << 20) / ((long long)BN * k * 2);
     group_n = group_n < 4 ? 4 : group_n;
     group_n = group_n > n_tiles ? n_tiles : group_n;
-    return (int)launch_pdl(tc_gemm_pair_kernel<EPI, BN>, dim3(2 * (total < pairs ? total : pairs)), dim3(TP_THREADS), smem, stream, map_a,
-                           map_b, (bf16*)out, m, n_out, k, inter, ldo, m_tiles, n_tiles, (int)group_n, err);
+    return (int)launch_pdl(tc_gemm_pair_kernel<EPI, BN>, dim3(2 * (total < pairs ? total : pairs)), dim3(TP_THREADS), smem, stream,
+                           map_a, map_b, (bf16*)out, m, n_out, k, inter, ldo, m_tiles, n_tiles, (int)group_n, err);
 }
 
 // Tiles of 256 columns, or of 192 where the wide ones' last round would leave many pairs idle: a round of the narrow ones takes
-// 0.8 of a wide one's time (measured 0.75 at K = 896, 0.81 at 2,048; 905 x 9728 x 896: 204 narrow tiles in three rounds of 74 pairs
-// 18.9 microseconds, 152 wide ones in three rounds 21.4; 1024 x 22016 x 2048: seven rounds 67.7, five 65.0). Tiles of 128
-// columns were never the fastest (23.5 and 86.4).
+// 0.8 of a wide one's time (measured 0.75 at K = 896, 0.81 at 2,048; with the results stored straight to memory, 905 x 9728 x 896: 204
+// narrow tiles in three rounds of 74 pairs 18.9 microseconds, 152 wide ones in three rounds 21.4; 1024 x 22016 x 2048: seven rounds
+// 67.7, five 65.0). Tiles of 128 columns were never the fastest (23.5 and 86.4).
 static int pair_columns(int epilogue, int m, int n_out) {
     const long long pairs = qf_sm_count() / 2 > 0 ? qf_sm_count() / 2 : 1, m_tiles = (m + 255) / 256;
     auto rounds = [&](int columns) {
