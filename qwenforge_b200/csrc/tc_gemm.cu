@@ -29,6 +29,7 @@ struct TcQkvArgs {
     const int* table;
     long long page_elems;
     int table_stride, n_heads, kv_heads, head_dim, write_cache;
+    const float* inv_freq;   // (the pairs' form) [head_dim / 2] frequencies, or null: no rotation
 };
 
 // One head (or half of one) of the TC_QKV epilogue for this thread's token row: P = D / 2 rotation pairs, W of them per
@@ -311,8 +312,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #define TP_THREADS 320
 #define TP_EPI_WARPS 8
 #define TP_PATCH_BYTES (32 * 128)
-template <int BN> struct PairGeometry {   // BN 256 or 192
-    static constexpr int stage_bytes = (TC_BM + BN / 2) * TC_BK * 2, stages = 6;
+template <int BN> struct PairGeometry {   // BN 256 or 192: six stages; 128: eight; 64: nine
+    static constexpr int stage_bytes = (TC_BM + BN / 2) * TC_BK * 2;
+    static constexpr int stages = BN >= 192 ? 6 : BN == 128 ? 8 : 9;
     static constexpr size_t smem = (size_t)stages * stage_bytes + TP_EPI_WARPS * TP_PATCH_BYTES + 1024;
     static_assert(qf_tmem_fits(512, smem) && smem + 512 <= 227 * 1024, "the rule of tcgen05.cuh; what an SM gives a block");
 };
@@ -339,11 +341,48 @@ __device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles, int gro
     tile_n = first + local % width;
 }
 
-template <int EPI, int BN>
+// The two epilogue warps of a quadrant of rows wait for each other.
+__device__ __forceinline__ void quadrant_sync(int quad) { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); }
+
+// 16 neighbouring rotation pairs of a head in this thread's row of the accumulator (first halves from column `lo` of its lane, second
+// halves from `hi`), with the bias of both, rotated by cs = (cos, sin) where `rotate`, as 16-byte pieces of the row.
+__device__ __forceinline__ void rotated_pairs(uint32_t lo, uint32_t hi, const bf16* bias_lo, const bf16* bias_hi, const float2* cs,
+                                              bool rotate, uint4 (&out_lo)[2], uint4 (&out_hi)[2]) {
+    uint32_t x[16], y[16];
+    tmem_load_two(lo, hi, x, y);
+#pragma unroll
+    for (int j0 = 0; j0 < 16; j0 += 8) {
+        uint32_t b1[4] = {0, 0, 0, 0}, b2[4] = {0, 0, 0, 0}, o1[4], o2[4];
+        if (bias_lo) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(bias_lo + j0)), v = __ldg(reinterpret_cast<const uint4*>(bias_hi + j0));
+            b1[0] = u.x, b1[1] = u.y, b1[2] = u.z, b1[3] = u.w;
+            b2[0] = v.x, b2[1] = v.y, b2[2] = v.z, b2[3] = v.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            float z1[2], z2[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float x1 = __uint_as_float(x[j0 + j + e]) + __uint_as_float(e ? b1[j / 2] & 0xffff0000u : b1[j / 2] << 16);
+                const float x2 = __uint_as_float(y[j0 + j + e]) + __uint_as_float(e ? b2[j / 2] & 0xffff0000u : b2[j / 2] << 16);
+                const float2 a = cs[j0 + j + e];
+                z1[e] = rotate ? x1 * a.x - x2 * a.y : x1;
+                z2[e] = rotate ? x2 * a.x + x1 * a.y : x2;
+            }
+            o1[j / 2] = pack_bf16(z1[0], z1[1]);
+            o2[j / 2] = pack_bf16(z2[0], z2[1]);
+        }
+        out_lo[j0 / 8] = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+        out_hi[j0 / 8] = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+    }
+}
+
+// P: rotation pairs of a head (TC_QKV; whole heads per tile)
+template <int EPI, int BN, int P = 0>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     bf16* __restrict__ out, int M, int n_out, int K, int inter, int ldo, int m_tiles, int n_tiles, int group_n,
-                    int* err) {
+                    int* err, const TcQkvArgs qa) {
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
     constexpr int STAGES = PairGeometry<BN>::stages, STAGE_BYTES = PairGeometry<BN>::stage_bytes;
@@ -458,13 +497,14 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ---- epilogue
         const int quad = warp & 3, half = (warp - 2) >> 2;
         unsigned char* patches = smem + (size_t)STAGES * STAGE_BYTES;
-        unsigned char* patch = patches + (warp - 2) * TP_PATCH_BYTES;   // this warp's own
+        unsigned char* patch = patches + (warp - 2) * TP_PATCH_BYTES;   // this warp's own (TC_QKV: shared by a quadrant's two warps, below)
         int i = 0;
+        if (EPI == TC_QKV) grid_dependency_wait();   // (positions, slots and page tables)
         for (int t = pair; t < total; t += pairs, ++i) {
             const int buf = i & 1;
             int tile_m, tile_n;
             tile_of(t, m_tiles, n_tiles, group_n, tile_m, tile_n);
-            const int row0 = (2 * tile_m + (int)rank) * TC_BM + quad * 32;
+            const int row0 = (2 * tile_m + (int)rank) * TC_BM + quad * 32, row = row0 + lane;   // the warp's first row, this thread's
             const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 256);
             auto sums_there = [&]() {
                 const bool there = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (i >> 1) & 1));
@@ -476,49 +516,118 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));
             };
-            if (!sums_there()) {
-                timed_out = true;
-                break;
-            }
-            // this warp's columns of results, up to 64 at a time
-            constexpr int OWN = EPI == TC_SWIGLU ? HALF / 2 : HALF;
-            const int col0 = (EPI == TC_SWIGLU ? tile_n * HALF : tile_n * BN) + half * OWN;
-#pragma unroll
-            for (int c = 0; c < OWN; c += 64) {
-                constexpr int W = OWN % 32 == 0 ? 32 : 16;   // columns a turn
-                const int n_cols = OWN - c < 64 ? OWN - c : 64;
-#pragma unroll
-                for (int e = 0; e < n_cols; e += W) {
-                    uint32_t packed[W / 2];
-                    if constexpr (EPI == TC_SWIGLU) {
-                        uint32_t g[W], u[W];
-                        tmem_load_two(lane_base + half * OWN + c + e, lane_base + HALF + half * OWN + c + e, g, u);
-#pragma unroll
-                        for (int j = 0; j < W / 2; ++j)
-                            packed[j] = pack_bf16(fast_silu(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
-                                                  fast_silu(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
-                    } else {
-                        uint32_t v[W];
-                        if constexpr (W == 32) tmem_load_32(lane_base + half * OWN + c + e, v);
-                        else tmem_load_16(lane_base + half * OWN + c + e, v);
-#pragma unroll
-                        for (int j = 0; j < W / 2; ++j) packed[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+            if constexpr (EPI == TC_QKV) {
+                constexpr int D = 2 * P, Q = P / 2;   // this thread makes pairs [half * Q, half * Q + Q) of every head in its row
+                // under the tile's products: the row's angles and its place in the cache
+                const int pos = row < M ? qa.tok_pos[row] : 0;
+                long long kv_at = -1;                 // element offset in the cache, -1: nowhere
+                if (row < M && qa.write_cache) {
+                    const int slot = qa.slots[qa.tok_seq[row]];
+                    if (slot >= 0) {
+                        const int page = qa.table[(long long)slot * qa.table_stride + pos / QF_PAGE];
+                        if (page < 0) atomicOr(err, QF_ERR_NO_PAGE);
+                        else kv_at = (long long)page * qa.page_elems + (long long)(pos % QF_PAGE) * D;
                     }
-#pragma unroll
-                    for (int j = 0; j < W / 8; ++j)
-                        *patch_at(patch, lane, e / 8 + j) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
                 }
-                if (c + 64 >= OWN) sums_read();
-                else __syncwarp();
-                // n_out is a multiple of eight: a piece is whole or beyond the matrix
-                const int pieces = n_cols / 8;
+                float2 cs[Q];
 #pragma unroll
-                for (int u = 0; u < pieces; ++u) {
-                    const int r = (u * 32 + lane) / pieces, piece = (u * 32 + lane) % pieces, col = col0 + c + 8 * piece;
-                    if (row0 + r < M && col < n_out)
-                        *reinterpret_cast<uint4*>(out + (size_t)(row0 + r) * ldo + col) = *patch_at(patch, r, piece);
+                for (int j = 0; j < Q; ++j) {
+                    cs[j] = make_float2(1.f, 0.f);
+                    if (qa.inv_freq) sincosf((float)pos * __ldg(qa.inv_freq + half * Q + j), &cs[j].y, &cs[j].x);
                 }
-                __syncwarp();
+                // A head goes out by way of the quadrant's two patches: 128 bytes a row in one (D = 64), first halves in one and
+                // second halves in the other (D = 128). Each warp then stores half of the quadrant's rows, eight lanes a row.
+                unsigned char* shared = patches + quad * 2 * TP_PATCH_BYTES;
+                long long out_at[4];
+                int out_row[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int r = (half * 4 + u) * 4 + (lane >> 3);
+                    out_row[u] = row0 + r, out_at[u] = __shfl_sync(0xffffffffu, kv_at, r);
+                }
+                // after a wait that ran out a warp still passes all barriers below, where its quadrant's other warp may wait for it
+                if (!timed_out && !sums_there()) timed_out = true;
+#pragma unroll 1
+                for (int h = 0; h < BN / D; ++h) {
+                    const int head = tile_n * (BN / D) + h;
+                    if (head >= qa.n_heads + 2 * qa.kv_heads) break;
+                    unsigned char* at = D == 64 ? shared + (h & 1) * TP_PATCH_BYTES : shared;
+                    const bool rotate = qa.inv_freq != nullptr && head < qa.n_heads + qa.kv_heads;
+#pragma unroll
+                    for (int j0 = 0; j0 < Q; j0 += 16) {   // 16 pairs a turn
+                        const uint32_t lo = lane_base + h * D + half * Q + j0;
+                        const bf16* bias = qa.bias ? qa.bias + head * D + half * Q + j0 : nullptr;
+                        uint4 first[2], second[2];
+                        rotated_pairs(lo, lo + P, bias, bias + P, cs + j0, rotate, first, second);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            *patch_at(at, lane, half * (Q / 8) + j0 / 8 + j) = first[j];
+                            if (D == 64) *patch_at(at, lane, 4 + half * (Q / 8) + j0 / 8 + j) = second[j];
+                            else *patch_at(at + TP_PATCH_BYTES, lane, half * (Q / 8) + j0 / 8 + j) = second[j];
+                        }
+                    }
+                    quadrant_sync(quad);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (out_row[u] >= M || timed_out) continue;
+                        bf16* dst = nullptr;
+                        if (head < qa.n_heads) dst = qa.q_out + ((size_t)out_row[u] * qa.n_heads + head) * D;
+                        else if (out_at[u] >= 0) dst = qa.kv_base + out_at[u] + (long long)(head - qa.n_heads) * QF_PAGE * D;   // keys, then values
+                        if (!dst) continue;
+                        const int r = (half * 4 + u) * 4 + (lane >> 3);
+#pragma unroll
+                        for (int part = 0; part < D / 64; ++part)
+                            *reinterpret_cast<uint4*>(dst + part * 64 + (lane & 7) * 8) = *patch_at(at + part * TP_PATCH_BYTES, r, lane & 7);
+                    }
+                    if (D == 128) quadrant_sync(quad);   // (D = 64: the next head goes by the other patch, and the one after by a barrier more)
+                }
+                if (D == 64) quadrant_sync(quad);
+                if (!timed_out) sums_read();
+            } else {
+                if (!sums_there()) {
+                    timed_out = true;
+                    break;
+                }
+                // this warp's columns of results, up to 64 at a time
+                constexpr int OWN = EPI == TC_SWIGLU ? HALF / 2 : HALF;
+                const int col0 = (EPI == TC_SWIGLU ? tile_n * HALF : tile_n * BN) + half * OWN;
+#pragma unroll
+                for (int c = 0; c < OWN; c += 64) {
+                    constexpr int W = OWN % 32 == 0 ? 32 : 16;   // columns a turn
+                    const int n_cols = OWN - c < 64 ? OWN - c : 64;
+#pragma unroll
+                    for (int e = 0; e < n_cols; e += W) {
+                        uint32_t packed[W / 2];
+                        if constexpr (EPI == TC_SWIGLU) {
+                            uint32_t g[W], u[W];
+                            tmem_load_two(lane_base + half * OWN + c + e, lane_base + HALF + half * OWN + c + e, g, u);
+#pragma unroll
+                            for (int j = 0; j < W / 2; ++j)
+                                packed[j] = pack_bf16(fast_silu(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
+                                                      fast_silu(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]));
+                        } else {
+                            uint32_t v[W];
+                            if constexpr (W == 32) tmem_load_32(lane_base + half * OWN + c + e, v);
+                            else tmem_load_16(lane_base + half * OWN + c + e, v);
+#pragma unroll
+                            for (int j = 0; j < W / 2; ++j) packed[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                        }
+#pragma unroll
+                        for (int j = 0; j < W / 8; ++j)
+                            *patch_at(patch, lane, e / 8 + j) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+                    }
+                    if (c + 64 >= OWN) sums_read();
+                    else __syncwarp();
+                    // n_out is a multiple of eight: a piece is whole or beyond the matrix
+                    const int pieces = n_cols / 8;
+#pragma unroll
+                    for (int u = 0; u < pieces; ++u) {
+                        const int r = (u * 32 + lane) / pieces, piece = (u * 32 + lane) % pieces, col = col0 + c + 8 * piece;
+                        if (row0 + r < M && col < n_out)
+                            *reinterpret_cast<uint4*>(out + (size_t)(row0 + r) * ldo + col) = *patch_at(patch, r, piece);
+                    }
+                    __syncwarp();
+                }
             }
         }
     }
@@ -530,13 +639,13 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32  %0, %1;" ::"r"(tmem), "r"(512));
 }
 
-template <int EPI, int BN>
+template <int EPI, int BN, int P = 0>
 static int launch_pair(const CUtensorMap& map_a, const void* w, int w_rows, int ldw, void* out, int m, int n_out, int k, int inter,
-                       int ldo, int* err, cudaStream_t stream) {
+                       int ldo, int* err, cudaStream_t stream, const TcQkvArgs& qa = TcQkvArgs{}) {
     constexpr size_t smem = PairGeometry<BN>::smem;
     CUtensorMap map_b;                // boxes of a block's half of a tile's weight rows
     if (!qf_make_map_bf16(&map_b, w, w_rows, k, ldw, BN / 2)) return (int)cudaErrorNotSupported;
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_pair_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(tc_gemm_pair_kernel<EPI, BN, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int tile_cols = EPI == TC_SWIGLU ? BN / 2 : BN;
     const int m_tiles = (m + 2 * TC_BM - 1) / (2 * TC_BM), n_tiles = (n_out + tile_cols - 1) / tile_cols;
@@ -545,8 +654,8 @@ static int launch_pair(const CUtensorMap& map_a, const void* w, int w_rows, int 
     long long group_n = (32ll << 20) / ((long long)BN * k * 2);
     group_n = group_n < 4 ? 4 : group_n;
     group_n = group_n > n_tiles ? n_tiles : group_n;
-    return (int)launch_pdl(tc_gemm_pair_kernel<EPI, BN>, dim3(2 * (total < pairs ? total : pairs)), dim3(TP_THREADS), smem, stream,
-                           map_a, map_b, (bf16*)out, m, n_out, k, inter, ldo, m_tiles, n_tiles, (int)group_n, err);
+    return (int)launch_pdl(tc_gemm_pair_kernel<EPI, BN, P>, dim3(2 * (total < pairs ? total : pairs)), dim3(TP_THREADS), smem, stream,
+                           map_a, map_b, (bf16*)out, m, n_out, k, inter, ldo, m_tiles, n_tiles, (int)group_n, err, qa);
 }
 
 // Tiles of 256 columns, or of 192 where the wide ones' last round would leave many pairs idle: a round of the narrow ones takes
@@ -686,4 +795,54 @@ QF_EXPORT int qf_tc_gemm_qkv(const void* a, int lda, const void* w, int ldw, int
     dim3 grid((n + 127) / 128, (m + TC_BM - 1) / TC_BM);
     tc_gemm_kernel<TC_QKV, 128><<<grid, TC_THREADS, smem, stream>>>(map_a, map_b, nullptr, m, n, k, 0, 0, q, err, TcGroups{});
     return (int)cudaGetLastError();
+}
+
+// Columns of the tiles of the pairs' QKV product (whole heads), and whether its tiles keep the pairs at work. A round of tiles of 192,
+// 128 and 64 columns takes 0.85, 0.75 and 0.66 of the time of one of 256 (905 x 1152 x 896: 9.4, 8.6, 8.5 and 11.1 microseconds, a round each;
+// 8192 x 1152 x 896: 24.1 in three rounds, 27.1 in four, 40.6 in eight, 27.2 in three).
+static int qkv_columns(int m, int n, int d, float* busy) {
+    const long long pairs = qf_sm_count() / 2 > 0 ? qf_sm_count() / 2 : 1, m_tiles = (m + 255) / 256;
+    const struct { int columns; float round; } forms[] = {{256, 1.f}, {192, 0.85f}, {128, 0.75f}, {64, 0.66f}};
+    int best = 0;
+    float least = 0.f;
+    for (const auto& f : forms) {
+        if (f.columns % d) continue;
+        const long long tiles = m_tiles * ((n + f.columns - 1) / f.columns), rounds = (tiles + pairs - 1) / pairs;
+        if (best == 0 || f.round * (float)rounds < least) {
+            best = f.columns, least = f.round * (float)rounds;
+            *busy = (float)tiles / (float)(rounds * pairs);
+        }
+    }
+    return best;
+}
+
+// Whether qf_tc_gemm_qkv_pairs is the faster way for these sizes, against the library's product and the rotation kernel behind it: beyond 512
+// rows where its tiles keep three quarters of the pairs at work (7358 x 2560 x 2048: 56 microseconds against 70; 1536 x 2560 x 2048 19.2
+// and 22.0, 60 of 74 pairs; 2048 x 2560 x 2048, 80 of 148, 28.7 and 26.4; 1536 x 4608 x 3584, 108 of 148, 47.8 and 44.5; 256 x 4608 x 3584
+// 20.7 and 18.4), and for heads of 64 with weights of up to 4 MB always (1152 x 896: 7.5 against 8.0 for 64 rows, 8.8 and 10.1 for 900).
+QF_EXPORT int qf_tc_gemm_qkv_pairs_pays(int m, int n, int k, int head_dim) {
+    if (m <= 0 || n <= 0 || (head_dim != 64 && head_dim != 128)) return 0;
+    if (head_dim == 64 && (long long)n * k * 2 <= (4ll << 20)) return 1;
+    float busy = 0.f;
+    qkv_columns(m, n, head_dim, &busy);
+    return m > 512 && busy >= 0.75f;
+}
+
+// The same on pairs of SMs, with the angles worked out in the epilogue (args->inv_freq; args->angles is not read): head sizes 64 and 128.
+QF_EXPORT int qf_tc_gemm_qkv_pairs(const void* a, int lda, const void* w, int ldw, int m, int k, const TcQkvArgs* args, int* err,
+                                   cudaStream_t stream) {
+    const TcQkvArgs& q = *args;
+    const int d = q.head_dim, n = (q.n_heads + 2 * q.kv_heads) * d;
+    if (m <= 0 || n <= 0) return 0;
+    if (d != 64 && d != 128) return (int)cudaErrorInvalidValue;
+    if (k <= 0 || k % 8 || lda % 8 || ldw % 8 || q.page_elems % 8) return (int)cudaErrorInvalidValue;
+    if (((uintptr_t)a | (uintptr_t)w | (uintptr_t)q.q_out | (uintptr_t)q.kv_base | (uintptr_t)q.bias) % 16) return (int)cudaErrorInvalidValue;
+    CUtensorMap map_a;
+    if (!qf_make_map_bf16(&map_a, a, m, k, lda, TC_BM)) return (int)cudaErrorNotSupported;
+#define QF_QKV(BN, P) launch_pair<TC_QKV, BN, P>(map_a, w, n, ldw, nullptr, m, n, k, 0, 0, err, stream, q)
+    float busy;
+    const int columns = qkv_columns(m, n, d, &busy);
+    if (d == 128) return columns == 256 ? QF_QKV(256, 64) : QF_QKV(128, 64);
+    return columns == 256 ? QF_QKV(256, 32) : columns == 192 ? QF_QKV(192, 32) : columns == 128 ? QF_QKV(128, 32) : QF_QKV(64, 32);
+#undef QF_QKV
 }

@@ -1174,7 +1174,7 @@ class _TcQkvArgs(ctypes.Structure):
     _fields_ = [("bias", ctypes.c_void_p), ("angles", ctypes.c_void_p), ("tok_pos", ctypes.c_void_p), ("tok_seq", ctypes.c_void_p),
                 ("slots", ctypes.c_void_p), ("q_out", ctypes.c_void_p), ("kv_base", ctypes.c_void_p), ("table", ctypes.c_void_p),
                 ("page_elems", ctypes.c_longlong), ("table_stride", _I), ("n_heads", _I), ("kv_heads", _I), ("head_dim", _I),
-                ("write_cache", _I)]
+                ("write_cache", _I), ("inv_freq", ctypes.c_void_p)]
 
 
 def rope_table(tok_pos: torch.Tensor, inv_freq: torch.Tensor, amplitude: float = 1.0) -> torch.Tensor:
@@ -1226,6 +1226,60 @@ def tc_gemm_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     if code == 801:
         raise KernelError("tc_gemm_qkv: the driver offers no tensor-map encoder (cuTensorMapEncodeTiled)")
     _check(code, "tc_gemm_qkv")
+
+
+QKV_PRODUCT_HEAD_DIMS = (64, 128)
+
+
+def qkv_product_takes(x: torch.Tensor, weight: torch.Tensor, rot_dim: int, site: KvSiteArgs) -> bool:
+    """Whether `qkv_product` takes these operands: what `tc_gemm_takes` asks, heads of 64 or 128 that are rotated whole or not at
+    all, and cache pages on 16-byte boundaries."""
+    return (site.head_dim in QKV_PRODUCT_HEAD_DIMS and rot_dim in (0, site.head_dim) and tc_gemm_takes(x, weight)
+            and site.page_elems % 8 == 0 and site.storage.data_ptr() % 16 == 0)
+
+
+def qkv_product_pays(m: int, weight: torch.Tensor, head_dim: int) -> bool:
+    """Whether `qkv_product` is the faster way for m rows, against `linear` and `rope_cache_write`."""
+    return library("tc_gemm").qf_tc_gemm_qkv_pairs_pays(_I(m), _I(weight.shape[0]), _I(weight.shape[1]), _I(head_dim)) != 0
+
+
+def qkv_product(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], inv_freq: Optional[torch.Tensor],
+                tok_seq: torch.Tensor, tok_pos: torch.Tensor, slots: torch.Tensor, n_heads: int, q_out: torch.Tensor,
+                site: KvSiteArgs, write_cache: bool, err: torch.Tensor) -> None:
+    """The query/key/value product of many token rows on pairs of SMs, with its bias, the rotation of q and k heads (angles
+    tok_pos * inv_freq, float32 [head_dim / 2]; None: no rotation) and the writes in its epilogue: q to `q_out`
+    [tokens, n_heads * head_dim], k and v to each token's place in its sequence's cache page."""
+    _dev("x", x, torch.bfloat16, contiguous=False)
+    _dev("weight", weight, torch.bfloat16, contiguous=False)
+    _dev("q_out", q_out, torch.bfloat16)
+    _dev("cache", site.storage, torch.bfloat16)
+    _dev("tok_seq", tok_seq, torch.int32)
+    _dev("tok_pos", tok_pos, torch.int32)
+    _dev("slots", slots, torch.int32)
+    d = site.head_dim
+    m, k = x.shape
+    if weight.shape != ((n_heads + 2 * site.kv_heads) * d, k) or q_out.shape != (m, n_heads * d):
+        raise KernelError("qkv_product: weight must be [(n_heads + 2 kv_heads) * head_dim, K] and q_out [tokens, n_heads * head_dim]")
+    if not qkv_product_takes(x, weight, 0 if inv_freq is None else 2 * inv_freq.numel(), site) or q_out.data_ptr() % 16:
+        raise KernelError(f"qkv_product: head_dim {d} (taken: {QKV_PRODUCT_HEAD_DIMS}), the rotated part or the operands' alignment is not taken")
+    if inv_freq is not None:
+        _dev("inv_freq", inv_freq, torch.float32)
+    if bias is not None:
+        _dev("bias", bias, torch.bfloat16)
+        if bias.numel() != weight.shape[0]:
+            raise KernelError("qkv_product: bias must have one element per projection column")
+    a = _TcQkvArgs()
+    a.bias = None if bias is None else bias.data_ptr()
+    a.inv_freq = None if inv_freq is None else inv_freq.data_ptr()
+    a.tok_pos, a.tok_seq, a.slots = tok_pos.data_ptr(), tok_seq.data_ptr(), slots.data_ptr()
+    a.q_out, a.kv_base, a.table = q_out.data_ptr(), site.storage.data_ptr(), site.table.data_ptr()
+    a.page_elems, a.table_stride = site.page_elems, site.table_stride
+    a.n_heads, a.kv_heads, a.head_dim, a.write_cache = n_heads, site.kv_heads, d, int(bool(write_cache))
+    code = library("tc_gemm").qf_tc_gemm_qkv_pairs(_ptr(x), _I(x.stride(0)), _ptr(weight), _I(weight.stride(0)), _I(m), _I(k),
+                                                   ctypes.byref(a), _ptr(err), _stream())
+    if code == 801:
+        raise KernelError("qkv_product: the driver offers no tensor-map encoder (cuTensorMapEncodeTiled)")
+    _check(code, "qkv_product")
 
 
 def tc_gemm_is_persistent(epilogue: int, m: int, n: int) -> bool:

@@ -220,6 +220,8 @@ class GqaAttention(Mixer):
             libs |= {"attention_decode", "attention_prefill", "skinny_gemm", "wide_gemm", "fold_project"}
             if self.head_dim in ops.TC_ATTENTION_HEAD_DIMS:
                 libs.add("attention_prefill_tc")
+            if self.head_dim in ops.QKV_PRODUCT_HEAD_DIMS:
+                libs.add("tc_gemm")
         return libs
 
     def cache_need(self):
@@ -297,20 +299,22 @@ class GqaAttention(Mixer):
                 and self.head_dim in ops.FAST_ATTENTION_HEAD_DIMS)
         plan = self.decode_plan(ctx) if fast and ctx.is_decode else None
         rotary = self.position.fused_rotary() if self.position is not None else None
-        # (The product with bias, rotation and cache write in its epilogue, `ops.tc_gemm_qkv`, was measured inside the
-        # prompt graph of 2,048 tokens at Qwen2.5-0.5B sizes: 2.88 ms for the step against 2.76 with the library product
-        # and the rotation kernel; it is not used here.)
-        late_bias = self.position is None or rotary is not None  # the kernel that rotates and stores adds the bias
-        qkv = ops.linear(x, self.qkv_weight, None if late_bias else self.qkv_bias_t)
-        if self.position is not None and rotary is None:
-            q_view = qkv[:, :self.q_width].view(n, self.n_heads, self.head_dim)
-            k_view = qkv[:, self.q_width:self.q_width + self.kv_width].view(n, self.n_kv, self.head_dim)
-            self.position.apply(q_view, k_view, ctx)
         inv_freq, rot_dim = rotary if rotary is not None else (None, 0)
         q = torch.empty((n, self.q_width), dtype=x.dtype, device=x.device)
         args = ops.KvSiteArgs(site.storage, site.table, self.n_kv, self.head_dim)
-        ops.rope_cache_write(qkv, ctx.tok_seq, ctx.tok_pos, ctx.slots, inv_freq, rot_dim, self.n_heads, q, args,
-                             writes_cache, ctx.err, bias=self.qkv_bias_t if late_bias else None)
+        late_bias = self.position is None or rotary is not None  # the kernel that rotates and stores adds the bias
+        if (fast and late_bias and ops.qkv_product_takes(x, self.qkv_weight, rot_dim, args)
+                and ops.qkv_product_pays(n, self.qkv_weight, self.head_dim)):
+            ops.qkv_product(x, self.qkv_weight, self.qkv_bias_t, inv_freq, ctx.tok_seq, ctx.tok_pos, ctx.slots, self.n_heads, q, args,
+                            writes_cache, ctx.err)
+        else:
+            qkv = ops.linear(x, self.qkv_weight, None if late_bias else self.qkv_bias_t)
+            if not late_bias:
+                q_view = qkv[:, :self.q_width].view(n, self.n_heads, self.head_dim)
+                k_view = qkv[:, self.q_width:self.q_width + self.kv_width].view(n, self.n_kv, self.head_dim)
+                self.position.apply(q_view, k_view, ctx)
+            ops.rope_cache_write(qkv, ctx.tok_seq, ctx.tok_pos, ctx.slots, inv_freq, rot_dim, self.n_heads, q, args,
+                                 writes_cache, ctx.err, bias=self.qkv_bias_t if late_bias else None)
         attended = torch.empty_like(q)
         if fast and ctx.is_decode:
             ops.attention_decode(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,

@@ -34,3 +34,54 @@ def test_edges_of_pair_tiles(gated, m, cols, k, columns):
     assert int(err) == 0
     assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-30).all())   # float32 sums, rounded once to eight bits
     assert bool((rows[0] == 7).all() and (rows[-1] == 7).all() and (rows[:, :8] == 7).all() and (rows[:, -8:] == 7).all())
+
+
+# every width of tiles (64, 128, 192 and 256 columns of heads of 64; 128 and 256 of heads of 128): ragged rows, columns and K, rows without
+# a slot, a cache that is not written, no rotation, no bias
+@pytest.mark.parametrize("m,heads,kv_heads,dim,k,rotated,biased", [
+    (301, 14, 2, 64, 896, True, True), (2047, 14, 2, 64, 72, True, True), (3001, 14, 2, 64, 136, True, False), (4601, 12, 2, 64, 64, True, True),
+    (257, 5, 1, 64, 8, False, True), (300, 16, 2, 128, 200, True, True), (1537, 16, 2, 128, 1032, True, True), (130, 3, 1, 128, 64, False, False)])
+def test_queries_keys_and_values_of_pairs(m, heads, kv_heads, dim, k, rotated, biased):
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(m)
+    n, first = (heads + 2 * kv_heads) * dim, [700, 0, 63]
+    lengths = [m - m // 3 - 40, 40, m // 3]                    # three sequences, the second one without a slot
+    x = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(n, k, generator=g, device=DEV) * k ** -0.5).bfloat16()
+    bias = torch.randn(n, generator=g, device=DEV).bfloat16() if biased else None
+    inv = 1e6 ** (-torch.arange(0, dim, 2, device=DEV).float() / dim) if rotated else None
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    seq = ints(sum(([i] * c for i, c in enumerate(lengths)), []))
+    pos = ints(sum((list(range(f, f + c)) for f, c in zip(first, lengths)), []))
+    pages = 2 * (-(-(700 + m) // 64))
+    table = torch.randperm(pages, generator=g, device=DEV).int().view(2, -1).contiguous()
+    storage = torch.full((pages, 2, kv_heads, 64, dim), 7.0, dtype=torch.bfloat16, device=DEV)
+    site, slots, err = ops.KvSiteArgs(storage, table, kv_heads, dim), ints([1, -1, 0]), ints([0])
+    q = torch.full((m, heads * dim), 7.0, dtype=torch.bfloat16, device=DEV)
+    assert ops.qkv_product_takes(x, w, dim if rotated else 0, site)
+    ops.qkv_product(x, w, bias, inv, seq, pos, slots, heads, q, site, True, err)
+    want = x.double() @ w.double().T + (bias.double() if biased else 0)
+    slack = (x.double().abs() @ w.double().abs().T + 1) * k * 2.0 ** -24
+    want, slack = want.view(m, -1, dim).clone(), slack.view(m, -1, dim)
+    if rotated:
+        angle = (pos.float()[:, None] * inv).double()[:, None]
+        cos, sin, turned = angle.cos(), angle.sin(), want[:, :heads + kv_heads]
+        a, b = turned[..., :dim // 2].clone(), turned[..., dim // 2:].clone()
+        turned[..., :dim // 2], turned[..., dim // 2:] = a * cos - b * sin, b * cos + a * sin
+        slack = slack + slack.roll(dim // 2, -1) + 2.0 ** -21 * (want.abs() + want.roll(dim // 2, -1).abs())   # (angles rounded to float32)
+    close = lambda got, want, slack: bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-30).all())
+    assert int(err) == 0
+    assert close(q.view(m, heads, dim), want[:, :heads], slack[:, :heads])
+    written = torch.zeros(pages, 64, dtype=torch.bool, device=DEV)
+    at = table[slots[seq].clamp(min=0).long(), (pos // 64).long()].long()
+    held = (seq != 1).nonzero()[:, 0]
+    written[at[held], (pos % 64).long()[held]] = True
+    got = storage[at, :, :, (pos % 64).long()].reshape(m, 2 * kv_heads, dim)
+    assert close(got[held], want[held, heads:], slack[held, heads:])
+    assert bool((storage.permute(0, 3, 1, 2, 4)[~written] == 7).all())
+    before, again = storage.clone(), torch.empty_like(q)
+    ops.qkv_product(x, w, bias, inv, seq, pos, slots, heads, again, site, False, err)   # the queries alone
+    assert torch.equal(before, storage) and torch.equal(again, q) and int(err) == 0
+    table[0, 0] = -1                                           # the third sequence's first page is not held
+    ops.qkv_product(x, w, bias, inv, seq, pos, slots, heads, again, site, True, err)
+    assert torch.equal(before, storage) and torch.equal(again, q) and int(err) == ops.ERR_NO_PAGE
