@@ -345,7 +345,9 @@ __device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles, int gro
 __device__ __forceinline__ void quadrant_sync(int quad) { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); }
 
 // 16 neighbouring rotation pairs of a head in this thread's row of the accumulator (first halves from column `lo` of its lane, second
-// halves from `hi`), with the bias of both, rotated by cs = (cos, sin) where `rotate`, as 16-byte pieces of the row.
+// halves from `hi`), with the bias of both, rotated by cs = (cos, sin) where `rotate`, as 16-byte pieces of the row. The sums are rounded
+// to bfloat16 first, as those of a product that is stored are: a row's queries, keys and values are the same whichever way the
+// sizes of its step choose.
 __device__ __forceinline__ void rotated_pairs(uint32_t lo, uint32_t hi, const bf16* bias_lo, const bf16* bias_hi, const float2* cs,
                                               bool rotate, uint4 (&out_lo)[2], uint4 (&out_hi)[2]) {
     uint32_t x[16], y[16];
@@ -361,10 +363,12 @@ __device__ __forceinline__ void rotated_pairs(uint32_t lo, uint32_t hi, const bf
 #pragma unroll
         for (int j = 0; j < 8; j += 2) {
             float z1[2], z2[2];
+            const uint32_t p1 = pack_bf16(__uint_as_float(x[j0 + j]), __uint_as_float(x[j0 + j + 1]));
+            const uint32_t p2 = pack_bf16(__uint_as_float(y[j0 + j]), __uint_as_float(y[j0 + j + 1]));
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const float x1 = __uint_as_float(x[j0 + j + e]) + __uint_as_float(e ? b1[j / 2] & 0xffff0000u : b1[j / 2] << 16);
-                const float x2 = __uint_as_float(y[j0 + j + e]) + __uint_as_float(e ? b2[j / 2] & 0xffff0000u : b2[j / 2] << 16);
+                const float x1 = __uint_as_float(e ? p1 & 0xffff0000u : p1 << 16) + __uint_as_float(e ? b1[j / 2] & 0xffff0000u : b1[j / 2] << 16);
+                const float x2 = __uint_as_float(e ? p2 & 0xffff0000u : p2 << 16) + __uint_as_float(e ? b2[j / 2] & 0xffff0000u : b2[j / 2] << 16);
                 const float2 a = cs[j0 + j + e];
                 z1[e] = rotate ? x1 * a.x - x2 * a.y : x1;
                 z2[e] = rotate ? x2 * a.x + x1 * a.y : x2;

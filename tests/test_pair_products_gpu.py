@@ -60,8 +60,9 @@ def test_queries_keys_and_values_of_pairs(m, heads, kv_heads, dim, k, rotated, b
     q = torch.full((m, heads * dim), 7.0, dtype=torch.bfloat16, device=DEV)
     assert ops.qkv_product_takes(x, w, dim if rotated else 0, site)
     ops.qkv_product(x, w, bias, inv, seq, pos, slots, heads, q, site, True, err)
-    want = x.double() @ w.double().T + (bias.double() if biased else 0)
-    slack = (x.double().abs() @ w.double().abs().T + 1) * k * 2.0 ** -24
+    want = x.double() @ w.double().T
+    slack = (x.double().abs() @ w.double().abs().T + 1) * k * 2.0 ** -24 + want.abs() * 2.0 ** -8   # (sums rounded to eight bits before the bias)
+    want = want + (bias.double() if biased else 0)
     want, slack = want.view(m, -1, dim).clone(), slack.view(m, -1, dim)
     if rotated:
         angle = (pos.float()[:, None] * inv).double()[:, None]
