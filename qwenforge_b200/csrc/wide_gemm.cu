@@ -9,8 +9,8 @@
 //   SWIGLU    out[m][i] = silu(gate_i) * up_i
 //   QKV       + bias, rotate q and k heads by position (float32 angles), q -> q_out, k and v -> cache pages
 //
-// One block computes one tile over its share of K. A tile is 128 weight rows and one accumulator, or, where an epilogue
-// needs two weight rows together, 2 x 128 rows and two accumulators whose lane r holds the two partners: gate row r
+// One block computes one tile over its share of K. A tile is 128 weight rows (or fewer, see spread_rows) and one accumulator, or, where
+// an epilogue needs two weight rows together, 2 x 128 rows and two accumulators whose lane r holds the two partners: gate row r
 // and up row r of 128 features (SWIGLU); component j and component j + D/2 of a head, for 256 / D heads (QKV). So the
 // thread that owns lane r finishes its outputs from its own registers, and neighbouring lanes write neighbouring
 // features of a token.
@@ -27,6 +27,8 @@
 // through distributed shared memory, and the owners add them in rank order, so results do not change from run to run.
 // Every wait on a barrier is bounded; one that runs out sets QF_ERR_COPY_TIMEOUT and the block still frees its tensor
 // memory and returns. No copy uses cluster multicast.
+#include <algorithm>
+
 #include <cooperative_groups.h>
 
 #include "skinny_common.cuh"
@@ -38,7 +40,6 @@
 #define WG_ROW_THREADS (WG_ROW_WARPS * 32)
 #define WG_THREADS (WG_ROW_THREADS + 64)
 #define WG_STAGES 6
-#define WG_ACC_BYTES (WG_BM * WG_BK * 2)  // 16 KB of weights per slab and accumulator
 #define WG_MAX_TOK 64
 #define WG_MAX_SPLIT 8
 #define WG_SETS (WG_ROW_WARPS / 4)
@@ -46,7 +47,9 @@
 
 struct WideGeometry {
     int ntok;        // token columns of an accumulator: the row count rounded up to 16
-    int tiles;       // tiles of 128 accumulator lanes
+    int tiles;       // tiles of `rows` weight rows per accumulator
+    int rows;        // weight rows of an accumulator: 128 lanes, or fewer where that puts more SMs to streaming
+    int acc_bytes;   // bytes of an accumulator's weights in a slab: whole groups of eight rows
     int accs;        // accumulators of a tile: 1, or 2 where the epilogue needs two weight rows together
     int box_rows;    // weight rows of one tiled copy
     int ksplit;      // blocks of a cluster sharing a tile
@@ -116,7 +119,8 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
 
     // A stage of the ring holds `group` consecutive slabs of K: its copies are issued together, slab after slab for the
     // same weight rows, so that the memory sees runs of group x 128 contiguous bytes per row.
-    const int group = geo.group, stages = geo.stages, slab_bytes = geo.slab_bytes;
+    const int group = geo.group, stages = geo.stages, slab_bytes = geo.slab_bytes, rows = geo.rows, acc_bytes = geo.acc_bytes;
+    const uint32_t slab_arrives = (uint32_t)((ACCS * rows + ntok) * WG_BK * 2);   // bytes that a slab's copies bring
     const int n_groups = (n_kb + group - 1) / group;
     // what the row threads keep from before the products to after them
     int tok_base = 0, tok_step = 1, tok_count = 0;  // the tokens this thread finishes: tok_base + i * tok_step, i < tok_count
@@ -130,15 +134,15 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         auto slabs_of = [&](int gi) { return min(group, n_kb - gi * group); };
         auto load_w = [&](int gi, int s) {
             unsigned char* base = ring + (size_t)s * geo.stage_bytes;
-            const int first = kb_begin + gi * group, count = slabs_of(gi), box = geo.box_rows, boxes = WG_BM / box;
+            const int first = kb_begin + gi * group, count = slabs_of(gi), box = geo.box_rows, boxes = EPI == EPI_QKV ? WG_BM / box : 1;
             for (int acc = 0; acc < ACCS; ++acc)
                 for (int b = 0; b < boxes; ++b) {
                     int row;  // first weight row of this box
-                    if (EPI == EPI_SWIGLU) row = acc * a.inter + tile * WG_BM + b * box;
+                    if (EPI == EPI_SWIGLU) row = acc * a.inter + tile * rows;
                     else if (EPI == EPI_QKV) row = (tile * boxes + b) * D + acc * P;   // a box is half a head
-                    else row = tile * WG_BM + b * box;
+                    else row = tile * rows;
                     for (int j = 0; j < count; ++j)
-                        tma_load_2d(base + (size_t)j * slab_bytes + acc * WG_ACC_BYTES + (size_t)b * box * WG_BK * 2, &w_map,
+                        tma_load_2d(base + (size_t)j * slab_bytes + acc * acc_bytes + (size_t)b * box * WG_BK * 2, &w_map,
                                     (first + j) * WG_BK, row, &full_bar[s]);
                 }
         };
@@ -146,13 +150,13 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
             unsigned char* base = ring + (size_t)s * geo.stage_bytes;
             const int first = kb_begin + gi * group, count = slabs_of(gi);
             for (int j = 0; j < count; ++j)
-                tma_load_2d(base + (size_t)j * slab_bytes + ACCS * WG_ACC_BYTES, &x_map, (first + j) * WG_BK, 0, &full_bar[s]);
+                tma_load_2d(base + (size_t)j * slab_bytes + ACCS * acc_bytes, &x_map, (first + j) * WG_BK, 0, &full_bar[s]);
         };
         // weights are nobody's output: those of the first stages are on their way before the kernel before this one ends
         const int early = min(n_groups, stages);
         if (leader)
             for (int gi = 0; gi < early; ++gi) {
-                mbar_expect_tx(&full_bar[gi], (uint32_t)(slabs_of(gi) * slab_bytes));
+                mbar_expect_tx(&full_bar[gi], (uint32_t)slabs_of(gi) * slab_arrives);
                 load_w(gi, gi);
             }
         __syncwarp();
@@ -168,7 +172,7 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
                 break;
             }
             if (leader) {
-                mbar_expect_tx(&full_bar[s], (uint32_t)(slabs_of(gi) * slab_bytes));
+                mbar_expect_tx(&full_bar[s], (uint32_t)slabs_of(gi) * slab_arrives);
                 load_w(gi, s);
                 load_x(gi, s);
             }
@@ -190,10 +194,10 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
             if (leader) {
                 for (int j = 0; j < count; ++j) {
                     const unsigned char* w_s = ring + (size_t)s * geo.stage_bytes + (size_t)j * slab_bytes;
-                    const uint64_t dx = smem_desc_sw128(w_s + ACCS * WG_ACC_BYTES);
+                    const uint64_t dx = smem_desc_sw128(w_s + ACCS * acc_bytes);
 #pragma unroll
                     for (int acc = 0; acc < ACCS; ++acc) {
-                        const uint64_t dw = smem_desc_sw128(w_s + acc * WG_ACC_BYTES);
+                        const uint64_t dw = smem_desc_sw128(w_s + acc * acc_bytes);
 #pragma unroll
                         for (int k4 = 0; k4 < WG_BK / 16; ++k4)
                             umma_bf16(tmem + 64 * acc, dw + 2 * k4, dx + 2 * k4, idesc, (gi > 0 || j > 0 || k4 > 0) ? 1u : 0u);
@@ -209,16 +213,16 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         // ---- the row threads: lane r of the accumulators is weight row n0 (and its partner n1)
         const int r = (warp & 3) * 32 + lane, set = warp >> 2;
         if (EPI == EPI_SWIGLU) {
-            n0 = tile * WG_BM + r;
+            n0 = tile * rows + r;
             n1 = a.inter + n0;
-            in0 = n0 < a.inter;
+            in0 = r < rows && n0 < a.inter;
         } else if (EPI == EPI_QKV) {
             n0 = (tile * (WG_BM / P) + r / P) * D + r % P;
             n1 = n0 + P;
             in0 = n0 < a.n;
         } else {
-            n0 = tile * WG_BM + r;
-            in0 = n0 < a.n;
+            n0 = tile * rows + r;
+            in0 = r < rows && n0 < a.n;
         }
         // the tokens this thread finishes: its set's columns, or every fourth of the tokens this block owns
         if (ksplit > 1) {
@@ -380,6 +384,47 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
 // ------------------------------------------------------------------------------------------------------------------
 // Host side.
 
+// Clusters of `ksplit` blocks that start together: clusters of 8 need 8 free SMs of one processing cluster, of which a GPU of 148 SMs has
+// about 14 at once; clusters of 4 about 32. (A split whose clusters do not all start together runs in two rounds and loses more
+// than it gains.)
+static int clusters_at_once(int ksplit, int sms) { return ksplit == 1 ? sms : ksplit == 2 ? sms / 2 : ksplit == 4 ? sms * 32 / 148 : sms * 14 / 148; }
+
+// K is split over the blocks of a cluster as far as that puts more SMs to streaming, while every block still has
+// two slabs or more to multiply.
+static void split_k(int sms, WideGeometry& geo) {
+    geo.ksplit = 1;
+    while (geo.ksplit < WG_MAX_SPLIT && geo.tiles * geo.ksplit * 2 <= sms && geo.slabs >= geo.ksplit * 4 &&
+           geo.tiles <= clusters_at_once(geo.ksplit * 2, sms))
+        geo.ksplit *= 2;
+}
+
+// How `units` weight rows per accumulator are dealt to blocks: tiles of 128 of them leave many SMs without a stream (16 tiles of a
+// 3B down product, split four times along K: 64 of 148), so a tile takes fewer rows where more blocks are done sooner. A block's
+// time is the larger of its stream (62 bytes a nanosecond and SM, 6.2 terabytes a second in all) and of its products (170 nanoseconds a
+// slab and accumulator, whatever the tile's rows), a cluster's exchange counts a microsecond. Norm, gate/up and
+// down of a step of 16 rows over weights that the L2 does not hold: 3B sizes 36.6 -> 35.0 microseconds (the down product 64 -> 128 blocks),
+// 7B 75.5 -> 72.4, 0.5B 15.7 -> 14.4. Weights below 16 MB stay in tiles of 128 (0.5B's output projection in 128 blocks instead of 28
+// 6.4 against 5.8 with the norm behind it).
+static void spread_rows(int units, int sms, WideGeometry& geo) {
+    float least = 0.f;
+    geo.tiles = (units + WG_BM - 1) / WG_BM;
+    geo.box_rows = geo.rows = WG_BM;
+    split_k(sms, geo);
+    if ((long long)geo.accs * units * geo.slabs * WG_BK * 2 < (16ll << 20)) return;
+    geo.tiles = 0;
+    for (int ksplit = 1; ksplit <= WG_MAX_SPLIT && (ksplit == 1 || geo.slabs >= 2 * ksplit); ksplit *= 2) {
+        const int at_once = clusters_at_once(ksplit, sms) > 0 ? clusters_at_once(ksplit, sms) : 1;
+        const int rows = std::min(WG_BM, std::max(8, (units + at_once - 1) / at_once)), tiles = (units + rows - 1) / rows;
+        const int rounds = (tiles + at_once - 1) / at_once, per = (geo.slabs + ksplit - 1) / ksplit;
+        const float block = (float)per * (float)(geo.accs * rows + geo.ntok) * WG_BK * 2;
+        const float all = (float)geo.accs * (float)units * (float)geo.slabs * WG_BK * 2 / 6200.f;   // nanoseconds
+        const float stream = std::max((float)rounds * block / 62.f, all), products = (float)rounds * (float)(per * geo.accs) * 170.f;
+        const float time = std::max(stream, products) + (ksplit > 1 ? 1000.f : 0.f);
+        if (geo.tiles == 0 || time < least) least = time, geo.rows = rows, geo.tiles = tiles, geo.ksplit = ksplit;
+    }
+    geo.box_rows = geo.rows;
+}
+
 // The geometry of a product, or false if this kernel does not take it: 1 <= m <= 64 token rows `x` (bf16, rows a
 // multiple of 8 elements apart, 16-byte aligned), K a multiple of 8, weight rows likewise; QKV: half a head divides
 // 128 lanes and is 8 rows or more, and the whole head is rotated if any of it is.
@@ -387,17 +432,19 @@ static bool wide_plan(int epilogue, const SkinnyArgs& a, int sms, WideGeometry& 
     if (sms <= 0 || a.m < 1 || a.m > WG_MAX_TOK || a.k <= 0 || a.k % 8 || a.ldw % 8 || a.ldx % 8 || a.n <= 0 || !a.x) return false;
     if (((uintptr_t)a.w | (uintptr_t)a.x) % 16) return false;
     geo.accs = 1;
-    geo.box_rows = 64;
+    geo.rows = WG_BM;
+    geo.ntok = (a.m + 15) / 16 * 16;
+    geo.slabs = (a.k + WG_BK - 1) / WG_BK;
     size_t angles = 0;
     switch (epilogue) {
         case EPI_PLAIN:
         case EPI_RESIDUAL:
-            geo.tiles = (a.n + WG_BM - 1) / WG_BM;
+            spread_rows(a.n, sms, geo);
             break;
         case EPI_SWIGLU:
             if (a.inter <= 0 || a.n != 2 * a.inter || a.bias) return false;
-            geo.tiles = (a.inter + WG_BM - 1) / WG_BM;
             geo.accs = 2;
+            spread_rows(a.inter, sms, geo);
             break;
         case EPI_QKV: {
             const int half = a.head_dim / 2;
@@ -409,25 +456,19 @@ static bool wide_plan(int epilogue, const SkinnyArgs& a, int sms, WideGeometry& 
             geo.accs = 2;
             geo.box_rows = half;
             angles = 2 * (size_t)WG_MAX_TOK * half * 4;
+            split_k(sms, geo);
             break;
         }
         default:
             return false;
     }
     if (geo.tiles < 1) return false;
-    geo.ntok = (a.m + 15) / 16 * 16;
-    geo.slabs = (a.k + WG_BK - 1) / WG_BK;
-    geo.slab_bytes = geo.accs * WG_ACC_BYTES + geo.ntok * WG_BK * 2;
-    // K is split over the blocks of a cluster as far as that puts more SMs to streaming, while every block still has
-    // two slabs or more to multiply
-    // (clusters of 8 need 8 free SMs of one processing cluster, of which a GPU of 148 SMs has about 14 at once; clusters
-    // of 4 about 32: a split whose clusters do not all start together runs in two rounds and loses more than it gains)
-    geo.ksplit = 1;
-    while (geo.ksplit < WG_MAX_SPLIT && geo.tiles * geo.ksplit * 2 <= sms && geo.slabs >= geo.ksplit * 4 &&
-           geo.tiles <= (geo.ksplit * 2 == 8 ? sms * 14 / 148 : sms * 32 / 148))
-        geo.ksplit *= 2;
+    geo.acc_bytes = (geo.rows + 7) / 8 * 8 * WG_BK * 2;
+    geo.slab_bytes = geo.accs * geo.acc_bytes + geo.ntok * WG_BK * 2;
     const int per = (geo.slabs + geo.ksplit - 1) / geo.ksplit;
-    const size_t extra = (geo.ksplit > 1 ? (size_t)geo.ntok * geo.accs * WG_BM * 4 : 0) + angles;
+    // (the products read 128 rows wherever a tile has fewer: behind the last slab's there must be room for that)
+    const int beyond = WG_BM * WG_BK * 2 - geo.acc_bytes - geo.ntok * WG_BK * 2;
+    const size_t extra = (geo.ksplit > 1 ? (size_t)geo.ntok * geo.accs * WG_BM * 4 : 0) + angles + (beyond > 0 ? beyond : 0);
     // stages of four slabs (512 contiguous bytes per weight row and refill) while two of them fit, else of two, else one
     for (geo.group = 4; geo.group >= 1; geo.group /= 2) {
         geo.stage_bytes = geo.group * geo.slab_bytes;

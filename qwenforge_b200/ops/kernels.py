@@ -918,6 +918,22 @@ def qkv_product_way(m: int, weight: torch.Tensor, n_heads: int, kv_heads: int, h
     return "wide" if wide and (m <= 48 or size < 20e6) else "unfused"
 
 
+def gate_product_way(m: int, weight: torch.Tensor) -> str:
+    """How `m` token rows (64 at most) are normalised, multiplied by a [gate | up] weight and gated fastest: "skinny" (the mma.sync
+    streamer with all of it inside), "wide" (a norm kernel, then the tcgen05 streamer with the gate in its epilogue) or "unfused" (norm,
+    library product, gate kernel). Measured as norm, gate/up and down together over weights that the L2 does not hold, microseconds,
+    the other way / "wide": 17 MB (Qwen2.5-0.5B's) 8 rows 10.4 / 13.2, 9 rows 14.9 / 14.4, 16 rows 15.1 / 14.4, 24 rows 16.8 / 15.7, 48 rows
+    18.1 / 17.6, 64 rows 17.7 / 18.7; 55 MB 1 row 23.5 / 22.0, 8 rows 24.9 / 23.1, 16 rows 27.6 / 23.8, 24 rows 25.3 / 24.9, 64 rows
+    27.8 / 26.8; 90 MB (3B's) 1 row 32.3 / 33.1, 4 rows 34.2 / 33.4, 8 rows 34.8 / 33.8, 16 rows 35.8 / 35.0, 64 rows 40.8 / 38.4; 272 MB (7B's)
+    1 row 76.9 / 69.5, 16 rows 79.5 / 72.4, 64 rows 85.2 / 78.3."""
+    size = weight.numel() * weight.element_size()
+    skinny = m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_SWIGLU, True) and skinny_gemm_pays(m, weight)
+    least = 16e6 if 9 <= m <= 48 else 32e6 if m >= 4 else 100e6
+    if (size >= least or (not skinny and size >= 100e6)) and wide_gemm_takes_rows(EPI_SWIGLU, m, weight):
+        return "wide"
+    return "skinny" if skinny else "unfused"
+
+
 def residual_product_way(m: int, weight: torch.Tensor) -> str:
     """How `m` token rows (64 at most) are multiplied by `weight` [N, K] and added into the residual stream fastest, by
     measurement on a B200 (`python -m qwenforge_b200.measure products`, Qwen2.5 0.5B / 3B / 7B sizes).

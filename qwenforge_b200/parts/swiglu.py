@@ -52,20 +52,12 @@ class SwiGlu(FeedForward):
         return ops.linear(act, self.down_weight)
 
     # ---- the form for steps of up to 64 tokens that works on the residual stream in place: norm + gate/up + SwiGLU in
-    # one kernel, down + residual in another. Each of the two products goes the way that is fastest by measurement
-    # (`python -m qwenforge_b200.measure products`). Gate/up: the mma.sync streamer where it takes the shape and pays
-    # (`ops.skinny_gemm_pays`); the tcgen05 streamer after the norm kernel for weights of 100 MB and more (Qwen2.5-7B:
-    # 50 microseconds against 52 unfused and 56 to 62 in the mma.sync streamer); else norm kernel, library product and
-    # gate kernel. Down: `ops.residual_product_way`.
+    # one kernel, down + residual in another. Each of the two products goes the way that is fastest by measurement. Gate/up: the
+    # tcgen05 streamer after the norm kernel where `ops.gate_product_way` says so; else the mma.sync streamer where it takes the
+    # shape and pays (`ops.skinny_gemm_pays`); else norm kernel, library product and gate kernel. Down: `ops.residual_product_way`.
     def _ways(self, ctx):
         rows = ctx.n_tokens
-        gate_up = "unfused"
-        if (rows <= ops.SKINNY_MAX_ROWS and ops.skinny_gemm_takes(rows, self.gate_up_weight, ops.EPI_SWIGLU, True)
-                and ops.skinny_gemm_pays(rows, self.gate_up_weight)):
-            gate_up = "skinny"
-        elif self.gate_up_weight.numel() * 2 >= 100e6 and ops.wide_gemm_takes_rows(ops.EPI_SWIGLU, rows, self.gate_up_weight):
-            gate_up = "wide"
-        return gate_up, ops.residual_product_way(rows, self.down_weight)
+        return ops.gate_product_way(rows, self.gate_up_weight), ops.residual_product_way(rows, self.down_weight)
 
     def fused_takes(self, ctx) -> bool:
         return (ctx.dtype == torch.bfloat16 and ctx.attention == "auto" and self.inter % 8 == 0
