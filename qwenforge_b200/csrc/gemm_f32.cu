@@ -22,28 +22,31 @@ __device__ __forceinline__ float2 halves(f32x2 x) {
     return r;
 }
 
-// A block makes a BM x BN tile with 32 * WM * WN threads; a warp makes (BM / WM) x (BN / WN) of it, its 4 x 8 lanes TM x TN each in
-// runs of four rows and columns, so that the lanes of a warp read a k's rows and columns of both operands as whole 16-byte
-// pieces without conflicts. BK columns of K at a time, the next ones on their way through registers (they are turned on the
-// way into shared memory). What bounds it is the multiply-add pipe (72 TFLOP/s) and the last tiles' round: 1,031 rows of the
-// 0.5B model's products (30.6 GFLOP) took 1,441 microseconds with 64 x 64 tiles read by single words, 845 so; 2,048 x 22,016 x 2,048
-// runs at 51 TFLOP/s (27 before).
-template <int BM, int BN, int BK, int WM, int WN>
-__global__ void __launch_bounds__(32 * WM * WN)
+// A block makes a BM x BN tile with WM x WN warps; a warp makes (4 TM) x (8 TN) of it, its 4 x 8 lanes TM x TN each in runs of four rows
+// and columns, so that the lanes of a warp read a k's rows and columns of both operands as whole 16-byte pieces without conflicts. 16
+// or 32 columns of K at a time, the next ones on their way through registers: they are turned on the way into shared memory, where
+// the rows of every eight k are swapped among themselves so that a warp's stores of four k a lane meet all 32 banks. Rows go two to
+// a register pair, and a column's number twice into one.
+// What bounds it is the multiply-add pipe (72 TFLOP/s; 79% of its cycles on 96 x 128 tiles) and, for small tiles, the shared memory's loads
+// (90% on 64 x 64), then the last tiles' round. 1,031 rows of the 0.5B model's products (30.6 GFLOP): 1,441 microseconds with 64 x 64
+// tiles read by single words, 840 with 64 x 128 and 64 x 64 tiles whose stores met half the banks, 714 so; 1,031 x 22,016 x 2,048
+// 1,911 before and 1,631 (57 TFLOP/s).
+template <int TM, int TN, int WM, int WN, int BK>
+__global__ void __launch_bounds__(32 * WM * WN, TM * TN >= 128 ? 256 / (32 * WM * WN) : TM * TN >= 64 ? 384 / (32 * WM * WN) : 512 / (32 * WM * WN))
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                 float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int vec) {
-    constexpr int THREADS = 32 * WM * WN, TM = BM / WM / 4, TN = BN / WN / 8, LA = BM + 4, LW = BN + 4, Q = BK / 4;
+    constexpr int THREADS = 32 * WM * WN, BM = 4 * TM * WM, BN = 8 * TN * WN, LA = BM + 4, LW = BN + 4, Q = BK / 4, SWAP = BK == 16 ? 8 : 4;
     constexpr int A_EACH = BM * Q / THREADS, W_EACH = BN * Q / THREADS;
-    static_assert(TM % 4 == 0 && TN % 4 == 0 && A_EACH >= 1 && W_EACH >= 1, "whole runs of four");
+    static_assert(TM % 4 == 0 && TN % 4 == 0 && BM * Q % THREADS == 0 && BN * Q % THREADS == 0 && BM % 16 == 0 && BN % 16 == 0, "whole runs of four");
     __shared__ __align__(16) float a_s[2][BK][LA], w_s[2][BK][LW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int row0 = (warp / WN) * (BM / WM) + (lane >> 3) * 4, col0 = (warp % WN) * (BN / WN) + (lane & 7) * 4;
-    f32x2 acc[TM][TN / 2];
+    const int row0 = (warp / WN) * 4 * TM + (lane >> 3) * 4, col0 = (warp % WN) * 8 * TN + (lane & 7) * 4;
+    f32x2 acc[TM / 2][TN];            // rows 2 i and 2 i + 1 of column j
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-        for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
 
     // four neighbouring k of a row per piece; rows beyond M or N and columns beyond K are zeros
     float4 a_next[A_EACH], w_next[W_EACH];
@@ -75,15 +78,16 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
         }
     };
     auto stash = [&](int buf) {
+        const int k = (threadIdx.x % Q) * 4, swap = k / 8 * SWAP;
 #pragma unroll
         for (int u = 0; u < A_EACH; ++u) {
-            const int i = threadIdx.x + u * THREADS, r = i / Q, k = (i % Q) * 4;
+            const int r = ((threadIdx.x + u * THREADS) / Q) ^ swap;
             a_s[buf][k][r] = a_next[u].x, a_s[buf][k + 1][r] = a_next[u].y;
             a_s[buf][k + 2][r] = a_next[u].z, a_s[buf][k + 3][r] = a_next[u].w;
         }
 #pragma unroll
         for (int u = 0; u < W_EACH; ++u) {
-            const int i = threadIdx.x + u * THREADS, r = i / Q, k = (i % Q) * 4;
+            const int r = ((threadIdx.x + u * THREADS) / Q) ^ swap;
             w_s[buf][k][r] = w_next[u].x, w_s[buf][k + 1][r] = w_next[u].y;
             w_s[buf][k + 2][r] = w_next[u].z, w_s[buf][k + 3][r] = w_next[u].w;
         }
@@ -95,23 +99,23 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
         if (k0 + BK < K) fetch(k0 + BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
-            float a[TM];
-            f32x2 w[TN / 2];
+            f32x2 a[TM / 2];
+            float w[TN];
 #pragma unroll
             for (int i = 0; i < TM; i += 4) {   // runs of four rows, 16 rows apart
-                const float4 v = *reinterpret_cast<const float4*>(&a_s[buf][k][row0 + 4 * i]);
-                a[i] = v.x, a[i + 1] = v.y, a[i + 2] = v.z, a[i + 3] = v.w;
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&a_s[buf][k][(row0 + 4 * i) ^ (k / 8 * SWAP)]);
+                a[i / 2] = v.x, a[i / 2 + 1] = v.y;
             }
 #pragma unroll
             for (int j = 0; j < TN; j += 4) {   // runs of four columns, 32 columns apart
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&w_s[buf][k][col0 + 8 * j]);
-                w[j / 2] = v.x, w[j / 2 + 1] = v.y;
+                const float4 v = *reinterpret_cast<const float4*>(&w_s[buf][k][(col0 + 8 * j) ^ (k / 8 * SWAP)]);
+                w[j] = v.x, w[j + 1] = v.y, w[j + 2] = v.z, w[j + 3] = v.w;
             }
 #pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                const f32x2 ai = both(a[i]);
+            for (int j = 0; j < TN; ++j) {
+                const f32x2 wj = both(w[j]);
 #pragma unroll
-                for (int j = 0; j < TN / 2; ++j) acc[i][j] = fma2(ai, w[j], acc[i][j]);
+                for (int i = 0; i < TM / 2; ++i) acc[i][j] = fma2(a[i], wj, acc[i][j]);
             }
         }
         if (k0 + BK < K) {
@@ -120,15 +124,17 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
         }
     }
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + row0 + (i / 4) * 16 + i % 4;
-        if (gm >= M) continue;
+    for (int i = 0; i < TM / 2; ++i) {
 #pragma unroll
-        for (int j = 0; j < TN / 2; ++j) {
-            const float2 v = halves(acc[i][j]);
-            const int gn = n0 + col0 + (j / 2) * 32 + (j % 2) * 2;
-            if (gn < N) C[(size_t)gm * ldc + gn] = v.x + (bias ? bias[gn] : 0.f);
-            if (gn + 1 < N) C[(size_t)gm * ldc + gn + 1] = v.y + (bias ? bias[gn + 1] : 0.f);
+        for (int h = 0; h < 2; ++h) {
+            const int gm = m0 + row0 + (i / 2) * 16 + (2 * i) % 4 + h;
+            if (gm >= M) continue;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const float2 v = halves(acc[i][j]);
+                const int gn = n0 + col0 + (j / 4) * 32 + j % 4;
+                if (gn < N) C[(size_t)gm * ldc + gn] = (h ? v.y : v.x) + (bias ? bias[gn] : 0.f);
+            }
         }
     }
 }
@@ -223,21 +229,27 @@ QF_EXPORT int qf_gemm_f32(const float* A, const float* W, const float* bias, flo
         return (int)cudaGetLastError();
     }
     const int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-    // The tile with which the busiest SM is done first. Measured at K = 896, microseconds for 1, 2 and many tiles per SM: 64 x 128
-    // 60, 97, then 41 a tile; 64 x 64 37, 60, 25; 32 x 64 29, 44, 18 (32 x 32 was never the fastest, 128 x 128 leaves too many
-    // SMs without a last tile): a first wait and a time per tile.
-    struct { int bm, bn; float wait, each; } const tiles[] = {{64, 128, 19.f, 41.f}, {64, 64, 12.f, 25.f}, {32, 64, 10.f, 18.f}};
+    // The tile with which the busiest SM is done first: a first wait and a time per tile, measured at K = 896 in microseconds (1, 4 and 18
+    // tiles per SM of 64 x 64 33, 92 and 380, of 32 x 64 24, 65 and 258; 1, 5 and 9 of 128 x 128 89, 385 and 683; 1, 6 and 12 of 96 x 128
+    // 72, 339 and 662; 1, 2 and 12 of 96 x 64 47, 74 and 382). Never the fastest by more than a twentieth: 64 x 128 and 64 x 256 with two
+    // or four warps, 32 x 64 with two warps, 128 x 64.
+    struct { int bm, bn; float wait, each; } const tiles[] = {{96, 128, 18.f, 53.7f}, {128, 128, 13.5f, 74.5f}, {96, 64, 15.f, 30.6f},
+                                                              {64, 64, 8.5f, 20.8f}, {32, 64, 8.f, 14.3f}};
     const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
     int best = 0;
     float least = 0.f;
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < 5; ++i) {
         const long long count = (long long)((M + tiles[i].bm - 1) / tiles[i].bm) * ((N + tiles[i].bn - 1) / tiles[i].bn);
         const float time = tiles[i].wait + (float)((count + sms - 1) / sms) * tiles[i].each;
         if (i == 0 || time < least) best = i, least = time;
     }
     const dim3 grid((N + tiles[best].bn - 1) / tiles[best].bn, (M + tiles[best].bm - 1) / tiles[best].bm);
-    if (best == 0) gemm_f32_kernel<64, 128, 16, 2, 2><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec);
-    else if (best == 1) gemm_f32_kernel<64, 64, 32, 2, 2><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec);
-    else gemm_f32_kernel<32, 64, 32, 2, 2><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec);
+#define QF_F32(TM, TN, BK) gemm_f32_kernel<TM, TN, 2, 2, BK><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec)
+    if (best == 0) QF_F32(12, 8, 16);
+    else if (best == 1) QF_F32(16, 8, 16);
+    else if (best == 2) QF_F32(12, 4, 16);
+    else if (best == 3) QF_F32(8, 4, 32);
+    else QF_F32(4, 4, 32);
+#undef QF_F32
     return (int)cudaGetLastError();
 }
