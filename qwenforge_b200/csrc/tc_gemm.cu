@@ -381,12 +381,19 @@ __device__ __forceinline__ void rotated_pairs(uint32_t lo, uint32_t hi, const bf
     }
 }
 
+// TC_PLAIN: the columns of W from n_out on, n_tail of them, are not rounded: their float32 sums go to tail [M][n_tail]. What a recurrent
+// mixer's gates are made of rides on its projections' product so, where it was a launch of its own (7 microseconds).
+struct TcTail {
+    float* tail;
+    int n_tail;
+};
+
 // P: rotation pairs of a head (TC_QKV; whole heads per tile)
 template <int EPI, int BN, int P = 0>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     bf16* __restrict__ out, int M, int n_out, int K, int inter, int ldo, int m_tiles, int n_tiles, int group_n,
-                    int* err, const TcQkvArgs qa) {
+                    int* err, const TcQkvArgs qa, const TcTail tail) {
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
     constexpr int STAGES = PairGeometry<BN>::stages, STAGE_BYTES = PairGeometry<BN>::stage_bytes;
@@ -613,6 +620,13 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             uint32_t v[W];
                             if constexpr (W == 32) tmem_load_32(lane_base + half * OWN + c + e, v);
                             else tmem_load_16(lane_base + half * OWN + c + e, v);
+                            const int beyond = col0 + c + e - n_out;   // of the turn's first column
+                            if (tail.n_tail > 0 && beyond > -W && beyond < tail.n_tail && row0 + lane < M) {
+                                float* dst = tail.tail + (size_t)(row0 + lane) * tail.n_tail + beyond;
+#pragma unroll
+                                for (int j = 0; j < W; ++j)
+                                    if (beyond + j >= 0 && beyond + j < tail.n_tail) dst[j] = __uint_as_float(v[j]);
+                            }
 #pragma unroll
                             for (int j = 0; j < W / 2; ++j) packed[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
                         }
@@ -645,21 +659,21 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
 template <int EPI, int BN, int P = 0>
 static int launch_pair(const CUtensorMap& map_a, const void* w, int w_rows, int ldw, void* out, int m, int n_out, int k, int inter,
-                       int ldo, int* err, cudaStream_t stream, const TcQkvArgs& qa = TcQkvArgs{}) {
+                       int ldo, int* err, cudaStream_t stream, const TcQkvArgs& qa = TcQkvArgs{}, const TcTail& tail = TcTail{}) {
     constexpr size_t smem = PairGeometry<BN>::smem;
     CUtensorMap map_b;                // boxes of a block's half of a tile's weight rows
     if (!qf_make_map_bf16(&map_b, w, w_rows, k, ldw, BN / 2)) return (int)cudaErrorNotSupported;
     cudaError_t e = cudaFuncSetAttribute(tc_gemm_pair_kernel<EPI, BN, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int tile_cols = EPI == TC_SWIGLU ? BN / 2 : BN;
-    const int m_tiles = (m + 2 * TC_BM - 1) / (2 * TC_BM), n_tiles = (n_out + tile_cols - 1) / tile_cols;
+    const int m_tiles = (m + 2 * TC_BM - 1) / (2 * TC_BM), n_tiles = (n_out + tail.n_tail + tile_cols - 1) / tile_cols;
     const int total = m_tiles * n_tiles, pairs = qf_sm_count() / 2;
     // column tiles whose weight rows together take about 32 MB, a quarter of the L2; 4 at least
     long long group_n = (32ll << 20) / ((long long)BN * k * 2);
     group_n = group_n < 4 ? 4 : group_n;
     group_n = group_n > n_tiles ? n_tiles : group_n;
     return (int)launch_pdl(tc_gemm_pair_kernel<EPI, BN, P>, dim3(2 * (total < pairs ? total : pairs)), dim3(TP_THREADS), smem, stream,
-                           map_a, map_b, (bf16*)out, m, n_out, k, inter, ldo, m_tiles, n_tiles, (int)group_n, err, qa);
+                           map_a, map_b, (bf16*)out, m, n_out, k, inter, ldo, m_tiles, n_tiles, (int)group_n, err, qa, tail);
 }
 
 // Tiles of 256 columns, or of 192 where the wide ones' last round would leave many pairs idle: a round of the narrow ones takes
@@ -849,4 +863,18 @@ QF_EXPORT int qf_tc_gemm_qkv_pairs(const void* a, int lda, const void* w, int ld
     if (d == 128) return columns == 256 ? QF_QKV(256, 64) : QF_QKV(128, 64);
     return columns == 256 ? QF_QKV(256, 32) : columns == 192 ? QF_QKV(192, 32) : columns == 128 ? QF_QKV(128, 32) : QF_QKV(64, 32);
 #undef QF_QKV
+}
+
+// a [m][lda] against w [n + n_tail][ldw]: the first n columns to out [m][ldo] in bfloat16, the others in float32 to tail [m][n_tail]. The
+// conditions of qf_tc_gemm, and n a multiple of 8.
+QF_EXPORT int qf_tc_gemm_tail(const void* a, int lda, const void* w, int ldw, void* out, int ldo, float* tail, int m, int n, int n_tail, int k,
+                              int* err, cudaStream_t stream) {
+    if (m <= 0) return 0;
+    if (n <= 0 || n_tail <= 0 || n % 8 || k <= 0 || k % 8 || lda % 8 || ldw % 8 || ldo % 8) return (int)cudaErrorInvalidValue;
+    if (((uintptr_t)a | (uintptr_t)w | (uintptr_t)out) % 16) return (int)cudaErrorInvalidValue;
+    CUtensorMap map_a;
+    if (!qf_make_map_bf16(&map_a, a, m, k, lda, TC_BM)) return (int)cudaErrorNotSupported;
+    const TcTail t{tail, n_tail};
+    return pair_columns(TC_PLAIN, m, n + n_tail) == 192 ? launch_pair<TC_PLAIN, 192>(map_a, w, n + n_tail, ldw, out, m, n, k, 0, ldo, err, stream, TcQkvArgs{}, t)
+                                                        : launch_pair<TC_PLAIN, 256>(map_a, w, n + n_tail, ldw, out, m, n, k, 0, ldo, err, stream, TcQkvArgs{}, t);
 }

@@ -1324,6 +1324,27 @@ def tc_gemm(epilogue: int, x: torch.Tensor, weight: torch.Tensor, out: torch.Ten
     _check(code, "tc_gemm")
 
 
+def tc_gemm_tail(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, tail: torch.Tensor, err: Optional[torch.Tensor] = None) -> None:
+    """x @ weight.T on pairs of SMs: the first out.shape[1] columns rounded to bfloat16, the others, float32 as they are summed, to
+    `tail` [M, N - out.shape[1]]."""
+    _dev("x", x, torch.bfloat16, contiguous=False)
+    _dev("weight", weight, torch.bfloat16, contiguous=False)
+    _dev("out", out, torch.bfloat16, contiguous=False)
+    _dev("tail", tail, torch.float32)
+    m, k = x.shape
+    n, extra = out.shape[1], tail.shape[1]
+    if weight.shape != (n + extra, k) or out.shape[0] != m or tail.shape[0] != m or out.stride(1) != 1:
+        raise KernelError(f"tc_gemm_tail: shapes {tuple(x.shape)} x {tuple(weight.shape)}^T -> {tuple(out.shape)} and {tuple(tail.shape)} do not agree")
+    if not tc_gemm_takes(x, weight) or n % 8 or out.stride(0) % 8 or out.data_ptr() % 16:
+        raise KernelError("tc_gemm_tail: operands must be bf16 with K, N and row strides multiples of 8 and 16-byte aligned")
+    err = err if err is not None else _err_word_for(x.device)
+    code = library("tc_gemm").qf_tc_gemm_tail(_ptr(x), _I(x.stride(0)), _ptr(weight), _I(weight.stride(0)), _ptr(out), _I(out.stride(0)),
+                                              _ptr(tail), _I(m), _I(n), _I(extra), _I(k), _ptr(err), _stream())
+    if code == 801:
+        raise KernelError("tc_gemm_tail: the driver offers no tensor-map encoder (cuTensorMapEncodeTiled)")
+    _check(code, "tc_gemm_tail")
+
+
 # ---------------------------------------------------------------------------------------------- parts of other designs
 
 def embed_positions(ids: torch.Tensor, tok_pos: torch.Tensor, table: torch.Tensor, positions: torch.Tensor,

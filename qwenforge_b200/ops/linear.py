@@ -83,6 +83,15 @@ def linear_rows(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch
     return linear(x, weight, None, out_dtype=out_dtype)
 
 
+def tail_rides(x: torch.Tensor, joint: torch.Tensor, n: int) -> bool:
+    """Whether x @ joint.T runs as one launch whose first n columns are bfloat16 and whose others stay float32 (`kernels.tc_gemm_tail`), and
+    is the faster way: more than 64 rows. Measured for 14 to 32 float32 columns, microseconds, two library products / one launch: n 2,688, K
+    896 10.6 / 7.9 for 128 rows, 18.8 / 12.9 for 2,048; 6,144, 2,048 14.0 / 12.9 for 65, 44.6 / 37.6 for 2,048, 107.5 / 107.9 for 6,144; 8,448,
+    2,048 104.9 / 99.8 for 4,206 (17 rows: 14.3 / 16.9)."""
+    return (x.is_cuda and x.dtype == torch.bfloat16 and joint.dtype == torch.bfloat16 and x.shape[0] > kernels.WIDE_MAX_ROWS and n % 8 == 0
+            and kernels.tc_gemm_takes(x, joint))
+
+
 def gated_rows(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, clamp=None) -> bool:
     """The fused [gate | up] product of a step of few rows with its gate in the product's epilogue, where this library's weight
     streamer takes the shape and is the faster way: out = silu(g) * u, or with clamp = (limit, alpha) the clamped gate of

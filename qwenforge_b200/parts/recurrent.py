@@ -59,6 +59,17 @@ from .base import Mixer, TensorSpec, fork, join, runs_side_by_side
 from .registry import build_part, register_part
 
 
+def _linear_and_tail(x, joint, main, tail, err):
+    """x main^T in the activation dtype and x tail^T with float32 results, for weights that lie one behind the other: `joint` is
+    [main rows | tail rows], the others its parts."""
+    if not ops.tail_rides(x, joint, main.shape[0]):
+        return ops.linear_rows(x, main), ops.linear_rows(x, tail, out_dtype=torch.float32)
+    out = torch.empty((x.shape[0], main.shape[0]), dtype=x.dtype, device=x.device)
+    rest = torch.empty((x.shape[0], tail.shape[0]), dtype=torch.float32, device=x.device)
+    ops.tc_gemm_tail(x, joint, out, rest, err)
+    return out, rest
+
+
 class MatrixMemory(Mixer):
     """params: hidden_size, num_heads, head_dim, value_dim, gate_cap, eps, floor.
     tensors: q_weight, k_weight [H*dim, W], v_weight, g_weight [H*vdim, W], o_weight [W, H*vdim], norm [H*vdim],
@@ -75,7 +86,7 @@ class MatrixMemory(Mixer):
         h, d, v = self.n_heads, self.dim, self.vdim
         self.s_offset, self.n_offset, self.m_offset = 0, h * d * v, h * d * v + h * d
         self.state_floats = h * d * v + h * d + h
-        self.proj_weight = self.gate_weight = self.gate_bias = self.norm = self.o_weight = None
+        self.joint_weight = self.proj_weight = self.gate_weight = self.gate_bias = self.norm = self.o_weight = None
 
     def tensor_specs(self):
         h, d, v, w = self.n_heads, self.dim, self.vdim, self.hidden
@@ -86,15 +97,16 @@ class MatrixMemory(Mixer):
                 TensorSpec(f("i_bias"), (h,), init="bias", keep="float32"), TensorSpec(f("f_bias"), (h,), init="bias", keep="float32")]
 
     def kernel_libraries(self, dtype):
-        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "state_chunks"})
+        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "state_chunks", "tc_gemm"})
 
     def cache_need(self):
         return StateNeed((self.state_floats,), torch.float32)
 
     def bind(self, tensors, dtype, device):
         t = lambda logical: tensors[self.file_name(logical)]
-        self.proj_weight = torch.cat((t("q_weight"), t("k_weight"), t("v_weight"), t("g_weight")), dim=0).contiguous()
-        self.gate_weight = torch.cat((t("i_weight"), t("f_weight")), dim=0).contiguous()
+        names = ("q_weight", "k_weight", "v_weight", "g_weight", "i_weight", "f_weight")
+        self.joint_weight = torch.cat([t(name) for name in names], dim=0).contiguous()
+        self.proj_weight, self.gate_weight = self.joint_weight[:-2 * self.n_heads], self.joint_weight[-2 * self.n_heads:]
         self.gate_bias = torch.cat((t("i_bias"), t("f_bias"))).to(torch.float32).contiguous()
         self.norm, self.o_weight = t("norm"), t("o_weight")
 
@@ -106,8 +118,8 @@ class MatrixMemory(Mixer):
             raise ValueError("matrix_memory: a recurrent state cannot be read from another schedule entry")
         n, h, d, v = x.shape[0], self.n_heads, self.dim, self.vdim
         f32 = dict(dtype=torch.float32, device=x.device)
-        proj = ops.linear_rows(x, self.proj_weight)                                   # [T, q | k | v | g]
-        pre = ops.linear_rows(x, self.gate_weight, out_dtype=torch.float32)           # [T, i | f], float32 sums
+        # [T, q | k | v | g] and [T, i | f], float32 sums
+        proj, pre = _linear_and_tail(x, self.joint_weight, self.proj_weight, self.gate_weight, ctx.err)
         q, k, values, gate = proj.split((h * d, h * d, h * v, h * v), dim=1)
         decay, take, floor, nq = torch.empty((4, n, h), **f32).unbind(0)
         ops.stabilized_gates(pre, self.gate_bias, self.cap, ctx.cu_q, ctx.slots, site.storage, self.m_offset, h, decay, take, floor)
@@ -141,7 +153,7 @@ class StateSpace(Mixer):
             raise ValueError(f"state_space: state_size up to {ops.OUTER_STATE_MAX_DIM} and 1 to {ops.CONV_MAX_TAPS} taps are supported")
         self.s_offset, self.conv_offset = 0, self.n_heads * self.n_state * self.vdim
         self.state_floats = self.conv_offset + (self.taps - 1) * self.channels
-        self.main_weight = self.dt_weight = self.conv_weight = self.conv_bias = self.dt_bias = self.rate_log = self.skip = None
+        self.joint_weight = self.main_weight = self.dt_weight = self.conv_weight = self.conv_bias = self.dt_bias = self.rate_log = self.skip = None
         self.norm = self.o_weight = None
 
     def tensor_specs(self):
@@ -154,16 +166,16 @@ class StateSpace(Mixer):
                 TensorSpec(f("o_weight"), (self.hidden, self.inner))]
 
     def kernel_libraries(self, dtype):
-        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "state_chunks"})
+        return {"recurrent"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "state_chunks", "tc_gemm"})
 
     def cache_need(self):
         return StateNeed((self.state_floats,), torch.float32)
 
     def bind(self, tensors, dtype, device):
         t = lambda logical: tensors[self.file_name(logical)]
-        w = t("in_weight")
-        self.main_weight = w[:self.inner + self.channels].contiguous()    # z | x | B | C
-        self.dt_weight = w[self.inner + self.channels:].contiguous()      # dt: its sums stay float32
+        self.joint_weight = t("in_weight").contiguous()
+        self.main_weight = self.joint_weight[:self.inner + self.channels]    # z | x | B | C
+        self.dt_weight = self.joint_weight[self.inner + self.channels:]      # dt: its sums stay float32
         self.conv_weight, self.conv_bias = t("conv_weight").float().contiguous(), t("conv_bias").float().contiguous()
         self.dt_bias, self.rate_log, self.skip = (t(k).float().contiguous() for k in ("dt_bias", "rate_log", "skip"))
         self.norm, self.o_weight = t("norm"), t("o_weight")
@@ -177,8 +189,8 @@ class StateSpace(Mixer):
             raise ValueError("state_space: a recurrent state cannot be read from another schedule entry")
         n, h, v, s, g = x.shape[0], self.n_heads, self.vdim, self.n_state, self.groups
         f32 = dict(dtype=torch.float32, device=x.device)
-        main = ops.linear_rows(x, self.main_weight)                                   # [T, z | x | B | C]
-        dt_pre = ops.linear_rows(x, self.dt_weight, out_dtype=torch.float32)          # [T, H], float32 sums
+        # [T, z | x | B | C] and [T, H], float32 sums
+        main, dt_pre = _linear_and_tail(x, self.joint_weight, self.main_weight, self.dt_weight, ctx.err)
         z, convolved = main.split((self.inner, self.channels), dim=1)
         xbc = torch.empty((n, self.channels), dtype=x.dtype, device=x.device)
         ops.causal_conv_silu(convolved, self.conv_weight, self.conv_bias, ctx.cu_q, ctx.tok_seq, ctx.slots, site.storage,
@@ -316,7 +328,7 @@ class GatedLinearAttention(Mixer):
         if self.dim > ops.OUTER_STATE_MAX_DIM or self.tau <= 0:
             raise ValueError(f"gated_linear_attention: head_dim up to {ops.OUTER_STATE_MAX_DIM} and a positive tau are supported")
         self.state_floats = self.n_heads * self.dim * self.vdim
-        self.proj_weight = self.a1 = self.a2 = self.a2_bias = self.norm = self.o_weight = None
+        self.joint_weight = self.proj_weight = self.a1 = self.a2 = self.a2_bias = self.norm = self.o_weight = None
 
     def tensor_specs(self):
         f, h, d, v, w = self.file_name, self.n_heads, self.dim, self.vdim, self.hidden
@@ -333,9 +345,10 @@ class GatedLinearAttention(Mixer):
 
     def bind(self, tensors, dtype, device):
         t = lambda logical: tensors[self.file_name(logical)]
-        self.proj_weight = torch.cat((t("q_weight"), t("k_weight"), t("v_weight"), t("g_weight")), dim=0).contiguous()
-        self.a1, self.a2 = t("a1").contiguous(), t("a2").contiguous()
-        self.rank = int(self.a1.shape[0])
+        self.joint_weight = torch.cat([t(name) for name in ("q_weight", "k_weight", "v_weight", "g_weight", "a1")], dim=0).contiguous()
+        self.rank = int(t("a1").shape[0])
+        self.proj_weight, self.a1 = self.joint_weight[:-self.rank], self.joint_weight[-self.rank:]
+        self.a2 = t("a2").contiguous()
         self.a2_bias = t("a2_bias").to(torch.float32).contiguous()
         self.norm = t("norm").repeat(self.n_heads).contiguous()      # the one weight [vdim] under every head
         self.o_weight = t("o_weight")
@@ -354,6 +367,10 @@ class GatedLinearAttention(Mixer):
                 pre = _low_rank(x, self.a1, self.a2, None)
             proj = ops.linear_rows(x, self.proj_weight)
             join(main, side, pre)
+        elif x.dtype == torch.bfloat16 and n > ops.WIDE_MAX_ROWS and self.rank % 8 == 0:   # long steps: the pair's middle as further columns
+            joint = ops.linear(x, self.joint_weight)                                     # [T, q | k | v | g | middle]
+            proj, low = joint[:, :-self.rank], joint[:, -self.rank:]
+            pre = ops.linear_rows(low, self.a2, out_dtype=torch.float32)                 # float32 sums
         else:
             proj = ops.linear_rows(x, self.proj_weight)                                  # [T, q | k | v | g]
             pre = _low_rank(x, self.a1, self.a2, None)                                   # float32 sums

@@ -86,3 +86,21 @@ def test_queries_keys_and_values_of_pairs(m, heads, kv_heads, dim, k, rotated, b
     table[0, 0] = -1                                           # the third sequence's first page is not held
     ops.qkv_product(x, w, bias, inv, seq, pos, slots, heads, again, site, True, err)
     assert torch.equal(before, storage) and torch.equal(again, q) and int(err) == ops.ERR_NO_PAGE
+
+
+@pytest.mark.parametrize("m,n,extra,k", [(65, 2688, 14, 896), (257, 264, 1, 72), (300, 248, 32, 8), (2049, 2560, 2, 136), (700, 1536, 40, 640)])
+def test_columns_that_stay_float32(m, n, extra, k):
+    """The tail of a product's columns: inside the last tile, across its border, alone in a tile of its own."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(m)
+    x = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(n + extra, k, generator=g, device=DEV) * k ** -0.5).bfloat16()
+    out, tail = torch.full((m + 1, n + 8), 7.0, dtype=torch.bfloat16, device=DEV), torch.full((m + 1, extra), 7.0, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.tc_gemm_tail(x, w, out[:m, :n], tail[:m], err)
+    want, slack = x.double() @ w.double().T, (x.double().abs() @ w.double().abs().T) * k * 2.0 ** -24
+    got = torch.cat((out[:m, :n].double(), tail[:m].double()), dim=1)
+    round_off = torch.full((n + extra,), 2.0 ** -8, dtype=torch.float64, device=DEV)
+    round_off[n:] = 0
+    assert int(err) == 0 and bool(((got - want).abs() <= want.abs() * round_off + slack + 1e-30).all())
+    assert bool((out[m] == 7).all() and (out[:, n:] == 7).all() and (tail[m] == 7).all())
