@@ -49,11 +49,15 @@ struct MmaFirst {
 struct MmaNext {
     __device__ __forceinline__ void operator()(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) const { mma_bf16_16816(d, a, b0, b1); }
 };
+// Two additions an instruction, each rounded as one alone.
 template <int N> __device__ __forceinline__ void add_sums(float (*to)[4], const float (&sum)[N][4]) {
 #pragma unroll
     for (int i = 0; i < N; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) to[i][e] += sum[i][e];
+        for (int e = 0; e < 4; e += 2)
+            asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+                : "+f"(to[i][e]), "+f"(to[i][e + 1])
+                : "f"(sum[i][e]), "f"(sum[i][e + 1]));
 }
 
 // Byte offset of 16-byte piece `piece` of row `row` in a tile of WIDTH bfloat16 columns, pieces permuted so that eight
