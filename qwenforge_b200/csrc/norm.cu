@@ -30,12 +30,15 @@ __global__ void add_rms_norm_kernel(float* __restrict__ hidden, const T* __restr
 // width <= 4 * 4 * blockDim (4096 at 256 threads).
 template <typename T> struct Vec4;
 template <> struct Vec4<float> {
+    typedef float4 Raw;
+    static __device__ __forceinline__ float4 open(float4 r) { return r; }
     static __device__ __forceinline__ float4 load(const float* p) { return *reinterpret_cast<const float4*>(p); }
     static __device__ __forceinline__ void store(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 };
 template <> struct Vec4<bf16> {
-    static __device__ __forceinline__ float4 load(const bf16* p) {
-        const uint2 r = *reinterpret_cast<const uint2*>(p);
+    typedef uint2 Raw;
+    static __device__ __forceinline__ float4 load(const bf16* p) { return open(*reinterpret_cast<const uint2*>(p)); }
+    static __device__ __forceinline__ float4 open(uint2 r) {
         const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
         const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
         return make_float4(a.x, a.y, b.x, b.y);
@@ -52,7 +55,14 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 add_rms_norm_vec_kernel(float* __restrict__ hidden, const T* __restrict__ delta, const T* __restrict__ weight,
                         T* __restrict__ out, int width, float eps) {
-    grid_chain_entry();
+    // the norm's weights, which no kernel writes, are on their way while the kernel before ends: asked for behind the row's sum, from
+    // memory that the layer's other weights have pushed out of the L2, they were the last round trip of a decode step's norm
+    grid_launch_dependents();
+    typename Vec4<T>::Raw w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (threadIdx.x + u * 256 < width / 4) w[u] = reinterpret_cast<const typename Vec4<T>::Raw*>(weight)[threadIdx.x + u * 256];
+    grid_dependency_wait();
     __shared__ float scratch[33];
     float* h = hidden + (size_t)blockIdx.x * width;
     const T* d = delta ? delta + (size_t)blockIdx.x * width : nullptr;
@@ -82,8 +92,8 @@ add_rms_norm_vec_kernel(float* __restrict__ hidden, const T* __restrict__ delta,
     for (int u = 0; u < 4; ++u) {
         const int c = threadIdx.x + u * 256;
         if (c < n4) {
-            const float4 w = Vec4<T>::load(weight + 4 * c);
-            Vec4<T>::store(o + 4 * c, make_float4(v[u].x * inv * w.x, v[u].y * inv * w.y, v[u].z * inv * w.z, v[u].w * inv * w.w));
+            const float4 by = Vec4<T>::open(w[u]);
+            Vec4<T>::store(o + 4 * c, make_float4(v[u].x * inv * by.x, v[u].y * inv * by.y, v[u].z * inv * by.z, v[u].w * inv * by.w));
         }
     }
 }

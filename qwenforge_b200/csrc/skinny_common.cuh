@@ -66,14 +66,21 @@ template <int NT> struct EpiloguePre {
     float res[NT][4];
 };
 
+// The constants of it (bias, frequency), which no kernel writes: before the wait for the kernel ahead.
 template <int NT, int EPI>
-__device__ __forceinline__ void skinny_epilogue_prefetch(const SkinnyArgs& a, int tile, int g, int t, EpiloguePre<NT>& pre) {
+__device__ __forceinline__ void skinny_epilogue_constants(const SkinnyArgs& a, int tile, int g, EpiloguePre<NT>& pre) {
     int ra, rb;
     tile_rows<EPI>(a, tile, g, ra, rb);
     if (a.bias && ra >= 0) pre.bias_a = __bfloat162float(a.bias[ra]);
     if (a.bias && rb >= 0) pre.bias_b = __bfloat162float(a.bias[rb]);
     if (EPI == EPI_QKV && a.inv_freq && ra >= 0) pre.freq = a.inv_freq[ra % a.head_dim];
+}
+
+template <int NT, int EPI>
+__device__ __forceinline__ void skinny_epilogue_prefetch(const SkinnyArgs& a, int tile, int g, int t, EpiloguePre<NT>& pre) {
     if (EPI == EPI_RESIDUAL) {
+        int ra, rb;
+        tile_rows<EPI>(a, tile, g, ra, rb);
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll

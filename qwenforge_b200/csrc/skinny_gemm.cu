@@ -123,7 +123,22 @@ __global__ void __launch_bounds__(SK_THREADS, 3) skinny_gemm_kernel(const Skinny
         dst_s[m] = dst;
     }
     grid_launch_dependents();
+    // What the epilogue and the norm read of constants is asked for before the wait as well: it comes from memory that the layers'
+    // weights have pushed out of the L2, a round trip that the step would otherwise wait for (0.3 microseconds a kernel).
+    const int wpt = SK_WARPS / tpb, tile_local = warp / wpt, sub = warp % wpt;
+    const bool tile_leader = sub == 0;
+    EpiloguePre<NT> pre;
+    if (tile_leader && rank == 0) skinny_epilogue_constants<NT, EPI>(a, block0 * tpb + tile_local, g, pre);
+    uint2 norm_first[NORM ? 8 : 1];   // the norm weights of this lane's first columns
+    if (NORM && warp < a.m) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int c = (u * 32 + lane) * 4;
+            norm_first[u] = c < kslice && k_begin + c < a.k ? *reinterpret_cast<const uint2*>(a.norm_w + k_begin + c) : make_uint2(0u, 0u);
+        }
+    }
     grid_dependency_wait();  // weights are nobody's output; everything below reads what earlier kernels wrote
+    if (tile_leader && rank == 0) skinny_epilogue_prefetch<NT, EPI>(a, block0 * tpb + tile_local, g, t, pre);
 
     // ---- this block's slice of the token rows, normalised on the way if asked
     if (NORM) {
@@ -145,7 +160,7 @@ __global__ void __launch_bounds__(SK_THREADS, 3) skinny_gemm_kernel(const Skinny
                         const int c = base + (u * 32 + lane) * 4, kk = k_begin + c;
                         const bool in = c < kslice && kk < a.k;
                         x[u] = in ? *reinterpret_cast<const float4*>(h + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        wv[u] = in ? *reinterpret_cast<const uint2*>(a.norm_w + kk) : make_uint2(0u, 0u);
+                        wv[u] = base == 0 ? norm_first[u] : in ? *reinterpret_cast<const uint2*>(a.norm_w + kk) : make_uint2(0u, 0u);
                     }
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
@@ -176,13 +191,8 @@ __global__ void __launch_bounds__(SK_THREADS, 3) skinny_gemm_kernel(const Skinny
         }
     }
     __syncthreads();  // the token rows are staged
-    const int wpt = SK_WARPS / tpb, tile_local = warp / wpt, sub = warp % wpt;
-    const bool tile_leader = sub == 0;
     const unsigned char* w_s = w_base;
     const int block = block0;
-    // What the epilogue reads from global memory is asked for now, so that it ends in stores, not in round trips
-    EpiloguePre<NT> pre;
-    if (tile_leader && rank == 0) skinny_epilogue_prefetch<NT, EPI>(a, block * tpb + tile_local, g, t, pre);
     if (!mbar_wait(&w_bar[0], 0) && lane == 0) atomicOr(a.err, QF_ERR_COPY_TIMEOUT);
 
     // ---- products: the warps of a tile take its k-blocks in turn
@@ -330,6 +340,16 @@ __global__ void __launch_bounds__(SK_STREAM_THREADS, 1) skinny_stream_kernel(con
     }
 
     // ---- the eight product warps
+    EpiloguePre<NT> first_pre;        // of the first tile: its constants, and the norm weights, before the wait (see the kernel above)
+    if (warp < NT && (int)blockIdx.x < tiles) skinny_epilogue_constants<NT, EPI>(a, blockIdx.x, g, first_pre);
+    uint2 norm_first[NORM ? 8 : 1];
+    if (NORM && warp < a.m) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int c = (u * 32 + lane) * 4;
+            norm_first[u] = c < a.k ? *reinterpret_cast<const uint2*>(a.norm_w + c) : make_uint2(0u, 0u);
+        }
+    }
     grid_dependency_wait();
     if (!XS) {
         const int kpad = a.k;  // a multiple of 32: whole k-blocks, no padding needed
@@ -348,7 +368,7 @@ __global__ void __launch_bounds__(SK_STREAM_THREADS, 1) skinny_stream_kernel(con
                             const int c = base + (u * 32 + lane) * 4;
                             const bool in = c < a.k;
                             x[u] = in ? *reinterpret_cast<const float4*>(h + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-                            wv[u] = in ? *reinterpret_cast<const uint2*>(a.norm_w + c) : make_uint2(0u, 0u);
+                            wv[u] = base == 0 ? norm_first[u] : in ? *reinterpret_cast<const uint2*>(a.norm_w + c) : make_uint2(0u, 0u);
                         }
 #pragma unroll
                         for (int u = 0; u < 8; ++u) {
@@ -383,8 +403,11 @@ __global__ void __launch_bounds__(SK_STREAM_THREADS, 1) skinny_stream_kernel(con
     int idx = 0;
     bool dead = false;  // a wait ran out: reported; the warp goes on without waiting, so that every barrier is still met
     for (int tile = blockIdx.x; tile < tiles; tile += plan.nblk) {
-        EpiloguePre<NT> pre;
-        if (warp < NT) skinny_epilogue_prefetch<NT, EPI>(a, tile, g, t, pre);
+        EpiloguePre<NT> pre = first_pre;
+        if (warp < NT) {
+            if (tile != (int)blockIdx.x) skinny_epilogue_constants<NT, EPI>(a, tile, g, pre);
+            skinny_epilogue_prefetch<NT, EPI>(a, tile, g, t, pre);
+        }
         float acc[NT][4];
 #pragma unroll
         for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
