@@ -24,13 +24,12 @@
 // logarithms: a chunk is cut into eighths of 16 tokens, and W_ij is (decays from the start of i's eighth to i) x (decays of the
 // whole eighths between) x (decays behind j to the end of j's eighth), each factor at most as large as the decays make it, so
 // nothing overflows or cancels.
-#include <type_traits>
-
 #include "chunks.cuh"
 
 #define SC_CHUNK 128
 #define SC_SUB 16
 #define SC_VT 64              // columns of v of a block, both kernels
+#define SC_OUT_THREADS 256    // of a block of outputs: a warp per eighth
 
 struct ChunkArgs {
     const bf16 *q, *k, *v;
@@ -244,13 +243,14 @@ chunk_chain_kernel(const ChunkArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// (3) Outputs of one chunk, one head, 64 columns of v. Four warps; a warp takes the chunk's eighths w and 7 - w (16 tokens each),
-// so that all have the same part of the triangle, and one load of a key's, value's or state's fragment serves both. First
-// S0^T q on the record's three parts, scaled by the decays up to the row; then, 16 earlier tokens at a time, scores, weights,
+// (3) Outputs of one chunk, one head, 64 columns of v. Eight warps, one for each of the chunk's eighths (16 tokens each), dealt so that
+// the two that share a scheduler have the same part of the triangle between them. (Four warps of two eighths each load every
+// fragment of a key, a value or the state once for both, and leave an SM eight warps, which waited for their own instructions: 34
+// chunks of 32 heads of 128 x 128 in 132 microseconds, 124 so.) First S0^T q on the record's three parts, scaled by the decays up to the row; then, 16 earlier tokens at a time, scores, weights,
 // and the products with v added on top. Queries move to registers before the keys arrive in the same place, so that two
 // blocks fit an SM.
 template <int D>
-__global__ void __launch_bounds__(128, 2)
+__global__ void __launch_bounds__(SC_OUT_THREADS, 2)
 chunk_outputs_kernel(const ChunkArgs a) {
     grid_chain_entry();
     extern __shared__ __align__(128) unsigned char sc_smem[];
@@ -268,24 +268,24 @@ chunk_outputs_kernel(const ChunkArgs a) {
     const bool with_n = a.n_offset >= 0 && v0 == 0;
     const long long record = record_of<SC_CHUNK>(a.portion, a.cu_q, seq, chunk) * a.n_heads + head;
 
-    fetch_tile<SC_CHUNK, D>(qk_s, a.q + (size_t)t0 * a.q_stride + group * D, a.q_stride, n_here, threadIdx.x, 128);
+    fetch_tile<SC_CHUNK, D>(qk_s, a.q + (size_t)t0 * a.q_stride + group * D, a.q_stride, n_here, threadIdx.x, SC_OUT_THREADS);
     cp_async_commit();
-    fetch_tile<SC_CHUNK, SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, 128);
+    fetch_tile<SC_CHUNK, SC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, SC_OUT_THREADS);
     cp_async_commit();
     const float2 gate = threadIdx.x < n_here ? gates_of(a, t0 + threadIdx.x, head) : make_float2(1.f, 0.f);   // this thread's token
     const float my_take = gate.y;
-    decay_s[threadIdx.x] = gate.x;
+    if (threadIdx.x < SC_CHUNK) decay_s[threadIdx.x] = gate.x;
     if (with_n && threadIdx.x < D) n_s[threadIdx.x] = a.n_records[record * D + threadIdx.x];
     const float* rec = a.records + record * D * a.vdim + (size_t)v0 * D;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        constexpr int EACH = SC_VT * D / 4 / 128 / 2;
+        constexpr int EACH = SC_VT * D / 4 / SC_OUT_THREADS / 2;
         float4 held[EACH];
 #pragma unroll
-        for (int u = 0; u < EACH; ++u) held[u] = *reinterpret_cast<const float4*>(rec + 4 * (threadIdx.x + 128 * (half * EACH + u)));
+        for (int u = 0; u < EACH; ++u) held[u] = *reinterpret_cast<const float4*>(rec + 4 * (threadIdx.x + SC_OUT_THREADS * (half * EACH + u)));
 #pragma unroll
         for (int u = 0; u < EACH; ++u) {
-            const int i = 4 * (threadIdx.x + 128 * (half * EACH + u)), row = i / D, col = i % D;
+            const int i = 4 * (threadIdx.x + SC_OUT_THREADS * (half * EACH + u)), row = i / D, col = i % D;
             const Thirds x = thirds(held[u].x, held[u].y), z = thirds(held[u].z, held[u].w);
             unsigned char* at = s_s + tile_at<D>(row, col >> 3) + (col & 7) * 2;
             *reinterpret_cast<uint2*>(at) = make_uint2(x.hi, z.hi);
@@ -296,15 +296,12 @@ chunk_outputs_kernel(const ChunkArgs a) {
     cp_async_wait<1>();
     __syncthreads();
 
-    const int tile[2] = {7 - warp, warp};             // this warp's eighths, the later one first
+    const int tile = warp < 4 ? warp : 11 - warp;     // this warp's eighth
     const int g = lane >> 2, t2 = (lane & 3) * 2;
-    uint32_t q_frag[2][D / 16][4];
+    uint32_t q_frag[D / 16][4];
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int kd = 0; kd < D / 16; ++kd)
-            ldmatrix_x4(q_frag[m][kd], qk_s + tile_at<D>(tile[m] * 16 + (lane & 15), kd * 2 + (lane >> 4)));
-    {   // the weights' factors: a thread takes a token
+    for (int kd = 0; kd < D / 16; ++kd) ldmatrix_x4(q_frag[kd], qk_s + tile_at<D>(tile * 16 + (lane & 15), kd * 2 + (lane >> 4)));
+    if (threadIdx.x < SC_CHUNK) {   // the weights' factors: a thread takes a token
         const int sub = threadIdx.x / SC_SUB, p = threadIdx.x % SC_SUB;
         float dec[SC_SUB], upto = 1.f, w = my_take;
 #pragma unroll
@@ -320,184 +317,160 @@ chunk_outputs_kernel(const ChunkArgs a) {
     }
     cp_async_wait<0>();
     __syncthreads();                   // the queries are in registers, v has arrived
-    fetch_tile<SC_CHUNK, D>(qk_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, 128);
+    fetch_tile<SC_CHUNK, D>(qk_s, a.k + (size_t)t0 * a.k_stride + group * D, a.k_stride, n_here, threadIdx.x, SC_OUT_THREADS);
     cp_async_commit();
     // A row of v that is not finite must not reach the tokens before it through a weight of zero: looked for here, kept apart below.
     int odd = 0;
 #pragma unroll
-    for (int i = 0; i < V_BYTES / 16 / 128; ++i) {
-        const uint4 x = *reinterpret_cast<const uint4*>(v_s + 16 * (threadIdx.x + 128 * i));
+    for (int i = 0; i < V_BYTES / 16 / SC_OUT_THREADS; ++i) {
+        const uint4 x = *reinterpret_cast<const uint4*>(v_s + 16 * (threadIdx.x + SC_OUT_THREADS * i));
         const uint32_t parts[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) odd |= (parts[e] & 0x7f80u) == 0x7f80u || (parts[e] & 0x7f800000u) == 0x7f800000u;
     }
 
     // ---- what the state before the chunk says
-    float acc[2][SC_VT / 8][4];
+    float acc[SC_VT / 8][4];
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int nt = 0; nt < SC_VT / 8; ++nt)
 #pragma unroll
-        for (int nt = 0; nt < SC_VT / 8; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[m][nt][e] = 0.f;
-    float n_sum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};   // n . q of rows g and g + 8 (this thread's part), then the scores' sums as well
+        for (int e = 0; e < 4; ++e) acc[nt][e] = 0.f;
+    float n_sum[2] = {0.f, 0.f};   // n . q of rows g and g + 8 (this thread's part), then the scores' sums as well
 #pragma unroll
     for (int kd = 0; kd < D / 16; ++kd) {
 #pragma unroll
-        for (int vp = 0; vp < SC_VT / 16; ++vp) {
-            uint32_t b[4];
-            auto fragment = [&](int part) {
-                ldmatrix_x4(b, s_s + part * S_PART + tile_at<D>(vp * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)));
-            };
-            float sum[2][2][4];
+        for (int vp = 0; vp < SC_VT / 16; vp += 2) {   // four sums in turn
+            float sum[4][4];
 #pragma unroll
-            for (int part = 2; part >= 0; --part) {
-                fragment(part);
+            for (int part = 2; part >= 0; --part)
 #pragma unroll
-                for (int m = 0; m < 2; ++m)
+                for (int p = 0; p < 2; ++p) {
+                    uint32_t b[4];
+                    ldmatrix_x4(b, s_s + part * S_PART + tile_at<D>((vp + p) * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)));
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        if (part == 2) MmaFirst{}(sum[m][h], q_frag[m][kd], b[2 * h], b[2 * h + 1]);
-                        else MmaNext{}(sum[m][h], q_frag[m][kd], b[2 * h], b[2 * h + 1]);
+                        if (part == 2) MmaFirst{}(sum[2 * p + h], q_frag[kd], b[2 * h], b[2 * h + 1]);
+                        else MmaNext{}(sum[2 * p + h], q_frag[kd], b[2 * h], b[2 * h + 1]);
                     }
-            }
-#pragma unroll
-            for (int m = 0; m < 2; ++m) add_sums(acc[m] + 2 * vp, sum[m]);
+                }
+            add_sums(acc + 2 * vp, sum);
         }
         if (with_n) {
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float* n_at = n_s + kd * 16 + (r >> 1) * 8 + t2;
-                    n_sum[m][r & 1] = fmaf(lower_bf16(q_frag[m][kd][r]), n_at[0], n_sum[m][r & 1]);
-                    n_sum[m][r & 1] = fmaf(upper_bf16(q_frag[m][kd][r]), n_at[1], n_sum[m][r & 1]);
-                }
+            for (int r = 0; r < 4; ++r) {
+                const float* n_at = n_s + kd * 16 + (r >> 1) * 8 + t2;
+                n_sum[r & 1] = fmaf(lower_bf16(q_frag[kd][r]), n_at[0], n_sum[r & 1]);
+                n_sum[r & 1] = fmaf(upper_bf16(q_frag[kd][r]), n_at[1], n_sum[r & 1]);
+            }
         }
     }
     cp_async_wait<0>();
     const bool not_finite = __syncthreads_or(odd) != 0;   // (and the keys have arrived)
-    float f[2][2];                     // the decays from the eighth in hand up to rows g and g + 8, and the scale of q
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        f[m][0] = upto_s[tile[m] * 16 + g] * a.q_scale, f[m][1] = upto_s[tile[m] * 16 + g + 8] * a.q_scale;
+    float f[2];                        // the decays from the eighth in hand up to rows g and g + 8, and the scale of q
+    {
+        f[0] = upto_s[tile * 16 + g] * a.q_scale, f[1] = upto_s[tile * 16 + g + 8] * a.q_scale;
         float before = 1.f;            // the decays of the whole eighths before this one
-        for (int c = 0; c < tile[m]; ++c) before *= upto_s[c * 16 + 15];
+        for (int c = 0; c < tile; ++c) before *= upto_s[c * 16 + 15];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const float all = f[m][r] * before;
+            const float all = f[r] * before;
 #pragma unroll
-            for (int nt = 0; nt < SC_VT / 8; ++nt) acc[m][nt][2 * r] *= all, acc[m][nt][2 * r + 1] *= all;
-            n_sum[m][r] *= all;
+            for (int nt = 0; nt < SC_VT / 8; ++nt) acc[nt][2 * r] *= all, acc[nt][2 * r + 1] *= all;
+            n_sum[r] *= all;
         }
     }
 
-    // ---- what the chunk's own tokens say, from each eighth's own tokens back to the chunk's first
-    auto eighth = [&](int c, auto both) {   // eighth c, seen by the warp's later eighth, or by both
-        constexpr int M = decltype(both)::value ? 2 : 1;
-        float s[M][2][4];
+    // ---- what the chunk's own tokens say, from the eighth's own tokens back to the chunk's first
+#pragma unroll 1
+    for (int c = tile; c >= 0; --c) {
+        float s[2][4];
 #pragma unroll
         for (int kd = 0; kd < D / 16; ++kd) {
             uint32_t b[4];
             ldmatrix_x4(b, qk_s + tile_at<D>(c * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)));
+            float sum[2][4];
+            MmaFirst{}(sum[0], q_frag[kd], b[0], b[1]);
+            MmaFirst{}(sum[1], q_frag[kd], b[2], b[3]);
+            if (kd > 0) add_sums(s, sum);
+            else
 #pragma unroll
-            for (int m = 0; m < M; ++m) {
-                float sum[2][4];
-                MmaFirst{}(sum[0], q_frag[m][kd], b[0], b[1]);
-                MmaFirst{}(sum[1], q_frag[m][kd], b[2], b[3]);
-                if (kd > 0) add_sums(s[m], sum);
-                else
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) s[m][0][e] = sum[0][e], s[m][1][e] = sum[1][e];
-            }
+                for (int e = 0; e < 4; ++e) s[0][e] = sum[0][e], s[1][e] = sum[1][e];
         }
-        uint32_t hi[M][4], mid[M][4], lo[M][4];
+        if (c == tile) {
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-            if (c == tile[m]) {
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int row = g + (e >> 1) * 8, col = h * 8 + t2 + (e & 1);
-                        s[m][h][e] = col <= row ? s[m][h][e] * a.q_scale * inner_s[c][row][col] : 0.f;
-                    }
-            } else {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float2 w = *reinterpret_cast<const float2*>(behind_s + c * 16 + h * 8 + t2);
-                    s[m][h][0] *= f[m][0] * w.x, s[m][h][1] *= f[m][0] * w.y;
-                    s[m][h][2] *= f[m][1] * w.x, s[m][h][3] *= f[m][1] * w.y;
+                for (int e = 0; e < 4; ++e) {
+                    const int row = g + (e >> 1) * 8, col = h * 8 + t2 + (e & 1);
+                    s[h][e] = col <= row ? s[h][e] * a.q_scale * inner_s[c][row][col] : 0.f;
                 }
-                const float all = upto_s[c * 16 + 15];
-                f[m][0] *= all, f[m][1] *= all;
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 w = *reinterpret_cast<const float2*>(behind_s + c * 16 + h * 8 + t2);
+                s[h][0] *= f[0] * w.x, s[h][1] *= f[0] * w.y;
+                s[h][2] *= f[1] * w.x, s[h][3] *= f[1] * w.y;
             }
-            n_sum[m][0] += (s[m][0][0] + s[m][0][1]) + (s[m][1][0] + s[m][1][1]);
-            n_sum[m][1] += (s[m][0][2] + s[m][0][3]) + (s[m][1][2] + s[m][1][3]);
-            if (c == tile[m] && not_finite) {   // token by token, so that what lies behind a row is left out and not multiplied by zero
+            const float all = upto_s[c * 16 + 15];
+            f[0] *= all, f[1] *= all;
+        }
+        n_sum[0] += (s[0][0] + s[0][1]) + (s[1][0] + s[1][1]);
+        n_sum[1] += (s[0][2] + s[0][3]) + (s[1][2] + s[1][3]);
+        if (c == tile && not_finite) {   // token by token, so that what lies behind a row is left out and not multiplied by zero
 #pragma unroll 1
-                for (int j = 0; j < SC_SUB; ++j) {
-                    const int from = (lane & ~3) | ((j & 7) >> 1);
-                    const float w0 = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? s[m][0][1] : s[m][0][0]) : (j & 1 ? s[m][1][1] : s[m][1][0]), from);
-                    const float w1 = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? s[m][0][3] : s[m][0][2]) : (j & 1 ? s[m][1][3] : s[m][1][2]), from);
+            for (int j = 0; j < SC_SUB; ++j) {
+                const int from = (lane & ~3) | ((j & 7) >> 1);
+                const float w0 = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? s[0][1] : s[0][0]) : (j & 1 ? s[1][1] : s[1][0]), from);
+                const float w1 = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? s[0][3] : s[0][2]) : (j & 1 ? s[1][3] : s[1][2]), from);
 #pragma unroll
-                    for (int nt = 0; nt < SC_VT / 8; ++nt) {
-                        const uint32_t x = *reinterpret_cast<const uint32_t*>(v_s + tile_at<SC_VT>(c * 16 + j, nt) + t2 * 2);
-                        if (j <= g) acc[m][nt][0] = fmaf(w0, lower_bf16(x), acc[m][nt][0]), acc[m][nt][1] = fmaf(w0, upper_bf16(x), acc[m][nt][1]);
-                        if (j <= g + 8) acc[m][nt][2] = fmaf(w1, lower_bf16(x), acc[m][nt][2]), acc[m][nt][3] = fmaf(w1, upper_bf16(x), acc[m][nt][3]);
-                    }
+                for (int nt = 0; nt < SC_VT / 8; ++nt) {
+                    const uint32_t x = *reinterpret_cast<const uint32_t*>(v_s + tile_at<SC_VT>(c * 16 + j, nt) + t2 * 2);
+                    if (j <= g) acc[nt][0] = fmaf(w0, lower_bf16(x), acc[nt][0]), acc[nt][1] = fmaf(w0, upper_bf16(x), acc[nt][1]);
+                    if (j <= g + 8) acc[nt][2] = fmaf(w1, lower_bf16(x), acc[nt][2]), acc[nt][3] = fmaf(w1, upper_bf16(x), acc[nt][3]);
                 }
             }
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const Thirds x = thirds(s[m][r >> 1][(r & 1) * 2], s[m][r >> 1][(r & 1) * 2 + 1]);
-                hi[m][r] = x.hi, mid[m][r] = x.mid, lo[m][r] = x.lo;
-            }
+            continue;
         }
-        uint32_t b[SC_VT / 16][4];
+        uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
-        for (int vp = 0; vp < SC_VT / 16; ++vp) ldmatrix_x4_trans(b[vp], v_s + tile_at<SC_VT>(c * 16 + (lane & 15), vp * 2 + (lane >> 4)));
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-            if (c == tile[m] && not_finite) continue;
-#pragma unroll
-            for (int v2 = 0; v2 < SC_VT / 16; v2 += 2) {
-                float sum[4][4];
-                auto part = [&](auto mma, const uint32_t (&x)[4]) {
-#pragma unroll
-                    for (int vp = 0; vp < 2; ++vp) {
-                        mma(sum[2 * vp], x, b[v2 + vp][0], b[v2 + vp][1]);
-                        mma(sum[2 * vp + 1], x, b[v2 + vp][2], b[v2 + vp][3]);
-                    }
-                };
-                part(MmaFirst{}, lo[m]);
-                part(MmaNext{}, mid[m]);
-                part(MmaNext{}, hi[m]);
-                add_sums(acc[m] + 2 * v2, sum);
-            }
+        for (int r = 0; r < 4; ++r) {
+            const Thirds x = thirds(s[r >> 1][(r & 1) * 2], s[r >> 1][(r & 1) * 2 + 1]);
+            hi[r] = x.hi, mid[r] = x.mid, lo[r] = x.lo;
         }
-    };
-    for (int c = tile[0]; c > tile[1]; --c) eighth(c, std::false_type{});
-    for (int c = tile[1]; c >= 0; --c) eighth(c, std::true_type{});
+#pragma unroll
+        for (int v2 = 0; v2 < SC_VT / 16; v2 += 2) {
+            uint32_t b[2][4];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) ldmatrix_x4_trans(b[p], v_s + tile_at<SC_VT>(c * 16 + (lane & 15), (v2 + p) * 2 + (lane >> 4)));
+            float sum[4][4];
+            auto part = [&](auto mma, const uint32_t (&x)[4]) {
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    mma(sum[2 * p], x, b[p][0], b[p][1]);
+                    mma(sum[2 * p + 1], x, b[p][2], b[p][3]);
+                }
+            };
+            part(MmaFirst{}, lo);
+            part(MmaNext{}, mid);
+            part(MmaNext{}, hi);
+            add_sums(acc + 2 * v2, sum);
+        }
+    }
 
-    const int width = a.n_heads * a.vdim;
+    const int width = a.n_heads * a.vdim, row = tile * 16 + g;
+    float* y0 = a.y + (size_t)(t0 + row) * width + head * a.vdim + v0 + t2;
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        const int row = tile[m] * 16 + g;
-        float* y0 = a.y + (size_t)(t0 + row) * width + head * a.vdim + v0 + t2;
+    for (int nt = 0; nt < SC_VT / 8; ++nt) {
+        if (row < n_here) *reinterpret_cast<float2*>(y0 + nt * 8) = make_float2(acc[nt][0], acc[nt][1]);
+        if (row + 8 < n_here) *reinterpret_cast<float2*>(y0 + 8 * (size_t)width + nt * 8) = make_float2(acc[nt][2], acc[nt][3]);
+    }
+    if (with_n) {
 #pragma unroll
-        for (int nt = 0; nt < SC_VT / 8; ++nt) {
-            if (row < n_here) *reinterpret_cast<float2*>(y0 + nt * 8) = make_float2(acc[m][nt][0], acc[m][nt][1]);
-            if (row + 8 < n_here) *reinterpret_cast<float2*>(y0 + 8 * (size_t)width + nt * 8) = make_float2(acc[m][nt][2], acc[m][nt][3]);
-        }
-        if (with_n) {
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                float sum = n_sum[m][r];
-                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                if ((lane & 3) == 0 && row + 8 * r < n_here) a.nq[(size_t)(t0 + row + 8 * r) * a.n_heads + head] = sum;
-            }
+        for (int r = 0; r < 2; ++r) {
+            float sum = n_sum[r];
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            if ((lane & 3) == 0 && row + 8 * r < n_here) a.nq[(size_t)(t0 + row + 8 * r) * a.n_heads + head] = sum;
         }
     }
 }
@@ -514,7 +487,7 @@ static int launch_chunks(ChunkArgs a, int n_seqs, int max_q_len, cudaStream_t st
         const dim3 grid(min(each, chunks - chunk0), a.vdim / SC_VT * a.n_heads, n_seqs);
         e = launch_pdl(chunk_parts_kernel<D>, grid, dim3(a.n_offset >= 0 ? 160 : 128), parts_smem, stream, a);
         if (e == cudaSuccess) e = launch_pdl(chunk_chain_kernel<D>, dim3((items + 7) / 8, a.n_heads, n_seqs), dim3(256), 0, stream, a);
-        if (e == cudaSuccess) e = launch_pdl(chunk_outputs_kernel<D>, grid, dim3(128), outputs_smem, stream, a);
+        if (e == cudaSuccess) e = launch_pdl(chunk_outputs_kernel<D>, grid, dim3(SC_OUT_THREADS), outputs_smem, stream, a);
     }
     return (int)e;
 }
