@@ -41,6 +41,7 @@ struct RowChunkArgs {
     float *records, *whole, *made;   // [record][heads][vdim][64], [record][heads][64], [T][heads * 64] (kind 0: not written)
     float* y;
     Portion portion;
+    int v_each;      // tiles of 64 columns of v that a block of outputs takes, one after the other
 };
 
 __device__ __forceinline__ float row_log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
@@ -214,14 +215,14 @@ row_outputs_kernel(const RowChunkArgs a) {
     unsigned char* kh_s = rc_smem;                                              // [3][64][64] keys times the decays behind them in their quarter
     float* qh_s = reinterpret_cast<float*>(kh_s + 3 * RC_PLANE);                // [64][RC_LD] queries times the decays of their quarter up to them
     bf16* k_s = reinterpret_cast<bf16*>(qh_s + RC_CHUNK * RC_LD);               // [64][RC_LH]
-    unsigned char* v_s = reinterpret_cast<unsigned char*>(k_s + RC_CHUNK * RC_LH);   // [64][64]
-    float* w_s = reinterpret_cast<float*>(v_s + RC_CHUNK * RC_VT * 2);          // [64][RC_LD]
+    unsigned char* v_all = reinterpret_cast<unsigned char*>(k_s + RC_CHUNK * RC_LH);   // [v_each][64][64]
+    float* w_s = reinterpret_cast<float*>(v_all + a.v_each * (RC_CHUNK * RC_VT * 2));   // [64][RC_LD]
     bf16* q_s = reinterpret_cast<bf16*>(w_s + RC_CHUNK * RC_LD);                // [64][RC_LH]
     unsigned char* s_s = reinterpret_cast<unsigned char*>(w_s);                 // [3][64 v][64] the state's parts, over w_s and q_s
     static_assert(3 * RC_VT * RC_D * 2 <= RC_CHUNK * RC_LD * 4 + RC_CHUNK * RC_LH * 2, "the state's parts find room there");
     __shared__ float pair_s[4][RC_SUB][RC_SUB + 1], all_s[4][RC_D];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seq = blockIdx.z;
-    const int v_tiles = a.vdim / RC_VT, head = blockIdx.y / v_tiles, v0 = (blockIdx.y % v_tiles) * RC_VT;
+    const int v_groups = a.vdim / RC_VT / a.v_each, head = blockIdx.y / v_groups, v_first = (blockIdx.y % v_groups) * a.v_each * RC_VT;
     const int chunk = a.portion.chunk0 + (int)blockIdx.x, t0 = a.cu_q[seq] + chunk * RC_CHUNK, n_here = min(RC_CHUNK, a.cu_q[seq + 1] - t0);
     if (n_here <= 0) return;
     const long long record = record_of<RC_CHUNK>(a.portion, a.cu_q, seq, chunk) * a.n_heads + head;
@@ -233,7 +234,9 @@ row_outputs_kernel(const RowChunkArgs a) {
         cp_async_16(k_s + row * RC_LH + c, there ? ks + (size_t)row * a.k_stride : ks, there);
         cp_async_16(q_s + row * RC_LH + c, there ? qs + (size_t)row * a.q_stride : qs, there);
     }
-    fetch_tile<RC_CHUNK, RC_VT>(v_s, a.v + (size_t)t0 * a.v_stride + head * a.vdim + v0, a.v_stride, n_here, threadIdx.x, 128);
+    for (int vt = 0; vt < a.v_each; ++vt)
+        fetch_tile<RC_CHUNK, RC_VT>(v_all + vt * (RC_CHUNK * RC_VT * 2), a.v + (size_t)t0 * a.v_stride + head * a.vdim + v_first + vt * RC_VT, a.v_stride,
+                                    n_here, threadIdx.x, 128);
     cp_async_commit();
     const float* w_src = (a.kind != 0 ? a.made : a.decay) + (size_t)t0 * width + head * RC_D;
 #pragma unroll
@@ -244,7 +247,7 @@ row_outputs_kernel(const RowChunkArgs a) {
     }
     constexpr int EACH = RC_VT * RC_D / 4 / 128;
     float4 held[EACH];
-    const float* rec = a.records + record * RC_D * a.vdim + (size_t)v0 * RC_D;
+    const float* rec = a.records + record * RC_D * a.vdim + (size_t)v_first * RC_D;
 #pragma unroll
     for (int u = 0; u < EACH; ++u) held[u] = *reinterpret_cast<const float4*>(rec + 4 * (threadIdx.x + 128 * u));
     cp_async_wait<0>();
@@ -280,200 +283,209 @@ row_outputs_kernel(const RowChunkArgs a) {
     // between gathering on it
     {
         const int i = lane & 15, half = lane >> 4, r0 = warp * RC_SUB;
-        float qp[32];
+        float2 qp[16];
 #pragma unroll
         for (int c = 0; c < 32; c += 8) {
             const uint4 x = *reinterpret_cast<const uint4*>(q_s + (r0 + i) * RC_LH + half * 32 + c);
             const uint32_t p[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) qp[c + 2 * e] = lower_bf16(p[e]) * a.q_scale, qp[c + 2 * e + 1] = upper_bf16(p[e]) * a.q_scale;
+            for (int e = 0; e < 4; ++e) qp[c / 2 + e] = make_float2(lower_bf16(p[e]) * a.q_scale, upper_bf16(p[e]) * a.q_scale);
         }
 #pragma unroll 1
         for (int s = 0; s < RC_SUB; ++s) {
             const int j = max(i - s, 0);
             const bf16* kj = k_s + (r0 + j) * RC_LH + half * 32;
             const float* wj = w_s + (r0 + j) * RC_LD + half * 32;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};   // two multiply-adds an instruction
 #pragma unroll
             for (int c = 0; c < 32; c += 8) {
                 const uint4 x = *reinterpret_cast<const uint4*>(kj + c);
                 const float4 wa = *reinterpret_cast<const float4*>(wj + c), wb = *reinterpret_cast<const float4*>(wj + c + 4);
-                float k[8] = {lower_bf16(x.x), upper_bf16(x.x), lower_bf16(x.y), upper_bf16(x.y),
-                              lower_bf16(x.z), upper_bf16(x.z), lower_bf16(x.w), upper_bf16(x.w)};
-                const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-                if (BONUS && s == 0) {
-                    const float* u = a.bonus + head * RC_D + half * 32 + c;
+                const uint32_t p[4] = {x.x, x.y, x.z, x.w};
+                const float2 w[4] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w), make_float2(wb.x, wb.y), make_float2(wb.z, wb.w)};
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) k[e] *= u[e];
-                }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    sum[e & 3] = fmaf(qp[c + e], k[e], sum[e & 3]);
-                    if (!BONUS || s > 0) qp[c + e] *= w[e];
+                for (int e = 0; e < 4; ++e) {
+                    float2 k = make_float2(lower_bf16(p[e]), upper_bf16(p[e]));
+                    if (BONUS && s == 0) {
+                        const float* u = a.bonus + head * RC_D + half * 32 + c + 2 * e;
+                        k.x *= u[0], k.y *= u[1];
+                    }
+                    sum[e & 1] = __ffma2_rn(qp[c / 2 + e], k, sum[e & 1]);
+                    if (!BONUS || s > 0) qp[c / 2 + e] = __fmul2_rn(qp[c / 2 + e], w[e]);
                 }
             }
-            float total = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            float total = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             total += __shfl_xor_sync(0xffffffffu, total, 16);
             if (half == 0 && i >= s) pair_s[warp][i][i - s] = total;
         }
     }
-    // A row of v that is not finite must not reach the tokens before it through a weight of zero: looked for here, kept apart below.
-    int odd = 0;
+#pragma unroll 1
+    for (int vt = 0; vt < a.v_each; ++vt) {
+        const unsigned char* v_s = v_all + vt * (RC_CHUNK * RC_VT * 2);
+        const int v0 = v_first + vt * RC_VT;
+        if (vt > 0) {
 #pragma unroll
-    for (int i = 0; i < RC_CHUNK * RC_VT * 2 / 16 / 128; ++i) {
-        const uint4 x = *reinterpret_cast<const uint4*>(v_s + 16 * (threadIdx.x + 128 * i));
-        const uint32_t p[4] = {x.x, x.y, x.z, x.w};
+            for (int u = 0; u < EACH; ++u) held[u] = *reinterpret_cast<const float4*>(rec + (size_t)vt * RC_VT * RC_D + 4 * (threadIdx.x + 128 * u));
+        }
+        // A row of v that is not finite must not reach the tokens before it through a weight of zero: looked for here, kept apart below.
+        int odd = 0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) odd |= (p[e] & 0x7f80u) == 0x7f80u || (p[e] & 0x7f800000u) == 0x7f800000u;
-    }
-    const bool not_finite = __syncthreads_or(odd) != 0;   // (and nobody reads the decays and the plain queries any more)
+        for (int i = 0; i < RC_CHUNK * RC_VT * 2 / 16 / 128; ++i) {
+            const uint4 x = *reinterpret_cast<const uint4*>(v_s + 16 * (threadIdx.x + 128 * i));
+            const uint32_t p[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-    for (int u = 0; u < EACH; ++u) {
-        const int i = 4 * (threadIdx.x + 128 * u), row = i / RC_D, col = i % RC_D;
-        const Thirds x = thirds(held[u].x, held[u].y), z = thirds(held[u].z, held[u].w);
-        unsigned char* at = s_s + tile_at<RC_D>(row, col >> 3) + (col & 7) * 2;
-        *reinterpret_cast<uint2*>(at) = make_uint2(x.hi, z.hi);
-        *reinterpret_cast<uint2*>(at + RC_VT * RC_D * 2) = make_uint2(x.mid, z.mid);
-        *reinterpret_cast<uint2*>(at + 2 * RC_VT * RC_D * 2) = make_uint2(x.lo, z.lo);
-    }
-    __syncthreads();
+            for (int e = 0; e < 4; ++e) odd |= (p[e] & 0x7f80u) == 0x7f80u || (p[e] & 0x7f800000u) == 0x7f800000u;
+        }
+        // (and nobody reads the decays and the plain queries, or the state of the tile before, any more)
+        const bool not_finite = __syncthreads_or(odd) != 0;
+#pragma unroll
+        for (int u = 0; u < EACH; ++u) {
+            const int i = 4 * (threadIdx.x + 128 * u), row = i / RC_D, col = i % RC_D;
+            const Thirds x = thirds(held[u].x, held[u].y), z = thirds(held[u].z, held[u].w);
+            unsigned char* at = s_s + tile_at<RC_D>(row, col >> 3) + (col & 7) * 2;
+            *reinterpret_cast<uint2*>(at) = make_uint2(x.hi, z.hi);
+            *reinterpret_cast<uint2*>(at + RC_VT * RC_D * 2) = make_uint2(x.mid, z.mid);
+            *reinterpret_cast<uint2*>(at + 2 * RC_VT * RC_D * 2) = make_uint2(x.lo, z.lo);
+        }
+        __syncthreads();
 
-    const int g = lane >> 2, t2 = (lane & 3) * 2;
-    // The products of the lesser parts, 2^8 times smaller, are summed apart; those of the leading parts 16 rows or tokens at a time
-    // (MmaFirst). Errors against 64 bits, outputs / states, 2,048 tokens of 7 heads of 64 x 128, decays sigmoid(z)^(1/16): 1.20e-7 /
-    // 6.0e-8, token by token 1.45e-7 / 1.14e-7 (the leading parts' sums left to the tensor cores: 2.5e-7 / 1.8e-7).
-    float acc[RC_VT / 8][4], low[RC_VT / 8][4];
+        const int g = lane >> 2, t2 = (lane & 3) * 2;
+        // The products of the lesser parts, 2^8 times smaller, are summed apart; those of the leading parts 16 rows or tokens at a time
+        // (MmaFirst). Errors against 64 bits, outputs / states, 2,048 tokens of 7 heads of 64 x 128, decays sigmoid(z)^(1/16): 1.20e-7 /
+        // 6.0e-8, token by token 1.45e-7 / 1.14e-7 (the leading parts' sums left to the tensor cores: 2.5e-7 / 1.8e-7).
+        float acc[RC_VT / 8][4], low[RC_VT / 8][4];
 #pragma unroll
-    for (int nt = 0; nt < RC_VT / 8; ++nt)
+        for (int nt = 0; nt < RC_VT / 8; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[nt][e] = low[nt][e] = 0.f;
-    // rows g and g + 8 of this warp's queries: two neighbouring columns at 2 t and at 2 t + 8 of every 16
-    float2 qf[RC_D / 16][4];
+            for (int e = 0; e < 4; ++e) acc[nt][e] = low[nt][e] = 0.f;
+        // rows g and g + 8 of this warp's queries: two neighbouring columns at 2 t and at 2 t + 8 of every 16
+        float2 qf[RC_D / 16][4];
 #pragma unroll
-    for (int kd = 0; kd < RC_D / 16; ++kd)
+        for (int kd = 0; kd < RC_D / 16; ++kd)
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-            qf[kd][r] = *reinterpret_cast<const float2*>(qh_s + (warp * RC_SUB + g + (r & 1) * 8) * RC_LD + kd * 16 + (r >> 1) * 8 + t2);
-    // Both operands in three parts, the six largest products of the nine: sum[h] += A (16 x 16) B (16 x 8, h-th), low[h] likewise
-    auto six = [&](const Thirds (&x)[4], const unsigned char* base, uint32_t plane, uint32_t at, float (&s0)[4], float (&s1)[4], float (&l0)[4],
-                   float (&l1)[4]) {
-        uint32_t hi[4], mid[4], lo[4], b[3][4];
+            for (int r = 0; r < 4; ++r)
+                qf[kd][r] = *reinterpret_cast<const float2*>(qh_s + (warp * RC_SUB + g + (r & 1) * 8) * RC_LD + kd * 16 + (r >> 1) * 8 + t2);
+        // Both operands in three parts, the six largest products of the nine: sum[h] += A (16 x 16) B (16 x 8, h-th), low[h] likewise
+        auto six = [&](const Thirds (&x)[4], const unsigned char* base, uint32_t plane, uint32_t at, float (&s0)[4], float (&s1)[4], float (&l0)[4],
+                       float (&l1)[4]) {
+            uint32_t hi[4], mid[4], lo[4], b[3][4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) hi[r] = x[r].hi, mid[r] = x[r].mid, lo[r] = x[r].lo;
+            for (int r = 0; r < 4; ++r) hi[r] = x[r].hi, mid[r] = x[r].mid, lo[r] = x[r].lo;
 #pragma unroll
-        for (int p = 0; p < 3; ++p) ldmatrix_x4(b[p], base + p * plane + at);
-        float sum[2][4];
-        MmaFirst{}(sum[0], hi, b[0][0], b[0][1]);
-        MmaFirst{}(sum[1], hi, b[0][2], b[0][3]);
+            for (int p = 0; p < 3; ++p) ldmatrix_x4(b[p], base + p * plane + at);
+            float sum[2][4];
+            MmaFirst{}(sum[0], hi, b[0][0], b[0][1]);
+            MmaFirst{}(sum[1], hi, b[0][2], b[0][3]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s0[e] += sum[0][e], s1[e] += sum[1][e];
-        mma_bf16_16816(l0, lo, b[0][0], b[0][1]);
-        mma_bf16_16816(l1, lo, b[0][2], b[0][3]);
-        mma_bf16_16816(l0, mid, b[1][0], b[1][1]);
-        mma_bf16_16816(l1, mid, b[1][2], b[1][3]);
-        mma_bf16_16816(l0, hi, b[2][0], b[2][1]);
-        mma_bf16_16816(l1, hi, b[2][2], b[2][3]);
-        mma_bf16_16816(l0, mid, b[0][0], b[0][1]);
-        mma_bf16_16816(l1, mid, b[0][2], b[0][3]);
-        mma_bf16_16816(l0, hi, b[1][0], b[1][1]);
-        mma_bf16_16816(l1, hi, b[1][2], b[1][3]);
-    };
-    auto values = [&](int c, const float (&s)[2][4]) {   // acc += s (16 x 16 tokens of quarter c) v
-        uint32_t part[3][4];
+            for (int e = 0; e < 4; ++e) s0[e] += sum[0][e], s1[e] += sum[1][e];
+            mma_bf16_16816(l0, lo, b[0][0], b[0][1]);
+            mma_bf16_16816(l1, lo, b[0][2], b[0][3]);
+            mma_bf16_16816(l0, mid, b[1][0], b[1][1]);
+            mma_bf16_16816(l1, mid, b[1][2], b[1][3]);
+            mma_bf16_16816(l0, hi, b[2][0], b[2][1]);
+            mma_bf16_16816(l1, hi, b[2][2], b[2][3]);
+            mma_bf16_16816(l0, mid, b[0][0], b[0][1]);
+            mma_bf16_16816(l1, mid, b[0][2], b[0][3]);
+            mma_bf16_16816(l0, hi, b[1][0], b[1][1]);
+            mma_bf16_16816(l1, hi, b[1][2], b[1][3]);
+        };
+        auto values = [&](int c, const float (&s)[2][4]) {   // acc += s (16 x 16 tokens of quarter c) v
+            uint32_t part[3][4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const Thirds x = thirds(s[r >> 1][(r & 1) * 2], s[r >> 1][(r & 1) * 2 + 1]);
-            part[0][r] = x.hi, part[1][r] = x.mid, part[2][r] = x.lo;
-        }
-        uint32_t b[RC_VT / 16][4];
+            for (int r = 0; r < 4; ++r) {
+                const Thirds x = thirds(s[r >> 1][(r & 1) * 2], s[r >> 1][(r & 1) * 2 + 1]);
+                part[0][r] = x.hi, part[1][r] = x.mid, part[2][r] = x.lo;
+            }
+            uint32_t b[RC_VT / 16][4];
 #pragma unroll
-        for (int vp = 0; vp < RC_VT / 16; ++vp) ldmatrix_x4_trans(b[vp], v_s + tile_at<RC_VT>(c * 16 + (lane & 15), vp * 2 + (lane >> 4)));
-        float sum[RC_VT / 8][4];
-#pragma unroll
-        for (int vp = 0; vp < RC_VT / 16; ++vp) {
-            MmaFirst{}(sum[2 * vp], part[0], b[vp][0], b[vp][1]);
-            MmaFirst{}(sum[2 * vp + 1], part[0], b[vp][2], b[vp][3]);
-        }
-#pragma unroll
-        for (int p = 2; p >= 1; --p)
+            for (int vp = 0; vp < RC_VT / 16; ++vp) ldmatrix_x4_trans(b[vp], v_s + tile_at<RC_VT>(c * 16 + (lane & 15), vp * 2 + (lane >> 4)));
+            float sum[RC_VT / 8][4];
 #pragma unroll
             for (int vp = 0; vp < RC_VT / 16; ++vp) {
-                mma_bf16_16816(low[2 * vp], part[p], b[vp][0], b[vp][1]);
-                mma_bf16_16816(low[2 * vp + 1], part[p], b[vp][2], b[vp][3]);
+                MmaFirst{}(sum[2 * vp], part[0], b[vp][0], b[vp][1]);
+                MmaFirst{}(sum[2 * vp + 1], part[0], b[vp][2], b[vp][3]);
             }
-        add_sums(acc, sum);
-    };
-    // ---- this quarter's own pairs
-    {
-        float s[2][4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+            for (int p = 2; p >= 1; --p)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int row = g + (e >> 1) * 8, col = h * 8 + t2 + (e & 1);
-                s[h][e] = col <= row ? pair_s[warp][row][col] : 0.f;
-            }
-        if (!not_finite) {
-            values(warp, s);
-        } else {   // token by token, so that what lies behind a row is left out and not multiplied by zero
+                for (int vp = 0; vp < RC_VT / 16; ++vp) {
+                    mma_bf16_16816(low[2 * vp], part[p], b[vp][0], b[vp][1]);
+                    mma_bf16_16816(low[2 * vp + 1], part[p], b[vp][2], b[vp][3]);
+                }
+            add_sums(acc, sum);
+        };
+        // ---- this quarter's own pairs
+        {
+            float s[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = g + (e >> 1) * 8, col = h * 8 + t2 + (e & 1);
+                    s[h][e] = col <= row ? pair_s[warp][row][col] : 0.f;
+                }
+            if (!not_finite) {
+                values(warp, s);
+            } else {   // token by token, so that what lies behind a row is left out and not multiplied by zero
 #pragma unroll 1
-            for (int j = 0; j < RC_SUB; ++j) {
-                const float p0 = j <= g ? pair_s[warp][g][j] : 0.f, p1 = j <= g + 8 ? pair_s[warp][g + 8][j] : 0.f;
+                for (int j = 0; j < RC_SUB; ++j) {
+                    const float p0 = j <= g ? pair_s[warp][g][j] : 0.f, p1 = j <= g + 8 ? pair_s[warp][g + 8][j] : 0.f;
 #pragma unroll
-                for (int nt = 0; nt < RC_VT / 8; ++nt) {
-                    const uint32_t x = *reinterpret_cast<const uint32_t*>(v_s + tile_at<RC_VT>(warp * 16 + j, nt) + t2 * 2);
-                    if (j <= g) acc[nt][0] = fmaf(p0, lower_bf16(x), acc[nt][0]), acc[nt][1] = fmaf(p0, upper_bf16(x), acc[nt][1]);
-                    if (j <= g + 8) acc[nt][2] = fmaf(p1, lower_bf16(x), acc[nt][2]), acc[nt][3] = fmaf(p1, upper_bf16(x), acc[nt][3]);
+                    for (int nt = 0; nt < RC_VT / 8; ++nt) {
+                        const uint32_t x = *reinterpret_cast<const uint32_t*>(v_s + tile_at<RC_VT>(warp * 16 + j, nt) + t2 * 2);
+                        if (j <= g) acc[nt][0] = fmaf(p0, lower_bf16(x), acc[nt][0]), acc[nt][1] = fmaf(p0, upper_bf16(x), acc[nt][1]);
+                        if (j <= g + 8) acc[nt][2] = fmaf(p1, lower_bf16(x), acc[nt][2]), acc[nt][3] = fmaf(p1, upper_bf16(x), acc[nt][3]);
+                    }
                 }
             }
         }
-    }
-    // ---- the quarters before it, the nearest first; the decays of each gather on the queries
-    for (int c = warp - 1; c >= 0; --c) {
-        float s[2][4], s_low[2][4];
+        // ---- the quarters before it, the nearest first; the decays of each gather on the queries
+        for (int c = warp - 1; c >= 0; --c) {
+            float s[2][4], s_low[2][4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) s[h][e] = s_low[h][e] = 0.f;
+                for (int e = 0; e < 4; ++e) s[h][e] = s_low[h][e] = 0.f;
+#pragma unroll
+            for (int kd = 0; kd < RC_D / 16; ++kd) {
+                Thirds x[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) x[r] = thirds(qf[kd][r].x, qf[kd][r].y);
+                six(x, kh_s, RC_PLANE, tile_at<RC_D>(c * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)), s[0], s[1], s_low[0], s_low[1]);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float2 all = *reinterpret_cast<const float2*>(&all_s[c][kd * 16 + (r >> 1) * 8 + t2]);
+                    qf[kd][r].x *= all.x, qf[kd][r].y *= all.y;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[h][e] += s_low[h][e];
+            values(c, s);
+        }
+        // ---- the state before the chunk
 #pragma unroll
         for (int kd = 0; kd < RC_D / 16; ++kd) {
             Thirds x[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) x[r] = thirds(qf[kd][r].x, qf[kd][r].y);
-            six(x, kh_s, RC_PLANE, tile_at<RC_D>(c * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)), s[0], s[1], s_low[0], s_low[1]);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float2 all = *reinterpret_cast<const float2*>(&all_s[c][kd * 16 + (r >> 1) * 8 + t2]);
-                qf[kd][r].x *= all.x, qf[kd][r].y *= all.y;
-            }
+            for (int vp = 0; vp < RC_VT / 16; ++vp)
+                six(x, s_s, RC_VT * RC_D * 2, tile_at<RC_D>(vp * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)), acc[2 * vp], acc[2 * vp + 1],
+                    low[2 * vp], low[2 * vp + 1]);
         }
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int nt = 0; nt < RC_VT / 8; ++nt)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) s[h][e] += s_low[h][e];
-        values(c, s);
-    }
-    // ---- the state before the chunk
+            for (int e = 0; e < 4; ++e) acc[nt][e] += low[nt][e];
+        const int row = warp * RC_SUB + g, y_width = a.n_heads * a.vdim;
+        float* y0 = a.y + (size_t)(t0 + row) * y_width + head * a.vdim + v0 + t2;
 #pragma unroll
-    for (int kd = 0; kd < RC_D / 16; ++kd) {
-        Thirds x[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) x[r] = thirds(qf[kd][r].x, qf[kd][r].y);
-#pragma unroll
-        for (int vp = 0; vp < RC_VT / 16; ++vp)
-            six(x, s_s, RC_VT * RC_D * 2, tile_at<RC_D>(vp * 16 + (lane & 7) + ((lane >> 4) << 3), kd * 2 + ((lane >> 3) & 1)), acc[2 * vp], acc[2 * vp + 1],
-                low[2 * vp], low[2 * vp + 1]);
-    }
-#pragma unroll
-    for (int nt = 0; nt < RC_VT / 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[nt][e] += low[nt][e];
-    const int row = warp * RC_SUB + g, y_width = a.n_heads * a.vdim;
-    float* y0 = a.y + (size_t)(t0 + row) * y_width + head * a.vdim + v0 + t2;
-#pragma unroll
-    for (int nt = 0; nt < RC_VT / 8; ++nt) {
-        if (row < n_here) *reinterpret_cast<float2*>(y0 + nt * 8) = make_float2(acc[nt][0], acc[nt][1]);
-        if (row + 8 < n_here) *reinterpret_cast<float2*>(y0 + 8 * (size_t)y_width + nt * 8) = make_float2(acc[nt][2], acc[nt][3]);
+        for (int nt = 0; nt < RC_VT / 8; ++nt) {
+            if (row < n_here) *reinterpret_cast<float2*>(y0 + nt * 8) = make_float2(acc[nt][0], acc[nt][1]);
+            if (row + 8 < n_here) *reinterpret_cast<float2*>(y0 + 8 * (size_t)y_width + nt * 8) = make_float2(acc[nt][2], acc[nt][3]);
+        }
     }
 }
 
@@ -495,10 +507,15 @@ QF_EXPORT int qf_row_chunks(const void* q, int q_stride, const void* k, int k_st
     float *whole = scratch + n_records * n_heads * dim * vdim, *carry = whole + n_records * n_heads * dim;
     float* made = carry + (each > 0 ? (long long)n_seqs * n_heads * dim * vdim : 0);
     RowChunkArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, decay, decay_bias, bonus, kind, inv_tau,
-                         cu_q, slots, state, slot_stride, s_offset, n_heads, vdim, q_scale, scratch, whole, made, y, Portion{0, each, each > 0 ? carry : nullptr}};
+                         cu_q, slots, state, slot_stride, s_offset, n_heads, vdim, q_scale, scratch, whole, made, y, Portion{0, each, each > 0 ? carry : nullptr}, 1};
     const int chunks = (max_q_len + RC_CHUNK - 1) / RC_CHUNK;
     const size_t parts_smem = 3 * RC_PLANE + RC_CHUNK * RC_LH * 2 + (size_t)RC_CHUNK * vdim * 2;
-    const size_t outputs_smem = 3 * RC_PLANE + 2 * RC_CHUNK * RC_LD * 4 + 2 * RC_CHUNK * RC_LH * 2 + RC_CHUNK * RC_VT * 2;
+    // A block of outputs takes two tiles of v one after the other, with the same weights, pairs and parts of the operands, where the blocks
+    // still fill the SMs' two places each (3,079 tokens of 16 heads of 64 x 128: 96 microseconds with one, 83 with two); else one.
+    const int v_tiles = vdim / RC_VT;
+    const long long at_most = each > 0 ? (long long)min(each, (max_q_len + RC_CHUNK - 1) / RC_CHUNK) * n_seqs : n_records;
+    a.v_each = v_tiles % 2 == 0 && at_most * n_heads * (v_tiles / 2) >= 2ll * qf_sm_count() ? 2 : 1;
+    const size_t outputs_smem = 3 * RC_PLANE + 2 * RC_CHUNK * RC_LD * 4 + 2 * RC_CHUNK * RC_LH * 2 + (size_t)a.v_each * RC_CHUNK * RC_VT * 2;
     auto outputs = bonus ? row_outputs_kernel<true> : row_outputs_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(row_parts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)parts_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(outputs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outputs_smem);
@@ -509,7 +526,7 @@ QF_EXPORT int qf_row_chunks(const void* q, int q_stride, const void* k, int k_st
         e = launch_pdl(row_parts_kernel, dim3(here, n_heads, n_seqs), dim3(128), parts_smem, stream, a);
         if (e == cudaSuccess)
             e = launch_pdl(row_chain_kernel, dim3((vdim / 8 * (RC_D / 16) + 7) / 8, n_heads, n_seqs), dim3(256), 0, stream, a);
-        if (e == cudaSuccess) e = launch_pdl(outputs, dim3(here, vdim / RC_VT * n_heads, n_seqs), dim3(128), outputs_smem, stream, a);
+        if (e == cudaSuccess) e = launch_pdl(outputs, dim3(here, v_tiles / a.v_each * n_heads, n_seqs), dim3(128), outputs_smem, stream, a);
     }
     return (int)e;
 }
