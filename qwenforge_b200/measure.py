@@ -23,7 +23,7 @@ decode-attention  the split-K decode attention's own time stamps (launched alone
            projection that folds the partial results
 scan       the recurrence of the recurrent mixers (recurrent.cu) alone, on a prompt and on a decode step
 gemm       a feed-forward's gate/up product on many rows: the library product, the library product and the gate kernel,
-           this library's tcgen05 product (one tile per block, and persistent) plain and with the gate in its epilogue
+           this library's tcgen05 product (one tile per block, and on pairs of SMs) plain and with the gate in its epilogue
 """
 from __future__ import annotations
 
@@ -378,13 +378,13 @@ def measure_gemm(args) -> None:
         print("  library product                                   " + rate(timed(lambda: torch.mm(x, w.t(), out=full))))
         print("  library product, then the gate kernel             " + rate(timed(lambda: (torch.mm(x, w.t(), out=full), ops.swiglu(full, act)))))
         try:
-            for mode, name in ((0, "one tile per block"), (1, "persistent")):
+            for mode, name in ((0, "one tile per block"), (1, "pairs of SMs")):
                 switch(ctypes.c_int(mode))
                 print(f"  tcgen05 product, {name:19s}              " + rate(timed(lambda: ops.tc_gemm(ops.TC_PLAIN, x, w, full))))
                 print(f"  tcgen05 product with the gate, {name:19s}" + rate(timed(lambda: ops.tc_gemm(ops.TC_SWIGLU, x, w, act))), flush=True)
         finally:
             switch(ctypes.c_int(1))
-        print(f"  (the persistent kernel {'runs' if ops.tc_gemm_is_persistent(ops.TC_SWIGLU, rows, 2 * inter) else 'does not run: too few tiles'} at this size)")
+        print(f"  (the pairs' kernel {'runs' if ops.tc_gemm_is_persistent(ops.TC_SWIGLU, rows, 2 * inter) else 'does not run: too few tiles'} at this size)")
         # the query/key/value product: library product and the rotation / cache-write kernel, against the tcgen05 product
         # with bias, rotation and cache write in its epilogue
         _, _, heads, kv_heads, head_dim = sizes_of(args.preset)
@@ -410,6 +410,9 @@ def measure_gemm(args) -> None:
             angles = ops.rope_table(tok_pos, inv_freq)
             print("  tcgen05 product with bias, rotation, cache write  " + rate_q(timed(lambda: ops.tc_gemm_qkv(
                 x, wq, bq, angles, tok_seq, tok_pos, slots, heads, q_out, pages.args(), True, err))), flush=True)
+        if ops.qkv_product_takes(x, wq, head_dim, pages.args()):
+            print("  the same on pairs of SMs, angles made inside      " + rate_q(timed(lambda: ops.qkv_product(
+                x, wq, bq, inv_freq, tok_seq, tok_pos, slots, heads, q_out, pages.args(), True, err))), flush=True)
         if int(err):
             raise RuntimeError(f"a kernel reported error word {int(err)}")
 
