@@ -265,20 +265,27 @@ __global__ void attention_generic_fold_kernel(T* __restrict__ out, const int* __
 // a load from shared memory feeds four multiply-adds (in the kernel above: one). Every score is one chain over the components,
 // every output one chain over the keys in rising order, pages at multiples of 64, so a row's arithmetic depends on its own
 // position and window only, as above and whatever RT (the two kernels differ by rounding). What bounds it is the
-// multiply-add pipe and the walk of the longest tile: one prompt of 1,031 tokens, 14 heads of 64: 893 -> 122 microseconds.
+// multiply-add pipe and the walk of the longest tile: one prompt of 1,031 tokens, 14 heads of 64: 893 -> 102 microseconds.
+// `wave` > 0: that many blocks (one for every SM) start at a time, longest walks first, the next ones in rising order, so that an SM's
+// second block is the shorter the longer its first is (118 microseconds there with all in falling order).
 #define FT_THREADS 256
 template <int D, int RT>
 __global__ void __launch_bounds__(FT_THREADS)
 attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, const int* __restrict__ cu_q,
                           const int* __restrict__ tok_pos, const int* __restrict__ slots, KvSite<float> site, int n_heads, float scale,
-                          int window, int* err) {
+                          int window, int* err, int wave) {
     constexpr int LD = D + 4, LP = QF_PAGE + 4, PIECES = D / 4, DT = D / 16, ROWS = 16 * RT;
     extern __shared__ __align__(16) float ft_smem[];
     float* q_s = ft_smem;                   // [ROWS][LD]
     float* k_s = q_s + ROWS * LD;           // [64][LD]
     float* v_s = k_s + QF_PAGE * LD;        // [64][LD]
     float* p_s = v_s + QF_PAGE * LD;        // [ROWS][LP]: the page's weights, a row per query
-    const int tile = (int)gridDim.y - 1 - (int)blockIdx.y, kvh = blockIdx.x, seq = blockIdx.z;   // the longest walks first
+    int turn = (int)(blockIdx.y * gridDim.x + blockIdx.x);
+    if (wave > 0 && turn / wave & 1) {
+        const int n = (int)(gridDim.x * gridDim.y), first = turn / wave * wave;
+        turn = first + min(first + wave, n) - 1 - turn;
+    }
+    const int tile = (int)gridDim.y - 1 - turn / (int)gridDim.x, kvh = turn % (int)gridDim.x, seq = blockIdx.z;   // the longest walks first
     const int group = n_heads / site.kv_heads, row0 = tile * ROWS;
     const int q_begin = cu_q[seq], q_rows = (cu_q[seq + 1] - q_begin) * group;
     if (row0 >= q_rows) return;
@@ -450,13 +457,13 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
 
 template <int D, int RT>
 static int launch_f32_tile(const float* q, float* out, const int* cu_q, const int* tok_pos, const int* slots, KvSite<float> site,
-                           int n_heads, int n_seqs, int max_q_len, float scale, int window, int* err, cudaStream_t stream) {
+                           int n_heads, int n_seqs, int max_q_len, float scale, int window, int* err, int wave, cudaStream_t stream) {
     constexpr size_t smem = (size_t)((16 * RT + 2 * QF_PAGE) * (D + 4) + 16 * RT * (QF_PAGE + 4)) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<D, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int rows = max_q_len * (n_heads / site.kv_heads);
     attention_f32_tile_kernel<D, RT><<<dim3(site.kv_heads, (rows + 16 * RT - 1) / (16 * RT), n_seqs), FT_THREADS, smem, stream>>>(
-        q, out, cu_q, tok_pos, slots, site, n_heads, scale, window, err);
+        q, out, cu_q, tok_pos, slots, site, n_heads, scale, window, err, wave);
     return (int)cudaGetLastError();
 }
 
@@ -542,10 +549,19 @@ QF_EXPORT int qf_attention_generic_biased(int is_bf16, const void* q, void* out,
         const KvSite<float> site{(float*)base, table, page_elems, table_stride, kv_heads, head_dim};
         // sequences of few rows in tiles of 16 (the same bits): 64 of two tokens from position 0, 14 kv heads of 64: 40 -> 13 microseconds
         const bool few = (long long)max_q_len * (n_heads / kv_heads) <= 16;
+        // One sequence: tiles of 32 rows (the same bits) where those of 64 would leave SMs without one, in waves of alternating order as
+        // long as all blocks find room at once (two or four of 32 rows and three of 64 with heads of 64 on an SM). Microseconds, tiles of 64 in falling
+        // order / so: 14 heads of 64, 70 tokens 14.4 / 11.4, 200 25.5 / 20.0, 500 48.3 / 40.5, 1,031 118 / 102, 1,500 190.3 / 190.5; 16 heads of 128,
+        // 70 tokens 22.5 / 16.7, 200 41.9 / 30.8, 500 80.4 / 64.4. Elsewhere the larger tile's fewer reads of shared memory and the falling order
+        // are ahead: 700 tokens, tiles of 32 rows 69.1 / 75.4 and 109 / 115; 1,031 tokens of 128 in waves 165 / 188; 3,000 of 64 504 / 535.
+        const int sms = qf_sm_count();
+        const long long blocks = ((long long)max_q_len * (n_heads / kv_heads) + 63) / 64 * kv_heads;
+        const bool half = n_seqs == 1 && blocks <= sms;
+        const int wave = half || (n_seqs == 1 && head_dim == 64 && blocks <= 3ll * sms) ? sms : 0;
 #define QF_F32_TILE(D, RT) \
-    launch_f32_tile<D, RT>((const float*)q, (float*)out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, stream)
-        if (head_dim == 64) return few ? QF_F32_TILE(64, 1) : QF_F32_TILE(64, 4);
-        return few ? QF_F32_TILE(128, 1) : QF_F32_TILE(128, 4);
+    launch_f32_tile<D, RT>((const float*)q, (float*)out, cu_q, tok_pos, slots, site, n_heads, n_seqs, max_q_len, scale, window, err, wave, stream)
+        if (head_dim == 64) return few ? QF_F32_TILE(64, 1) : half ? QF_F32_TILE(64, 2) : QF_F32_TILE(64, 4);
+        return few ? QF_F32_TILE(128, 1) : half ? QF_F32_TILE(128, 2) : QF_F32_TILE(128, 4);
 #undef QF_F32_TILE
     }
     QF_GENERIC_DISPATCH(launch, q, out, cu_q, tok_pos, slots, base, table, page_elems, table_stride, kv_heads, head_dim,

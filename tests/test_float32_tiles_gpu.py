@@ -103,3 +103,23 @@ def test_short_sequences_alone_and_beside_long_ones(heads, kv_heads, dim):
         ops.attention_generic(q[rows].contiguous(), alone, ints([0, n]), ints(pos[rows]), ints([s]), site, heads, 1, n, dim ** -0.5, 0, err)
         assert torch.equal(alone, out[rows])
     assert int(err) == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,tokens", [(14, 2, 64, 70), (14, 2, 64, 676), (14, 2, 64, 677), (14, 2, 64, 1360), (14, 2, 64, 2030), (8, 2, 128, 1184),
+                                                       (8, 2, 128, 1185), (3, 3, 128, 33)])
+def test_a_sequence_alone_in_smaller_tiles_and_alternating_waves(heads, kv_heads, dim, tokens):
+    """Alone a sequence takes tiles of 32 rows where 64 leave SMs idle, and waves of alternating order; beside another neither: the same bits."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pages = (tokens + 63) // 64 + 1
+    storage = torch.randn(pages + 1, 2, kv_heads, 64, dim, generator=g, device=DEV)
+    table = torch.full((2, pages), -1, dtype=torch.int32)
+    table[0], table[1, 0] = torch.arange(pages), pages
+    site, err = ops.KvSiteArgs(storage, table.to(DEV), kv_heads, dim), ints([0])
+    pos = list(range(11, 11 + tokens))
+    q = torch.randn(tokens + 1, heads * dim, generator=g, device=DEV)
+    both, alone = torch.empty_like(q), torch.full((tokens, heads * dim), float("nan"), device=DEV)
+    ops.attention_generic(q, both, ints([0, tokens, tokens + 1]), ints(pos + [0]), ints([0, 1]), site, heads, 2, tokens, dim ** -0.5, 0, err)
+    ops.attention_generic(q[:tokens].contiguous(), alone, ints([0, tokens]), ints(pos), ints([0]), site, heads, 1, tokens, dim ** -0.5, 0, err)
+    assert int(err) == 0 and torch.equal(alone, both[:tokens])
