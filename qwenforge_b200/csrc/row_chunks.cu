@@ -15,7 +15,7 @@
 // or is divided. Every float32 operand of a product on the tensor cores is the exact sum of three bfloat16 numbers; of
 // the nine products of two of them the six largest are taken (what is left out is below 2^-24 of the product, of either sign).
 // What bounds it: the scan is a chain of one update per token (0.18 microseconds each); here the chain is one step per 64 tokens, the
-// rest products and the quarters' own pairs. Measured, 2,048 tokens, 16 heads of 64 x 128: 283 -> 100
+// rest products and the quarters' own pairs. Measured, 2,048 tokens, 16 heads of 64 x 128: 283 -> 70
 // microseconds; 7 heads: 262 -> 56.
 #include "chunks.cuh"
 

@@ -9,7 +9,7 @@
 // chunk's own sum; (2) `chain`: the states before every chunk; (3) `outputs`.
 // What bounds it: the scan is a chain of one update per token (0.12 microseconds each, whatever the width of the GPU); here
 // the chain is one step per 128 tokens and everything else is products. Measured on one prompt of 2,048 tokens, 7 heads of
-// 64 x 128: 200 -> 30 microseconds; 32 heads of 128 x 128: 427 -> 104.
+// 64 x 128: 200 -> 29 microseconds; 32 heads of 128 x 128: 427 -> 97.
 // (One block walking a sequence's chunks with its tile of S in registers moves fewer bytes than parts and chain, and took
 // 46 and 105 microseconds where these take 16 and 71: a link of that chain is a chunk's products, 3 microseconds.)
 // 128 tokens per chunk: with 64 the records (32 heads x 64 KB a chunk) are twice the bytes, with 256 the products inside

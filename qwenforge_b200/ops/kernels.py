@@ -1932,7 +1932,7 @@ def _chunks_pay(n: int, n_seqs: int, longest: int, state: int, chunk: int, scan:
 STATE_CHUNK = 128   # SC_CHUNK of csrc/state_chunks.cu
 # The longest sequence of a step from which the chunked form is the faster one. Measured inside a graph, one sequence, scan / chunks in
 # microseconds: 7 heads of 64 x 128: 192 tokens 21 / 18, 256: 28 / 18, 2,048: 200 / 30; 16 heads 23 / 23, 29 / 23, 214 / 41; 32 heads of
-# 128 x 128: 43 / 32, 57 / 32, 427 / 104. Three launches and a buffer instead of one launch cost the host about 10 microseconds more,
+# 128 x 128: 43 / 32, 57 / 32, 427 / 97. Three launches and a buffer instead of one launch cost the host about 10 microseconds more,
 # which a step that is issued launch by launch feels up to some 200 tokens.
 STATE_CHUNKS_MIN_TOKENS = 192
 # Beside other sequences (`_chunks_pay`), inside a graph, scan / chunks: 7 heads of 64 x 128: 192 + 31 x 1 tokens 24 / 41, 512 + 31 x 1
@@ -2431,8 +2431,8 @@ ROW_CHUNK = 64   # RC_CHUNK of csrc/row_chunks.cu
 # launches and a buffer more cost it 5 of 103 microseconds.
 ROW_CHUNKS_MIN_TOKENS = 512
 # Beside other sequences (`_chunks_pay`), inside a graph, scan / chunks: 7 heads of 64 x 128: 512 + 31 x 1 tokens 71 / 60, 512 + 63 x 1
-# 77 / 93, 64 x 512 1,235 / 598; 16 heads: 512 + 31 x 1 89 / 109, 1,024 + 31 x 1 173 / 138; 32 heads of 64 x 64: 1,024 + 63 x 1
-# 178 / 266, 4 x 1,024 406 / 230.
+# 74 / 84, 64 x 512 1,238 / 416; 16 heads: 512 + 31 x 1 88 / 104, 1,024 + 31 x 1 172 / 123; 32 heads of 64 x 64: 1,024 + 63 x 1
+# 176 / 288, 4 x 1,024 400 / 164.
 ROW_CHUNKS_COSTS = ((0.13, 0.0, 0.04, 0.2), (20.0, 1.3))
 
 
