@@ -123,3 +123,20 @@ def test_a_sequence_alone_in_smaller_tiles_and_alternating_waves(heads, kv_heads
     ops.attention_generic(q, both, ints([0, tokens, tokens + 1]), ints(pos + [0]), ints([0, 1]), site, heads, 2, tokens, dim ** -0.5, 0, err)
     ops.attention_generic(q[:tokens].contiguous(), alone, ints([0, tokens]), ints(pos), ints([0]), site, heads, 1, tokens, dim ** -0.5, 0, err)
     assert int(err) == 0 and torch.equal(alone, both[:tokens])
+
+
+@pytest.mark.parametrize("rows,inter", [(1, 4), (3, 20), (700, 1028), (1031, 4864)])
+def test_the_gate_four_numbers_at_a_time(rows, inter):
+    """Rows on 16-byte boundaries and the same rows off them (the kernel of single numbers): the same bits, also of what is not finite."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    gu = 4 * torch.randn(rows, 2 * inter, generator=g, device=DEV)
+    gu[0, :4] = torch.tensor([float("inf"), float("-inf"), float("nan"), -200.0], device=DEV)
+    out, off = torch.empty(rows, inter, device=DEV), torch.empty(1 + rows * inter, device=DEV)[1:].view(rows, inter)
+    ops.swiglu(gu, out)
+    ops.swiglu(gu, off)
+    assert torch.equal(out.view(torch.int32), off.view(torch.int32).contiguous())
+    want = torch.nn.functional.silu(gu[:, :inter].double()) * gu[:, inter:].double()
+    fine = torch.isfinite(want) & (want.abs() > 1e-30)
+    # expf within 2 units, a sum, a quotient and a product: below eight roundings of 2^-24
+    assert bool(((out.double() - want).abs() <= 8 * 2.0 ** -24 * want.abs())[fine].all())
