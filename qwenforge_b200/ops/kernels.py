@@ -919,19 +919,17 @@ def qkv_product_way(m: int, weight: torch.Tensor, n_heads: int, kv_heads: int, h
 
 
 def gate_product_way(m: int, weight: torch.Tensor) -> str:
-    """How `m` token rows (64 at most) are normalised, multiplied by a [gate | up] weight and gated fastest: "skinny" (the mma.sync
-    streamer with all of it inside), "wide" (a norm kernel, then the tcgen05 streamer with the gate in its epilogue) or "unfused" (norm,
-    library product, gate kernel). Measured as norm, gate/up and down together over weights that the L2 does not hold, microseconds,
-    the other way / "wide": 17 MB (Qwen2.5-0.5B's) 8 rows 10.4 / 13.2, 9 rows 14.9 / 14.4, 16 rows 15.1 / 14.4, 24 rows 16.8 / 15.7, 48 rows
-    18.1 / 17.6, 64 rows 17.7 / 18.7; 55 MB 1 row 23.5 / 22.0, 8 rows 24.9 / 23.1, 16 rows 27.6 / 23.8, 24 rows 25.3 / 24.9, 64 rows
-    27.8 / 26.8; 90 MB (3B's) 1 row 32.3 / 33.1, 4 rows 34.2 / 33.4, 8 rows 34.8 / 33.8, 16 rows 35.8 / 35.0, 64 rows 40.8 / 38.4; 272 MB (7B's)
-    1 row 76.9 / 69.5, 16 rows 79.5 / 72.4, 64 rows 85.2 / 78.3."""
+    """How `m` token rows (64 at most) are normalised, multiplied by a [gate | up] weight and gated: "skinny" (the mma.sync streamer with
+    all of it inside) where it takes the shape and pays (`skinny_gemm_pays`), else "wide" (a norm kernel, then the tcgen05 streamer with
+    the gate in its epilogue) for weights of 100 MB and more, else "unfused" (norm, library product, gate kernel). Measured as norm, gate/up
+    and down together over weights that the L2 does not hold, microseconds, the other way / "wide": 272 MB (Qwen2.5-7B's) 1 row 76.9 / 69.5,
+    16 rows 79.5 / 72.4, 64 rows 85.2 / 78.3; 90 MB (3B's) 1 row 32.3 / 33.1, 8 rows 34.8 / 33.8, 16 rows 35.8 / 35.0; 17 MB (0.5B's) 8 rows
+    10.4 / 13.2, 16 rows 15.1 / 14.4. "wide" would be ahead by 2 to 5 percent from 4 rows of 32 MB and 9 rows of 16 MB on too, but its gate uses the
+    hardware's exponential and division (an error of 2^-20) where the other two ways use float32's own: that band stays with them."""
     size = weight.numel() * weight.element_size()
-    skinny = m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_SWIGLU, True) and skinny_gemm_pays(m, weight)
-    least = 16e6 if 9 <= m <= 48 else 32e6 if m >= 4 else 100e6
-    if (size >= least or (not skinny and size >= 100e6)) and wide_gemm_takes_rows(EPI_SWIGLU, m, weight):
-        return "wide"
-    return "skinny" if skinny else "unfused"
+    if m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_SWIGLU, True) and skinny_gemm_pays(m, weight):
+        return "skinny"
+    return "wide" if size >= 100e6 and wide_gemm_takes_rows(EPI_SWIGLU, m, weight) else "unfused"
 
 
 def residual_product_way(m: int, weight: torch.Tensor) -> str:

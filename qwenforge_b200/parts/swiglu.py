@@ -52,9 +52,8 @@ class SwiGlu(FeedForward):
         return ops.linear(act, self.down_weight)
 
     # ---- the form for steps of up to 64 tokens that works on the residual stream in place: norm + gate/up + SwiGLU in
-    # one kernel, down + residual in another. Each of the two products goes the way that is fastest by measurement. Gate/up: the
-    # tcgen05 streamer after the norm kernel where `ops.gate_product_way` says so; else the mma.sync streamer where it takes the
-    # shape and pays (`ops.skinny_gemm_pays`); else norm kernel, library product and gate kernel. Down: `ops.residual_product_way`.
+    # one kernel, down + residual in another. Each of the two products chooses its way for itself: gate/up by `ops.gate_product_way`,
+    # down by `ops.residual_product_way`.
     def _ways(self, ctx):
         rows = ctx.n_tokens
         return ops.gate_product_way(rows, self.gate_up_weight), ops.residual_product_way(rows, self.down_weight)
