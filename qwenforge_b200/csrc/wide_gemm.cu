@@ -401,11 +401,14 @@ static void split_k(int sms, WideGeometry& geo) {
 // How `units` weight rows per accumulator are dealt to blocks: tiles of 128 of them leave many SMs without a stream (16 tiles of a
 // 3B down product, split four times along K: 64 of 148), so a tile takes fewer rows where more blocks are done sooner. A block's
 // time is the larger of its stream (62 bytes a nanosecond and SM, 6.2 terabytes a second in all) and of its products (170 nanoseconds a
-// slab and accumulator, whatever the tile's rows), a cluster's exchange counts a microsecond. Norm, gate/up and
+// slab and accumulator, whatever the tile's rows), a cluster's exchange counts a microsecond. All of it is worked out for 16 token columns,
+// however many the step has: the split of K decides in which order a sum is added, so it follows from the weight's shape and the GPU alone,
+// and a row has the same bits beside any number of others. Norm, gate/up and
 // down of a step of 16 rows over weights that the L2 does not hold: 3B sizes 36.6 -> 35.0 microseconds (the down product 64 -> 128 blocks),
 // 7B 75.5 -> 72.4, 0.5B 15.7 -> 14.4. Weights below 16 MB stay in tiles of 128 (0.5B's output projection in 128 blocks instead of 28
 // 6.4 against 5.8 with the norm behind it).
 static void spread_rows(int units, int sms, WideGeometry& geo) {
+    constexpr int NTOK = 16;
     float least = 0.f;
     geo.tiles = (units + WG_BM - 1) / WG_BM;
     geo.box_rows = geo.rows = WG_BM;
@@ -416,7 +419,7 @@ static void spread_rows(int units, int sms, WideGeometry& geo) {
         const int at_once = clusters_at_once(ksplit, sms) > 0 ? clusters_at_once(ksplit, sms) : 1;
         const int rows = std::min(WG_BM, std::max(8, (units + at_once - 1) / at_once)), tiles = (units + rows - 1) / rows;
         const int rounds = (tiles + at_once - 1) / at_once, per = (geo.slabs + ksplit - 1) / ksplit;
-        const float block = (float)per * (float)(geo.accs * rows + geo.ntok) * WG_BK * 2;
+        const float block = (float)per * (float)(geo.accs * rows + NTOK) * WG_BK * 2;
         const float all = (float)geo.accs * (float)units * (float)geo.slabs * WG_BK * 2 / 6200.f;   // nanoseconds
         const float stream = std::max((float)rounds * block / 62.f, all), products = (float)rounds * (float)(per * geo.accs) * 170.f;
         const float time = std::max(stream, products) + (ksplit > 1 ? 1000.f : 0.f);

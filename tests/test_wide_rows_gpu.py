@@ -46,3 +46,20 @@ def test_gate_and_up(m, inter, k):
     slack = 1.1 * (slack[:, :inter] * (up.abs() + 1) + slack[:, inter:] * (gate.abs() + 1)) + want.abs() * 2.0 ** -20
     assert int(err) == 0 and bool(((out[:m].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-30).all())
     assert bool((out[m] == 7).all())
+
+
+@pytest.mark.parametrize("n,k", [(6656, 1536), (2048, 11008), (3584, 18944), (1030, 8200), (7000, 1224)])
+def test_a_row_has_the_same_bits_beside_any_number_of_others(n, k):
+    """The split of K, which decides the order of a sum, follows from the weight's shape and not from the step's rows."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x, w = torch.randn(64, k, generator=g, device=DEV).bfloat16(), (torch.randn(n, k, generator=g, device=DEV) * k ** -0.5).bfloat16()
+    stream, err = torch.randn(64, n, generator=g, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    results = []
+    for m in (1, 16, 17, 33, 64):
+        got = stream[:m].clone()
+        ops.wide_gemm(ops.EPI_RESIDUAL, w, x=x[:m], residual=got, err=err)
+        results.append(got)
+    assert int(err) == 0
+    for got in results[:-1]:
+        assert torch.equal(got, results[-1][:got.shape[0]])
