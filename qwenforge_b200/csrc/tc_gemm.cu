@@ -636,13 +636,18 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     }
                     if (c + 64 >= OWN) sums_read();
                     else __syncwarp();
-                    // n_out is a multiple of eight: a piece is whole or beyond the matrix
                     const int pieces = n_cols / 8;
 #pragma unroll
                     for (int u = 0; u < pieces; ++u) {
                         const int r = (u * 32 + lane) / pieces, piece = (u * 32 + lane) % pieces, col = col0 + c + 8 * piece;
-                        if (row0 + r < M && col < n_out)
-                            *reinterpret_cast<uint4*>(out + (size_t)(row0 + r) * ldo + col) = *patch_at(patch, r, piece);
+                        if (row0 + r >= M || col >= n_out) continue;
+                        bf16* dst = out + (size_t)(row0 + r) * ldo + col;
+                        const uint4* src = patch_at(patch, r, piece);
+                        if (EPI != TC_PLAIN || col + 8 <= n_out) {   // (TC_SWIGLU: n_out is a multiple of eight)
+                            *reinterpret_cast<uint4*>(dst) = *src;
+                        } else {                                    // a ragged last piece: what lies behind the row's columns is not this product's
+                            for (int j = 0; j < n_out - col; ++j) dst[j] = reinterpret_cast<const bf16*>(src)[j];
+                        }
                     }
                     __syncwarp();
                 }

@@ -104,3 +104,21 @@ def test_columns_that_stay_float32(m, n, extra, k):
     round_off[n:] = 0
     assert int(err) == 0 and bool(((got - want).abs() <= want.abs() * round_off + slack + 1e-30).all())
     assert bool((out[m] == 7).all() and (out[:, n:] == 7).all() and (tail[m] == 7).all())
+
+
+@pytest.mark.parametrize("m,cols,columns", [(2047, 4861, 192), (1793, 2561, 192), (4100, 2564, 256), (4100, 2567, 256), (100, 77, 0)])
+def test_columns_that_are_no_whole_pieces(m, cols, columns):
+    """A last piece of one to seven columns: they are the product's, what stands behind them in the rows' padding stays as it is."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.csrc import library
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    x, w = torch.randn(m, 72, generator=g, device=DEV).bfloat16(), (torch.randn(cols, 72, generator=g, device=DEV) / 8).bfloat16()
+    assert ops.tc_gemm_is_persistent(ops.TC_PLAIN, m, cols) == (columns > 0)
+    assert columns == 0 or library("tc_gemm").qf_tc_gemm_pair_columns(ctypes.c_int(ops.TC_PLAIN), ctypes.c_int(m), ctypes.c_int(cols)) == columns
+    rows = torch.full((m, cols // 8 * 8 + 16), 7.0, dtype=torch.bfloat16, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.tc_gemm(ops.TC_PLAIN, x, w, rows[:, :cols], err)
+    want = x.double() @ w.double().T
+    slack = (x.double().abs() @ w.double().abs().T) * 72 * 2.0 ** -24
+    assert int(err) == 0 and bool(((rows[:, :cols].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-30).all())
+    assert bool((rows[:, cols:] == 7).all())
