@@ -23,7 +23,8 @@ TIMED = ("embed_gather", "gather_rows", "add_rms_norm", "residual_add", "linear"
          "head_gate", "pool_cache_write", "add_rms_norm_scaled", "residual_add_scaled", "rms_norm_cols", "mix_rows", "bias_glu",
          "shift_mix", "channel_decay", "outer_state_scan_rows", "row_chunks", "rows_prepare", "causal_conv_cached", "delta_scan", "delta_token",
          "streams_norm", "rotate_heads", "sigmoid_gate", "pair_rms_norm", "map_difference", "rope_maps_cache_write", "rope_table",
-         "retention_chunks", "retention_token", "retention_rows")
+         "retention_chunks", "retention_token", "retention_rows", "qkv_product", "tc_gemm_tail", "gated_rows", "attention_decode_plan",
+         "decode_advance_embed")
 
 
 class KernelTimer:
@@ -43,7 +44,8 @@ class KernelTimer:
             start.record()
             out = fn(*args, **kwargs)
             end.record()
-            self.records.append((label, start, end))
+            if out is not False:   # (`gated_rows` says so where it launched nothing)
+                self.records.append((label, start, end))
             return out
         return timed
 
