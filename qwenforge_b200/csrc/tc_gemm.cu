@@ -842,13 +842,17 @@ static int qkv_columns(int m, int n, int d, float* busy) {
 // Whether qf_tc_gemm_qkv_pairs is the faster way for these sizes, against the library's product and the rotation kernel behind it: beyond 512
 // rows where its tiles keep three quarters of the pairs at work (7358 x 2560 x 2048: 56 microseconds against 70; 1536 x 2560 x 2048 19.2
 // and 22.0, 60 of 74 pairs; 2048 x 2560 x 2048, 80 of 148, 28.7 and 26.4; 1536 x 4608 x 3584, 108 of 148, 47.8 and 44.5; 256 x 4608 x 3584
-// 20.7 and 18.4), and for heads of 64 with weights of up to 4 MB always (1152 x 896: 7.5 against 8.0 for 64 rows, 8.8 and 10.1 for 900).
+// 20.7 and 18.4), and for heads of 64 with weights of up to 4 MB and K up to 1,280 columns and to the product's own always (1152 x 896: 7.5
+// against 8.0 for 64 rows, 8.8 and 10.1 for 900). A narrow tile's time is its copies of A, K by K, while the library cuts a long K
+// among blocks, so tiles of 64 columns are the faster way up to K = 1,536 and of 128 up to 3,072. With the norm kernel ahead, this
+// way / the other: 64 x 512 x 4096 18.8 / 12.4, 64 x 512 x 1024 9.4 / 8.9, 300 x 1024 x 2048 12.6 / 11.2, 2048 x 512 x 3072 19.9 / 17.3 and
+// 1300 x 1280 x 4096 24.1 / 22.5; within the lines 900 x 1024 x 1536 12.5 / 12.5, 700 x 2560 x 2048 15.4 / 17.6, 4096 x 512 x 3072 28.2 / 30.5.
 QF_EXPORT int qf_tc_gemm_qkv_pairs_pays(int m, int n, int k, int head_dim) {
     if (m <= 0 || n <= 0 || (head_dim != 64 && head_dim != 128)) return 0;
-    if (head_dim == 64 && (long long)n * k * 2 <= (4ll << 20)) return 1;
+    if (head_dim == 64 && (long long)n * k * 2 <= (4ll << 20) && k <= 1280 && k <= n) return 1;
     float busy = 0.f;
-    qkv_columns(m, n, head_dim, &busy);
-    return m > 512 && busy >= 0.75f;
+    const int columns = qkv_columns(m, n, head_dim, &busy);
+    return m > 512 && busy >= 0.75f && (columns > 128 || k <= 24 * columns);
 }
 
 // The same on pairs of SMs, with the angles worked out in the epilogue (args->inv_freq; args->angles is not read): head sizes 64 and 128.

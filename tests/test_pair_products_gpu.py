@@ -122,3 +122,14 @@ def test_columns_that_are_no_whole_pieces(m, cols, columns):
     slack = (x.double().abs() @ w.double().abs().T) * 72 * 2.0 ** -24
     assert int(err) == 0 and bool(((rows[:, :cols].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-30).all())
     assert bool((rows[:, cols:] == 7).all())
+
+
+def test_where_the_qkv_product_on_pairs_pays():
+    """Both sides of the rule's lines: rows, pairs at work, and a K that is long for the tiles' columns."""
+    from qwenforge_b200 import ops
+    pays = lambda m, n, k, dim: ops.qkv_product_pays(m, torch.empty(n, k, dtype=torch.bfloat16, device=DEV), dim)
+    assert all(pays(m, 1152, 896, 64) for m in (1, 64, 900, 8192)) and pays(64, 1536, 1280, 64) and pays(5, 320, 192, 64)
+    assert not any(pays(m, 512, 4096, 64) for m in (1, 64, 900, 2048)) and not pays(64, 512, 1024, 64) and not pays(300, 1024, 2048, 64)
+    assert not pays(900, 1024, 2048, 64) and pays(900, 1152, 1536, 64) and not pays(2048, 512, 3072, 64) and pays(4096, 512, 3072, 64)
+    assert pays(7358, 2560, 2048, 128) and not pays(2048, 2560, 2048, 128) and not pays(512, 2560, 2048, 128) and pays(513, 2560, 2048, 128)
+    assert not pays(1300, 1280, 4096, 128) and pays(3000, 1280, 4096, 128) and not pays(64, 2304, 2048, 64) and pays(900, 2304, 2048, 64)
