@@ -51,18 +51,22 @@ template <> struct Vec4<bf16> {
     }
 };
 
-template <typename T>
+// CONSTANT: no kernel in flight writes the norm's weights, so they are on their way while the kernel before ends: asked for behind the row's
+// sum, from memory that the layer's other weights have pushed out of the L2, they were the last round trip of a decode step's norm.
+template <typename T, bool CONSTANT>
 __global__ void __launch_bounds__(256)
 add_rms_norm_vec_kernel(float* __restrict__ hidden, const T* __restrict__ delta, const T* __restrict__ weight,
                         T* __restrict__ out, int width, float eps) {
-    // the norm's weights, which no kernel writes, are on their way while the kernel before ends: asked for behind the row's sum, from
-    // memory that the layer's other weights have pushed out of the L2, they were the last round trip of a decode step's norm
     grid_launch_dependents();
     typename Vec4<T>::Raw w[4];
+    auto weights = [&]() {
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-        if (threadIdx.x + u * 256 < width / 4) w[u] = reinterpret_cast<const typename Vec4<T>::Raw*>(weight)[threadIdx.x + u * 256];
+        for (int u = 0; u < 4; ++u)
+            if (threadIdx.x + u * 256 < width / 4) w[u] = reinterpret_cast<const typename Vec4<T>::Raw*>(weight)[threadIdx.x + u * 256];
+    };
+    if (CONSTANT) weights();
     grid_dependency_wait();
+    if (!CONSTANT) weights();
     __shared__ float scratch[33];
     float* h = hidden + (size_t)blockIdx.x * width;
     const T* d = delta ? delta + (size_t)blockIdx.x * width : nullptr;
@@ -148,7 +152,7 @@ add_rms_norm_warp_kernel(float* __restrict__ hidden, const T* __restrict__ delta
 
 template <typename T>
 static int launch(float* hidden, const void* delta, const void* weight, void* out, int rows, int width, float eps,
-                  cudaStream_t stream) {
+                  int constant, cudaStream_t stream) {
     if (rows <= 0) return 0;
     const uintptr_t align = (uintptr_t)hidden | (uintptr_t)delta | (uintptr_t)weight | (uintptr_t)out;
     if (width % 4 == 0 && width <= 4 * 32 * NW_MAX && align % 16 == 0) {
@@ -156,15 +160,17 @@ static int launch(float* hidden, const void* delta, const void* weight, void* ou
                                                                                               (T*)out, rows, width, eps);
     }
     if (width % 4 == 0 && width <= 4096 && align % 16 == 0) {
-        return (int)launch_pdl(add_rms_norm_vec_kernel<T>, dim3(rows), dim3(256), 0, stream, hidden, (const T*)delta, (const T*)weight, (T*)out, width, eps);
+        return (int)launch_pdl(constant ? add_rms_norm_vec_kernel<T, true> : add_rms_norm_vec_kernel<T, false>, dim3(rows), dim3(256), 0, stream, hidden,
+                               (const T*)delta, (const T*)weight, (T*)out, width, eps);
     }
     return (int)launch_pdl(add_rms_norm_kernel<T>, dim3(rows), dim3(256), 0, stream, hidden, (const T*)delta, (const T*)weight, (T*)out, width, eps);
 }
 
+// constant: 1 promises that no kernel still in flight on the stream writes `weight`.
 QF_EXPORT int qf_add_rms_norm(int is_bf16, float* hidden, const void* delta, const void* weight, void* out, int rows,
-                              int width, float eps, cudaStream_t stream) {
-    return is_bf16 ? launch<bf16>(hidden, delta, weight, out, rows, width, eps, stream)
-                   : launch<float>(hidden, delta, weight, out, rows, width, eps, stream);
+                              int width, float eps, int constant, cudaStream_t stream) {
+    return is_bf16 ? launch<bf16>(hidden, delta, weight, out, rows, width, eps, constant, stream)
+                   : launch<float>(hidden, delta, weight, out, rows, width, eps, constant, stream);
 }
 
 template <typename T> __global__ void residual_add_kernel(float* __restrict__ hidden, const T* __restrict__ delta, long long n) {

@@ -34,6 +34,8 @@ struct SkinnyArgs {
     int* err;
     // SWIGLU with gate_limit > 0: the clamped gate min(g, limit) sigmoid(gate_alpha min(g, limit)) (clamp(u, -limit, limit) + 1)
     float gate_limit, gate_alpha;
+    // no kernel in flight writes bias, norm_w and inv_freq: skinny_gemm.cu may read them before it waits for the kernel ahead
+    int constants;
 };
 
 template <int EPI> __device__ __forceinline__ void tile_rows(const SkinnyArgs& a, int tile, int g, int& ra, int& rb) {
@@ -66,7 +68,7 @@ template <int NT> struct EpiloguePre {
     float res[NT][4];
 };
 
-// The constants of it (bias, frequency), which no kernel writes: before the wait for the kernel ahead.
+// The constants of it (bias, frequency): before the wait for the kernel ahead (see `starts_early` in skinny_gemm.cu).
 template <int NT, int EPI>
 __device__ __forceinline__ void skinny_epilogue_constants(const SkinnyArgs& a, int tile, int g, EpiloguePre<NT>& pre) {
     int ra, rb;

@@ -80,9 +80,9 @@ def layer_products(rows: int, hidden: int, inter: int, heads: int, kv_heads: int
     err = torch.zeros(1, dtype=torch.int32, device=device)
     products = [
         ops.FusedProduct(ops.EPI_RESIDUAL, o_w, x=attended, residual=stream),
-        ops.FusedProduct(ops.EPI_SWIGLU, gu_w, hidden=stream, norm_weight=n1, eps=1e-6, out=act),
+        ops.FusedProduct(ops.EPI_SWIGLU, gu_w, hidden=stream, norm_weight=n1, eps=1e-6, out=act, constants=True),
         ops.FusedProduct(ops.EPI_RESIDUAL, down_w, x=act, residual=stream),
-        ops.FusedProduct(ops.EPI_QKV, qkv_w, hidden=stream, norm_weight=n2, eps=1e-6, bias=qkv_b,
+        ops.FusedProduct(ops.EPI_QKV, qkv_w, hidden=stream, norm_weight=n2, eps=1e-6, bias=qkv_b, constants=True,
                          qkv=dict(n_heads=heads, site=pages.args(), inv_freq=inv_freq, rot_dim=head_dim, tok_pos=tok_pos,
                                   tok_seq=tok_seq, slots=slots, q_out=q_out, write_cache=True, err=err)),
     ]
@@ -116,7 +116,7 @@ def unfused(product: ops.FusedProduct, err: torch.Tensor) -> None:
     t = product.tensors
     if "hidden" in t:
         x = torch.empty(t["hidden"].shape, dtype=torch.bfloat16, device=t["hidden"].device)
-        ops.add_rms_norm(t["hidden"], None, t["norm_weight"], t["eps"], x)
+        ops.add_rms_norm(t["hidden"], None, t["norm_weight"], t["eps"], x, constant_weight=True)
     else:
         x = t["x"]
     y = ops.linear(x, product.weight)
@@ -144,7 +144,7 @@ def wide(product: ops.FusedProduct, x: torch.Tensor) -> None:
     """The product by wide_gemm.cu, after the norm kernel where the product normalises its rows."""
     t = product.tensors
     if "hidden" in t:
-        ops.add_rms_norm(t["hidden"], None, t["norm_weight"], t["eps"], x)
+        ops.add_rms_norm(t["hidden"], None, t["norm_weight"], t["eps"], x, constant_weight=True)
     ops.wide_gemm(product.epilogue, product.weight, **wide_tensors(product, x))
 
 
@@ -172,7 +172,7 @@ def measure_products(args) -> None:
                 # the norm kernel, then the many-row tcgen05 product with the gate in its epilogue (one tile per block here)
                 def own(l):
                     t = layers[l][0][i].tensors
-                    ops.add_rms_norm(t["hidden"], None, t["norm_weight"], t["eps"], xs[l])
+                    ops.add_rms_norm(t["hidden"], None, t["norm_weight"], t["eps"], xs[l], constant_weight=True)
                     ops.tc_gemm(ops.TC_SWIGLU, xs[l], layers[l][0][i].weight, t["out"], err)
                 line += f"  tc_gemm {graph_time_us(lambda: [own(l) for l in range(repeat)], repeat):7.2f} us"
             print(line, flush=True)

@@ -167,8 +167,10 @@ def gather_rows_norm(hidden: torch.Tensor, delta: Optional[torch.Tensor], rows: 
 
 
 def add_rms_norm(hidden: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor, eps: float,
-                 out: torch.Tensor) -> None:
-    """hidden += delta (if given); out = rmsnorm(hidden) * weight. hidden float32 [R, W]; out, weight, delta share a dtype."""
+                 out: torch.Tensor, constant_weight: bool = False) -> None:
+    """hidden += delta (if given); out = rmsnorm(hidden) * weight. hidden float32 [R, W]; out, weight, delta share a dtype.
+    `constant_weight` promises that no kernel still in flight on the stream writes `weight` (a bound model's weights): it is then
+    read while the kernel ahead ends."""
     _dev("hidden", hidden, torch.float32)
     _dev("weight", weight)
     _dev("out", out, weight.dtype)
@@ -180,7 +182,8 @@ def add_rms_norm(hidden: torch.Tensor, delta: Optional[torch.Tensor], weight: to
         if delta.shape != hidden.shape:
             raise KernelError("add_rms_norm: delta and hidden differ in shape")
     _check(library("norm").qf_add_rms_norm(_I(_is_bf16(weight.dtype)), _ptr(hidden), _ptr(delta), _ptr(weight),
-                                           _ptr(out), _I(rows), _I(width), _F(eps), _stream()), "add_rms_norm")
+                                           _ptr(out), _I(rows), _I(width), _F(eps), _I(int(bool(constant_weight))), _stream()),
+           "add_rms_norm")
 
 
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> None:
@@ -722,6 +725,7 @@ class _SkinnyArgs(ctypes.Structure):
         ("n_heads", _I), ("kv_heads", _I), ("head_dim", _I), ("rot_dim", _I), ("write_cache", _I),
         ("inv_freq", _P), ("tok_pos", _P), ("tok_seq", _P), ("slots", _P), ("q_out", _P), ("kv_base", _P),
         ("table", _P), ("page_elems", _LL), ("table_stride", _I), ("err", _P), ("gate_limit", _F), ("gate_alpha", _F),
+        ("constants", _I),
     ]
 
 
@@ -777,11 +781,12 @@ def _skinny_args(epilogue: int, weight: torch.Tensor, *, x: Optional[torch.Tenso
                  hidden: Optional[torch.Tensor] = None, norm_weight: Optional[torch.Tensor] = None, eps: float = 0.0,
                  bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
                  residual: Optional[torch.Tensor] = None, qkv: Optional[dict] = None,
-                 err: Optional[torch.Tensor] = None, clamp=None):
+                 err: Optional[torch.Tensor] = None, clamp=None, constants: bool = False):
     """Checks one fused product's tensors and fills the kernels' argument block; returns (block, norm flag).
     clamp = (limit, alpha) with EPI_SWIGLU: the clamped gate in the silu gate's place (see `clamped_glu`)."""
     _dev("weight", weight, torch.bfloat16, contiguous=False)
     a = _SkinnyArgs()
+    a.constants = int(bool(constants))
     a.w, a.n, a.k, a.ldw = weight.data_ptr(), weight.shape[0], weight.shape[1], weight.stride(0)
     if bias is not None:
         _dev("bias", bias, torch.bfloat16)
@@ -841,6 +846,9 @@ def skinny_gemm(epilogue: int, weight: torch.Tensor, **tensors) -> None:
     """One fused product for up to 16 token rows. Input rows are either `x` [m, K] bf16, or the float32 residual
     stream `hidden` [m, K] normalised on the fly with `norm_weight`, `eps`. Keywords: x | hidden, norm_weight, eps;
     bias; out (PLAIN, SWIGLU); residual (RESIDUAL); err; see csrc/skinny_gemm.cu for the epilogues.
+    A product of `x` alone reads `weight` while the kernel ahead on the stream ends: no kernel in flight may be writing it. With a norm, a
+    bias or a rotation the launch waits for everything ahead of it, unless constants=True promises that no kernel in flight writes
+    weight, norm_weight, bias, inv_freq, positions, slots or page tables (a bound model's step).
     qkv (EPI_QKV): dict(n_heads, site=KvSiteArgs, inv_freq, rot_dim, tok_pos, tok_seq, slots, q_out, write_cache, err)."""
     a, norm = _skinny_args(epilogue, weight, **tensors)
     code = library("skinny_gemm").qf_skinny_gemm(_I(epilogue), _I(int(norm)), ctypes.byref(a), _stream())

@@ -458,12 +458,12 @@ class GqaAttention(Mixer):
             if delta is not None:
                 ops.residual_add(hidden, delta)
             ops.skinny_gemm(ops.EPI_QKV, self.qkv_weight, hidden=hidden, norm_weight=rms[0], eps=rms[1],
-                            bias=self.qkv_bias_t,
+                            bias=self.qkv_bias_t, constants=True,
                             qkv=dict(n_heads=self.n_heads, site=args, inv_freq=inv_freq, rot_dim=rot_dim, tok_pos=ctx.tok_pos,
                                      tok_seq=ctx.tok_seq, slots=ctx.slots, q_out=q, write_cache=writes_cache, err=ctx.err))
         else:
             x = torch.empty(hidden.shape, dtype=torch.bfloat16, device=hidden.device)
-            ops.add_rms_norm(hidden, delta, rms[0], rms[1], x)   # the norm kernel adds the pending delta on its way
+            ops.add_rms_norm(hidden, delta, rms[0], rms[1], x, constant_weight=True)   # the norm kernel adds the pending delta on its way
             if qkv_way == "wide":
                 ops.wide_gemm(ops.EPI_QKV, self.qkv_weight, x=x, bias=self.qkv_bias_t,
                               qkv=dict(n_heads=self.n_heads, site=args, inv_freq=inv_freq, rot_dim=rot_dim, tok_pos=ctx.tok_pos,

@@ -68,10 +68,11 @@ class SwiGlu(FeedForward):
         if gate_up == "skinny":
             if delta is not None:
                 ops.residual_add(hidden, delta)
-            ops.skinny_gemm(ops.EPI_SWIGLU, self.gate_up_weight, hidden=hidden, norm_weight=rms[0], eps=rms[1], out=act)
+            ops.skinny_gemm(ops.EPI_SWIGLU, self.gate_up_weight, hidden=hidden, norm_weight=rms[0], eps=rms[1], out=act,
+                            constants=True)
         else:
             x = torch.empty(hidden.shape, dtype=torch.bfloat16, device=hidden.device)
-            ops.add_rms_norm(hidden, delta, rms[0], rms[1], x)   # the norm kernel adds the pending delta on its way
+            ops.add_rms_norm(hidden, delta, rms[0], rms[1], x, constant_weight=True)   # the norm kernel adds the pending delta on its way
             if gate_up == "wide":
                 ops.wide_gemm(ops.EPI_SWIGLU, self.gate_up_weight, x=x, out=act, err=ctx.err)
             else:
