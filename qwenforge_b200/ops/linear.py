@@ -85,10 +85,14 @@ def linear_rows(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch
 
 def tail_rides(x: torch.Tensor, joint: torch.Tensor, n: int) -> bool:
     """Whether x @ joint.T runs as one launch whose first n columns are bfloat16 and whose others stay float32 (`kernels.tc_gemm_tail`), and
-    is the faster way: more than 64 rows. Measured for 14 to 32 float32 columns, microseconds, two library products / one launch: n 2,688, K
-    896 10.6 / 7.9 for 128 rows, 18.8 / 12.9 for 2,048; 6,144, 2,048 14.0 / 12.9 for 65, 44.6 / 37.6 for 2,048, 107.5 / 107.9 for 6,144; 8,448,
-    2,048 104.9 / 99.8 for 4,206 (17 rows: 14.3 / 16.9)."""
-    return (x.is_cuda and x.dtype == torch.bfloat16 and joint.dtype == torch.bfloat16 and x.shape[0] > kernels.WIDE_MAX_ROWS and n % 8 == 0
+    is the faster way: more than 64 rows, a K of up to 2,048 and columns enough, twice K, or more than 1,024 rows. Measured for 8 to 64
+    float32 columns with the norm ahead, microseconds, two library products / one launch: n 2,688, K 896 14.9 / 9.9 for 100 rows, 21.7 / 15.4 for
+    2,048; 6,144, 2,048 15.0 / 14.6 for 65, 47.5 / 42.7 for 2,048; 8,448, 2,048 22.8 / 20.2 for 512, 109.8 / 108.4 for 4,096 (17 rows alone: 14.3 /
+    16.9). Beyond, the library cuts K among blocks or has the better rate: 12,288, 4,096 37.2 / 46.6 for 300, 93.5 / 101.3 for 1,200 (301.8 /
+    286.2 for 4,096); 768, 2,048 11.6 / 13.0 for 65, 12.7 / 13.9 for 512, 18.8 / 17.4 for 2,048; 1,536, 1,536 12.0 / 12.6 for 512, 15.8 / 14.3 for 1,200."""
+    m, k = x.shape
+    return (x.is_cuda and x.dtype == torch.bfloat16 and joint.dtype == torch.bfloat16 and m > kernels.WIDE_MAX_ROWS and n % 8 == 0
+            and k <= 2048 and (n >= 2 * k or m > 1024)
             and kernels.tc_gemm_takes(x, joint))
 
 

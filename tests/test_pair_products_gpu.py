@@ -133,3 +133,12 @@ def test_where_the_qkv_product_on_pairs_pays():
     assert not pays(900, 1024, 2048, 64) and pays(900, 1152, 1536, 64) and not pays(2048, 512, 3072, 64) and pays(4096, 512, 3072, 64)
     assert pays(7358, 2560, 2048, 128) and not pays(2048, 2560, 2048, 128) and not pays(512, 2560, 2048, 128) and pays(513, 2560, 2048, 128)
     assert not pays(1300, 1280, 4096, 128) and pays(3000, 1280, 4096, 128) and not pays(64, 2304, 2048, 64) and pays(900, 2304, 2048, 64)
+
+
+def test_where_the_float32_columns_ride():
+    """Both sides of the rule's lines: rows, a long K, columns that are few beside K."""
+    from qwenforge_b200 import ops
+    rides = lambda m, n, extra, k: ops.tail_rides(torch.empty(m, k, dtype=torch.bfloat16, device=DEV), torch.empty(n + extra, k, dtype=torch.bfloat16, device=DEV), n)
+    assert rides(65, 2688, 14, 896) and rides(2048, 2688, 14, 896) and rides(65, 6144, 32, 2048) and rides(4206, 8448, 32, 2048)
+    assert not rides(64, 2688, 14, 896) and not rides(300, 12288, 64, 4096) and not rides(65, 768, 8, 2048) and not rides(512, 1536, 8, 1536)
+    assert not rides(1024, 768, 8, 2048) and rides(1025, 768, 8, 2048) and not rides(300, 2692, 14, 896)
