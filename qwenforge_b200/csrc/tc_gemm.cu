@@ -777,22 +777,19 @@ QF_EXPORT int qf_tc_gemm(int epilogue, const void* a, int lda, const void* w, in
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0 || k % 8 || lda % 8 || ldw % 8 || ldo % 8) return (int)cudaErrorInvalidValue;
     if (((uintptr_t)a | (uintptr_t)w | (uintptr_t)out) % 16) return (int)cudaErrorInvalidValue;
-    CUtensorMap map_a, map_b;
-    if (!qf_make_map_bf16(&map_a, a, m, k, lda, TC_BM) || !qf_make_map_bf16(&map_b, w, n, k, ldw, 64)) return (int)cudaErrorNotSupported;
+    if (epilogue != TC_PLAIN && (epilogue != TC_SWIGLU || n % 2 || (n / 2) % 8)) return (int)cudaErrorInvalidValue;
+    CUtensorMap map_a, map_b;         // (a launch on pairs makes the weights' map itself, with its own boxes)
+    if (!qf_make_map_bf16(&map_a, a, m, k, lda, TC_BM)) return (int)cudaErrorNotSupported;
     // wide tiles when there are enough of them to fill the SMs; narrow ones otherwise
-    const int out_cols = epilogue == TC_SWIGLU ? n / 2 : n;
-    const int m_tiles = (m + TC_BM - 1) / TC_BM;
-    if (epilogue == TC_SWIGLU) {
-        if (n % 2 || (n / 2) % 8) return (int)cudaErrorInvalidValue;
-        const int inter = n / 2;
-        const bool wide = (long long)m_tiles * ((inter + 127) / 128) >= qf_sm_count();
-        if (wide && g_persistent) return launch_persistent<TC_SWIGLU>(map_a, w, n, ldw, out, m, inter, k, inter, ldo, err, stream);
+    const int inter = n / 2, m_tiles = (m + TC_BM - 1) / TC_BM;
+    const bool wide = (long long)m_tiles * (epilogue == TC_SWIGLU ? (inter + 127) / 128 : (n + 255) / 256) >= qf_sm_count();
+    if (wide && g_persistent)
+        return epilogue == TC_SWIGLU ? launch_persistent<TC_SWIGLU>(map_a, w, n, ldw, out, m, inter, k, inter, ldo, err, stream)
+                                     : launch_persistent<TC_PLAIN>(map_a, w, n, ldw, out, m, n, k, 0, ldo, err, stream);
+    if (!qf_make_map_bf16(&map_b, w, n, k, ldw, 64)) return (int)cudaErrorNotSupported;
+    if (epilogue == TC_SWIGLU)
         return wide ? launch_tc<TC_SWIGLU, 256>(map_a, map_b, out, m, inter, k, inter, ldo, err, dim3((inter + 127) / 128, m_tiles), stream)
                     : launch_tc<TC_SWIGLU, 128>(map_a, map_b, out, m, inter, k, inter, ldo, err, dim3((inter + 63) / 64, m_tiles), stream);
-    }
-    if (epilogue != TC_PLAIN) return (int)cudaErrorInvalidValue;
-    const bool wide = (long long)m_tiles * ((out_cols + 255) / 256) >= qf_sm_count();
-    if (wide && g_persistent) return launch_persistent<TC_PLAIN>(map_a, w, n, ldw, out, m, n, k, 0, ldo, err, stream);
     return wide ? launch_tc<TC_PLAIN, 256>(map_a, map_b, out, m, n, k, 0, ldo, err, dim3((n + 255) / 256, m_tiles), stream)
                 : launch_tc<TC_PLAIN, 128>(map_a, map_b, out, m, n, k, 0, ldo, err, dim3((n + 127) / 128, m_tiles), stream);
 }
