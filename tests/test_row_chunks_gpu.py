@@ -76,3 +76,53 @@ def test_what_the_chunked_form_takes():
     assert takes(q[:, :64])
     assert not takes(q[:, :64].float()) and not takes(q[:, 1:65]) and not takes(q[:, :64], dim=128) and not takes(q[:, :64], vdim=96)
     assert not takes(q[:, :64], longest=16) and not takes(q[:, :64], vdim=576)
+
+
+# Where the blocks fill the SMs a block of outputs takes two tiles of 64 columns of v; a call on 64 columns takes one.
+@pytest.mark.parametrize("heads,vdim,lengths,form,odd", [
+    (40, 128, (300, 1, 129), "after", None), (40, 128, (300, 1, 129), "bonus", None), (40, 128, (300, 1, 129), "sigmoid_root", None),
+    (20, 256, (300, 1, 129), "double_exp", None), (74, 128, (63, 64, 65), "after", float("inf")), (74, 128, (63, 64, 65), "bonus", float("nan"))])
+def test_two_tiles_of_v_a_block(heads, vdim, lengths, form, odd, monkeypatch):
+    from qwenforge_b200 import ops
+    from qwenforge_b200.ops import kernels
+    g = torch.Generator(device=DEV).manual_seed(heads + vdim)
+    dim, slots, cu, s_off = 64, [3, -1, 1], [0], 4
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    n, records = cu[-1], cu[-1] // 64 + len(lengths)
+    assert records * heads * (vdim // 128) >= 2 * ops.sm_count(torch.device(DEV))
+    q, k, v = (torch.randn(n, heads * c, generator=g, device=DEV).bfloat16() for c in (dim, dim, vdim))
+    bad = lengths[0] - 10                                      # a token of the first sequence, and a column of the second tile of head 1
+    if odd is not None:
+        v[bad, vdim + 70] = odd
+    start = torch.randn(5, s_off + heads * dim * vdim, generator=g, device=DEV)
+    bonus = torch.randn(heads, dim, generator=g, device=DEV) if form in ("bonus", "double_exp") else None
+    if form in ("after", "bonus"):
+        decay, decay_from = torch.exp(-torch.exp(3 * torch.randn(n, heads * dim, generator=g, device=DEV) - 3)), None
+    else:
+        decay, decay_from = torch.randn(n, heads * dim, generator=g, device=DEV), (form, torch.randn(heads * dim, generator=g, device=DEV), 8.0)
+    more = dict(bonus=bonus, decay_from=decay_from)
+
+    def whole():
+        state, y = start.clone(), torch.full((n, heads * vdim), 7.0, device=DEV)
+        ops.row_chunks(q, k, v, decay, ints(cu), ints(slots), max(lengths), state, s_off, heads, dim, vdim, 0.3, y, **more)
+        return state, y
+    state, y = whole()
+    tiles = start[:, s_off:].view(5, heads, dim, vdim // 64, 64)
+    bits = lambda t: t.contiguous().view(torch.int32)
+    for at in range(vdim // 64):
+        part, out = tiles[:, :, :, at].reshape(5, -1).contiguous(), torch.empty(n, heads * 64, device=DEV)
+        ops.row_chunks(q, k, v.view(n, heads, -1, 64)[:, :, at].reshape(n, -1).contiguous(), decay, ints(cu), ints(slots), max(lengths), part, 0, heads,
+                       dim, 64, 0.3, out, **more)
+        assert torch.equal(bits(out), bits(y.view(n, heads, -1, 64)[:, :, at].reshape(n, -1)))
+        assert torch.equal(bits(part), bits(state[:, s_off:].view(5, heads, dim, -1, 64)[:, :, :, at].reshape(5, -1)))
+    if odd is not None:
+        hit = ~torch.isfinite(y.view(n, heads, vdim))
+        assert bool(hit[bad:lengths[0], 1, 70].any()) and not bool(hit[:bad].any()) and not bool(hit[lengths[0]:].any())
+        hit[:, 1, 70] = False
+        assert not bool(hit.any())
+    # in portions of two chunks of every sequence a block takes one tile again: the same bits
+    assert min(2, -(-max(lengths) // 64)) * len(lengths) * heads * (vdim // 128) < 2 * ops.sm_count(torch.device(DEV)) or heads == 74
+    monkeypatch.setattr(kernels, "_chunk_portions", lambda n, n_seqs, chunk, floats: (2 * n_seqs, 2))
+    cut_state, cut_y = whole()
+    assert torch.equal(bits(cut_y), bits(y)) and torch.equal(bits(cut_state), bits(state))
