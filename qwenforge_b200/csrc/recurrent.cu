@@ -15,8 +15,8 @@
 
 // 1 / d for d >= 1 (infinity and NaN as the division gives them) and z / d with it, by Newton's step and Markstein's correction of the
 // quotient ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): the remainders are exact in a fused
-// multiply-add, so both come out rounded to the nearest as the division rounds them, without the division's branches. Compared
-// with `/` on every d from 1 to 2^128 and on 2^32 pairs: the same bits, below 2^-126 (1 / d for d beyond 2^126) but for the last.
+// multiply-add, so both come out rounded to the nearest as the division rounds them, without the division's branches. Tested on every
+// z and its d = 1 + e^-z: the bits of `/`, below 2^-126 but for the last; and on every bfloat16 gate: the norm that `/` leaves.
 struct Over {
     float d, r;
     __device__ __forceinline__ explicit Over(float d_) : d(d_) {

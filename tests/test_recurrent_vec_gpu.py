@@ -115,3 +115,47 @@ def test_silu_behind_the_convolution():
     assert bool(((got - want).abs()[fine] <= 4 * 2.0 ** -23 * want.abs()[fine]).all())
     row = out[-1, :odd.numel()].tolist()
     assert row[0] == row[1] == 0 and row[2] == 100 and abs(row[3]) < 1e-35 and abs(row[4]) < 1e-35 and row[5] == float("inf") and row[6] != row[6]
+
+
+def test_silu_has_the_bits_of_the_division():
+    """Every float32 number through the convolution's silu, against 1 + e^-z and z / that as CUDA rounds them: the same bits; results
+    below 2^-126 are one unit (2^-149) apart at most. In runs of tokens, and a sample token by token."""
+    from qwenforge_b200 import ops
+    n = c = 8192
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    cu, seq, state = ints([0, n]), torch.zeros(n, dtype=torch.int32, device=DEV), torch.zeros(1, c, device=DEV)
+    last = torch.tensor([[0.0, 1.0]], device=DEV).repeat(c, 1)                # only the newest input counts
+    offsets = torch.arange(n * c, dtype=torch.int32, device=DEV)
+    wrong = torch.zeros(2, dtype=torch.int64, device=DEV)
+    out = torch.empty(n, c, device=DEV)
+    for chunk in range(64):
+        x = (offsets + (chunk * n * c - (1 << 31))).view(torch.float32).view(n, c)
+        x = torch.where(torch.isfinite(x), x, torch.zeros_like(x)) + 0.0   # (a number that is not finite would reach the next token)
+        want = x / (torch.exp(-x) + 1.0)
+        for taps in ((last, last[:, 1:].contiguous()) if chunk % 16 == 0 else (last,)):
+            ops.causal_conv_silu(x, taps, None, cu, seq, ints([-1]), state, 0, out)
+            small = want.abs() < 2.0 ** -126
+            wrong[0] += (~small & (out != want)).sum()
+            wrong[1] += (small & ((out - want).abs() > 2.0 ** -149)).sum()
+    assert wrong.tolist() == [0, 0]
+
+
+@pytest.mark.parametrize("gate,first", [("sigmoid", False), ("silu", False), ("silu", True)])
+def test_gates_of_the_norm_have_the_bits_of_the_division(gate, first):
+    """Every bfloat16 gate, in pieces of eight columns and (rows that no 16-byte load can address) number by number with `/`."""
+    from qwenforge_b200 import ops
+    values = torch.arange(-32768, 32768, dtype=torch.int32, device=DEV).short().view(torch.bfloat16)
+    values = values[torch.isfinite(values) & (values.abs() < 1e18)].repeat_interleave(8).view(-1, 8)   # (a row per gate: `first` squares it)
+    n = values.shape[0]
+    off = torch.zeros(n, 16, dtype=torch.bfloat16, device=DEV)
+    off[:, 1:9] = values
+    g = torch.Generator(device=DEV).manual_seed(1)
+    # one number a row, so that the sum of squares is the same in any order
+    y, weight = torch.zeros(n, 8, device=DEV), torch.randn(8, generator=g, device=DEV).bfloat16()
+    y.scatter_(1, torch.randint(0, 8, (n, 1), generator=g, device=DEV), torch.randn(n, 1, generator=g, device=DEV))
+    results = []
+    for gates in (values, off[:, 1:9]):
+        out = torch.empty(n, 8, dtype=torch.bfloat16, device=DEV)
+        ops.gated_group_norm(y, gates, weight, 1e-5, out, 1, 1, gate, first)
+        results.append(out)
+    assert torch.equal(*results) and bool(torch.isfinite(results[0]).all())
