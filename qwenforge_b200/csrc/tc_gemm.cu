@@ -346,8 +346,8 @@ __device__ __forceinline__ void quadrant_sync(int quad) { asm volatile("bar.sync
 
 // 16 neighbouring rotation pairs of a head in this thread's row of the accumulator (first halves from column `lo` of its lane, second
 // halves from `hi`), with the bias of both, rotated by cs = (cos, sin) where `rotate`, as 16-byte pieces of the row. The sums are rounded
-// to bfloat16 first, as those of a product that is stored are: a row's queries, keys and values are the same whichever way the
-// sizes of its step choose.
+// to bfloat16 first, as those of a product that is stored are: from the same sums come the queries, keys and values of such a product with
+// the rotation kernel behind it, bit for bit (the library's product may add K in another order and so give other sums).
 __device__ __forceinline__ void rotated_pairs(uint32_t lo, uint32_t hi, const bf16* bias_lo, const bf16* bias_hi, const float2* cs,
                                               bool rotate, uint4 (&out_lo)[2], uint4 (&out_hi)[2]) {
     uint32_t x[16], y[16];

@@ -88,6 +88,34 @@ def test_queries_keys_and_values_of_pairs(m, heads, kv_heads, dim, k, rotated, b
     assert torch.equal(before, storage) and torch.equal(again, q) and int(err) == ops.ERR_NO_PAGE
 
 
+@pytest.mark.parametrize("m,heads,kv_heads,dim,rotated,biased", [(301, 14, 2, 64, True, True), (2047, 14, 2, 64, True, False), (600, 16, 2, 128, True, True),
+                                                                 (130, 3, 1, 128, False, True)])
+def test_the_bits_of_product_and_rotation(m, heads, kv_heads, dim, rotated, biased):
+    """Whole numbers, whose sums are exact in any order: queries, keys and values are those of the stored product with the rotation
+    kernel behind it, bit for bit, at positions far out as well."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(m)
+    n, k = (heads + 2 * kv_heads) * dim, 264
+    x, w = (torch.randint(-9, 10, shape, generator=g, device=DEV).bfloat16() for shape in ((m, k), (n, k)))
+    bias = torch.randn(n, generator=g, device=DEV).bfloat16() if biased else None
+    inv = 1e6 ** (-torch.arange(0, dim, 2, device=DEV).float() / dim) if rotated else None
+    first = 40000
+    pages = -(-(first + m) // 64)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    seq, pos, slots, err = ints([0] * m), ints(list(range(first, first + m))), ints([0]), ints([0])
+    table = torch.full((1, pages), -1, dtype=torch.int32)
+    table[0, first // 64:] = torch.arange(pages - first // 64)
+    results = []
+    for own in (True, False):
+        storage = torch.zeros(pages - first // 64, 2, kv_heads, 64, dim, dtype=torch.bfloat16, device=DEV)
+        site, q = ops.KvSiteArgs(storage, table.to(DEV), kv_heads, dim), torch.empty(m, heads * dim, dtype=torch.bfloat16, device=DEV)
+        if own:
+            ops.qkv_product(x, w, bias, inv, seq, pos, slots, heads, q, site, True, err)
+        else:
+            ops.rope_cache_write(ops.linear(x, w), seq, pos, slots, inv, dim if rotated else 0, heads, q, site, True, err, bias=bias)
+        results.append((q, storage))
+    assert int(err) == 0 and all(torch.equal(a, b) for a, b in zip(*results))
+
 @pytest.mark.parametrize("m,n,extra,k", [(65, 2688, 14, 896), (257, 264, 1, 72), (300, 248, 32, 8), (2049, 2560, 2, 136), (700, 1536, 40, 640)])
 def test_columns_that_stay_float32(m, n, extra, k):
     """The tail of a product's columns: inside the last tile, across its border, alone in a tile of its own."""
