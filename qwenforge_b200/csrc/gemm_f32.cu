@@ -220,6 +220,27 @@ gemm_f32_few_rows_kernel(const float* __restrict__ A, const float* __restrict__ 
     }
 }
 
+// The tile with which the busiest SM is done first: a first wait and a time per tile, measured at K = 896 in microseconds (1, 4 and 18
+// tiles per SM of 64 x 64 33, 92 and 380, of 32 x 64 24, 65 and 258; 1, 5 and 9 of 128 x 128 89, 385 and 683; 1, 6 and 12 of 96 x 128
+// 72, 339 and 662; 1, 2 and 12 of 96 x 64 47, 74 and 382). Never the fastest by more than a twentieth: 64 x 128 and 64 x 256 with two
+// or four warps, 32 x 64 with two warps, 128 x 64. (With K a tile's time grows and its wait does not: the waits, which count here as at
+// K = 896, decide between tiles whose rounds take nearly the same time.)
+static const struct { int bm, bn; float wait, each; } f32_tiles[] = {{96, 128, 18.f, 53.7f}, {128, 128, 13.5f, 74.5f}, {96, 64, 15.f, 30.6f},
+                                                                     {64, 64, 8.5f, 20.8f}, {32, 64, 8.f, 14.3f}};
+static int best_tile(int M, int N) {
+    const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
+    int best = 0;
+    float least = 0.f;
+    for (int i = 0; i < 5; ++i) {
+        const long long count = (long long)((M + f32_tiles[i].bm - 1) / f32_tiles[i].bm) * ((N + f32_tiles[i].bn - 1) / f32_tiles[i].bn);
+        const float time = f32_tiles[i].wait + (float)((count + sms - 1) / sms) * f32_tiles[i].each;
+        if (i == 0 || time < least) best = i, least = time;
+    }
+    return best;
+}
+// Which tile a product of more than 16 rows takes: 1,000 x its rows + its columns.
+QF_EXPORT int qf_gemm_f32_tile(int M, int N) { return f32_tiles[best_tile(M, N)].bm * 1000 + f32_tiles[best_tile(M, N)].bn; }
+
 QF_EXPORT int qf_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
                           int ldw, int ldc, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
@@ -229,21 +250,8 @@ QF_EXPORT int qf_gemm_f32(const float* A, const float* W, const float* bias, flo
         return (int)cudaGetLastError();
     }
     const int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-    // The tile with which the busiest SM is done first: a first wait and a time per tile, measured at K = 896 in microseconds (1, 4 and 18
-    // tiles per SM of 64 x 64 33, 92 and 380, of 32 x 64 24, 65 and 258; 1, 5 and 9 of 128 x 128 89, 385 and 683; 1, 6 and 12 of 96 x 128
-    // 72, 339 and 662; 1, 2 and 12 of 96 x 64 47, 74 and 382). Never the fastest by more than a twentieth: 64 x 128 and 64 x 256 with two
-    // or four warps, 32 x 64 with two warps, 128 x 64.
-    struct { int bm, bn; float wait, each; } const tiles[] = {{96, 128, 18.f, 53.7f}, {128, 128, 13.5f, 74.5f}, {96, 64, 15.f, 30.6f},
-                                                              {64, 64, 8.5f, 20.8f}, {32, 64, 8.f, 14.3f}};
-    const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
-    int best = 0;
-    float least = 0.f;
-    for (int i = 0; i < 5; ++i) {
-        const long long count = (long long)((M + tiles[i].bm - 1) / tiles[i].bm) * ((N + tiles[i].bn - 1) / tiles[i].bn);
-        const float time = tiles[i].wait + (float)((count + sms - 1) / sms) * tiles[i].each;
-        if (i == 0 || time < least) best = i, least = time;
-    }
-    const dim3 grid((N + tiles[best].bn - 1) / tiles[best].bn, (M + tiles[best].bm - 1) / tiles[best].bm);
+    const int best = best_tile(M, N);
+    const dim3 grid((N + f32_tiles[best].bn - 1) / f32_tiles[best].bn, (M + f32_tiles[best].bm - 1) / f32_tiles[best].bm);
 #define QF_F32(TM, TN, BK) gemm_f32_kernel<TM, TN, 2, 2, BK><<<grid, 128, 0, stream>>>(A, W, bias, C, M, N, K, lda, ldw, ldc, vec)
     if (best == 0) QF_F32(12, 8, 16);
     else if (best == 1) QF_F32(16, 8, 16);

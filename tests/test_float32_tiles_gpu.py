@@ -24,6 +24,27 @@ def test_products_keep_the_order_of_a_single_chain(m, n, k):
     assert torch.equal(out, rows)
 
 
+# every size of tile, with ragged last tiles both ways, a K of no whole piece of 16 and one below it
+@pytest.mark.parametrize("m,n,k,tile", [(1031, 4865, 33, 96128), (1031, 9728, 20, 96128), (1057, 22016, 17, 96128), (300, 6200, 48, 128128), (700, 1025, 16, 96064),
+                                        (65, 19100, 35, 96064), (257, 5000, 9, 64064), (70, 130, 40, 32064)])
+def test_every_tile_keeps_the_order_of_a_single_chain(m, n, k, tile):
+    import ctypes
+    from qwenforge_b200 import ops
+    from qwenforge_b200.csrc import library
+    assert library("gemm_f32").qf_gemm_f32_tile(ctypes.c_int(m), ctypes.c_int(n)) == tile
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    x, w, b = torch.randn(m, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV), torch.randn(n, generator=g, device=DEV)
+    out, rows = torch.full((m + 1, n), 7.0, device=DEV), torch.empty(m, n, device=DEV)
+    ops.gemm_f32(x, w, b, out[:m])
+    for at in range(0, m, 16):
+        ops.gemm_f32(x[at:at + 16], w, b, rows[at:at + 16])
+    assert torch.equal(out[:m], rows) and bool((out[m] == 7).all())
+    wide = torch.zeros(m, k + 3, device=DEV)      # rows that no 16-byte load can address
+    wide[:, 1:k + 1] = x
+    ops.gemm_f32(wide[:, 1:k + 1], w, b, out[:m])
+    assert torch.equal(out[:m], rows)
+
+
 @pytest.mark.parametrize("dim,heads,kv_heads,window", [(64, 14, 2, 0), (128, 4, 4, 0), (64, 4, 1, 70), (128, 2, 1, 1)])
 def test_attention_tiles(dim, heads, kv_heads, window):
     from qwenforge_b200 import ops
