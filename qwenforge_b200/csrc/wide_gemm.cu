@@ -70,7 +70,7 @@ __device__ __forceinline__ void stamp(const WideGeometry& geo, int slot) {
 }
 
 __device__ __forceinline__ void row_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(WG_ROW_THREADS) : "memory"); }
-__device__ __forceinline__ float wide_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+__device__ __forceinline__ float wide_silu(float x) { return x / (1.0f + expf(-x)); }   // as the other ways of this product
 
 template <int EPI>
 __global__ void __launch_bounds__(WG_THREADS, 1)

@@ -928,16 +928,22 @@ def qkv_product_way(m: int, weight: torch.Tensor, n_heads: int, kv_heads: int, h
 
 def gate_product_way(m: int, weight: torch.Tensor) -> str:
     """How `m` token rows (64 at most) are normalised, multiplied by a [gate | up] weight and gated: "skinny" (the mma.sync streamer with
-    all of it inside) where it takes the shape and pays (`skinny_gemm_pays`), else "wide" (a norm kernel, then the tcgen05 streamer with
-    the gate in its epilogue) for weights of 100 MB and more, else "unfused" (norm, library product, gate kernel). Measured as norm, gate/up
-    and down together over weights that the L2 does not hold, microseconds, the other way / "wide": 272 MB (Qwen2.5-7B's) 1 row 76.9 / 69.5,
-    16 rows 79.5 / 72.4, 64 rows 85.2 / 78.3; 90 MB (3B's) 1 row 32.3 / 33.1, 8 rows 34.8 / 33.8, 16 rows 35.8 / 35.0; 17 MB (0.5B's) 8 rows
-    10.4 / 13.2, 16 rows 15.1 / 14.4. "wide" would be ahead by 2 to 5 percent from 4 rows of 32 MB and 9 rows of 16 MB on too, but its gate uses the
-    hardware's exponential and division (an error of 2^-20) where the other two ways use float32's own: that band stays with them."""
+    all of it inside), "wide" (a norm kernel, then the tcgen05 streamer with the gate in its epilogue) or "unfused" (norm, library product,
+    gate kernel). Where the mma.sync streamer pays (`skinny_gemm_pays`) "wide" takes its place from 9 rows of 16 MB and 4 rows of 32 MB on; where
+    it does not, "wide" takes weights of 100 MB and more. Measured as norm, gate/up and down together over weights that the L2 does not
+    hold, microseconds, skinny / wide / unfused: 17 MB (Qwen2.5-0.5B's) 8 rows 11.8 / 13.1 / 13.4, 12 rows 14.9 / 15.0 / 15.9 (a whole step of 12
+    rows 888 / 873 / -), 24 rows - / 16.0 / 16.4; 57 MB 1 row 23.1 / 23.8 / 25.3, 4 rows 24.8 / 24.5 / 25.3, 9 rows 27.4 / 24.7 / 25.7, 24 rows
+    - / 25.5 / 25.8; 90 MB (3B's) 1 row 32.0 / 31.4 / 33.5, 4 rows 34.4 / 32.2 / 34.3, 8 rows 34.2 / 32.6 / 34.7, 16 rows 37.4 / 33.9 / 34.5, 48
+    rows - / 35.1 / 38.9; 272 MB (7B's) 1 row 81.0 / 67.5 / 74.1, 16 rows 87.7 / 70.9 / 77.2, 64 rows - / 76.8 / 83.7. Errors against 64 bits of a
+    step's gated rows: 0.0028 to 0.0031 / 0.0028 to 0.0030 / 0.0038 to 0.0041 (the stored sums are rounded to eight bits).
+    Below 100 MB the library product keeps the steps of 17 rows and more, and of 9 from 64 MB on: "wide" would be ahead there too, but it
+    adds K in another order, and their outputs (0.8 percent of the logits of 16 sequences at 3B sizes) stay the ones that they were."""
     size = weight.numel() * weight.element_size()
-    if m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_SWIGLU, True) and skinny_gemm_pays(m, weight):
-        return "skinny"
-    return "wide" if size >= 100e6 and wide_gemm_takes_rows(EPI_SWIGLU, m, weight) else "unfused"
+    skinny = m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_SWIGLU, True) and skinny_gemm_pays(m, weight)
+    least = 100e6 if not skinny or m < 4 else 32e6 if m < 9 else 16e6
+    if size >= least and wide_gemm_takes_rows(EPI_SWIGLU, m, weight):
+        return "wide"
+    return "skinny" if skinny else "unfused"
 
 
 def residual_product_way(m: int, weight: torch.Tensor) -> str:
