@@ -951,11 +951,11 @@ def residual_product_way(m: int, weight: torch.Tensor) -> str:
     measurement on a B200 (`python -m qwenforge_b200.measure products`, Qwen2.5 0.5B / 3B / 7B sizes).
     Up to 16 rows the choice is between the two kernels that add in place: "skinny" (the mma.sync streamer) up to 8 rows
     while the weight is under 20 MB (0.5B: 3.0 and 4.8 microseconds against 3.4 and 5.5 on the tcgen05 streamer; 7B's
-    26 MB output projection: 9.0 against 8.0), "wide" (the tcgen05 streamer) beyond (16 rows: 3.4 / 5.5 against 4.1 /
-    6.6 at 0.5B, 14.9 against 16.2 at 3B's down product, 25.8 against 50 at 7B's).
+    26 MB output projection: 9.2 against 8.5), "wide" (the tcgen05 streamer) beyond (16 rows: 3.6 / 4.9 against 4.1 /
+    6.0 at 0.5B, 13.4 against 16.3 at 3B's down product, 24.4 against 50 at 7B's).
     From 17 rows on the other way is the library product, whose result the next norm kernel adds at no cost: "wide" is
     the faster one only for products with a long K (a feed-forward's down product: 7.2 against 9 microseconds at 0.5B
-    with 64 rows, 29.5 against 31.6 at 7B; an output projection: 4.6 against 3.1), so it needs K >= 2 N there.
+    with 64 rows, 28.3 against 33.8 at 7B; an output projection: 4.6 against 3.1), so it needs K >= 2 N there.
     "unfused" (library product, addition by the next norm) is what remains."""
     size = weight.numel() * weight.element_size()
     skinny = m <= SKINNY_MAX_ROWS and skinny_gemm_takes(m, weight, EPI_RESIDUAL, False)
@@ -2444,7 +2444,8 @@ ROW_CHUNK = 64   # RC_CHUNK of csrc/row_chunks.cu
 ROW_CHUNKS_MIN_TOKENS = 512
 # Beside other sequences (`_chunks_pay`), inside a graph, scan / chunks: 7 heads of 64 x 128: 512 + 31 x 1 tokens 71 / 60, 512 + 63 x 1
 # 74 / 84, 64 x 512 1,238 / 416; 16 heads: 512 + 31 x 1 88 / 104, 1,024 + 31 x 1 172 / 123; 32 heads of 64 x 64: 1,024 + 63 x 1
-# 176 / 288, 4 x 1,024 400 / 164.
+# 176 / 288, 4 x 1,024 400 / 164. (The chunked form's cost per record below is that of an earlier form of its outputs and up to 1.6 times
+# today's: near the line the rule keeps the scan where the chunks would now be done first, 675 for the 416 of 64 x 512.)
 ROW_CHUNKS_COSTS = ((0.13, 0.0, 0.04, 0.2), (20.0, 1.3))
 
 
