@@ -405,8 +405,8 @@ static void split_k(int sms, WideGeometry& geo) {
 // however many the step has: the split of K decides in which order a sum is added, so it follows from the weight's shape and the GPU alone,
 // and a row has the same bits beside any number of others. Products of 16 rows over weights that the L2 does not hold, microseconds, tiles of 128
 // rows / so: 3B's down 15.1 / 13.4 (64 blocks, 128), with 64 rows 18.7 / 16.1; 7B's down 26.5 / 24.4; norm and gate/up of 3B 21.2 / 20.6,
-// of 0.5B 11.5 / 9.9; 7B's output projection 8.6 / 8.5, with 8 rows 8.3 / 8.5. Weights below 16 MB stay in tiles of 128 (0.5B's output projection in 128 blocks instead of 28
-// 6.4 against 5.8 with the norm behind it).
+// of 0.5B 11.5 / 9.9; 7B's output projection 8.6 / 8.5, with 8 rows 8.3 / 8.5. Weights below 16 MB stay in tiles of 128 (0.5B's output
+// projection in 128 blocks instead of 28 6.4 against 5.8 with the norm behind it).
 static void spread_rows(int units, int sms, WideGeometry& geo) {
     constexpr int NTOK = 16;
     float least = 0.f;
