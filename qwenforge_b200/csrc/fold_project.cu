@@ -19,9 +19,7 @@
 // out = sum_s 2^(m_s - M) o_s / sum_s 2^(m_s - M) l_s, rounded to bfloat16 like the attended rows it replaces.
 #include "mma.cuh"
 
-#define FP_KS 32        // inputs per block
-#define FP_LD 40        // shared-memory row in bf16 elements: 80 bytes, so that eight rows of a ldmatrix meet no bank twice
-#define FP_THREADS 256
+#define FP_KS 32        // inputs per block, at least
 #define FP_MAX_ROWS 16
 
 struct FoldProjectArgs {
@@ -31,28 +29,38 @@ struct FoldProjectArgs {
     const bf16* w;          // [n][ldw], K = n_heads * head_dim inputs per output
     float* hidden;          // [rows][n]
     int rows, n, ldw, n_heads, head_dim, max_splits;
+    float* sums;            // [rows][n] or null: moved into the stream on the way, zeros left behind (feed_forward.cu)
 };
 
-__global__ void __launch_bounds__(FP_THREADS) fold_project_kernel(FoldProjectArgs a) {
+template <int KS, int THREADS, bool SUMS>
+__global__ void __launch_bounds__(THREADS) fold_project_kernel(FoldProjectArgs a) {
+    constexpr int LD = KS + 8;   // shared-memory row in elements: an odd number of 16-byte pieces, so that eight rows of a ldmatrix meet no bank twice
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    bf16* w_s = reinterpret_cast<bf16*>(smem_raw);                     // [n][FP_LD]
-    bf16* x_s = w_s + (size_t)a.n * FP_LD;                             // [16][FP_LD]
+    bf16* w_s = reinterpret_cast<bf16*>(smem_raw);                     // [n][LD]
+    bf16* x_s = w_s + (size_t)a.n * LD;                                // [16][LD]
     grid_launch_dependents();
-    const int k0 = blockIdx.x * FP_KS;
+    const int k0 = blockIdx.x * KS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = threadIdx.x; c < a.n * (FP_KS / 8); c += FP_THREADS) {
-        const int n = c / (FP_KS / 8), part = c % (FP_KS / 8);
-        cp_async_16(w_s + (size_t)n * FP_LD + part * 8, a.w + (size_t)n * a.ldw + k0 + part * 8, true);
+    for (int c = threadIdx.x; c < a.n * (KS / 8); c += THREADS) {
+        const int n = c / (KS / 8), part = c % (KS / 8);
+        cp_async_16(w_s + (size_t)n * LD + part * 8, a.w + (size_t)n * a.ldw + k0 + part * 8, true);
     }
     cp_async_commit();
-    for (int i = threadIdx.x; i < 16 * FP_LD / 2; i += FP_THREADS) reinterpret_cast<uint32_t*>(x_s)[i] = 0u;
+    for (int i = threadIdx.x; i < 16 * LD / 2; i += THREADS) reinterpret_cast<uint32_t*>(x_s)[i] = 0u;
+    // (integer divisions behind the wait would be a part of the chain: 1 microsecond a layer)
+    const int per = SUMS ? (a.n / 4 + gridDim.x - 1) / gridDim.x : 0, quad0 = blockIdx.x * per, quads = min(per, a.n / 4 - quad0);
+    const int head = k0 / a.head_dim, d0 = k0 % a.head_dim;
     grid_dependency_wait();
     __syncthreads();  // the zeros are in place before the folded rows go on top of them
 
+    // a slice of what the feed-forward before left, if there is any: every block moves its own columns, a warp per row. The kernels that read it
+    // have ended
+    float4 moved = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (SUMS && warp < a.rows && lane < quads) moved = reinterpret_cast<const float4*>(a.sums + (size_t)warp * a.n)[quad0 + lane];
+
     // ---- fold: thread (row, d) takes input k0 + d of its row over the row's runs
-    const int head = k0 / a.head_dim, d0 = k0 % a.head_dim;
-    for (int item = threadIdx.x; item < a.rows * FP_KS; item += FP_THREADS) {
-        const int r = item / FP_KS, d = item % FP_KS;
+    for (int item = threadIdx.x; item < a.rows * KS; item += THREADS) {
+        const int r = item / KS, d = item % KS;
         const int n_runs = min(max(a.runs[r], 1), a.max_splits);
         const size_t base = ((size_t)r * a.n_heads + head) * a.max_splits;
         const float2* ml = reinterpret_cast<const float2*>(a.part_ml) + base;
@@ -81,23 +89,23 @@ __global__ void __launch_bounds__(FP_THREADS) fold_project_kernel(FoldProjectArg
                 num += w * v[j];
             }
         }
-        x_s[r * FP_LD + d] = __float2bfloat16_rn(den > 0.f ? num * (1.f / den) : 0.f);
+        x_s[r * LD + d] = __float2bfloat16_rn(den > 0.f ? num * (1.f / den) : 0.f);
     }
     cp_async_wait<0>();
     __syncthreads();
 
     // ---- product: warp w takes the outputs 16 g .. 16 g + 15 for g = w, w + 8, ...
-    uint32_t xa[FP_KS / 16][4];
+    uint32_t xa[KS / 16][4];
 #pragma unroll
-    for (int ks = 0; ks < FP_KS / 16; ++ks) ldmatrix_x4(xa[ks], x_s + (lane & 15) * FP_LD + 16 * ks + (lane >> 4) * 8);
+    for (int ks = 0; ks < KS / 16; ++ks) ldmatrix_x4(xa[ks], x_s + (lane & 15) * LD + 16 * ks + (lane >> 4) * 8);
     const int row = lane >> 2, pair = (lane & 3) >> 1;
     const bool odd = lane & 1;
-    for (int g = warp; g < a.n / 16; g += FP_THREADS / 32) {
+    for (int g = warp; g < a.n / 16; g += THREADS / 32) {
         float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-        for (int ks = 0; ks < FP_KS / 16; ++ks) {
+        for (int ks = 0; ks < KS / 16; ++ks) {
             uint32_t wf[4];
-            ldmatrix_x4(wf, w_s + (size_t)(16 * g + (lane >> 4) * 8 + (lane & 7)) * FP_LD + 16 * ks + ((lane >> 3) & 1) * 8);
+            ldmatrix_x4(wf, w_s + (size_t)(16 * g + (lane >> 4) * 8 + (lane & 7)) * LD + 16 * ks + ((lane >> 3) & 1) * 8);
             mma_bf16_16816(c[0], xa[ks], wf[0], wf[1]);
             mma_bf16_16816(c[1], xa[ks], wf[2], wf[3]);
         }
@@ -116,9 +124,16 @@ __global__ void __launch_bounds__(FP_THREADS) fold_project_kernel(FoldProjectArg
             }
         }
     }
+    for (int r = SUMS ? warp : a.rows; r < a.rows; r += THREADS / 32)
+        for (int q = lane; q < quads; q += 32) {
+            float4* from = reinterpret_cast<float4*>(a.sums + (size_t)r * a.n) + quad0 + q;
+            if (r != warp || q != lane) moved = *from;
+            *from = make_float4(0.f, 0.f, 0.f, 0.f);
+            atomicAdd(reinterpret_cast<float4*>(a.hidden + (size_t)r * a.n) + quad0 + q, moved);
+        }
 }
 
-static size_t fold_project_smem(int n) { return ((size_t)n + 16) * FP_LD * sizeof(bf16); }
+static size_t fold_project_smem(int n, int ks) { return ((size_t)n + 16) * (ks + 8) * sizeof(bf16); }
 
 // Whether the kernel takes the shape: the inputs of a block lie inside one head, the outputs come in groups of 16, the
 // weight's rows start on 16 bytes, its slice fits into shared memory, and there are at most 16 rows.
@@ -126,15 +141,19 @@ QF_EXPORT int qf_fold_project_takes(int rows, int n, int ldw, int n_heads, int h
     if (rows < 1 || rows > FP_MAX_ROWS || n < 16 || n % 16 || n_heads < 1 || head_dim < FP_KS || head_dim % FP_KS) return 0;
     if (ldw < n_heads * head_dim || ldw % 8) return 0;
     if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(hidden) & 15)) return 0;
-    return fold_project_smem(n) <= 200 * 1024 ? 1 : 0;
+    return fold_project_smem(n, FP_KS) <= 200 * 1024 ? 1 : 0;
 }
 
 QF_EXPORT int qf_fold_project(const FoldProjectArgs* args, cudaStream_t stream) {
     const FoldProjectArgs& a = *args;
-    if (!qf_fold_project_takes(a.rows, a.n, a.ldw, a.n_heads, a.head_dim, a.w, a.hidden) || a.max_splits < 1)
+    if (!qf_fold_project_takes(a.rows, a.n, a.ldw, a.n_heads, a.head_dim, a.w, a.hidden) || a.max_splits < 1 || (uintptr_t)a.sums % 16)
         return (int)cudaErrorInvalidValue;
-    const size_t smem = fold_project_smem(a.n);
-    cudaError_t e = cudaFuncSetAttribute(fold_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // 64 inputs a block where there are sums: half the blocks, so that the feed-forward behind, a block to an SM's whole shared memory, finds its
+    // SMs free (a decode step at 0.5B sizes, microseconds, 32 / 64 inputs: 1 sequence of 4,000 tokens 563 / 550, 4 613 / 592, 8 671 / 648)
+    const bool whole = a.sums && a.head_dim % 64 == 0 && fold_project_smem(a.n, 64) <= 200 * 1024;
+    const size_t smem = fold_project_smem(a.n, whole ? 64 : 32);
+    auto kernel = whole ? fold_project_kernel<64, 512, true> : a.sums ? fold_project_kernel<32, 256, true> : fold_project_kernel<32, 256, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return (int)launch_pdl(fold_project_kernel, dim3(a.n_heads * a.head_dim / FP_KS), dim3(FP_THREADS), smem, stream, a);
+    return (int)launch_pdl(kernel, dim3(a.n_heads * a.head_dim / (whole ? 64 : 32)), dim3(whole ? 512 : 256), smem, stream, a);
 }

@@ -36,6 +36,8 @@ struct SkinnyArgs {
     float gate_limit, gate_alpha;
     // no kernel in flight writes bias, norm_w and inv_freq: skinny_gemm.cu may read them before it waits for the kernel ahead
     int constants;
+    // NORM, or null: what has not reached the stream yet, [m][k]; a row is hidden + pending (feed_forward.cu leaves it)
+    const float* pending;
 };
 
 template <int EPI> __device__ __forceinline__ void tile_rows(const SkinnyArgs& a, int tile, int g, int& ra, int& rb) {

@@ -33,7 +33,9 @@ struct SkinnyPlan {
     int nblk;      // blocks (clusters) launched
 };
 
-template <int NT, int EPI, bool NORM>
+// PEND (the QKV product): the rows are hidden + pending; few rows are shared by the warps, 8, 4 or 2 to a row, so that a lane has no more than
+// four pieces of both on their way at once (three blocks an SM: few SMs are free beside the feed-forward that leaves `pending`).
+template <int NT, int EPI, bool NORM, bool PEND = false>
 __global__ void __launch_bounds__(SK_THREADS, 3) skinny_gemm_kernel(const SkinnyArgs a, const SkinnyPlan plan) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -129,8 +131,20 @@ __global__ void __launch_bounds__(SK_THREADS, 3) skinny_gemm_kernel(const Skinny
     const bool tile_leader = sub == 0;
     EpiloguePre<NT> pre;
     if (tile_leader && rank == 0) skinny_epilogue_constants<NT, EPI>(a, block0 * tpb + tile_local, g, pre);
-    uint2 norm_first[NORM ? 8 : 1];   // the norm weights of this lane's first columns
-    if (NORM && warp < a.m) {
+    // PEND: `share` warps a row, each a run [c0, c1) of its columns (K is not split then)
+    const int share_log = a.m == 1 ? 3 : a.m == 2 ? 2 : a.m <= 4 ? 1 : 0, share = 1 << share_log;
+    const int pend_row = warp >> share_log, run = (a.k / 4 + share - 1) >> share_log << 2, c0 = (warp & (share - 1)) * run, c1 = min(a.k, c0 + run);
+    uint2 norm_first[PEND ? 4 : NORM ? 8 : 1];   // the norm weights of this lane's first columns
+    if constexpr (PEND) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = c0 + (u * 32 + lane) * 4;
+            norm_first[u] = pend_row < a.m && c < c1 ? *reinterpret_cast<const uint2*>(a.norm_w + c) : make_uint2(0u, 0u);
+        }
+        for (int m = warp; m < MP; m += SK_WARPS)   // rows that do not exist, and columns beyond K
+            for (int i = (m < a.m ? a.k / 8 : 0) + lane; i < plan.stride_x / 16; i += 32)
+                *reinterpret_cast<uint4*>(x_s + (size_t)m * plan.stride_x + i * 16) = make_uint4(0, 0, 0, 0);
+    } else if (NORM && warp < a.m) {
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int c = (u * 32 + lane) * 4;
@@ -141,7 +155,38 @@ __global__ void __launch_bounds__(SK_THREADS, 3) skinny_gemm_kernel(const Skinny
     if (tile_leader && rank == 0) skinny_epilogue_prefetch<NT, EPI>(a, block0 * tpb + tile_local, g, t, pre);
 
     // ---- this block's slice of the token rows, normalised on the way if asked
-    if (NORM) {
+    if constexpr (PEND) {
+        const int row = pend_row;
+        if (row < a.m) {
+            const size_t at = (size_t)row * a.k;
+            bf16* dst = reinterpret_cast<bf16*>(x_s + (size_t)row * plan.stride_x);
+            float ss = 0.f;
+            for (int base = c0; base < c1; base += 32 * 4 * 4) {
+                float4 x[4], y[4];
+                uint2 wv[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int c = base + (u * 32 + lane) * 4;
+                    x[u] = c < c1 ? *reinterpret_cast<const float4*>(a.hidden + at + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    y[u] = c < c1 ? *reinterpret_cast<const float4*>(a.pending + at + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    wv[u] = base == c0 ? norm_first[u] : c < c1 ? *reinterpret_cast<const uint2*>(a.norm_w + c) : make_uint2(0u, 0u);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int c = base + (u * 32 + lane) * 4;
+                    if (c >= c1) continue;
+                    x[u].x += y[u].x, x[u].y += y[u].y, x[u].z += y[u].z, x[u].w += y[u].w;
+                    ss += x[u].x * x[u].x + x[u].y * x[u].y + x[u].z * x[u].z + x[u].w * x[u].w;
+                    const __nv_bfloat162 w01 = *reinterpret_cast<const __nv_bfloat162*>(&wv[u].x);
+                    const __nv_bfloat162 w23 = *reinterpret_cast<const __nv_bfloat162*>(&wv[u].y);
+                    *reinterpret_cast<uint2*>(dst + c) = make_uint2(pack_bf16(x[u].x * __low2float(w01), x[u].y * __high2float(w01)),
+                                                                    pack_bf16(x[u].z * __low2float(w23), x[u].w * __high2float(w23)));
+                }
+            }
+            ss = warp_sum(ss);
+            if (lane == 0) ss_part[0][warp] = ss;
+        }
+    } else if (NORM) {
         // rmsnorm(x) W^T = (x * norm_weight) W^T / rms(x): the rows go into the product scaled by the norm weights only,
         // in one pass over this block's slice, and the row's 1 / rms, a float32 scalar, multiplies the sums in the
         // epilogue. A block adds up the squares of its own slice; the blocks of a cluster add theirs in rank order.
@@ -191,6 +236,11 @@ __global__ void __launch_bounds__(SK_THREADS, 3) skinny_gemm_kernel(const Skinny
         }
     }
     __syncthreads();  // the token rows are staged
+    if (PEND && threadIdx.x < a.m) {   // (read behind the barriers below)
+        float ss = 0.f;
+        for (int p = 0; p < share; ++p) ss += ss_part[0][threadIdx.x * share + p];
+        ss_s[threadIdx.x] = ss;
+    }
     const unsigned char* w_s = w_base;
     const int block = block0;
     if (!mbar_wait(&w_bar[0], 0) && lane == 0) atomicOr(a.err, QF_ERR_COPY_TIMEOUT);
@@ -589,11 +639,12 @@ static int launch_stream_variant(const SkinnyArgs& a, const Decision& d, cudaStr
     return (int)launch_pdl(kernel, dim3(d.stream.nblk), dim3(SK_STREAM_THREADS), d.smem, stream, a, d.stream, d.tiles);
 }
 
-template <int NT, int EPI, bool NORM> static int launch_one(const SkinnyArgs& a, const Decision& d, cudaStream_t stream) {
+template <int NT, int EPI, bool NORM, bool PEND = false> static int launch_one(const SkinnyArgs& a, const Decision& d, cudaStream_t stream) {
+    if (PEND && d.kind != SK_WAVE) return (int)cudaErrorInvalidValue;
     if (d.kind == SK_STREAM) return launch_stream_variant<NT, EPI, NORM, false>(a, d, stream);
     if (d.kind == SK_STREAM_XS) return launch_stream_variant<NT, EPI, false, true>(a, d, stream);
     const SkinnyPlan& p = d.wave;
-    auto kernel = skinny_gemm_kernel<NT, EPI, NORM>;
+    auto kernel = skinny_gemm_kernel<NT, EPI, NORM, PEND>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.smem);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t config = {};
@@ -624,6 +675,10 @@ QF_EXPORT int qf_skinny_gemm(int epilogue, int norm, const SkinnyArgs* args, cud
     const SkinnyArgs& a = *args;
     const Decision d = decide(epilogue, norm != 0, a, qf_sm_count());
     if (d.kind == SK_NONE) return (int)cudaErrorInvalidValue;
+    if (a.pending) {   // (SK_WAVE is the answer 1 of qf_skinny_gemm_takes)
+        if (epilogue != EPI_QKV || !norm || a.m > 8 || d.wave.ksplit != 1 || (uintptr_t)a.pending % 16) return (int)cudaErrorInvalidValue;
+        return launch_one<1, EPI_QKV, true, true>(a, d, stream);
+    }
     switch (epilogue) {
         case EPI_PLAIN:
             return norm ? launch_epi<EPI_PLAIN, true>(a, d, stream) : launch_epi<EPI_PLAIN, false>(a, d, stream);
@@ -657,4 +712,20 @@ QF_EXPORT int qf_skinny_gemm_takes(int epilogue, int norm, int m, int n, int k, 
     a.rot_dim = rot_dim;
     a.inv_freq = rotary ? reinterpret_cast<const float*>(&a) : nullptr;  // only tested against null
     return decide(epilogue, norm != 0, a, qf_sm_count()).kind;
+}
+
+// Whether `qf_skinny_gemm` takes such a QKV product with `pending`: up to eight rows in the one-wave kernel, K not split.
+QF_EXPORT int qf_skinny_gemm_reads_pending(int m, int n, int k, int ldw, int n_heads, int kv_heads, int head_dim, int rotary, int rot_dim) {
+    SkinnyArgs a = {};
+    a.m = m;
+    a.n = n;
+    a.k = k;
+    a.ldw = ldw;
+    a.n_heads = n_heads;
+    a.kv_heads = kv_heads;
+    a.head_dim = head_dim;
+    a.rot_dim = rot_dim;
+    a.inv_freq = rotary ? reinterpret_cast<const float*>(&a) : nullptr;  // only tested against null
+    const Decision d = decide(EPI_QKV, true, a, qf_sm_count());
+    return d.kind == SK_WAVE && m <= 8 && d.wave.ksplit == 1;
 }

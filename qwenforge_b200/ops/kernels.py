@@ -567,7 +567,7 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, tok
 
 class _FoldProjectArgs(ctypes.Structure):
     _fields_ = [("part_o", _P), ("part_ml", _P), ("runs", _P), ("w", _P), ("hidden", _P), ("rows", _I), ("n", _I),
-                ("ldw", _I), ("n_heads", _I), ("head_dim", _I), ("max_splits", _I)]
+                ("ldw", _I), ("n_heads", _I), ("head_dim", _I), ("max_splits", _I), ("sums", _P)]
 
 
 def fold_project_takes(rows: int, weight: torch.Tensor, hidden: torch.Tensor, n_heads: int, head_dim: int) -> bool:
@@ -592,20 +592,25 @@ def fold_project_pays(rows: int, weight: torch.Tensor) -> bool:
 
 
 def fold_project(plan: torch.Tensor, scratch: DecodeScratch, weight: torch.Tensor, hidden: torch.Tensor, n_heads: int,
-                 head_dim: int, n_splits: int) -> None:
+                 head_dim: int, n_splits: int, sums: Optional[torch.Tensor] = None) -> None:
     """hidden[r, :] += fold(the partial results of sequence r) @ weight^T, after `attention_decode(..., fold_later=True)`
     with the same `plan`, `scratch` and `n_splits` in a step whose row r is sequence r (one token per sequence).
     bfloat16 weight [N, n_heads * head_dim], float32 hidden [rows, N]; the blocks' shares are added with atomic
-    reductions, in no fixed order."""
+    reductions, in no fixed order. `sums`: what `feed_forward` left; it goes into hidden as well, and zeros stay in its place."""
     _dev("weight", weight, torch.bfloat16, contiguous=False)
     _dev("hidden", hidden, torch.float32)
     rows = hidden.shape[0]
+    if sums is not None:
+        _dev("sums", sums, torch.float32)
+        if sums.shape != hidden.shape or sums.data_ptr() % 16:
+            raise KernelError("fold_project: sums must have hidden's shape and lie on a 16-byte boundary")
     if not fold_project_takes(rows, weight, hidden, n_heads, head_dim):
         raise KernelError(f"fold_project: does not take {rows} rows, weight {tuple(weight.shape)}, {n_heads} heads of {head_dim}")
     if scratch.part_o is None or scratch.part_o.numel() < rows * n_heads * n_splits * head_dim:
         raise KernelError("fold_project: the scratch does not hold this step's partial results")
     a = _FoldProjectArgs(scratch.part_o.data_ptr(), scratch.part_ml.data_ptr(), plan.data_ptr(), weight.data_ptr(),
-                         hidden.data_ptr(), rows, weight.shape[0], weight.stride(0), n_heads, head_dim, n_splits)
+                         hidden.data_ptr(), rows, weight.shape[0], weight.stride(0), n_heads, head_dim, n_splits,
+                         None if sums is None else sums.data_ptr())
     _check(library("fold_project").qf_fold_project(ctypes.byref(a), _stream()), "fold_project")
 
 
@@ -725,7 +730,7 @@ class _SkinnyArgs(ctypes.Structure):
         ("n_heads", _I), ("kv_heads", _I), ("head_dim", _I), ("rot_dim", _I), ("write_cache", _I),
         ("inv_freq", _P), ("tok_pos", _P), ("tok_seq", _P), ("slots", _P), ("q_out", _P), ("kv_base", _P),
         ("table", _P), ("page_elems", _LL), ("table_stride", _I), ("err", _P), ("gate_limit", _F), ("gate_alpha", _F),
-        ("constants", _I),
+        ("constants", _I), ("pending", _P),
     ]
 
 
@@ -766,6 +771,15 @@ def skinny_gemm_takes(m: int, weight: torch.Tensor, epilogue: int = EPI_PLAIN, n
     return answer
 
 
+def skinny_gemm_reads_pending(m: int, weight: torch.Tensor, n_heads: int, kv_heads: int, head_dim: int, rot_dim: int) -> bool:
+    """Whether `skinny_gemm` takes these rows of a QKV product with `pending`: up to 8 in its one-wave kernel, K not split."""
+    if not (weight.is_cuda and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.stride(1) == 1):
+        return False
+    n, k = weight.shape
+    return library("skinny_gemm").qf_skinny_gemm_reads_pending(_I(int(m)), _I(n), _I(k), _I(weight.stride(0)), _I(n_heads), _I(kv_heads),
+                                                               _I(head_dim), _I(1 if rot_dim > 0 else 0), _I(rot_dim)) != 0
+
+
 def skinny_gemm_pays(m: int, weight: torch.Tensor) -> bool:
     """Whether the weight-streaming kernel is the faster way to run `m` token rows against `weight`, by measurement on
     a B200 (`python -m qwenforge_b200.measure products`): for weights of 100 MB and more it loses to the norm kernel,
@@ -781,7 +795,7 @@ def _skinny_args(epilogue: int, weight: torch.Tensor, *, x: Optional[torch.Tenso
                  hidden: Optional[torch.Tensor] = None, norm_weight: Optional[torch.Tensor] = None, eps: float = 0.0,
                  bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
                  residual: Optional[torch.Tensor] = None, qkv: Optional[dict] = None,
-                 err: Optional[torch.Tensor] = None, clamp=None, constants: bool = False):
+                 err: Optional[torch.Tensor] = None, clamp=None, constants: bool = False, pending: Optional[torch.Tensor] = None):
     """Checks one fused product's tensors and fills the kernels' argument block; returns (block, norm flag).
     clamp = (limit, alpha) with EPI_SWIGLU: the clamped gate in the silu gate's place (see `clamped_glu`)."""
     _dev("weight", weight, torch.bfloat16, contiguous=False)
@@ -798,6 +812,11 @@ def _skinny_args(epilogue: int, weight: torch.Tensor, *, x: Optional[torch.Tenso
         if hidden.shape[1] != a.k or norm_weight.numel() != a.k:
             raise KernelError("skinny_gemm: hidden/norm_weight widths do not match the weight's K")
         a.hidden, a.norm_w, a.eps, a.m = hidden.data_ptr(), norm_weight.data_ptr(), eps, hidden.shape[0]
+        if pending is not None:
+            _dev("pending", pending, torch.float32)
+            if pending.shape != hidden.shape or pending.data_ptr() % 16:
+                raise KernelError("skinny_gemm: pending must have hidden's shape and lie on a 16-byte boundary")
+            a.pending = pending.data_ptr()
     else:
         _dev("x", x, torch.bfloat16, contiguous=False)
         if x.shape[1] != a.k or x.stride(1) != 1:
@@ -849,7 +868,8 @@ def skinny_gemm(epilogue: int, weight: torch.Tensor, **tensors) -> None:
     A product of `x` alone reads `weight` while the kernel ahead on the stream ends: no kernel in flight may be writing it. With a norm, a
     bias or a rotation the launch waits for everything ahead of it, unless constants=True promises that no kernel in flight writes
     weight, norm_weight, bias, inv_freq, positions, slots or page tables (a bound model's step).
-    qkv (EPI_QKV): dict(n_heads, site=KvSiteArgs, inv_freq, rot_dim, tok_pos, tok_seq, slots, q_out, write_cache, err)."""
+    qkv (EPI_QKV): dict(n_heads, site=KvSiteArgs, inv_freq, rot_dim, tok_pos, tok_seq, slots, q_out, write_cache, err).
+    pending (EPI_QKV with hidden, where `skinny_gemm_reads_pending`): the rows are hidden + pending, both float32."""
     a, norm = _skinny_args(epilogue, weight, **tensors)
     code = library("skinny_gemm").qf_skinny_gemm(_I(epilogue), _I(int(norm)), ctypes.byref(a), _stream())
     if code == 1:  # cudaErrorInvalidValue: a shape the kernel does not take
@@ -1051,6 +1071,62 @@ def skinny_chain_repeated(products, repeats: int, steps, sync: torch.Tensor, err
     if code == 1:
         raise KernelError("skinny_chain: these products do not fit the chain kernel; run them one by one")
     _check(code, "skinny_chain_repeated")
+
+
+class _FeedForwardArgs(ctypes.Structure):
+    _fields_ = [("hidden", _P), ("norm_w", _P), ("gate_up", _P), ("down", _P), ("sums", _P), ("err", _P), ("eps", _F), ("rows", _I),
+                ("width", _I), ("inter", _I), ("ldg", _I), ("ldd", _I), ("cols", _I), ("row_warps_log", _I), ("each", _I), ("each_recip", _I)]
+
+
+FEED_FORWARD_MAX_REDUCTIONS = 250_000
+
+
+def feed_forward_takes(rows: int, gate_up: torch.Tensor, down: torch.Tensor) -> bool:
+    """Whether `feed_forward` takes `rows` rows of a SwiGLU layer [gate | up] [2 I, W], down [W, I] and is the faster way: bfloat16 weights
+    whose shares find room in the SMs' shared memory, and no more than 250,000 16-byte reductions (blocks x rows x W / 4). The reductions
+    grow with the rows and what one kernel saves does not: at 896 x 4,864 (122 blocks) a decode step gains 12 to 15 percent with 1 to 4 rows
+    (27,000 to 109,000 reductions) and 4 to 14 with 8 (218,000); more have not been measured. Two products otherwise."""
+    if not (gate_up.is_cuda and down.is_cuda and gate_up.dtype == torch.bfloat16 and down.dtype == torch.bfloat16 and rows <= 8):
+        return False
+    width, inter = down.shape
+    if (gate_up.shape != (2 * inter, width) or gate_up.stride(1) != 1 or down.stride(1) != 1 or gate_up.stride(0) % 8 or down.stride(0) % 8
+            or gate_up.data_ptr() % 16 or down.data_ptr() % 16):
+        return False
+    blocks = library("feed_forward").qf_feed_forward_blocks(_I(int(rows)), _I(width), _I(inter))
+    return blocks > 0 and blocks * rows * width // 4 <= FEED_FORWARD_MAX_REDUCTIONS
+
+
+def feed_forward(hidden: torch.Tensor, norm_weight: torch.Tensor, eps: float, gate_up: torch.Tensor, down: torch.Tensor, sums: torch.Tensor,
+                 err: Optional[torch.Tensor] = None) -> None:
+    """sums += down (silu(g) u) with [g | u] = gate_up (rmsnorm(hidden) * norm_weight), up to 8 rows in one kernel. hidden and sums float32
+    [rows, W], weights bfloat16 [2 I, W] and [W, I]. The blocks' shares are added with atomic reductions, in no fixed order. No kernel in
+    flight may be writing the weights or norm_weight: they are read while the kernel ahead ends."""
+    _dev("hidden", hidden, torch.float32)
+    _dev("sums", sums, torch.float32)
+    _dev("norm_weight", norm_weight, torch.bfloat16)
+    _dev("gate_up", gate_up, torch.bfloat16, contiguous=False)
+    _dev("down", down, torch.bfloat16, contiguous=False)
+    rows, width = hidden.shape
+    inter = down.shape[1]
+    if (gate_up.shape != (2 * inter, width) or down.shape[0] != width or norm_weight.numel() != width or sums.shape != hidden.shape
+            or gate_up.stride(1) != 1 or down.stride(1) != 1):
+        raise KernelError("feed_forward: gate_up must be [2 I, W], down [W, I], sums like hidden")
+    a = _FeedForwardArgs(hidden.data_ptr(), norm_weight.data_ptr(), gate_up.data_ptr(), down.data_ptr(), sums.data_ptr(),
+                         (err if err is not None else _err_word_for(hidden.device)).data_ptr(), eps, rows, width, inter,
+                         gate_up.stride(0), down.stride(0))
+    code = library("feed_forward").qf_feed_forward(ctypes.byref(a), _stream())
+    if code == 1:
+        raise KernelError(f"feed_forward: {rows} rows of {width} x {inter}, or the operands' alignment, are not taken")
+    _check(code, "feed_forward")
+
+
+def take_sums(hidden: torch.Tensor, sums: torch.Tensor) -> None:
+    """hidden += sums; sums = 0 (float32)."""
+    _dev("hidden", hidden, torch.float32)
+    _dev("sums", sums, torch.float32)
+    if sums.shape != hidden.shape:
+        raise KernelError("take_sums: shapes differ")
+    _check(library("feed_forward").qf_take_sums(_ptr(hidden), _ptr(sums), _LL(hidden.numel()), _stream()), "take_sums")
 
 
 def residual_add(hidden: torch.Tensor, delta: torch.Tensor) -> None:

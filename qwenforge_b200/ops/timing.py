@@ -24,7 +24,7 @@ TIMED = ("embed_gather", "gather_rows", "add_rms_norm", "residual_add", "linear"
          "shift_mix", "channel_decay", "outer_state_scan_rows", "row_chunks", "rows_prepare", "causal_conv_cached", "delta_scan", "delta_token",
          "streams_norm", "rotate_heads", "sigmoid_gate", "pair_rms_norm", "map_difference", "rope_maps_cache_write", "rope_table",
          "retention_chunks", "retention_token", "retention_rows", "qkv_product", "tc_gemm_tail", "gated_rows", "attention_decode_plan",
-         "decode_advance_embed")
+         "decode_advance_embed", "feed_forward", "take_sums")
 
 
 class KernelTimer:

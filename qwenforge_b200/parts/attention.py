@@ -50,7 +50,7 @@ import torch
 
 from .. import ops
 from ..cache import PAGE_TOKENS, BundleNeed, KvNeed, StateNeed
-from .base import Mixer, TensorSpec
+from .base import Mixer, PendingSums, TensorSpec
 from .registry import build_part, register_part
 
 
@@ -447,9 +447,28 @@ class GqaAttention(Mixer):
             return False
         return self._ways(ctx) != ("unfused", "unfused")
 
+    def _folds(self, hidden, ctx, o_way) -> bool:
+        """Whether the output projection folds the attention's partial results itself."""
+        n = hidden.shape[0]
+        return (o_way == "skinny" and n == ctx.n_seqs and ops.fold_project_pays(n, self.o_weight)
+                and ops.fold_project_takes(n, self.o_weight, hidden, self.n_heads, self.head_dim))
+
+    def takes_sums(self, hidden, ctx) -> bool:
+        """Whether `fused_forward` will be run on this step and takes a `PendingSums`: the QKV product reads it beside the stream, the
+        projection moves it there."""
+        if not self.fused_takes(ctx):
+            return False
+        qkv_way, o_way = self._ways(ctx)
+        rotary = self.position.fused_rotary() if self.position is not None else None
+        return (qkv_way == "skinny" and self._folds(hidden, ctx, o_way)
+                and ops.skinny_gemm_reads_pending(hidden.shape[0], self.qkv_weight, self.n_heads, self.n_kv, self.head_dim, rotary[1] if rotary else 0))
+
     def fused_forward(self, hidden, rms, ctx, site, writes_cache, delta=None):
         n = hidden.shape[0]
         qkv_way, o_way = self._ways(ctx)
+        sums = None
+        if isinstance(delta, PendingSums):   # (`takes_sums` has said yes)
+            sums, delta = delta.sums, None
         plan = self.decode_plan(ctx)
         inv_freq, rot_dim = self.position.fused_rotary() if self.position is not None else (None, 0)
         args = ops.KvSiteArgs(site.storage, site.table, self.n_kv, self.head_dim)
@@ -458,7 +477,7 @@ class GqaAttention(Mixer):
             if delta is not None:
                 ops.residual_add(hidden, delta)
             ops.skinny_gemm(ops.EPI_QKV, self.qkv_weight, hidden=hidden, norm_weight=rms[0], eps=rms[1],
-                            bias=self.qkv_bias_t, constants=True,
+                            bias=self.qkv_bias_t, constants=True, pending=sums,
                             qkv=dict(n_heads=self.n_heads, site=args, inv_freq=inv_freq, rot_dim=rot_dim, tok_pos=ctx.tok_pos,
                                      tok_seq=ctx.tok_seq, slots=ctx.slots, q_out=q, write_cache=writes_cache, err=ctx.err))
         else:
@@ -472,12 +491,11 @@ class GqaAttention(Mixer):
                 ops.rope_cache_write(ops.linear(x, self.qkv_weight), ctx.tok_seq, ctx.tok_pos, ctx.slots, inv_freq, rot_dim,
                                      self.n_heads, q, args, writes_cache, ctx.err, bias=self.qkv_bias_t)
         n_splits = self.decode_splits(ctx)
-        if (o_way == "skinny" and n == ctx.n_seqs and ops.fold_project_pays(n, self.o_weight)
-                and ops.fold_project_takes(n, self.o_weight, hidden, self.n_heads, self.head_dim)):
+        if self._folds(hidden, ctx, o_way):
             # the attention kernel stops at its runs' partial results; the projection folds them on its way in
             ops.attention_decode(q, None, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs, self.scale,
                                  self.window, n_splits, ctx.decode_scratch, ctx.err, plan, fold_later=True)
-            ops.fold_project(plan, ctx.decode_scratch, self.o_weight, hidden, self.n_heads, self.head_dim, n_splits)
+            ops.fold_project(plan, ctx.decode_scratch, self.o_weight, hidden, self.n_heads, self.head_dim, n_splits, sums)
             return
         attended = torch.empty_like(q)
         ops.attention_decode(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,

@@ -213,6 +213,22 @@ class PendingScaled(Pending):
         return out if self.b is None else out + self.b.to(torch.float32) * self.scale_b
 
 
+class PendingSums(Pending):
+    """A feed-forward's output in float32 rows of their own (`ops.feed_forward`), zeros again once it is in the stream. A decode step's
+    QKV product reads the stream and these rows together, and its output projection moves them into the stream."""
+    __slots__ = ("sums",)
+
+    def __init__(self, sums: torch.Tensor):
+        self.sums = sums
+
+    def add_to(self, hidden: torch.Tensor) -> None:
+        from .. import ops
+        ops.take_sums(hidden, self.sums)
+
+    def value(self) -> torch.Tensor:
+        return self.sums
+
+
 class PendingNormed(Pending):
     """A sublayer's output that still has to be normalised (RMS, weight, eps) and added to the residual stream: what a
     block with norms after its sublayers hands to whoever runs next, so that the addition rides on that part's first norm

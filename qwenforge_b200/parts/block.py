@@ -9,7 +9,7 @@ import torch
 
 from .. import ops
 from ..cache import BundleNeed
-from .base import Norm, Part, Pending, PendingNormed, PendingPair, PendingScaled, PendingStreams, RowSum, fork, join, runs_side_by_side
+from .base import Norm, Part, Pending, PendingNormed, PendingPair, PendingScaled, PendingStreams, PendingSums, RowSum, fork, join, runs_side_by_side
 from .registry import build_part, register_part
 
 
@@ -19,7 +19,7 @@ class PreNormBlock(Part):
     h += m * mixer(norm_1(h));  h += m * feed_forward(norm_2(h))  (the product and the sum in float32, inside the next norm's
     kernel). A mixer may hand back two outputs under a factor each (`PendingScaled`); they go the same way."""
 
-    accepts_pending = (PendingScaled,)
+    accepts_pending = (PendingScaled, PendingSums)
 
     def __init__(self, layer_spec):
         self.kind = "pre_norm"
@@ -48,6 +48,10 @@ class PreNormBlock(Part):
         return PendingScaled.of(self.feed_forward.forward(x, ctx), self.residual_mult)
 
     def forward(self, hidden, delta, ctx, site, writes_cache):
+        if isinstance(delta, PendingSums) and (self.mixer_norm.fused_rms() is None or self.residual_mult != 1.0 or self.feed_forward is None
+                                               or not getattr(self.mixer, "takes_sums", lambda *_: False)(hidden, ctx)):
+            delta.add_to(hidden)
+            delta = None
         if self.residual_mult != 1.0 or self.feed_forward is None or getattr(self.mixer, "scaled_outputs", False) \
                 or isinstance(delta, PendingScaled):
             return self._forward_scaled(hidden, delta, ctx, site, writes_cache)
@@ -60,8 +64,7 @@ class PreNormBlock(Part):
             delta = self.mixer.forward(x, ctx, site, writes_cache)
         rms = self.feed_forward_norm.fused_rms()
         if rms is not None and self.feed_forward.fused_takes(ctx):
-            self.feed_forward.fused_forward(hidden, rms, ctx, delta)
-            return None
+            return self.feed_forward.fused_forward(hidden, rms, ctx, delta)
         x = self.feed_forward_norm.forward(hidden, delta)
         return self.feed_forward.forward(x, ctx)
 

@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from .. import ops
-from .base import FeedForward, TensorSpec
+from .base import FeedForward, PendingSums, TensorSpec
 from .registry import register_part
 
 
@@ -26,7 +26,7 @@ class SwiGlu(FeedForward):
         ]
 
     def kernel_libraries(self, dtype):
-        return {"activation"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "tc_gemm", "wide_gemm"})
+        return {"activation"} | ({"gemm_f32"} if dtype == torch.float32 else {"skinny_gemm", "tc_gemm", "wide_gemm", "feed_forward"})
 
     def bind(self, tensors, dtype, device):
         self.gate_up_weight = torch.cat((tensors[self.file_name("gate_weight")], tensors[self.file_name("up_weight")]),
@@ -63,6 +63,15 @@ class SwiGlu(FeedForward):
                 and ctx.n_tokens <= ops.WIDE_MAX_ROWS and self._ways(ctx) != ("unfused", "unfused"))
 
     def fused_forward(self, hidden, rms, ctx, delta=None):
+        """Adds to the stream, or returns what is still to reach it."""
+        if delta is None and ctx.step_memo is not None and ops.feed_forward_takes(hidden.shape[0], self.gate_up_weight, self.down_weight):
+            # the whole layer out of the SMs' shared memory, in one kernel; its output stands in rows of its own that all layers share
+            key = ("swiglu.sums", tuple(hidden.shape))
+            sums = ctx.step_memo.get(key)
+            if sums is None:
+                sums = ctx.step_memo[key] = torch.zeros_like(hidden)
+            ops.feed_forward(hidden, rms[0], rms[1], self.gate_up_weight, self.down_weight, sums, ctx.err)
+            return PendingSums(sums)
         gate_up, down = self._ways(ctx)
         act = torch.empty((hidden.shape[0], self.inter), dtype=torch.bfloat16, device=hidden.device)
         if gate_up == "skinny":
@@ -83,6 +92,7 @@ class SwiGlu(FeedForward):
             ops.wide_gemm(ops.EPI_RESIDUAL, self.down_weight, x=act, residual=hidden, err=ctx.err)
         else:
             ops.residual_add(hidden, ops.linear(act, self.down_weight))
+        return None
 
 
 register_part("feed_forward", "swiglu", SwiGlu)

@@ -1,0 +1,109 @@
+"""The feed-forward of a step of few rows as one kernel, and the two kernels that take its sums along."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _layer(width, inter, rows, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device=DEV)
+    return (rnd(rows, width), (1 + 0.1 * rnd(width)).bfloat16(), (rnd(2 * inter, width) * width ** -0.5).bfloat16(),
+            (rnd(width, inter) * inter ** -0.5).bfloat16(), rnd(rows, width))
+
+
+# every number of warps a row and of warps a tile (8 to 128 columns a block), a half step of K in the down product, a ragged last block
+@pytest.mark.parametrize("width,inter", [(896, 4864), (896, 4872), (1024, 3000), (512, 1184), (128, 2368), (64, 18944), (288, 4720), (1536, 1184)])
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8])
+def test_against_float64(width, inter, rows):
+    from qwenforge_b200 import ops
+    hidden, norm, gate_up, down, before = _layer(width, inter, rows, width + inter + rows)
+    assert ops.feed_forward_takes(rows, gate_up, down) or rows * width * 148 // 4 > 250_000
+    sums, kept, err = before.clone(), hidden.clone(), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.feed_forward(hidden, norm, 1e-6, gate_up, down, sums, err)
+    h = hidden.double()
+    y = h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * norm.double() @ gate_up.double().T
+    want = (torch.nn.functional.silu(y[:, :inter]) * y[:, inter:]) @ down.double().T
+    assert int(err) == 0 and torch.equal(hidden, kept)
+    # the rows and the activations are rounded to eight bits (2^-9 each at worst); what is added to lies in float32
+    assert float(((sums - before).double() - want).norm()) < 2.0 ** -8 * float(want.norm())
+
+
+def test_what_is_not_taken():
+    from qwenforge_b200 import ops
+    hidden, norm, gate_up, down, sums = _layer(896, 4864, 9, 1)
+    assert not ops.feed_forward_takes(9, gate_up, down)                   # rows
+    with pytest.raises(ops.KernelError if hasattr(ops, "KernelError") else Exception):
+        ops.feed_forward(hidden, norm, 1e-6, gate_up, down, sums)
+    _, _, wide, narrow, _ = _layer(2048, 11008, 1, 1)                     # weights beyond the shared memory
+    assert not ops.feed_forward_takes(1, wide, narrow)
+    _, _, odd, odd_down, _ = _layer(900, 4864, 1, 1)                      # a width of no whole blocks of 32
+    assert not ops.feed_forward_takes(1, odd, odd_down)
+
+
+@pytest.mark.parametrize("seqs", [1, 2, 3, 8])
+def test_decode_steps_with_and_without(seqs, monkeypatch):
+    """Three layers of the smallest preset's sizes, prompts and then single tokens: the logits of the layers as two kernels, within the
+    rounding of activations to eight bits; launch by launch, each step from the same cache."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.config import preset_config
+    from qwenforge_b200.engine import Model
+    config = preset_config("qwen2.5-0.5b", num_hidden_layers=3, vocab_size=512)
+    model = Model.from_random(config, 3)
+    logits, ran = {}, []
+    real = ops.feed_forward
+    monkeypatch.setattr(ops, "feed_forward", lambda *a, **k: (ran.append(1), real(*a, **k))[1])
+    for on in (True, False):
+        if not on:
+            monkeypatch.setattr(ops, "feed_forward_takes", lambda *a: False)
+        cache = model.new_cache(64 * 4 * seqs, seqs)
+        slots = [cache.open() for _ in range(seqs)]
+        model.step(cache, [(s, list(range(1, 20 + 7 * i))) for i, s in enumerate(slots)])
+        logits[on] = [model.step(cache, [(s, [5 + i + n]) for i, s in enumerate(slots)]) for n in range(4)]
+    assert len(ran) == 3 * 4
+    model.raise_on_kernel_error()
+    for a, b in zip(logits[True], logits[False]):
+        assert float((a - b).norm()) < 2e-2 * float(b.norm())
+
+
+@pytest.mark.parametrize("rows,heads,dim", [(1, 14, 64), (8, 14, 64), (3, 4, 96), (5, 2, 128)])
+def test_the_projection_moves_the_sums(rows, heads, dim):
+    """With sums the stream is what it is without, plus the sums; zeros stay behind. (96: blocks of 32 inputs; the others of 64.)"""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(rows + dim)
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device=DEV)
+    width, splits = 272, 3
+    scratch = ops.DecodeScratch(torch.device(DEV))
+    scratch.part_o = rnd(rows * heads * splits * dim)
+    scratch.part_ml = torch.rand(rows * heads * splits * 2, generator=g, device=DEV) + 0.5
+    plan = torch.tensor([1 + i % splits for i in range(8)], dtype=torch.int32, device=DEV)
+    weight, hidden, sums = (rnd(width, heads * dim) * 0.05).bfloat16(), rnd(rows, width), rnd(rows, width)
+    plain, both, left = hidden.clone(), hidden.clone(), sums.clone()
+    ops.fold_project(plan, scratch, weight, plain, heads, dim, splits)
+    ops.fold_project(plan, scratch, weight, both, heads, dim, splits, left)
+    assert not bool(left.any())
+    # the shares of up to 56 blocks are added in any order: 56 roundings of 2^-24 of numbers of size up to about 8
+    assert float((both - (plain + sums)).abs().max()) < 57 * 2.0 ** -24 * 8
+    left = sums.clone()
+    ops.take_sums(plain, left)
+    assert not bool(left.any()) and float((both - plain).abs().max()) < 57 * 2.0 ** -24 * 8
+
+
+@pytest.mark.parametrize("rows", [1, 2, 4, 7, 8])
+def test_the_qkv_product_reads_stream_and_sums(rows):
+    from qwenforge_b200 import ops
+    from qwenforge_b200.measure import layer_products
+    products, state = layer_products(rows, 904, 1024, 14, 2, 64)    # (a K of no whole block of 32)
+    t = products[3].tensors
+    assert ops.skinny_gemm_reads_pending(rows, products[3].weight, 14, 2, 64, 64)
+    products[3].run()
+    want_q, want_cache = state["q_out"].clone(), state["cache"].clone()
+    part = torch.randn_like(t["hidden"])
+    rest = t["hidden"] - part
+    ops.skinny_gemm(ops.EPI_QKV, products[3].weight, **{**t, "hidden": rest, "pending": t["hidden"] - rest})
+    assert int(state["err"]) == 0
+    for got, want in ((state["q_out"], want_q), (state["cache"], want_cache)):
+        # (hidden - rest) + rest is hidden to a rounding of 2^-24; results lie one step of eight bits apart at most
+        assert float((got.float() - want.float()).abs().max()) <= 2.0 ** -7 * float(want.float().abs().max())
+        assert float((got.float() - want.float()).norm()) <= 2.0 ** -9 * float(want.float().norm())
