@@ -37,11 +37,12 @@ struct Over {
 // time, a run of four neighbouring tokens to a thread. Every thread works out its tokens' two log gates (tanh, logsigmoid). What
 // its run does to the maximum m before it is  max(f_4 + (f_3 + (f_2 + (f_1 + m))), b)  with b the chain of the run alone (from minus
 // infinity): a rounded addition keeps the order of its arguments, so that the maxima may be taken after the additions, with the very
-// bits of the chain token by token. So one thread takes m from run to run by four additions and a maximum, and every thread then
-// walks its own tokens from the m before them. Neighbouring tokens share the very same m, so what a token's gates say cancels in
-// the mixer's quotient, and the bits are the same for every cut of a sequence, in both precisions. What bounds it is that one
-// thread's chain: 2,048 tokens of 7 heads take 14.5 microseconds (37 with a warp that hands every link on by shuffles; 256 tokens 4.1
-// and 5.9, a single token 2.1 either way).
+// bits of the chain token by token. By the same rule four runs of neighbouring threads are one: what they do to m is 16 additions and a
+// maximum with the chain of the four alone, which the threads make among themselves. So one thread takes m from four runs to the next four,
+// leaving the sums between them behind, and every thread then takes its run's maximum and walks its own tokens from it. Neighbouring tokens
+// share the very same m, so what a token's gates say cancels in the mixer's quotient, and the bits are the same for every cut of a
+// sequence, in both precisions. What bounds it is that one thread's chain, four cycles a token, and what the
+// threads make around it: 2,048 tokens of 7 heads take 12.8 microseconds (14.2 with a turn of the chain for every two runs; 256 tokens 3.7 and 3.8).
 #define GATE_THREADS 512
 #define GATE_EACH 4
 #define GATE_TOKENS (GATE_THREADS * GATE_EACH)
@@ -54,15 +55,15 @@ stabilized_gates_kernel(const float* __restrict__ pre, int pre_stride, const flo
                         long long slot_stride, long long m_offset, int n_heads, float* __restrict__ decay,
                         float* __restrict__ take, float* __restrict__ floor_out) {
     grid_chain_entry();
-    __shared__ __align__(16) float4 f_s[GATE_THREADS];
-    __shared__ __align__(8) float end_s[GATE_THREADS], before_s[GATE_THREADS + 2];   // a run's own chain at its end; the maximum before a run
+    __shared__ __align__(16) float4 f_s[GATE_THREADS], before_s[GATE_THREADS / 4];   // before_s: the maximum before four runs, sums behind three
+    __shared__ float end_s[GATE_THREADS / 4], last_s;                                // four runs' own chain at their end
     const int seq = blockIdx.x / n_heads, head = blockIdx.x % n_heads;
     const int begin = cu_q[seq], end = cu_q[seq + 1], slot = slots[seq];
     float* m_ptr = slot >= 0 ? state + slot * slot_stride + m_offset + head : nullptr;
     float m = m_ptr ? *m_ptr : 0.f;   // the maximum before the tokens in hand
     const float bi = bias[head], bf = bias[n_heads + head];
     for (int t0 = begin; t0 < end; t0 += GATE_TOKENS) {
-        const int n_here = min(GATE_TOKENS, end - t0), n_pairs = (n_here + 2 * GATE_EACH - 1) / (2 * GATE_EACH);   // two runs a turn of the chain
+        const int n_here = min(GATE_TOKENS, end - t0), n_fours = (n_here + 4 * GATE_EACH - 1) / (4 * GATE_EACH);   // four runs a turn of the chain
         const int first = threadIdx.x * GATE_EACH, count = max(0, min(GATE_EACH, n_here - first));   // this thread's tokens
         float a[GATE_EACH], f[GATE_EACH], b = -INFINITY;
 #pragma unroll
@@ -80,29 +81,46 @@ stabilized_gates_kernel(const float* __restrict__ pre, int pre_stride, const flo
             f[i] = log_sigmoid(cap * tanhf((f[i] + bf) / cap));
             b = i == 0 ? a[i] : fmaxf(f[i] + b, a[i]);
         }
-        if (threadIdx.x < 2 * n_pairs) f_s[threadIdx.x] = make_float4(f[0], f[1], f[2], f[3]), end_s[threadIdx.x] = b;
+        // the chains of the runs up to this thread's, of its four, alone
+        float own = b, before_own = -INFINITY;
+#pragma unroll
+        for (int r = 1; r < 4; ++r) {
+            const float ahead = __shfl_up_sync(0xffffffffu, own, 1);
+            if ((threadIdx.x & 3) == r) before_own = ahead, own = fmaxf(f[3] + (f[2] + (f[1] + (f[0] + ahead))), b);
+        }
+        if (threadIdx.x < 4 * n_fours) {
+            f_s[threadIdx.x] = make_float4(f[0], f[1], f[2], f[3]);
+            if ((threadIdx.x & 3) == 3) end_s[threadIdx.x >> 2] = own;
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
-            const float2* e2 = reinterpret_cast<const float2*>(end_s);
-            float4 x = f_s[0], y = f_s[1];
-            float2 e = e2[0];
-            float run = m;
-            for (int p = 0; p < n_pairs; ++p) {
-                const float4 u = x, v = y;
-                const float2 at = e;
-                const int next = min(p + 1, n_pairs - 1);
-                x = f_s[2 * next], y = f_s[2 * next + 1], e = e2[next];
-                float2 before;
+            float4 x[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) x[r] = f_s[r];
+            float e = end_s[0], run = m;
+            for (int p = 0; p < n_fours; ++p) {
+                float4 u[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) u[r] = x[r];
+                const float at = e;
+                const int next = min(p + 1, n_fours - 1);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) x[r] = f_s[4 * next + r];
+                e = end_s[next];
+                float4 before;
                 before.x = run;
-                before.y = fmaxf(u.w + (u.z + (u.y + (u.x + run))), at.x);
-                run = fmaxf(v.w + (v.z + (v.y + (v.x + before.y))), at.y);
-                reinterpret_cast<float2*>(before_s)[p] = before;
+                before.y = u[0].w + (u[0].z + (u[0].y + (u[0].x + run)));
+                before.z = u[1].w + (u[1].z + (u[1].y + (u[1].x + before.y)));
+                before.w = u[2].w + (u[2].z + (u[2].y + (u[2].x + before.z)));
+                run = fmaxf(u[3].w + (u[3].z + (u[3].y + (u[3].x + before.w))), at);
+                before_s[p] = before;
             }
-            before_s[2 * n_pairs] = run;
+            last_s = run;
         }
         __syncthreads();
         if (count > 0) {
-            m = before_s[threadIdx.x];
+            m = reinterpret_cast<const float*>(before_s)[threadIdx.x];
+            if (threadIdx.x & 3) m = fmaxf(m, before_own);
 #pragma unroll
             for (int i = 0; i < GATE_EACH; ++i) {
                 if (i >= count) break;
@@ -114,7 +132,7 @@ stabilized_gates_kernel(const float* __restrict__ pre, int pre_stride, const flo
                 m = m_new;
             }
         }
-        m = before_s[2 * n_pairs];   // (written again only behind the next barrier)
+        m = last_s;   // (written again only behind the next barrier)
     }
     if (m_ptr && threadIdx.x == 0 && begin < end) *m_ptr = m;
 }
@@ -123,7 +141,13 @@ QF_EXPORT int qf_stabilized_gates(const float* pre, int pre_stride, const float*
                                   const int* slots, int n_seqs, float* state, long long slot_stride, long long m_offset,
                                   int n_heads, float* decay, float* take, float* floor_out, cudaStream_t stream) {
     if (n_seqs <= 0 || n_heads <= 0) return 0;
-    return (int)launch_pdl(stabilized_gates_kernel, dim3(n_seqs * n_heads), dim3(GATE_THREADS), 0, stream, pre, pre_stride, bias, cap,
+    // Few blocks ask for more than half of an SM's shared memory, which they do not use: launched while the product ahead still holds the SMs,
+    // they would all go to the first ones that it leaves, four to an SM (behind the mLSTM's projections, 2,048 tokens of 7 heads, from the
+    // product's end to this kernel's 22 microseconds, 15 so).
+    const size_t spread = n_seqs * n_heads <= qf_sm_count() ? 116 * 1024 : 0;
+    const cudaError_t e = cudaFuncSetAttribute(stabilized_gates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    return (int)launch_pdl(stabilized_gates_kernel, dim3(n_seqs * n_heads), dim3(GATE_THREADS), spread, stream, pre, pre_stride, bias, cap,
                            cu_q, slots, n_seqs, state, slot_stride, m_offset, n_heads, decay, take, floor_out);
 }
 
