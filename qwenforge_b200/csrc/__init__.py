@@ -1,3 +1,3 @@
-from .build import KernelLibraryError, build_all, library, library_names, prepare
+from .build import KernelLibraryError, build_all, host_module, library, library_names, prepare
 
-__all__ = ["KernelLibraryError", "build_all", "library", "library_names", "prepare"]
+__all__ = ["KernelLibraryError", "build_all", "host_module", "library", "library_names", "prepare"]

@@ -11,6 +11,9 @@ Built files go to `_build/` beside the sources when that folder can be written, 
 `$QWENFORGE_B200_BUILD_DIR`, else to a per-user folder under the system's temporary
 directory. Nothing here needs HOME or a network.
 
+One source, `host.cpp`, is a Python module instead (`host_module()`): it launches the others' kernels from native code. It is built the
+same way, against the headers of the torch in use, whose version is part of its name.
+
 There is no fallback: if nvcc is missing or a compilation fails, `KernelLibraryError`
 says which file and why, and nothing runs.
 """
@@ -33,7 +36,9 @@ _NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared",
 ]
+_HOST = "host"           # the one source that is a Python module
 _loaded: dict[str, ctypes.CDLL] = {}
+_modules: dict = {}
 _lock = threading.Lock()
 
 
@@ -42,7 +47,23 @@ class KernelLibraryError(RuntimeError):
 
 
 def library_names() -> list[str]:
-    return sorted(p.stem for p in _SRC.glob("*.cu"))
+    return sorted([p.stem for p in _SRC.glob("*.cu")] + [_HOST])
+
+
+def _source(name: str) -> Path:
+    return _SRC / f"{name}.{'cpp' if name == _HOST else 'cu'}"
+
+
+def _flags(name: str) -> list[str]:
+    if name != _HOST:
+        return _NVCC_FLAGS
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    return ["-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-I", sysconfig.get_paths()["include"], "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
+            "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
 
 
 def _say(message: str) -> None:
@@ -85,8 +106,13 @@ def _build_dir() -> Path:
 
 def _digest(name: str) -> str:
     h = hashlib.sha256()
-    h.update(" ".join(_NVCC_FLAGS).encode())
-    for path in sorted(_SRC.glob("*.cuh")) + sorted(_SRC.glob("*.h")) + [_SRC / f"{name}.cu"]:
+    if name == _HOST:
+        import torch
+        h.update(f"{torch.__version__} {sys.version}".encode())
+    else:
+        h.update(" ".join(_NVCC_FLAGS).encode())
+    shared = [] if name == _HOST else sorted(_SRC.glob("*.cuh")) + sorted(_SRC.glob("*.h"))
+    for path in shared + [_source(name)]:
         h.update(path.name.encode())
         h.update(path.read_bytes())
     return h.hexdigest()[:16]
@@ -105,7 +131,7 @@ def _find_built(name: str, digest: str) -> Path | None:
 
 
 def _compile(name: str) -> Path:
-    source = _SRC / f"{name}.cu"
+    source = _source(name)
     if not source.exists():
         raise KernelLibraryError(f"no kernel source {source.name}; known: {', '.join(library_names())}")
     digest = _digest(name)
@@ -115,7 +141,7 @@ def _compile(name: str) -> Path:
     out_dir = _build_dir()
     target = out_dir / f"{name}.{digest}.so"
     partial = out_dir / f".{name}.{digest}.{os.getpid()}.{threading.get_ident()}.tmp.so"
-    command = [_nvcc(), *_NVCC_FLAGS, "-I", str(_SRC), "-o", str(partial), str(source)]
+    command = [_nvcc(), *_flags(name), "-I", str(_SRC), "-o", str(partial), str(source)]
     _say(f"compiling {source.name} for sm_100a ...")
     started = time.time()
     env = dict(os.environ)
@@ -155,10 +181,33 @@ def library(name: str) -> ctypes.CDLL:
     return lib
 
 
+def host_module():
+    """The module of `host.cpp` (compiling it first if no current build exists); a kernel library's address is handed to it by whoever
+    loads one (`ops/host.py`)."""
+    module = _modules.get(_HOST)
+    if module is None:
+        with _lock:
+            module = _modules.get(_HOST)
+            if module is None:
+                import importlib.machinery
+                import importlib.util
+
+                import torch  # noqa: F401  (its libraries are what the module is linked against)
+                path = str(_compile(_HOST))
+                loader = importlib.machinery.ExtensionFileLoader("qf_host", path)
+                try:
+                    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("qf_host", path, loader=loader))
+                    loader.exec_module(module)
+                except ImportError as exc:
+                    raise KernelLibraryError(f"cannot load {path}: {exc}") from exc
+                _modules[_HOST] = module
+    return module
+
+
 def prepare(names) -> None:
     """Compile (in parallel) and load the named libraries; used when a model is built, so
     that all compilation happens up front with progress lines instead of inside the first step."""
-    todo = [n for n in sorted(set(names)) if n not in _loaded]
+    todo = [n for n in sorted(set(names)) if n not in _loaded and n not in _modules]
     if not todo:
         return
     missing = [n for n in todo if _find_built(n, _digest(n)) is None]
@@ -167,7 +216,7 @@ def prepare(names) -> None:
         with ThreadPoolExecutor(max_workers=min(8, len(missing))) as pool:
             list(pool.map(_compile, missing))
     for n in todo:
-        library(n)
+        host_module() if n == _HOST else library(n)
 
 
 def build_all() -> list[str]:

@@ -1,0 +1,219 @@
+// The launches of a prompt step's longest stretches, issued from native code: a norm; queries, keys and values, attention and output
+// projection; gate, up and down; a matrix memory's whole mixer. The kernels and the library products are those that the Python entries of
+// ops/kernels.py launch one by one, where a layer of few microseconds a kernel waits for its arguments to be made (a launch 4 to 5
+// microseconds of host time beside 2 to 3 of the driver's own, a buffer 3 to 5; here 3 and 1).
+// Every function looks at its tensors as those entries do and answers None, having done nothing, for what it does not take: the caller then
+// goes their way, where the same condition is reported or another kernel chosen. Nothing is kept between calls but the entries' addresses.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+namespace {
+
+typedef cudaStream_t Stream;
+struct QkvArgs {   // TcQkvArgs of tc_gemm.cu
+    const void* bias;
+    const void* angles;
+    const int *tok_pos, *tok_seq, *slots;
+    void *q_out, *kv_base;
+    const int* table;
+    long long page_elems;
+    int table_stride, n_heads, kv_heads, head_dim, write_cache;
+    const float* inv_freq;
+};
+
+int (*add_rms_norm)(int, float*, const void*, const void*, void*, int, int, float, int, Stream);
+int (*qkv_pairs_pays)(int, int, int, int);
+int (*qkv_pairs)(const void*, int, const void*, int, int, int, const QkvArgs*, int*, Stream);
+int (*prefill_tc)(const void*, void*, const int*, const int*, const int*, void*, const int*, long long, int, int, int, int, int, int, int, int,
+                  float, int, int*, const float*, int, Stream);
+int (*tc_is_persistent)(int, int, int);
+int (*tc_gemm)(int, const void*, int, const void*, int, void*, int, int, int, int, int*, Stream);
+int (*tc_gemm_tail)(const void*, int, const void*, int, void*, int, float*, int, int, int, int, int*, Stream);
+int (*stabilized_gates)(const float*, int, const float*, float, const int*, const int*, int, float*, long long, long long, int, float*, float*,
+                        float*, Stream);
+int (*state_chunks)(const void*, int, const void*, int, const void*, int, const float*, const float*, const float*, const float*, int, const int*,
+                    const int*, int, int, float*, long long, long long, long long, int, int, int, int, float, float*, long long, int, float*,
+                    float*, Stream);
+int (*gated_group_norm)(int, const float*, const void*, int, const void*, float, void*, int, int, int, int, int, int, const float*, const float*,
+                        float, const float*, const void*, int, Stream);
+PyObject* kernel_error = nullptr;
+
+const struct {
+    const char* name;
+    void** to;
+} entries[] = {{"qf_add_rms_norm", (void**)&add_rms_norm}, {"qf_tc_gemm_qkv_pairs_pays", (void**)&qkv_pairs_pays},
+               {"qf_tc_gemm_qkv_pairs", (void**)&qkv_pairs}, {"qf_attention_prefill_tc_ex", (void**)&prefill_tc},
+               {"qf_tc_gemm_is_persistent", (void**)&tc_is_persistent}, {"qf_tc_gemm", (void**)&tc_gemm}, {"qf_tc_gemm_tail", (void**)&tc_gemm_tail},
+               {"qf_stabilized_gates", (void**)&stabilized_gates}, {"qf_state_chunks", (void**)&state_chunks},
+               {"qf_gated_group_norm", (void**)&gated_group_norm}};
+
+// setup(KernelError, {name: address}): some of the entries, or more of them later.
+PyObject* setup(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2 || !PyDict_Check(args[1])) return PyErr_Format(PyExc_TypeError, "setup(error, addresses)");
+    Py_INCREF(args[0]);
+    Py_XDECREF(kernel_error);
+    kernel_error = args[0];
+    for (const auto& e : entries)
+        if (PyObject* at = PyDict_GetItemString(args[1], e.name)) *e.to = PyLong_AsVoidPtr(at);
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+}
+
+// ---- arguments
+const at::Tensor* tensor(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+long long number(PyObject* o) { return PyLong_AsLongLong(o); }
+
+bool whole(const at::Tensor* t, at::ScalarType type) { return t && t->is_cuda() && t->scalar_type() == type && t->is_contiguous(); }
+const int* ints(const at::Tensor* t) { return t->const_data_ptr<int>(); }
+template <typename T = void> T* at_ptr(const at::Tensor& t) { return static_cast<T*>(t.data_ptr()); }
+bool on16(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+// What `tc_gemm_takes` asks of a matrix: rows on 16-byte boundaries.
+bool rows16(const at::Tensor* t) {
+    return t && t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 2 && t->stride(1) == 1 && t->size(1) % 8 == 0 && t->stride(0) % 8 == 0 && on16(*t);
+}
+Stream stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+bool ok(int code, const char* what) {
+    if (code == 0) return true;
+    if (code == 801) PyErr_Format(kernel_error, "%s: the driver offers no tensor-map encoder (cuTensorMapEncodeTiled)", what);
+    else PyErr_Format(kernel_error, "%s: CUDA error %d at launch", what, code);
+    return false;
+}
+
+// rms_norm(hidden, delta or None, weight, eps) -> out: `add_rms_norm` into a new tensor.
+PyObject* rms_norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 4) return PyErr_Format(PyExc_TypeError, "rms_norm: 4 arguments");
+    const at::Tensor *hidden = tensor(args[0]), *delta = tensor(args[1]), *weight = tensor(args[2]);
+    if (!add_rms_norm || !whole(hidden, at::kFloat) || hidden->dim() != 2 || (!delta && args[1] != Py_None) || !weight ||
+        (weight->scalar_type() != at::kBFloat16 && weight->scalar_type() != at::kFloat) || !whole(weight, weight->scalar_type()) ||
+        weight->dim() != 1 || weight->size(0) != hidden->size(1) || (delta && (!whole(delta, weight->scalar_type()) || delta->sizes() != hidden->sizes())))
+        Py_RETURN_NONE;
+    const double eps = PyFloat_AsDouble(args[3]);
+    if (PyErr_Occurred()) return nullptr;
+    at::Tensor out = at::empty(hidden->sizes(), weight->options());
+    if (!ok(add_rms_norm(weight->scalar_type() == at::kBFloat16, at_ptr<float>(*hidden), delta ? delta->data_ptr() : nullptr, weight->data_ptr(),
+                         out.data_ptr(), (int)hidden->size(0), (int)hidden->size(1), (float)eps, 0, stream()), "add_rms_norm"))
+        return nullptr;
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+// prompt_attention(x, qkv_weight, bias, inv_freq, o_weight, tok_seq, tok_pos, slots, cu_q, storage, table, err,
+//                  n_heads, kv_heads, head_dim, n_seqs, max_q_len, max_kv_len, scale, window, write_cache) -> out
+// `qkv_product`, `attention_prefill_tc` and the output projection by the library.
+PyObject* prompt_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 21) return PyErr_Format(PyExc_TypeError, "prompt_attention: 21 arguments");
+    const at::Tensor *x = tensor(args[0]), *w = tensor(args[1]), *bias = tensor(args[2]), *freq = tensor(args[3]), *o = tensor(args[4]);
+    const at::Tensor *seq = tensor(args[5]), *pos = tensor(args[6]), *slots = tensor(args[7]), *cu = tensor(args[8]), *storage = tensor(args[9]);
+    const at::Tensor *table = tensor(args[10]), *err = tensor(args[11]);
+    const long long heads = number(args[12]), kv = number(args[13]), d = number(args[14]), n_seqs = number(args[15]), longest = number(args[16]);
+    const long long keys = number(args[17]), window = number(args[19]), write = number(args[20]);
+    const double scale = PyFloat_AsDouble(args[18]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!qkv_pairs_pays || !qkv_pairs || !prefill_tc || !rows16(x) || !rows16(w) || (!bias && args[2] != Py_None) || (!freq && args[3] != Py_None) ||
+        !o || !o->is_cuda() || o->scalar_type() != at::kBFloat16 || o->dim() != 2 || o->size(1) != heads * d || !whole(seq, at::kInt) ||
+        !whole(pos, at::kInt) || !whole(slots, at::kInt) || !whole(cu, at::kInt) || !whole(storage, at::kBFloat16) || !table || !table->is_cuda() ||
+        table->scalar_type() != at::kInt || !whole(err, at::kInt))
+        Py_RETURN_NONE;
+    const long long m = x->size(0), k = x->size(1), page = storage->stride(0);
+    if ((d != 64 && d != 128) || heads <= 0 || kv <= 0 || heads % kv || w->size(0) != (heads + 2 * kv) * d || w->size(1) != k ||
+        (bias && (!whole(bias, at::kBFloat16) || bias->numel() != w->size(0) || !on16(*bias))) ||
+        (freq && (!whole(freq, at::kFloat) || 2 * freq->numel() != d)) || storage->dim() < 2 || !on16(*storage) || page % 8 ||
+        page != 2 * kv * storage->size(-2) * d || seq->numel() != m || pos->numel() != m || slots->numel() < n_seqs || cu->numel() < n_seqs + 1 ||
+        !qkv_pairs_pays((int)m, (int)w->size(0), (int)k, (int)d))
+        Py_RETURN_NONE;
+    at::Tensor q = at::empty({m, heads * d}, x->options()), attended = at::empty({m, heads * d}, x->options());
+    const QkvArgs a = {bias ? bias->data_ptr() : nullptr, nullptr, ints(pos), ints(seq), ints(slots), q.data_ptr(), storage->data_ptr(), ints(table), page,
+                       (int)table->stride(0), (int)heads, (int)kv, (int)d, write != 0, freq ? freq->const_data_ptr<float>() : nullptr};
+    const Stream s = stream();
+    if (!ok(qkv_pairs(x->data_ptr(), (int)x->stride(0), w->data_ptr(), (int)w->stride(0), (int)m, (int)k, &a, at_ptr<int>(*err), s), "qkv_product") ||
+        !ok(prefill_tc(q.data_ptr(), attended.data_ptr(), ints(cu), ints(pos), ints(slots), storage->data_ptr(), ints(table), page, (int)table->stride(0),
+                       (int)kv, (int)d, (int)heads, (int)n_seqs, (int)m, (int)longest, (int)keys, (float)scale, (int)window, at_ptr<int>(*err), nullptr,
+                       0, s), "attention_prefill_tc"))
+        return nullptr;
+    return THPVariable_Wrap(at::linear(attended, *o));
+    END_HANDLE_TH_ERRORS
+}
+
+// gated_feed_forward(x, gate_up, down, err) -> out: `tc_gemm` with the gate in its epilogue on pairs of SMs, down by the library.
+PyObject* gated_feed_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 4) return PyErr_Format(PyExc_TypeError, "gated_feed_forward: 4 arguments");
+    const at::Tensor *x = tensor(args[0]), *gate_up = tensor(args[1]), *down = tensor(args[2]), *err = tensor(args[3]);
+    if (!tc_gemm || !tc_is_persistent || !rows16(x) || !rows16(gate_up) || !down || !down->is_cuda() || down->scalar_type() != at::kBFloat16 || down->dim() != 2 ||
+        !whole(err, at::kInt))
+        Py_RETURN_NONE;
+    const long long m = x->size(0), k = x->size(1), inter = gate_up->size(0) / 2;
+    if (gate_up->size(0) != 2 * inter || inter % 8 || gate_up->size(1) != k || down->size(1) != inter || !tc_is_persistent(1, (int)m, (int)(2 * inter)))
+        Py_RETURN_NONE;
+    at::Tensor act = at::empty({m, inter}, x->options());
+    if (!ok(tc_gemm(1, x->data_ptr(), (int)x->stride(0), gate_up->data_ptr(), (int)gate_up->stride(0), act.data_ptr(), (int)inter, (int)m, (int)(2 * inter),
+                    (int)k, at_ptr<int>(*err), stream()), "tc_gemm"))
+        return nullptr;
+    return THPVariable_Wrap(at::linear(act, *down));
+    END_HANDLE_TH_ERRORS
+}
+
+// matrix_memory(x, joint, gate_bias, norm, o_weight, state, cu_q, slots, err, heads, dim, vdim, max_q_len, records, each, s_offset, n_offset,
+//               m_offset, cap, eps, floor) -> out: `tc_gemm_tail`, `stabilized_gates`, `state_chunks`, `gated_group_norm` and the output
+// projection by the library. The caller has found the tail and the chunks to be the ways to go; joint is [q | k | v | gate | i | f].
+PyObject* matrix_memory(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 21) return PyErr_Format(PyExc_TypeError, "matrix_memory: 21 arguments");
+    const at::Tensor *x = tensor(args[0]), *joint = tensor(args[1]), *gate_bias = tensor(args[2]), *norm = tensor(args[3]), *o = tensor(args[4]);
+    const at::Tensor *state = tensor(args[5]), *cu = tensor(args[6]), *slots = tensor(args[7]), *err = tensor(args[8]);
+    long long v[9];
+    for (int i = 0; i < 9; ++i) v[i] = number(args[9 + i]);
+    const long long h = v[0], d = v[1], vd = v[2], longest = v[3], records = v[4], each = v[5], s_at = v[6], n_at = v[7], m_at = v[8];
+    const double cap = PyFloat_AsDouble(args[18]), eps = PyFloat_AsDouble(args[19]), floor_add = PyFloat_AsDouble(args[20]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!tc_gemm_tail || !stabilized_gates || !state_chunks || !gated_group_norm || !rows16(x) || !rows16(joint) || !whole(gate_bias, at::kFloat) ||
+        !whole(norm, at::kBFloat16) || !o || !o->is_cuda() || o->scalar_type() != at::kBFloat16 || o->dim() != 2 || !whole(state, at::kFloat) || state->dim() != 2 ||
+        !whole(cu, at::kInt) || !whole(slots, at::kInt) || !whole(err, at::kInt))
+        Py_RETURN_NONE;
+    const long long t = x->size(0), main = 2 * h * (d + vd), inner = h * vd, seqs = cu->numel() - 1, floats = state->size(1);
+    if (h <= 0 || (d != 64 && d != 128) || vd <= 0 || vd % 64 || seqs <= 0 || seqs > 65535 || inner / 64 > 65535 || joint->size(0) != main + 2 * h ||
+        joint->size(1) != x->size(1) || gate_bias->numel() != 2 * h || norm->numel() != inner || o->size(1) != inner || slots->numel() < seqs ||
+        s_at < 0 || s_at + h * d * vd > floats || n_at < 0 || n_at + h * d > floats || m_at < 0 || m_at + h > floats || records <= 0 || each < 0)
+        Py_RETURN_NONE;
+    at::Tensor proj = at::empty({t, main}, x->options()), out = at::empty({t, inner}, x->options());
+    auto round4 = [](long long f) { return (f + 3) / 4 * 4; };     // every buffer on a 16-byte boundary
+    const long long gates = round4(t * h), pre_n = round4(2 * t * h), y_n = round4(t * inner);
+    const long long scratch_n = records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0);
+    at::Tensor room = at::empty({4 * gates + pre_n + y_n + scratch_n}, state->options());
+    float* decay = at_ptr<float>(room);
+    float *take = decay + gates, *floor = take + gates, *nq = floor + gates, *pre = nq + gates, *y = pre + pre_n, *scratch = y + y_n;
+    unsigned char* p = at_ptr<unsigned char>(proj);
+    const unsigned char *q = p, *k = p + 2 * h * d, *vals = p + 4 * h * d, *gate = vals + 2 * inner;
+    const Stream s = stream();
+    const long long slot = state->stride(0);
+    if (!ok(tc_gemm_tail(x->data_ptr(), (int)x->stride(0), joint->data_ptr(), (int)joint->stride(0), p, (int)main, pre, (int)t, (int)main, (int)(2 * h),
+                         (int)x->size(1), at_ptr<int>(*err), s), "tc_gemm_tail") ||
+        !ok(stabilized_gates(pre, (int)(2 * h), gate_bias->const_data_ptr<float>(), (float)cap, ints(cu), ints(slots), (int)seqs, at_ptr<float>(*state), slot,
+                             m_at, (int)h, decay, take, floor, s), "stabilized_gates") ||
+        !ok(state_chunks(q, (int)main, k, (int)main, vals, (int)main, decay, take, nullptr, nullptr, (int)h, ints(cu), ints(slots), (int)seqs, (int)longest,
+                         at_ptr<float>(*state), slot, s_at, n_at, (int)h, (int)h, (int)d, (int)vd, (float)std::pow((double)d, -0.5), scratch, records,
+                         (int)each, y, nq, s), "state_chunks") ||
+        !ok(gated_group_norm(1, y, gate, (int)main, norm->data_ptr(), (float)eps, out.data_ptr(), (int)t, (int)inner, (int)h, (int)h, 0, 0, nq, floor,
+                             (float)floor_add, nullptr, nullptr, 0, s), "gated_group_norm"))
+        return nullptr;
+    return THPVariable_Wrap(at::linear(out, *o));
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {{"setup", (PyCFunction)(void (*)())setup, METH_FASTCALL, nullptr},
+                         {"rms_norm", (PyCFunction)(void (*)())rms_norm, METH_FASTCALL, nullptr},
+                         {"prompt_attention", (PyCFunction)(void (*)())prompt_attention, METH_FASTCALL, nullptr},
+                         {"gated_feed_forward", (PyCFunction)(void (*)())gated_feed_forward, METH_FASTCALL, nullptr},
+                         {"matrix_memory", (PyCFunction)(void (*)())matrix_memory, METH_FASTCALL, nullptr},
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "qf_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_qf_host() { return PyModule_Create(&module); }

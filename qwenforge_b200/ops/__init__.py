@@ -13,6 +13,8 @@ from .kernels import (TC_PLAIN, TC_SWIGLU, QKV_PRODUCT_HEAD_DIMS, tc_gemm, tc_ge
                       retention_chunks, retention_chunks_take, retention_token, retention_rows)
 from .linear import linear, tail_rides, linear_rows, gated_rows, own_tensor_core_products, use_own_tensor_core_products
 
+from . import host  # noqa: E402
+
 __all__ = [
     "pair_rms_norm", "map_difference", "rope_maps_cache_write", "MAP_DIFFERENCE_MAX_VDIM", "PAIR_NORM_ROW_SUM_MAX", "RETENTION_CHUNK", "retention_chunks", "retention_chunks_take", "retention_token", "retention_rows",
     "add_rms_norm_scaled", "residual_add_scaled", "rms_norm_cols", "mix_rows", "bias_glu", "shift_mix", "channel_decay",

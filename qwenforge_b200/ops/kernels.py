@@ -2029,14 +2029,25 @@ STATE_CHUNKS_MIN_TOKENS = 192
 STATE_CHUNKS_COSTS = ((0.09, 0.015, 0.022, 0.25), (14.0, 0.98))
 
 
+def state_chunks_pay(n: int, dim: int, vdim: int, n_heads: int, max_q_len: int, n_seqs: int) -> bool:
+    """Whether the chunked form takes a step of `n` tokens by its sizes and is the faster one (`state_chunks_take` looks at the rows as well)."""
+    return (max_q_len >= STATE_CHUNKS_MIN_TOKENS and dim in (64, 128) and vdim % 64 == 0
+            and n_heads * vdim // 64 <= 65535 and n_seqs <= 65535   # (a grid's second and third extent)
+            and _chunks_pay(n, n_seqs, max_q_len, dim * n_heads * vdim, STATE_CHUNK, *STATE_CHUNKS_COSTS))
+
+
+def state_chunk_records(n: int, n_seqs: int, n_heads: int, dim: int, vdim: int) -> tuple:
+    """(records, chunks of every sequence at a time or 0 for all) of `state_chunks`."""
+    return _chunk_portions(n, n_seqs, STATE_CHUNK, n_heads * (dim * vdim + dim + 1))
+
+
 def state_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dim: int, vdim: int, max_q_len: int, n_seqs: int = 1) -> bool:
     """Whether a step's recurrence runs on `state_chunks`: bfloat16 rows that 16-byte accesses can address, sizes the kernels are
     made for, a sequence long enough (STATE_CHUNKS_MIN_TOKENS) and not too many short ones beside it. Otherwise
     `outer_state_scan` takes it."""
-    return (max_q_len >= STATE_CHUNKS_MIN_TOKENS and dim in (64, 128) and vdim % 64 == 0 and q.dtype == torch.bfloat16 and q.is_cuda
-            and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0
-            and v.shape[1] // 64 <= 65535 and n_seqs <= 65535   # (a grid's second and third extent)
-            and _chunks_pay(q.shape[0], n_seqs, max_q_len, dim * v.shape[1], STATE_CHUNK, *STATE_CHUNKS_COSTS))
+    return (q.dtype == torch.bfloat16 and q.is_cuda and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0
+            and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0
+            and state_chunks_pay(q.shape[0], dim, vdim, v.shape[1] // vdim, max_q_len, n_seqs))
 
 
 def state_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: Optional[torch.Tensor], take: Optional[torch.Tensor],
@@ -2065,7 +2076,7 @@ def state_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: Optio
     if q.dtype != torch.bfloat16:
         raise KernelError("state_chunks: bfloat16 rows only (state_chunks_take)")
     n_seqs = cu_q.numel() - 1
-    records, each = _chunk_portions(n, n_seqs, STATE_CHUNK, n_heads * (dim * vdim + dim + 1))
+    records, each = state_chunk_records(n, n_seqs, n_heads, dim, vdim)
     carry = n_seqs * n_heads * (dim * vdim + dim) if each else 0
     scratch = torch.empty(records * n_heads * (dim * vdim + dim + 1) + carry, dtype=torch.float32, device=q.device)
     _check(library("state_chunks").qf_state_chunks(

@@ -300,9 +300,19 @@ class GqaAttention(Mixer):
         plan = self.decode_plan(ctx) if fast and ctx.is_decode else None
         rotary = self.position.fused_rotary() if self.position is not None else None
         inv_freq, rot_dim = rotary if rotary is not None else (None, 0)
+        late_bias = self.position is None or rotary is not None  # the kernel that rotates and stores adds the bias
+        prefill = None
+        if fast and not ctx.is_decode:
+            prefill = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window, max_q_len=ctx.max_q_len, n_seqs=ctx.n_seqs,
+                                        n_heads=self.n_heads, kv_heads=self.n_kv)
+            if late_bias and self.o_bias_t is None and prefill is ops.kernels.attention_prefill_tc:
+                # the three steps below, issued from native code
+                out = ops.host.prompt_attention(x, self.qkv_weight, self.qkv_bias_t, inv_freq, self.o_weight, ctx, site, self.n_heads, self.n_kv,
+                                                self.head_dim, self.scale, self.window, writes_cache)
+                if out is not None:
+                    return out
         q = torch.empty((n, self.q_width), dtype=x.dtype, device=x.device)
         args = ops.KvSiteArgs(site.storage, site.table, self.n_kv, self.head_dim)
-        late_bias = self.position is None or rotary is not None  # the kernel that rotates and stores adds the bias
         if (fast and late_bias and ops.qkv_product_takes(x, self.qkv_weight, rot_dim, args)
                 and ops.qkv_product_pays(n, self.qkv_weight, self.head_dim)):
             ops.qkv_product(x, self.qkv_weight, self.qkv_bias_t, inv_freq, ctx.tok_seq, ctx.tok_pos, ctx.slots, self.n_heads, q, args,
@@ -320,8 +330,6 @@ class GqaAttention(Mixer):
             ops.attention_decode(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,
                                  self.scale, self.window, self.decode_splits(ctx), ctx.decode_scratch, ctx.err, plan)
         elif fast:
-            prefill = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window, max_q_len=ctx.max_q_len, n_seqs=ctx.n_seqs,
-                                        n_heads=self.n_heads, kv_heads=self.n_kv)
             prefill(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,
                     ctx.max_q_len, self.scale, self.window, ctx.err, max_kv_len=ctx.max_kv_len)
         else:

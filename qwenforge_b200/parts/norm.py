@@ -34,6 +34,10 @@ class RmsNorm(Norm):
     def forward(self, hidden: torch.Tensor, delta) -> torch.Tensor:
         """delta: None, a tensor, or a `PendingScaled` (outputs that enter the stream under a factor each, added by this
         norm's kernel on its way)."""
+        if not isinstance(delta, PendingScaled):
+            out = ops.host.rms_norm(hidden, delta, self.weight, self.eps)
+            if out is not None:
+                return out
         out = torch.empty(hidden.shape, dtype=self.weight.dtype, device=hidden.device)
         if isinstance(delta, PendingScaled):
             ops.add_rms_norm_scaled(hidden, delta.a, delta.scale_a, delta.b, delta.scale_b, self.weight, self.eps, out)

@@ -117,6 +117,11 @@ class MatrixMemory(Mixer):
         if not writes_cache:
             raise ValueError("matrix_memory: a recurrent state cannot be read from another schedule entry")
         n, h, d, v = x.shape[0], self.n_heads, self.dim, self.vdim
+        if n > ops.WIDE_MAX_ROWS and x.dtype == torch.bfloat16:   # the step below where it runs in chunks, issued from native code
+            out = ops.host.matrix_memory(x, self.joint_weight, self.gate_bias, self.norm, self.o_weight, ctx, site.storage, h, d, v,
+                                         (self.s_offset, self.n_offset, self.m_offset), self.cap, self.eps, self.floor)
+            if out is not None:
+                return out
         f32 = dict(dtype=torch.float32, device=x.device)
         # [T, q | k | v | g] and [T, i | f], float32 sums
         proj, pre = _linear_and_tail(x, self.joint_weight, self.proj_weight, self.gate_weight, ctx.err)

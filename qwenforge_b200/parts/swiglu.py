@@ -37,6 +37,10 @@ class SwiGlu(FeedForward):
         return [self.gate_up_weight, self.down_weight]
 
     def forward(self, x, ctx):
+        if ctx is not None and x.dtype == torch.bfloat16:   # the two products below where the first has its gate inside, issued from native code
+            out = ops.host.gated_feed_forward(x, self.gate_up_weight, self.down_weight, ctx.err)
+            if out is not None:
+                return out
         act = torch.empty((x.shape[0], self.inter), dtype=x.dtype, device=x.device)
         # Steps with tiles for every SM run gate/up with the gate in the product's epilogue on this library's
         # persistent tcgen05 kernel: measured at 2048 x 9728 x 896 it takes 27 microseconds where the library product

@@ -1,0 +1,119 @@
+"""What native code launches (csrc/host.cpp) is what the Python entries launch one by one: the same bits, and their way where it steps aside."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+STRETCHES = ("rms_norm", "prompt_attention", "gated_feed_forward", "matrix_memory")
+
+
+def _model(preset, layer=None):
+    from qwenforge_b200.config import config_from_dict, preset_config
+    from qwenforge_b200.engine import Model
+    if layer is None:
+        return Model.from_random(preset_config(preset, num_hidden_layers=1, vocab_size=128), 5)
+    kept = preset_config(preset).to_dict()
+    kept["layers"] = [dict(next(entry for entry in kept["layers"] if entry["type"] == layer), mlp=None)]
+    kept["vocab"] = 128
+    return Model.from_random(config_from_dict(kept), 5)
+
+
+def _step(model, lengths, before):
+    from qwenforge_b200.cache import SequenceCache
+    from qwenforge_b200.engine import build_context
+    cache = SequenceCache(model.cache_needs(), sum(-(-(n + before) // 64) * 64 for n in lengths), len(lengths), model.spec.max_positions, model.dtype, model.device)
+    slots = [cache.open() for _ in lengths]
+    cache.reserve([(s, n + before) for s, n in zip(slots, lengths)])
+    cache.flush()
+    ctx = build_context([(s, before, np.zeros(n, dtype=np.int32)) for s, n in zip(slots, lengths)], None, model.err, model.dtype, model.device,
+                        model.attention, model.decode_scratch)
+    ctx.step_memo = {}
+    return cache.site(0), ctx
+
+
+def _watch(monkeypatch, on):
+    """Which stretches native code took, by name; `on` False: none."""
+    from qwenforge_b200 import ops
+    took = []
+    for name in STRETCHES:
+        real = getattr(ops.host, name)
+
+        def watched(*args, name=name, real=real):
+            out = real(*args) if on else None
+            if out is not None:
+                took.append(name)
+            return out
+        monkeypatch.setattr(ops.host, name, watched)
+    return took
+
+
+# (tokens beyond the 64 of the decode form, too few for gate/up on pairs, the benchmark's, unequal and with a portion before, heads of 128)
+@pytest.mark.parametrize("preset,lengths,before,taken", [
+    ("qwen2.5-0.5b", [65], 0, {"rms_norm"}), ("qwen2.5-0.5b", [300], 0, {"rms_norm", "prompt_attention"}),
+    ("qwen2.5-0.5b", [2048], 0, {"rms_norm", "prompt_attention", "gated_feed_forward"}),
+    ("qwen2.5-0.5b", [201, 517, 133], 70, {"rms_norm", "prompt_attention", "gated_feed_forward"}),
+    ("qwen2.5-3b", [700], 0, {"rms_norm", "prompt_attention", "gated_feed_forward"})])
+def test_a_layer(preset, lengths, before, taken, monkeypatch):
+    model = _model(preset)
+    x = torch.randn(sum(lengths), model.blocks[0].mixer.hidden, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV)
+    pending = torch.randn(x.shape, generator=torch.Generator(device=DEV).manual_seed(2), device=DEV).bfloat16()
+    results = []
+    for on in (True, False):
+        with monkeypatch.context() as patch:
+            took = _watch(patch, on)
+            site, ctx = _step(model, lengths, before)
+            site.storage.zero_()
+            stream = x.clone()
+            delta = model.blocks[0].forward(stream, pending, ctx, site, True)
+        results.append((stream, delta, site.storage.clone()))
+        if on:
+            assert set(took) >= taken - {"prompt_attention"} and ("gated_feed_forward" in took) == ("gated_feed_forward" in taken)
+        else:
+            assert not took
+    model.raise_on_kernel_error()
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("lengths,taken", [([100], False), ([192], True), ([2048], True), ([700, 193, 5], True)])
+def test_a_matrix_memory(lengths, taken, monkeypatch):
+    model = _model("zebovik-0.5b", "mlstm")
+    mixer, results = model.blocks[0].mixer, []
+    x = torch.randn(sum(lengths), mixer.hidden, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).bfloat16()
+    for on in (True, False):
+        with monkeypatch.context() as patch:
+            took = _watch(patch, on)
+            site, ctx = _step(model, lengths, 0)
+            outs = [mixer.forward(x, ctx, site, True) for _ in range(2)]
+        results.append((*outs, site.storage.clone()))
+        assert ("matrix_memory" in took) == (on and taken)
+    model.raise_on_kernel_error()
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+def test_whoever_replaces_a_kernel_sees_its_calls():
+    from qwenforge_b200.ops.timing import KernelTimer
+    model = _model("qwen2.5-0.5b")
+    site, ctx = _step(model, [2048], 0)
+    with KernelTimer() as timer:
+        model.blocks[0].forward(torch.randn(2048, 896, device=DEV), None, ctx, site, True)
+    seen = [label.split("[")[0] for label, *_ in timer.records]
+    assert sorted(seen) == sorted(["add_rms_norm", "qkv_product", "attention_prefill_tc", "linear", "add_rms_norm", "tc_gemm", "linear"])
+
+
+def test_what_is_not_taken():
+    from qwenforge_b200 import ops
+    hidden, weight = torch.randn(8, 64, device=DEV), torch.ones(64, device=DEV).bfloat16()
+    assert ops.host.rms_norm(hidden, None, weight, 1e-6) is not None
+    assert ops.host.rms_norm(hidden.t().contiguous().t(), None, weight, 1e-6) is None                  # rows that are not contiguous
+    assert ops.host.rms_norm(hidden, hidden, weight, 1e-6) is None                                     # a pending output of another type
+    assert ops.host.rms_norm(hidden, None, weight.as_subclass(type("Other", (torch.Tensor,), {})), 1e-6) is None   # a subclass of tensor
+    assert ops.host.rms_norm(hidden.cpu(), None, weight, 1e-6) is None
+    x, gate_up, down = torch.randn(2048, 896, device=DEV).bfloat16(), torch.randn(9728, 896, device=DEV).bfloat16(), torch.randn(896, 4864, device=DEV).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    assert ops.host.gated_feed_forward(x, gate_up, down, err) is not None
+    assert ops.host.gated_feed_forward(x[:16], gate_up, down, err) is None                             # too few tiles
+    assert ops.host.gated_feed_forward(x[:, :892], gate_up[:, :892], down, err) is None                # a K of no whole pieces of eight
+    assert ops.host.gated_feed_forward(x, gate_up, down[:, :4856], err) is None                        # shapes that do not agree
