@@ -265,7 +265,7 @@ __global__ void attention_generic_fold_kernel(T* __restrict__ out, const int* __
 // a load from shared memory feeds four multiply-adds (in the kernel above: one). Every score is one chain over the components,
 // every output one chain over the keys in rising order, pages at multiples of 64, so a row's arithmetic depends on its own
 // position and window only, as above and whatever RT (the two kernels differ by rounding). What bounds it is the
-// multiply-add pipe and the walk of the longest tile: one prompt of 1,031 tokens, 14 heads of 64: 893 -> 102 microseconds.
+// multiply-add pipe and the walk of the longest tile: one prompt of 1,031 tokens, 14 heads of 64: 893 -> 96 microseconds.
 // `wave` > 0: that many blocks (one for every SM) start at a time, longest walks first, the next ones in rising order, so that an SM's
 // second block is the shorter the longer its first is (118 microseconds there with all in falling order).
 #define FT_THREADS 256
@@ -325,7 +325,10 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
     fetch(k_s, page_begin, 0);
     fetch(v_s, page_begin, 1);
 
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    // Neighbouring lanes share tx: a warp's 16-byte loads of 16 keys' (or columns') pieces then take two cycles of the shared memory, four with tx
+    // in the low bits. Microseconds, so / with tx there: 14 heads of 64, 200 tokens 19.7 / 23.4, 500 35.9 / 43.0, 1,031 95.6 / 103.8, 2,048 247 / 266;
+    // 16 heads of 128, 200 27.9 / 34.0, 1,031 156 / 167; the same bits.
+    const int tx = threadIdx.x >> 1 & 15, ty = (threadIdx.x >> 5) * 2 + (threadIdx.x & 1);
     float m[RT], l[RT], o[RT][DT];
     int pos[RT], lo[RT];
 #pragma unroll
@@ -377,7 +380,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
                 top = fmaxf(top, s[r][j]);
             }
 #pragma unroll
-            for (int w = 8; w > 0; w >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, w));
+            for (int w = 16; w > 1; w >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, w));
             const float m_new = fmaxf(m[r], top), alpha = expf(m[r] - m_new);
             float sum = 0.f;
 #pragma unroll
@@ -387,7 +390,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
                 sum += p;
             }
 #pragma unroll
-            for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+            for (int w = 16; w > 1; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
             l[r] = l[r] * alpha + sum;
             m[r] = m_new;
 #pragma unroll
