@@ -23,7 +23,10 @@ __device__ __forceinline__ float2 halves(f32x2 x) {
 }
 
 // A block makes a BM x BN tile with WM x WN warps; a warp makes (4 TM) x (8 TN) of it, its 4 x 8 lanes TM x TN each in runs of four rows
-// and columns, so that the lanes of a warp read a k's rows and columns of both operands as whole 16-byte pieces without conflicts. 16
+// (two, where a lane's are no whole fours) and columns, so that the lanes of a warp read a k's rows and columns of both operands as whole
+// pieces without conflicts. Which rows and columns a lane has: neighbouring lanes share one of the two, and a 16-byte load of eight pieces takes two cycles of
+// the shared memory, four where eight neighbours have eight (32 x 64 tiles 12 to 15% faster so, the larger ones up to 2%; 64 x 64 in few rounds
+// 1.5% slower, so not there). 16
 // or 32 columns of K at a time, the next ones on their way through registers: they are turned on the way into shared memory, where
 // the rows of every eight k are swapped among themselves so that a warp's stores of four k a lane meet all 32 banks. Rows go two to
 // a register pair, and a column's number twice into one.
@@ -36,12 +39,14 @@ __global__ void __launch_bounds__(32 * WM * WN, TM * TN >= 128 ? 256 / (32 * WM 
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                 float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int vec) {
     constexpr int THREADS = 32 * WM * WN, BM = 4 * TM * WM, BN = 8 * TN * WN, LA = BM + 4, LW = BN + 4, Q = BK / 4, SWAP = BK == 16 ? 8 : 4;
-    constexpr int A_EACH = BM * Q / THREADS, W_EACH = BN * Q / THREADS;
-    static_assert(TM % 4 == 0 && TN % 4 == 0 && BM * Q % THREADS == 0 && BN * Q % THREADS == 0 && BM % 16 == 0 && BN % 16 == 0, "whole runs of four");
+    constexpr int A_EACH = (BM * Q + THREADS - 1) / THREADS, W_EACH = (BN * Q + THREADS - 1) / THREADS, RA = TM % 4 ? 2 : 4, RW = TN % 4 ? 2 : 4;
+    static_assert(TM % 2 == 0 && TN % 2 == 0 && BM % 16 == 0 && BN % 16 == 0, "whole runs");
     __shared__ __align__(16) float a_s[2][BK][LA], w_s[2][BK][LW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int row0 = (warp / WN) * 4 * TM + (lane >> 3) * 4, col0 = (warp % WN) * 8 * TN + (lane & 7) * 4;
+    constexpr bool SHARED = !(TM == 8 && TN == 4);
+    const int row0 = (warp / WN) * 4 * TM + (SHARED ? lane >> 1 & 3 : lane >> 3) * RA;
+    const int col0 = (warp % WN) * 8 * TN + (SHARED ? (lane & 1) | (lane >> 2 & 6) : lane & 7) * RW;
     f32x2 acc[TM / 2][TN];            // rows 2 i and 2 i + 1 of column j
 #pragma unroll
     for (int i = 0; i < TM / 2; ++i)
@@ -69,24 +74,26 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 #pragma unroll
         for (int u = 0; u < A_EACH; ++u) {
             const int i = threadIdx.x + u * THREADS;
-            a_next[u] = piece(A, lda, m0 + i / Q, M, k0 + (i % Q) * 4);
+            a_next[u] = piece(A, lda, BM * Q % THREADS == 0 || i < BM * Q ? m0 + i / Q : M, M, k0 + (i % Q) * 4);
         }
 #pragma unroll
         for (int u = 0; u < W_EACH; ++u) {
             const int i = threadIdx.x + u * THREADS;
-            w_next[u] = piece(W, ldw, n0 + i / Q, N, k0 + (i % Q) * 4);
+            w_next[u] = piece(W, ldw, BN * Q % THREADS == 0 || i < BN * Q ? n0 + i / Q : N, N, k0 + (i % Q) * 4);
         }
     };
     auto stash = [&](int buf) {
         const int k = (threadIdx.x % Q) * 4, swap = k / 8 * SWAP;
 #pragma unroll
         for (int u = 0; u < A_EACH; ++u) {
+            if (BM * Q % THREADS && threadIdx.x + u * THREADS >= BM * Q) continue;
             const int r = ((threadIdx.x + u * THREADS) / Q) ^ swap;
             a_s[buf][k][r] = a_next[u].x, a_s[buf][k + 1][r] = a_next[u].y;
             a_s[buf][k + 2][r] = a_next[u].z, a_s[buf][k + 3][r] = a_next[u].w;
         }
 #pragma unroll
         for (int u = 0; u < W_EACH; ++u) {
+            if (BN * Q % THREADS && threadIdx.x + u * THREADS >= BN * Q) continue;
             const int r = ((threadIdx.x + u * THREADS) / Q) ^ swap;
             w_s[buf][k][r] = w_next[u].x, w_s[buf][k + 1][r] = w_next[u].y;
             w_s[buf][k + 2][r] = w_next[u].z, w_s[buf][k + 3][r] = w_next[u].w;
@@ -102,14 +109,16 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
             f32x2 a[TM / 2];
             float w[TN];
 #pragma unroll
-            for (int i = 0; i < TM; i += 4) {   // runs of four rows, 16 rows apart
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&a_s[buf][k][(row0 + 4 * i) ^ (k / 8 * SWAP)]);
-                a[i / 2] = v.x, a[i / 2 + 1] = v.y;
+            for (int i = 0; i < TM; i += RA) {
+                const float* p = &a_s[buf][k][(row0 + 4 * i) ^ (k / 8 * SWAP)];
+                if (RA == 4) { const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p); a[i / 2] = v.x, a[(i / 2 + 1) % (TM / 2)] = v.y; }
+                else a[i / 2] = *reinterpret_cast<const f32x2*>(p);
             }
 #pragma unroll
-            for (int j = 0; j < TN; j += 4) {   // runs of four columns, 32 columns apart
-                const float4 v = *reinterpret_cast<const float4*>(&w_s[buf][k][(col0 + 8 * j) ^ (k / 8 * SWAP)]);
-                w[j] = v.x, w[j + 1] = v.y, w[j + 2] = v.z, w[j + 3] = v.w;
+            for (int j = 0; j < TN; j += RW) {
+                const float* p = &w_s[buf][k][(col0 + 8 * j) ^ (k / 8 * SWAP)];
+                if (RW == 4) { const float4 v = *reinterpret_cast<const float4*>(p); w[j] = v.x, w[j + 1] = v.y, w[(j + 2) % TN] = v.z, w[(j + 3) % TN] = v.w; }
+                else { const float2 v = *reinterpret_cast<const float2*>(p); w[j] = v.x, w[j + 1] = v.y; }
             }
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
@@ -127,12 +136,12 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     for (int i = 0; i < TM / 2; ++i) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int gm = m0 + row0 + (i / 2) * 16 + (2 * i) % 4 + h;
+            const int gm = m0 + row0 + 2 * i / RA * 4 * RA + (2 * i) % RA + h;
             if (gm >= M) continue;
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
                 const float2 v = halves(acc[i][j]);
-                const int gn = n0 + col0 + (j / 4) * 32 + j % 4;
+                const int gn = n0 + col0 + j / RW * 8 * RW + j % RW;
                 if (gn < N) C[(size_t)gm * ldc + gn] = (h ? v.y : v.x) + (bias ? bias[gn] : 0.f);
             }
         }
@@ -222,16 +231,17 @@ gemm_f32_few_rows_kernel(const float* __restrict__ A, const float* __restrict__ 
 
 // The tile with which the busiest SM is done first: a first wait and a time per tile, measured at K = 896 in microseconds (1, 4 and 18
 // tiles per SM of 64 x 64 33, 92 and 380, of 32 x 64 24, 65 and 258; 1, 5 and 9 of 128 x 128 89, 385 and 683; 1, 6 and 12 of 96 x 128
-// 72, 339 and 662; 1, 2 and 12 of 96 x 64 47, 74 and 382). Never the fastest by more than a twentieth: 64 x 128 and 64 x 256 with two
+// 72, 339 and 662; 1, 2 and 12 of 96 x 64 47, 74 and 382; 1 and 8 of 96 x 96 61 and 371: 1,031 x 1,152 x 896 in one round of them 61
+// microseconds, in three of 64 x 64 73). Never the fastest by more than a twentieth: 64 x 128 and 64 x 256 with two
 // or four warps, 32 x 64 with two warps, 128 x 64. (With K a tile's time grows and its wait does not: the waits, which count here as at
 // K = 896, decide between tiles whose rounds take nearly the same time.)
-static const struct { int bm, bn; float wait, each; } f32_tiles[] = {{96, 128, 18.f, 53.7f}, {128, 128, 13.5f, 74.5f}, {96, 64, 15.f, 30.6f},
-                                                                     {64, 64, 8.5f, 20.8f}, {32, 64, 8.f, 14.3f}};
+static const struct { int bm, bn; float wait, each; } f32_tiles[] = {{96, 128, 18.f, 53.7f}, {128, 128, 13.5f, 74.5f}, {96, 64, 15.f, 30.f},
+                                                                     {64, 64, 8.5f, 20.8f}, {32, 64, 8.f, 14.3f}, {96, 96, 17.f, 44.2f}};
 static int best_tile(int M, int N) {
     const int sms = qf_sm_count() > 0 ? qf_sm_count() : 1;
     int best = 0;
     float least = 0.f;
-    for (int i = 0; i < 5; ++i) {
+    for (int i = 0; i < 6; ++i) {
         const long long count = (long long)((M + f32_tiles[i].bm - 1) / f32_tiles[i].bm) * ((N + f32_tiles[i].bn - 1) / f32_tiles[i].bn);
         const float time = f32_tiles[i].wait + (float)((count + sms - 1) / sms) * f32_tiles[i].each;
         if (i == 0 || time < least) best = i, least = time;
@@ -257,7 +267,8 @@ QF_EXPORT int qf_gemm_f32(const float* A, const float* W, const float* bias, flo
     else if (best == 1) QF_F32(16, 8, 16);
     else if (best == 2) QF_F32(12, 4, 16);
     else if (best == 3) QF_F32(8, 4, 32);
-    else QF_F32(4, 4, 32);
+    else if (best == 4) QF_F32(4, 4, 32);
+    else QF_F32(12, 6, 16);
 #undef QF_F32
     return (int)cudaGetLastError();
 }
