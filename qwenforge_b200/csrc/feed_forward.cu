@@ -6,7 +6,7 @@
 // reductions of it into `sums`, float32 [rows][width]. As two kernels (skinny_gemm.cu) the activations went through the L2 behind a second
 // kernel's launch. What bounds it is that chain, then the reductions, blocks x rows x width / 4 of them (218,000 for eight rows of 896 x 4,864; a
 // row: 5.4 microseconds from the end of the kernel ahead to its own, 8.9 for the two kernels). A decode step at Qwen2.5-0.5B sizes, microseconds,
-// two kernels / this one: 1 sequence of 1,024 tokens 624 / 547, 4 662 / 566, 8 670 / 595; 1 of 4,000 626 / 532, 8 671 / 642.
+// two kernels / this one: 1 sequence of 1,024 tokens 626 / 517, 4 660 / 534, 8 671 / 564; 1 of 4,000 627 / 511, 8 669 / 609.
 // `sums` is a buffer of its own, zero before the launch: added into the stream in place, a block's share would reach rows that other blocks are
 // still reading. The next layer's QKV product reads stream and sums together, and its output projection (fold_project.cu) moves the sums into
 // the stream and leaves zeros. The shares arrive in no fixed order, as there.
@@ -42,7 +42,7 @@ __device__ __forceinline__ void mma_bf16_16808(float (&d)[4], uint32_t a0, uint3
 __global__ void __launch_bounds__(FF_THREADS, 1) feed_forward_kernel(const FeedForwardArgs a) {
     extern __shared__ __align__(16) unsigned char ff_smem[];
     __shared__ __align__(8) uint64_t w_bar[1];
-    __shared__ float ss_s[FF_WARPS];
+    __shared__ float ss_s[FF_WARPS], inv_s[FF_MAX_ROWS];
     const int wide = ff_stride(a.width), narrow = ff_stride(a.cols);
     unsigned char* w_s = ff_smem;                                  // [2 * cols][wide]: eight gate rows, the same eight up rows, ...
     unsigned char* x_s = w_s + (size_t)2 * a.cols * wide;          // [8][wide]
@@ -116,6 +116,11 @@ __global__ void __launch_bounds__(FF_THREADS, 1) feed_forward_kernel(const FeedF
         if (lane == 0) ss_s[warp] = ss;
     }
     __syncthreads();
+    if (threadIdx.x >= FF_THREADS - 32 && lane < a.rows) {         // (read behind the next barriers)
+        float ss = 0.f;
+        for (int p = 0; p < share; ++p) ss += ss_s[lane * share + p];
+        inv_s[lane] = 1.0f / sqrtf(ss / (float)a.width + a.eps);
+    }
     if (!mbar_wait(&w_bar[0], 0) && lane == 0) atomicOr(a.err, QF_ERR_COPY_TIMEOUT);
 
     // ---- gate and up: a tile is eight columns, its M side their gate and their up rows; the warps of a tile take blocks of 32 k in turn
@@ -150,9 +155,7 @@ __global__ void __launch_bounds__(FF_THREADS, 1) feed_forward_kernel(const FeedF
             const int m = 2 * t + e;
             float out = 0.f;
             if (m < a.rows) {
-                float ss = 0.f;
-                for (int p = 0; p < share; ++p) ss += ss_s[m * share + p];
-                const float inv = 1.0f / sqrtf(ss / (float)a.width + a.eps), gate = sum[e] * inv, up = sum[2 + e] * inv;
+                const float gate = sum[e] * inv_s[m], up = sum[2 + e] * inv_s[m];
                 out = gate / (1.0f + expf(-gate)) * up;
             }
             *reinterpret_cast<bf16*>(act_s + (size_t)m * narrow + (warp * 8 + g) * 2) = __float2bfloat16_rn(out);

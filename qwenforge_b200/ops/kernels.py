@@ -1084,8 +1084,8 @@ FEED_FORWARD_MAX_REDUCTIONS = 250_000
 def feed_forward_takes(rows: int, gate_up: torch.Tensor, down: torch.Tensor) -> bool:
     """Whether `feed_forward` takes `rows` rows of a SwiGLU layer [gate | up] [2 I, W], down [W, I] and is the faster way: bfloat16 weights
     whose shares find room in the SMs' shared memory, and no more than 250,000 16-byte reductions (blocks x rows x W / 4). The reductions
-    grow with the rows and what one kernel saves does not: at 896 x 4,864 (122 blocks) a decode step gains 12 to 15 percent with 1 to 4 rows
-    (27,000 to 109,000 reductions) and 4 to 14 with 8 (218,000); more have not been measured. Two products otherwise."""
+    grow with the rows and what one kernel saves does not: at 896 x 4,864 (122 blocks) a decode step gains 15 to 20 percent with 1 to 4 rows
+    (27,000 to 109,000 reductions) and 9 to 17 with 8 (218,000); more have not been measured. Two products otherwise."""
     if not (gate_up.is_cuda and down.is_cuda and gate_up.dtype == torch.bfloat16 and down.dtype == torch.bfloat16 and rows <= 8):
         return False
     width, inter = down.shape
