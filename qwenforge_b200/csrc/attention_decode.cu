@@ -228,11 +228,13 @@ decode_split_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16* __re
         mbar_init(&bars[warp][1], 1);
     }
     __syncwarp();
+    // the warp's first 32 page numbers, a lane each: looked up one by one they were a round trip behind the wait for every further page
+    const int my_table = lane < my_pages ? table_row[p_begin + warp + lane * DEC_WARPS] : -1;
     auto half_live = [&](int i, int& page, int& key0) {
         if (i >= n_halves) return false;
         const int p = p_begin + warp + (i >> 1) * DEC_WARPS;
         key0 = p * QF_PAGE + (i & 1) * HALF;
-        page = table_row[p];
+        page = (i >> 1) < 32 ? __shfl_sync(0xffffffffu, my_table, i >> 1) : table_row[p];
         if (page < 0) {
             if (lane == 0 && (i & 1) == 0) atomicOr(err, QF_ERR_NO_PAGE);
             return false;
