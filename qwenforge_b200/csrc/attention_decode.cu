@@ -703,16 +703,21 @@ QF_EXPORT long long qf_attention_decode_plan_size(int n_seqs, int kv_heads, int 
 
 // The plan of one step for attention of this shape (see decode_plan_kernel); the same plan serves every layer of the
 // step that has this shape. `n_splits` is the most runs that one sequence may get.
-QF_EXPORT int qf_attention_decode_plan_masked(const int* cu_q, const int* tok_pos, const int* slots, int n_seqs, int kv_heads,
+// `leave`: block slots that the plan does not fill, for blocks of the kernel behind that find no room beside one of these.
+QF_EXPORT int qf_attention_decode_plan_leaving(const int* cu_q, const int* tok_pos, const int* slots, int n_seqs, int kv_heads,
                                               int head_dim, int n_heads, int window, int n_splits, void* plan, int mask_block,
-                                              cudaStream_t stream) {
+                                               int leave, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     if (kv_heads <= 0 || n_heads % kv_heads || n_splits < 1 || n_splits > 0x7fff || !qf_attention_decode_warps(head_dim))
         return (int)cudaErrorInvalidValue;
     const int kvc = kv_heads * ((n_heads / kv_heads + 15) / 16);
     return (int)launch_pdl(decode_plan_kernel, dim3(1), dim3(32), 0, stream, cu_q, tok_pos, slots, n_seqs, kvc,
-                           decode_slots(head_dim), qf_attention_decode_warps(head_dim), window, n_splits, (int4*)plan,
+                           std::max(decode_slots(head_dim) - std::max(leave, 0), 1), qf_attention_decode_warps(head_dim), window, n_splits, (int4*)plan,
                            (int)plan_pairs(n_seqs, kv_heads, n_heads, head_dim, n_splits), mask_block);
+}
+QF_EXPORT int qf_attention_decode_plan_masked(const int* cu_q, const int* tok_pos, const int* slots, int n_seqs, int kv_heads, int head_dim, int n_heads,
+                                              int window, int n_splits, void* plan, int mask_block, cudaStream_t stream) {
+    return qf_attention_decode_plan_leaving(cu_q, tok_pos, slots, n_seqs, kv_heads, head_dim, n_heads, window, n_splits, plan, mask_block, 0, stream);
 }
 
 QF_EXPORT int qf_attention_decode_plan(const int* cu_q, const int* tok_pos, const int* slots, int n_seqs, int kv_heads,

@@ -483,12 +483,12 @@ def attention_decode_warps(head_dim: int) -> int:
 
 def attention_decode_plan(cu_q: torch.Tensor, tok_pos: torch.Tensor, slots: torch.Tensor, kv_heads: int, head_dim: int,
                           n_heads: int, n_seqs: int, window: int, n_splits: int, scratch: DecodeScratch,
-                          chunk: int = 0) -> torch.Tensor:
+                          chunk: int = 0, leave: int = 0) -> torch.Tensor:
     """The plan of one decode step for attention of this shape: which block takes which run of which sequence, worked
     out on the device from the batch's lengths (sequences of unequal lengths get blocks of about equal work; a batch
     that fills the SMs unsplit stays unsplit). One plan serves every layer of the step with this shape. `n_splits` is
-    the most runs one sequence may get. The tensor belongs to `scratch` and is overwritten by the next plan of the
-    same shape."""
+    the most runs one sequence may get; `leave` block slots stay free for the kernel behind. The tensor belongs to `scratch` and is
+    overwritten by the next plan of the same shape."""
     for name, t in (("cu_q", cu_q), ("tok_pos", tok_pos), ("slots", slots)):
         _dev(name, t, torch.int32)
     if not 1 <= n_splits <= 128:
@@ -500,9 +500,9 @@ def attention_decode_plan(cu_q: torch.Tensor, tok_pos: torch.Tensor, slots: torc
     records = int(lib.qf_attention_decode_plan_size(_I(n_seqs), _I(kv_heads), _I(n_heads), _I(head_dim), _I(n_splits)))
     if records <= 0:
         raise KernelError(f"attention_decode: head_dim {head_dim} has no tensor-core kernel (have {FAST_ATTENTION_HEAD_DIMS})")
-    plan = scratch.plan((n_seqs, kv_heads, n_heads, head_dim, window, n_splits, chunk), records)
-    _check(lib.qf_attention_decode_plan_masked(_ptr(cu_q), _ptr(tok_pos), _ptr(slots), _I(n_seqs), _I(kv_heads), _I(head_dim),
-                                               _I(n_heads), _I(window), _I(n_splits), _ptr(plan), _I(int(chunk)), _stream()),
+    plan = scratch.plan((n_seqs, kv_heads, n_heads, head_dim, window, n_splits, chunk) + ((int(leave),) if leave else ()), records)
+    _check(lib.qf_attention_decode_plan_leaving(_ptr(cu_q), _ptr(tok_pos), _ptr(slots), _I(n_seqs), _I(kv_heads), _I(head_dim),
+                                               _I(n_heads), _I(window), _I(n_splits), _ptr(plan), _I(int(chunk)), _I(int(leave)), _stream()),
            "attention_decode_plan")
     return plan
 

@@ -66,9 +66,13 @@ class SwiGlu(FeedForward):
         return (ctx.dtype == torch.bfloat16 and ctx.attention == "auto" and self.inter % 8 == 0
                 and ctx.n_tokens <= ops.WIDE_MAX_ROWS and self._ways(ctx) != ("unfused", "unfused"))
 
+    def leaves_sums(self, hidden, ctx) -> bool:
+        """Whether `fused_forward` with nothing pending runs as one kernel and returns a `PendingSums`."""
+        return ctx.step_memo is not None and ops.feed_forward_takes(hidden.shape[0], self.gate_up_weight, self.down_weight)
+
     def fused_forward(self, hidden, rms, ctx, delta=None):
         """Adds to the stream, or returns what is still to reach it."""
-        if delta is None and ctx.step_memo is not None and ops.feed_forward_takes(hidden.shape[0], self.gate_up_weight, self.down_weight):
+        if delta is None and self.leaves_sums(hidden, ctx):
             # the whole layer out of the SMs' shared memory, in one kernel; its output stands in rows of its own that all layers share
             key = ("swiglu.sums", tuple(hidden.shape))
             sums = ctx.step_memo.get(key)

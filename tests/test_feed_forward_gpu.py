@@ -107,3 +107,28 @@ def test_the_qkv_product_reads_stream_and_sums(rows):
         # (hidden - rest) + rest is hidden to a rounding of 2^-24; results lie one step of eight bits apart at most
         assert float((got.float() - want.float()).abs().max()) <= 2.0 ** -7 * float(want.float().abs().max())
         assert float((got.float() - want.float()).norm()) <= 2.0 ** -9 * float(want.float().norm())
+
+
+@pytest.mark.parametrize("lengths", [[4100] * 8, [1] * 8, [700], [4100, 64, 65, 3000]])
+def test_a_plan_that_leaves_slots(lengths):
+    """No more runs than fit beside what is left free (or one a sequence); the attention of either plan."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.measure import Pages
+    heads, kv, dim, leave, n = 14, 2, 64, 14, len(lengths)
+    g = torch.Generator(device=DEV).manual_seed(n)
+    pages = Pages(n, max(lengths), kv, dim, DEV)
+    pages.storage.normal_(generator=g)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q, err = torch.randn(n, heads * dim, generator=g, device=DEV).bfloat16(), ints([0])
+    cu, pos, slots, splits = ints(list(range(n + 1))), ints([x - 1 for x in lengths]), ints(list(range(n))), max(1, -(-max(lengths) // 512))
+    outs, runs = [], []
+    for free in (0, leave):
+        scratch, out = ops.DecodeScratch(torch.device(DEV)), torch.empty_like(q)
+        plan = ops.attention_decode_plan(cu, pos, slots, kv, dim, heads, n, 0, splits, scratch, leave=free)
+        ops.attention_decode(q, out, cu, pos, slots, pages.args(), heads, n, dim ** -0.5, 0, splits, scratch, err, plan)
+        runs.append(plan.flatten()[:n].tolist())
+        outs.append(out.float())
+    assert int(err) == 0
+    assert sum(runs[1]) * kv <= max(ops.sm_count(DEV) - leave, n * kv) and all(b <= a for a, b in zip(*runs))
+    # both are sums of the same weighted values with weights in bfloat16, rounded to bfloat16
+    assert float((outs[0] - outs[1]).norm()) < 2.0 ** -7 * float(outs[0].norm())
