@@ -2045,8 +2045,8 @@ def state_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dim: in
     """Whether a step's recurrence runs on `state_chunks`: bfloat16 rows that 16-byte accesses can address, sizes the kernels are
     made for, a sequence long enough (STATE_CHUNKS_MIN_TOKENS) and not too many short ones beside it. Otherwise
     `outer_state_scan` takes it."""
-    return (q.dtype == torch.bfloat16 and q.is_cuda and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0
-            and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0
+    return (max_q_len >= STATE_CHUNKS_MIN_TOKENS and q.dtype == torch.bfloat16 and q.is_cuda
+            and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0
             and state_chunks_pay(q.shape[0], dim, vdim, v.shape[1] // vdim, max_q_len, n_seqs))
 
 
@@ -2536,16 +2536,27 @@ ROW_CHUNKS_MIN_TOKENS = 512
 ROW_CHUNKS_COSTS = ((0.13, 0.0, 0.04, 0.2), (20.0, 1.3))
 
 
+def row_chunks_pay(n: int, dim: int, vdim: int, n_heads: int, max_q_len: int, n_seqs: int) -> bool:
+    """Whether the chunked form takes a step of `n` tokens by its sizes and is the faster one (`row_chunks_take` looks at the rows as well)."""
+    return (max_q_len >= ROW_CHUNKS_MIN_TOKENS and dim == 64 and vdim % 64 == 0 and vdim <= 512
+            and n_heads * vdim // 64 <= 65535 and n_seqs <= 65535   # (a grid's second and third extent)
+            and _chunks_pay(n, n_seqs, max_q_len, dim * n_heads * vdim, ROW_CHUNK, *ROW_CHUNKS_COSTS))
+
+
+def row_chunk_records(n: int, n_seqs: int, n_heads: int, dim: int, vdim: int) -> tuple:
+    """(records, chunks of every sequence at a time or 0 for all) of `row_chunks`."""
+    return _chunk_portions(n, n_seqs, ROW_CHUNK, n_heads * (dim * vdim + dim))
+
+
 def row_chunks_take(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, dim: int, vdim: int, max_q_len: int,
                     n_seqs: int = 1) -> bool:
     """Whether a step's recurrence with a decay per row runs on `row_chunks`: bfloat16 rows that 16-byte accesses can address, 64 rows and
     whole 64 columns (up to 512) of a head's state, a sequence long enough and not too many short ones beside it. Otherwise
     `outer_state_scan_rows` takes it."""
-    return (max_q_len >= ROW_CHUNKS_MIN_TOKENS and dim == 64 and vdim % 64 == 0 and vdim <= 512 and q.dtype == torch.bfloat16 and q.is_cuda
+    return (max_q_len >= ROW_CHUNKS_MIN_TOKENS and q.dtype == torch.bfloat16 and q.is_cuda
             and (q.stride(0) | k.stride(0) | v.stride(0)) % 8 == 0
             and (q.data_ptr() | k.data_ptr() | v.data_ptr() | decay.data_ptr()) % 16 == 0
-            and v.shape[1] // 64 <= 65535 and n_seqs <= 65535   # (a grid's second and third extent)
-            and _chunks_pay(q.shape[0], n_seqs, max_q_len, dim * v.shape[1], ROW_CHUNK, *ROW_CHUNKS_COSTS))
+            and row_chunks_pay(q.shape[0], dim, vdim, v.shape[1] // vdim, max_q_len, n_seqs))
 
 
 def row_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, cu_q: torch.Tensor, slots: torch.Tensor,
@@ -2558,7 +2569,7 @@ def row_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     if q.dtype != torch.bfloat16:
         raise KernelError("row_chunks: bfloat16 rows only (row_chunks_take)")
     n, n_seqs = q.shape[0], cu_q.numel() - 1
-    records, each = _chunk_portions(n, n_seqs, ROW_CHUNK, n_heads * (dim * vdim + dim))
+    records, each = row_chunk_records(n, n_seqs, n_heads, dim, vdim)
     carry = n_seqs * n_heads * dim * vdim if each else 0
     scratch = torch.empty(records * n_heads * (dim * vdim + dim) + carry + (n * n_heads * dim if kind else 0), dtype=torch.float32,
                           device=q.device)

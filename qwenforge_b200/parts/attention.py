@@ -306,7 +306,7 @@ class GqaAttention(Mixer):
             prefill = prefill_attention(self.head_dim, n, ctx.max_kv_len, self.window, max_q_len=ctx.max_q_len, n_seqs=ctx.n_seqs,
                                         n_heads=self.n_heads, kv_heads=self.n_kv)
             if late_bias and self.o_bias_t is None and prefill is ops.kernels.attention_prefill_tc:
-                # the three steps below, issued from native code
+                # what follows, issued from native code
                 out = ops.host.prompt_attention(x, self.qkv_weight, self.qkv_bias_t, inv_freq, self.o_weight, ctx, site, self.n_heads, self.n_kv,
                                                 self.head_dim, self.scale, self.window, writes_cache)
                 if out is not None:

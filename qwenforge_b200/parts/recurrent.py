@@ -117,7 +117,7 @@ class MatrixMemory(Mixer):
         if not writes_cache:
             raise ValueError("matrix_memory: a recurrent state cannot be read from another schedule entry")
         n, h, d, v = x.shape[0], self.n_heads, self.dim, self.vdim
-        if n > ops.WIDE_MAX_ROWS and x.dtype == torch.bfloat16:   # the step below where it runs in chunks, issued from native code
+        if n > ops.WIDE_MAX_ROWS and ctx.max_q_len >= ops.kernels.STATE_CHUNKS_MIN_TOKENS and x.dtype == torch.bfloat16:   # the step below where it runs in chunks, from native code
             out = ops.host.matrix_memory(x, self.joint_weight, self.gate_bias, self.norm, self.o_weight, ctx, site.storage, h, d, v,
                                          (self.s_offset, self.n_offset, self.m_offset), self.cap, self.eps, self.floor)
             if out is not None:
@@ -193,6 +193,11 @@ class StateSpace(Mixer):
         if not writes_cache:
             raise ValueError("state_space: a recurrent state cannot be read from another schedule entry")
         n, h, v, s, g = x.shape[0], self.n_heads, self.vdim, self.n_state, self.groups
+        if n > ops.WIDE_MAX_ROWS and ctx.max_q_len >= ops.kernels.STATE_CHUNKS_MIN_TOKENS and x.dtype == torch.bfloat16:   # the step below where it runs in chunks, from native code
+            out = ops.host.state_space(x, self.joint_weight, self.conv_weight, self.conv_bias, self.dt_bias, self.rate_log, self.skip, self.norm, self.o_weight,
+                                       ctx, site.storage, h, v, s, g, self.norm_parts, (self.s_offset, self.conv_offset), self.eps)
+            if out is not None:
+                return out
         f32 = dict(dtype=torch.float32, device=x.device)
         # [T, z | x | B | C] and [T, H], float32 sums
         main, dt_pre = _linear_and_tail(x, self.joint_weight, self.main_weight, self.dt_weight, ctx.err)
@@ -373,6 +378,11 @@ class GatedLinearAttention(Mixer):
             proj = ops.linear_rows(x, self.proj_weight)
             join(main, side, pre)
         elif x.dtype == torch.bfloat16 and n > ops.WIDE_MAX_ROWS and self.rank % 8 == 0:   # long steps: the pair's middle as further columns
+            # (where the step runs in chunks, all of it is issued from native code)
+            out = None if ctx.max_q_len < ops.kernels.ROW_CHUNKS_MIN_TOKENS else ops.host.gated_linear_attention(
+                x, self.joint_weight, self.a2, self.a2_bias, self.norm, self.o_weight, ctx, site.storage, h, d, v, self.tau, self.eps)
+            if out is not None:
+                return out
             joint = ops.linear(x, self.joint_weight)                                     # [T, q | k | v | g | middle]
             proj, low = joint[:, :-self.rank], joint[:, -self.rank:]
             pre = ops.linear_rows(low, self.a2, out_dtype=torch.float32)                 # float32 sums

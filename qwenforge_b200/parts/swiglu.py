@@ -37,7 +37,7 @@ class SwiGlu(FeedForward):
         return [self.gate_up_weight, self.down_weight]
 
     def forward(self, x, ctx):
-        if ctx is not None and x.dtype == torch.bfloat16:   # the two products below where the first has its gate inside, issued from native code
+        if ctx is not None and x.dtype == torch.bfloat16:   # what follows, issued from native code
             out = ops.host.gated_feed_forward(x, self.gate_up_weight, self.down_weight, ctx.err)
             if out is not None:
                 return out
