@@ -117,7 +117,8 @@ class MatrixMemory(Mixer):
         if not writes_cache:
             raise ValueError("matrix_memory: a recurrent state cannot be read from another schedule entry")
         n, h, d, v = x.shape[0], self.n_heads, self.dim, self.vdim
-        if n > ops.WIDE_MAX_ROWS and ctx.max_q_len >= ops.kernels.STATE_CHUNKS_MIN_TOKENS and x.dtype == torch.bfloat16:   # the step below where it runs in chunks, from native code
+        # the step below where it runs in chunks, issued from native code
+        if n > ops.WIDE_MAX_ROWS and ctx.max_q_len >= ops.kernels.STATE_CHUNKS_MIN_TOKENS and x.dtype == torch.bfloat16:
             out = ops.host.matrix_memory(x, self.joint_weight, self.gate_bias, self.norm, self.o_weight, ctx, site.storage, h, d, v,
                                          (self.s_offset, self.n_offset, self.m_offset), self.cap, self.eps, self.floor)
             if out is not None:
@@ -193,7 +194,8 @@ class StateSpace(Mixer):
         if not writes_cache:
             raise ValueError("state_space: a recurrent state cannot be read from another schedule entry")
         n, h, v, s, g = x.shape[0], self.n_heads, self.vdim, self.n_state, self.groups
-        if n > ops.WIDE_MAX_ROWS and ctx.max_q_len >= ops.kernels.STATE_CHUNKS_MIN_TOKENS and x.dtype == torch.bfloat16:   # the step below where it runs in chunks, from native code
+        # the step below where it runs in chunks, issued from native code
+        if n > ops.WIDE_MAX_ROWS and ctx.max_q_len >= ops.kernels.STATE_CHUNKS_MIN_TOKENS and x.dtype == torch.bfloat16:
             out = ops.host.state_space(x, self.joint_weight, self.conv_weight, self.conv_bias, self.dt_bias, self.rate_log, self.skip, self.norm, self.o_weight,
                                        ctx, site.storage, h, v, s, g, self.norm_parts, (self.s_offset, self.conv_offset), self.eps)
             if out is not None:
