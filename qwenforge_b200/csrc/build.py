@@ -15,7 +15,8 @@ One source, `host.cpp`, is a Python module instead (`host_module()`): it launche
 same way, against the headers of the torch in use, whose version is part of its name.
 
 There is no fallback: if nvcc is missing or a compilation fails, `KernelLibraryError`
-says which file and why, and nothing runs.
+says which file and why, and nothing runs. `host.cpp` alone can be done without: it needs Python's and torch's C++ headers, which a
+machine with nvcc may lack, and what it launches can be launched one by one (`ops/host.py`).
 """
 from __future__ import annotations
 
@@ -39,6 +40,7 @@ _NVCC_FLAGS = [
 _HOST = "host"           # the one source that is a Python module
 _loaded: dict[str, ctypes.CDLL] = {}
 _modules: dict = {}
+_unavailable: dict = {}  # what was tried and could not be had, and why: not tried again in this process
 _lock = threading.Lock()
 
 
@@ -183,40 +185,60 @@ def library(name: str) -> ctypes.CDLL:
 
 def host_module():
     """The module of `host.cpp` (compiling it first if no current build exists); a kernel library's address is handed to it by whoever
-    loads one (`ops/host.py`)."""
+    loads one (`ops/host.py`). `KernelLibraryError` where it cannot be built or loaded, at every call and tried once."""
     module = _modules.get(_HOST)
     if module is None:
         with _lock:
             module = _modules.get(_HOST)
             if module is None:
-                import importlib.machinery
-                import importlib.util
-
-                import torch  # noqa: F401  (its libraries are what the module is linked against)
-                path = str(_compile(_HOST))
-                loader = importlib.machinery.ExtensionFileLoader("qf_host", path)
+                if _HOST in _unavailable:
+                    raise KernelLibraryError(_unavailable[_HOST])
                 try:
-                    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("qf_host", path, loader=loader))
-                    loader.exec_module(module)
-                except ImportError as exc:
-                    raise KernelLibraryError(f"cannot load {path}: {exc}") from exc
-                _modules[_HOST] = module
+                    module = _modules[_HOST] = _load_module(_compile(_HOST))
+                except KernelLibraryError as exc:
+                    _unavailable[_HOST] = str(exc)
+                    _say(f"no native launches of prompt steps (they only save time): {exc}")
+                    raise
     return module
 
 
-def prepare(names) -> None:
+def _load_module(path: Path):
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries are what the module is linked against)
+    loader = importlib.machinery.ExtensionFileLoader("qf_host", str(path))
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("qf_host", str(path), loader=loader))
+        loader.exec_module(module)
+    except ImportError as exc:
+        raise KernelLibraryError(f"cannot load {path}: {exc}") from exc
+    return module
+
+
+def prepare(names, optional=()) -> None:
     """Compile (in parallel) and load the named libraries; used when a model is built, so
-    that all compilation happens up front with progress lines instead of inside the first step."""
-    todo = [n for n in sorted(set(names)) if n not in _loaded and n not in _modules]
+    that all compilation happens up front with progress lines instead of inside the first step. One of `optional` that cannot be had
+    is left out."""
+    left_out = set(optional) - set(names)
+    todo = [n for n in sorted(set(names) | left_out) if n not in _loaded and n not in _modules and not (n in left_out and n in _unavailable)]
     if not todo:
         return
+
+    def get(n: str, how) -> None:
+        try:
+            host_module() if n == _HOST else how(n)
+        except KernelLibraryError:
+            if n not in left_out:
+                raise
+
     missing = [n for n in todo if _find_built(n, _digest(n)) is None]
     if missing:
         _say(f"{len(missing)} kernel librar{'y' if len(missing) == 1 else 'ies'} to compile: {', '.join(missing)}")
         with ThreadPoolExecutor(max_workers=min(8, len(missing))) as pool:
-            list(pool.map(_compile, missing))
+            list(pool.map(lambda n: get(n, _compile), missing))
     for n in todo:
-        host_module() if n == _HOST else library(n)
+        get(n, library)
 
 
 def build_all() -> list[str]:

@@ -2,7 +2,7 @@
 
 Every function answers None, having launched nothing, for what it does not take; the caller then launches the kernels one by one, where the
 same condition is reported or another kernel chosen. So do they while one of these kernels' names in `ops` is not the function of
-`ops.kernels`: whoever puts something in its place (`ops.timing.KernelTimer`) sees every call.
+`ops.kernels`: whoever puts something in its place (`ops.timing.KernelTimer`) sees every call; and where the native module cannot be built.
 """
 from __future__ import annotations
 
@@ -12,7 +12,7 @@ from typing import Optional
 
 import torch
 
-from ..csrc import host_module, library
+from ..csrc import KernelLibraryError, host_module, library
 from . import kernels
 from .linear import linear, linear_rows, own_tensor_core_products, tail_rides
 
@@ -26,10 +26,13 @@ _OWN = {"linear_rows": linear_rows, "tail_rides": tail_rides}   # (of `ops.linea
 
 
 def _host(*libraries: str):
-    """The native module, told the entries of these kernel libraries."""
+    """The native module, told the entries of these kernel libraries; None where it cannot be had (`host_module` has said why)."""
     global _module
     if _module is None:
-        _module = host_module()
+        try:
+            _module = host_module()
+        except KernelLibraryError:
+            return None
     for name in libraries:
         if name not in _known:
             loaded = library(name)
@@ -44,7 +47,10 @@ def _untouched(*names: str) -> bool:
     return ops.linear is linear and all(getattr(ops, name) is (_OWN.get(name) or getattr(kernels, name)) for name in names)
 
 
-def _counted(out: Optional[torch.Tensor], launches: int) -> Optional[torch.Tensor]:
+def _launch(name: str, launches: int, libraries: tuple, *args) -> Optional[torch.Tensor]:
+    """The native module's function `name`; the kernels of this package that it launched are counted."""
+    module = _host(*libraries)
+    out = None if module is None else getattr(module, name)(*args)
     if out is not None:
         kernels.launches += launches
     return out
@@ -54,7 +60,7 @@ def rms_norm(hidden: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.
     """`add_rms_norm` into a new tensor."""
     if not (hidden.is_cuda and _untouched("add_rms_norm")):
         return None
-    return _counted(_host("norm").rms_norm(hidden, delta, weight, eps), 1)
+    return _launch("rms_norm", 1, ("norm",), hidden, delta, weight, eps)
 
 
 def prompt_attention(x: torch.Tensor, qkv_weight: torch.Tensor, bias: Optional[torch.Tensor], inv_freq: Optional[torch.Tensor], o_weight: torch.Tensor,
@@ -64,9 +70,10 @@ def prompt_attention(x: torch.Tensor, qkv_weight: torch.Tensor, bias: Optional[t
     if not (x.is_cuda and _untouched("qkv_product", "qkv_product_takes", "qkv_product_pays", "rope_cache_write", "attention_prefill_tc")) \
             or own_tensor_core_products(x, o_weight) or own_tensor_core_products(x, qkv_weight):
         return None
-    return _counted(_host("tc_gemm", "rope_cache", "attention_prefill_tc").prompt_attention(
+    return _launch(
+        "prompt_attention", 2, ("tc_gemm", "rope_cache", "attention_prefill_tc"),
         x, qkv_weight, bias, inv_freq, o_weight, ctx.tok_seq, ctx.tok_pos, ctx.slots, ctx.cu_q, site.storage, site.table, ctx.err, n_heads, kv_heads,
-        head_dim, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len, scale, window, int(bool(write_cache))), 2)
+        head_dim, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len, scale, window, int(bool(write_cache)))
 
 
 def gated_feed_forward(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, err: torch.Tensor) -> Optional[torch.Tensor]:
@@ -74,7 +81,7 @@ def gated_feed_forward(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
     if not (x.is_cuda and _untouched("tc_gemm", "tc_gemm_takes", "tc_gemm_is_persistent", "swiglu")) or own_tensor_core_products(x, down) \
             or own_tensor_core_products(x, gate_up):
         return None
-    return _counted(_host("tc_gemm", "activation").gated_feed_forward(x, gate_up, down, err), 1)
+    return _launch("gated_feed_forward", 1, ("tc_gemm", "activation"), x, gate_up, down, err)
 
 
 def matrix_memory(x: torch.Tensor, joint: torch.Tensor, gate_bias: torch.Tensor, norm: torch.Tensor, o_weight: torch.Tensor, ctx, state: torch.Tensor,
@@ -89,9 +96,10 @@ def matrix_memory(x: torch.Tensor, joint: torch.Tensor, gate_bias: torch.Tensor,
     if not tail_rides(x, joint, 2 * n_heads * (dim + vdim)):
         return None
     records, each = kernels.state_chunk_records(n, ctx.n_seqs, n_heads, dim, vdim)
-    return _counted(_host("tc_gemm", "recurrent", "state_chunks").matrix_memory(
+    return _launch(
+        "matrix_memory", 4, ("tc_gemm", "recurrent", "state_chunks"),
         x, joint, gate_bias, norm, o_weight, state, ctx.cu_q, ctx.slots, ctx.err, n_heads, dim, vdim, ctx.max_q_len, records, each, *offsets,
-        cap, eps, floor), 4)
+        cap, eps, floor)
 
 
 def state_space(x: torch.Tensor, joint: torch.Tensor, conv_weight: torch.Tensor, conv_bias: torch.Tensor, dt_bias: torch.Tensor, rate_log: torch.Tensor,
@@ -107,9 +115,10 @@ def state_space(x: torch.Tensor, joint: torch.Tensor, conv_weight: torch.Tensor,
     if not tail_rides(x, joint, joint.shape[0] - n_heads):
         return None
     records, each = kernels.state_chunk_records(n, ctx.n_seqs, n_heads, n_state, vdim)
-    return _counted(_host("tc_gemm", "recurrent", "state_chunks").state_space(
+    return _launch(
+        "state_space", 4, ("tc_gemm", "recurrent", "state_chunks"),
         x, joint, conv_weight, conv_bias, dt_bias, rate_log, skip, norm, o_weight, state, ctx.cu_q, ctx.tok_seq, ctx.slots, ctx.err, n_heads, vdim, n_state,
-        groups, norm_parts, ctx.max_q_len, records, each, *offsets, eps), 4)
+        groups, norm_parts, ctx.max_q_len, records, each, *offsets, eps)
 
 
 def gated_linear_attention(x: torch.Tensor, joint: torch.Tensor, a2: torch.Tensor, a2_bias: torch.Tensor, norm: torch.Tensor, o_weight: torch.Tensor, ctx,
@@ -122,5 +131,6 @@ def gated_linear_attention(x: torch.Tensor, joint: torch.Tensor, a2: torch.Tenso
             or own_tensor_core_products(x, o_weight) or own_tensor_core_products(x, joint):
         return None
     records, each = kernels.row_chunk_records(n, ctx.n_seqs, n_heads, dim, vdim)
-    return _counted(_host("recurrent", "row_chunks").gated_linear_attention(
-        x, joint, a2, a2_bias, norm, o_weight, state, ctx.cu_q, ctx.slots, n_heads, dim, vdim, ctx.max_q_len, records, each, 1.0 / tau, eps), 2)
+    return _launch(
+        "gated_linear_attention", 2, ("recurrent", "row_chunks"),
+        x, joint, a2, a2_bias, norm, o_weight, state, ctx.cu_q, ctx.slots, n_heads, dim, vdim, ctx.max_q_len, records, each, 1.0 / tau, eps)
