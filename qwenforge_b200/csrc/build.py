@@ -216,32 +216,31 @@ def _load_module(path: Path):
     return module
 
 
-def prepare(names, optional=()) -> None:
+def prepare(names) -> None:
     """Compile (in parallel) and load the named libraries; used when a model is built, so
-    that all compilation happens up front with progress lines instead of inside the first step. One of `optional` that cannot be had
-    is left out."""
-    left_out = set(optional) - set(names)
-    todo = [n for n in sorted(set(names) | left_out) if n not in _loaded and n not in _modules and not (n in left_out and n in _unavailable)]
+    that all compilation happens up front with progress lines instead of inside the first step. The one that can be done without is
+    left out where it cannot be had (`host_module` says so)."""
+    todo = [n for n in sorted(set(names)) if n not in _loaded and n not in _modules and n not in _unavailable]
     if not todo:
         return
 
-    def get(n: str, how) -> None:
+    def host() -> None:
         try:
-            host_module() if n == _HOST else how(n)
+            host_module()
         except KernelLibraryError:
-            if n not in left_out:
-                raise
+            pass
 
     missing = [n for n in todo if _find_built(n, _digest(n)) is None]
     if missing:
         _say(f"{len(missing)} kernel librar{'y' if len(missing) == 1 else 'ies'} to compile: {', '.join(missing)}")
         with ThreadPoolExecutor(max_workers=min(8, len(missing))) as pool:
-            list(pool.map(lambda n: get(n, _compile), missing))
+            list(pool.map(lambda n: host() if n == _HOST else _compile(n), missing))
     for n in todo:
-        get(n, library)
+        host() if n == _HOST else library(n)
 
 
 def build_all() -> list[str]:
     names = library_names()
     prepare(names)
+    host_module()   # (whoever builds everything hears of it)
     return names

@@ -84,10 +84,10 @@ class Model:
         ops.require_cuda(self.device, "the model")
         if self.device.type == "cuda" and self.device.index is not None:
             torch.cuda.set_device(self.device)  # the kernels launch on the current device's current stream
-        libraries = {"embed", "norm"}
+        libraries = {"embed", "norm", "host"}
         for part in self.parts():
             libraries |= part.kernel_libraries(self.dtype)
-        prepare(libraries, optional={"host"})
+        prepare(libraries)
         for part in self.parts():
             part.bind(tensors, self.dtype, self.device)
         self.err = torch.zeros(1, dtype=torch.int32, device=self.device)
