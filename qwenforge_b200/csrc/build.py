@@ -57,15 +57,23 @@ def _source(name: str) -> Path:
 
 
 def _flags(name: str) -> list[str]:
+    """What makes a build what it is; where the headers and libraries lie is `_places`' part."""
     if name != _HOST:
         return _NVCC_FLAGS
+    import torch
+    return ["-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
+def _places(name: str) -> list[str]:
+    if name != _HOST:
+        return ["-I", str(_SRC)]
     import sysconfig
 
     import torch
     root = Path(torch.__file__).resolve().parent
-    return ["-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-            "-I", sysconfig.get_paths()["include"], "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
-            "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    return ["-I", sysconfig.get_paths()["include"], "-I", str(root / "include"), "-I", str(root / "include/torch/csrc/api/include"),
+            "-L", str(root / "lib")]
 
 
 def _say(message: str) -> None:
@@ -110,9 +118,8 @@ def _digest(name: str) -> str:
     h = hashlib.sha256()
     if name == _HOST:
         import torch
-        h.update(f"{torch.__version__} {sys.version}".encode())
-    else:
-        h.update(" ".join(_NVCC_FLAGS).encode())
+        h.update(f"{torch.__version__} {sys.version} ".encode())
+    h.update(" ".join(_flags(name)).encode())
     shared = [] if name == _HOST else sorted(_SRC.glob("*.cuh")) + sorted(_SRC.glob("*.h"))
     for path in shared + [_source(name)]:
         h.update(path.name.encode())
@@ -143,7 +150,7 @@ def _compile(name: str) -> Path:
     out_dir = _build_dir()
     target = out_dir / f"{name}.{digest}.so"
     partial = out_dir / f".{name}.{digest}.{os.getpid()}.{threading.get_ident()}.tmp.so"
-    command = [_nvcc(), *_flags(name), "-I", str(_SRC), "-o", str(partial), str(source)]
+    command = [_nvcc(), *_places(name), *_flags(name), "-o", str(partial), str(source)]
     _say(f"compiling {source.name} for sm_100a ...")
     started = time.time()
     env = dict(os.environ)

@@ -37,3 +37,10 @@ def test_its_functions_answer_none_without_it(monkeypatch):
     before, rows = ops.kernels.launches, SimpleNamespace(is_cuda=True)
     assert ops.host.rms_norm(rows, None, None, 1e-6) is None and ops.host.rms_norm(rows, None, None, 1e-6) is None
     assert tried == ["host"] and ops.kernels.launches == before
+
+
+@pytest.mark.parametrize("name", ["host", "norm"])
+def test_changed_flags_are_another_build(name, monkeypatch):
+    before, flags = build._digest(name), build._flags
+    monkeypatch.setattr(build, "_flags", lambda which: [*flags(which), "-DANOTHER"])
+    assert build._digest(name) != before
