@@ -215,7 +215,8 @@ class PendingScaled(Pending):
 
 class PendingSums(Pending):
     """A feed-forward's output in float32 rows of their own (`ops.feed_forward`), zeros again once it is in the stream. A decode step's
-    QKV product reads the stream and these rows together, and its output projection moves them into the stream."""
+    QKV product reads the stream and these rows together, and its output projection moves them into the stream. All layers of a step
+    share the rows: they have to reach the stream (`add_to`, or a block that takes them) before the next layer's feed-forward."""
     __slots__ = ("sums",)
 
     def __init__(self, sums: torch.Tensor):
@@ -226,7 +227,7 @@ class PendingSums(Pending):
         ops.take_sums(hidden, self.sums)
 
     def value(self) -> torch.Tensor:
-        return self.sums
+        return self.sums.clone()   # (the next layer leaves zeros in the rows)
 
 
 class PendingNormed(Pending):
