@@ -298,7 +298,7 @@ PyObject* gated_linear_attention(PyObject*, PyObject* const* args, Py_ssize_t n)
         slots->numel() < seqs || h * d * vd > state->size(1) || records <= 0 || each < 0)
         Py_RETURN_NONE;
     at::Tensor all = at::linear(*x, *joint), pre = at::mm(all.narrow(1, main, rank), a2->t(), at::kFloat), out = at::empty({m, inner}, x->options());
-    if (!on16(all) || !on16(pre) || !pre.is_contiguous()) Py_RETURN_NONE;
+    TORCH_CHECK(on16(all) && on16(pre) && pre.is_contiguous(), "gated_linear_attention: the allocator's rows begin on no 16-byte boundary");
     const long long y_n = m * inner;
     at::Tensor room = at::empty({y_n + records * h * (d * vd + d) + (each ? seqs * h * d * vd : 0) + m * h * d}, state->options());
     float *y = at_ptr<float>(room), *scratch = y + y_n;
