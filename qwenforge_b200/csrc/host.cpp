@@ -83,6 +83,10 @@ bool on16(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()
 bool rows16(const at::Tensor* t) {
     return t && t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 2 && t->stride(1) == 1 && t->size(1) % 8 == 0 && t->stride(0) % 8 == 0 && on16(*t);
 }
+// Floats of a buffer, up to whole 256 bytes, where small buffers share an allocation. The large ones, rows in float32 and the chunks' records,
+// have allocations of their own: a state space of 28 heads, microseconds of a pass, one allocation of parts on 16 bytes / on 256 / apart: 5,003
+// tokens 203.5 / 196.8 / 195.5, 2,501 and 2,500 202.4 / 194.7 / 193.6 (a warp's loads meet a fifth line, its stores straddle sectors).
+long long whole_lines(long long floats) { return (floats + 63) / 64 * 64; }
 Stream stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 bool ok(int code, const char* what) {
     if (code == 0) return true;
@@ -203,12 +207,11 @@ PyObject* matrix_memory(PyObject*, PyObject* const* args, Py_ssize_t n) {
         s_at < 0 || s_at + h * d * vd > floats || n_at < 0 || n_at + h * d > floats || m_at < 0 || m_at + h > floats || records <= 0 || each < 0)
         Py_RETURN_NONE;
     at::Tensor proj = at::empty({t, main}, x->options()), out = at::empty({t, inner}, x->options());
-    auto round4 = [](long long f) { return (f + 3) / 4 * 4; };     // every buffer on a 16-byte boundary
-    const long long gates = round4(t * h), pre_n = round4(2 * t * h), y_n = round4(t * inner);
-    const long long scratch_n = records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0);
-    at::Tensor room = at::empty({4 * gates + pre_n + y_n + scratch_n}, state->options());
+    const long long gates = whole_lines(t * h);
+    at::Tensor room = at::empty({6 * gates}, state->options()), made = at::empty({t * inner}, state->options());
+    at::Tensor kept = at::empty({records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0)}, state->options());
     float* decay = at_ptr<float>(room);
-    float *take = decay + gates, *floor = take + gates, *nq = floor + gates, *pre = nq + gates, *y = pre + pre_n, *scratch = y + y_n;
+    float *take = decay + gates, *floor = take + gates, *nq = floor + gates, *pre = nq + gates, *y = at_ptr<float>(made), *scratch = at_ptr<float>(kept);
     unsigned char* p = at_ptr<unsigned char>(proj);
     const unsigned char *q = p, *k = p + 2 * h * d, *vals = p + 4 * h * d, *gate = vals + 2 * inner;
     const Stream s = stream();
@@ -255,9 +258,9 @@ PyObject* state_space(PyObject*, PyObject* const* args, Py_ssize_t n) {
         conv_at + (taps - 1) * channels > state->size(1) || records <= 0 || each < 0)
         Py_RETURN_NONE;
     at::Tensor made = at::empty({m, main}, x->options()), mixed = at::empty({m, channels}, x->options()), out = at::empty({m, inner}, x->options());
-    const long long dt_n = (m * h + 3) / 4 * 4, y_n = m * inner;     // (every buffer on a 16-byte boundary: inner is a multiple of 64)
-    at::Tensor room = at::empty({dt_n + y_n + records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0)}, state->options());
-    float *dt = at_ptr<float>(room), *y = dt + dt_n, *scratch = y + y_n;
+    at::Tensor pre = at::empty({m * h}, state->options()), sums = at::empty({m * inner}, state->options());
+    at::Tensor kept = at::empty({records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0)}, state->options());
+    float *dt = at_ptr<float>(pre), *y = at_ptr<float>(sums), *scratch = at_ptr<float>(kept);
     const unsigned char *z = at_ptr<unsigned char>(made), *vals = at_ptr<unsigned char>(mixed), *k = vals + 2 * inner, *q = k + 2 * groups * d;
     const Stream s = stream();
     const long long slot = state->stride(0);
@@ -299,9 +302,9 @@ PyObject* gated_linear_attention(PyObject*, PyObject* const* args, Py_ssize_t n)
         Py_RETURN_NONE;
     at::Tensor all = at::linear(*x, *joint), pre = at::mm(all.narrow(1, main, rank), a2->t(), at::kFloat), out = at::empty({m, inner}, x->options());
     TORCH_CHECK(on16(all) && on16(pre) && pre.is_contiguous(), "gated_linear_attention: the allocator's rows begin on no 16-byte boundary");
-    const long long y_n = m * inner;
-    at::Tensor room = at::empty({y_n + records * h * (d * vd + d) + (each ? seqs * h * d * vd : 0) + m * h * d}, state->options());
-    float *y = at_ptr<float>(room), *scratch = y + y_n;
+    at::Tensor sums = at::empty({m * inner}, state->options());
+    at::Tensor kept = at::empty({records * h * (d * vd + d) + (each ? seqs * h * d * vd : 0) + m * h * d}, state->options());
+    float *y = at_ptr<float>(sums), *scratch = at_ptr<float>(kept);
     const unsigned char *q = at_ptr<unsigned char>(all), *k = q + 2 * h * d, *vals = k + 2 * h * d, *gate = vals + 2 * inner;
     const Stream s = stream();
     if (!ok(row_chunks(q, (int)wide, k, (int)wide, vals, (int)wide, pre.const_data_ptr<float>(), bias->const_data_ptr<float>(), 2, (float)inv_tau, nullptr, ints(cu),

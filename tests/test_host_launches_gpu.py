@@ -95,6 +95,38 @@ def test_a_recurrent_mixer(preset, layer, stretch, lengths, monkeypatch):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("layer", ["mlstm", "mamba2"])
+def test_buffers_of_one_allocation_begin_on_whole_lines(layer):
+    """Heads x tokens of no whole line: the addresses that the kernels are given (by entries that write them down and launch nothing)."""
+    import ctypes
+
+    from qwenforge_b200 import ops
+    from qwenforge_b200.csrc import library
+    p, i, n, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    entries = {"qf_stabilized_gates": ("recurrent", (p, i, p, f, p, p, i, p, n, n, i, p, p, p, p), (0, 11, 12, 13)),
+               "qf_state_chunks": ("state_chunks", (p, i, p, i, p, i, p, p, p, p, i, p, p, i, i, p, n, n, n, i, i, i, i, f, p, n, i, p, p, p), (24, 27, 28)),
+               "qf_gated_group_norm": ("recurrent", (i, p, p, i, p, f, p, i, i, i, i, i, i, p, p, f, p, p, i, p), (1, 6, 13, 14))}
+    model = _model("zebovik-0.5b", layer)
+    mixer, seen, kept = model.blocks[0].mixer, [], []
+    x = torch.randn(701, mixer.hidden, device=DEV).bfloat16()
+    site, ctx = _step(model, [701], 0)
+    mixer.forward(x, ctx, site, True)
+    module = ops.host._host("recurrent", "state_chunks")
+    fakes = {}
+    for name, (_, types, which) in entries.items():
+        def write_down(*args, which=which):
+            seen.extend(args[at] for at in which if args[at])
+            return 0
+        kept.append(ctypes.CFUNCTYPE(i, *types)(write_down))
+        fakes[name] = ctypes.cast(kept[-1], p).value
+    try:
+        module.setup(ops.KernelError, fakes)
+        mixer.forward(x, ctx, site, True)
+    finally:
+        module.setup(ops.KernelError, {name: ctypes.cast(getattr(library(source), name), p).value for name, (source, *_) in entries.items()})
+    assert len(seen) >= 4 and all(address % 128 == 0 for address in seen)
+
+
 def test_whoever_replaces_a_kernel_sees_its_calls():
     from qwenforge_b200.ops.timing import KernelTimer
     model = _model("qwen2.5-0.5b")
