@@ -88,11 +88,33 @@ bool rows16(const at::Tensor* t) {
 // tokens 203.5 / 196.8 / 195.5, 2,501 and 2,500 202.4 / 194.7 / 193.6 (a warp's loads meet a fifth line, its stores straddle sectors).
 long long whole_lines(long long floats) { return (floats + 63) / 64 * 64; }
 Stream stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
-bool ok(int code, const char* what) {
-    if (code == 0) return true;
-    if (code == 801) PyErr_Format(kernel_error, "%s: the driver offers no tensor-map encoder (cuTensorMapEncodeTiled)", what);
-    else PyErr_Format(kernel_error, "%s: CUDA error %d at launch", what, code);
-    return false;
+
+// What a launch was refused with; said once the interpreter's lock is held again.
+struct Refusal {
+    int code = 0;
+    const char* what = nullptr;
+    bool ok(int answer, const char* name) {
+        if (answer == 0) return true;
+        code = answer, what = name;
+        return false;
+    }
+};
+struct Unlocked {   // without the interpreter's lock, however the block is left
+    PyThreadState* state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+// What `launch` returns, run without the interpreter's lock, as the calls that it stands for are: a launch into a full queue and an allocation that
+// asks the driver may block, and a server's other threads go on meanwhile. (The caller's frame holds the tensors.)
+template <typename Launch> PyObject* unlocked(Launch launch) {
+    Refusal refused;
+    at::Tensor out;
+    {
+        Unlocked without;
+        out = launch(refused);
+    }
+    if (!refused.what) return THPVariable_Wrap(std::move(out));
+    if (refused.code == 801) return PyErr_Format(kernel_error, "%s: the driver offers no tensor-map encoder (cuTensorMapEncodeTiled)", refused.what);
+    return PyErr_Format(kernel_error, "%s: CUDA error %d at launch", refused.what, refused.code);
 }
 
 // rms_norm(hidden, delta or None, weight, eps) -> out: `add_rms_norm` into a new tensor.
@@ -106,11 +128,13 @@ PyObject* rms_norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_RETURN_NONE;
     const double eps = PyFloat_AsDouble(args[3]);
     if (PyErr_Occurred()) return nullptr;
-    at::Tensor out = at::empty(hidden->sizes(), weight->options());
-    if (!ok(add_rms_norm(weight->scalar_type() == at::kBFloat16, at_ptr<float>(*hidden), delta ? delta->data_ptr() : nullptr, weight->data_ptr(),
-                         out.data_ptr(), (int)hidden->size(0), (int)hidden->size(1), (float)eps, 0, stream()), "add_rms_norm"))
-        return nullptr;
-    return THPVariable_Wrap(std::move(out));
+    return unlocked([&](Refusal& refused) {
+        at::Tensor out = at::empty(hidden->sizes(), weight->options());
+        if (!refused.ok(add_rms_norm(weight->scalar_type() == at::kBFloat16, at_ptr<float>(*hidden), delta ? delta->data_ptr() : nullptr, weight->data_ptr(),
+                             out.data_ptr(), (int)hidden->size(0), (int)hidden->size(1), (float)eps, 0, stream()), "add_rms_norm"))
+            return at::Tensor();
+        return out;
+    });
     END_HANDLE_TH_ERRORS
 }
 
@@ -138,25 +162,27 @@ PyObject* prompt_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
         (freq && (!whole(freq, at::kFloat) || 2 * freq->numel() > d)) || storage->dim() < 2 || !on16(*storage) || page % 8 ||
         page != 2 * kv * storage->size(-2) * d || seq->numel() != m || pos->numel() != m || slots->numel() < n_seqs || cu->numel() < n_seqs + 1)
         Py_RETURN_NONE;
-    at::Tensor q = at::empty({m, heads * d}, x->options()), attended = at::empty({m, heads * d}, x->options());
-    const Stream s = stream();
-    const float* angles = freq ? freq->const_data_ptr<float>() : nullptr;
-    if ((!freq || 2 * freq->numel() == d) && qkv_pairs_pays((int)m, (int)w->size(0), (int)k, (int)d)) {
-        const QkvArgs a = {bias ? bias->data_ptr() : nullptr, nullptr, ints(pos), ints(seq), ints(slots), q.data_ptr(), storage->data_ptr(), ints(table), page,
-                           (int)table->stride(0), (int)heads, (int)kv, (int)d, write != 0, angles};
-        if (!ok(qkv_pairs(x->data_ptr(), (int)x->stride(0), w->data_ptr(), (int)w->stride(0), (int)m, (int)k, &a, at_ptr<int>(*err), s), "qkv_product")) return nullptr;
-    } else {
-        at::Tensor qkv = at::linear(*x, *w);
-        if (!ok(rope_cache_write(1, qkv.data_ptr(), bias ? bias->data_ptr() : nullptr, (int)qkv.stride(0), ints(seq), ints(pos), ints(slots), angles,
-                                 freq ? (int)(2 * freq->numel()) : 0, (int)heads, q.data_ptr(), storage->data_ptr(), ints(table), page, (int)table->stride(0),
-                                 (int)kv, (int)d, write != 0, (int)m, at_ptr<int>(*err), s), "rope_cache_write"))
-            return nullptr;
-    }
-    if (!ok(prefill_tc(q.data_ptr(), attended.data_ptr(), ints(cu), ints(pos), ints(slots), storage->data_ptr(), ints(table), page, (int)table->stride(0),
-                       (int)kv, (int)d, (int)heads, (int)n_seqs, (int)m, (int)longest, (int)keys, (float)scale, (int)window, at_ptr<int>(*err), nullptr,
-                       0, s), "attention_prefill_tc"))
-        return nullptr;
-    return THPVariable_Wrap(at::linear(attended, *o));
+    return unlocked([&](Refusal& refused) {
+        at::Tensor q = at::empty({m, heads * d}, x->options()), attended = at::empty({m, heads * d}, x->options());
+        const Stream s = stream();
+        const float* angles = freq ? freq->const_data_ptr<float>() : nullptr;
+        if ((!freq || 2 * freq->numel() == d) && qkv_pairs_pays((int)m, (int)w->size(0), (int)k, (int)d)) {
+            const QkvArgs a = {bias ? bias->data_ptr() : nullptr, nullptr, ints(pos), ints(seq), ints(slots), q.data_ptr(), storage->data_ptr(), ints(table), page,
+                               (int)table->stride(0), (int)heads, (int)kv, (int)d, write != 0, angles};
+            if (!refused.ok(qkv_pairs(x->data_ptr(), (int)x->stride(0), w->data_ptr(), (int)w->stride(0), (int)m, (int)k, &a, at_ptr<int>(*err), s), "qkv_product")) return at::Tensor();
+        } else {
+            at::Tensor qkv = at::linear(*x, *w);
+            if (!refused.ok(rope_cache_write(1, qkv.data_ptr(), bias ? bias->data_ptr() : nullptr, (int)qkv.stride(0), ints(seq), ints(pos), ints(slots), angles,
+                                     freq ? (int)(2 * freq->numel()) : 0, (int)heads, q.data_ptr(), storage->data_ptr(), ints(table), page, (int)table->stride(0),
+                                     (int)kv, (int)d, write != 0, (int)m, at_ptr<int>(*err), s), "rope_cache_write"))
+                return at::Tensor();
+        }
+        if (!refused.ok(prefill_tc(q.data_ptr(), attended.data_ptr(), ints(cu), ints(pos), ints(slots), storage->data_ptr(), ints(table), page, (int)table->stride(0),
+                           (int)kv, (int)d, (int)heads, (int)n_seqs, (int)m, (int)longest, (int)keys, (float)scale, (int)window, at_ptr<int>(*err), nullptr,
+                           0, s), "attention_prefill_tc"))
+            return at::Tensor();
+        return at::linear(attended, *o);
+    });
     END_HANDLE_TH_ERRORS
 }
 
@@ -171,16 +197,18 @@ PyObject* gated_feed_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_RETURN_NONE;
     const long long m = x->size(0), k = x->size(1), inter = gate_up->size(0) / 2;
     if (gate_up->size(0) != 2 * inter || inter % 8 || gate_up->size(1) != k || down->size(1) != inter) Py_RETURN_NONE;
-    at::Tensor act = at::empty({m, inter}, x->options());
-    if (tc_is_persistent(1, (int)m, (int)(2 * inter))) {
-        if (!ok(tc_gemm(1, x->data_ptr(), (int)x->stride(0), gate_up->data_ptr(), (int)gate_up->stride(0), act.data_ptr(), (int)inter, (int)m, (int)(2 * inter),
-                        (int)k, at_ptr<int>(*err), stream()), "tc_gemm"))
-            return nullptr;
-    } else {
-        at::Tensor both = at::linear(*x, *gate_up);
-        if (!ok(swiglu(1, both.data_ptr(), act.data_ptr(), (int)m, (int)inter, stream()), "swiglu")) return nullptr;
-    }
-    return THPVariable_Wrap(at::linear(act, *down));
+    return unlocked([&](Refusal& refused) {
+        at::Tensor act = at::empty({m, inter}, x->options());
+        if (tc_is_persistent(1, (int)m, (int)(2 * inter))) {
+            if (!refused.ok(tc_gemm(1, x->data_ptr(), (int)x->stride(0), gate_up->data_ptr(), (int)gate_up->stride(0), act.data_ptr(), (int)inter, (int)m, (int)(2 * inter),
+                            (int)k, at_ptr<int>(*err), stream()), "tc_gemm"))
+                return at::Tensor();
+        } else {
+            at::Tensor both = at::linear(*x, *gate_up);
+            if (!refused.ok(swiglu(1, both.data_ptr(), act.data_ptr(), (int)m, (int)inter, stream()), "swiglu")) return at::Tensor();
+        }
+        return at::linear(act, *down);
+    });
     END_HANDLE_TH_ERRORS
 }
 
@@ -206,27 +234,29 @@ PyObject* matrix_memory(PyObject*, PyObject* const* args, Py_ssize_t n) {
         joint->size(1) != x->size(1) || gate_bias->numel() != 2 * h || norm->numel() != inner || o->size(1) != inner || slots->numel() < seqs ||
         s_at < 0 || s_at + h * d * vd > floats || n_at < 0 || n_at + h * d > floats || m_at < 0 || m_at + h > floats || records <= 0 || each < 0)
         Py_RETURN_NONE;
-    at::Tensor proj = at::empty({t, main}, x->options()), out = at::empty({t, inner}, x->options());
-    const long long gates = whole_lines(t * h);
-    at::Tensor room = at::empty({6 * gates}, state->options()), made = at::empty({t * inner}, state->options());
-    at::Tensor kept = at::empty({records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0)}, state->options());
-    float* decay = at_ptr<float>(room);
-    float *take = decay + gates, *floor = take + gates, *nq = floor + gates, *pre = nq + gates, *y = at_ptr<float>(made), *scratch = at_ptr<float>(kept);
-    unsigned char* p = at_ptr<unsigned char>(proj);
-    const unsigned char *q = p, *k = p + 2 * h * d, *vals = p + 4 * h * d, *gate = vals + 2 * inner;
-    const Stream s = stream();
-    const long long slot = state->stride(0);
-    if (!ok(tc_gemm_tail(x->data_ptr(), (int)x->stride(0), joint->data_ptr(), (int)joint->stride(0), p, (int)main, pre, (int)t, (int)main, (int)(2 * h),
-                         (int)x->size(1), at_ptr<int>(*err), s), "tc_gemm_tail") ||
-        !ok(stabilized_gates(pre, (int)(2 * h), gate_bias->const_data_ptr<float>(), (float)cap, ints(cu), ints(slots), (int)seqs, at_ptr<float>(*state), slot,
-                             m_at, (int)h, decay, take, floor, s), "stabilized_gates") ||
-        !ok(state_chunks(q, (int)main, k, (int)main, vals, (int)main, decay, take, nullptr, nullptr, (int)h, ints(cu), ints(slots), (int)seqs, (int)longest,
-                         at_ptr<float>(*state), slot, s_at, n_at, (int)h, (int)h, (int)d, (int)vd, (float)std::pow((double)d, -0.5), scratch, records,
-                         (int)each, y, nq, s), "state_chunks") ||
-        !ok(gated_group_norm(1, y, gate, (int)main, norm->data_ptr(), (float)eps, out.data_ptr(), (int)t, (int)inner, (int)h, (int)h, 0, 0, nq, floor,
-                             (float)floor_add, nullptr, nullptr, 0, s), "gated_group_norm"))
-        return nullptr;
-    return THPVariable_Wrap(at::linear(out, *o));
+    return unlocked([&](Refusal& refused) {
+        at::Tensor proj = at::empty({t, main}, x->options()), out = at::empty({t, inner}, x->options());
+        const long long gates = whole_lines(t * h);
+        at::Tensor room = at::empty({6 * gates}, state->options()), made = at::empty({t * inner}, state->options());
+        at::Tensor kept = at::empty({records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0)}, state->options());
+        float* decay = at_ptr<float>(room);
+        float *take = decay + gates, *floor = take + gates, *nq = floor + gates, *pre = nq + gates, *y = at_ptr<float>(made), *scratch = at_ptr<float>(kept);
+        unsigned char* p = at_ptr<unsigned char>(proj);
+        const unsigned char *q = p, *k = p + 2 * h * d, *vals = p + 4 * h * d, *gate = vals + 2 * inner;
+        const Stream s = stream();
+        const long long slot = state->stride(0);
+        if (!refused.ok(tc_gemm_tail(x->data_ptr(), (int)x->stride(0), joint->data_ptr(), (int)joint->stride(0), p, (int)main, pre, (int)t, (int)main, (int)(2 * h),
+                             (int)x->size(1), at_ptr<int>(*err), s), "tc_gemm_tail") ||
+            !refused.ok(stabilized_gates(pre, (int)(2 * h), gate_bias->const_data_ptr<float>(), (float)cap, ints(cu), ints(slots), (int)seqs, at_ptr<float>(*state), slot,
+                                 m_at, (int)h, decay, take, floor, s), "stabilized_gates") ||
+            !refused.ok(state_chunks(q, (int)main, k, (int)main, vals, (int)main, decay, take, nullptr, nullptr, (int)h, ints(cu), ints(slots), (int)seqs, (int)longest,
+                             at_ptr<float>(*state), slot, s_at, n_at, (int)h, (int)h, (int)d, (int)vd, (float)std::pow((double)d, -0.5), scratch, records,
+                             (int)each, y, nq, s), "state_chunks") ||
+            !refused.ok(gated_group_norm(1, y, gate, (int)main, norm->data_ptr(), (float)eps, out.data_ptr(), (int)t, (int)inner, (int)h, (int)h, 0, 0, nq, floor,
+                                 (float)floor_add, nullptr, nullptr, 0, s), "gated_group_norm"))
+            return at::Tensor();
+        return at::linear(out, *o);
+    });
     END_HANDLE_TH_ERRORS
 }
 
@@ -257,24 +287,26 @@ PyObject* state_space(PyObject*, PyObject* const* args, Py_ssize_t n) {
         seq->numel() != m || slots->numel() < seqs || s_at < 0 || s_at + h * d * vd > state->size(1) || conv_at < 0 ||
         conv_at + (taps - 1) * channels > state->size(1) || records <= 0 || each < 0)
         Py_RETURN_NONE;
-    at::Tensor made = at::empty({m, main}, x->options()), mixed = at::empty({m, channels}, x->options()), out = at::empty({m, inner}, x->options());
-    at::Tensor pre = at::empty({m * h}, state->options()), sums = at::empty({m * inner}, state->options());
-    at::Tensor kept = at::empty({records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0)}, state->options());
-    float *dt = at_ptr<float>(pre), *y = at_ptr<float>(sums), *scratch = at_ptr<float>(kept);
-    const unsigned char *z = at_ptr<unsigned char>(made), *vals = at_ptr<unsigned char>(mixed), *k = vals + 2 * inner, *q = k + 2 * groups * d;
-    const Stream s = stream();
-    const long long slot = state->stride(0);
-    if (!ok(tc_gemm_tail(x->data_ptr(), (int)x->stride(0), joint->data_ptr(), (int)joint->stride(0), made.data_ptr(), (int)main, dt, (int)m, (int)main, (int)h,
-                         (int)x->size(1), at_ptr<int>(*err), s), "tc_gemm_tail") ||
-        !ok(causal_conv(1, z + 2 * inner, (int)main, conv_w->const_data_ptr<float>(), conv_b->const_data_ptr<float>(), ints(cu), ints(seq), ints(slots), (int)seqs,
-                        at_ptr<float>(*state), slot, conv_at, (int)taps, (int)m, (int)channels, mixed.data_ptr(), 0, 0, s), "causal_conv_silu") ||
-        !ok(state_chunks(q, (int)channels, k, (int)channels, vals, (int)channels, dt, nullptr, dt_bias->const_data_ptr<float>(), rate->const_data_ptr<float>(),
-                         (int)h, ints(cu), ints(slots), (int)seqs, (int)longest, at_ptr<float>(*state), slot, s_at, -1, (int)h, (int)groups, (int)d, (int)vd, 1.f,
-                         scratch, records, (int)each, y, nullptr, s), "state_chunks") ||
-        !ok(gated_group_norm(1, y, z, (int)main, norm->data_ptr(), (float)eps, out.data_ptr(), (int)m, (int)inner, (int)parts, (int)h, 1, 1, nullptr, nullptr, 0.f,
-                             skip->const_data_ptr<float>(), vals, (int)channels, s), "gated_group_norm"))
-        return nullptr;
-    return THPVariable_Wrap(at::linear(out, *o));
+    return unlocked([&](Refusal& refused) {
+        at::Tensor made = at::empty({m, main}, x->options()), mixed = at::empty({m, channels}, x->options()), out = at::empty({m, inner}, x->options());
+        at::Tensor pre = at::empty({m * h}, state->options()), sums = at::empty({m * inner}, state->options());
+        at::Tensor kept = at::empty({records * h * (d * vd + d + 1) + (each ? seqs * h * (d * vd + d) : 0)}, state->options());
+        float *dt = at_ptr<float>(pre), *y = at_ptr<float>(sums), *scratch = at_ptr<float>(kept);
+        const unsigned char *z = at_ptr<unsigned char>(made), *vals = at_ptr<unsigned char>(mixed), *k = vals + 2 * inner, *q = k + 2 * groups * d;
+        const Stream s = stream();
+        const long long slot = state->stride(0);
+        if (!refused.ok(tc_gemm_tail(x->data_ptr(), (int)x->stride(0), joint->data_ptr(), (int)joint->stride(0), made.data_ptr(), (int)main, dt, (int)m, (int)main, (int)h,
+                             (int)x->size(1), at_ptr<int>(*err), s), "tc_gemm_tail") ||
+            !refused.ok(causal_conv(1, z + 2 * inner, (int)main, conv_w->const_data_ptr<float>(), conv_b->const_data_ptr<float>(), ints(cu), ints(seq), ints(slots), (int)seqs,
+                            at_ptr<float>(*state), slot, conv_at, (int)taps, (int)m, (int)channels, mixed.data_ptr(), 0, 0, s), "causal_conv_silu") ||
+            !refused.ok(state_chunks(q, (int)channels, k, (int)channels, vals, (int)channels, dt, nullptr, dt_bias->const_data_ptr<float>(), rate->const_data_ptr<float>(),
+                             (int)h, ints(cu), ints(slots), (int)seqs, (int)longest, at_ptr<float>(*state), slot, s_at, -1, (int)h, (int)groups, (int)d, (int)vd, 1.f,
+                             scratch, records, (int)each, y, nullptr, s), "state_chunks") ||
+            !refused.ok(gated_group_norm(1, y, z, (int)main, norm->data_ptr(), (float)eps, out.data_ptr(), (int)m, (int)inner, (int)parts, (int)h, 1, 1, nullptr, nullptr, 0.f,
+                                 skip->const_data_ptr<float>(), vals, (int)channels, s), "gated_group_norm"))
+            return at::Tensor();
+        return at::linear(out, *o);
+    });
     END_HANDLE_TH_ERRORS
 }
 
@@ -300,20 +332,22 @@ PyObject* gated_linear_attention(PyObject*, PyObject* const* args, Py_ssize_t n)
         joint->size(1) != x->size(1) || a2->size(0) != h * d || bias->numel() != h * d || norm->numel() != inner || o->size(1) != inner ||
         slots->numel() < seqs || h * d * vd > state->size(1) || records <= 0 || each < 0)
         Py_RETURN_NONE;
-    at::Tensor all = at::linear(*x, *joint), pre = at::mm(all.narrow(1, main, rank), a2->t(), at::kFloat), out = at::empty({m, inner}, x->options());
-    TORCH_CHECK(on16(all) && on16(pre) && pre.is_contiguous(), "gated_linear_attention: the allocator's rows begin on no 16-byte boundary");
-    at::Tensor sums = at::empty({m * inner}, state->options());
-    at::Tensor kept = at::empty({records * h * (d * vd + d) + (each ? seqs * h * d * vd : 0) + m * h * d}, state->options());
-    float *y = at_ptr<float>(sums), *scratch = at_ptr<float>(kept);
-    const unsigned char *q = at_ptr<unsigned char>(all), *k = q + 2 * h * d, *vals = k + 2 * h * d, *gate = vals + 2 * inner;
-    const Stream s = stream();
-    if (!ok(row_chunks(q, (int)wide, k, (int)wide, vals, (int)wide, pre.const_data_ptr<float>(), bias->const_data_ptr<float>(), 2, (float)inv_tau, nullptr, ints(cu),
-                       ints(slots), (int)seqs, (int)longest, at_ptr<float>(*state), state->stride(0), 0, (int)h, (int)d, (int)vd, (float)std::pow((double)d, -0.5),
-                       scratch, records, (int)each, y, s), "row_chunks") ||
-        !ok(gated_group_norm(1, y, gate, (int)wide, norm->data_ptr(), (float)eps, out.data_ptr(), (int)m, (int)inner, (int)h, (int)h, 1, 0, nullptr, nullptr, 0.f,
-                             nullptr, nullptr, 0, s), "gated_group_norm"))
-        return nullptr;
-    return THPVariable_Wrap(at::linear(out, *o));
+    return unlocked([&](Refusal& refused) {
+        at::Tensor all = at::linear(*x, *joint), pre = at::mm(all.narrow(1, main, rank), a2->t(), at::kFloat), out = at::empty({m, inner}, x->options());
+        TORCH_CHECK(on16(all) && on16(pre) && pre.is_contiguous(), "gated_linear_attention: the allocator's rows begin on no 16-byte boundary");
+        at::Tensor sums = at::empty({m * inner}, state->options());
+        at::Tensor kept = at::empty({records * h * (d * vd + d) + (each ? seqs * h * d * vd : 0) + m * h * d}, state->options());
+        float *y = at_ptr<float>(sums), *scratch = at_ptr<float>(kept);
+        const unsigned char *q = at_ptr<unsigned char>(all), *k = q + 2 * h * d, *vals = k + 2 * h * d, *gate = vals + 2 * inner;
+        const Stream s = stream();
+        if (!refused.ok(row_chunks(q, (int)wide, k, (int)wide, vals, (int)wide, pre.const_data_ptr<float>(), bias->const_data_ptr<float>(), 2, (float)inv_tau, nullptr, ints(cu),
+                           ints(slots), (int)seqs, (int)longest, at_ptr<float>(*state), state->stride(0), 0, (int)h, (int)d, (int)vd, (float)std::pow((double)d, -0.5),
+                           scratch, records, (int)each, y, s), "row_chunks") ||
+            !refused.ok(gated_group_norm(1, y, gate, (int)wide, norm->data_ptr(), (float)eps, out.data_ptr(), (int)m, (int)inner, (int)h, (int)h, 1, 0, nullptr, nullptr, 0.f,
+                                 nullptr, nullptr, 0, s), "gated_group_norm"))
+            return at::Tensor();
+        return at::linear(out, *o);
+    });
     END_HANDLE_TH_ERRORS
 }
 

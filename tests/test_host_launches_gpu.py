@@ -151,3 +151,40 @@ def test_what_is_not_taken():
     assert ops.host.gated_feed_forward(x[:16], gate_up, down, err) is not None
     assert ops.host.gated_feed_forward(x[:, :892], gate_up[:, :892], down, err) is None                # a K of no whole pieces of eight
     assert ops.host.gated_feed_forward(x, gate_up, down[:, :4856], err) is None                        # shapes that do not agree
+
+
+def test_other_threads_run_while_a_launch_waits():
+    """Launches behind a busy stream until the driver's queue is full and one of them waits: another thread's clock goes on."""
+    import threading
+    import time
+
+    from qwenforge_b200 import ops
+    hidden, weight = torch.randn(8, 64, device=DEV), torch.ones(64, device=DEV).bfloat16()
+    norm = lambda: ops.host.rms_norm(hidden, None, weight, 1e-6)
+    assert norm() is not None
+    torch.cuda.synchronize()
+    gaps, done = [], threading.Event()
+
+    def clock():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(1e-3)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+    watcher = threading.Thread(target=clock)
+    torch.cuda._sleep(2_000_000_000)   # about a second
+    watcher.start()
+    began, longest = time.perf_counter(), 0.0
+    while time.perf_counter() - began < 0.2 or longest < 0.1:   # (until a call has waited)
+        at = time.perf_counter()
+        norm()
+        longest = max(longest, time.perf_counter() - at)
+        if time.perf_counter() - began > 5:
+            break
+    done.set()
+    watcher.join()
+    torch.cuda.synchronize()
+    if longest < 0.1:
+        pytest.skip("no launch waited on this machine")
+    assert max(gaps) < 0.5 * longest
