@@ -806,6 +806,8 @@ def _skinny_args(epilogue: int, weight: torch.Tensor, *, x: Optional[torch.Tenso
         _dev("bias", bias, torch.bfloat16)
         a.bias = bias.data_ptr()
     norm = hidden is not None
+    if pending is not None and (not norm or epilogue != EPI_QKV):
+        raise KernelError("skinny_gemm: pending goes with hidden and the QKV epilogue only")
     if norm:
         _dev("hidden", hidden, torch.float32)
         _dev("norm_weight", norm_weight, torch.bfloat16)
@@ -991,7 +993,7 @@ def wide_gemm(epilogue: int, weight: torch.Tensor, **tensors) -> None:
     """One fused product for up to 64 token rows on the tcgen05 tensor cores (csrc/wide_gemm.cu): the keywords of
     `skinny_gemm`, with the input rows always given as `x` [m, K] bf16 (already normalised)."""
     a, norm = _skinny_args(epilogue, weight, **tensors)
-    if norm:
+    if norm:   # (`pending` comes with `hidden` only)
         raise KernelError("wide_gemm: the input rows must be given as x (normalise them first)")
     code = library("wide_gemm").qf_wide_gemm(_I(epilogue), ctypes.byref(a), _stream())
     if code == 1:
@@ -1025,6 +1027,8 @@ _chain_answers: dict = {}
 def _chain_array(products):
     array = (_ChainProduct * len(products))()
     for i, product in enumerate(products):
+        if product.tensors.get("pending") is not None:
+            raise KernelError("skinny_chain: the chain kernel does not read pending; run the product alone")
         a, norm = _skinny_args(product.epilogue, product.weight, **product.tensors)
         array[i].epilogue, array[i].norm, array[i].a = product.epilogue, int(norm), a
     return array
@@ -1033,6 +1037,8 @@ def _chain_array(products):
 def skinny_chain_takes(products) -> bool:
     """Whether `skinny_chain` runs these products as ONE persistent kernel (the library's own planning, launching nothing)."""
     if not 1 <= len(products) <= CHAIN_MAX_PRODUCTS:
+        return False
+    if any(p.tensors.get("pending") is not None for p in products):   # (the chain kernel does not read it)
         return False
     key = tuple((p.epilogue, p.weight.shape, p.weight.stride(0), "hidden" in p.tensors,
                  (p.tensors.get("hidden") if "hidden" in p.tensors else p.tensors["x"]).shape[0],

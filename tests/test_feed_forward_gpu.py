@@ -109,6 +109,29 @@ def test_the_qkv_product_reads_stream_and_sums(rows):
         assert float((got.float() - want.float()).norm()) <= 2.0 ** -9 * float(want.float().norm())
 
 
+def test_pending_rows_are_refused_where_nothing_reads_them():
+    """With x in the place of the stream, with another epilogue, on the kernel of up to 64 rows and in a chain of products."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.measure import layer_products
+    products, _ = layer_products(2, 896, 1024, 14, 2, 64)
+    qkv = next(p for p in products if p.epilogue == ops.EPI_QKV)
+    rows = torch.zeros_like(qkv.tensors["hidden"])
+    by_x = {name: t for name, t in qkv.tensors.items() if name not in ("hidden", "norm_weight", "eps")}
+    by_x["x"] = rows.bfloat16()
+    for run in (ops.skinny_gemm, ops.wide_gemm):
+        run(ops.EPI_QKV, qkv.weight, **by_x)
+        with pytest.raises(ops.KernelError, match="pending"):
+            run(ops.EPI_QKV, qkv.weight, **by_x, pending=rows)
+    plain = dict(hidden=qkv.tensors["hidden"], norm_weight=qkv.tensors["norm_weight"], eps=1e-6, out=torch.empty(2, qkv.weight.shape[0], device=DEV))
+    ops.skinny_gemm(ops.EPI_PLAIN, qkv.weight, **plain)
+    with pytest.raises(ops.KernelError, match="pending"):
+        ops.skinny_gemm(ops.EPI_PLAIN, qkv.weight, **plain, pending=rows)
+    chained = ops.FusedProduct(ops.EPI_QKV, qkv.weight, **qkv.tensors, pending=rows)
+    assert not ops.skinny_chain_takes([chained])
+    with pytest.raises(ops.KernelError, match="pending"):
+        ops.skinny_chain([chained], torch.zeros(2, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV))
+
+
 @pytest.mark.parametrize("lengths", [[4100] * 8, [1] * 8, [700], [4100, 64, 65, 3000]])
 def test_a_plan_that_leaves_slots(lengths):
     """No more runs than fit beside what is left free (or one a sequence); the attention of either plan."""
