@@ -127,7 +127,7 @@ class Model:
     # ------------------------------------------------------------------ the step
     def forward(self, ctx: StepContext, cache: SequenceCache) -> Optional[torch.Tensor]:
         """Run the schedule over the context's tokens; logits of ctx.want_rows (None if nothing is wanted)."""
-        ctx.step_memo = {}
+        ctx.step_memo = {"model.resolves_sums": True}   # (below)
         hidden = ctx.embedded if ctx.embedded is not None else self.embedding.forward(ctx.token_ids, ctx)
         delta = None
         # the embedding's output as it is, for stream parts that mix it in again later (the stream itself is updated in place)

@@ -39,7 +39,9 @@ class StepContext:
     # step's rows there); the model then starts at its first layer
     embedded: Optional[torch.Tensor] = None
     # what the parts of one step share: the model empties it before every run of its schedule; a part keeps there
-    # what it works out once per step for all layers of its kind (key: a tuple that starts with the part's own name)
+    # what it works out once per step for all layers of its kind (key: a tuple that starts with the part's own name).
+    # The model's own entry "model.resolves_sums": it sees to it that a `PendingSums` reaches the stream; whoever runs a block without that
+    # entry has a feed-forward's output in the stream, or as rows of its own, when the block returns
     step_memo: Optional[dict] = None
     # host copies, for parts that plan on the host (absent when a captured graph replays the step)
     host_slots: Optional[list] = None

@@ -67,11 +67,11 @@ class SwiGlu(FeedForward):
                 and ctx.n_tokens <= ops.WIDE_MAX_ROWS and self._ways(ctx) != ("unfused", "unfused"))
 
     def leaves_sums(self, hidden, ctx) -> bool:
-        """Whether `fused_forward` with nothing pending runs as one kernel and returns a `PendingSums`."""
-        return ctx.step_memo is not None and ops.feed_forward_takes(hidden.shape[0], self.gate_up_weight, self.down_weight)
+        """Whether `fused_forward` with nothing pending runs as one kernel and returns a `PendingSums`: where the model runs the layers."""
+        return bool(ctx.step_memo) and "model.resolves_sums" in ctx.step_memo and ops.feed_forward_takes(hidden.shape[0], self.gate_up_weight, self.down_weight)
 
     def fused_forward(self, hidden, rms, ctx, delta=None):
-        """Adds to the stream, or returns what is still to reach it."""
+        """Adds to the stream, or (`leaves_sums`) returns what is still to reach it."""
         if delta is None and self.leaves_sums(hidden, ctx):
             # the whole layer out of the SMs' shared memory, in one kernel; its output stands in rows of its own that all layers share
             key = ("swiglu.sums", tuple(hidden.shape))

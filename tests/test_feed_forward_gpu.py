@@ -67,6 +67,35 @@ def test_decode_steps_with_and_without(seqs, monkeypatch):
         assert float((a - b).norm()) < 2e-2 * float(b.norm())
 
 
+@pytest.mark.parametrize("rows", [1, 8])
+def test_a_layer_that_the_model_does_not_run(rows):
+    """A caller of `block.forward` has the feed-forward's output in the stream when the call returns, as with layers beyond the one kernel."""
+    import numpy as np
+    from qwenforge_b200 import ops
+    from qwenforge_b200.cache import SequenceCache
+    from qwenforge_b200.config import preset_config
+    from qwenforge_b200.engine import Model, build_context
+    model = Model.from_random(preset_config("qwen2.5-0.5b", num_hidden_layers=1, vocab_size=128), 5)
+    block = model.blocks[0]
+    cache = SequenceCache(model.cache_needs(), 64 * rows, rows, model.spec.max_positions, model.dtype, model.device)
+    slots = [cache.open() for _ in range(rows)]
+    cache.reserve([(s, 1) for s in slots])
+    cache.flush()
+    ctx = build_context([(s, 0, np.zeros(1, dtype=np.int32)) for s in slots], None, model.err, model.dtype, model.device, model.attention, model.decode_scratch)
+    before = torch.randn(rows, 896, generator=torch.Generator(device=DEV).manual_seed(rows), device=DEV)
+    ctx.step_memo = {}
+    stream = before.clone()
+    assert block.forward(stream, None, ctx, cache.site(0), True) is None
+    ctx.step_memo = {"model.resolves_sums": True}
+    left = before.clone()
+    pending = block.forward(left, None, ctx, cache.site(0), True)
+    assert ops.feed_forward_takes(rows, block.feed_forward.gate_up_weight, block.feed_forward.down_weight) and pending is not None
+    assert float((stream - left).norm()) > 0.1 * float(left.norm())
+    pending.add_to(left)
+    # both round the normalised rows and the activations to eight bits
+    assert float((stream - left).norm()) < 2.0 ** -8 * float(left.norm())
+
+
 @pytest.mark.parametrize("rows,heads,dim", [(1, 14, 64), (8, 14, 64), (3, 4, 96), (5, 2, 128)])
 def test_the_projection_moves_the_sums(rows, heads, dim):
     """With sums the stream is what it is without, plus the sums; zeros stay behind. (96: blocks of 32 inputs; the others of 64.)"""
