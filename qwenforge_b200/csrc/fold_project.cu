@@ -146,13 +146,21 @@ QF_EXPORT int qf_fold_project_takes(int rows, int n, int ldw, int n_heads, int h
     return fold_project_smem(n, FP_KS) <= 200 * 1024 ? 1 : 0;
 }
 
+// Whether a block takes 64 inputs: where there are sums, half the blocks of the other form, so that the feed-forward behind, a block to an SM's
+// whole shared memory, finds its SMs free (a decode step at 0.5B sizes, microseconds, 32 / 64 inputs: 1 sequence of 4,000 tokens 563 / 550, 4 613 /
+// 592, 8 671 / 648)
+static bool fold_project_whole(int n, int head_dim) { return head_dim % 64 == 0 && fold_project_smem(n, 64) <= 200 * 1024; }
+
+// Blocks of that form for a layer with sums (0: the blocks of 32 inputs run): 16 warps each, and none finds room beside a block of the decode attention.
+QF_EXPORT int qf_fold_project_large_blocks(int n, int n_heads, int head_dim) {
+    return fold_project_whole(n, head_dim) ? n_heads * head_dim / 64 : 0;
+}
+
 QF_EXPORT int qf_fold_project(const FoldProjectArgs* args, cudaStream_t stream) {
     const FoldProjectArgs& a = *args;
     if (!qf_fold_project_takes(a.rows, a.n, a.ldw, a.n_heads, a.head_dim, a.w, a.hidden) || a.max_splits < 1 || (uintptr_t)a.sums % 16)
         return (int)cudaErrorInvalidValue;
-    // 64 inputs a block where there are sums: half the blocks, so that the feed-forward behind, a block to an SM's whole shared memory, finds its
-    // SMs free (a decode step at 0.5B sizes, microseconds, 32 / 64 inputs: 1 sequence of 4,000 tokens 563 / 550, 4 613 / 592, 8 671 / 648)
-    const bool whole = a.sums && a.head_dim % 64 == 0 && fold_project_smem(a.n, 64) <= 200 * 1024;
+    const bool whole = a.sums && fold_project_whole(a.n, a.head_dim);
     const size_t smem = fold_project_smem(a.n, whole ? 64 : 32);
     auto kernel = whole ? fold_project_kernel<64, 512, true> : a.sums ? fold_project_kernel<32, 256, true> : fold_project_kernel<32, 256, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -583,6 +583,11 @@ def fold_project_takes(rows: int, weight: torch.Tensor, hidden: torch.Tensor, n_
 FOLD_PROJECT_MAX_REDUCTIONS = 150_000
 
 
+def fold_project_large_blocks(weight: torch.Tensor, n_heads: int, head_dim: int) -> int:
+    """How many blocks `fold_project` with sums runs with that find no room on an SM beside a block of the decode attention (0: its blocks are small)."""
+    return library("fold_project").qf_fold_project_large_blocks(_I(weight.shape[0]), _I(n_heads), _I(head_dim))
+
+
 def fold_project_pays(rows: int, weight: torch.Tensor) -> bool:
     """Whether `fold_project` is the faster way for this projection. What it saves is the attention kernel's life after
     its pages (about 3 microseconds); what it costs grows with the 16-byte reductions into the stream, rows x N / 4 from

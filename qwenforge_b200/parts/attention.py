@@ -477,7 +477,15 @@ class GqaAttention(Mixer):
         sums = None
         if isinstance(delta, PendingSums):   # (`takes_sums` has said yes)
             sums, delta = delta.sums, None
-        plan = self.decode_plan(ctx)
+        folds = self._folds(hidden, ctx, o_way)
+        # Before a feed-forward that takes the SMs' whole shared memory the projection's blocks may be few and large, and none of them fits beside an
+        # attention block: the plan leaves them SMs, so that they and the feed-forward behind them start under the attention (eight steps of 8
+        # sequences of 4,096 tokens at 0.5B sizes 5,241 -> 5,112 microseconds: 9 runs a sequence, 144 blocks, become 8 and 128;
+        # layers of 256 to 1,024 by 1,184 to 8,192 with 8 sequences of 4,000 within a hundredth). At the head sizes of such blocks an SM is one slot.
+        leave = 0
+        if folds and ctx.step_memo and ctx.step_memo.get("pre_norm.feed_forward_leaves_sums"):
+            leave = ops.fold_project_large_blocks(self.o_weight, self.n_heads, self.head_dim)
+        plan = self.decode_plan(ctx, leave)
         inv_freq, rot_dim = self.position.fused_rotary() if self.position is not None else (None, 0)
         args = ops.KvSiteArgs(site.storage, site.table, self.n_kv, self.head_dim)
         q = torch.empty((n, self.q_width), dtype=torch.bfloat16, device=hidden.device)
@@ -499,7 +507,7 @@ class GqaAttention(Mixer):
                 ops.rope_cache_write(ops.linear(x, self.qkv_weight), ctx.tok_seq, ctx.tok_pos, ctx.slots, inv_freq, rot_dim,
                                      self.n_heads, q, args, writes_cache, ctx.err, bias=self.qkv_bias_t)
         n_splits = self.decode_splits(ctx)
-        if self._folds(hidden, ctx, o_way):
+        if folds:
             # the attention kernel stops at its runs' partial results; the projection folds them on its way in
             ops.attention_decode(q, None, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs, self.scale,
                                  self.window, n_splits, ctx.decode_scratch, ctx.err, plan, fold_later=True)
@@ -515,15 +523,11 @@ class GqaAttention(Mixer):
         else:
             ops.residual_add(hidden, ops.linear(attended, self.o_weight))
 
-    def decode_plan(self, ctx) -> torch.Tensor:
+    def decode_plan(self, ctx, leave: int = 0) -> torch.Tensor:
         """Which block of the decode attention takes which run of which sequence: made once per step, by the first
-        layer of this shape that runs, and shared through the step's memo by the others."""
+        layer of this shape that runs, and shared through the step's memo by the others. `leave`: block slots that stay free."""
         n_splits = self.decode_splits(ctx)
         memo = ctx.step_memo if ctx.step_memo is not None else {}
-        # Before a feed-forward that takes the SMs' whole shared memory the output projection's blocks are few and large, and none of them fits beside
-        # an attention block: the plan leaves them SMs, so that they and the feed-forward behind them start under the attention (eight steps of 8
-        # sequences of 4,096 tokens at 0.5B sizes 5,241 -> 5,112 microseconds: 9 runs a sequence, 144 blocks, become 8 and 128)
-        leave = -(-self.q_width // 64) if memo.get("pre_norm.feed_forward_leaves_sums") else 0
         key = ("gqa_attention.decode_plan", self.n_kv, self.n_heads, self.head_dim, self.window, n_splits, self.chunk, leave)
         plan = memo.get(key)
         if plan is None:

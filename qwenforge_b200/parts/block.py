@@ -57,9 +57,10 @@ class PreNormBlock(Part):
             return self._forward_scaled(hidden, delta, ctx, site, writes_cache)
         rms = self.mixer_norm.fused_rms()
         if rms is not None and self.mixer.fused_takes(ctx):
-            ahead = self.feed_forward
-            if hasattr(ahead, "leaves_sums") and self.feed_forward_norm.fused_rms() is not None and ahead.fused_takes(ctx) and ahead.leaves_sums(hidden, ctx):
-                ctx.step_memo["pre_norm.feed_forward_leaves_sums"] = True   # (a decode attention's plan is made with that in mind)
+            if ctx.step_memo is not None:   # (a decode attention's plan is made with this layer's feed-forward in mind)
+                ahead = self.feed_forward
+                ctx.step_memo["pre_norm.feed_forward_leaves_sums"] = (hasattr(ahead, "leaves_sums") and self.feed_forward_norm.fused_rms() is not None
+                                                                      and ahead.fused_takes(ctx) and ahead.leaves_sums(hidden, ctx))
             self.mixer.fused_forward(hidden, rms, ctx, site, writes_cache, delta)
             delta = None
         else:

@@ -161,6 +161,28 @@ def test_pending_rows_are_refused_where_nothing_reads_them():
         ops.skinny_chain([chained], torch.zeros(2, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV))
 
 
+@pytest.mark.parametrize("heads,dim,folds,free", [(14, 64, True, 14), (8, 96, True, 0), (4, 128, True, 8), (14, 64, False, 0)])
+def test_a_plan_leaves_slots_for_large_blocks_only(heads, dim, folds, free, monkeypatch):
+    """The projection's blocks of 64 inputs; not those of 32 (heads of 96), and nothing where it does not fold the partial results."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.config import preset_config
+    from qwenforge_b200.engine import Model
+    model = Model.from_random(preset_config("qwen2.5-0.5b", num_hidden_layers=2, vocab_size=128, hidden_size=heads * dim, intermediate_size=1184,
+                                            num_attention_heads=heads, num_key_value_heads=2, head_dim=dim), 5)
+    left, ran = [], []
+    plan, forward = ops.attention_decode_plan, ops.feed_forward
+    monkeypatch.setattr(ops, "attention_decode_plan", lambda *a: (left.append(a[11] if len(a) > 11 else 0), plan(*a))[1])
+    monkeypatch.setattr(ops, "feed_forward", lambda *a, **k: (ran.append(1), forward(*a, **k))[1])
+    if not folds:
+        monkeypatch.setattr(ops, "fold_project_pays", lambda *a: False)
+    cache = model.new_cache(256, 2)
+    slots = [cache.open() for _ in range(2)]
+    model.step(cache, [(s, list(range(1, 20))) for s in slots])
+    model.step(cache, [(s, [5]) for s in slots])
+    model.raise_on_kernel_error()
+    assert left == [free] and len(ran) == 2
+
+
 @pytest.mark.parametrize("lengths", [[4100] * 8, [1] * 8, [700], [4100, 64, 65, 3000]])
 def test_a_plan_that_leaves_slots(lengths):
     """No more runs than fit beside what is left free (or one a sequence); the attention of either plan."""
