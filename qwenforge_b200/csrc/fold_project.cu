@@ -30,6 +30,7 @@ struct FoldProjectArgs {
     float* hidden;          // [rows][n]
     int rows, n, ldw, n_heads, head_dim, max_splits;
     float* sums;            // [rows][n] or null: moved into the stream on the way, zeros left behind (feed_forward.cu)
+    int settled;            // no kernel in flight writes `runs`: they are read before the wait for the kernel ahead
 };
 
 template <int KS, int THREADS, bool SUMS>
@@ -50,8 +51,9 @@ __global__ void __launch_bounds__(THREADS) fold_project_kernel(FoldProjectArgs a
     // (integer divisions behind the wait would be a part of the chain: 1 microsecond a layer)
     const int per = SUMS ? (a.n / 4 + gridDim.x - 1) / gridDim.x : 0, quad0 = blockIdx.x * per, quads = min(per, a.n / 4 - quad0);
     const int head = k0 / a.head_dim, d0 = k0 % a.head_dim;
-    // the plan is made before the step's first layer, by a kernel that lets none start early: a round trip that need not stand behind the wait
-    const int first_runs = (int)threadIdx.x < a.rows * KS ? a.runs[threadIdx.x / KS] : 1;
+    // a plan that was made before the step's first layer, by a kernel that lets none start early: a round trip that need not stand behind the wait
+    int first_runs = 1;
+    if (a.settled && (int)threadIdx.x < a.rows * KS) first_runs = a.runs[threadIdx.x / KS];
     grid_dependency_wait();
     __syncthreads();  // the zeros are in place before the folded rows go on top of them
 
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(THREADS) fold_project_kernel(FoldProjectArgs a
     // ---- fold: thread (row, d) takes input k0 + d of its row over the row's runs
     for (int item = threadIdx.x; item < a.rows * KS; item += THREADS) {
         const int r = item / KS, d = item % KS;
-        const int n_runs = min(max(item < THREADS ? first_runs : a.runs[r], 1), a.max_splits);
+        const int n_runs = min(max(a.settled && item < THREADS ? first_runs : a.runs[r], 1), a.max_splits);
         const size_t base = ((size_t)r * a.n_heads + head) * a.max_splits;
         const float2* ml = reinterpret_cast<const float2*>(a.part_ml) + base;
         const float* po = a.part_o + base * a.head_dim + d0 + d;

@@ -329,7 +329,7 @@ def measure_decode_attention(args) -> None:
                 kernels._ptr(stamps), kernels._stream()), "attention_decode")
             mid.record()
             if fold_later:
-                ops.fold_project(plan, scratch, o_w, hidden, heads, d, n_splits)
+                ops.fold_project(plan, scratch, o_w, hidden, heads, d, n_splits, settled=True)
             end.record()
             torch.cuda.synchronize()
         if int(err):

@@ -567,7 +567,7 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, tok
 
 class _FoldProjectArgs(ctypes.Structure):
     _fields_ = [("part_o", _P), ("part_ml", _P), ("runs", _P), ("w", _P), ("hidden", _P), ("rows", _I), ("n", _I),
-                ("ldw", _I), ("n_heads", _I), ("head_dim", _I), ("max_splits", _I), ("sums", _P)]
+                ("ldw", _I), ("n_heads", _I), ("head_dim", _I), ("max_splits", _I), ("sums", _P), ("settled", _I)]
 
 
 def fold_project_takes(rows: int, weight: torch.Tensor, hidden: torch.Tensor, n_heads: int, head_dim: int) -> bool:
@@ -597,11 +597,13 @@ def fold_project_pays(rows: int, weight: torch.Tensor) -> bool:
 
 
 def fold_project(plan: torch.Tensor, scratch: DecodeScratch, weight: torch.Tensor, hidden: torch.Tensor, n_heads: int,
-                 head_dim: int, n_splits: int, sums: Optional[torch.Tensor] = None) -> None:
+                 head_dim: int, n_splits: int, sums: Optional[torch.Tensor] = None, settled: bool = False) -> None:
     """hidden[r, :] += fold(the partial results of sequence r) @ weight^T, after `attention_decode(..., fold_later=True)`
     with the same `plan`, `scratch` and `n_splits` in a step whose row r is sequence r (one token per sequence).
     bfloat16 weight [N, n_heads * head_dim], float32 hidden [rows, N]; the blocks' shares are added with atomic
-    reductions, in no fixed order. `sums`: what `feed_forward` left; it goes into hidden as well, and zeros stay in its place."""
+    reductions, in no fixed order. `sums`: what `feed_forward` left; it goes into hidden as well, and zeros stay in its place.
+    `settled` promises that no kernel still in flight on the stream writes `plan` (made by `attention_decode_plan` ahead of a whole layer's
+    attention): it is then read while the kernel ahead ends. The weight is read so in any case."""
     _dev("weight", weight, torch.bfloat16, contiguous=False)
     _dev("hidden", hidden, torch.float32)
     rows = hidden.shape[0]
@@ -615,7 +617,7 @@ def fold_project(plan: torch.Tensor, scratch: DecodeScratch, weight: torch.Tenso
         raise KernelError("fold_project: the scratch does not hold this step's partial results")
     a = _FoldProjectArgs(scratch.part_o.data_ptr(), scratch.part_ml.data_ptr(), plan.data_ptr(), weight.data_ptr(),
                          hidden.data_ptr(), rows, weight.shape[0], weight.stride(0), n_heads, head_dim, n_splits,
-                         None if sums is None else sums.data_ptr())
+                         None if sums is None else sums.data_ptr(), int(bool(settled)))
     _check(library("fold_project").qf_fold_project(ctypes.byref(a), _stream()), "fold_project")
 
 

@@ -511,7 +511,7 @@ class GqaAttention(Mixer):
             # the attention kernel stops at its runs' partial results; the projection folds them on its way in
             ops.attention_decode(q, None, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs, self.scale,
                                  self.window, n_splits, ctx.decode_scratch, ctx.err, plan, fold_later=True)
-            ops.fold_project(plan, ctx.decode_scratch, self.o_weight, hidden, self.n_heads, self.head_dim, n_splits, sums)
+            ops.fold_project(plan, ctx.decode_scratch, self.o_weight, hidden, self.n_heads, self.head_dim, n_splits, sums, settled=True)
             return
         attended = torch.empty_like(q)
         ops.attention_decode(q, attended, ctx.cu_q, ctx.tok_pos, ctx.slots, args, self.n_heads, ctx.n_seqs,

@@ -119,6 +119,33 @@ def test_the_projection_moves_the_sums(rows, heads, dim):
     assert not bool(left.any()) and float((both - plain).abs().max()) < 57 * 2.0 ** -24 * 8
 
 
+@pytest.mark.parametrize("rows,dim,summed", [(1, 64, True), (8, 64, True), (7, 64, False), (16, 64, False), (13, 96, True), (16, 64, True)])
+def test_the_projection_reads_the_plan_before_or_behind_its_wait(rows, dim, summed):
+    """`settled` or not, up to more rows than a block has threads for at once: the same runs are folded."""
+    from qwenforge_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(rows + dim)
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device=DEV)
+    width, heads, splits = 272, 4, 3
+    scratch = ops.DecodeScratch(torch.device(DEV))
+    scratch.part_o = rnd(rows * heads * splits * dim)
+    scratch.part_ml = torch.rand(rows * heads * splits * 2, generator=g, device=DEV) + 0.5
+    plan = torch.tensor([1 + i % splits for i in range(16)], dtype=torch.int32, device=DEV)
+    weight, hidden, sums = (rnd(width, heads * dim) * 0.05).bfloat16(), rnd(rows, width), rnd(rows, width) if summed else None
+    streams = []
+    for settled in (False, True):
+        stream = hidden.clone()
+        ops.fold_project(plan, scratch, weight, stream, heads, dim, splits, None if sums is None else sums.clone(), settled=settled)
+        streams.append(stream)
+    n_runs = plan[:rows].long()
+    ml = scratch.part_ml.view(rows, heads, splits, 2).double()
+    live = (torch.arange(splits, device=DEV)[None] < n_runs[:, None])[:, None]
+    share = torch.where(live, 2.0 ** (ml[..., 0] - ml[..., 0].amax(-1, keepdim=True)), 0.0)   # (no more than a factor of 2 between the runs' maxima)
+    folded = (share[..., None] * scratch.part_o.view(rows, heads, splits, dim).double()).sum(2) / (share * ml[..., 1]).sum(2)[..., None]
+    want = hidden.double() + folded.reshape(rows, -1).bfloat16().double() @ weight.double().T + (0 if sums is None else sums.double())
+    for stream in streams:   # folded rows may round to the other of two neighbours in eight bits; shares of up to 12 blocks arrive in any order
+        assert float((stream.double() - want).norm()) < 2.0 ** -9 * float(want.norm())
+
+
 @pytest.mark.parametrize("rows", [1, 2, 4, 7, 8])
 def test_the_qkv_product_reads_stream_and_sums(rows):
     from qwenforge_b200 import ops
