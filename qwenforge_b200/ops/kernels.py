@@ -1096,9 +1096,14 @@ FEED_FORWARD_MAX_REDUCTIONS = 250_000
 
 def feed_forward_takes(rows: int, gate_up: torch.Tensor, down: torch.Tensor) -> bool:
     """Whether `feed_forward` takes `rows` rows of a SwiGLU layer [gate | up] [2 I, W], down [W, I] and is the faster way: bfloat16 weights
-    whose shares find room in the SMs' shared memory, and no more than 250,000 16-byte reductions (blocks x rows x W / 4). The reductions
-    grow with the rows and what one kernel saves does not: at 896 x 4,864 (122 blocks) a decode step gains 15 to 20 percent with 1 to 4 rows
-    (27,000 to 109,000 reductions) and 9 to 17 with 8 (218,000); more have not been measured. Two products otherwise."""
+    whose shares find room in the SMs' shared memory, no more than 250,000 16-byte reductions (blocks x rows x W / 4), and no more than 96
+    columns a block where W is below 256. The reductions grow with the rows and what one kernel saves does not. Twelve layers' decode steps with
+    300 positions, microseconds, two products / this: 896 x 4,864 317 / 262 with 1 row, 348 / 297 with 8 (218,000 reductions); 512 x 1,184 249 / 208
+    and 262 / 241; 256 x 4,096 244 / 195 and 267 / 209; 640 x 6,000 299 / 252 and 330 / 271; 1,024 x 3,000 with 4 rows 343 / 266; 128 x 9,472 237 /
+    228 and 268 / 247 (with `take_sums` behind every layer in a QKV product's place: 289, 309, 218, 250, 205, 219, 256, 274, 291, 217, 236). Beyond
+    250,000 it is ahead with 300 positions (1,536 x 1,184, 8 rows, 455,000 reductions: 386 / 333) and behind with 4,000 (384 / 395). Narrow layers
+    of many columns a block are one block's chain: 64 x 18,944 (128 columns) 227 / 274, 64 x 16,576 (112) 244 / 259, 192 x 18,944 283 / 294, but 64 x
+    14,208 (96) 277 / 243, 192 x 14,208 298 / 267 and 256 x 16,576 300 / 293. (64 x 11,840 is 3 percent behind with one row.)"""
     if not (gate_up.is_cuda and down.is_cuda and gate_up.dtype == torch.bfloat16 and down.dtype == torch.bfloat16 and rows <= 8):
         return False
     width, inter = down.shape
@@ -1106,7 +1111,7 @@ def feed_forward_takes(rows: int, gate_up: torch.Tensor, down: torch.Tensor) -> 
             or gate_up.data_ptr() % 16 or down.data_ptr() % 16):
         return False
     blocks = library("feed_forward").qf_feed_forward_blocks(_I(int(rows)), _I(width), _I(inter))
-    return blocks > 0 and blocks * rows * width // 4 <= FEED_FORWARD_MAX_REDUCTIONS
+    return blocks > 0 and blocks * rows * width // 4 <= FEED_FORWARD_MAX_REDUCTIONS and (width >= 256 or inter <= 96 * blocks)
 
 
 def feed_forward(hidden: torch.Tensor, norm_weight: torch.Tensor, eps: float, gate_up: torch.Tensor, down: torch.Tensor, sums: torch.Tensor,

@@ -1,4 +1,6 @@
 """The feed-forward of a step of few rows as one kernel, and the two kernels that take its sums along."""
+import ctypes
+
 import pytest
 import torch
 
@@ -18,8 +20,10 @@ def _layer(width, inter, rows, seed):
 @pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8])
 def test_against_float64(width, inter, rows):
     from qwenforge_b200 import ops
+    from qwenforge_b200.csrc import library
     hidden, norm, gate_up, down, before = _layer(width, inter, rows, width + inter + rows)
-    assert ops.feed_forward_takes(rows, gate_up, down) or rows * width * 148 // 4 > 250_000
+    blocks = library("feed_forward").qf_feed_forward_blocks(ctypes.c_int(rows), ctypes.c_int(width), ctypes.c_int(inter))
+    assert blocks > 0 and ops.feed_forward_takes(rows, gate_up, down) == (blocks * rows * width // 4 <= 250_000 and (width, inter) != (64, 18944))
     sums, kept, err = before.clone(), hidden.clone(), torch.zeros(1, dtype=torch.int32, device=DEV)
     ops.feed_forward(hidden, norm, 1e-6, gate_up, down, sums, err)
     h = hidden.double()
