@@ -228,13 +228,18 @@ decode_split_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16* __re
         mbar_init(&bars[warp][1], 1);
     }
     __syncwarp();
-    // the warp's first 32 page numbers, a lane each: looked up one by one they were a round trip behind the wait for every further page
-    const int my_table = lane < my_pages ? table_row[p_begin + warp + lane * DEC_WARPS] : -1;
+    // The number of the warp's first page, and a lane each those of its first 32: looked up when a page's turn came they were a round trip behind the
+    // wait for every further page. The many are asked for once the first page is on its way: microseconds of a decode step, each number by itself /
+    // all ahead of the first page / so: 0.5B, 4 and 8 sequences of 16,000 tokens 683 and 857 / 653 and 816 / 653 and 816, of 1,024 533 and 565 / 533
+    // and 565 / 531 and 562; eighteen layers with 16 heads of 128 and a capped score, 1 and 4 sequences of 256 2,728 and 2,805 / 2,736 and 2,815 /
+    // 2,730 and 2,808; thirty-six without a cap, 4 sequences of 300 1,844 / 1,856 / 1,860, of 2,048 1,920 / 1,895 / 1,896.
+    int my_table = -1;
+    const int table0 = my_pages > 0 ? table_row[p_begin + warp] : -1;
     auto half_live = [&](int i, int& page, int& key0) {
         if (i >= n_halves) return false;
         const int p = p_begin + warp + (i >> 1) * DEC_WARPS;
         key0 = p * QF_PAGE + (i & 1) * HALF;
-        page = (i >> 1) < 32 ? __shfl_sync(0xffffffffu, my_table, i >> 1) : table_row[p];
+        page = (i >> 1) == 0 ? table0 : (i >> 1) < 32 ? __shfl_sync(0xffffffffu, my_table, i >> 1) : table_row[p];
         if (page < 0) {
             if (lane == 0 && (i & 1) == 0) atomicOr(err, QF_ERR_NO_PAGE);
             return false;
@@ -280,6 +285,7 @@ decode_split_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16* __re
     const int page0_end = (p_begin + warp + 1) * QF_PAGE;
     const int n_early = n_halves == 0 ? 0 : page0_end <= L - 1 ? 2 : page0_end - HALF <= L - 1 ? 1 : 0;
     for (int i = 0; i < n_early; ++i) issue(i);
+    if (lane < my_pages) my_table = table_row[p_begin + warp + lane * DEC_WARPS];
     stamp(1);
     grid_dependency_wait();
     stamp(2);
