@@ -23,7 +23,7 @@ __device__ __forceinline__ float2 halves(f32x2 x) {
 }
 
 // A block makes a BM x BN tile with WM x WN warps; a warp makes (4 TM) x (8 TN) of it, its 4 x 8 lanes TM x TN each in runs of four rows
-// (two, where a lane's are no whole fours) and columns, so that the lanes of a warp read a k's rows and columns of both operands as whole
+// and columns (two columns, where a lane's are no whole fours), so that the lanes of a warp read a k's rows and columns of both operands as whole
 // pieces without conflicts. Which rows and columns a lane has: neighbouring lanes share one of the two, and a 16-byte load of eight pieces takes two cycles of
 // the shared memory, four where eight neighbours have eight (32 x 64 tiles 12 to 15% faster so, the larger ones up to 2%; 64 x 64 in few rounds
 // 1.5% slower, so not there). 16
@@ -39,13 +39,13 @@ __global__ void __launch_bounds__(32 * WM * WN, TM * TN >= 128 ? 256 / (32 * WM 
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                 float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int vec) {
     constexpr int THREADS = 32 * WM * WN, BM = 4 * TM * WM, BN = 8 * TN * WN, LA = BM + 4, LW = BN + 4, Q = BK / 4, SWAP = BK == 16 ? 8 : 4;
-    constexpr int A_EACH = (BM * Q + THREADS - 1) / THREADS, W_EACH = (BN * Q + THREADS - 1) / THREADS, RA = TM % 4 ? 2 : 4, RW = TN % 4 ? 2 : 4;
-    static_assert(TM % 2 == 0 && TN % 2 == 0 && BM % 16 == 0 && BN % 16 == 0, "whole runs");
+    constexpr int A_EACH = BM * Q / THREADS, W_EACH = BN * Q / THREADS, RW = TN % 4 ? 2 : 4;
+    static_assert(TM % 4 == 0 && TN % 2 == 0 && BM * Q % THREADS == 0 && BN * Q % THREADS == 0 && BM % 16 == 0 && BN % 16 == 0, "whole runs");
     __shared__ __align__(16) float a_s[2][BK][LA], w_s[2][BK][LW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     constexpr bool SHARED = !(TM == 8 && TN == 4);
-    const int row0 = (warp / WN) * 4 * TM + (SHARED ? lane >> 1 & 3 : lane >> 3) * RA;
+    const int row0 = (warp / WN) * 4 * TM + (SHARED ? lane >> 1 & 3 : lane >> 3) * 4;
     const int col0 = (warp % WN) * 8 * TN + (SHARED ? (lane & 1) | (lane >> 2 & 6) : lane & 7) * RW;
     f32x2 acc[TM / 2][TN];            // rows 2 i and 2 i + 1 of column j
 #pragma unroll
@@ -74,26 +74,24 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 #pragma unroll
         for (int u = 0; u < A_EACH; ++u) {
             const int i = threadIdx.x + u * THREADS;
-            a_next[u] = piece(A, lda, BM * Q % THREADS == 0 || i < BM * Q ? m0 + i / Q : M, M, k0 + (i % Q) * 4);
+            a_next[u] = piece(A, lda, m0 + i / Q, M, k0 + (i % Q) * 4);
         }
 #pragma unroll
         for (int u = 0; u < W_EACH; ++u) {
             const int i = threadIdx.x + u * THREADS;
-            w_next[u] = piece(W, ldw, BN * Q % THREADS == 0 || i < BN * Q ? n0 + i / Q : N, N, k0 + (i % Q) * 4);
+            w_next[u] = piece(W, ldw, n0 + i / Q, N, k0 + (i % Q) * 4);
         }
     };
     auto stash = [&](int buf) {
         const int k = (threadIdx.x % Q) * 4, swap = k / 8 * SWAP;
 #pragma unroll
         for (int u = 0; u < A_EACH; ++u) {
-            if (BM * Q % THREADS && threadIdx.x + u * THREADS >= BM * Q) continue;
             const int r = ((threadIdx.x + u * THREADS) / Q) ^ swap;
             a_s[buf][k][r] = a_next[u].x, a_s[buf][k + 1][r] = a_next[u].y;
             a_s[buf][k + 2][r] = a_next[u].z, a_s[buf][k + 3][r] = a_next[u].w;
         }
 #pragma unroll
         for (int u = 0; u < W_EACH; ++u) {
-            if (BN * Q % THREADS && threadIdx.x + u * THREADS >= BN * Q) continue;
             const int r = ((threadIdx.x + u * THREADS) / Q) ^ swap;
             w_s[buf][k][r] = w_next[u].x, w_s[buf][k + 1][r] = w_next[u].y;
             w_s[buf][k + 2][r] = w_next[u].z, w_s[buf][k + 3][r] = w_next[u].w;
@@ -109,13 +107,12 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
             f32x2 a[TM / 2];
             float w[TN];
 #pragma unroll
-            for (int i = 0; i < TM; i += RA) {
-                const float* p = &a_s[buf][k][(row0 + 4 * i) ^ (k / 8 * SWAP)];
-                if (RA == 4) { const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p); a[i / 2] = v.x, a[(i / 2 + 1) % (TM / 2)] = v.y; }
-                else a[i / 2] = *reinterpret_cast<const f32x2*>(p);
+            for (int i = 0; i < TM; i += 4) {   // runs of four rows, 16 rows apart
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&a_s[buf][k][(row0 + 4 * i) ^ (k / 8 * SWAP)]);
+                a[i / 2] = v.x, a[i / 2 + 1] = v.y;
             }
 #pragma unroll
-            for (int j = 0; j < TN; j += RW) {
+            for (int j = 0; j < TN; j += RW) {   // runs of four columns, 32 apart, or of two, 16 apart
                 const float* p = &w_s[buf][k][(col0 + 8 * j) ^ (k / 8 * SWAP)];
                 if (RW == 4) { const float4 v = *reinterpret_cast<const float4*>(p); w[j] = v.x, w[j + 1] = v.y, w[(j + 2) % TN] = v.z, w[(j + 3) % TN] = v.w; }
                 else { const float2 v = *reinterpret_cast<const float2*>(p); w[j] = v.x, w[j + 1] = v.y; }
@@ -136,7 +133,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     for (int i = 0; i < TM / 2; ++i) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int gm = m0 + row0 + 2 * i / RA * 4 * RA + (2 * i) % RA + h;
+            const int gm = m0 + row0 + (i / 2) * 16 + (2 * i) % 4 + h;
             if (gm >= M) continue;
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
@@ -229,12 +226,13 @@ gemm_f32_few_rows_kernel(const float* __restrict__ A, const float* __restrict__ 
     }
 }
 
-// The tile with which the busiest SM is done first: a first wait and a time per tile, measured at K = 896 in microseconds (1, 4 and 18
-// tiles per SM of 64 x 64 33, 92 and 380, of 32 x 64 24, 65 and 258; 1, 5 and 9 of 128 x 128 89, 385 and 683; 1, 6 and 12 of 96 x 128
-// 72, 339 and 662; 1, 2 and 12 of 96 x 64 47, 74 and 382; 1 and 8 of 96 x 96 61 and 371: 1,031 x 1,152 x 896 in one round of them 61
-// microseconds, in three of 64 x 64 73). Never the fastest by more than a twentieth: 64 x 128 and 64 x 256 with two
-// or four warps, 32 x 64 with two warps, 128 x 64. (With K a tile's time grows and its wait does not: the waits, which count here as at
-// K = 896, decide between tiles whose rounds take nearly the same time.)
+// The tile with which the busiest SM is done first: a first wait and a time per tile, measured at K = 896 in microseconds (between events, a launch's
+// 8 to 10 among them, 1 and 18 tiles per SM of 64 x 64 40 and 392, of 128 x 128 97 and 1,364, of 96 x 128 82 and 995, of 96 x 64 53 and 566, of
+// 96 x 96 67 and 825: a time per tile is a seventeenth of the difference; 1,031 x 1,152 x 896 in one round of 96 x 96 61 microseconds, in three of
+// 64 x 64 73). The 32 x 64 tile's time is the one that it had before its lanes shared operands; now 30 and 229, 11.7 a tile, with which it
+// would be taken in more places (700 x 2,048 x 2,048 165 / 155, 300 x 2,560 x 2,048 116 / 100, but 330 x 9,728 x 896 153 / 156). Never the
+// fastest by more than a twentieth: 64 x 128 and 64 x 256 with two or four warps, 32 x 64 with two warps, 128 x 64. (With K a tile's time grows
+// and its wait does not: the waits, which count here as at K = 896, decide between tiles whose rounds take nearly the same time.)
 static const struct { int bm, bn; float wait, each; } f32_tiles[] = {{96, 128, 18.f, 53.7f}, {128, 128, 13.5f, 74.5f}, {96, 64, 15.f, 30.f},
                                                                      {64, 64, 8.5f, 20.8f}, {32, 64, 8.f, 14.3f}, {96, 96, 17.f, 44.2f}};
 static int best_tile(int M, int N) {
