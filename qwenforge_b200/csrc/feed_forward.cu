@@ -6,7 +6,7 @@
 // reductions of it into `sums`, float32 [rows][width]. As two kernels (skinny_gemm.cu) the activations went through the L2 behind a second
 // kernel's launch. What bounds it is that chain, then the reductions, blocks x rows x width / 4 of them (218,000 for eight rows of 896 x 4,864; a
 // row: 5.4 microseconds from the end of the kernel ahead to its own, 8.9 for the two kernels). A decode step at Qwen2.5-0.5B sizes, microseconds,
-// two kernels / this one: 1 sequence of 1,024 tokens 626 / 517, 4 660 / 534, 8 671 / 564; 1 of 4,000 627 / 511, 8 669 / 609.
+// two kernels / this one: 1 sequence of 1,024 tokens 627 / 525, 4 667 / 544, 8 675 / 569; 1 of 4,000 627 / 525, 8 680 / 606.
 // `sums` is a buffer of its own, zero before the launch: added into the stream in place, a block's share would reach rows that other blocks are
 // still reading. The next layer's QKV product reads stream and sums together, and its output projection (fold_project.cu) moves the sums into
 // the stream and leaves zeros. The shares arrive in no fixed order, as there.

@@ -7,9 +7,9 @@
 // fold on instead, where it costs one trip that the projection has to make anyway (it would load the attended rows
 // at that point): hidden[r, :] += fold(partials of row r) @ W^T.
 //
-// So that no block reads more partials than it needs, the product is cut along K: block b owns the 32 inputs
-// [32 b, 32 b + 32), which lie inside ONE head, folds exactly those (rows x 32 numerators from each run), multiplies
-// them with its slice W[:, 32 b : 32 b + 32] (fetched by 16-byte asynchronous copies before the kernel waits for the
+// So that no block reads more partials than it needs, the product is cut along K: block b owns the KS inputs (32, or 64
+// beside sums) from KS b on, which lie inside ONE head, folds exactly those (rows x KS numerators from each run), multiplies
+// them with its KS columns of W (fetched by 16-byte asynchronous copies before the kernel waits for the
 // attention kernel, since no kernel writes weights) on the tensor cores (mma.sync m16n8k16, float32 accumulation),
 // and adds its [rows, N] share into the float32 residual stream with 16-byte vector reductions. The order in which
 // the blocks' shares arrive is not fixed, so the stream's last bits can differ from run to run, as they do for every
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(THREADS) fold_project_kernel(FoldProjectArgs a
     cp_async_wait<0>();
     __syncthreads();
 
-    // ---- product: warp w takes the outputs 16 g .. 16 g + 15 for g = w, w + 8, ...
+    // ---- product: warp w takes the outputs 16 g .. 16 g + 15 for g = w, w + the block's warps, ...
     uint32_t xa[KS / 16][4];
 #pragma unroll
     for (int ks = 0; ks < KS / 16; ++ks) ldmatrix_x4(xa[ks], x_s + (lane & 15) * LD + 16 * ks + (lane >> 4) * 8);
@@ -149,8 +149,8 @@ QF_EXPORT int qf_fold_project_takes(int rows, int n, int ldw, int n_heads, int h
 }
 
 // Whether a block takes 64 inputs: where there are sums, half the blocks of the other form, so that the feed-forward behind, a block to an SM's
-// whole shared memory, finds its SMs free (a decode step at 0.5B sizes, microseconds, 32 / 64 inputs: 1 sequence of 4,000 tokens 563 / 550, 4 613 /
-// 592, 8 671 / 648)
+// whole shared memory, finds its SMs free (a decode step at 0.5B sizes, microseconds, 32 / 64 inputs: 1 sequence of 4,000 tokens 541 / 525, 4 570 /
+// 554, 8 625 / 607)
 static bool fold_project_whole(int n, int head_dim) { return head_dim % 64 == 0 && fold_project_smem(n, 64) <= 200 * 1024; }
 
 // Blocks of that form for a layer with sums (0: the blocks of 32 inputs run): 16 warps each, and none finds room beside a block of the decode attention.
