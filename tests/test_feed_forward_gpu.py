@@ -71,6 +71,39 @@ def test_decode_steps_with_and_without(seqs, monkeypatch):
         assert float((a - b).norm()) < 2e-2 * float(b.norm())
 
 
+@pytest.mark.parametrize("takes", [True, False])
+def test_a_stack_whose_second_mixer_takes_the_sums_or_does_not(takes, monkeypatch):
+    """Sums that the next mixer reads, and sums that its block moves into the stream first; an observer sees every layer's stream as two products
+    leave it, also after the step."""
+    from qwenforge_b200 import ops
+    from qwenforge_b200.config import preset_config
+    from qwenforge_b200.engine import Model
+    model = Model.from_random(preset_config("qwen2.5-0.5b", num_hidden_layers=2, vocab_size=512), 3)
+    moved, ran = [], []
+    take, forward = ops.take_sums, ops.feed_forward
+    monkeypatch.setattr(ops, "take_sums", lambda *a: (moved.append(1), take(*a))[1])
+    monkeypatch.setattr(ops, "feed_forward", lambda *a, **k: (ran.append(1), forward(*a, **k))[1])
+    if not takes:
+        model.blocks[1].mixer.takes_sums = lambda *a: False
+    logits, seen = {}, {}
+    for on in (True, False):
+        if not on:
+            monkeypatch.setattr(ops, "feed_forward_takes", lambda *a: False)
+        cache = model.new_cache(64 * 3, 3)
+        slots = [cache.open() for _ in range(3)]
+        model.step(cache, [(s, list(range(1, 20 + 7 * i))) for i, s in enumerate(slots)])
+        kept = seen[on] = []
+        model.observer = lambda index, hidden, delta: kept.append((hidden.clone(), delta))
+        logits[on] = model.step(cache, [(s, [5 + i]) for i, s in enumerate(slots)])
+        model.observer = None
+    model.raise_on_kernel_error()
+    assert len(ran) == 2 and len(moved) == (1 if takes else 2)      # (once at the stack's end)
+    streams = {on: [h if d is None else h + d.float() for h, d in kept] for on, kept in seen.items()}
+    assert len(streams[True]) == 3 and any(d is not None and bool(d.any()) for _, d in seen[True])
+    for a, b in (*zip(streams[True], streams[False]), (logits[True], logits[False])):
+        assert float((a - b).norm()) < 2e-2 * float(b.norm())
+
+
 @pytest.mark.parametrize("rows", [1, 8])
 def test_a_layer_that_the_model_does_not_run(rows):
     """A caller of `block.forward` has the feed-forward's output in the stream when the call returns, as with layers beyond the one kernel."""
